@@ -25,15 +25,18 @@ enum : u64
     CSA_ST_UNSERVED         = 1ull << 3,   // an invariant of the doubling step did not hold
 };
 
+constexpr int CSA_COUNTS_WORD = 40;         // of d_scalars: the counters of a resident build (Build_Counts)
+constexpr int CSA_STATUS_WORD = 63;         // of d_scalars: the status word
+
 // One per (device, host thread): a stream, the device status word, a grow-only scratch arena and pinned
 // scalars for the small device-to-host reads of the build loop.
 struct csa_ctx
 {
     int device = 0;
     cudaStream_t stream = nullptr;
-    u64* d_status = nullptr;       // device status word
     u64* h_scalars = nullptr;      // pinned, 64 words
     u64* d_scalars = nullptr;      // device, 64 words
+    u64* d_status = nullptr;       // device status word: the last of d_scalars, so that a read-back of counters brings it along
     void* arena = nullptr;         // grow-only scratch
     size_t arena_bytes = 0;
     void* aux = nullptr;           // a second grow-only buffer, for data that must survive a regrowth of the arena
@@ -45,6 +48,7 @@ struct csa_ctx
     const u32* symbol_range = nullptr;     // optional first-symbol table of csa_partition_ids (see partition_install_symbol_ranges)
     u32* symbol_table = nullptr;           // the table's memory where csa_install_pivots made it (65536 words, owned)
     bool ties_in_any_order = false;        // set by callers whose sorts may leave records of equal keys in any order (see radix_sort.cu)
+    cudaEvent_t phase_event[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};     // phases of a resident build, made on first use
     void* pass_timer = nullptr;            // digit-pass event timing of the sorts on this context (owned by radix_sort.cu)
     // Extra streams ("lanes") of the chunked host-batch pipelines, each with an event; made on first use.
     static constexpr int LANES = 3;

@@ -17,10 +17,9 @@ extern "C" int csa_ctx_create(int device, csa_ctx** out)
     cudaError_t e;
     if((e = cudaSetDevice(device)) != cudaSuccess) return fail(e);
     if((e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
-    if((e = cudaMalloc(&ctx->d_status, sizeof(u64))) != cudaSuccess) return fail(e);
-    if((e = cudaMemset(ctx->d_status, 0, sizeof(u64))) != cudaSuccess) return fail(e);
     if((e = cudaMalloc(&ctx->d_scalars, 64 * sizeof(u64))) != cudaSuccess) return fail(e);
     if((e = cudaMemset(ctx->d_scalars, 0, 64 * sizeof(u64))) != cudaSuccess) return fail(e);
+    ctx->d_status = ctx->d_scalars + CSA_STATUS_WORD;
     if((e = cudaMallocHost(&ctx->h_scalars, 64 * sizeof(u64))) != cudaSuccess) return fail(e);
     std::memset(ctx->h_scalars, 0, 64 * sizeof(u64));
     *out = ctx;
@@ -36,11 +35,11 @@ extern "C" void csa_ctx_destroy(csa_ctx* ctx)
     for(int g = 0; g < CSA_MAX_GPUS; ++g) if(ctx->peer_open[g]) cudaIpcCloseMemHandle(ctx->peer_base[g]);
     if(ctx->arena) cudaFree(ctx->arena);
     if(ctx->aux) cudaFree(ctx->aux);
-    if(ctx->d_status) cudaFree(ctx->d_status);
     if(ctx->d_scalars) cudaFree(ctx->d_scalars);
     if(ctx->h_scalars) cudaFreeHost(ctx->h_scalars);
     if(ctx->host_aux) cudaFreeHost(ctx->host_aux);
     if(ctx->symbol_table) cudaFree(ctx->symbol_table);
+    for(auto e : ctx->phase_event) if(e) cudaEventDestroy(e);
     for(int l = 0; l < csa_ctx::LANES; ++l)
     {
         if(ctx->lane_event[l]) cudaEventDestroy(ctx->lane_event[l]);
@@ -54,9 +53,9 @@ extern "C" int csa_sync(csa_ctx* ctx, uint64_t* status_bits)
 {
     if(!ctx) return CSA_E_INVALID;
     CSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 63, ctx->d_status, sizeof(u64), cudaMemcpyDeviceToHost, ctx->stream));
+    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + CSA_STATUS_WORD, ctx->d_status, sizeof(u64), cudaMemcpyDeviceToHost, ctx->stream));
     CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const u64 bits = ctx->h_scalars[63];
+    const u64 bits = ctx->h_scalars[CSA_STATUS_WORD];
     if(status_bits) *status_bits = bits;
     if(bits != 0)
     {

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(1024) rank_carry_kernel(u32* __restrict__ agg,
 __global__ void __launch_bounds__(RANK_BLOCK) rank_apply_kernel(const u64* __restrict__ keys, const u32* pos, const u64 count,
                                                                const int prim_shift, const u32 fixed_head, const Isa_View isa, const Slot_Map map,
                                                                u32* sa, u32* __restrict__ next_head, u32* __restrict__ next_pos,
-                                                               const u32* __restrict__ agg, u64* __restrict__ updates)
+                                                               const u32* __restrict__ agg, u64* __restrict__ updates, const bool open_tied)
 {
     __shared__ u32 s_prim[RANK_BLOCK / 32], s_full[RANK_BLOCK / 32], s_act[RANK_BLOCK / 32];
     __shared__ u32 s_next_head[RANK_TILE], s_next_pos[RANK_TILE];     // the tile's tied records, gathered for a coalesced write
@@ -253,7 +253,8 @@ __global__ void __launch_bounds__(RANK_BLOCK) rank_apply_kernel(const u64* __res
             const u32 head = (prim_shift < 64) ? u32(k[i] >> prim_shift) : fixed_head;
             const u32 slot = head + (u32(idx) - group_start);
             const u32 new_head = head + (sub_start - group_start);
-            if(sa + slot != pos + idx) sa[slot] = ps[i];
+            if(open_tied && (f.active & (1u << i))) sa[slot] = 0xFFFFFFFFu;
+            else if(sa + slot != pos + idx) sa[slot] = ps[i];
             // The new rank goes straight into the inverse array, or, when the array is spread over several GPUs, into a list
             // of (position, rank) updates that is applied in address order (and, over several GPUs, routed to the positions' owners).
             const u32 global_rank = u32(global_of(map, head) + (new_head - head));      // a group lies inside one partition
@@ -338,7 +339,7 @@ int launch_keys_gen(csa_ctx* ctx, const u32* head, const u32* pos, u64 count, u6
 }
 
 int launch_rank_and_compact(csa_ctx* ctx, const u64* keys, const u32* pos, u64 count, int prim_shift, u32 fixed_head, Isa_View isa,
-                            Slot_Map map, u32* sa, u32* next_head, u32* next_pos, u64* act_count, u32* scratch, u64* updates)
+                            Slot_Map map, u32* sa, u32* next_head, u32* next_pos, u64* act_count, u32* scratch, u64* updates, bool open_tied)
 {
     if(count == 0) return CSA_OK;
     const u64 tiles = div_up(count, RANK_TILE);
@@ -347,7 +348,7 @@ int launch_rank_and_compact(csa_ctx* ctx, const u64* keys, const u32* pos, u64 c
     rank_carry_kernel<<<1, 1024, 0, ctx->stream>>>(scratch, tiles, act_count);
     CSA_LAUNCH_CHECK(ctx);
     rank_apply_kernel<<<unsigned(tiles), RANK_BLOCK, 0, ctx->stream>>>(keys, pos, count, prim_shift, fixed_head, isa, map, sa, next_head,
-                                                                       next_pos, scratch, updates);
+                                                                       next_pos, scratch, updates, open_tied);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -49,9 +49,10 @@ int launch_keys_gen(csa_ctx* ctx, const u32* head, const u32* pos, u64 count, u6
 // scratch holds 3 words per tile of RANK_TILE records.
 constexpr int RANK_BLOCK = 256, RANK_ITEMS = 8, RANK_TILE = RANK_BLOCK * RANK_ITEMS;
 // If `updates` is non-null the new ranks are not written into the inverse array but listed there, record i of the sorted
-// list as (position << 32) | rank, for a bulk exchange between GPUs.
+// list as (position << 32) | rank, for a bulk exchange between GPUs. With open_tied the slots of suffixes that are still tied
+// receive 0xFFFFFFFF instead of a position.
 int launch_rank_and_compact(csa_ctx* ctx, const u64* keys, const u32* pos, u64 count, int prim_shift, u32 fixed_head, Isa_View isa,
-                            Slot_Map map, u32* sa, u32* next_head, u32* next_pos, u64* act_count, u32* scratch, u64* updates = nullptr);
+                            Slot_Map map, u32* sa, u32* next_head, u32* next_pos, u64* act_count, u32* scratch, u64* updates = nullptr, bool open_tied = false);
 
 // ---- bulk exchange of ranks between GPUs (exchange.cu) ----------------------------------------------------------------
 // counts[g] += the records whose position (offset by h; positions at or past n are skipped) lies in shard g.
@@ -68,8 +69,7 @@ int launch_apply_updates(csa_ctx* ctx, u32* isa_local, const u64* upd, u64 count
 // The same after one keys-only radix pass on the top bits of the index (positions_bits of them are in use), so that the
 // writes of one stretch of the list fall into one L2-sized stretch of the array. alt holds count records; sort_ws is a
 // sort workspace. Short lists are applied directly.
-int apply_updates_in_address_order(csa_ctx* ctx, u32* isa_local, u64* upd, u64* alt, u64 count, int position_bits, void* sort_ws, size_t sort_ws_bytes,
-                                   bool every_position_once = false);
+int apply_updates_in_address_order(csa_ctx* ctx, u32* isa_local, u64* upd, u64* alt, u64 count, int position_bits, void* sort_ws, size_t sort_ws_bytes);
 // keys[k] = head[k] << sec_bits | (n - 1 + h - x if x = pos[k] + h >= n, else 0)
 int launch_keys_init(csa_ctx* ctx, const u32* head, const u32* pos, u64 count, u64 n, u64 h, int sec_bits, u64* keys);
 // keys[perm[j]] += resp[j] + h

@@ -1,0 +1,889 @@
+// Generation 0 of the resident build: the suffixes sorted by the first bits of their ENCODED symbols.
+//
+// Token ids are far from uniform: of the 16 bits of a symbol a Zipf text fills about 9.4, so a radix sort of raw symbols
+// spends nearly half of its digit passes on bits that say nothing, and four raw symbols (64 bits) still leave 30 % of the
+// suffixes of a 2e9-token text tied. Here the symbols are first given an order-preserving prefix code made from a sample of the
+// text (a weight-balanced binary tree over the 65536 symbols in numeric order: within 0.1 bit of the entropy on Zipf
+// text). Encoded suffixes have nearly uniform bits, which pays four times:
+//   * 42 bits tell 2e9 suffixes apart but for a few in a thousand (they cover about 4.4 symbols);
+//   * a record is 8 bytes, 32 key bits + 32 position bits, as the bits of the first split need not be kept;
+//   * a split by the TOP bits makes evenly filled buckets, so it needs no sampling of splitters, and as its order inside
+//     a bucket is free it needs no stable ranking and no look-back: two unordered splits of up to 10 + 11 bits leave buckets
+//     ("children") of about 2000 suffixes;
+//   * inside a child the keys are so even that a record's place follows from its key by interpolation, give or take a record
+//     or two: one block finishes a run of children in shared memory.
+// So a suffix is moved three times (two splits, one local sort) where a least-significant-digit sort of 64 bits moves it eight
+// times. Any text is sorted correctly; what an uneven text (one symbol repeated, a few symbols in a pattern) changes is only
+// how many children do not fit a block and go through the radix sort instead.
+//
+// It stands for select_pivots, partition and the sort of initial_rank (src/GPU_SACA.cu:290-364, 737-826, 1111-1331).
+#include "prefix_sort.cuh"
+
+#include <atomic>
+
+namespace
+{
+
+constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of an encoding block
+constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
+constexpr int MAX_B1 = 10, MAX_B2 = 11;
+constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
+constexpr int LOCAL_BLOCK = 512, LOCAL_ITEMS = 16, LOCAL_CAP = LOCAL_BLOCK * LOCAL_ITEMS;
+constexpr u32 LOCAL_CHUNK = LOCAL_CAP / 2;  // children that start inside one chunk of slots belong to one block
+
+// ---- the code ----------------------------------------------------------------------------------------------------------------
+
+constexpr int HIST_BLOCK = 1024;
+constexpr size_t HIST_SMEM = 65536 * 2;
+
+// Symbol counts of `vectors` pieces of 8 symbols spread evenly over the text (all pieces where vectors = whole pieces of the
+// text; the last n % 8 symbols are then counted too). A block counts in shared memory, two 16-bit counters a word: it takes
+// fewer than 65536 symbols.
+__global__ void __launch_bounds__(HIST_BLOCK) sample_symbols_kernel(const u16* __restrict__ T, const u64 n, const u64 vectors, u32* __restrict__ hist)
+{
+    extern __shared__ __align__(16) u32 h[];
+    for(u32 i = threadIdx.x; i < 32768; i += HIST_BLOCK) h[i] = 0;
+    __syncthreads();
+    const u64 pieces = n / 8;
+    for(u64 v = u64(blockIdx.x) * HIST_BLOCK + threadIdx.x; v < vectors; v += u64(gridDim.x) * HIST_BLOCK)
+    {
+        const u64 at = vectors == pieces ? v : v * pieces / vectors;
+        const uint4 q = reinterpret_cast<const uint4*>(T)[at];
+        const u32 w[4] = {q.x, q.y, q.z, q.w};
+        #pragma unroll
+        for(int k = 0; k < 4; ++k)
+        {
+            const u32 a = w[k] & 0xFFFFu, b = w[k] >> 16;
+            atomicAdd(&h[a >> 1], (a & 1) ? 0x10000u : 1u);
+            atomicAdd(&h[b >> 1], (b & 1) ? 0x10000u : 1u);
+        }
+    }
+    if(blockIdx.x == 0 && vectors == pieces && threadIdx.x < n % 8)
+    {
+        const u32 a = T[pieces * 8 + threadIdx.x];
+        atomicAdd(&h[a >> 1], (a & 1) ? 0x10000u : 1u);
+    }
+    __syncthreads();
+    for(u32 i = threadIdx.x; i < 32768; i += HIST_BLOCK)
+    {
+        const u32 c = h[i];
+        if(c & 0xFFFFu) atomicAdd(&hist[2 * i], c & 0xFFFFu);
+        if(c >> 16) atomicAdd(&hist[2 * i + 1], c >> 16);
+    }
+}
+
+__device__ __forceinline__ u32 warp_inclusive(u32 v)
+{
+    #pragma unroll
+    for(int o = 1; o < 32; o <<= 1)
+    {
+        const u32 t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if(int(lane_id()) >= o) v += t;
+    }
+    return v;
+}
+
+// Exclusive sum over the block's threads; every thread calls it. warp_tot: BLOCK / 32 words. Returns the exclusive sum, and the
+// total in `total`. Ends with a barrier.
+template <int BLOCK>
+__device__ __forceinline__ u32 block_exclusive(const u32 v, u32* warp_tot, u32& total)
+{
+    const u32 inc = warp_inclusive(v);
+    if(lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+    __syncthreads();
+    u32 pre = 0, all = 0;
+    #pragma unroll
+    for(int w = 0; w < BLOCK / 32; ++w)
+    {
+        const u32 t = warp_tot[w];
+        if(w < int(threadIdx.x >> 5)) pre += t;
+        all += t;
+    }
+    __syncthreads();
+    total = all;
+    return pre + inc - v;
+}
+
+// Prefix sums of the symbols' weights, scale * count + 1 (every symbol must have a code word: the sample may have missed it).
+__global__ void __launch_bounds__(1024) code_prefix_kernel(const u32* __restrict__ hist, const u32 scale, u32* __restrict__ prefix)
+{
+    __shared__ u32 warp_tot[32];
+    const uint4* src = reinterpret_cast<const uint4*>(hist) + threadIdx.x * 16;
+    u32 sum = 0;
+    uint4 c[16];
+    #pragma unroll
+    for(int i = 0; i < 16; ++i) { c[i] = src[i]; sum += scale * (c[i].x + c[i].y + c[i].z + c[i].w) + 4; }
+    u32 total;
+    u32 run = block_exclusive<1024>(sum, warp_tot, total);
+    uint4* dst = reinterpret_cast<uint4*>(prefix) + threadIdx.x * 16;
+    #pragma unroll
+    for(int i = 0; i < 16; ++i)
+    {
+        uint4 o;
+        o.x = run; run += scale * c[i].x + 1;
+        o.y = run; run += scale * c[i].y + 1;
+        o.z = run; run += scale * c[i].z + 1;
+        o.w = run; run += scale * c[i].w + 1;
+        dst[i] = o;
+    }
+    if(threadIdx.x == 1023) prefix[65536] = total;
+}
+
+// One symbol per thread walks down the tree: a node is a range of symbols, split where the weights of its halves come closest,
+// but never so that a half has more symbols than code words are left for it. All symbols of a node find the same split.
+__global__ void __launch_bounds__(256) code_assign_kernel(const u32* __restrict__ prefix, u32* __restrict__ code)
+{
+    const u32 s = blockIdx.x * 256 + threadIdx.x;
+    u32 lo = 0, hi = 65536, word = 0;
+    int left = CODE_MAX_LEN;            // bits left below the node
+    u32 plo = 0, phi = __ldg(prefix + 65536);
+    while(hi - lo > 1)
+    {
+        const u32 twice_mid = plo + phi;
+        u32 a = lo + 1, b = hi - 1;     // the split m: first boundary at or past the middle, kept inside (lo, hi)
+        while(a < b)
+        {
+            const u32 m = (a + b) >> 1;
+            if(2 * __ldg(prefix + m) >= twice_mid) b = m; else a = m + 1;
+        }
+        u32 m = a;
+        u32 pm = __ldg(prefix + m);
+        if(m > lo + 1)
+        {
+            const u32 pb = __ldg(prefix + m - 1);
+            if(2 * pm >= twice_mid && twice_mid - 2 * pb <= 2 * pm - twice_mid) { --m; pm = pb; }
+        }
+        const u32 room = 1u << (left - 1);
+        if(m - lo > room) { m = lo + room; pm = __ldg(prefix + m); }
+        else if(hi - m > room) { m = hi - room; pm = __ldg(prefix + m); }
+        --left;
+        if(s < m) { hi = m; phi = pm; }
+        else { lo = m; plo = pm; word |= 1u << (31 - (CODE_MAX_LEN - 1 - left)); }
+    }
+    code[s] = word | u32(CODE_MAX_LEN - left);
+}
+
+// ---- encoding a tile of the text ------------------------------------------------------------------------------------------------
+
+// A block of BLOCK threads takes BLOCK * TEXT_ITEMS consecutive symbols, of which the last LOOKAHEAD only complete the keys of
+// those before them: a tile yields the keys of TILE_POSITIONS suffixes.
+template <int BLOCK> constexpr int TILE_POSITIONS = BLOCK * TEXT_ITEMS - LOOKAHEAD;
+template <int BLOCK> constexpr int STREAM_WORDS = (BLOCK * TEXT_ITEMS * CODE_MAX_LEN / 32 + 4 + 3) / 4 * 4;
+
+// Writes the code words of the symbols [first, first + BLOCK * TEXT_ITEMS) one behind the other into `stream` (bit 31 of word 0
+// first) and returns the bit at which the thread's first symbol starts; ent holds its symbols' code entries. Symbols past the
+// text's end count as 0. first is a multiple of 16 and T is 16-byte aligned with CSA_TEXT_PAD readable symbols behind n.
+template <int BLOCK>
+__device__ __forceinline__ u32 encode_tile(const u16* __restrict__ T, const u64 n, const u64 first, const u32* __restrict__ code, u32* stream, u32* warp_tot,
+                                           u32 (&ent)[TEXT_ITEMS])
+{
+    const u64 at = first + u64(threadIdx.x) * TEXT_ITEMS;
+    u32 sym2[TEXT_ITEMS / 2];
+    if(at + TEXT_ITEMS <= n + CSA_TEXT_PAD)
+    {
+        const uint4 a = *reinterpret_cast<const uint4*>(T + at), b = *reinterpret_cast<const uint4*>(T + at + 8);
+        sym2[0] = a.x; sym2[1] = a.y; sym2[2] = a.z; sym2[3] = a.w;
+        sym2[4] = b.x; sym2[5] = b.y; sym2[6] = b.z; sym2[7] = b.w;
+    }
+    else
+    {
+        #pragma unroll
+        for(int i = 0; i < TEXT_ITEMS / 2; ++i)
+            sym2[i] = (at + 2 * i < n ? u32(T[at + 2 * i]) : 0u) | (at + 2 * i + 1 < n ? u32(T[at + 2 * i + 1]) << 16 : 0u);
+    }
+    for(u32 i = threadIdx.x; i < STREAM_WORDS<BLOCK> / 4; i += BLOCK) reinterpret_cast<uint4*>(stream)[i] = make_uint4(0, 0, 0, 0);
+    u32 bits = 0;
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i) ent[i] = __ldg(code + ((i & 1) ? sym2[i >> 1] >> 16 : sym2[i >> 1] & 0xFFFFu));
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i) bits += ent[i] & 31u;
+    u32 total;
+    const u32 begin = block_exclusive<BLOCK>(bits, warp_tot, total);      // its barriers also stand between the clearing and the writing
+    u32 word = begin >> 5, fill = begin & 31u, acc = 0;
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i)
+    {
+        const u32 c = ent[i] & ~31u, len = ent[i] & 31u;
+        acc |= c >> fill;
+        fill += len;
+        if(fill >= 32)
+        {
+            atomicOr(&stream[word++], acc);         // a word may be shared with the thread before or behind
+            fill -= 32;
+            acc = fill ? c << (len - fill) : 0u;
+        }
+    }
+    if(acc) atomicOr(&stream[word], acc);
+    __syncthreads();
+    return begin;
+}
+
+// The 64 bits of the stream from bit `off` on.
+__device__ __forceinline__ void stream_bits(const u32* stream, const u32 off, u32& high, u32& low)
+{
+    const u32 w = off >> 5, s = off & 31u;
+    const u32 a = stream[w], b = stream[w + 1], c = stream[w + 2];
+    high = __funnelshift_l(b, a, s);
+    low = __funnelshift_l(c, b, s);
+}
+
+// ---- first split: by the top bits, straight from the text -----------------------------------------------------------------------
+
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK) count_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits, u32* __restrict__ counts)
+{
+    extern __shared__ __align__(16) u32 smem_words[];
+    u32* const stream = smem_words;
+    u32* const cnt = stream + STREAM_WORDS<BLOCK>;
+    __shared__ u32 warp_tot[BLOCK / 32];
+    const u32 bins = 1u << bits;
+    for(u32 i = threadIdx.x; i < bins; i += BLOCK) cnt[i] = 0;
+    const u64 first = u64(blockIdx.x) * TILE_POSITIONS<BLOCK>;
+    u32 ent[TEXT_ITEMS];
+    u32 off = encode_tile<BLOCK>(T, n, first, code, stream, warp_tot, ent);
+    const u32 local = threadIdx.x * TEXT_ITEMS;
+    const u64 room = n - first;
+    const u32 valid = room < u64(TILE_POSITIONS<BLOCK>) ? u32(room) : u32(TILE_POSITIONS<BLOCK>);
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i)
+    {
+        const u32 w = off >> 5;
+        const u32 high = __funnelshift_l(stream[w + 1], stream[w], off & 31u);
+        if(local + i < valid) atomicAdd(&cnt[high >> (32 - bits)], 1u);
+        off += ent[i] & 31u;
+    }
+    __syncthreads();
+    for(u32 i = threadIdx.x; i < bins; i += BLOCK)
+        if(cnt[i]) atomicAdd(&counts[i], cnt[i]);
+}
+
+// Offsets of the parents and the work lists that follow from their sizes. one_level: there is no second split, the bins are
+// the children of one parent that holds everything.
+__global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restrict__ counts, const u32 bins, const u32 n, const int one_level, u32* __restrict__ cursor,
+                                                             u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ chunk0, u32* __restrict__ child_off, const u32 p,
+                                                             Build_Counts* __restrict__ stats)
+{
+    __shared__ u32 warp_tot[32];
+    __shared__ u32 part[CSA_MAX_PARTITIONS];
+    const u32 t = threadIdx.x;
+    for(u32 i = t; i < p; i += 1024) part[i] = 0;
+    const u32 c = t < bins ? (bins == 1 ? n : counts[t]) : 0;
+    u32 total;
+    const u32 off = block_exclusive<1024>(c, warp_tot, total);
+    if(t < bins) cursor[t] = off;
+    // the statistics' partitions: a bucket belongs to the p-th part of the suffix array in which it starts
+    if(c) atomicAdd(&part[u64(off) * p / n], c);
+    __syncthreads();
+    u32 formed = 0, longest = 0;
+    for(u32 i = t; i < p; i += 1024) { formed += part[i] != 0; longest = max(longest, part[i]); }
+    if(formed) { atomicAdd(&stats->partitions, formed); atomicMax(&stats->max_partition, longest); }
+    if(one_level)
+    {
+        if(t < bins) child_off[t] = off;
+        if(t == 0) { child_off[bins] = n; par_off[0] = 0; par_off[1] = n; chunk0[0] = 0; chunk0[1] = (n + LOCAL_CHUNK - 1) / LOCAL_CHUNK; }
+        return;
+    }
+    const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE, chunks = (c + LOCAL_CHUNK - 1) / LOCAL_CHUNK;
+    u32 all_tiles, all_chunks;
+    const u32 t0 = block_exclusive<1024>(tiles, warp_tot, all_tiles);
+    const u32 c0 = block_exclusive<1024>(chunks, warp_tot, all_chunks);
+    if(t < bins) { par_off[t] = off; tile0[t] = t0; chunk0[t] = c0; }
+    if(t == 0) { par_off[bins] = n; tile0[bins] = all_tiles; chunk0[bins] = all_chunks; }
+}
+
+template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<BLOCK>) * 8 + size_t(TILE_POSITIONS<BLOCK>) * 2;
+static_assert(SCATTER_TEXT_SMEM<512> >= STREAM_WORDS<512> * 4 && SCATTER_TEXT_SMEM<128> >= STREAM_WORDS<128> * 4, "the stream lies where the records are staged later");
+
+// Scatter by the top `bits` bits: the places inside a bucket come from shared-memory atomics and, for the tile's run of a bucket,
+// from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs.
+// keep_top: the record keeps the top bits (there is no second split), else its key starts behind them.
+template <int BLOCK>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits,
+                                                                          const int keep_top, u32* __restrict__ cursor, u64* __restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u32* const stream = reinterpret_cast<u32*>(smem_raw);
+    u64* const stage = reinterpret_cast<u64*>(smem_raw);
+    u16* const stage_bin = reinterpret_cast<u16*>(stage + TILE_POSITIONS<BLOCK>);
+    __shared__ u32 cnt[1 << MAX_B1];            // counts, then the bins' starts inside the tile
+    __shared__ u32 base[1 << MAX_B1];           // where the tile's run of a bin goes, minus the run's start
+    __shared__ u32 warp_tot[BLOCK / 32];
+    const u32 bins = 1u << bits;
+    for(u32 i = threadIdx.x; i < bins; i += BLOCK) cnt[i] = 0;
+    const u64 first = u64(blockIdx.x) * TILE_POSITIONS<BLOCK>;
+    u32 ent[TEXT_ITEMS];
+    u32 off = encode_tile<BLOCK>(T, n, first, code, stream, warp_tot, ent);
+    const u32 local = threadIdx.x * TEXT_ITEMS;
+    const u64 room = n - first;
+    const u32 valid = room < u64(TILE_POSITIONS<BLOCK>) ? u32(room) : u32(TILE_POSITIONS<BLOCK>);
+    u32 key[TEXT_ITEMS], place[TEXT_ITEMS];      // place: bin << 16 | rank inside the tile's run of the bin
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i)
+    {
+        u32 high, low;
+        stream_bits(stream, off, high, low);
+        off += ent[i] & 31u;
+        const u32 bin = bits ? high >> (32 - bits) : 0u;
+        key[i] = keep_top ? high : __funnelshift_l(low, high, bits);
+        place[i] = bin << 16;
+        if(local + i < valid) place[i] |= atomicAdd(&cnt[bin], 1u);
+    }
+    __syncthreads();
+    constexpr int PER = (1 << MAX_B1) / BLOCK;      // bins per thread
+    u32 mine[PER], sum = 0;
+    #pragma unroll
+    for(int k = 0; k < PER; ++k) { const u32 b = threadIdx.x * PER + k; mine[k] = b < bins ? cnt[b] : 0; sum += mine[k]; }
+    u32 total;
+    u32 run = block_exclusive<BLOCK>(sum, warp_tot, total);
+    #pragma unroll
+    for(int k = 0; k < PER; ++k)
+    {
+        const u32 b = threadIdx.x * PER + k;
+        if(b < bins)
+        {
+            cnt[b] = run;
+            if(mine[k]) base[b] = atomicAdd(&cursor[b], mine[k]) - run;
+        }
+        run += mine[k];
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < TEXT_ITEMS; ++i)
+        if(local + i < valid)
+        {
+            const u32 bin = place[i] >> 16, at = cnt[bin] + (place[i] & 0xFFFFu);
+            stage[at] = (u64(key[i]) << 32) | u32(first + local + i);
+            stage_bin[at] = u16(bin);
+        }
+    __syncthreads();
+    for(u32 j = threadIdx.x; j < valid; j += BLOCK) out[base[stage_bin[j]] + j] = stage[j];
+}
+
+// ---- second split: every parent by the next bits ----------------------------------------------------------------------------------
+
+// The parent whose run of blocks holds block `b` (first[p] <= b < first[p + 1]), found by all threads together; `found` is a
+// word of shared memory. Returns parents if there is none. Ends with a barrier.
+__device__ __forceinline__ u32 parent_of_block(const u32* __restrict__ first, const u32 parents, const u32 b, u32* found)
+{
+    if(threadIdx.x == 0) *found = parents;
+    __syncthreads();
+    for(u32 p = threadIdx.x; p < parents; p += blockDim.x)
+        if(__ldg(first + p) <= b && b < __ldg(first + p + 1)) *found = p;
+    __syncthreads();
+    return *found;
+}
+
+__global__ void __launch_bounds__(SPLIT_BLOCK) count_children_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ tile0,
+                                                                    const u32 parents, const int bits, u32* __restrict__ counts)
+{
+    __shared__ u32 cnt[1 << MAX_B2];
+    __shared__ u32 found;
+    const u32 children = 1u << bits;
+    for(u32 i = threadIdx.x; i < children; i += SPLIT_BLOCK) cnt[i] = 0;
+    const u32 p = parent_of_block(tile0, parents, blockIdx.x, &found);
+    if(p >= parents) return;
+    const u32 end = par_off[p + 1], first = par_off[p] + (blockIdx.x - tile0[p]) * SPLIT_TILE;
+    const u32 valid = end - first < u32(SPLIT_TILE) ? end - first : u32(SPLIT_TILE);
+    const u32* const words = reinterpret_cast<const u32*>(rec + first);
+    u32 k[SPLIT_ITEMS];
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+    {
+        const u32 j = threadIdx.x + i * SPLIT_BLOCK;
+        if(j < valid) k[i] = words[2 * j + 1];
+    }
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+        if(threadIdx.x + i * SPLIT_BLOCK < valid) atomicAdd(&cnt[k[i] >> (32 - bits)], 1u);
+    __syncthreads();
+    for(u32 i = threadIdx.x; i < children; i += SPLIT_BLOCK)
+        if(cnt[i]) atomicAdd(&counts[u64(p) * children + i], cnt[i]);
+}
+
+// One block per parent: the children's counts become their places (in counts, running) and their offsets (child_off).
+__global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ counts, const u32* __restrict__ par_off, const u32 parents, const u32 children,
+                                                            u32* __restrict__ child_off)
+{
+    __shared__ u32 warp_tot[32];
+    const u32 p = blockIdx.x, t = threadIdx.x;
+    u32* const c = counts + u64(p) * children;
+    const u32 i0 = 2 * t, i1 = 2 * t + 1;          // up to 2048 children
+    const u32 a = i0 < children ? c[i0] : 0, b = i1 < children ? c[i1] : 0;
+    u32 total;
+    const u32 off = par_off[p] + block_exclusive<1024>(a + b, warp_tot, total);
+    if(i0 < children) { c[i0] = off; child_off[u64(p) * children + i0] = off; }
+    if(i1 < children) { c[i1] = off + a; child_off[u64(p) * children + i1] = off + a; }
+    if(p == parents - 1 && t == 0) child_off[u64(parents) * children] = par_off[parents];
+}
+
+constexpr size_t SPLIT_SMEM = size_t(SPLIT_TILE) * 8;
+
+__global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ tile0,
+                                                                         const u32 parents, const int bits, u32* __restrict__ cursor, u64* __restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u64* const stage = reinterpret_cast<u64*>(smem_raw);
+    __shared__ u32 cnt[1 << MAX_B2];
+    __shared__ u32 base[1 << MAX_B2];
+    __shared__ u32 warp_tot[SPLIT_BLOCK / 32];
+    __shared__ u32 found;
+    const u32 children = 1u << bits;
+    for(u32 i = threadIdx.x; i < children; i += SPLIT_BLOCK) cnt[i] = 0;
+    const u32 p = parent_of_block(tile0, parents, blockIdx.x, &found);
+    if(p >= parents) return;
+    const u32 end = par_off[p + 1], first = par_off[p] + (blockIdx.x - tile0[p]) * SPLIT_TILE;
+    const u32 valid = end - first < u32(SPLIT_TILE) ? end - first : u32(SPLIT_TILE);
+    u64 r[SPLIT_ITEMS];
+    u32 place2[SPLIT_ITEMS / 2];         // ranks below 8192, two a register
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+    {
+        const u32 j = threadIdx.x + i * SPLIT_BLOCK;
+        if(j < valid) r[i] = rec[first + j];
+    }
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+    {
+        u32 at = 0;
+        if(threadIdx.x + i * SPLIT_BLOCK < valid) at = atomicAdd(&cnt[u32(r[i] >> 32) >> (32 - bits)], 1u);
+        if(i & 1) place2[i >> 1] |= at << 16; else place2[i >> 1] = at;
+    }
+    __syncthreads();
+    constexpr int PER = (1 << MAX_B2) / SPLIT_BLOCK;
+    u32 mine[PER], sum = 0;
+    #pragma unroll
+    for(int k = 0; k < PER; ++k) { const u32 b = threadIdx.x * PER + k; mine[k] = b < children ? cnt[b] : 0; sum += mine[k]; }
+    u32 total;
+    u32 run = block_exclusive<SPLIT_BLOCK>(sum, warp_tot, total);
+    #pragma unroll
+    for(int k = 0; k < PER; ++k)
+    {
+        const u32 b = threadIdx.x * PER + k;
+        if(b < children)
+        {
+            cnt[b] = run;
+            if(mine[k]) base[b] = atomicAdd(&cursor[u64(p) * children + b], mine[k]) - run;
+        }
+        run += mine[k];
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+        if(threadIdx.x + i * SPLIT_BLOCK < valid)
+            stage[cnt[u32(r[i] >> 32) >> (32 - bits)] + ((place2[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu)] = r[i];
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < SPLIT_ITEMS; ++i)
+    {
+        const u32 j = threadIdx.x + i * SPLIT_BLOCK;
+        if(j < valid)
+        {
+            const u64 v = stage[j];
+            out[base[u32(v >> 32) >> (32 - bits)] + j] = v;
+        }
+    }
+}
+
+// ---- local sort: runs of children in shared memory --------------------------------------------------------------------------------
+
+constexpr size_t LOCAL_SMEM = size_t(LOCAL_CAP) * 8 + (LOCAL_CAP / 2 + 4) * 4 + ((1 << MAX_B2) + 4) * 4;
+constexpr u32 LONG_BIN = 256;       // a bin with more records is not ordered by comparing all with all
+static_assert(LOCAL_CAP <= 8192, "slots of a batch take 13 bits");
+
+// Appends the records whose bit is set in `mask` (by their place in the sorted batch) to a list; returns, for the caller's
+// records, where the flagged records before word w begin (pre[w]) and the list position of the first (at). Every thread calls it.
+// pre: LOCAL_CAP / 32 words; slot: one word of shared memory.
+__device__ __forceinline__ u32 list_places(const u32* mask, u32* pre, u32* warp_tot, u32* slot, u32* count)
+{
+    static_assert(LOCAL_CAP / 32 <= LOCAL_BLOCK, "a thread per word");
+    const u32 c = threadIdx.x < LOCAL_CAP / 32 ? __popc(mask[threadIdx.x]) : 0;
+    u32 total;
+    const u32 before = block_exclusive<LOCAL_BLOCK>(c, warp_tot, total);
+    if(threadIdx.x < LOCAL_CAP / 32) pre[threadIdx.x] = before;
+    if(threadIdx.x == 0) *slot = total ? atomicAdd(count, total) : 0;
+    __syncthreads();
+    return *slot;
+}
+
+__global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ chunk0,
+                                                                   const u32 parents, const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa,
+                                                                   u64* __restrict__ list, const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u64* const stage = reinterpret_cast<u64*>(smem_raw);                            // [LOCAL_CAP]
+    u32* const bin = reinterpret_cast<u32*>(stage + LOCAL_CAP);                      // [LOCAL_CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
+    u16* const start = reinterpret_cast<u16*>(bin);
+    u32* const coff = bin + LOCAL_CAP / 2 + 4;                                       // [children + 1] offsets of the parent's children
+    __shared__ u32 mask_small[LOCAL_CAP / 32], mask_large[LOCAL_CAP / 32], pre[LOCAL_CAP / 32];
+    __shared__ u32 warp_tot[LOCAL_BLOCK / 32];
+    __shared__ u32 found, s_first, s_last, s_slot;
+    const u32 tid = threadIdx.x;
+    const u32 children = 1u << bits;
+    const int rbits = 32 - bits;                    // key bits behind the child's
+    const u32 rmask = rbits == 32 ? 0xFFFFFFFFu : (1u << rbits) - 1;
+
+    const u32 p = parent_of_block(chunk0, parents, blockIdx.x, &found);
+    if(p >= parents) return;
+    const u32 par_end = par_off[p + 1];
+    const u32 lo = par_off[p] + (blockIdx.x - chunk0[p]) * LOCAL_CHUNK;
+    const u32 hi = par_end - lo < LOCAL_CHUNK ? par_end : lo + LOCAL_CHUNK;
+    for(u32 d = tid; d <= children; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + u64(p) * children + d);
+    __syncthreads();
+    // the children that start in [lo, hi)
+    for(u32 d = tid; d <= children; d += LOCAL_BLOCK)
+    {
+        if(coff[d] >= lo && (d == 0 || coff[d - 1] < lo)) s_first = d;
+        if((coff[d] >= hi || d == children) && (d == 0 || coff[d - 1] < hi)) s_last = d;
+    }
+    __syncthreads();
+    u32 cur = s_first;
+    const u32 last = s_last;
+
+    while(cur < last)
+    {
+        // a batch: as many children as fit
+        u32 e = last;
+        const u32 base = coff[cur];
+        if(coff[e] - base > u32(LOCAL_CAP))
+        {
+            u32 a = cur, b = last;                  // the last e with coff[e] - base <= LOCAL_CAP
+            while(b - a > 1)
+            {
+                const u32 m = (a + b) >> 1;
+                if(coff[m] - base <= u32(LOCAL_CAP)) a = m; else b = m;
+            }
+            e = a;
+            if(e == cur)
+            {
+                // a child that does not fit: left to the radix sort
+                if(tid == 0)
+                {
+                    over[atomicAdd(&counts->oversize, 1u)] = p * children + cur;
+                    atomicAdd(&counts->oversize_records, coff[cur + 1] - base);
+                }
+                ++cur;
+                continue;
+            }
+        }
+        const u32 m = coff[e] - base;
+        cur = e;
+        if(m == 0) continue;
+
+        // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
+        for(u32 i = tid; i < m / 2 + 2; i += LOCAL_BLOCK) bin[i] = 0;
+        for(u32 i = tid; i < LOCAL_CAP / 32; i += LOCAL_BLOCK) { mask_small[i] = 0; mask_large[i] = 0; }
+        u64 r[LOCAL_ITEMS];
+        u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later place | head << 13 | tied << 26
+        #pragma unroll
+        for(int i = 0; i < LOCAL_ITEMS; ++i)
+        {
+            const u32 j = tid + i * LOCAL_BLOCK;
+            if(j < m) r[i] = rec[base + j];
+        }
+        __syncthreads();
+        auto bin_of = [&](const u32 key) -> u32
+        {
+            const u32 d = bits ? key >> rbits : 0u;
+            const u32 c0 = coff[d];
+            return c0 - base + u32((u64(key & rmask) * (coff[d + 1] - c0)) >> rbits);
+        };
+        #pragma unroll
+        for(int i = 0; i < LOCAL_ITEMS; ++i)
+            if(tid + i * LOCAL_BLOCK < m)
+            {
+                const u32 b = bin_of(u32(r[i] >> 32));
+                const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
+                pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
+            }
+        __syncthreads();
+        // exclusive sums of the bins' counts, in place; start[m] = m
+        u32 longest = 0;
+        {
+            constexpr int WORDS = LOCAL_CAP / 2 / LOCAL_BLOCK;      // 8 words, 16 bins a thread
+            u32 c[WORDS], sum = 0;
+            const u32 w0 = tid * WORDS;
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k)
+            {
+                c[k] = 2 * (w0 + k) < m ? bin[w0 + k] : 0;
+                const u32 a = c[k] & 0xFFFFu, b = c[k] >> 16;
+                sum += a + b;
+                longest = max(longest, max(a, b));
+            }
+            u32 total;
+            u32 run = block_exclusive<LOCAL_BLOCK>(sum, warp_tot, total);
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k)
+            {
+                const u32 a = run, b = run + (c[k] & 0xFFFFu);
+                run = b + (c[k] >> 16);
+                if(2 * (w0 + k) < m) bin[w0 + k] = a | (b << 16);
+            }
+            __syncthreads();
+            if(tid == 0) start[m] = u16(m);
+        }
+        const bool by_network = __syncthreads_or(longest > LONG_BIN);
+        #pragma unroll
+        for(int i = 0; i < LOCAL_ITEMS; ++i)
+            if(tid + i * LOCAL_BLOCK < m) stage[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = r[i];
+        __syncthreads();
+
+        if(!by_network)
+        {
+            // Order inside the bins: a record counts the smaller and the equal keys of its bin.
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            {
+                const u32 j = tid + i * LOCAL_BLOCK;
+                if(j >= m) break;
+                const u64 v = stage[j];
+                const u32 key = u32(v >> 32);
+                const u32 b = bin_of(key);
+                const u32 s = start[b], t = start[b + 1];
+                u32 less = 0, eq_before = 0, eq = 0;
+                for(u32 k = s; k < t; ++k)
+                {
+                    const u32 o = u32(stage[k] >> 32);
+                    less += o < key;
+                    const u32 same = o == key;
+                    eq += same;
+                    eq_before += same && k < j;
+                }
+                const u32 place = s + less + eq_before;
+                pl[i] = place | ((s + less) << 13) | (eq == 1 ? 0u : (eq <= SMALL_GROUP ? 1u << 26 : 2u << 26));
+                sa[base + place] = eq == 1 ? u32(v) : SA_OPEN;
+            }
+        }
+        else
+        {
+            // Many records in one bin: a sorting network over the batch (keys and positions), then every record finds its
+            // group's ends by bisection.
+            u32 size = 1;
+            while(size < m) size <<= 1;
+            for(u32 j = m + tid; j < size; j += LOCAL_BLOCK) stage[j] = ~0ull;
+            __syncthreads();
+            for(u32 k = 2; k <= size; k <<= 1)
+                for(u32 d = k >> 1; d > 0; d >>= 1)
+                {
+                    for(u32 t = tid; t < size / 2; t += LOCAL_BLOCK)
+                    {
+                        const u32 a = 2 * t - (t & (d - 1)), b = a + d;
+                        const u64 x = stage[a], y = stage[b];
+                        if((x > y) == ((a & k) == 0)) { stage[a] = y; stage[b] = x; }
+                    }
+                    __syncthreads();
+                }
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            {
+                const u32 j = tid + i * LOCAL_BLOCK;
+                if(j >= m) break;
+                const u64 v = stage[j];
+                const u32 key = u32(v >> 32);
+                u32 a = 0, b = j;                   // first record with this key
+                while(a < b) { const u32 mid = (a + b) >> 1; if(u32(stage[mid] >> 32) < key) a = mid + 1; else b = mid; }
+                u32 c = j + 1, f = m;               // first record behind with a greater key
+                while(c < f) { const u32 mid = (c + f) >> 1; if(u32(stage[mid] >> 32) <= key) c = mid + 1; else f = mid; }
+                const u32 eq = c - a;
+                pl[i] = j | (a << 13) | (eq == 1 ? 0u : (eq <= SMALL_GROUP ? 1u << 26 : 2u << 26));
+                sa[base + j] = eq == 1 ? u32(v) : SA_OPEN;
+            }
+        }
+        u32 tied = 0;
+        #pragma unroll
+        for(int i = 0; i < LOCAL_ITEMS; ++i)
+        {
+            if(tid + i * LOCAL_BLOCK >= m) break;
+            const u32 kind = pl[i] >> 26, place = pl[i] & 8191u;
+            tied |= kind;
+            if(kind == 1) atomicOr(&mask_small[place >> 5], 1u << (place & 31));
+            else if(kind == 2) atomicOr(&mask_large[place >> 5], 1u << (place & 31));
+        }
+        // The tied records go to the list in the order of their places, so that a group's records lie side by side.
+        for(u32 kind = 1; kind <= 2; ++kind)
+        {
+            if(!__syncthreads_or((tied & kind) != 0)) continue;
+            u32* const mask = kind == 1 ? mask_small : mask_large;
+            const u32 at = list_places(mask, pre, warp_tot, &s_slot, kind == 1 ? &counts->small : &counts->large);
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            {
+                const u32 j = tid + i * LOCAL_BLOCK;
+                if(j >= m) break;
+                if((pl[i] >> 26) == kind)
+                {
+                    const u32 place = pl[i] & 8191u;
+                    const u64 k = u64(at) + pre[place >> 5] + __popc(mask[place >> 5] & ((1u << (place & 31)) - 1));
+                    list[kind == 1 ? k : list_cap - 1 - k] = (u64(base + ((pl[i] >> 13) & 8191u)) << 32) | u32(stage[j]);
+                }
+            }
+            __syncthreads();
+        }
+        __syncthreads();        // the next batch reuses the shared arrays
+    }
+}
+
+// Every oversize child is copied by the blocks of one grid row (blockIdx.y): keys = (first slot << 32) | key, vals = position.
+__global__ void __launch_bounds__(256) gather_oversize_kernel(const u64* __restrict__ rec, const u32* __restrict__ over, const u32 oversize, const u32* __restrict__ child_off,
+                                                             u64* __restrict__ keys, u32* __restrict__ vals, u32* __restrict__ cursor)
+{
+    __shared__ u32 s_at;
+    for(u32 o = blockIdx.y; o < oversize; o += gridDim.y)
+    {
+        const u32 first = child_off[over[o]], end = child_off[over[o] + 1];
+        for(u64 b = u64(first) + u64(blockIdx.x) * 2048; b < end; b += u64(gridDim.x) * 2048)
+        {
+            const u32 c = end - b < 2048 ? u32(end - b) : 2048u;
+            if(threadIdx.x == 0) s_at = atomicAdd(cursor, c);
+            __syncthreads();
+            for(u32 j = threadIdx.x; j < c; j += 256)
+            {
+                const u64 v = rec[b + j];
+                keys[s_at + j] = (u64(first) << 32) | (v >> 32);
+                vals[s_at + j] = u32(v);
+            }
+            __syncthreads();
+        }
+    }
+}
+
+template <typename K>
+int shared_bytes(csa_ctx* ctx, K kern, size_t bytes, std::atomic<bool>* configured)
+{
+    if(!configured[ctx->device & 63])
+    {
+        CSA_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+        configured[ctx->device & 63] = true;
+    }
+    return CSA_OK;
+}
+
+template <int BLOCK>
+int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, u32* counts)
+{
+    static std::atomic<bool> configured[64];
+    constexpr size_t smem = (STREAM_WORDS<BLOCK> + (1 << MAX_B1)) * 4;
+    CSA_TRY(shared_bytes(ctx, count_text_kernel<BLOCK>, smem, configured));
+    count_text_kernel<BLOCK><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, smem, ctx->stream>>>(T, n, code, bits, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+template <int BLOCK>
+int launch_scatter_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, int keep_top, u32* cursor, u64* out)
+{
+    static std::atomic<bool> configured[64];
+    CSA_TRY(shared_bytes(ctx, scatter_text_kernel<BLOCK>, SCATTER_TEXT_SMEM<BLOCK>, configured));
+    scatter_text_kernel<BLOCK><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, SCATTER_TEXT_SMEM<BLOCK>, ctx->stream>>>(T, n, code, bits, keep_top, cursor, out);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+}   // namespace
+
+Prefix_Sort prefix_sort_plan(u64 n)
+{
+    Prefix_Sort ps;
+    ps.n = n;
+    int t = 0;                                          // children of at most 2048 suffixes on average
+    while(t < MAX_B1 + MAX_B2 && (n >> t) > 2048) ++t;
+    ps.b1 = t <= MAX_B1 ? 0 : t / 2;
+    ps.b2 = t - ps.b1;
+    ps.key_bits = ps.b1 + 32;
+    ps.parents = 1u << ps.b1;
+    ps.children = 1u << ps.b2;
+    return ps;
+}
+
+size_t prefix_sort_table_bytes(const Prefix_Sort& ps)
+{
+    const u64 all = u64(ps.parents) * ps.children;
+    return align_up256(65536 * 4) * 2 + align_up256(65537 * 4) + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + 4096;
+}
+
+bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
+{
+    const u64 all = u64(ps.parents) * ps.children;
+    t.hist = cv.take<u32>(65536);
+    t.cnt1 = cv.take<u32>(size_t(1) << MAX_B1);        // directly behind hist: one clear covers both
+    t.prefix = cv.take<u32>(65537);
+    t.code = cv.take<u32>(65536);
+    t.cur1 = cv.take<u32>(size_t(1) << MAX_B1);
+    t.par_off = cv.take<u32>((size_t(1) << MAX_B1) + 1);
+    t.tile0 = cv.take<u32>((size_t(1) << MAX_B1) + 1);
+    t.chunk0 = cv.take<u32>((size_t(1) << MAX_B1) + 1);
+    t.cnt2 = cv.take<u32>(all);
+    t.child_off = cv.take<u32>(all + 1);
+    t.over = cv.take<u32>(all);
+    return cv.ok;
+}
+
+int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
+                       u64** list, u64** records, cudaEvent_t after_first_split)
+{
+    const u64 n = ps.n;
+    CSA_CUDA(ctx, cudaMemsetAsync(t.hist, 0, size_t(reinterpret_cast<u8*>(t.cnt1) - reinterpret_cast<u8*>(t.hist)) + (size_t(4) << MAX_B1), ctx->stream));
+    CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
+    // the code, from every symbol of a small text or a million of a large one
+    {
+        static std::atomic<bool> configured[64];
+        CSA_TRY(shared_bytes(ctx, sample_symbols_kernel, HIST_SMEM, configured));
+        const u64 pieces = n / 8, vectors = pieces < (u64(1) << 17) ? pieces : (u64(1) << 17);
+        const u64 samples = vectors == pieces ? n : vectors * 8;
+        const u64 blocks = div_up(vectors, HIST_BLOCK);
+        sample_symbols_kernel<<<unsigned(blocks < 1 ? 1 : (blocks > 148 ? 148 : blocks)), HIST_BLOCK, HIST_SMEM, ctx->stream>>>(T, n, vectors, t.hist);
+        CSA_LAUNCH_CHECK(ctx);
+        code_prefix_kernel<<<1, 1024, 0, ctx->stream>>>(t.hist, u32((u64(1) << 22) / samples ? (u64(1) << 22) / samples : 1), t.prefix);
+        CSA_LAUNCH_CHECK(ctx);
+        code_assign_kernel<<<256, 256, 0, ctx->stream>>>(t.prefix, t.code);
+        CSA_LAUNCH_CHECK(ctx);
+    }
+    const bool one_level = ps.b1 == 0;
+    const int bits = one_level ? ps.b2 : ps.b1;
+    const u32 bins = 1u << bits;
+    const bool wide = n >= (u64(1) << 22);          // small texts take small tiles, so that every SM gets one
+    if(bits > 0) CSA_TRY(wide ? launch_count_text<512>(ctx, T, n, t.code, bits, t.cnt1) : launch_count_text<128>(ctx, T, n, t.code, bits, t.cnt1));
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, bins, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, p, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    CSA_TRY(wide ? launch_scatter_text<512>(ctx, T, n, t.code, bits, one_level ? 1 : 0, t.cur1, recA)
+                 : launch_scatter_text<128>(ctx, T, n, t.code, bits, one_level ? 1 : 0, t.cur1, recA));
+    CSA_CUDA(ctx, cudaEventRecord(after_first_split, ctx->stream));
+    ctx->counters[1] += one_level ? 1 : 2;
+    ctx->counters[2] += one_level ? n : 2 * n;
+    u64* rec = recA;
+    u64* other = recB;
+    if(!one_level)
+    {
+        const unsigned tiles = unsigned(n / SPLIT_TILE + ps.parents);
+        CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(ps.parents) * ps.children * 4, ctx->stream));
+        count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, ps.parents, ps.b2, t.cnt2);
+        CSA_LAUNCH_CHECK(ctx);
+        child_offsets_kernel<<<ps.parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, ps.parents, ps.children, t.child_off);
+        CSA_LAUNCH_CHECK(ctx);
+        static std::atomic<bool> configured[64];
+        CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
+        scatter_children_kernel<<<tiles, SPLIT_BLOCK, SPLIT_SMEM, ctx->stream>>>(recA, t.par_off, t.tile0, ps.parents, ps.b2, t.cnt2, recB);
+        CSA_LAUNCH_CHECK(ctx);
+        rec = recB; other = recA;
+    }
+    {
+        static std::atomic<bool> configured[64];
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel, LOCAL_SMEM, configured));
+        local_sort_kernel<<<unsigned(n / LOCAL_CHUNK + ps.parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.par_off, t.chunk0, ps.parents, ps.b2, t.child_off, sa, other, n,
+                                                                                                          counts, t.over);
+        CSA_LAUNCH_CHECK(ctx);
+    }
+    *list = other;
+    *records = rec;
+    return CSA_OK;
+}
+
+int launch_gather_oversize(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, u32 oversize, const u64* records, u64* keys, u32* vals, u32* cursor)
+{
+    (void)ps;
+    if(oversize == 0) return CSA_OK;
+    CSA_CUDA(ctx, cudaMemsetAsync(cursor, 0, 4, ctx->stream));
+    gather_oversize_kernel<<<dim3(32, oversize < 1024 ? oversize : 1024), 256, 0, ctx->stream>>>(records, t.over, oversize, t.child_off, keys, vals, cursor);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}

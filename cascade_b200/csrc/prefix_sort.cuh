@@ -1,0 +1,65 @@
+// Internal declarations of the resident build's generation 0: suffixes sorted by the first bits of their encoded symbols.
+#pragma once
+#include "common.cuh"
+
+// An order-preserving prefix code of the 16-bit symbols: entry s of a 65536-word table holds the symbol's code word in the top
+// bits and its length (1 .. CODE_MAX_LEN) in the low 5 bits. Code words compare as their symbols do, so the bit strings of two
+// suffixes compare as the suffixes do, and frequent symbols take few bits.
+constexpr int CODE_MAX_LEN = 22;
+
+// Groups of up to this many tied suffixes are ordered inside one block; larger ones go through the radix sort.
+constexpr u32 SMALL_GROUP = 256;
+// What an entry of the suffix array holds while its suffix is still tied (no position: a resident build's n is below 2^32 - 2^26).
+constexpr u32 SA_OPEN = 0xFFFFFFFFu;
+
+// Counters that the kernels of a build leave for one another and for the host.
+struct Build_Counts
+{
+    u32 small;          // entries of the list of small tied groups (filled from the front of its buffer)
+    u32 large;          // entries of the list of large tied groups (filled from the back)
+    u32 oversize;       // children that did not fit a block's local sort
+    u32 oversize_records;
+    u32 next_small;     // the same of the list being made
+    u32 partitions;     // contiguous ranges of the suffix array, at most as many as asked for, that the first split's buckets form
+    u32 max_partition;  // suffixes of the largest
+    u32 pad;
+};
+static_assert(sizeof(Build_Counts) <= (CSA_STATUS_WORD - CSA_COUNTS_WORD) * 8, "the counters lie before the status word");
+
+struct Prefix_Sort
+{
+    u64 n;
+    int b1, b2;             // bits of the first and the second split; b1 = 0: one split (or none) of b2 bits
+    int key_bits;           // bits by which the suffixes end up sorted: b1 + 32
+    u32 parents, children;  // 1 << b1, 1 << b2
+};
+
+Prefix_Sort prefix_sort_plan(u64 n);
+// Device bytes of the tables (code, counts, offsets) beside the two record buffers of n 8-byte records.
+size_t prefix_sort_table_bytes(const Prefix_Sort& ps);
+
+struct Prefix_Tables
+{
+    u32* hist;          // 65536 symbol counts of the sample, cleared by the sort
+    u32* prefix;        // 65537 prefix sums of the symbols' weights
+    u32* code;          // 65536 entries of the code
+    u32* cnt1;          // [parents] records by first digit
+    u32* cur1;          // [parents] running places
+    u32* par_off;       // [parents + 1] where each parent starts in the suffix array
+    u32* tile0;         // [parents + 1] first tile of each parent in the second split
+    u32* chunk0;        // [parents + 1] first chunk of each parent in the local sort
+    u32* cnt2;          // [parents][children] records by second digit, then running places
+    u32* child_off;     // [parents * children + 1] where each child starts in the suffix array
+    u32* over;          // children that did not fit a block: their indices
+};
+bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t);
+
+// Orders the suffixes of T by the first key_bits bits of their encoding. recA and recB: n records each. sa receives every
+// suffix that is alone with its key, at its final place, and SA_OPEN elsewhere; the tied ones go to `list` (the record buffer
+// that is returned as *list; *records is the other one), small groups from the front, large ones from the back, as
+// (first slot of the group << 32) | position, group by group. p only says how many partitions the statistics tell apart. Nothing is read back.
+int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
+                       u64** list, u64** records, cudaEvent_t after_first_split);
+// The records of the children that did not fit a block, as sort records: keys = (first slot of the child << 32) | key,
+// vals = position.
+int launch_gather_oversize(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, u32 oversize, const u64* records, u64* keys, u32* vals, u32* cursor);

@@ -1,0 +1,30 @@
+// Internal declarations of the steps that order tied suffixes after the initial sort of the resident build.
+// A list holds (first slot of the group << 32) | position, group by group; small groups (up to SMALL_GROUP suffixes) fill a
+// list's buffer from the front, large ones from the back.
+#pragma once
+#include "common.cuh"
+#include "prefix_sort.cuh"
+
+// Orders the small groups of `list` by their suffixes' symbols [from, to) read straight from the text (a suffix that ends
+// inside them comes before those that go on): every group that is left shares `to` symbols. Suffixes that are alone now go to
+// their slots of sa, the others to next (front; counts->next_small entries). `expected`: about how many entries the list holds
+// (its length is counts->small).
+int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, Build_Counts* counts, u64 expected);
+
+// secs[i] = what the i-th entry of the list is ordered by in the generation that compares h symbols further on: the rank of the
+// suffix h symbols on, or, where the text ends before, a smaller number that falls with the position.
+constexpr u64 MAX_SMALL_H = u64(1) << 26;
+int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u64 h, u32* secs);
+// Orders the small groups of the list by secs; new ranks go into isa, single suffixes into sa, the others to `next` behind the
+// counts->next_small entries that are there.
+int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts);
+
+// Splits a list (heads, positions) of groups of any size into small groups (behind the counts->next_small entries at the front
+// of next) and large ones (in front of the counts->large entries at the back of next, which holds cap entries). The list holds
+// *count_dev entries, at most `most`. scratch: 2 words per RANK_TILE entries.
+int launch_split_by_size(csa_ctx* ctx, const u32* head, const u32* pos, u64 most, const u64* count_dev, u64* next, u64 cap, Build_Counts* counts, u32* scratch);
+// Heads and positions of the entries of a list.
+int launch_unpack_list(csa_ctx* ctx, const u64* list, u64 count, u32* head, u32* pos);
+
+// The inverse array from sa (final slots) and the lists of tied suffixes. updates: n entries of scratch and 256 words.
+int launch_make_inverse(csa_ctx* ctx, const u32* sa, u64 n, const u64* small_list, u64 small, const u64* large_list, u64 large, u32* isa, u64* updates);

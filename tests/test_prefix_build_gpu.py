@@ -1,0 +1,67 @@
+"""The resident build at the edges of its kernels' tiles and of its dispatch (one split or two, small and wide tiles), and on
+texts that take its rarer paths: children that do not fit a block, groups of more than 256 tied suffixes, bins with many
+records, suffixes that end inside the symbols compared. Each array byte for byte against the oracle's."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from cascade_b200 import api
+    c = api.Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, oracle, T):
+    from cascade_b200 import api
+    T = np.ascontiguousarray(T, dtype=np.uint16)
+    n = len(T)
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    sa, st = api.build_sa(ctx, Td, n, 8)
+    assert np.array_equal(sa[:5 * n].cpu().numpy(), oracle.build_sa40(T)[:5 * n])
+    return st
+
+
+def _zipf(n, seed, sigma=50257):
+    rng = np.random.default_rng(seed)
+    return np.minimum(rng.zipf(1.2, n), sigma).astype(np.uint16)
+
+
+# tile of 128 threads: 1984 positions; child: 2048 suffixes; batch of the local sort: 8192; window of a list: 1792 + 256;
+# second split above 2^21, wide tiles (8128 positions) from 2^22 on
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 63, 64, 65, 1983, 1984, 1985, 2047, 2048, 2049, 3968, 3969, 4096, 4097, 8191, 8192, 8193, 16385, (1 << 21) - 1, 1 << 21, (1 << 21) + 1,
+                               (1 << 22) - 1, (1 << 22) + 1])
+def test_sizes_at_the_edges(ctx, oracle, n):
+    _check(ctx, oracle, _zipf(n, n))
+
+
+@pytest.mark.parametrize("n", [257, 1793, 2049, 8193, 70_001, 2_200_000])
+@pytest.mark.parametrize("kind", ["one", "two", "period", "phrase", "stretch", "zeros_at_the_end", "wide"])
+def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
+    rng = np.random.default_rng(n)
+    if kind == "one":                   # one group of everything, halved by every generation
+        T = np.full(min(n, 70_001), 7)
+    elif kind == "two":
+        T = rng.integers(0, 2, n) * 9
+    elif kind == "period":              # a few huge groups
+        T = np.resize(rng.integers(0, 5, 7), min(n, 70_001))
+    elif kind == "phrase":              # a phrase of 12 symbols every 30: groups of thousands, and bins with as many records
+        T = rng.integers(0, 60000, n)
+        for k in range(12):
+            T[k + 5::30] = 1000 + k
+    elif kind == "stretch":             # copies of a long stretch: groups below and above 256 members, many generations
+        T = rng.integers(0, 3000, n)
+        L = max(8, n // 700)
+        for a in range(0, n - L, 2 * L):
+            T[a:a + L] = T[:L]
+    elif kind == "zeros_at_the_end":    # suffixes that differ from others by their end alone
+        T = rng.integers(0, 3, n)
+        T[-min(n, 300):] = 0
+    else:
+        T = rng.integers(0, 65536, n)
+    st = _check(ctx, oracle, T)
+    assert st.n == len(T) and 1 <= st.partitions <= 8 and 0 < st.max_partition <= len(T)
