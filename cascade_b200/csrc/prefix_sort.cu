@@ -104,39 +104,89 @@ __device__ __forceinline__ u32 block_exclusive(const u32 v, u32* warp_tot, u32& 
     return pre + inc - v;
 }
 
-// Prefix sums of the symbols' weights, scale * count + 1 (every symbol must have a code word: the sample may have missed it).
-__global__ void __launch_bounds__(1024) code_prefix_kernel(const u32* __restrict__ hist, const u32 scale, u32* __restrict__ prefix)
-{
-    __shared__ u32 warp_tot[32];
-    const uint4* src = reinterpret_cast<const uint4*>(hist) + threadIdx.x * 16;
-    u32 sum = 0;
-    uint4 c[16];
-    #pragma unroll
-    for(int i = 0; i < 16; ++i) { c[i] = src[i]; sum += scale * (c[i].x + c[i].y + c[i].z + c[i].w) + 4; }
-    u32 total;
-    u32 run = block_exclusive<1024>(sum, warp_tot, total);
-    uint4* dst = reinterpret_cast<uint4*>(prefix) + threadIdx.x * 16;
-    #pragma unroll
-    for(int i = 0; i < 16; ++i)
-    {
-        uint4 o;
-        o.x = run; run += scale * c[i].x + 1;
-        o.y = run; run += scale * c[i].y + 1;
-        o.z = run; run += scale * c[i].z + 1;
-        o.w = run; run += scale * c[i].w + 1;
-        dst[i] = o;
-    }
-    if(threadIdx.x == 1023) prefix[65536] = total;
-}
-
+// Weights and code words in one launch. Every block holds the prefix sums of all 65536 weights in shared memory, 24 bits each (16
+// and 8 apart), and gives CODE_BLOCK symbols their words; the weights are scale * count + 1 (every symbol must have a code word:
+// the sample may have missed it), below 2^23 together. COUNT: the text is short, and every block counts its symbols by itself.
+//
 // One symbol per thread walks down the tree: a node is a range of symbols, split where the weights of its halves come closest,
-// but never so that a half has more symbols than code words are left for it. All symbols of a node find the same split.
-__global__ void __launch_bounds__(256) code_assign_kernel(const u32* __restrict__ prefix, u32* __restrict__ code)
+// but never so that a half has more symbols than code words are left for it. All symbols of a node find the same split. The walk
+// is one chain of some 150 dependent reads, which is why the sums lie in shared memory: with the sums made by one block and read
+// through L2, the two launches took 98 us of a short build's 190.
+constexpr int CODE_BLOCK = 1024;
+constexpr u64 CODE_COUNT_MAX = 1 << 14;         // longest text that every block counts by itself (16-bit counters)
+constexpr u32 CODE_LOW_BYTES = (65536 + 8) * 2;
+constexpr size_t CODE_SMEM = CODE_LOW_BYTES + 65536 + 8;
+
+template <bool COUNT>
+__global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __restrict__ T, const u32 n, const u32* __restrict__ hist, const u32 scale, u32* __restrict__ code,
+                                                              u32* __restrict__ cnt1, u32* __restrict__ counts)
 {
-    const u32 s = blockIdx.x * 256 + threadIdx.x;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u16* const low = reinterpret_cast<u16*>(smem_raw);
+    u8* const high = smem_raw + CODE_LOW_BYTES;
+    __shared__ u32 warp_tot[CODE_BLOCK / 32];
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    if(blockIdx.x == 0)         // the counters that the kernels behind this one start from
+    {
+        cnt1[tid] = 0;
+        if(tid < sizeof(Build_Counts) / 4) counts[tid] = 0;
+    }
+    if(COUNT)
+    {
+        for(u32 i = tid; i < 65536 * 2 / 16; i += CODE_BLOCK) reinterpret_cast<uint4*>(low)[i] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        for(u32 i = tid; i < n; i += CODE_BLOCK)
+        {
+            const u32 a = T[i];
+            atomicAdd(reinterpret_cast<u32*>(low) + (a >> 1), (a & 1) ? 0x10000u : 1u);
+        }
+        __syncthreads();
+    }
+    // a warp sums 2048 consecutive symbols, 128 at a time
+    u32 run = 0;
+    #pragma unroll 8
+    for(int k = 0; k < 16; ++k)
+    {
+        const u32 s = warp * 2048 + k * 128 + lane * 4;
+        uint4 c;
+        if(COUNT)
+        {
+            const ushort4 v = *reinterpret_cast<const ushort4*>(low + s);
+            c = make_uint4(v.x, v.y, v.z, v.w);
+        }
+        else c = __ldg(reinterpret_cast<const uint4*>(hist + s));
+        const u32 sum = scale * (c.x + c.y + c.z + c.w) + 4;
+        const u32 inc = warp_inclusive(sum);
+        const u32 x = run + inc - sum, y = x + scale * c.x + 1, z = y + scale * c.y + 1, w = z + scale * c.z + 1;
+        *reinterpret_cast<ushort4*>(low + s) = make_ushort4(u16(x), u16(y), u16(z), u16(w));
+        *reinterpret_cast<uchar4*>(high + s) = make_uchar4(u8(x >> 16), u8(y >> 16), u8(z >> 16), u8(w >> 16));
+        run += __shfl_sync(0xFFFFFFFFu, inc, 31);
+    }
+    if(lane == 0) warp_tot[warp] = run;
+    __syncthreads();
+    {
+        u32 base = 0, all = 0;
+        #pragma unroll
+        for(int w = 0; w < CODE_BLOCK / 32; ++w) { const u32 t = warp_tot[w]; if(w < int(warp)) base += t; all += t; }
+        #pragma unroll 4
+        for(int k = 0; k < 16; ++k)
+        {
+            const u32 s = warp * 2048 + k * 128 + lane * 4;
+            const ushort4 l = *reinterpret_cast<const ushort4*>(low + s);
+            const uchar4 h = *reinterpret_cast<const uchar4*>(high + s);
+            const u32 x = base + (l.x | u32(h.x) << 16), y = base + (l.y | u32(h.y) << 16), z = base + (l.z | u32(h.z) << 16), w = base + (l.w | u32(h.w) << 16);
+            *reinterpret_cast<ushort4*>(low + s) = make_ushort4(u16(x), u16(y), u16(z), u16(w));
+            *reinterpret_cast<uchar4*>(high + s) = make_uchar4(u8(x >> 16), u8(y >> 16), u8(z >> 16), u8(w >> 16));
+        }
+        if(tid == 0) { low[65536] = u16(all); high[65536] = u8(all >> 16); }
+    }
+    __syncthreads();
+    auto prefix = [&](const u32 m) { return u32(low[m]) | u32(high[m]) << 16; };
+
+    const u32 s = blockIdx.x * CODE_BLOCK + tid;
     u32 lo = 0, hi = 65536, word = 0;
     int left = CODE_MAX_LEN;            // bits left below the node
-    u32 plo = 0, phi = __ldg(prefix + 65536);
+    u32 plo = 0, phi = prefix(65536);
     while(hi - lo > 1)
     {
         const u32 twice_mid = plo + phi;
@@ -144,18 +194,18 @@ __global__ void __launch_bounds__(256) code_assign_kernel(const u32* __restrict_
         while(a < b)
         {
             const u32 m = (a + b) >> 1;
-            if(2 * __ldg(prefix + m) >= twice_mid) b = m; else a = m + 1;
+            if(2 * prefix(m) >= twice_mid) b = m; else a = m + 1;
         }
         u32 m = a;
-        u32 pm = __ldg(prefix + m);
+        u32 pm = prefix(m);
         if(m > lo + 1)
         {
-            const u32 pb = __ldg(prefix + m - 1);
+            const u32 pb = prefix(m - 1);
             if(2 * pm >= twice_mid && twice_mid - 2 * pb <= 2 * pm - twice_mid) { --m; pm = pb; }
         }
         const u32 room = 1u << (left - 1);
-        if(m - lo > room) { m = lo + room; pm = __ldg(prefix + m); }
-        else if(hi - m > room) { m = hi - room; pm = __ldg(prefix + m); }
+        if(m - lo > room) { m = lo + room; pm = prefix(m); }
+        else if(hi - m > room) { m = hi - room; pm = prefix(m); }
         --left;
         if(s < m) { hi = m; phi = pm; }
         else { lo = m; plo = pm; word |= 1u << (31 - (CODE_MAX_LEN - 1 - left)); }
@@ -798,15 +848,14 @@ Prefix_Sort prefix_sort_plan(u64 n)
 size_t prefix_sort_table_bytes(const Prefix_Sort& ps)
 {
     const u64 all = u64(ps.parents) * ps.children;
-    return align_up256(65536 * 4) * 2 + align_up256(65537 * 4) + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + 4096;
+    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + 4096;
 }
 
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
 {
     const u64 all = u64(ps.parents) * ps.children;
     t.hist = cv.take<u32>(65536);
-    t.cnt1 = cv.take<u32>(size_t(1) << MAX_B1);        // directly behind hist: one clear covers both
-    t.prefix = cv.take<u32>(65537);
+    t.cnt1 = cv.take<u32>(size_t(1) << MAX_B1);
     t.code = cv.take<u32>(65536);
     t.cur1 = cv.take<u32>(size_t(1) << MAX_B1);
     t.par_off = cv.take<u32>((size_t(1) << MAX_B1) + 1);
@@ -822,20 +871,28 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
                        u64** list, u64** records, cudaEvent_t after_first_split)
 {
     const u64 n = ps.n;
-    CSA_CUDA(ctx, cudaMemsetAsync(t.hist, 0, size_t(reinterpret_cast<u8*>(t.cnt1) - reinterpret_cast<u8*>(t.hist)) + (size_t(4) << MAX_B1), ctx->stream));
-    CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
     // the code, from every symbol of a small text or a million of a large one
+    static_assert(CODE_BLOCK == 1 << MAX_B1, "block 0 of make_code_kernel clears a counter of the first split per thread");
+    if(n <= CODE_COUNT_MAX)
     {
         static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, sample_symbols_kernel, HIST_SMEM, configured));
+        CSA_TRY(shared_bytes(ctx, make_code_kernel<true>, CODE_SMEM, configured));
+        make_code_kernel<true><<<65536 / CODE_BLOCK, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), nullptr, u32((u64(1) << 22) / n), t.code, t.cnt1, reinterpret_cast<u32*>(counts));
+        CSA_LAUNCH_CHECK(ctx);
+    }
+    else
+    {
+        static std::atomic<bool> configured[2][64];
+        CSA_TRY(shared_bytes(ctx, sample_symbols_kernel, HIST_SMEM, configured[0]));
+        CSA_TRY(shared_bytes(ctx, make_code_kernel<false>, CODE_SMEM, configured[1]));
         const u64 pieces = n / 8, vectors = pieces < (u64(1) << 17) ? pieces : (u64(1) << 17);
         const u64 samples = vectors == pieces ? n : vectors * 8;
         const u64 blocks = div_up(vectors, HIST_BLOCK);
-        sample_symbols_kernel<<<unsigned(blocks < 1 ? 1 : (blocks > 148 ? 148 : blocks)), HIST_BLOCK, HIST_SMEM, ctx->stream>>>(T, n, vectors, t.hist);
+        CSA_CUDA(ctx, cudaMemsetAsync(t.hist, 0, 65536 * 4, ctx->stream));
+        sample_symbols_kernel<<<unsigned(blocks > 148 ? 148 : blocks), HIST_BLOCK, HIST_SMEM, ctx->stream>>>(T, n, vectors, t.hist);
         CSA_LAUNCH_CHECK(ctx);
-        code_prefix_kernel<<<1, 1024, 0, ctx->stream>>>(t.hist, u32((u64(1) << 22) / samples ? (u64(1) << 22) / samples : 1), t.prefix);
-        CSA_LAUNCH_CHECK(ctx);
-        code_assign_kernel<<<256, 256, 0, ctx->stream>>>(t.prefix, t.code);
+        make_code_kernel<false><<<65536 / CODE_BLOCK, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), t.hist, u32((u64(1) << 22) / samples), t.code, t.cnt1,
+                                                                                          reinterpret_cast<u32*>(counts));
         CSA_LAUNCH_CHECK(ctx);
     }
     const bool one_level = ps.b1 == 0;

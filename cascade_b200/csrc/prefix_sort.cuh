@@ -40,8 +40,7 @@ size_t prefix_sort_table_bytes(const Prefix_Sort& ps);
 
 struct Prefix_Tables
 {
-    u32* hist;          // 65536 symbol counts of the sample, cleared by the sort
-    u32* prefix;        // 65537 prefix sums of the symbols' weights
+    u32* hist;          // 65536 symbol counts of the sample
     u32* code;          // 65536 entries of the code
     u32* cnt1;          // [parents] records by first digit
     u32* cur1;          // [parents] running places
