@@ -44,7 +44,7 @@ Build_Layout layout_for(u64 n)
 
 // Text is compared up to this depth before ranks are: past it one more doubling costs a suffix less (an inverse rank, 64 bytes of
 // DRAM traffic) than its next symbols do.
-constexpr u64 TEXT_DEPTH = 64;
+constexpr u64 TEXT_DEPTH = 61;         // what tied suffixes share at least (1) + a wide round (refine.cu)
 constexpr u64 SMALL_BUILD = u64(1) << 22;       // up to here the output is packed before the host knows whether ties are left
 
 struct Build
@@ -267,7 +267,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             CSA_TRY(b.generation(h, idle));
             if(debug) std::fprintf(stderr, "[csa] generation %u: h=%llu active %llu -> %llu (%llu in large groups)\n", gen, h, active, b.small + b.large, b.large);
             if(h > (u64(1) << 40)) return csa_fail(ctx, CSA_E_DEVICE, "build: doubling did not terminate");
-            h *= 2;
+            h = h < depth && 2 * h > depth ? depth : 2 * h;     // the idle groups join when exactly their depth is reached
         }
     }
     st.generations = gen;

@@ -16,17 +16,6 @@ constexpr int RW_BLOCK = 256, RW_ITEMS = 8, RW_WINDOW = RW_BLOCK * RW_ITEMS;
 constexpr u32 RW_TILE = RW_WINDOW - SMALL_GROUP;        // groups that start in the tile end inside the window
 constexpr u32 NO_GROUP = 0xFFFFu;
 
-__device__ __forceinline__ u32 warp_max(u32 v)
-{
-    #pragma unroll
-    for(int o = 1; o < 32; o <<= 1)
-    {
-        const u32 t = __shfl_up_sync(0xFFFFFFFFu, v, o);
-        if(int(lane_id()) >= o) v = max(v, t);
-    }
-    return v;
-}
-
 __device__ __forceinline__ u32 warp_sum(u32 v)
 {
     #pragma unroll
@@ -38,10 +27,141 @@ __device__ __forceinline__ u32 warp_sum(u32 v)
     return v;
 }
 
-// A block's window of a list: slot j holds entry first + j. gs[j]: the slot where j's group starts, NO_GROUP where that is not
-// inside the block's tile (the group belongs to another block) or past the list's end; ge[gs[j]]: where the group ends.
+// Groups of a block's window of a list (slot j = entry first + j), found by bit operations: bit j of `starts` says that a group (or
+// what lies past the list's end) begins at slot j.
+struct Group_Starts
+{
+    u32 starts[RW_WINDOW / 32];
+};
+
+// A thread's records are the slots tid + i * RW_BLOCK: e[i] gets the entries (~0 past the list's end: no group starts at slot
+// 2^32 - 1). Ends with a barrier.
+__device__ __forceinline__ void load_entries(Group_Starts& g, const u64* __restrict__ list, const u64 count, const u64 first, u64 (&e)[RW_ITEMS])
+{
+    const u32 tid = threadIdx.x, lane = lane_id();
+    u32 before[RW_ITEMS];       // of lane 0: the head before its slot
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u64 k = first + tid + i * RW_BLOCK;
+        e[i] = k < count ? list[k] : ~0ull;
+        before[i] = 0xFFFFFFFEu;        // another number than any head
+        if(lane == 0 && k > 0) before[i] = k - 1 < count ? u32(list[k - 1] >> 32) : 0xFFFFFFFFu;
+    }
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 h = u32(e[i] >> 32), up = __shfl_up_sync(0xFFFFFFFFu, h, 1);
+        const u32 m = __ballot_sync(0xFFFFFFFFu, h != (lane ? up : before[i]));
+        if(lane == 0) g.starts[i * (RW_BLOCK / 32) + (tid >> 5)] = m;
+    }
+    __syncthreads();
+}
+
+// First and end slot of the group of slot tid + i * RW_BLOCK; first = NO_GROUP where the group does not start inside the block's
+// tile (it belongs to another block) or the slot lies past the list's end. Every lane of a warp calls it.
+__device__ __forceinline__ void find_group(const Group_Starts& g, const u64 entry, const int i, u32& s, u32& e)
+{
+    const u32 lane = lane_id();
+    const int word = i * (RW_BLOCK / 32) + int(threadIdx.x >> 5);
+    s = NO_GROUP; e = 0;
+    if(__all_sync(0xFFFFFFFFu, entry == ~0ull)) return;
+    const u32 m = g.starts[word];
+    u32 last = NO_GROUP, next = RW_WINDOW;      // of the words before and behind: the same for all lanes
+    constexpr int REACH = SMALL_GROUP / 32 + 1;
+    if((m & 1u) == 0)
+        for(int k = word - 1; k >= 0 && k >= word - REACH; --k)
+            if(const u32 v = g.starts[k]) { last = k * 32 + 31 - __clz(v); break; }
+    for(int k = word + 1; k < RW_WINDOW / 32 && k <= word + REACH; ++k)
+        if(const u32 v = g.starts[k]) { next = k * 32 + __ffs(v) - 1; break; }
+    const u32 upto = m & (0xFFFFFFFFu >> (31 - lane)), behind = m & ~(0xFFFFFFFFu >> (31 - lane));
+    s = upto ? word * 32 + 31 - __clz(upto) : last;
+    e = behind ? word * 32 + __ffs(behind) - 1 : next;
+    if(s >= RW_TILE || entry == ~0ull) s = NO_GROUP;
+}
+
+// Where the members of a window's groups go, found without comparing all with all: most members of a group equal its first member
+// (in near-duplicate documents two copies differ in one symbol of a thousand), and only the others, the odd ones, are counted
+// against one another.
+struct Odd_Members
+{
+    u32 odd[RW_WINDOW / 32 + 1];            // a bit per slot: another key than the group's first member
+    u32 less[RW_WINDOW / 32 + 1];           // of those, the smaller ones
+    u32 before[RW_WINDOW / 32 + 1];         // per word: odd members before it | smaller ones before it << 16
+};
+
+// The bits of slot tid + i * RW_BLOCK; every lane calls it.
+__device__ __forceinline__ void mark_odd(Odd_Members& m, const int i, const bool odd, const bool less)
+{
+    const u32 o = __ballot_sync(0xFFFFFFFFu, odd), l = __ballot_sync(0xFFFFFFFFu, less);
+    if(lane_id() == 0) { m.odd[i * (RW_BLOCK / 32) + (threadIdx.x >> 5)] = o; m.less[i * (RW_BLOCK / 32) + (threadIdx.x >> 5)] = l; }
+}
+
+// Between barriers: the sums over the words.
+__device__ __forceinline__ void sum_odd(Odd_Members& m)
+{
+    static_assert(RW_WINDOW / 32 == 64, "two words a lane");
+    if(threadIdx.x < 32)
+    {
+        const u32 k = 2 * threadIdx.x;
+        const u32 a = __popc(m.odd[k]) | __popc(m.less[k]) << 16, b = __popc(m.odd[k + 1]) | __popc(m.less[k + 1]) << 16;
+        const u32 inc = warp_sum(a + b);
+        m.before[k] = inc - a - b;
+        m.before[k + 1] = inc - b;
+        if(threadIdx.x == 31) { m.before[64] = inc; m.odd[64] = 0; m.less[64] = 0; }
+    }
+}
+
+// Odd members before slot j | smaller ones << 16 (j up to RW_WINDOW).
+__device__ __forceinline__ u32 odd_before(const Odd_Members& m, const u32 j)
+{
+    const u32 below = (1u << (j & 31)) - 1;
+    return m.before[j >> 5] + (__popc(m.odd[j >> 5] & below) | __popc(m.less[j >> 5] & below) << 16);
+}
+
+// How many of the odd keys [a, b) are smaller than `mine`, how many equal it, and how many of those come before entry `me`: in bits
+// 0, 16 and 32 on. A call, so that the eight places that need it do not each carry the loop (instruction fetch bounds the callers).
+template <typename K>
+__device__ __noinline__ u64 count_odd(const K* keys, const u32 a, const u32 b, const u32 me, const K mine)
+{
+    u32 less = 0, eq_before = 0, eq = 0;
+    for(u32 k = a; k < b; ++k)
+    {
+        const K o = keys[k];
+        less += o < mine;
+        const u32 same = o == mine;
+        eq += same;
+        eq_before += same && k < me;
+    }
+    return u64(less | eq << 16) | u64(eq_before) << 32;
+}
+
+// The place of member j of the group [s, e), and the new group that it lands in. keys: the odd members' keys, side by side in slot order.
+template <typename K>
+__device__ __forceinline__ void member_place(const Odd_Members& m, const K* keys, const u32 j, const u32 s, const u32 e, const bool odd, const bool smaller, const K mine,
+                                             u32& at, u32& to_s, u32& to_e)
+{
+    const u32 bs = odd_before(m, s), be = odd_before(m, e), bj = odd_before(m, j);
+    const u32 equals = (e - s) - ((be - bs) & 0xFFFFu);
+    if(!odd)
+    {
+        to_s = s + ((be >> 16) - (bs >> 16));
+        to_e = to_s + equals;
+        at = to_s + (j - s) - ((bj - bs) & 0xFFFFu);
+        return;
+    }
+    const u64 c = count_odd(keys, bs & 0xFFFFu, be & 0xFFFFu, bj & 0xFFFFu, mine);
+    const u32 less = u32(c) & 0xFFFFu, eq = u32(c) >> 16, eq_before = u32(c >> 32);
+    to_s = s + less + (smaller ? 0 : equals);
+    at = to_s + eq_before;
+    to_e = to_s + eq;
+}
+
+// The window of a list with its groups in shared memory, where a kernel changes them: gs[j]: first slot of j's group or NO_GROUP;
+// ge[gs[j]]: where the group ends; head[j]: j's place in the suffix array.
 struct Window
 {
+    Group_Starts groups;
     u32 head[RW_WINDOW];
     u32 pos[RW_WINDOW];
     u16 gs[RW_WINDOW];
@@ -52,57 +172,30 @@ struct Window
     u32 slot;
 };
 
-// Loads the window and finds the groups. A thread's records are the slots tid + i * RW_BLOCK. Ends with a barrier.
+// Ends with a barrier.
 __device__ __forceinline__ void load_window(Window& w, const u64* __restrict__ list, const u64 count, const u64 first)
 {
-    const u32 tid = threadIdx.x;
+    u64 entry[RW_ITEMS];
+    load_entries(w.groups, list, count, first, entry);
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
-        const u32 j = tid + i * RW_BLOCK;
-        const u64 e = first + j < count ? list[first + j] : ~0ull;      // no group starts at slot 2^32 - 1
-        w.head[j] = u32(e >> 32);
-        w.pos[j] = u32(e);
-    }
-    const u32 before = first > 0 ? u32(list[first - 1] >> 32) : 0xFFFFFFFEu;    // another number than any head
-    __syncthreads();
-    // running last start (as slot + 1, 0 = none) over consecutive slots
-    const u32 j0 = tid * RW_ITEMS;
-    u32 last = 0, mine[RW_ITEMS];
-    u32 prev = j0 > 0 ? w.head[j0 - 1] : before;
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        const u32 h = w.head[j0 + i];
-        if(h != prev) last = j0 + i + 1;
-        mine[i] = last;
-        prev = h;
-    }
-    const u32 inc = warp_max(last);
-    if(lane_id() == 31) w.warp_tot[tid >> 5] = inc;
-    __syncthreads();
-    u32 carry = __shfl_up_sync(0xFFFFFFFFu, inc, 1);
-    if(lane_id() == 0) carry = 0;
-    for(u32 k = 0; k < (tid >> 5); ++k) carry = max(carry, w.warp_tot[k]);
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        const u32 s = max(mine[i], carry);
-        w.gs[j0 + i] = (s == 0 || s > RW_TILE || w.head[j0 + i] == 0xFFFFFFFFu) ? u16(NO_GROUP) : u16(s - 1);
-    }
-    __syncthreads();
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-        if(s != NO_GROUP && (j + 1 == RW_WINDOW || w.gs[j + 1] != s)) w.ge[s] = u16(j + 1);
+        const u32 j = threadIdx.x + i * RW_BLOCK;
+        u32 s, e;
+        find_group(w.groups, entry[i], i, s, e);
+        w.head[j] = u32(entry[i] >> 32) + (s == NO_GROUP ? 0 : j - s);
+        w.pos[j] = u32(entry[i]);
+        w.gs[j] = u16(s);
+        if(s == j) w.ge[j] = u16(e);
     }
     __syncthreads();
 }
 
 // Appends the slots flagged in w.mask (cleared before, set by atomics, no barrier needed in between) to a list whose length
-// *count is advanced; returns the list position of the first. Every thread calls it; the result holds after the call.
-__device__ __forceinline__ u32 window_places(Window& w, u32* count)
+// *count is advanced; returns the list position of the first. Every thread calls it; the result holds after the call. W: a struct
+// with mask, pre, warp_tot and slot as in Window.
+template <typename W>
+__device__ __forceinline__ u32 window_places(W& w, u32* count)
 {
     __syncthreads();
     constexpr int WORDS = RW_WINDOW / 32;       // 64
@@ -136,101 +229,232 @@ __device__ __forceinline__ ulonglong2 eight_symbols(const u16* __restrict__ T, c
     return make_ulonglong2((u64(r[0]) << 32) | r[1], (u64(r[2]) << 32) | r[3]);
 }
 
-// Orders groups by the symbols [from, to) of their suffixes, eight at a time; the window stays in shared memory over all steps.
-// What bounds it is the read of the text: a suffix's symbols are one to five 32-byte sectors in a row.
-__global__ void __launch_bounds__(RW_BLOCK) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
-                                                                 u64* __restrict__ next, u32* __restrict__ sa, Build_Counts* __restrict__ counts)
+// How a member of a group compares with the group's first member from the group's depth on, as one number that orders the members:
+// class (0 less, 1 equal as far as compared, 2 greater) at bit 40, then the pair of symbols in which the two differ first (more
+// equal pairs: nearer to the first member), then that pair and how many symbols of it the suffix has.
+constexpr u64 KEY_EQUAL = 1ull << 40;
+
+__device__ __forceinline__ u64 pair_key(const u32 pair, const u32 mine, const u32 have, const u32 lead, const u32 lead_have)
+{
+    const bool less = mine < lead || (mine == lead && have < lead_have);
+    return (less ? 0ull : 2ull << 40) | (u64(less ? pair : 31 - pair) << 34) | (u64(mine) << 2) | have;
+}
+// Symbols that members with this key share beyond the group's depth (`reach`: as far as was compared).
+__device__ __forceinline__ u32 shared_by_key(const u64 key, const u32 reach)
+{
+    if(key == KEY_EQUAL) return reach;
+    const u32 p = u32(key >> 34) & 31u;
+    return 2 * ((key >> 40) ? 31 - p : p) + 2;
+}
+
+constexpr u32 WIDE_REACH = 60;      // symbols that half a warp compares at once: four per lane; the last lane only completes the four before it
+constexpr u32 QUICK_REACH = 8;
+
+// Orders groups by the symbols [from, to) of their suffixes. In a round every member of a group is compared with the group's first
+// member, and the members are put in order by their first difference from it; a group that falls apart goes on as several, each
+// with its own depth. The window stays in shared memory over all rounds.
+//
+// A WIDE round has half a warp read 60 symbols of one suffix with one load (a thread that reads 8 symbols of a suffix of its own at a time
+// costs an L1 look-up per lane and 8-byte piece). Where few suffixes are tied, nearly all of them differ within a few symbols and
+// the chain of loads counts: the first round is then QUICK, 8 symbols by one thread, all of a thread's suffixes in flight together.
+// Where nearly all of 4e8 suffixes are tied, 8 symbols a round and all members against all took 136 ms, this way XX_MS.
+__global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
+                                                                    u64* __restrict__ next, u32* __restrict__ sa, Build_Counts* __restrict__ counts)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Window& w = *reinterpret_cast<Window*>(smem_raw);
-    ulonglong2* const word = reinterpret_cast<ulonglong2*>(smem_raw + (sizeof(Window) + 15) / 16 * 16);     // [RW_WINDOW] the symbols compared in this step
-    u8* const split = reinterpret_cast<u8*>(word + RW_WINDOW);      // [RW_WINDOW] by first slot: the group's members differ
-    u8* const rest = split + RW_WINDOW;                             // [RW_WINDOW] symbols of the step that the suffix still has, 8 = all
-    const u32 tid = threadIdx.x;
+    u64* const key = reinterpret_cast<u64*>(smem_raw + (sizeof(Window) + 15) / 16 * 16);     // [RW_WINDOW]
+    u32* const depth = reinterpret_cast<u32*>(key + RW_WINDOW);     // [RW_WINDOW] by first slot: symbols that the group's members share (below 2^32: no more than n)
+    Odd_Members& odds = *reinterpret_cast<Odd_Members*>(depth + RW_WINDOW);
+    const u32 tid = threadIdx.x, lane = lane_id();
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
     for(u64 first = u64(blockIdx.x) * RW_TILE; first < count; first += u64(gridDim.x) * RW_TILE)
     {
         load_window(w, list, count, first);
-        // from here on head[j] is the suffix-array slot of window slot j, for slots of the block's own groups
         #pragma unroll
-        for(int i = 0; i < RW_ITEMS; ++i)
+        for(int i = 0; i < RW_ITEMS; ++i) depth[tid + i * RW_BLOCK] = u32(from);
+        __syncthreads();
+        bool quick = from < QUICK_REACH && to - from >= QUICK_REACH && count * 4 < n;
+        while(true)
         {
-            const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-            if(s != NO_GROUP) w.head[j] += j - s;
-        }
-        for(u64 d = from; d < to; d += 8)
-        {
+            const u32 reach = quick ? QUICK_REACH : WIDE_REACH;
             bool open = false;
-            #pragma unroll
-            for(int i = 0; i < RW_ITEMS; ++i)
+            if(quick)
             {
-                const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-                if(s == NO_GROUP || u32(w.ge[s]) - s < 2) continue;
-                open = true;
-                const u64 x = u64(w.pos[j]) + d;
-                ulonglong2 v = make_ulonglong2(0, 0);
-                if(x < n) v = eight_symbols(T, x);
-                u64 have = x < n ? n - x : 0;
-                u64 want = to - d < 8 ? to - d : 8;
-                if(want < 8)        // only the symbols before `to` count
+                #pragma unroll 4
+                for(int i = 0; i < RW_ITEMS; ++i)
                 {
-                    if(want <= 4) { v.y = 0; v.x = want == 4 ? v.x : v.x & ~(~0ull >> (16 * want)); }
-                    else v.y &= ~(~0ull >> (16 * (want - 4)));
+                    const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
+                    if(s == j) key[j] = KEY_EQUAL;
+                    if(s == NO_GROUP || j == s) continue;
+                    open = true;
+                    const u64 x = u64(w.pos[j]) + from, y = u64(w.pos[s]) + from;
+                    const ulonglong2 none = make_ulonglong2(0, 0);
+                    const ulonglong2 a = x < n ? eight_symbols(T, x) : none, b = y < n ? eight_symbols(T, y) : none;
+                    const u64 has_a = x < n ? n - x : 0, has_b = y < n ? n - y : 0;
+                    const u32 pa[4] = {u32(a.x >> 32), u32(a.x), u32(a.y >> 32), u32(a.y)}, pb[4] = {u32(b.x >> 32), u32(b.x), u32(b.y >> 32), u32(b.y)};
+                    u64 k = KEY_EQUAL;
+                    #pragma unroll
+                    for(int q = 3; q >= 0; --q)
+                    {
+                        const u32 ha = has_a > 2 * q + 1 ? 2 : (has_a > 2 * q ? 1 : 0), hb = has_b > 2 * q + 1 ? 2 : (has_b > 2 * q ? 1 : 0);
+                        if(pa[q] != pb[q] || ha != hb) k = pair_key(q, pa[q], ha, pb[q], hb);
+                    }
+                    key[j] = k;
                 }
-                word[j] = v;
-                rest[j] = u8(have < want ? have : want);
-                split[j] = 0;
+            }
+            else
+            {
+                // The slots of half a warp, 16 at a time, whose places and depths the lanes look up together.
+                constexpr u32 PER_HALF = RW_WINDOW / (RW_BLOCK / 16);
+                const u32 hl = lane & 15, half = lane & 16;
+                u32 lead_x = 0, lead_y = 0, lead_have = 0, lead_slot = NO_GROUP;
+                const u32 base = (tid >> 4) * PER_HALF;
+                for(u32 j0 = base; j0 < base + PER_HALF; j0 += 16)
+                {
+                    const u32 s = w.gs[j0 + hl];
+                    u32 at = 0, cnt = 0;
+                    bool mine = false;
+                    auto place = [&](const u32 slot, const u32 d, u32& x0, u32& c0)     // where a suffix is read from, and how many symbols count
+                    {
+                        const u64 x = u64(w.pos[slot]) + d;
+                        x0 = x < n ? u32(x) : u32(n);
+                        const u64 c = min(n - x0, to - d);
+                        c0 = c < WIDE_REACH ? u32(c) : WIDE_REACH;
+                    };
+                    if(s != NO_GROUP && u32(w.ge[s]) - s >= 2 && u64(depth[s]) < to) { mine = true; place(j0 + hl, depth[s], at, cnt); }
+                    const u32 both = __ballot_sync(0xFFFFFFFFu, mine);
+                    if(both == 0) continue;
+                    open = true;
+                    if(mine) key[j0 + hl] = KEY_EQUAL;
+                    const u32 todo = (both >> half) & 0xFFFFu;
+                    const u32 leads = (__ballot_sync(0xFFFFFFFFu, mine && s == j0 + hl) >> half) & 0xFFFFu;
+                    // a group that began in another half's slots: its first member is read here too
+                    const u32 s0 = __shfl_sync(0xFFFFFFFFu, s, half + (todo ? __ffs(todo) - 1 : 0));
+                    const u32 s_last = __shfl_sync(0xFFFFFFFFu, s, half + (todo ? 31 - __clz(todo) : 0));
+                    const bool fetch = todo != 0 && s0 != lead_slot && s0 < j0;
+                    auto read = [&](const u32 a, const u32 c) -> uint2
+                    {
+                        uint2 v = make_uint2(0, 0);
+                        if(4 * hl < c + 4) v = __ldg(reinterpret_cast<const uint2*>(T) + ((a >> 2) + hl));      // T is 16-byte aligned
+                        return v;
+                    };
+                    auto settle = [&](uint2& v, const u32 a)      // four symbols from the suffix's first, most significant first
+                    {
+                        u32 nx = __shfl_down_sync(0xFFFFFFFFu, v.x, 1, 16);
+                        const u32 ny = __shfl_down_sync(0xFFFFFFFFu, v.y, 1, 16);
+                        if(a & 2) { v.x = v.y; v.y = nx; nx = ny; }
+                        const u32 pick = (a & 1) ? 0x3254 : 0x1032;
+                        v.x = __byte_perm(v.x, v.y, pick);
+                        v.y = __byte_perm(v.y, nx, pick);
+                    };
+                    auto cut = [&](uint2& v, const u32 c) -> u32      // how many of the four count
+                    {
+                        const int h = min(4, int(c) - int(4 * hl));
+                        if(h < 4)
+                        {
+                            const u64 keep = h > 0 ? ~0ull << (64 - 16 * h) : 0ull;
+                            v.x &= u32(keep >> 32); v.y &= u32(keep);
+                        }
+                        return h > 0 ? u32(h) : 0u;
+                    };
+                    if(__any_sync(0xFFFFFFFFu, fetch))
+                    {
+                        uint2 v = make_uint2(0, 0);
+                        u32 a = 0, c = 0;
+                        if(fetch) { place(s0, depth[s0], a, c); v = read(a, c); }
+                        settle(v, a);
+                        const u32 h = cut(v, c);
+                        if(fetch) { lead_x = v.x; lead_y = v.y; lead_have = h; }
+                    }
+                    if(todo) lead_slot = s_last;
+                    const bool whole = __all_sync(0xFFFFFFFFu, !mine || cnt == WIDE_REACH);     // no suffix ends inside, `to` is not reached
+                    constexpr int BATCH = 4;
+                    #pragma unroll 1
+                    for(int q = 0; q < 16; q += BATCH)
+                    {
+                        if((both & (0xF000Fu << q)) == 0) continue;
+                        uint2 word[BATCH];
+                        u32 from_at[BATCH];
+                        #pragma unroll
+                        for(int b = 0; b < BATCH; ++b)
+                        {
+                            from_at[b] = __shfl_sync(0xFFFFFFFFu, at, q + b, 16);
+                            const u32 c = whole ? WIDE_REACH : __shfl_sync(0xFFFFFFFFu, cnt, q + b, 16);
+                            word[b] = make_uint2(0, 0);
+                            if(todo >> (q + b) & 1u) word[b] = read(from_at[b], c);
+                        }
+                        #pragma unroll
+                        for(int b = 0; b < BATCH; ++b)
+                        {
+                            settle(word[b], from_at[b]);
+                            u32 have = hl < 15 ? 4 : 0;
+                            if(!whole) have = cut(word[b], __shfl_sync(0xFFFFFFFFu, cnt, q + b, 16));
+                            else if(hl == 15) word[b] = make_uint2(0, 0);
+                            const u32 x = word[b].x, y = word[b].y;
+                            if(leads >> (q + b) & 1u) { lead_x = x; lead_y = y; lead_have = have; }
+                            const bool differs = (todo >> (q + b) & 1u) && (x != lead_x || y != lead_y || have != lead_have);
+                            const u32 all = __ballot_sync(0xFFFFFFFFu, differs);
+                            if(all == 0) continue;
+                            const u32 differ = (all >> half) & 0xFFFFu;
+                            if(differ && hl == __ffs(differ) - 1)
+                            {
+                                const u32 hx = min(have, 2u), lx = min(lead_have, 2u);
+                                key[j0 + q + b] = x != lead_x || hx != lx ? pair_key(2 * hl, x, hx, lead_x, lx) : pair_key(2 * hl + 1, y, have - hx, lead_y, lead_have - lx);
+                            }
+                        }
+                    }
+                }
             }
             if(!__syncthreads_or(open)) break;
-            bool differs = false;
+            // the members take their new places
+            u64 mine[RW_ITEMS];
             #pragma unroll
             for(int i = 0; i < RW_ITEMS; ++i)
             {
                 const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-                if(s == NO_GROUP || u32(w.ge[s]) - s < 2) continue;
-                const ulonglong2 a = word[j], b = word[s];
-                if(a.x != b.x || a.y != b.y || rest[j] != rest[s]) { split[s] = 1; differs = true; }
+                mine[i] = KEY_EQUAL;
+                if(s != NO_GROUP && u32(w.ge[s]) - s >= 2 && u64(depth[s]) < to) mine[i] = key[j];
+                mark_odd(odds, i, mine[i] != KEY_EQUAL, mine[i] < KEY_EQUAL);
             }
-            if(!__syncthreads_or(differs)) continue;
-            // the members of a group that differs count those before them; then they change places
-            u32 p[RW_ITEMS], at[RW_ITEMS], to_s[RW_ITEMS], to_e[RW_ITEMS];
+            __syncthreads();
+            sum_odd(odds);
+            __syncthreads();
+            #pragma unroll
+            for(int i = 0; i < RW_ITEMS; ++i)
+                if(mine[i] != KEY_EQUAL) key[odd_before(odds, tid + i * RW_BLOCK) & 0xFFFFu] = mine[i];
+            __syncthreads();
+            u32 p[RW_ITEMS], deeper[RW_ITEMS];          // position, depth of the member's new group
+            u32 go[RW_ITEMS], to_e[RW_ITEMS];           // new slot | first slot of the new group << 16, its end
             #pragma unroll
             for(int i = 0; i < RW_ITEMS; ++i)
             {
                 const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-                at[i] = NO_GROUP;
+                go[i] = NO_GROUP;
                 if(s == NO_GROUP) continue;
                 const u32 e = w.ge[s];
-                if(e - s < 2 || !split[s]) continue;
-                const ulonglong2 a = word[j];
-                const u32 ra = rest[j];
-                u32 less = 0, eq_before = 0, eq = 0;
-                for(u32 k = s; k < e; ++k)
-                {
-                    const ulonglong2 b = word[k];
-                    const u32 rb = rest[k];
-                    const bool same_words = b.x == a.x && b.y == a.y;
-                    less += (b.x < a.x) || (b.x == a.x && b.y < a.y) || (same_words && rb < ra);
-                    const u32 same = same_words && rb == ra;
-                    eq += same;
-                    eq_before += same && k < j;
-                }
+                const u32 d = depth[s];
+                if(e - s < 2 || d >= to) continue;
                 p[i] = w.pos[j];
-                to_s[i] = s + less;
-                at[i] = s + less + eq_before;
-                to_e[i] = s + less + eq;
+                u32 at, to_s;
+                member_place(odds, key, j, s, e, mine[i] != KEY_EQUAL, mine[i] < KEY_EQUAL, mine[i], at, to_s, to_e[i]);
+                go[i] = at | to_s << 16;
+                const u32 more = shared_by_key(mine[i], reach);
+                deeper[i] = to - d < more ? u32(to) : d + more;
             }
             __syncthreads();
             #pragma unroll
             for(int i = 0; i < RW_ITEMS; ++i)
-                if(at[i] != NO_GROUP)
+                if(go[i] != NO_GROUP)
                 {
-                    w.pos[at[i]] = p[i];
-                    w.gs[at[i]] = u16(to_s[i]);
-                    if(at[i] == to_s[i]) w.ge[at[i]] = u16(to_e[i]);
+                    const u32 at = go[i] & 0xFFFFu, s = go[i] >> 16;
+                    w.pos[at] = p[i];
+                    w.gs[at] = u16(s);
+                    if(at == s) { w.ge[at] = u16(to_e[i]); depth[at] = deeper[i]; }
                 }
             __syncthreads();
+            quick = false;
         }
         __syncthreads();
         if(tid < RW_WINDOW / 32) w.mask[tid] = 0;
@@ -259,7 +483,7 @@ __global__ void __launch_bounds__(RW_BLOCK) refine_by_text_kernel(const u16* __r
     }
 }
 
-constexpr size_t TEXT_SMEM = (sizeof(Window) + 15) / 16 * 16 + size_t(RW_WINDOW) * 16 + 2 * RW_WINDOW;
+constexpr size_t TEXT_SMEM = (sizeof(Window) + 15) / 16 * 16 + size_t(RW_WINDOW) * (8 + 4) + sizeof(Odd_Members);
 
 constexpr int GATHER_UNROLL = 8;
 __global__ void __launch_bounds__(256) gather_ranks_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ isa, const u64 n, const u64 h,
@@ -283,57 +507,68 @@ __global__ void __launch_bounds__(256) gather_ranks_kernel(const u64* __restrict
     }
 }
 
-__global__ void __launch_bounds__(RW_BLOCK) refine_by_ranks_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ isa,
-                                                                  u32* __restrict__ sa, u64* __restrict__ next, Build_Counts* __restrict__ counts)
+struct Rank_Window
 {
-    __shared__ Window w;
-    __shared__ u32 sec[RW_WINDOW];
-    __shared__ u8 split[RW_WINDOW];
+    Group_Starts groups;
+    u32 mask[RW_WINDOW / 32];
+    u32 pre[RW_WINDOW / 32];
+    u32 warp_tot[RW_BLOCK / 32];
+    u32 slot;
+    u32 sec[RW_WINDOW];
+    Odd_Members odds;
+};
+
+__global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ isa,
+                                                                     u32* __restrict__ sa, u64* __restrict__ next, Build_Counts* __restrict__ counts)
+{
+    __shared__ Rank_Window w;
     const u32 tid = threadIdx.x;
     const u64 first = u64(blockIdx.x) * RW_TILE;
+    u32 sec[RW_ITEMS];
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
         const u32 j = tid + i * RW_BLOCK;
-        sec[j] = first + j < count ? secs[first + j] : 0;
-        split[j] = 0;
+        sec[i] = first + j < count ? __ldcs(secs + first + j) : 0;
+        w.sec[j] = sec[i];
     }
     if(tid < RW_WINDOW / 32) w.mask[tid] = 0;
-    load_window(w, list, count, first);
+    u64 entry[RW_ITEMS];
+    load_entries(w.groups, list, count, first, entry);
+    u32 group[RW_ITEMS];        // first slot | end << 16
+    u32 odd = 0, smaller = 0;   // a bit per record
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
-        const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-        if(s != NO_GROUP && sec[j] != sec[s]) split[s] = 1;
+        u32 s, e;
+        find_group(w.groups, entry[i], i, s, e);
+        group[i] = s | e << 16;
+        const u32 lead = s != NO_GROUP ? w.sec[s] : sec[i];
+        odd |= u32(sec[i] != lead) << i;
+        smaller |= u32(sec[i] < lead) << i;
+        mark_odd(w.odds, i, sec[i] != lead, sec[i] < lead);
     }
+    __syncthreads();
+    sum_odd(w.odds);
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+        if(odd >> i & 1u) w.sec[odd_before(w.odds, tid + i * RW_BLOCK) & 0xFFFFu] = sec[i];
     __syncthreads();
     u32 place[RW_ITEMS], new_head[RW_ITEMS];        // place: NO_GROUP = not this block's, or alone now
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
-        const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
+        const u32 j = tid + i * RW_BLOCK, s = group[i] & 0xFFFFu;
         place[i] = NO_GROUP;
         if(s == NO_GROUP) continue;
-        const u32 head = w.head[j];
-        if(!split[s]) { place[i] = j; new_head[i] = head; }
-        else
-        {
-            const u32 e = w.ge[s], mine = sec[j];
-            u32 less = 0, eq_before = 0, eq = 0;
-            for(u32 k = s; k < e; ++k)
-            {
-                const u32 o = sec[k];
-                less += o < mine;
-                const u32 same = o == mine;
-                eq += same;
-                eq_before += same && k < j;
-            }
-            const u32 nh = head + less, x = w.pos[j];
-            if(less) isa[x] = nh;
-            if(eq == 1) sa[nh] = x;
-            else { place[i] = s + less + eq_before; new_head[i] = nh; }
-        }
-        if(place[i] != NO_GROUP) atomicOr(&w.mask[place[i] >> 5], 1u << (place[i] & 31));
+        u32 at, to_s, to_e;
+        member_place(w.odds, w.sec, j, s, group[i] >> 16, (odd >> i & 1u) != 0, (smaller >> i & 1u) != 0, sec[i], at, to_s, to_e);
+        const u32 x = u32(entry[i]);
+        new_head[i] = u32(entry[i] >> 32) + (to_s - s);
+        if(to_s != s) isa[x] = new_head[i];
+        if(to_e - to_s == 1) sa[new_head[i]] = x;
+        else { place[i] = at; atomicOr(&w.mask[at >> 5], 1u << (at & 31)); }
     }
     const u32 base = window_places(w, &counts->next_small);
     #pragma unroll
@@ -341,7 +576,7 @@ __global__ void __launch_bounds__(RW_BLOCK) refine_by_ranks_kernel(const u64* __
         if(place[i] != NO_GROUP)
         {
             const u32 q = place[i];
-            next[base + w.pre[q >> 5] + __popc(w.mask[q >> 5] & ((1u << (q & 31)) - 1))] = (u64(new_head[i]) << 32) | w.pos[tid + i * RW_BLOCK];
+            next[base + w.pre[q >> 5] + __popc(w.mask[q >> 5] & ((1u << (q & 31)) - 1))] = (u64(new_head[i]) << 32) | u32(entry[i]);
         }
 }
 
@@ -545,9 +780,10 @@ int ranks_from(csa_ctx* ctx, const u32* sa, const u64* list, u64 count, u64 n, u
 
 int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, Build_Counts* counts, u64 expected)
 {
+    to = to < n ? to : n;           // no two suffixes share as much
     CSA_CUDA(ctx, cudaFuncSetAttribute(refine_by_text_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TEXT_SMEM)));
     const u64 tiles = div_up(expected ? expected : 1, RW_TILE);
-    refine_by_text_kernel<<<unsigned(tiles < 148 * 3 ? tiles : 148 * 3), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, counts);
+    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -40,7 +40,7 @@ def test_sizes_at_the_edges(ctx, oracle, n):
 
 
 @pytest.mark.parametrize("n", [257, 1793, 2049, 8193, 70_001, 2_200_000])
-@pytest.mark.parametrize("kind", ["one", "two", "period", "phrase", "stretch", "zeros_at_the_end", "wide"])
+@pytest.mark.parametrize("kind", ["one", "two", "period", "phrase", "stretch", "zeros_at_the_end", "copies", "wide"])
 def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
     rng = np.random.default_rng(n)
     if kind == "one":                   # one group of everything, halved by every generation
@@ -61,6 +61,10 @@ def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
     elif kind == "zeros_at_the_end":    # suffixes that differ from others by their end alone
         T = rng.integers(0, 3, n)
         T[-min(n, 300):] = 0
+    elif kind == "copies":              # near-duplicate documents of an odd length: nearly all suffixes tied, in groups that mostly agree
+        base = rng.integers(0, 200, (5, 331))
+        T = base[rng.integers(0, 5, n // 331 + 1)].ravel()[:n].copy()
+        T[rng.random(n) < 0.004] = 60000
     else:
         T = rng.integers(0, 65536, n)
     st = _check(ctx, oracle, T)
