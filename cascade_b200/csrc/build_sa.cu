@@ -42,9 +42,6 @@ Build_Layout layout_for(u64 n)
     return L;
 }
 
-// Text is compared up to this depth before ranks are: past it one more doubling costs a suffix less (an inverse rank, 64 bytes of
-// DRAM traffic) than its next symbols do.
-constexpr u64 TEXT_DEPTH = 61;         // what tied suffixes share at least (1) + a wide round (refine.cu)
 constexpr u64 SMALL_BUILD = u64(1) << 22;       // up to here the output is packed before the host knows whether ties are left
 
 struct Build
@@ -68,16 +65,7 @@ struct Build
 
     u64* large_list(u64* buf) const { return buf + (n - large); }
 
-    int read_counts(Build_Counts& c)
-    {
-        CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + CSA_COUNTS_WORD, ctx->d_scalars + CSA_COUNTS_WORD, (CSA_STATUS_WORD + 1 - CSA_COUNTS_WORD) * 8, cudaMemcpyDeviceToHost,
-                                      ctx->stream));
-        CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        if(ctx->h_scalars[CSA_STATUS_WORD] != 0) { u64 b = 0; return csa_sync(ctx, reinterpret_cast<uint64_t*>(&b)); }
-        c = *reinterpret_cast<const Build_Counts*>(ctx->h_scalars + CSA_COUNTS_WORD);
-        if(c.small > n || u64(c.next_small) + c.large > n) return csa_fail(ctx, CSA_E_DEVICE, "build: the lists of tied suffixes do not add up");
-        return CSA_OK;
-    }
+    int read_counts(Build_Counts& c) { return read_build_counts(ctx, n, c); }
 
     int set_count(u32 Build_Counts::*field, u32 value)
     {

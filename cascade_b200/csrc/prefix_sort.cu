@@ -346,10 +346,12 @@ static_assert(SCATTER_TEXT_SMEM<512> >= STREAM_WORDS<512> * 4 && SCATTER_TEXT_SM
 
 // Scatter by the top `bits` bits: the places inside a bucket come from shared-memory atomics and, for the tile's run of a bucket,
 // from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs.
-// keep_top: the record keeps the top bits (there is no second split), else its key starts behind them.
-template <int BLOCK>
+// keep_top: the record keeps the top bits (there is no second split), else its key starts behind them. PART: only the suffixes of the
+// buckets [first_bin, first_bin + part_bins) are taken, and the cursors are theirs.
+template <int BLOCK, bool PART>
 __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits,
-                                                                          const int keep_top, u32* __restrict__ cursor, u64* __restrict__ out)
+                                                                          const int keep_top, const u32 first_bin, const u32 part_bins, u32* __restrict__ cursor,
+                                                                          u64* __restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u32* const stream = reinterpret_cast<u32*>(smem_raw);
@@ -358,7 +360,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     __shared__ u32 cnt[1 << MAX_B1];            // counts, then the bins' starts inside the tile
     __shared__ u32 base[1 << MAX_B1];           // where the tile's run of a bin goes, minus the run's start
     __shared__ u32 warp_tot[BLOCK / 32];
-    const u32 bins = 1u << bits;
+    const u32 bins = PART ? part_bins : 1u << bits;
     for(u32 i = threadIdx.x; i < bins; i += BLOCK) cnt[i] = 0;
     const u64 first = u64(blockIdx.x) * TILE_POSITIONS<BLOCK>;
     u32 ent[TEXT_ITEMS];
@@ -367,16 +369,17 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     const u64 room = n - first;
     const u32 valid = room < u64(TILE_POSITIONS<BLOCK>) ? u32(room) : u32(TILE_POSITIONS<BLOCK>);
     u32 key[TEXT_ITEMS], place[TEXT_ITEMS];      // place: bin << 16 | rank inside the tile's run of the bin
+    u32 taken = 0;                               // a bit per suffix
     #pragma unroll
     for(int i = 0; i < TEXT_ITEMS; ++i)
     {
         u32 high, low;
         stream_bits(stream, off, high, low);
         off += ent[i] & 31u;
-        const u32 bin = bits ? high >> (32 - bits) : 0u;
+        const u32 bin = (bits ? high >> (32 - bits) : 0u) - (PART ? first_bin : 0u);
         key[i] = keep_top ? high : __funnelshift_l(low, high, bits);
         place[i] = bin << 16;
-        if(local + i < valid) place[i] |= atomicAdd(&cnt[bin], 1u);
+        if(local + i < valid && (!PART || bin < bins)) { place[i] |= atomicAdd(&cnt[bin], 1u); taken |= PART ? 1u << i : 0u; }
     }
     __syncthreads();
     constexpr int PER = (1 << MAX_B1) / BLOCK;      // bins per thread
@@ -399,14 +402,15 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     __syncthreads();
     #pragma unroll
     for(int i = 0; i < TEXT_ITEMS; ++i)
-        if(local + i < valid)
+        if(PART ? (taken >> i & 1u) != 0 : local + i < valid)
         {
             const u32 bin = place[i] >> 16, at = cnt[bin] + (place[i] & 0xFFFFu);
             stage[at] = (u64(key[i]) << 32) | u32(first + local + i);
             stage_bin[at] = u16(bin);
         }
     __syncthreads();
-    for(u32 j = threadIdx.x; j < valid; j += BLOCK) out[base[stage_bin[j]] + j] = stage[j];
+    const u32 staged = PART ? total : valid;
+    for(u32 j = threadIdx.x; j < staged; j += BLOCK) out[base[stage_bin[j]] + j] = stage[j];
 }
 
 // ---- second split: every parent by the next bits ----------------------------------------------------------------------------------
@@ -819,15 +823,18 @@ int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bi
     return CSA_OK;
 }
 
-template <int BLOCK>
-int launch_scatter_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, int keep_top, u32* cursor, u64* out)
+template <int BLOCK, bool PART>
+int launch_scatter_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, int keep_top, u32 first_bin, u32 part_bins, u32* cursor, u64* out)
 {
     static std::atomic<bool> configured[64];
-    CSA_TRY(shared_bytes(ctx, scatter_text_kernel<BLOCK>, SCATTER_TEXT_SMEM<BLOCK>, configured));
-    scatter_text_kernel<BLOCK><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, SCATTER_TEXT_SMEM<BLOCK>, ctx->stream>>>(T, n, code, bits, keep_top, cursor, out);
+    CSA_TRY(shared_bytes(ctx, scatter_text_kernel<BLOCK, PART>, SCATTER_TEXT_SMEM<BLOCK>, configured));
+    scatter_text_kernel<BLOCK, PART><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, SCATTER_TEXT_SMEM<BLOCK>, ctx->stream>>>(T, n, code, bits, keep_top, first_bin, part_bins,
+                                                                                                                                cursor, out);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
+
+bool wide_tiles(u64 n) { return n >= (u64(1) << 22); }         // small texts take small tiles, so that every SM gets one
 
 }   // namespace
 
@@ -867,10 +874,12 @@ bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
     return cv.ok;
 }
 
-int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
-                       u64** list, u64** records, cudaEvent_t after_first_split)
+namespace
 {
-    const u64 n = ps.n;
+
+// The code of the text's symbols; the counters of the first split and of the build are cleared on the way.
+int launch_code(csa_ctx* ctx, const Prefix_Tables& t, const u16* T, const u64 n, Build_Counts* counts)
+{
     // the code, from every symbol of a small text or a million of a large one
     static_assert(CODE_BLOCK == 1 << MAX_B1, "block 0 of make_code_kernel clears a counter of the first split per thread");
     if(n <= CODE_COUNT_MAX)
@@ -895,15 +904,54 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
                                                                                           reinterpret_cast<u32*>(counts));
         CSA_LAUNCH_CHECK(ctx);
     }
+    return CSA_OK;
+}
+
+int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, u32* counts)
+{
+    return wide_tiles(n) ? launch_count_text<512>(ctx, T, n, code, bits, counts) : launch_count_text<128>(ctx, T, n, code, bits, counts);
+}
+
+// The second split of `parents` buckets with n records in all (recA to recB).
+int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB)
+{
+    const unsigned tiles = unsigned(n / SPLIT_TILE + parents);
+    const u32 children = 1u << b2;
+    CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(parents) * children * 4, ctx->stream));
+    count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2);
+    CSA_LAUNCH_CHECK(ctx);
+    child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off);
+    CSA_LAUNCH_CHECK(ctx);
+    static std::atomic<bool> configured[64];
+    CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
+    scatter_children_kernel<<<tiles, SPLIT_BLOCK, SPLIT_SMEM, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2, recB);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
+{
+    static std::atomic<bool> configured[64];
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel, LOCAL_SMEM, configured));
+    local_sort_kernel<<<unsigned(n / LOCAL_CHUNK + parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.par_off, t.chunk0, parents, b2, t.child_off, sa, list, n, counts, t.over);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+}   // namespace
+
+int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
+                       u64** list, u64** records, cudaEvent_t after_first_split)
+{
+    const u64 n = ps.n;
+    CSA_TRY(launch_code(ctx, t, T, n, counts));
     const bool one_level = ps.b1 == 0;
     const int bits = one_level ? ps.b2 : ps.b1;
-    const u32 bins = 1u << bits;
-    const bool wide = n >= (u64(1) << 22);          // small texts take small tiles, so that every SM gets one
-    if(bits > 0) CSA_TRY(wide ? launch_count_text<512>(ctx, T, n, t.code, bits, t.cnt1) : launch_count_text<128>(ctx, T, n, t.code, bits, t.cnt1));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, bins, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, p, counts);
+    if(bits > 0) CSA_TRY(launch_count_text(ctx, T, n, t.code, bits, t.cnt1));
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, p, counts);
     CSA_LAUNCH_CHECK(ctx);
-    CSA_TRY(wide ? launch_scatter_text<512>(ctx, T, n, t.code, bits, one_level ? 1 : 0, t.cur1, recA)
-                 : launch_scatter_text<128>(ctx, T, n, t.code, bits, one_level ? 1 : 0, t.cur1, recA));
+    CSA_TRY(wide_tiles(n) ? (launch_scatter_text<512, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA))
+                          : (launch_scatter_text<128, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA)));
     CSA_CUDA(ctx, cudaEventRecord(after_first_split, ctx->stream));
     ctx->counters[1] += one_level ? 1 : 2;
     ctx->counters[2] += one_level ? n : 2 * n;
@@ -911,27 +959,45 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     u64* other = recB;
     if(!one_level)
     {
-        const unsigned tiles = unsigned(n / SPLIT_TILE + ps.parents);
-        CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(ps.parents) * ps.children * 4, ctx->stream));
-        count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, ps.parents, ps.b2, t.cnt2);
-        CSA_LAUNCH_CHECK(ctx);
-        child_offsets_kernel<<<ps.parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, ps.parents, ps.children, t.child_off);
-        CSA_LAUNCH_CHECK(ctx);
-        static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
-        scatter_children_kernel<<<tiles, SPLIT_BLOCK, SPLIT_SMEM, ctx->stream>>>(recA, t.par_off, t.tile0, ps.parents, ps.b2, t.cnt2, recB);
-        CSA_LAUNCH_CHECK(ctx);
+        CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB));
         rec = recB; other = recA;
     }
-    {
-        static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel, LOCAL_SMEM, configured));
-        local_sort_kernel<<<unsigned(n / LOCAL_CHUNK + ps.parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.par_off, t.chunk0, ps.parents, ps.b2, t.child_off, sa, other, n,
-                                                                                                          counts, t.over);
-        CSA_LAUNCH_CHECK(ctx);
-    }
+    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, n, rec, sa, other, counts));
     *list = other;
     *records = rec;
+    return CSA_OK;
+}
+
+Prefix_Sort prefix_sort_part_plan(u64 n)
+{
+    Prefix_Sort ps = prefix_sort_plan(n);
+    const int t = ps.b1 + ps.b2;
+    ps.b1 = t - 1 < 1 ? 1 : (t - 1 > MAX_B1 ? MAX_B1 : t - 1);
+    ps.b2 = t - ps.b1 < 1 ? 1 : t - ps.b1;
+    ps.key_bits = ps.b1 + 32;
+    ps.parents = 1u << ps.b1;
+    ps.children = 1u << ps.b2;
+    return ps;
+}
+
+int launch_prefix_counts(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, Build_Counts* counts)
+{
+    CSA_TRY(launch_code(ctx, t, T, ps.n, counts));
+    return launch_count_text(ctx, T, ps.n, t.code, ps.b1, t.cnt1);
+}
+
+int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u32 first_bin, u32 bins, u64 size, u64* recA, u64* recB, u32* sa,
+                            Build_Counts* counts)
+{
+    CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, 1, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
+                             : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));
+    CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB));
+    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, size, recB, sa, recA, counts));
+    ctx->counters[1] += 2;
+    ctx->counters[2] += 2 * size;
     return CSA_OK;
 }
 

@@ -62,3 +62,12 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
 // The records of the children that did not fit a block, as sort records: keys = (first slot of the child << 32) | key,
 // vals = position.
 int launch_gather_oversize(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, u32 oversize, const u64* records, u64* keys, u32* vals, u32* cursor);
+
+// The same for a text whose records do not all fit the device: one contiguous range of the suffix array at a time. The first split's
+// buckets are counted once (cnt1, 1 << b1 of them); a part is a run of buckets with `size` suffixes in all, for which the text is
+// encoded again. There are always two splits.
+Prefix_Sort prefix_sort_part_plan(u64 n);
+int launch_prefix_counts(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, Build_Counts* counts);
+// recA, recB, sa: `size` entries each; slots count from the part's first. The list of tied suffixes is left in recA.
+int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u32 first_bin, u32 bins, u64 size, u64* recA, u64* recB, u32* sa,
+                            Build_Counts* counts);

@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
         #pragma unroll
         for(int i = 0; i < RW_ITEMS; ++i) depth[tid + i * RW_BLOCK] = u32(from);
         __syncthreads();
-        bool quick = from < QUICK_REACH && to - from >= QUICK_REACH && count * 4 < n;
+        int quick = from < QUICK_REACH && to - from >= 2 * QUICK_REACH && count * 4 < n ? 2 : 0;       // rounds of that kind
         while(true)
         {
             const u32 reach = quick ? QUICK_REACH : WIDE_REACH;
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
                     if(s == j) key[j] = KEY_EQUAL;
                     if(s == NO_GROUP || j == s) continue;
                     open = true;
-                    const u64 x = u64(w.pos[j]) + from, y = u64(w.pos[s]) + from;
+                    const u64 x = u64(w.pos[j]) + depth[s], y = u64(w.pos[s]) + depth[s];
                     const ulonglong2 none = make_ulonglong2(0, 0);
                     const ulonglong2 a = x < n ? eight_symbols(T, x) : none, b = y < n ? eight_symbols(T, y) : none;
                     const u64 has_a = x < n ? n - x : 0, has_b = y < n ? n - y : 0;
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
                     if(at == s) { w.ge[at] = u16(to_e[i]); depth[at] = deeper[i]; }
                 }
             __syncthreads();
-            quick = false;
+            quick -= quick > 0;
         }
         __syncthreads();
         if(tid < RW_WINDOW / 32) w.mask[tid] = 0;
@@ -777,6 +777,17 @@ int ranks_from(csa_ctx* ctx, const u32* sa, const u64* list, u64 count, u64 n, u
 }
 
 }   // namespace
+
+int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c)
+{
+    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + CSA_COUNTS_WORD, ctx->d_scalars + CSA_COUNTS_WORD, (CSA_STATUS_WORD + 1 - CSA_COUNTS_WORD) * 8, cudaMemcpyDeviceToHost,
+                                  ctx->stream));
+    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if(ctx->h_scalars[CSA_STATUS_WORD] != 0) { u64 b = 0; return csa_sync(ctx, reinterpret_cast<uint64_t*>(&b)); }
+    c = *reinterpret_cast<const Build_Counts*>(ctx->h_scalars + CSA_COUNTS_WORD);
+    if(c.small > most || u64(c.next_small) + c.large > most) return csa_fail(ctx, CSA_E_DEVICE, "build: the lists of tied suffixes do not add up");
+    return CSA_OK;
+}
 
 int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, Build_Counts* counts, u64 expected)
 {

@@ -5,6 +5,14 @@
 #include "common.cuh"
 #include "prefix_sort.cuh"
 
+// Text is compared up to this depth before ranks are: past it one more doubling costs a suffix less (an inverse rank, 64 bytes of
+// DRAM traffic) than its next symbols do.
+constexpr u64 TEXT_DEPTH = 61;         // what tied suffixes share at least (1) + a wide round (refine.cu)
+
+// The counters of the build as the stream leaves them; waits for the stream. Fails if a kernel reported an error or if the lists
+// hold more than `most` entries.
+int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c);
+
 // Orders the small groups of `list` by their suffixes' symbols [from, to) read straight from the text (a suffix that ends
 // inside them comes before those that go on): every group that is left shares `to` symbols. Suffixes that are alone now go to
 // their slots of sa, the others to next (front; counts->next_small entries). `expected`: about how many entries the list holds

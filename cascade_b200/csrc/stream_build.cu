@@ -22,8 +22,13 @@
 // Where the reference pushes (target, rank) messages into the host inboxes of other partitions and joins them by search,
 // a part here writes its new ranks as (position, rank) messages into an outbox on the device, and the exchange applies
 // them to R after the generation's last part: every read of a generation sees the ranks of the generation before.
+//
+// A text without long repeats needs none of this: direct_parts below orders one range of the array after the other from the text
+// alone, and the protocol above is what a text falls back to.
 #include "common.cuh"
 #include "part.cuh"
+#include "prefix_sort.cuh"
+#include "refine.cuh"
 
 #include "sort.cuh"
 
@@ -830,6 +835,120 @@ struct Part_Files
 };
 }
 
+namespace
+{
+
+// A part is encoded from the whole text again (6 ps a position and part on the device), where the lists of the general way cost
+// about 0.9 ns a suffix over PCIe: up to this many parts the direct way moves less.
+constexpr u64 DIRECT_MAX_PARTS = 64;
+constexpr u64 DIRECT_MIN = 1 << 14;
+
+// The parts of the suffix array one after the other, straight from the text on the device: the suffixes whose encoding starts
+// with a run of leading bits are sorted by prefix_sort.cu, their ties are ordered by the text, and the finished range of the
+// array is copied out under the sorting of the next. No list leaves the device and no ranks are kept: PCIe carries the text in and
+// the array out once (7 bytes a suffix; the lists take 41). `done` stays false where that is not enough (a part with groups of many tied
+// suffixes or with long shared stretches, a run of bits with more suffixes than a part may hold): the caller then starts over the
+// general way, whatever was copied out.
+int direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, const u64 part_suffixes, u8* sa40_host, csa_build_stats& bs, bool& done)
+{
+    const auto t_start = std::chrono::steady_clock::now();
+    const Prefix_Sort ps = prefix_sort_part_plan(n);
+    const u64 most = n < part_suffixes ? n : part_suffixes;
+    const size_t rec = align_up256(most * 8), slots = align_up256(most * 4 + 64), out_bytes = align_up256(most * 5 + CSA_SA_PAD_BYTES);
+    const size_t total = align_up256(prefix_sort_table_bytes(ps)) + 2 * rec + slots + 2 * out_bytes + 4096;
+    void* ws = nullptr;
+    CSA_TRY(csa_arena(ctx, total, &ws));
+    Carver cv(ws, total);
+    Prefix_Tables tab;
+    u64* const recA = cv.take<u64>(rec / 8);
+    u64* const recB = cv.take<u64>(rec / 8);
+    u32* const sa = cv.take<u32>(slots / 4);
+    u8* const out[2] = {cv.take<u8>(out_bytes), cv.take<u8>(out_bytes)};
+    if(!cv.ok || !prefix_sort_carve(cv, ps, tab)) return csa_fail(ctx, CSA_E_NOMEM, "streamed build: workspace too small");
+    CSA_TRY(csa_lanes(ctx));
+    Build_Counts* const counts = reinterpret_cast<Build_Counts*>(ctx->d_scalars + CSA_COUNTS_WORD);
+
+    CSA_TRY(launch_prefix_counts(ctx, ps, tab, T, counts));
+    std::vector<u32> size(ps.parents);
+    CSA_CUDA(ctx, cudaMemcpyAsync(size.data(), tab.cnt1, size.size() * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    std::vector<u32> first_bin(1, 0);           // of every part, and the end
+    std::vector<u64> part_off(1, 0);
+    u64 sum = 0;
+    std::vector<u64> formed(p, 0);              // the statistics' partitions: a bucket belongs to the p-th part of the array in which it starts
+    for(u32 b = 0; b < ps.parents; ++b)
+    {
+        if(size[b] > most) return CSA_OK;
+        if(sum + size[b] - part_off.back() > most) { first_bin.push_back(b); part_off.push_back(sum); }
+        if(size[b]) formed[size_t(sum * p / n)] += size[b];
+        sum += size[b];
+    }
+    if(sum != n) return csa_fail(ctx, CSA_E_DEVICE, "streamed build: the counts do not add up to n");
+    first_bin.push_back(ps.parents);
+    part_off.push_back(n);
+    const u32 parts = u32(part_off.size() - 1);
+    if(parts > DIRECT_MAX_PARTS) return CSA_OK;
+    const double ms_counted = ms_since(t_start);
+
+    const u64 depth0 = u64(ps.key_bits / CODE_MAX_LEN);
+    const cudaStream_t copy_stream = ctx->lane[0];
+    const cudaEvent_t packed = ctx->lane_event[0], copied[2] = {ctx->lane_event[1], ctx->lane_event[2]};
+    struct Drain { cudaStream_t s; ~Drain() { cudaStreamSynchronize(s); } } drain{copy_stream};       // no copy outlives the call, nor runs under the general way
+    u64 active = 0;
+    u32 rounds = 0;
+    for(u32 u = 0; u < parts; ++u)
+    {
+        const u64 S = part_off[u + 1] - part_off[u];
+        if(S == 0) continue;
+        CSA_TRY(launch_prefix_sort_part(ctx, ps, tab, T, first_bin[u], first_bin[u + 1] - first_bin[u], S, recA, recB, sa, counts));
+        u64* list = recA;
+        u64* next = recB;
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
+        Build_Counts c;
+        CSA_TRY(read_build_counts(ctx, S, c));
+        if(c.oversize || c.large) return CSA_OK;
+        active += c.small;
+        u32 r = c.small ? 1 : 0;
+        u64 depth = TEXT_DEPTH;
+        for(u64 small = c.next_small; small; small = c.next_small)
+        {
+            if(small * depth > S || depth >= n) return CSA_OK;      // as in the resident build: from here on ranks are cheaper than text
+            std::swap(list, next);
+            CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
+            CSA_CUDA(ctx, cudaMemsetAsync(&counts->next_small, 0, 4, ctx->stream));
+            CSA_TRY(launch_refine_by_text(ctx, T, n, depth, 4 * depth, list, next, sa, counts, small));
+            CSA_TRY(read_build_counts(ctx, S, c));
+            depth *= 4;
+            ++r;
+        }
+        if(r > rounds) rounds = r;
+        CSA_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, copied[u & 1], 0));       // the copy out of this buffer, two parts ago
+        CSA_TRY(launch_pack_sa40(ctx, sa, S, out[u & 1]));
+        CSA_CUDA(ctx, cudaEventRecord(packed, ctx->stream));
+        CSA_CUDA(ctx, cudaStreamWaitEvent(copy_stream, packed, 0));
+        CSA_CUDA(ctx, cudaMemcpyAsync(sa40_host + 5 * part_off[u], out[u & 1], 5 * S, cudaMemcpyDeviceToHost, copy_stream));
+        CSA_CUDA(ctx, cudaEventRecord(copied[u & 1], copy_stream));
+    }
+    CSA_CUDA(ctx, cudaStreamSynchronize(copy_stream));
+    u64 status = 0;
+    CSA_TRY(csa_sync(ctx, reinterpret_cast<uint64_t*>(&status)));
+    for(const u64 f : formed)
+    {
+        bs.partitions += f != 0;
+        if(f > bs.max_partition) bs.max_partition = f;
+    }
+    bs.active_after_gen0 = active;
+    if(active) bs.active_per_gen[0] = active;
+    bs.generations = rounds;
+    bs.ms_partition = ms_counted;
+    bs.ms_gen0 = ms_since(t_start) - ms_counted;
+    bs.host_parts = parts;
+    done = true;
+    return CSA_OK;
+}
+
+}   // namespace
+
 extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint64_t n, uint32_t p, uint64_t seed, uint8_t* sa40_host,
                                    const csa_tier_options* options, csa_build_stats* stats)
 {
@@ -851,11 +970,27 @@ extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint
     // ---- text and partition ids on the device ------------------------------------------------------------------------------
     Dev_Buffer text_b, pid_b, small_b, stage_b;
     CSA_TRY(text_b.alloc(ctx, (n + CSA_TEXT_PAD) * 2 + 256));
-    CSA_TRY(pid_b.alloc(ctx, n * 2 + 256));
     u16* T = static_cast<u16*>(text_b.p);
-    u16* pid = static_cast<u16*>(pid_b.p);
     CSA_CUDA(ctx, cudaMemcpyAsync(T, text_host, n * 2, cudaMemcpyHostToDevice, ctx->stream));
     CSA_CUDA(ctx, cudaMemsetAsync(T + n, 0, CSA_TEXT_PAD * 2, ctx->stream));
+    if(part_suffixes == 0) part_suffixes = u64(1) << 27;
+    if(part_suffixes >= (u64(1) << 31)) part_suffixes = (u64(1) << 31) - 1;
+    // The direct way serves texts of 31-bit positions whose array goes to memory and whose lists, were they needed, would too.
+    if(sa40_host && !options->output_path && offset == 0 && n >= DIRECT_MIN && n < (u64(1) << 31) && options->host_list_bytes >= 9 * n)
+    {
+        bool done = false;
+        CSA_TRY(direct_parts(ctx, T, n, p, part_suffixes, sa40_host, bs, done));
+        if(done)
+        {
+            bs.ms_total = ms_since(t_start);
+            bs.kernel_launches = ctx->counters[0] - launches_before;
+            bs.sort_passes = ctx->counters[1] - passes_before;
+            bs.sort_records = ctx->counters[2] - records_before;
+            return CSA_OK;
+        }
+    }
+    CSA_TRY(pid_b.alloc(ctx, n * 2 + 256));
+    u16* pid = static_cast<u16*>(pid_b.p);
     constexpr u64 MAX_SAMPLES = 1u << 19;
     const size_t split_bytes = align_up256(pick_splitters_scratch_bytes(MAX_SAMPLES));
     CSA_TRY(small_b.alloc(ctx, split_bytes + align_up256(size_t(2) * p * 8) + 3 * align_up256(size_t(CSA_MAX_PARTITIONS) * 8) + align_up256(65536 * 4) + 4096));
@@ -893,8 +1028,6 @@ extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint
     CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
 
     // ---- parts: runs of whole partitions, each below the size asked for (and below 2^31) -----------------------------------
-    if(part_suffixes == 0) part_suffixes = u64(1) << 27;
-    if(part_suffixes >= (u64(1) << 31)) part_suffixes = (u64(1) << 31) - 1;
     std::vector<u16> part_of_pid(p_eff);
     std::vector<u64> part_off(1, 0);
     {

@@ -301,3 +301,21 @@ def test_rank_shard_primitives(ctx):
     assert int(one.item()) == 0
     ctx.check(L.csa_rank_shard_read(ctx.h, shard.data_ptr(), lo, cnt, asked.data_ptr(), 1, one.data_ptr()))
     ctx.sync()                                        # the context works on
+
+
+@pytest.mark.parametrize("n,part_suffixes", [(1 << 14, 0), (70_001, 20_000), (70_001, 1500), ((1 << 21) + 3, 1 << 18), ((1 << 22) + 5, 1_000_003)])
+@pytest.mark.parametrize("tail", ["zipf", "few_long_repeats", "period_in_the_last_part"])
+def test_parts_straight_from_the_text(ctx, oracle, n, part_suffixes, tail):
+    """Texts whose parts need the text alone, texts with a long repeat that is read further, and texts that show only in their last part
+    that they need the general way (parts of 1500 suffixes are more than the direct way takes, too)."""
+    from cascade_b200 import api
+    rng = np.random.default_rng(n)
+    T = np.minimum(rng.zipf(1.3, n), 50000).astype(np.uint16)
+    if tail == "few_long_repeats":
+        T[n // 2:n // 2 + 40] = T[:40]
+        T[-100:] = T[300:400]
+    elif tail == "period_in_the_last_part":
+        T[n // 3:n // 3 + 3000] = np.resize([65535, 65534, 65535], 3000)
+    sa, st = api.build_sa_streamed(ctx, _padded(T), n, 16, part_suffixes=part_suffixes)
+    assert np.array_equal(sa[:5 * n], oracle.build_sa40(T)[:5 * n])
+    assert 1 <= st.partitions <= 16 and 0 < st.max_partition <= n and st.host_parts >= 1
