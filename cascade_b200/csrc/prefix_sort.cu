@@ -29,7 +29,9 @@ constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at m
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
 constexpr int LOCAL_BLOCK = 512, LOCAL_ITEMS = 16, LOCAL_CAP = LOCAL_BLOCK * LOCAL_ITEMS;
-constexpr u32 LOCAL_CHUNK = LOCAL_CAP / 2;  // children that start inside one chunk of slots belong to one block
+// Children that start inside one chunk of slots belong to one block: two children as a rule, or one in a short text (one split, up
+// to 2^21 suffixes), where every SM should get a block.
+constexpr u32 LOCAL_CHUNK = LOCAL_CAP / 2, SHORT_CHUNK = LOCAL_CAP / 8;
 
 // ---- the code ----------------------------------------------------------------------------------------------------------------
 
@@ -91,14 +93,9 @@ __device__ __forceinline__ u32 block_exclusive(const u32 v, u32* warp_tot, u32& 
     const u32 inc = warp_inclusive(v);
     if(lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
     __syncthreads();
-    u32 pre = 0, all = 0;
-    #pragma unroll
-    for(int w = 0; w < BLOCK / 32; ++w)
-    {
-        const u32 t = warp_tot[w];
-        if(w < int(threadIdx.x >> 5)) pre += t;
-        all += t;
-    }
+    const u32 t = lane_id() < BLOCK / 32 ? warp_tot[lane_id()] : 0;        // every warp sums the warps' totals
+    const u32 upto = warp_inclusive(t);
+    const u32 all = __shfl_sync(0xFFFFFFFFu, upto, 31), pre = __shfl_sync(0xFFFFFFFFu, upto - t, threadIdx.x >> 5);
     __syncthreads();
     total = all;
     return pre + inc - v;
@@ -218,14 +215,24 @@ __global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __rest
 // A block of BLOCK threads takes BLOCK * TEXT_ITEMS consecutive symbols, of which the last LOOKAHEAD only complete the keys of
 // those before them: a tile yields the keys of TILE_POSITIONS suffixes.
 template <int BLOCK> constexpr int TILE_POSITIONS = BLOCK * TEXT_ITEMS - LOOKAHEAD;
-template <int BLOCK> constexpr int STREAM_WORDS = (BLOCK * TEXT_ITEMS * CODE_MAX_LEN / 32 + 4 + 3) / 4 * 4;
 
-// Writes the code words of the symbols [first, first + BLOCK * TEXT_ITEMS) one behind the other into `stream` (bit 31 of word 0
-// first) and returns the bit at which the thread's first symbol starts; ent holds its symbols' code entries. Symbols past the
-// text's end count as 0. first is a multiple of 16 and T is 16-byte aligned with CSA_TEXT_PAD readable symbols behind n.
+// The first 64 bits of a suffix's encoding follow from those of the next suffix: its own symbol's code word, then the other's bits.
+// So a thread walks its symbols from the last to the first with one 64-bit window, and needs only the window behind its last symbol.
+__device__ __forceinline__ u64 before(const u32 entry, const u64 window) { return u64(entry & ~31u) << 32 | window >> (entry & 31u); }
+
+template <int BLOCK> struct Tile_Code
+{
+    u64 window[BLOCK];      // of every thread: the first bits of its symbols
+    u32 bits[BLOCK];        // and how many its symbols have
+};
+
+// The code entries of the thread's symbols [first + threadIdx.x * TEXT_ITEMS, + TEXT_ITEMS) in ent, and the window behind the last. Symbols
+// past the text's end count as 0. first is a multiple of 16 and T is 16-byte aligned with CSA_TEXT_PAD readable symbols behind n.
+// The windows of the last LOOKAHEAD symbols' threads are not complete. Ends without a barrier behind the reads of `tc`.
+// (Writing the code words one behind the other into shared memory and reading every suffix's words from there, the scatter at 2e9 symbols
+// took 12.9 ms, at 88 % of L1's wavefronts; this way 10.7 ms.)
 template <int BLOCK>
-__device__ __forceinline__ u32 encode_tile(const u16* __restrict__ T, const u64 n, const u64 first, const u32* __restrict__ code, u32* stream, u32* warp_tot,
-                                           u32 (&ent)[TEXT_ITEMS])
+__device__ __forceinline__ u64 encode_tile(const u16* __restrict__ T, const u64 n, const u64 first, const u32* __restrict__ code, Tile_Code<BLOCK>& tc, u32 (&ent)[TEXT_ITEMS])
 {
     const u64 at = first + u64(threadIdx.x) * TEXT_ITEMS;
     u32 sym2[TEXT_ITEMS / 2];
@@ -241,40 +248,19 @@ __device__ __forceinline__ u32 encode_tile(const u16* __restrict__ T, const u64 
         for(int i = 0; i < TEXT_ITEMS / 2; ++i)
             sym2[i] = (at + 2 * i < n ? u32(T[at + 2 * i]) : 0u) | (at + 2 * i + 1 < n ? u32(T[at + 2 * i + 1]) << 16 : 0u);
     }
-    for(u32 i = threadIdx.x; i < STREAM_WORDS<BLOCK> / 4; i += BLOCK) reinterpret_cast<uint4*>(stream)[i] = make_uint4(0, 0, 0, 0);
-    u32 bits = 0;
     #pragma unroll
     for(int i = 0; i < TEXT_ITEMS; ++i) ent[i] = __ldg(code + ((i & 1) ? sym2[i >> 1] >> 16 : sym2[i >> 1] & 0xFFFFu));
+    u64 own = 0;
+    u32 bits = 0;
     #pragma unroll
-    for(int i = 0; i < TEXT_ITEMS; ++i) bits += ent[i] & 31u;
-    u32 total;
-    const u32 begin = block_exclusive<BLOCK>(bits, warp_tot, total);      // its barriers also stand between the clearing and the writing
-    u32 word = begin >> 5, fill = begin & 31u, acc = 0;
-    #pragma unroll
-    for(int i = 0; i < TEXT_ITEMS; ++i)
-    {
-        const u32 c = ent[i] & ~31u, len = ent[i] & 31u;
-        acc |= c >> fill;
-        fill += len;
-        if(fill >= 32)
-        {
-            atomicOr(&stream[word++], acc);         // a word may be shared with the thread before or behind
-            fill -= 32;
-            acc = fill ? c << (len - fill) : 0u;
-        }
-    }
-    if(acc) atomicOr(&stream[word], acc);
+    for(int i = TEXT_ITEMS - 1; i >= 0; --i) { own = before(ent[i], own); bits += ent[i] & 31u; }
+    tc.window[threadIdx.x] = own;
+    tc.bits[threadIdx.x] = bits;
     __syncthreads();
-    return begin;
-}
-
-// The 64 bits of the stream from bit `off` on.
-__device__ __forceinline__ void stream_bits(const u32* stream, const u32 off, u32& high, u32& low)
-{
-    const u32 w = off >> 5, s = off & 31u;
-    const u32 a = stream[w], b = stream[w + 1], c = stream[w + 2];
-    high = __funnelshift_l(b, a, s);
-    low = __funnelshift_l(c, b, s);
+    u64 behind = 0;
+    u32 have = 0;       // a thread's symbols have 16 bits or more: four threads fill a window, one as a rule
+    for(u32 t = threadIdx.x + 1; t < BLOCK && have < 64; ++t) { behind |= tc.window[t] >> have; have += tc.bits[t]; }
+    return behind;
 }
 
 // ---- first split: by the top bits, straight from the text -----------------------------------------------------------------------
@@ -282,36 +268,101 @@ __device__ __forceinline__ void stream_bits(const u32* stream, const u32 off, u3
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) count_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits, u32* __restrict__ counts)
 {
-    extern __shared__ __align__(16) u32 smem_words[];
-    u32* const stream = smem_words;
-    u32* const cnt = stream + STREAM_WORDS<BLOCK>;
-    __shared__ u32 warp_tot[BLOCK / 32];
+    __shared__ Tile_Code<BLOCK> tc;
+    __shared__ u32 cnt[1 << MAX_B1];
     const u32 bins = 1u << bits;
     for(u32 i = threadIdx.x; i < bins; i += BLOCK) cnt[i] = 0;
     const u64 first = u64(blockIdx.x) * TILE_POSITIONS<BLOCK>;
     u32 ent[TEXT_ITEMS];
-    u32 off = encode_tile<BLOCK>(T, n, first, code, stream, warp_tot, ent);
+    u64 window = encode_tile<BLOCK>(T, n, first, code, tc, ent);
     const u32 local = threadIdx.x * TEXT_ITEMS;
     const u64 room = n - first;
     const u32 valid = room < u64(TILE_POSITIONS<BLOCK>) ? u32(room) : u32(TILE_POSITIONS<BLOCK>);
     #pragma unroll
-    for(int i = 0; i < TEXT_ITEMS; ++i)
+    for(int i = TEXT_ITEMS - 1; i >= 0; --i)
     {
-        const u32 w = off >> 5;
-        const u32 high = __funnelshift_l(stream[w + 1], stream[w], off & 31u);
-        if(local + i < valid) atomicAdd(&cnt[high >> (32 - bits)], 1u);
-        off += ent[i] & 31u;
+        window = before(ent[i], window);
+        if(local + i < valid) atomicAdd(&cnt[u32(window >> 32) >> (32 - bits)], 1u);
     }
     __syncthreads();
     for(u32 i = threadIdx.x; i < bins; i += BLOCK)
         if(cnt[i]) atomicAdd(&counts[i], cnt[i]);
 }
 
+// The same for long texts: one block an SM holds the whole code in shared memory, cut to what the first split looks at (12 bits
+// of the code word and a length up to 15: 16 bits a symbol), since a gather from the 256 KB table through L1 is what bounds the
+// kernel above (5.5 ms at 2e9 symbols, this way 1.7 ms). A warp goes through strips of 512 symbols by itself; the last lane's 16
+// only complete the windows before them.
+constexpr int COUNT_BLOCK = 1024;
+constexpr u32 STRIP = 31 * TEXT_ITEMS;
+constexpr size_t COUNT_SMEM = 65536 * 2;
+static_assert(MAX_B1 <= 12 && TEXT_ITEMS >= 12, "12 bits of a code word are kept, and the next lane's symbols have as many");
+
+__global__ void __launch_bounds__(COUNT_BLOCK) count_long_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits, u32* __restrict__ counts)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u16* const table = reinterpret_cast<u16*>(smem_raw);
+    __shared__ u32 cnt[1 << MAX_B1];
+    const u32 bins = 1u << bits, lane = lane_id();
+    for(u32 i = threadIdx.x; i < bins; i += COUNT_BLOCK) cnt[i] = 0;
+    for(u32 i = threadIdx.x; i < 65536 / 4; i += COUNT_BLOCK)
+    {
+        const uint4 c = __ldg(reinterpret_cast<const uint4*>(code) + i);
+        auto cut = [](const u32 e) { return u16((e >> 16 & 0xFFF0u) | min(e & 31u, 15u)); };
+        reinterpret_cast<ushort4*>(table)[i] = make_ushort4(cut(c.x), cut(c.y), cut(c.z), cut(c.w));
+    }
+    __syncthreads();
+    const u64 strips = (n + STRIP - 1) / STRIP, step = u64(gridDim.x) * (COUNT_BLOCK / 32);
+    u64 strip = u64(blockIdx.x) * (COUNT_BLOCK / 32) + (threadIdx.x >> 5);
+    auto load = [&](const u64 s, uint4& a, uint4& b)
+    {
+        const u64 at = s * STRIP + lane * TEXT_ITEMS;
+        a = make_uint4(0, 0, 0, 0); b = a;
+        if(s < strips && at + TEXT_ITEMS <= n + CSA_TEXT_PAD)       // what is cut off lies past the text and counts as 0
+        {
+            a = *reinterpret_cast<const uint4*>(T + at);
+            b = *reinterpret_cast<const uint4*>(T + at + 8);
+        }
+    };
+    uint4 a, b;
+    load(strip, a, b);
+    for(; strip < strips; strip += step)
+    {
+        const u32 sym2[TEXT_ITEMS / 2] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        load(strip + step, a, b);
+        u32 ent[TEXT_ITEMS];
+        #pragma unroll
+        for(int i = 0; i < TEXT_ITEMS; ++i) ent[i] = table[(i & 1) ? sym2[i >> 1] >> 16 : sym2[i >> 1] & 0xFFFFu];
+        auto step_back = [](const u32 e, const u32 w) { return (e & 0xFFF0u) << 16 | w >> (e & 15u); };
+        u32 own = 0;
+        #pragma unroll
+        for(int i = 11; i >= 0; --i) own = step_back(ent[i], own);     // 12 symbols have 12 bits or more
+        u32 window = __shfl_down_sync(0xFFFFFFFFu, own, 1);
+        const u64 at = strip * STRIP + lane * TEXT_ITEMS;
+        const u32 valid = lane == 31 || at >= n ? 0u : (n - at < TEXT_ITEMS ? u32(n - at) : u32(TEXT_ITEMS));
+        #pragma unroll
+        for(int i = TEXT_ITEMS - 1; i >= 0; --i)
+        {
+            window = step_back(ent[i], window);
+            if(u32(i) < valid) atomicAdd(&cnt[window >> (32 - bits)], 1u);
+        }
+    }
+    __syncthreads();
+    for(u32 i = threadIdx.x; i < bins; i += COUNT_BLOCK)
+        if(cnt[i]) atomicAdd(&counts[i], cnt[i]);
+}
+
+// Child `next - 1` occupies the slots [r0, r1) of its parent: the chunks that begin behind its start begin with the next child.
+__device__ __forceinline__ void first_children(u32* __restrict__ chunk_first, const u32 chunks, const u32 chunk, const u32 r0, const u32 r1, const u32 next)
+{
+    for(u32 k = r0 / chunk + 1; k <= r1 / chunk && k < chunks; ++k) chunk_first[k] = next;
+}
+
 // Offsets of the parents and the work lists that follow from their sizes. one_level: there is no second split, the bins are
 // the children of one parent that holds everything.
 __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restrict__ counts, const u32 bins, const u32 n, const int one_level, u32* __restrict__ cursor,
-                                                             u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ chunk0, u32* __restrict__ child_off, const u32 p,
-                                                             Build_Counts* __restrict__ stats)
+                                                             u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ chunk0, u32* __restrict__ child_off, u32* __restrict__ chunk_first,
+                                                             const u32 p, Build_Counts* __restrict__ stats)
 {
     __shared__ u32 warp_tot[32];
     __shared__ u32 part[CSA_MAX_PARTITIONS];
@@ -329,8 +380,9 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
     if(formed) { atomicAdd(&stats->partitions, formed); atomicMax(&stats->max_partition, longest); }
     if(one_level)
     {
-        if(t < bins) child_off[t] = off;
-        if(t == 0) { child_off[bins] = n; par_off[0] = 0; par_off[1] = n; chunk0[0] = 0; chunk0[1] = (n + LOCAL_CHUNK - 1) / LOCAL_CHUNK; }
+        const u32 chunks = (n + SHORT_CHUNK - 1) / SHORT_CHUNK;
+        if(t < bins) { child_off[t] = off; first_children(chunk_first, chunks, SHORT_CHUNK, off, off + c, t + 1); }
+        if(t == 0) { child_off[bins] = n; chunk0[1] = chunks; chunk_first[0] = 0; chunk_first[chunks] = bins; }
         return;
     }
     const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE, chunks = (c + LOCAL_CHUNK - 1) / LOCAL_CHUNK;
@@ -342,7 +394,7 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
 }
 
 template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<BLOCK>) * 8 + size_t(TILE_POSITIONS<BLOCK>) * 2;
-static_assert(SCATTER_TEXT_SMEM<512> >= STREAM_WORDS<512> * 4 && SCATTER_TEXT_SMEM<128> >= STREAM_WORDS<128> * 4, "the stream lies where the records are staged later");
+static_assert(SCATTER_TEXT_SMEM<512> >= sizeof(Tile_Code<512>) && SCATTER_TEXT_SMEM<128> >= sizeof(Tile_Code<128>), "the windows lie where the records are staged later");
 
 // Scatter by the top `bits` bits: the places inside a bucket come from shared-memory atomics and, for the tile's run of a bucket,
 // from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs.
@@ -354,7 +406,6 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
                                                                           u64* __restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    u32* const stream = reinterpret_cast<u32*>(smem_raw);
     u64* const stage = reinterpret_cast<u64*>(smem_raw);
     u16* const stage_bin = reinterpret_cast<u16*>(stage + TILE_POSITIONS<BLOCK>);
     __shared__ u32 cnt[1 << MAX_B1];            // counts, then the bins' starts inside the tile
@@ -364,18 +415,17 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     for(u32 i = threadIdx.x; i < bins; i += BLOCK) cnt[i] = 0;
     const u64 first = u64(blockIdx.x) * TILE_POSITIONS<BLOCK>;
     u32 ent[TEXT_ITEMS];
-    u32 off = encode_tile<BLOCK>(T, n, first, code, stream, warp_tot, ent);
+    u64 window = encode_tile<BLOCK>(T, n, first, code, *reinterpret_cast<Tile_Code<BLOCK>*>(smem_raw), ent);
     const u32 local = threadIdx.x * TEXT_ITEMS;
     const u64 room = n - first;
     const u32 valid = room < u64(TILE_POSITIONS<BLOCK>) ? u32(room) : u32(TILE_POSITIONS<BLOCK>);
     u32 key[TEXT_ITEMS], place[TEXT_ITEMS];      // place: bin << 16 | rank inside the tile's run of the bin
     u32 taken = 0;                               // a bit per suffix
     #pragma unroll
-    for(int i = 0; i < TEXT_ITEMS; ++i)
+    for(int i = TEXT_ITEMS - 1; i >= 0; --i)
     {
-        u32 high, low;
-        stream_bits(stream, off, high, low);
-        off += ent[i] & 31u;
+        window = before(ent[i], window);
+        const u32 high = u32(window >> 32), low = u32(window);
         const u32 bin = (bits ? high >> (32 - bits) : 0u) - (PART ? first_bin : 0u);
         key[i] = keep_top ? high : __funnelshift_l(low, high, bits);
         place[i] = bin << 16;
@@ -456,7 +506,7 @@ __global__ void __launch_bounds__(SPLIT_BLOCK) count_children_kernel(const u64* 
 
 // One block per parent: the children's counts become their places (in counts, running) and their offsets (child_off).
 __global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ counts, const u32* __restrict__ par_off, const u32 parents, const u32 children,
-                                                            u32* __restrict__ child_off)
+                                                            u32* __restrict__ child_off, const u32* __restrict__ chunk0, u32* __restrict__ chunk_first)
 {
     __shared__ u32 warp_tot[32];
     const u32 p = blockIdx.x, t = threadIdx.x;
@@ -464,10 +514,14 @@ __global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ c
     const u32 i0 = 2 * t, i1 = 2 * t + 1;          // up to 2048 children
     const u32 a = i0 < children ? c[i0] : 0, b = i1 < children ? c[i1] : 0;
     u32 total;
-    const u32 off = par_off[p] + block_exclusive<1024>(a + b, warp_tot, total);
+    const u32 rel = block_exclusive<1024>(a + b, warp_tot, total), off = par_off[p] + rel;
+    const u32 chunks = chunk0[p + 1] - chunk0[p];
+    if(i0 < children) first_children(chunk_first + chunk0[p], chunks, LOCAL_CHUNK, rel, rel + a, p * children + i0 + 1);
+    if(i1 < children) first_children(chunk_first + chunk0[p], chunks, LOCAL_CHUNK, rel + a, rel + a + b, p * children + i1 + 1);
+    if(t == 0 && chunks) chunk_first[chunk0[p]] = p * children;
     if(i0 < children) { c[i0] = off; child_off[u64(p) * children + i0] = off; }
     if(i1 < children) { c[i1] = off + a; child_off[u64(p) * children + i1] = off + a; }
-    if(p == parents - 1 && t == 0) child_off[u64(parents) * children] = par_off[parents];
+    if(p == parents - 1 && t == 0) { child_off[u64(parents) * children] = par_off[parents]; chunk_first[chunk0[parents]] = parents * children; }
 }
 
 constexpr size_t SPLIT_SMEM = size_t(SPLIT_TILE) * 8;
@@ -544,54 +598,42 @@ constexpr size_t LOCAL_SMEM = size_t(LOCAL_CAP) * 8 + (LOCAL_CAP / 2 + 4) * 4 + 
 constexpr u32 LONG_BIN = 256;       // a bin with more records is not ordered by comparing all with all
 static_assert(LOCAL_CAP <= 8192, "slots of a batch take 13 bits");
 
-// Appends the records whose bit is set in `mask` (by their place in the sorted batch) to a list; returns, for the caller's
-// records, where the flagged records before word w begin (pre[w]) and the list position of the first (at). Every thread calls it.
-// pre: LOCAL_CAP / 32 words; slot: one word of shared memory.
-__device__ __forceinline__ u32 list_places(const u32* mask, u32* pre, u32* warp_tot, u32* slot, u32* count)
+// A record's place in its batch (13 bits), then the first place of its group or, where that is its own, the group's size (14 bits)
+// and FIRST; SMALL or LARGE by the group's size, neither for a record that is alone.
+constexpr u32 PL_SMALL = 1u << 27, PL_LARGE = 1u << 28, PL_FIRST = 1u << 29;
+__device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, const u32 size)
 {
-    static_assert(LOCAL_CAP / 32 <= LOCAL_BLOCK, "a thread per word");
-    const u32 c = threadIdx.x < LOCAL_CAP / 32 ? __popc(mask[threadIdx.x]) : 0;
-    u32 total;
-    const u32 before = block_exclusive<LOCAL_BLOCK>(c, warp_tot, total);
-    if(threadIdx.x < LOCAL_CAP / 32) pre[threadIdx.x] = before;
-    if(threadIdx.x == 0) *slot = total ? atomicAdd(count, total) : 0;
-    __syncthreads();
-    return *slot;
+    return place | (place == head ? size << 13 | PL_FIRST : head << 13) | (size == 1 ? 0u : (size <= SMALL_GROUP ? PL_SMALL : PL_LARGE));
 }
 
-__global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ chunk0,
-                                                                   const u32 parents, const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa,
-                                                                   u64* __restrict__ list, const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over)
+// What bounds it is latency and the issue of instructions, not memory (12 bytes a record at 0.8 TB/s): two blocks of 16 warps an SM
+// go through barriers between dependent steps. So a block finds its children in two dependent reads (chunk_first, child_off),
+// and tied records get their list places from one counter in shared memory.
+__global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
+                                                                   const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u64* __restrict__ list,
+                                                                   const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);                            // [LOCAL_CAP]
     u32* const bin = reinterpret_cast<u32*>(stage + LOCAL_CAP);                      // [LOCAL_CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
     u16* const start = reinterpret_cast<u16*>(bin);
-    u32* const coff = bin + LOCAL_CAP / 2 + 4;                                       // [children + 1] offsets of the parent's children
-    __shared__ u32 mask_small[LOCAL_CAP / 32], mask_large[LOCAL_CAP / 32], pre[LOCAL_CAP / 32];
+    u32* const coff = bin + LOCAL_CAP / 2 + 4;                                       // [children of the chunk + 1] their offsets
     __shared__ u32 warp_tot[LOCAL_BLOCK / 32];
-    __shared__ u32 found, s_first, s_last, s_slot;
+    __shared__ u32 s_tied[2], s_slot[2];            // records of small and of large groups in the batch, and their places in the list
     const u32 tid = threadIdx.x;
     const u32 children = 1u << bits;
     const int rbits = 32 - bits;                    // key bits behind the child's
     const u32 rmask = rbits == 32 ? 0xFFFFFFFFu : (1u << rbits) - 1;
 
-    const u32 p = parent_of_block(chunk0, parents, blockIdx.x, &found);
-    if(p >= parents) return;
-    const u32 par_end = par_off[p + 1];
-    const u32 lo = par_off[p] + (blockIdx.x - chunk0[p]) * LOCAL_CHUNK;
-    const u32 hi = par_end - lo < LOCAL_CHUNK ? par_end : lo + LOCAL_CHUNK;
-    for(u32 d = tid; d <= children; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + u64(p) * children + d);
+    if(blockIdx.x >= *chunks) return;
+    // the block's children: at most all of one parent
+    const u32 child0 = __ldg(chunk_first + blockIdx.x);
+    const u32 last = min(__ldg(chunk_first + blockIdx.x + 1), ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
+    const u32 first_digit = child0 & (children - 1);
+    for(u32 d = tid; d <= last; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + child0 + d);
+    if(tid < 2) s_tied[tid] = 0;
     __syncthreads();
-    // the children that start in [lo, hi)
-    for(u32 d = tid; d <= children; d += LOCAL_BLOCK)
-    {
-        if(coff[d] >= lo && (d == 0 || coff[d - 1] < lo)) s_first = d;
-        if((coff[d] >= hi || d == children) && (d == 0 || coff[d - 1] < hi)) s_last = d;
-    }
-    __syncthreads();
-    u32 cur = s_first;
-    const u32 last = s_last;
+    u32 cur = 0;
 
     while(cur < last)
     {
@@ -612,7 +654,7 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
                 // a child that does not fit: left to the radix sort
                 if(tid == 0)
                 {
-                    over[atomicAdd(&counts->oversize, 1u)] = p * children + cur;
+                    over[atomicAdd(&counts->oversize, 1u)] = child0 + cur;
                     atomicAdd(&counts->oversize_records, coff[cur + 1] - base);
                 }
                 ++cur;
@@ -624,31 +666,34 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
         if(m == 0) continue;
 
         // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
-        for(u32 i = tid; i < m / 2 + 2; i += LOCAL_BLOCK) bin[i] = 0;
-        for(u32 i = tid; i < LOCAL_CAP / 32; i += LOCAL_BLOCK) { mask_small[i] = 0; mask_large[i] = 0; }
+        for(u32 i = tid; i < ((m + 1) / 2 + 7) / 8 * 2; i += LOCAL_BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
         u64 r[LOCAL_ITEMS];
         u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later place | head << 13 | tied << 26
         #pragma unroll
         for(int i = 0; i < LOCAL_ITEMS; ++i)
         {
+            if(i * LOCAL_BLOCK >= m) break;          // of all threads: half of a full batch is the rule
             const u32 j = tid + i * LOCAL_BLOCK;
             if(j < m) r[i] = rec[base + j];
         }
         __syncthreads();
         auto bin_of = [&](const u32 key) -> u32
         {
-            const u32 d = bits ? key >> rbits : 0u;
+            const u32 d = (bits ? key >> rbits : 0u) - first_digit;
             const u32 c0 = coff[d];
             return c0 - base + u32((u64(key & rmask) * (coff[d + 1] - c0)) >> rbits);
         };
         #pragma unroll
         for(int i = 0; i < LOCAL_ITEMS; ++i)
+        {
+            if(i * LOCAL_BLOCK >= m) break;
             if(tid + i * LOCAL_BLOCK < m)
             {
                 const u32 b = bin_of(u32(r[i] >> 32));
                 const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
                 pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
             }
+        }
         __syncthreads();
         // exclusive sums of the bins' counts, in place; start[m] = m
         u32 longest = 0;
@@ -656,22 +701,34 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
             constexpr int WORDS = LOCAL_CAP / 2 / LOCAL_BLOCK;      // 8 words, 16 bins a thread
             u32 c[WORDS], sum = 0;
             const u32 w0 = tid * WORDS;
-            #pragma unroll
-            for(int k = 0; k < WORDS; ++k)
+            const bool any = 2 * w0 < m;            // the words up to a multiple of WORDS were cleared
+            if(any)
             {
-                c[k] = 2 * (w0 + k) < m ? bin[w0 + k] : 0;
-                const u32 a = c[k] & 0xFFFFu, b = c[k] >> 16;
-                sum += a + b;
-                longest = max(longest, max(a, b));
+                #pragma unroll
+                for(int k = 0; k < WORDS / 4; ++k)
+                {
+                    const uint4 v = reinterpret_cast<const uint4*>(bin)[tid * (WORDS / 4) + k];
+                    c[4 * k] = v.x; c[4 * k + 1] = v.y; c[4 * k + 2] = v.z; c[4 * k + 3] = v.w;
+                }
+                u32 both = 0;           // two sums side by side: below 2^16 each
+                #pragma unroll
+                for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16)); }
+                sum = (both & 0xFFFFu) + (both >> 16);
             }
             u32 total;
             u32 run = block_exclusive<LOCAL_BLOCK>(sum, warp_tot, total);
-            #pragma unroll
-            for(int k = 0; k < WORDS; ++k)
+            if(any)
             {
-                const u32 a = run, b = run + (c[k] & 0xFFFFu);
-                run = b + (c[k] >> 16);
-                if(2 * (w0 + k) < m) bin[w0 + k] = a | (b << 16);
+                #pragma unroll
+                for(int k = 0; k < WORDS; ++k)
+                {
+                    const u32 a = run, b = run + (c[k] & 0xFFFFu);
+                    run = b + (c[k] >> 16);
+                    c[k] = a | (b << 16);
+                }
+                #pragma unroll
+                for(int k = 0; k < WORDS / 4; ++k)
+                    reinterpret_cast<uint4*>(bin)[tid * (WORDS / 4) + k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
             }
             __syncthreads();
             if(tid == 0) start[m] = u16(m);
@@ -679,7 +736,10 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
         const bool by_network = __syncthreads_or(longest > LONG_BIN);
         #pragma unroll
         for(int i = 0; i < LOCAL_ITEMS; ++i)
+        {
+            if(i * LOCAL_BLOCK >= m) break;
             if(tid + i * LOCAL_BLOCK < m) stage[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = r[i];
+        }
         __syncthreads();
 
         if(!by_network)
@@ -704,7 +764,7 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
                     eq_before += same && k < j;
                 }
                 const u32 place = s + less + eq_before;
-                pl[i] = place | ((s + less) << 13) | (eq == 1 ? 0u : (eq <= SMALL_GROUP ? 1u << 26 : 2u << 26));
+                pl[i] = packed_place(place, s + less, eq);
                 sa[base + place] = eq == 1 ? u32(v) : SA_OPEN;
             }
         }
@@ -739,39 +799,40 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
                 u32 c = j + 1, f = m;               // first record behind with a greater key
                 while(c < f) { const u32 mid = (c + f) >> 1; if(u32(stage[mid] >> 32) <= key) c = mid + 1; else f = mid; }
                 const u32 eq = c - a;
-                pl[i] = j | (a << 13) | (eq == 1 ? 0u : (eq <= SMALL_GROUP ? 1u << 26 : 2u << 26));
+                pl[i] = packed_place(j, a, eq);
                 sa[base + j] = eq == 1 ? u32(v) : SA_OPEN;
             }
         }
+        // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
         u32 tied = 0;
         #pragma unroll
         for(int i = 0; i < LOCAL_ITEMS; ++i)
         {
-            if(tid + i * LOCAL_BLOCK >= m) break;
-            const u32 kind = pl[i] >> 26, place = pl[i] & 8191u;
-            tied |= kind;
-            if(kind == 1) atomicOr(&mask_small[place >> 5], 1u << (place & 31));
-            else if(kind == 2) atomicOr(&mask_large[place >> 5], 1u << (place & 31));
+            if(i * LOCAL_BLOCK >= m) break;
+            if(tid + i * LOCAL_BLOCK < m) tied |= (pl[i] & (PL_SMALL | PL_LARGE)) ? 1u << i : 0u;
         }
-        // The tied records go to the list in the order of their places, so that a group's records lie side by side.
-        for(u32 kind = 1; kind <= 2; ++kind)
+        if(__syncthreads_or(tied != 0))
         {
-            if(!__syncthreads_or((tied & kind) != 0)) continue;
-            u32* const mask = kind == 1 ? mask_small : mask_large;
-            const u32 at = list_places(mask, pre, warp_tot, &s_slot, kind == 1 ? &counts->small : &counts->large);
             #pragma unroll
             for(int i = 0; i < LOCAL_ITEMS; ++i)
+                if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
+            __syncthreads();
+            if(tid < 2)
             {
-                const u32 j = tid + i * LOCAL_BLOCK;
-                if(j >= m) break;
-                if((pl[i] >> 26) == kind)
-                {
-                    const u32 place = pl[i] & 8191u;
-                    const u64 k = u64(at) + pre[place >> 5] + __popc(mask[place >> 5] & ((1u << (place & 31)) - 1));
-                    list[kind == 1 ? k : list_cap - 1 - k] = (u64(base + ((pl[i] >> 13) & 8191u)) << 32) | u32(stage[j]);
-                }
+                const u32 c = s_tied[tid];
+                s_slot[tid] = c ? atomicAdd(tid ? &counts->large : &counts->small, c) : 0;
+                s_tied[tid] = 0;
             }
             __syncthreads();
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+                if(tied >> i & 1u)
+                {
+                    const u32 place = pl[i] & 8191u, head = (pl[i] & PL_FIRST) ? place : pl[i] >> 13 & 8191u;
+                    const bool small = (pl[i] & PL_SMALL) != 0;
+                    const u64 k = u64(s_slot[small ? 0 : 1]) + start[head] + (place - head);
+                    list[small ? k : list_cap - 1 - k] = (u64(base + head) << 32) | u32(stage[tid + i * LOCAL_BLOCK]);
+                }
         }
         __syncthreads();        // the next batch reuses the shared arrays
     }
@@ -812,17 +873,6 @@ int shared_bytes(csa_ctx* ctx, K kern, size_t bytes, std::atomic<bool>* configur
     return CSA_OK;
 }
 
-template <int BLOCK>
-int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, u32* counts)
-{
-    static std::atomic<bool> configured[64];
-    constexpr size_t smem = (STREAM_WORDS<BLOCK> + (1 << MAX_B1)) * 4;
-    CSA_TRY(shared_bytes(ctx, count_text_kernel<BLOCK>, smem, configured));
-    count_text_kernel<BLOCK><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, smem, ctx->stream>>>(T, n, code, bits, counts);
-    CSA_LAUNCH_CHECK(ctx);
-    return CSA_OK;
-}
-
 template <int BLOCK, bool PART>
 int launch_scatter_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, int keep_top, u32 first_bin, u32 part_bins, u32* cursor, u64* out)
 {
@@ -855,7 +905,7 @@ Prefix_Sort prefix_sort_plan(u64 n)
 size_t prefix_sort_table_bytes(const Prefix_Sort& ps)
 {
     const u64 all = u64(ps.parents) * ps.children;
-    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + 4096;
+    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + align_up256((ps.n / SHORT_CHUNK + (size_t(1) << MAX_B1) + 2) * 4) + 4096;
 }
 
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
@@ -871,6 +921,7 @@ bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
     t.cnt2 = cv.take<u32>(all);
     t.child_off = cv.take<u32>(all + 1);
     t.over = cv.take<u32>(all);
+    t.chunk_first = cv.take<u32>(ps.n / SHORT_CHUNK + (u64(1) << MAX_B1) + 2);
     return cv.ok;
 }
 
@@ -909,7 +960,15 @@ int launch_code(csa_ctx* ctx, const Prefix_Tables& t, const u16* T, const u64 n,
 
 int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bits, u32* counts)
 {
-    return wide_tiles(n) ? launch_count_text<512>(ctx, T, n, code, bits, counts) : launch_count_text<128>(ctx, T, n, code, bits, counts);
+    if(wide_tiles(n))
+    {
+        static std::atomic<bool> configured[64];
+        CSA_TRY(shared_bytes(ctx, count_long_text_kernel, COUNT_SMEM, configured));
+        count_long_text_kernel<<<148, COUNT_BLOCK, COUNT_SMEM, ctx->stream>>>(T, n, code, bits, counts);
+    }
+    else count_text_kernel<128><<<unsigned(div_up(n, TILE_POSITIONS<128>)), 128, 0, ctx->stream>>>(T, n, code, bits, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
 }
 
 // The second split of `parents` buckets with n records in all (recA to recB).
@@ -920,7 +979,7 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
     CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(parents) * children * 4, ctx->stream));
     count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2);
     CSA_LAUNCH_CHECK(ctx);
-    child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off);
+    child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off, t.chunk0, t.chunk_first);
     CSA_LAUNCH_CHECK(ctx);
     static std::atomic<bool> configured[64];
     CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
@@ -929,11 +988,11 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
     return CSA_OK;
 }
 
-int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
+int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u32 chunk, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
 {
     static std::atomic<bool> configured[64];
     CSA_TRY(shared_bytes(ctx, local_sort_kernel, LOCAL_SMEM, configured));
-    local_sort_kernel<<<unsigned(n / LOCAL_CHUNK + parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.par_off, t.chunk0, parents, b2, t.child_off, sa, list, n, counts, t.over);
+    local_sort_kernel<<<unsigned(n / chunk + parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.chunk_first, t.chunk0 + parents, b2, t.child_off, sa, list, n, counts, t.over);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -948,7 +1007,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     const bool one_level = ps.b1 == 0;
     const int bits = one_level ? ps.b2 : ps.b1;
     if(bits > 0) CSA_TRY(launch_count_text(ctx, T, n, t.code, bits, t.cnt1));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, p, counts);
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, p, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(n) ? (launch_scatter_text<512, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA))
                           : (launch_scatter_text<128, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA)));
@@ -962,7 +1021,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
         CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB));
         rec = recB; other = recA;
     }
-    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, n, rec, sa, other, counts));
+    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, one_level ? SHORT_CHUNK : LOCAL_CHUNK, n, rec, sa, other, counts));
     *list = other;
     *records = rec;
     return CSA_OK;
@@ -990,12 +1049,12 @@ int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Ta
                             Build_Counts* counts)
 {
     CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, 1, counts);
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, 1, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
                              : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));
     CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB));
-    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, size, recB, sa, recA, counts));
+    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, LOCAL_CHUNK, size, recB, sa, recA, counts));
     ctx->counters[1] += 2;
     ctx->counters[2] += 2 * size;
     return CSA_OK;

@@ -49,6 +49,7 @@ struct Prefix_Tables
     u32* chunk0;        // [parents + 1] first chunk of each parent in the local sort
     u32* cnt2;          // [parents][children] records by second digit, then running places
     u32* child_off;     // [parents * children + 1] where each child starts in the suffix array
+    u32* chunk_first;   // first child of every chunk of the local sort (parent * children + child), and the end
     u32* over;          // children that did not fit a block: their indices
 };
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t);
