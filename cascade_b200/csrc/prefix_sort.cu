@@ -28,10 +28,10 @@ constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of
 constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
-constexpr int LOCAL_BLOCK = 512, LOCAL_ITEMS = 16, LOCAL_CAP = LOCAL_BLOCK * LOCAL_ITEMS;
-// Children that start inside one chunk of slots belong to one block: two children as a rule, or one in a short text (one split, up
-// to 2^21 suffixes), where every SM should get a block.
-constexpr u32 LOCAL_CHUNK = LOCAL_CAP / 2, SHORT_CHUNK = LOCAL_CAP / 8;
+constexpr int LOCAL_ITEMS = 16;
+template <int BLOCK> constexpr int LOCAL_CAP = BLOCK * LOCAL_ITEMS;     // records that a block of the local sort holds
+// Children that start inside one chunk of slots belong to one block: one child as a rule.
+constexpr u32 LOCAL_CHUNK = 2048, SHORT_CHUNK = 1024;
 
 // ---- the code ----------------------------------------------------------------------------------------------------------------
 
@@ -102,7 +102,7 @@ __device__ __forceinline__ u32 block_exclusive(const u32 v, u32* warp_tot, u32& 
 }
 
 // Weights and code words in one launch. Every block holds the prefix sums of all 65536 weights in shared memory, 24 bits each (16
-// and 8 apart), and gives CODE_BLOCK symbols their words; the weights are scale * count + 1 (every symbol must have a code word:
+// and 8 apart), and gives CODE_WALKERS symbols their words; the weights are scale * count + 1 (every symbol must have a code word:
 // the sample may have missed it), below 2^23 together. COUNT: the text is short, and every block counts its symbols by itself.
 //
 // One symbol per thread walks down the tree: a node is a range of symbols, split where the weights of its halves come closest,
@@ -110,6 +110,7 @@ __device__ __forceinline__ u32 block_exclusive(const u32 v, u32* warp_tot, u32& 
 // is one chain of some 150 dependent reads, which is why the sums lie in shared memory: with the sums made by one block and read
 // through L2, the two launches took 98 us of a short build's 190.
 constexpr int CODE_BLOCK = 1024;
+constexpr u32 CODE_WALKERS = 512;               // threads of a block that walk: more warps would wait for shared memory, not for its latency
 constexpr u64 CODE_COUNT_MAX = 1 << 14;         // longest text that every block counts by itself (16-bit counters)
 constexpr u32 CODE_LOW_BYTES = (65536 + 8) * 2;
 constexpr size_t CODE_SMEM = CODE_LOW_BYTES + 65536 + 8;
@@ -180,7 +181,8 @@ __global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __rest
     __syncthreads();
     auto prefix = [&](const u32 m) { return u32(low[m]) | u32(high[m]) << 16; };
 
-    const u32 s = blockIdx.x * CODE_BLOCK + tid;
+    if(tid >= CODE_WALKERS) return;
+    const u32 s = blockIdx.x * CODE_WALKERS + tid;
     u32 lo = 0, hi = 65536, word = 0;
     int left = CODE_MAX_LEN;            // bits left below the node
     u32 plo = 0, phi = prefix(65536);
@@ -594,9 +596,9 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
 
 // ---- local sort: runs of children in shared memory --------------------------------------------------------------------------------
 
-constexpr size_t LOCAL_SMEM = size_t(LOCAL_CAP) * 8 + (LOCAL_CAP / 2 + 4) * 4 + ((1 << MAX_B2) + 4) * 4;
+template <int BLOCK> constexpr size_t LOCAL_SMEM = size_t(LOCAL_CAP<BLOCK>) * 8 + (LOCAL_CAP<BLOCK> / 2 + 4) * 4 + ((1 << MAX_B2) + 4) * 4;
 constexpr u32 LONG_BIN = 256;       // a bin with more records is not ordered by comparing all with all
-static_assert(LOCAL_CAP <= 8192, "slots of a batch take 13 bits");
+static_assert(LOCAL_CAP<512> <= 8192, "slots of a batch take 13 bits");
 
 // A record's place in its batch (13 bits), then the first place of its group or, where that is its own, the group's size (14 bits)
 // and FIRST; SMALL or LARGE by the group's size, neither for a record that is alone.
@@ -606,13 +608,19 @@ __device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, con
     return place | (place == head ? size << 13 | PL_FIRST : head << 13) | (size == 1 ? 0u : (size <= SMALL_GROUP ? PL_SMALL : PL_LARGE));
 }
 
-// What bounds it is latency and the issue of instructions, not memory (12 bytes a record at 0.8 TB/s): two blocks of 16 warps an SM
-// go through barriers between dependent steps. So a block finds its children in two dependent reads (chunk_first, child_off),
-// and tied records get their list places from one counter in shared memory.
-__global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
+// What bounds it is latency and the issue of instructions, not memory (12 bytes a record at 0.9 TB/s): a block goes through
+// barriers between dependent steps. So a block finds its children in two dependent reads (chunk_first, child_off), tied records get
+// their list places from one counter in shared memory, and four small blocks share an SM (two of 512 threads: 27.7 ms at 2e9
+// records, four of 256: 24.5 ms, and 0.5 ms for the children that need the larger ones).
+// MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
+// there if a block of 512 threads holds them, and to the front, for the radix sort, if not.
+constexpr u32 MEDIUM_CAP = LOCAL_CAP<512>;
+template <int BLOCK, bool MEDIUM>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
                                                                    const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u64* __restrict__ list,
-                                                                   const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over)
+                                                                   const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap)
 {
+    constexpr int LOCAL_BLOCK = BLOCK, LOCAL_CAP = BLOCK * LOCAL_ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);                            // [LOCAL_CAP]
     u32* const bin = reinterpret_cast<u32*>(stage + LOCAL_CAP);                      // [LOCAL_CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
@@ -625,216 +633,223 @@ __global__ void __launch_bounds__(LOCAL_BLOCK, 2) local_sort_kernel(const u64* _
     const int rbits = 32 - bits;                    // key bits behind the child's
     const u32 rmask = rbits == 32 ? 0xFFFFFFFFu : (1u << rbits) - 1;
 
-    if(blockIdx.x >= *chunks) return;
-    // the block's children: at most all of one parent
-    const u32 child0 = __ldg(chunk_first + blockIdx.x);
-    const u32 last = min(__ldg(chunk_first + blockIdx.x + 1), ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
-    const u32 first_digit = child0 & (children - 1);
-    for(u32 d = tid; d <= last; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + child0 + d);
-    if(tid < 2) s_tied[tid] = 0;
-    __syncthreads();
-    u32 cur = 0;
-
-    while(cur < last)
+    const u32 works = MEDIUM ? counts->medium : *chunks;
+    for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
-        // a batch: as many children as fit
-        u32 e = last;
-        const u32 base = coff[cur];
-        if(coff[e] - base > u32(LOCAL_CAP))
-        {
-            u32 a = cur, b = last;                  // the last e with coff[e] - base <= LOCAL_CAP
-            while(b - a > 1)
-            {
-                const u32 m = (a + b) >> 1;
-                if(coff[m] - base <= u32(LOCAL_CAP)) a = m; else b = m;
-            }
-            e = a;
-            if(e == cur)
-            {
-                // a child that does not fit: left to the radix sort
-                if(tid == 0)
-                {
-                    over[atomicAdd(&counts->oversize, 1u)] = child0 + cur;
-                    atomicAdd(&counts->oversize_records, coff[cur + 1] - base);
-                }
-                ++cur;
-                continue;
-            }
-        }
-        const u32 m = coff[e] - base;
-        cur = e;
-        if(m == 0) continue;
+        // the block's children: at most all of one parent
+        const u32 child0 = MEDIUM ? over[over_cap - 1 - work] : __ldg(chunk_first + work);
+        const u32 last = MEDIUM ? 1u : min(__ldg(chunk_first + work + 1), ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
+        const u32 first_digit = child0 & (children - 1);
+        for(u32 d = tid; d <= last; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + child0 + d);
+        if(tid < 2) s_tied[tid] = 0;
+        __syncthreads();
+        u32 cur = 0;
 
-        // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
-        for(u32 i = tid; i < ((m + 1) / 2 + 7) / 8 * 2; i += LOCAL_BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
-        u64 r[LOCAL_ITEMS];
-        u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later place | head << 13 | tied << 26
-        #pragma unroll
-        for(int i = 0; i < LOCAL_ITEMS; ++i)
+        while(cur < last)
         {
-            if(i * LOCAL_BLOCK >= m) break;          // of all threads: half of a full batch is the rule
-            const u32 j = tid + i * LOCAL_BLOCK;
-            if(j < m) r[i] = rec[base + j];
-        }
-        __syncthreads();
-        auto bin_of = [&](const u32 key) -> u32
-        {
-            const u32 d = (bits ? key >> rbits : 0u) - first_digit;
-            const u32 c0 = coff[d];
-            return c0 - base + u32((u64(key & rmask) * (coff[d + 1] - c0)) >> rbits);
-        };
-        #pragma unroll
-        for(int i = 0; i < LOCAL_ITEMS; ++i)
-        {
-            if(i * LOCAL_BLOCK >= m) break;
-            if(tid + i * LOCAL_BLOCK < m)
+            // a batch: as many children as fit
+            u32 e = last;
+            const u32 base = coff[cur];
+            if(coff[e] - base > u32(LOCAL_CAP))
             {
-                const u32 b = bin_of(u32(r[i] >> 32));
-                const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
-                pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
-            }
-        }
-        __syncthreads();
-        // exclusive sums of the bins' counts, in place; start[m] = m
-        u32 longest = 0;
-        {
-            constexpr int WORDS = LOCAL_CAP / 2 / LOCAL_BLOCK;      // 8 words, 16 bins a thread
-            u32 c[WORDS], sum = 0;
-            const u32 w0 = tid * WORDS;
-            const bool any = 2 * w0 < m;            // the words up to a multiple of WORDS were cleared
-            if(any)
-            {
-                #pragma unroll
-                for(int k = 0; k < WORDS / 4; ++k)
+                u32 a = cur, b = last;                  // the last e with coff[e] - base <= LOCAL_CAP
+                while(b - a > 1)
                 {
-                    const uint4 v = reinterpret_cast<const uint4*>(bin)[tid * (WORDS / 4) + k];
-                    c[4 * k] = v.x; c[4 * k + 1] = v.y; c[4 * k + 2] = v.z; c[4 * k + 3] = v.w;
+                    const u32 m = (a + b) >> 1;
+                    if(coff[m] - base <= u32(LOCAL_CAP)) a = m; else b = m;
                 }
-                u32 both = 0;           // two sums side by side: below 2^16 each
-                #pragma unroll
-                for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16)); }
-                sum = (both & 0xFFFFu) + (both >> 16);
-            }
-            u32 total;
-            u32 run = block_exclusive<LOCAL_BLOCK>(sum, warp_tot, total);
-            if(any)
-            {
-                #pragma unroll
-                for(int k = 0; k < WORDS; ++k)
+                e = a;
+                if(e == cur)
                 {
-                    const u32 a = run, b = run + (c[k] & 0xFFFFu);
-                    run = b + (c[k] >> 16);
-                    c[k] = a | (b << 16);
-                }
-                #pragma unroll
-                for(int k = 0; k < WORDS / 4; ++k)
-                    reinterpret_cast<uint4*>(bin)[tid * (WORDS / 4) + k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
-            }
-            __syncthreads();
-            if(tid == 0) start[m] = u16(m);
-        }
-        const bool by_network = __syncthreads_or(longest > LONG_BIN);
-        #pragma unroll
-        for(int i = 0; i < LOCAL_ITEMS; ++i)
-        {
-            if(i * LOCAL_BLOCK >= m) break;
-            if(tid + i * LOCAL_BLOCK < m) stage[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = r[i];
-        }
-        __syncthreads();
-
-        if(!by_network)
-        {
-            // Order inside the bins: a record counts the smaller and the equal keys of its bin.
-            #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
-            {
-                const u32 j = tid + i * LOCAL_BLOCK;
-                if(j >= m) break;
-                const u64 v = stage[j];
-                const u32 key = u32(v >> 32);
-                const u32 b = bin_of(key);
-                const u32 s = start[b], t = start[b + 1];
-                u32 less = 0, eq_before = 0, eq = 0;
-                for(u32 k = s; k < t; ++k)
-                {
-                    const u32 o = u32(stage[k] >> 32);
-                    less += o < key;
-                    const u32 same = o == key;
-                    eq += same;
-                    eq_before += same && k < j;
-                }
-                const u32 place = s + less + eq_before;
-                pl[i] = packed_place(place, s + less, eq);
-                sa[base + place] = eq == 1 ? u32(v) : SA_OPEN;
-            }
-        }
-        else
-        {
-            // Many records in one bin: a sorting network over the batch (keys and positions), then every record finds its
-            // group's ends by bisection.
-            u32 size = 1;
-            while(size < m) size <<= 1;
-            for(u32 j = m + tid; j < size; j += LOCAL_BLOCK) stage[j] = ~0ull;
-            __syncthreads();
-            for(u32 k = 2; k <= size; k <<= 1)
-                for(u32 d = k >> 1; d > 0; d >>= 1)
-                {
-                    for(u32 t = tid; t < size / 2; t += LOCAL_BLOCK)
+                    // a child that does not fit: left to the radix sort
+                    if(tid == 0)
                     {
-                        const u32 a = 2 * t - (t & (d - 1)), b = a + d;
-                        const u64 x = stage[a], y = stage[b];
-                        if((x > y) == ((a & k) == 0)) { stage[a] = y; stage[b] = x; }
+                        if(!MEDIUM && coff[cur + 1] - base <= MEDIUM_CAP) over[over_cap - 1 - atomicAdd(&counts->medium, 1u)] = child0 + cur;
+                        else
+                        {
+                            over[atomicAdd(&counts->oversize, 1u)] = child0 + cur;
+                            atomicAdd(&counts->oversize_records, coff[cur + 1] - base);
+                        }
                     }
-                    __syncthreads();
+                    ++cur;
+                    continue;
                 }
+            }
+            const u32 m = coff[e] - base;
+            cur = e;
+            if(m == 0) continue;
+
+            // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
+            for(u32 i = tid; i < ((m + 1) / 2 + 7) / 8 * 2; i += LOCAL_BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+            u64 r[LOCAL_ITEMS];
+            u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later place | head << 13 | tied << 26
             #pragma unroll
             for(int i = 0; i < LOCAL_ITEMS; ++i)
             {
+                if(i * LOCAL_BLOCK >= m) break;          // of all threads: half of a full batch is the rule
                 const u32 j = tid + i * LOCAL_BLOCK;
-                if(j >= m) break;
-                const u64 v = stage[j];
-                const u32 key = u32(v >> 32);
-                u32 a = 0, b = j;                   // first record with this key
-                while(a < b) { const u32 mid = (a + b) >> 1; if(u32(stage[mid] >> 32) < key) a = mid + 1; else b = mid; }
-                u32 c = j + 1, f = m;               // first record behind with a greater key
-                while(c < f) { const u32 mid = (c + f) >> 1; if(u32(stage[mid] >> 32) <= key) c = mid + 1; else f = mid; }
-                const u32 eq = c - a;
-                pl[i] = packed_place(j, a, eq);
-                sa[base + j] = eq == 1 ? u32(v) : SA_OPEN;
+                if(j < m) r[i] = rec[base + j];
             }
-        }
-        // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
-        u32 tied = 0;
-        #pragma unroll
-        for(int i = 0; i < LOCAL_ITEMS; ++i)
-        {
-            if(i * LOCAL_BLOCK >= m) break;
-            if(tid + i * LOCAL_BLOCK < m) tied |= (pl[i] & (PL_SMALL | PL_LARGE)) ? 1u << i : 0u;
-        }
-        if(__syncthreads_or(tied != 0))
-        {
-            #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
-                if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
             __syncthreads();
-            if(tid < 2)
+            auto bin_of = [&](const u32 key) -> u32
             {
-                const u32 c = s_tied[tid];
-                s_slot[tid] = c ? atomicAdd(tid ? &counts->large : &counts->small, c) : 0;
-                s_tied[tid] = 0;
-            }
-            __syncthreads();
+                const u32 d = (bits ? key >> rbits : 0u) - first_digit;
+                const u32 c0 = coff[d];
+                return c0 - base + u32((u64(key & rmask) * (coff[d + 1] - c0)) >> rbits);
+            };
             #pragma unroll
             for(int i = 0; i < LOCAL_ITEMS; ++i)
-                if(tied >> i & 1u)
+            {
+                if(i * LOCAL_BLOCK >= m) break;
+                if(tid + i * LOCAL_BLOCK < m)
                 {
-                    const u32 place = pl[i] & 8191u, head = (pl[i] & PL_FIRST) ? place : pl[i] >> 13 & 8191u;
-                    const bool small = (pl[i] & PL_SMALL) != 0;
-                    const u64 k = u64(s_slot[small ? 0 : 1]) + start[head] + (place - head);
-                    list[small ? k : list_cap - 1 - k] = (u64(base + head) << 32) | u32(stage[tid + i * LOCAL_BLOCK]);
+                    const u32 b = bin_of(u32(r[i] >> 32));
+                    const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
+                    pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
                 }
+            }
+            __syncthreads();
+            // exclusive sums of the bins' counts, in place; start[m] = m
+            u32 longest = 0;
+            {
+                constexpr int WORDS = LOCAL_CAP / 2 / LOCAL_BLOCK;      // 8 words, 16 bins a thread
+                u32 c[WORDS], sum = 0;
+                const u32 w0 = tid * WORDS;
+                const bool any = 2 * w0 < m;            // the words up to a multiple of WORDS were cleared
+                if(any)
+                {
+                    #pragma unroll
+                    for(int k = 0; k < WORDS / 4; ++k)
+                    {
+                        const uint4 v = reinterpret_cast<const uint4*>(bin)[tid * (WORDS / 4) + k];
+                        c[4 * k] = v.x; c[4 * k + 1] = v.y; c[4 * k + 2] = v.z; c[4 * k + 3] = v.w;
+                    }
+                    u32 both = 0;           // two sums side by side: below 2^16 each
+                    #pragma unroll
+                    for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16)); }
+                    sum = (both & 0xFFFFu) + (both >> 16);
+                }
+                u32 total;
+                u32 run = block_exclusive<LOCAL_BLOCK>(sum, warp_tot, total);
+                if(any)
+                {
+                    #pragma unroll
+                    for(int k = 0; k < WORDS; ++k)
+                    {
+                        const u32 a = run, b = run + (c[k] & 0xFFFFu);
+                        run = b + (c[k] >> 16);
+                        c[k] = a | (b << 16);
+                    }
+                    #pragma unroll
+                    for(int k = 0; k < WORDS / 4; ++k)
+                        reinterpret_cast<uint4*>(bin)[tid * (WORDS / 4) + k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
+                }
+                __syncthreads();
+                if(tid == 0) start[m] = u16(m);
+            }
+            const bool by_network = __syncthreads_or(longest > LONG_BIN);
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            {
+                if(i * LOCAL_BLOCK >= m) break;
+                if(tid + i * LOCAL_BLOCK < m) stage[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = r[i];
+            }
+            __syncthreads();
+
+            if(!by_network)
+            {
+                // Order inside the bins: a record counts the smaller and the equal keys of its bin.
+                #pragma unroll
+                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                {
+                    const u32 j = tid + i * LOCAL_BLOCK;
+                    if(j >= m) break;
+                    const u64 v = stage[j];
+                    const u32 key = u32(v >> 32);
+                    const u32 b = bin_of(key);
+                    const u32 s = start[b], t = start[b + 1];
+                    u32 less = 0, eq_before = 0, eq = 0;
+                    for(u32 k = s; k < t; ++k)
+                    {
+                        const u32 o = u32(stage[k] >> 32);
+                        less += o < key;
+                        const u32 same = o == key;
+                        eq += same;
+                        eq_before += same && k < j;
+                    }
+                    const u32 place = s + less + eq_before;
+                    pl[i] = packed_place(place, s + less, eq);
+                    sa[base + place] = eq == 1 ? u32(v) : SA_OPEN;
+                }
+            }
+            else
+            {
+                // Many records in one bin: a sorting network over the batch (keys and positions), then every record finds its
+                // group's ends by bisection.
+                u32 size = 1;
+                while(size < m) size <<= 1;
+                for(u32 j = m + tid; j < size; j += LOCAL_BLOCK) stage[j] = ~0ull;
+                __syncthreads();
+                for(u32 k = 2; k <= size; k <<= 1)
+                    for(u32 d = k >> 1; d > 0; d >>= 1)
+                    {
+                        for(u32 t = tid; t < size / 2; t += LOCAL_BLOCK)
+                        {
+                            const u32 a = 2 * t - (t & (d - 1)), b = a + d;
+                            const u64 x = stage[a], y = stage[b];
+                            if((x > y) == ((a & k) == 0)) { stage[a] = y; stage[b] = x; }
+                        }
+                        __syncthreads();
+                    }
+                #pragma unroll
+                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                {
+                    const u32 j = tid + i * LOCAL_BLOCK;
+                    if(j >= m) break;
+                    const u64 v = stage[j];
+                    const u32 key = u32(v >> 32);
+                    u32 a = 0, b = j;                   // first record with this key
+                    while(a < b) { const u32 mid = (a + b) >> 1; if(u32(stage[mid] >> 32) < key) a = mid + 1; else b = mid; }
+                    u32 c = j + 1, f = m;               // first record behind with a greater key
+                    while(c < f) { const u32 mid = (c + f) >> 1; if(u32(stage[mid] >> 32) <= key) c = mid + 1; else f = mid; }
+                    const u32 eq = c - a;
+                    pl[i] = packed_place(j, a, eq);
+                    sa[base + j] = eq == 1 ? u32(v) : SA_OPEN;
+                }
+            }
+            // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
+            u32 tied = 0;
+            #pragma unroll
+            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            {
+                if(i * LOCAL_BLOCK >= m) break;
+                if(tid + i * LOCAL_BLOCK < m) tied |= (pl[i] & (PL_SMALL | PL_LARGE)) ? 1u << i : 0u;
+            }
+            if(__syncthreads_or(tied != 0))
+            {
+                #pragma unroll
+                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                    if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
+                __syncthreads();
+                if(tid < 2)
+                {
+                    const u32 c = s_tied[tid];
+                    s_slot[tid] = c ? atomicAdd(tid ? &counts->large : &counts->small, c) : 0;
+                    s_tied[tid] = 0;
+                }
+                __syncthreads();
+                #pragma unroll
+                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                    if(tied >> i & 1u)
+                    {
+                        const u32 place = pl[i] & 8191u, head = (pl[i] & PL_FIRST) ? place : pl[i] >> 13 & 8191u;
+                        const bool small = (pl[i] & PL_SMALL) != 0;
+                        const u64 k = u64(s_slot[small ? 0 : 1]) + start[head] + (place - head);
+                        list[small ? k : list_cap - 1 - k] = (u64(base + head) << 32) | u32(stage[tid + i * LOCAL_BLOCK]);
+                    }
+            }
+            __syncthreads();        // the next batch reuses the shared arrays
         }
-        __syncthreads();        // the next batch reuses the shared arrays
     }
 }
 
@@ -937,7 +952,7 @@ int launch_code(csa_ctx* ctx, const Prefix_Tables& t, const u16* T, const u64 n,
     {
         static std::atomic<bool> configured[64];
         CSA_TRY(shared_bytes(ctx, make_code_kernel<true>, CODE_SMEM, configured));
-        make_code_kernel<true><<<65536 / CODE_BLOCK, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), nullptr, u32((u64(1) << 22) / n), t.code, t.cnt1, reinterpret_cast<u32*>(counts));
+        make_code_kernel<true><<<65536 / CODE_WALKERS, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), nullptr, u32((u64(1) << 22) / n), t.code, t.cnt1, reinterpret_cast<u32*>(counts));
         CSA_LAUNCH_CHECK(ctx);
     }
     else
@@ -951,7 +966,7 @@ int launch_code(csa_ctx* ctx, const Prefix_Tables& t, const u16* T, const u64 n,
         CSA_CUDA(ctx, cudaMemsetAsync(t.hist, 0, 65536 * 4, ctx->stream));
         sample_symbols_kernel<<<unsigned(blocks > 148 ? 148 : blocks), HIST_BLOCK, HIST_SMEM, ctx->stream>>>(T, n, vectors, t.hist);
         CSA_LAUNCH_CHECK(ctx);
-        make_code_kernel<false><<<65536 / CODE_BLOCK, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), t.hist, u32((u64(1) << 22) / samples), t.code, t.cnt1,
+        make_code_kernel<false><<<65536 / CODE_WALKERS, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), t.hist, u32((u64(1) << 22) / samples), t.code, t.cnt1,
                                                                                           reinterpret_cast<u32*>(counts));
         CSA_LAUNCH_CHECK(ctx);
     }
@@ -988,11 +1003,25 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
     return CSA_OK;
 }
 
-int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u32 chunk, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
+// The second launch takes the children of 4097 to 8192 suffixes; a short text, where a launch counts, goes to the larger blocks at once.
+int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, bool one_level, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
 {
-    static std::atomic<bool> configured[64];
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel, LOCAL_SMEM, configured));
-    local_sort_kernel<<<unsigned(n / chunk + parents), LOCAL_BLOCK, LOCAL_SMEM, ctx->stream>>>(rec, t.chunk_first, t.chunk0 + parents, b2, t.child_off, sa, list, n, counts, t.over);
+    const u32 over_cap = parents << b2;
+    const u32* const chunks = t.chunk0 + parents;
+    if(one_level)
+    {
+        static std::atomic<bool> configured[64];
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, false>, LOCAL_SMEM<512>, configured));
+        local_sort_kernel<512, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+        CSA_LAUNCH_CHECK(ctx);
+        return CSA_OK;
+    }
+    static std::atomic<bool> configured[2][64];
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<256, false>, LOCAL_SMEM<256>, configured[0]));
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, true>, LOCAL_SMEM<512>, configured[1]));
+    local_sort_kernel<256, false><<<unsigned(n / LOCAL_CHUNK + parents), 256, LOCAL_SMEM<256>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    CSA_LAUNCH_CHECK(ctx);
+    local_sort_kernel<512, true><<<148 * 2, 512, LOCAL_SMEM<512>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1021,7 +1050,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
         CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB));
         rec = recB; other = recA;
     }
-    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, one_level ? SHORT_CHUNK : LOCAL_CHUNK, n, rec, sa, other, counts));
+    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, one_level, n, rec, sa, other, counts));
     *list = other;
     *records = rec;
     return CSA_OK;
@@ -1054,7 +1083,7 @@ int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Ta
     CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
                              : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));
     CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB));
-    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, LOCAL_CHUNK, size, recB, sa, recA, counts));
+    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, false, size, recB, sa, recA, counts));
     ctx->counters[1] += 2;
     ctx->counters[2] += 2 * size;
     return CSA_OK;

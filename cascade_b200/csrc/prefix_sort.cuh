@@ -22,7 +22,7 @@ struct Build_Counts
     u32 next_small;     // the same of the list being made
     u32 partitions;     // contiguous ranges of the suffix array, at most as many as asked for, that the first split's buckets form
     u32 max_partition;  // suffixes of the largest
-    u32 pad;
+    u32 medium;         // children that fit the local sort's larger blocks only
 };
 static_assert(sizeof(Build_Counts) <= (CSA_STATUS_WORD - CSA_COUNTS_WORD) * 8, "the counters lie before the status word");
 

@@ -40,7 +40,7 @@ def test_sizes_at_the_edges(ctx, oracle, n):
 
 
 @pytest.mark.parametrize("n", [257, 1793, 2049, 8193, 70_001, 2_200_000])
-@pytest.mark.parametrize("kind", ["one", "two", "period", "phrase", "stretch", "zeros_at_the_end", "copies", "wide"])
+@pytest.mark.parametrize("kind", ["one", "two", "period", "phrase", "stretch", "zeros_at_the_end", "copies", "phrase_of_thousands", "wide"])
 def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
     rng = np.random.default_rng(n)
     if kind == "one":                   # one group of everything, halved by every generation
@@ -53,6 +53,10 @@ def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
         T = rng.integers(0, 60000, n)
         for k in range(12):
             T[k + 5::30] = 1000 + k
+    elif kind == "phrase_of_thousands":     # at 2.2 million a child of some 6300 suffixes: for the larger blocks of the local sort alone
+        T = rng.integers(0, 60000, n)
+        for k in range(6):
+            T[k + 5::350][:len(T) // 350] = 1000 + k
     elif kind == "stretch":             # copies of a long stretch: groups below and above 256 members, many generations
         T = rng.integers(0, 3000, n)
         L = max(8, n // 700)
