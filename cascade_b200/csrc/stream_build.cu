@@ -23,7 +23,7 @@
 // a part here writes its new ranks as (position, rank) messages into an outbox on the device, and the exchange applies
 // them to R after the generation's last part: every read of a generation sees the ranks of the generation before.
 //
-// A text without long repeats needs none of this: direct_parts below orders one range of the array after the other from the text
+// A text without long repeats needs none of this: build_direct_parts below orders one range of the array after the other from the text
 // alone, and the protocol above is what a text falls back to.
 #include "common.cuh"
 #include "part.cuh"
@@ -843,13 +843,15 @@ namespace
 constexpr u64 DIRECT_MAX_PARTS = 64;
 constexpr u64 DIRECT_MIN = 1 << 14;
 
+}   // namespace
+
 // The parts of the suffix array one after the other, straight from the text on the device: the suffixes whose encoding starts
 // with a run of leading bits are sorted by prefix_sort.cu, their ties are ordered by the text, and the finished range of the
 // array is copied out under the sorting of the next. No list leaves the device and no ranks are kept: PCIe carries the text in and
 // the array out once (7 bytes a suffix; the lists take 41). `done` stays false where that is not enough (a part with groups of many tied
 // suffixes or with long shared stretches, a run of bits with more suffixes than a part may hold): the caller then starts over the
 // general way, whatever was copied out.
-int direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, const u64 part_suffixes, u8* sa40_host, csa_build_stats& bs, bool& done)
+int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, const u64 part_suffixes, u8* sa40_host, csa_build_stats& bs, bool& done)
 {
     const auto t_start = std::chrono::steady_clock::now();
     const Prefix_Sort ps = prefix_sort_part_plan(n);
@@ -947,8 +949,6 @@ int direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, const u64
     return CSA_OK;
 }
 
-}   // namespace
-
 extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint64_t n, uint32_t p, uint64_t seed, uint8_t* sa40_host,
                                    const csa_tier_options* options, csa_build_stats* stats)
 {
@@ -979,7 +979,7 @@ extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint
     if(sa40_host && !options->output_path && offset == 0 && n >= DIRECT_MIN && n < (u64(1) << 31) && options->host_list_bytes >= 9 * n)
     {
         bool done = false;
-        CSA_TRY(direct_parts(ctx, T, n, p, part_suffixes, sa40_host, bs, done));
+        CSA_TRY(build_direct_parts(ctx, T, n, p, part_suffixes, sa40_host, bs, done));
         if(done)
         {
             bs.ms_total = ms_since(t_start);
