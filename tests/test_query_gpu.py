@@ -239,3 +239,30 @@ def test_host_batches_of_several_chunks_over_the_lanes(ctx, oracle):
     with pytest.raises(api.CascadeError) as e:
         idx.query_host(off, sym, 20, small)
     assert e.value.code == 3
+
+
+@pytest.mark.parametrize("n,stride", [(40, 1), (1000, 16), (33 * 64, 64), (70_001, 1), (70_001, 32)])
+def test_small_batches_agree_with_large_ones(ctx, oracle, n, stride):
+    """Up to 8192 queries a warp searches for each, above it a thread: both against the oracle, with the same patterns (none longer than the
+    text, empty ones, frequent ones, ones behind and before everything)."""
+    rng = np.random.default_rng(n)
+    T = np.minimum(rng.zipf(1.4, n), 300).astype(np.uint16)
+    T[n // 2:n // 2 + min(n // 4, 300)] = 7
+    sa = oracle.build_sa40(T)
+    idx = _index(ctx, T, sa, stride)
+    q = 8192
+    pats = []
+    for i in range(q):
+        m = int(rng.integers(0, 17))
+        at = int(rng.integers(0, max(1, n - m)))
+        pats.append(T[at:at + m] if i % 3 else rng.integers(0, 310, m).astype(np.uint16))
+    pats[0], pats[1], pats[2] = np.zeros(9, np.uint16), np.full(3, 65535, np.uint16), np.full(12, 7, np.uint16)
+    off = np.concatenate([[0], np.cumsum([len(x) for x in pats])]).astype(np.int64)
+    sym = np.concatenate(pats + [np.zeros(8, np.uint16)]).astype(np.uint16)
+    o, sy = _dev(off.astype(np.uint64), sym)
+    small = idx.find(o, sy, q).cpu().numpy().view(np.uint64)
+    o, sy = _dev(np.concatenate([off, [off[-1]]]).astype(np.uint64), sym)         # one empty pattern more: the other kernel
+    large = idx.find(o, sy, q + 1).cpu().numpy().view(np.uint64)
+    want = oracle.find_batch(T, sa, off, sym)
+    assert np.array_equal(small, want)
+    assert np.array_equal(large[:2 * q], want)
