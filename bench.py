@@ -34,10 +34,9 @@ C2_PARTITIONS = 64
 C2_MEAN_DOC = 1024
 C3_TOKENS = 1_000_000_000
 C5_QUERIES = 4_000_000
-# DRAM read + write per record of one launch of the digit-pass kernel (24 B algorithmic), from an ncu capture of a launch over
-# 1e8 records (a 1e8-token build); traffic grows with the records of a launch, so the benchmark scales it to its own launch
-# (generation 0 moves all n records per launch). It is a figure from that capture, not measured by the run that prints it.
-ONESWEEP_TRAFFIC_PER_RECORD_FROM_PROFILE = 23.71
+# What the passes of a resident build over a text without long repeats move per suffix: count (text) 2, first split (text, record) 2 + 8, count
+# of the second split 8, second split 8 + 8, local sort (record, position) 8 + 4, output 4 + 5.
+BUILD_BYTES_PER_SUFFIX = 57
 
 
 def measured_peak_gbs():
@@ -187,7 +186,7 @@ def workload_config(args, n_gpus):
     return {"workload": "in-HBM suffix-array build, BASELINE config 2" if args.tokens == C2_TOKENS else "in-HBM suffix-array build (reduced size)",
             "tokens": args.tokens, "symbol_bytes": 2, "vocab": 50257, "zipf_s": 1.1, "mean_doc": C2_MEAN_DOC, "separator": 65535,
             "partitions": C2_PARTITIONS, "kgram": 8, "output": "sa40", "seed": 0, "gpus": n_gpus,
-            "l2": "inputs (4 GB text, 24 GB of sort records per pass at full size) exceed the 126 MB L2; no flush needed"}
+            "l2": "inputs (4 GB text, 16 GB of records per pass at full size) exceed the 126 MB L2; no flush needed"}
 
 
 def run_reference(args):
@@ -219,7 +218,15 @@ def run_reference(args):
 
 # ---- the GPU side -----------------------------------------------------------------------------------------------------
 
-def pass_roofline(ctx, peak, peak_kind, step_ms_total, traffic):
+def build_roofline(n, ms, peak, peak_kind):
+    """The resident build against the copy bandwidth: bytes of its passes over its device time."""
+    achieved = BUILD_BYTES_PER_SUFFIX * n / (ms * 1e-3) / 1e9
+    return {"bound": "hbm", "kernel": "the whole build: count_long_text, scatter_text, count_children, scatter_children, local_sort, pack_sa40", "achieved": achieved,
+            "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"of {peak_kind}", "traffic": BUILD_BYTES_PER_SUFFIX * n,
+            "traffic_note": "the bytes that the passes read and write by design, not measured by this run"}
+
+
+def pass_roofline(ctx, peak, peak_kind, step_ms_total):
     from cascade_b200._lib import c_u64
     pm, pc, pr, pb = ctypes.c_double(0), c_u64(0), c_u64(0), c_u64(0)
     ctx.L.csa_get_pass_timing(ctx.h, ctypes.byref(pm), ctypes.byref(pc), ctypes.byref(pr), ctypes.byref(pb))
@@ -229,11 +236,8 @@ def pass_roofline(ctx, peak, peak_kind, step_ms_total, traffic):
     achieved = pb.value / (pm.value * 1e-3) / 1e9 if pm.value > 0 else 0.0
     r = {"bound": "hbm", "kernel": "one 8-bit digit pass of the LSD radix sort (onesweep_seg_pass_kernel over all partitions in generation 0, onesweep_pass_kernel "
                                    "over the tied suffixes later: the same tile code)", "achieved": achieved, "peak": peak,
-         "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"of {peak_kind}", "traffic": traffic,
+         "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"of {peak_kind}",
          "passes": pc.value, "records": pr.value, "pass_ms_total": pm.value}
-    if traffic is not None:
-        r["traffic_note"] = ("DRAM bytes of one generation-0 launch (all records of the build; algorithmic: 24 B per record), scaled by the records from an ncu "
-                             "capture of the same kernel over 1e8 records (23.71 B per record); not measured by this run")
     if step_ms_total:
         r["share_of_step"] = pm.value / step_ms_total
     return r
@@ -341,7 +345,6 @@ def run_ours(args):
 
     for _ in range(args.warmup):
         api.build_sa(ctx, T, n, p, out=out)
-    ctx.L.csa_set_pass_timing(ctx.h, 1)
     ctx.reset_counters()
     torch.cuda.synchronize()
     step_ms, launches, stats = [], 0, None
@@ -355,7 +358,7 @@ def run_ours(args):
         torch.cuda.synchronize()
         wall_ms = 1e3 * (time.perf_counter() - t0) / args.steps
     ms = sum(step_ms) / len(step_ms)
-    roofline = pass_roofline(ctx, peak, peak_kind, ms * args.steps, ONESWEEP_TRAFFIC_PER_RECORD_FROM_PROFILE * n)
+    roofline = build_roofline(n, ms, peak, peak_kind)
     validation = api.validate_sa(ctx, T, n, out)         # the whole array, outside the timed region
 
     # ---- end to end through the host-buffer entry point --------------------------------------------------------------
@@ -511,7 +514,7 @@ def run_ours_multi(args):
         dist.barrier()
         torch.cuda.synchronize()
     ms = sum(step_ms) / len(step_ms)
-    roofline = pass_roofline(ctx, peak, peak_kind, None, None)
+    roofline = pass_roofline(ctx, peak, peak_kind, None)
     roofline["kernel"] += ", rank 0"
     count = sum(c for _, c in segs)
     total = _sum_over_ranks(count, dev)

@@ -19,6 +19,7 @@
 // It stands for select_pivots, partition and the sort of initial_rank (src/GPU_SACA.cu:290-364, 737-826, 1111-1331).
 #include "prefix_sort.cuh"
 
+#include <algorithm>
 #include <atomic>
 
 namespace
@@ -634,16 +635,30 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
     const u32 rmask = rbits == 32 ? 0xFFFFFFFFu : (1u << rbits) - 1;
 
     const u32 works = MEDIUM ? counts->medium : *chunks;
+    u32 next_first = 0, next_end = 0;       // the children of the chunk after this one, read ahead
+    auto look_up = [&](const u32 w)
+    {
+        next_first = MEDIUM ? over[over_cap - 1 - w] : __ldg(chunk_first + w);
+        next_end = MEDIUM ? next_first + 1 : __ldg(chunk_first + w + 1);
+    };
+    if(blockIdx.x < works) look_up(blockIdx.x);
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
         // the block's children: at most all of one parent
-        const u32 child0 = MEDIUM ? over[over_cap - 1 - work] : __ldg(chunk_first + work);
-        const u32 last = MEDIUM ? 1u : min(__ldg(chunk_first + work + 1), ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
+        const u32 child0 = next_first;
+        const u32 last = min(next_end, ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
+        const bool more = work + gridDim.x < works;
+        if(more) look_up(work + gridDim.x);
         const u32 first_digit = child0 & (children - 1);
         for(u32 d = tid; d <= last; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + child0 + d);
         if(tid < 2) s_tied[tid] = 0;
         __syncthreads();
         u32 cur = 0;
+        if(!MEDIUM && more)         // the next chunk's records on their way to L2: 16 to a line
+        {
+            const u64 at = u64(__ldg(child_off + next_first)) + tid * 16;
+            if(at < list_cap) asm volatile("prefetch.global.L2 [%0];" :: "l"(rec + at));
+        }
 
         while(cur < last)
         {
@@ -1019,7 +1034,7 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
     static std::atomic<bool> configured[2][64];
     CSA_TRY(shared_bytes(ctx, local_sort_kernel<256, false>, LOCAL_SMEM<256>, configured[0]));
     CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, true>, LOCAL_SMEM<512>, configured[1]));
-    local_sort_kernel<256, false><<<unsigned(n / LOCAL_CHUNK + parents), 256, LOCAL_SMEM<256>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    local_sort_kernel<256, false><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 4 * 8)), 256, LOCAL_SMEM<256>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
     local_sort_kernel<512, true><<<148 * 2, 512, LOCAL_SMEM<512>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);

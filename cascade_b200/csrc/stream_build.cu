@@ -969,14 +969,18 @@ extern "C" int csa_build_sa_tiered(csa_ctx* ctx, const uint16_t* text_host, uint
 
     // ---- text and partition ids on the device ------------------------------------------------------------------------------
     Dev_Buffer text_b, pid_b, small_b, stage_b;
-    CSA_TRY(text_b.alloc(ctx, (n + CSA_TEXT_PAD) * 2 + 256));
-    u16* T = static_cast<u16*>(text_b.p);
+    // The direct way serves texts of 31-bit positions whose array goes to memory and whose lists, were they needed, would too. Its text lies in
+    // the context's second buffer, which a second build of this size does not allocate again.
+    const bool direct = sa40_host && !options->output_path && offset == 0 && n >= DIRECT_MIN && n < (u64(1) << 31) && options->host_list_bytes >= 9 * n;
+    void* text_p = nullptr;
+    if(direct) CSA_TRY(csa_aux(ctx, (n + CSA_TEXT_PAD) * 2 + 256, &text_p));
+    else { CSA_TRY(text_b.alloc(ctx, (n + CSA_TEXT_PAD) * 2 + 256)); text_p = text_b.p; }
+    u16* T = static_cast<u16*>(text_p);
     CSA_CUDA(ctx, cudaMemcpyAsync(T, text_host, n * 2, cudaMemcpyHostToDevice, ctx->stream));
     CSA_CUDA(ctx, cudaMemsetAsync(T + n, 0, CSA_TEXT_PAD * 2, ctx->stream));
     if(part_suffixes == 0) part_suffixes = u64(1) << 27;
     if(part_suffixes >= (u64(1) << 31)) part_suffixes = (u64(1) << 31) - 1;
-    // The direct way serves texts of 31-bit positions whose array goes to memory and whose lists, were they needed, would too.
-    if(sa40_host && !options->output_path && offset == 0 && n >= DIRECT_MIN && n < (u64(1) << 31) && options->host_list_bytes >= 9 * n)
+    if(direct)
     {
         bool done = false;
         CSA_TRY(build_direct_parts(ctx, T, n, p, part_suffixes, sa40_host, bs, done));
