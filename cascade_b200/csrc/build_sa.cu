@@ -37,8 +37,8 @@ Build_Layout layout_for(u64 n)
     L.tables = align256(prefix_sort_table_bytes(prefix_sort_plan(n)));
     L.total = 2 * L.rec + L.sa + L.tables + 4096;
     L.sort_ws = align256(csa_sort_workspace_bytes(n));
-    L.scratch = align256(div_up(n, RANK_TILE) * 3 * 4 + 256);
-    L.work = align256(n * 12) + 16 * 256;
+    L.scratch = oversize_scratch_bytes(n);
+    L.work = oversize_work_bytes(n);
     L.more = L.isa + L.sort_ws + L.scratch + L.work + 4096;
     return L;
 }
@@ -47,6 +47,13 @@ Build_Layout layout_for(u64 n)
 // the sorting: 14.4 ms. Below it the parts' launches cost what the overlap gives.
 constexpr u64 HOST_PARTS_MIN = u64(1) << 23;
 constexpr u64 SMALL_BUILD = u64(1) << 22;       // up to here the output is packed before the host knows whether ties are left
+
+int set_build_count(csa_ctx* ctx, u32* at, u32 value)
+{
+    if(value == 0) CSA_CUDA(ctx, cudaMemsetAsync(at, 0, 4, ctx->stream));
+    else CSA_CUDA(ctx, cudaMemcpyAsync(at, &value, 4, cudaMemcpyHostToDevice, ctx->stream));     // pageable: copied before the call returns
+    return CSA_OK;
+}
 
 struct Build
 {
@@ -71,13 +78,7 @@ struct Build
 
     int read_counts(Build_Counts& c) { return read_build_counts(ctx, n, c); }
 
-    int set_count(u32 Build_Counts::*field, u32 value)
-    {
-        u32* const at = &(counts->*field);
-        if(value == 0) CSA_CUDA(ctx, cudaMemsetAsync(at, 0, 4, ctx->stream));
-        else CSA_CUDA(ctx, cudaMemcpyAsync(at, &value, 4, cudaMemcpyHostToDevice, ctx->stream));     // pageable: copied before the call returns
-        return CSA_OK;
-    }
+    int set_count(u32 Build_Counts::*field, u32 value) { return set_build_count(ctx, &(counts->*field), value); }
 
     // The buffers for ranking, from the context's second buffer.
     int more_memory()
@@ -93,34 +94,10 @@ struct Build
         return cv.ok ? CSA_OK : csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
     }
 
-    // Children that did not fit a block: sorted by (child, key) and ranked. The records are in `other`; the hole between the two
-    // ends of the list takes the keys.
     int sort_oversize(const Build_Counts& c)
     {
-        const u64 M = c.oversize_records;
-        if(M > n || u64(c.small) + c.large + M > n) return csa_fail(ctx, CSA_E_DEVICE, "build: oversize children do not add up");
         CSA_TRY(more_memory());
-        u64* const keysA = front + c.small;
-        u64* const keysB = other;
-        Carver cv(work, L.work);
-        u32* posA = cv.take<u32>(M);
-        u32* posB = cv.take<u32>(M);
-        u32* head = cv.take<u32>(M);
-        if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
-        CSA_TRY(launch_gather_oversize(ctx, ps, tab, c.oversize, other, keysA, posA, scratch));
-        int in_alt = 0;
-        CSA_TRY(csa_sort_pairs(ctx, reinterpret_cast<uint64_t*>(keysA), reinterpret_cast<uint64_t*>(keysB), posA, posB, 4, M, 0, 64, sort_ws, L.sort_ws, &in_alt));
-        u64* const ks = in_alt ? keysB : keysA;
-        CSA_CUDA(ctx, cudaMemsetAsync(ctx->d_scalars, 0, 8, ctx->stream));
-        Isa_View none{};
-        const Slot_Map whole{nullptr, nullptr, 0, 0};
-        CSA_TRY(launch_rank_and_compact(ctx, ks, in_alt ? posB : posA, M, 32, 0, none, whole, sa, head, in_alt ? posA : posB, ctx->d_scalars, scratch, in_alt ? keysA : keysB, true));
-        CSA_TRY(set_count(&Build_Counts::next_small, c.small));
-        CSA_TRY(launch_split_by_size(ctx, head, in_alt ? posA : posB, M, ctx->d_scalars, front, n, counts, scratch));
-        CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
-        CSA_TRY(set_count(&Build_Counts::next_small, 0));
-        CSA_TRY(set_count(&Build_Counts::oversize, 0));
-        return CSA_OK;
+        return sort_oversize_children(ctx, ps, tab, c, n, front, other, sa, counts, {sort_ws, L.sort_ws, scratch, work, L.work});
     }
 
     // One generation of prefix doubling: the suffixes of every group ordered by the ranks of those h symbols further on. The first
@@ -296,6 +273,37 @@ int check_build_args(csa_ctx* ctx, const void* text, u64 n, u32 p, const void* o
 }
 
 }   // namespace
+
+size_t oversize_scratch_bytes(u64 records) { return align256(div_up(records, RANK_TILE) * 3 * 4 + 256); }
+size_t oversize_work_bytes(u64 records) { return align256(records * 12) + 16 * 256; }
+
+int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& tab, const Build_Counts& c, u64 n, u64* front, u64* other, u32* sa, Build_Counts* counts,
+                           const Oversize_Buffers& b)
+{
+    const u64 M = c.oversize_records;
+    if(M > n || u64(c.small) + c.large + M > n) return csa_fail(ctx, CSA_E_DEVICE, "build: oversize children do not add up");
+    const Ties_In_Any_Order free_ties(ctx);
+    u64* const keysA = front + c.small;
+    u64* const keysB = other;
+    Carver cv(b.work, b.work_bytes);
+    u32* posA = cv.take<u32>(M);
+    u32* posB = cv.take<u32>(M);
+    u32* head = cv.take<u32>(M);
+    if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
+    CSA_TRY(launch_gather_oversize(ctx, ps, tab, c.oversize, other, keysA, posA, b.scratch));
+    int in_alt = 0;
+    CSA_TRY(csa_sort_pairs(ctx, reinterpret_cast<uint64_t*>(keysA), reinterpret_cast<uint64_t*>(keysB), posA, posB, 4, M, 0, 64, b.sort_ws, b.sort_bytes, &in_alt));
+    u64* const ks = in_alt ? keysB : keysA;
+    CSA_CUDA(ctx, cudaMemsetAsync(ctx->d_scalars, 0, 8, ctx->stream));
+    Isa_View none{};
+    const Slot_Map whole{nullptr, nullptr, 0, 0};
+    CSA_TRY(launch_rank_and_compact(ctx, ks, in_alt ? posB : posA, M, 32, 0, none, whole, sa, head, in_alt ? posA : posB, ctx->d_scalars, b.scratch, in_alt ? keysA : keysB, true));
+    CSA_TRY(set_build_count(ctx, &counts->next_small, c.small));
+    CSA_TRY(launch_split_by_size(ctx, head, in_alt ? posA : posB, M, ctx->d_scalars, front, n, counts, b.scratch));
+    CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
+    CSA_TRY(set_build_count(ctx, &counts->next_small, 0));
+    return set_build_count(ctx, &counts->oversize, 0);
+}
 
 extern "C" size_t csa_build_device_bytes(uint64_t n, uint32_t p)
 {

@@ -65,8 +65,9 @@ struct csa_ctx
 struct Ties_In_Any_Order
 {
     csa_ctx* ctx;
-    explicit Ties_In_Any_Order(csa_ctx* c) : ctx(c) { ctx->ties_in_any_order = true; }
-    ~Ties_In_Any_Order() { ctx->ties_in_any_order = false; }
+    bool before;
+    explicit Ties_In_Any_Order(csa_ctx* c) : ctx(c), before(c->ties_in_any_order) { ctx->ties_in_any_order = true; }
+    ~Ties_In_Any_Order() { ctx->ties_in_any_order = before; }
     Ties_In_Any_Order(const Ties_In_Any_Order&) = delete;
     Ties_In_Any_Order& operator=(const Ties_In_Any_Order&) = delete;
 };

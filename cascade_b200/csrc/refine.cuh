@@ -36,3 +36,17 @@ int launch_unpack_list(csa_ctx* ctx, const u64* list, u64 count, u32* head, u32*
 
 // The inverse array from sa (final slots) and the lists of tied suffixes. updates: n entries of scratch and 256 words.
 int launch_make_inverse(csa_ctx* ctx, const u32* sa, u64 n, const u64* small_list, u64 small, const u64* large_list, u64 large, u32* isa, u64* updates);
+
+// Children that did not fit a block's local sort (c: the counters read back, c.oversize > 0): sorted by (child, key) by the radix sort and
+// ranked. The records are in `other`; the hole between the two ends of the list in front (n entries) takes the keys. The counters then
+// stand as if the children had been sorted with the others, and launch_refine_by_text, which left the list alone, can be called again.
+struct Oversize_Buffers
+{
+    void* sort_ws; size_t sort_bytes;       // csa_sort_workspace_bytes of the records
+    u32* scratch;                           // oversize_scratch_bytes
+    u8* work; size_t work_bytes;            // oversize_work_bytes
+};
+size_t oversize_scratch_bytes(u64 records);
+size_t oversize_work_bytes(u64 records);
+int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& tab, const Build_Counts& c, u64 n, u64* front, u64* other, u32* sa, Build_Counts* counts,
+                           const Oversize_Buffers& b);

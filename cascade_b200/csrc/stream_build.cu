@@ -842,6 +842,7 @@ namespace
 // about 0.9 ns a suffix over PCIe: up to this many parts the direct way moves less.
 constexpr u64 DIRECT_MAX_PARTS = 64;
 constexpr u64 DIRECT_MIN = 1 << 14;
+constexpr u64 DIRECT_OVERSIZE = 64;         // up to this share of a part's suffixes may lie in children that go through the radix sort
 
 }   // namespace
 
@@ -896,6 +897,8 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     const cudaStream_t copy_stream = ctx->lane[0];
     const cudaEvent_t packed = ctx->lane_event[0], copied[2] = {ctx->lane_event[1], ctx->lane_event[2]};
     struct Drain { cudaStream_t s; ~Drain() { cudaStreamSynchronize(s); } } drain{copy_stream};       // no copy outlives the call, nor runs under the general way
+    Dev_Buffer extra;           // for children that go through the radix sort
+    size_t extra_bytes = 0;
     u64 active = 0;
     u32 rounds = 0;
     for(u32 u = 0; u < parts; ++u)
@@ -908,6 +911,21 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
         CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
         Build_Counts c;
         CSA_TRY(read_build_counts(ctx, S, c));
+        if(c.oversize && c.oversize_records <= S / DIRECT_OVERSIZE)
+        {
+            const u64 M = c.oversize_records;
+            const size_t sort_bytes = align_up256(csa_sort_workspace_bytes(M)), scratch_bytes = align_up256(oversize_scratch_bytes(M)), work_bytes = oversize_work_bytes(M);
+            if(extra_bytes < sort_bytes + scratch_bytes + work_bytes)
+            {
+                if(extra.p) { CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); cudaFree(extra.p); extra.p = nullptr; }
+                extra_bytes = 2 * (sort_bytes + scratch_bytes + work_bytes);
+                CSA_TRY(extra.alloc(ctx, extra_bytes));
+            }
+            u8* const at = static_cast<u8*>(extra.p);
+            CSA_TRY(sort_oversize_children(ctx, ps, tab, c, S, list, next, sa, counts, {at, sort_bytes, reinterpret_cast<u32*>(at + sort_bytes), at + sort_bytes + scratch_bytes, work_bytes}));
+            CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
+            CSA_TRY(read_build_counts(ctx, S, c));
+        }
         if(c.oversize || c.large) return CSA_OK;
         active += c.small;
         u32 r = c.small ? 1 : 0;

@@ -304,7 +304,7 @@ def test_rank_shard_primitives(ctx):
 
 
 @pytest.mark.parametrize("n,part_suffixes", [(1 << 14, 0), (70_001, 20_000), (70_001, 1500), ((1 << 21) + 3, 1 << 18), ((1 << 22) + 5, 1_000_003)])
-@pytest.mark.parametrize("tail", ["zipf", "few_long_repeats", "period_in_the_last_part"])
+@pytest.mark.parametrize("tail", ["zipf", "few_long_repeats", "pair_of_thousands", "period_in_the_last_part"])
 def test_parts_straight_from_the_text(ctx, oracle, n, part_suffixes, tail):
     """Texts whose parts need the text alone, texts with a long repeat that is read further, and texts that show only in their last part
     that they need the general way (parts of 1500 suffixes are more than the direct way takes, too)."""
@@ -314,6 +314,8 @@ def test_parts_straight_from_the_text(ctx, oracle, n, part_suffixes, tail):
     if tail == "few_long_repeats":
         T[n // 2:n // 2 + 40] = T[:40]
         T[-100:] = T[300:400]
+    elif tail == "pair_of_thousands":       # at 4 million a bucket of 9000 suffixes that differ soon: too many for a block, ordered by the radix sort
+        T[5:-1:460], T[6::460] = 60001, 60002
     elif tail == "period_in_the_last_part":
         T[n // 3:n // 3 + 3000] = np.resize([65535, 65534, 65535], 3000)
     sa, st = api.build_sa_streamed(ctx, _padded(T), n, 16, part_suffixes=part_suffixes)
