@@ -612,7 +612,7 @@ __device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, con
 // What bounds it is latency and the issue of instructions, not memory (12 bytes a record at 0.9 TB/s): a block goes through
 // barriers between dependent steps. So a block finds its children in two dependent reads (chunk_first, child_off), tied records get
 // their list places from one counter in shared memory, and four small blocks share an SM (two of 512 threads: 27.7 ms at 2e9
-// records, four of 256: 24.5 ms, and 0.5 ms for the children that need the larger ones).
+// records, four of 256: 24.5 ms, and 0.5 ms for the children that need the larger ones). A block reads its next chunk ahead (2^24 tokens: 618 -> 605 us a build).
 // MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
 // there if a block of 512 threads holds them, and to the front, for the radix sort, if not.
 constexpr u32 MEDIUM_CAP = LOCAL_CAP<512>;
@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
             // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
             for(u32 i = tid; i < ((m + 1) / 2 + 7) / 8 * 2; i += LOCAL_BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
             u64 r[LOCAL_ITEMS];
-            u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later place | head << 13 | tied << 26
+            u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later packed_place
             #pragma unroll
             for(int i = 0; i < LOCAL_ITEMS; ++i)
             {
