@@ -175,8 +175,8 @@ typedef struct csa_build_stats
 size_t csa_build_device_bytes(uint64_t n, uint32_t p);
 /* Builds the suffix array of text_dev[0, n) (n < 2^32 - 2^26; CSA_TEXT_PAD zero symbols must follow the text)
  * into sa40_dev as 5-byte little-endian entries in numeric symbol order with shorter suffixes first
- * (5 n bytes are written; the buffer must hold 5 n + CSA_SA_PAD_BYTES). p is the number of partitions asked for
- * (K-gram splitters, CSA_K symbols); seed drives the sampling only (the suffix array does not depend on it).
+ * (5 n bytes are written; the buffer must hold 5 n + CSA_SA_PAD_BYTES). p is the number of partitions asked for: of a build
+ * on one GPU the statistics tell as many ranges apart, and neither p nor seed changes its work.
  * Replaces GPU_SACA::build_SA (src/GPU_SACA.cu:124-216) for a text resident in device memory. */
 int csa_build_sa(csa_ctx* ctx, const uint16_t* text_dev, uint64_t n, uint32_t p, uint64_t seed, uint8_t* sa40_dev,
                  csa_build_stats* stats);
