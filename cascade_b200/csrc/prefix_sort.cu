@@ -679,11 +679,12 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                     // a child that does not fit: left to the radix sort
                     if(tid == 0)
                     {
-                        if(!MEDIUM && coff[cur + 1] - base <= MEDIUM_CAP) over[over_cap - 1 - atomicAdd(&counts->medium, 1u)] = child0 + cur;
+                        const u32 size = coff[cur + 1] - base;
+                        if(!MEDIUM && size <= MEDIUM_CAP) over[over_cap - 1 - atomicAdd(&counts->medium, 1u)] = child0 + cur;
                         else
                         {
                             over[atomicAdd(&counts->oversize, 1u)] = child0 + cur;
-                            atomicAdd(&counts->oversize_records, coff[cur + 1] - base);
+                            atomicAdd(&counts->oversize_records, size);
                         }
                     }
                     ++cur;
@@ -865,6 +866,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
             }
             __syncthreads();        // the next batch reuses the shared arrays
         }
+        __syncthreads();            // a chunk may end in a child that was left or in an empty one: coff is still being read then
     }
 }
 

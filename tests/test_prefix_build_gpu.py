@@ -73,3 +73,36 @@ def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
         T = rng.integers(0, 65536, n)
     st = _check(ctx, oracle, T)
     assert st.n == len(T) and 1 <= st.partitions <= 8 and 0 < st.max_partition <= len(T)
+
+
+def _pairs_text(n, medium, oversize, seed):
+    """Random symbols, and pairs of symbols that stand together many times: a child of 4097 to 8192 suffixes for each of the `medium`
+    pairs, one of more than 8192 for each of the `oversize` ones, spread over the whole array."""
+    rng = np.random.default_rng(seed)
+    T = rng.integers(0, 65000, n, dtype=np.uint16)
+    sizes = np.concatenate([rng.integers(4300, 7500, medium), rng.integers(8600, 9500, oversize)])
+    rng.shuffle(sizes)
+    slots = 2 * rng.permutation((n - 2) // 2)[:sizes.sum()]
+    which = np.repeat(np.arange(len(sizes)), sizes)
+    T[slots] = 100 + 255 * which
+    T[slots + 1] = 101 + 255 * which
+    return T
+
+
+def test_blocks_that_go_on_behind_a_child_left_to_others(ctx, oracle):
+    """More chunks of the local sort than blocks (4736), so that blocks take two or three: chunks that end in a child too large for the block
+    stand among their first, middle and last ones. Resident, and as one part straight from the text."""
+    from cascade_b200 import api
+    T = _pairs_text(21_000_003, 230, 24, 5)
+    n = len(T)
+    want = oracle.build_sa40(T)[:5 * n]
+    Tp = np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)])
+    Td = torch.from_numpy(Tp.view(np.int16)).cuda().view(torch.uint16)
+    for _ in range(3):
+        sa, st = api.build_sa(ctx, Td, n, 8)
+        assert np.array_equal(sa[:5 * n].cpu().numpy(), want)
+        assert st.sort_passes > 2, "no child went through the radix sort"
+    for _ in range(3):
+        sa, st = api.build_sa_streamed(ctx, Tp, n, 8)
+        assert np.array_equal(sa[:5 * n], want)
+        assert st.sort_passes > 2 and st.generations == 1, "not straight from the text, or no child went through the radix sort"
