@@ -73,6 +73,12 @@ struct Build
     void* sort_ws = nullptr;
     u32* scratch = nullptr;
     u8* work = nullptr;
+    // Large groups as the last generation left them, `large` entries in arrays instead of the buffer's back (see generation)
+    bool in_arrays = false;
+    u64 array_cap = 0;
+    u32* head = nullptr;
+    u32* pos = nullptr;
+    u32* pos_other = nullptr;
 
     u64* large_list(u64* buf) const { return buf + (n - large); }
 
@@ -102,51 +108,64 @@ struct Build
 
     // One generation of prefix doubling: the suffixes of every group ordered by the ranks of those h symbols further on. The first
     // `idle` entries of the list share 2 h symbols already and stay as they are.
+    //
+    // What is left of the large groups is counted by size. Where few of them have become small (up to one in eight), they all stay in the arrays
+    // that the ranking left, and the radix sort takes the small ones once more: to write the two lists and read them again costs 40 bytes a
+    // suffix, a suffix too many in a radix sort some 200.
     int generation(u64 h, u64 idle)
     {
         const bool all_by_sort = h > MAX_SMALL_H;       // small groups compare 32-bit numbers, which need h below that
         const u64 ns = all_by_sort ? 0 : small - idle, nl = large + (all_by_sort ? small - idle : 0);
-        Carver cv(work, L.work);
-        u32* secs = cv.take<u32>(ns);
-        u32* posA = cv.take<u32>(nl);
-        u32* posB = cv.take<u32>(nl);
-        u32* head = cv.take<u32>(nl);
-        if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
+        if(!in_arrays) array_cap = nl;
+        const size_t one = align256(array_cap * 4);
+        if(nl > array_cap || align256(ns * 4) + 3 * one > L.work) return csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
+        u32* const secs = reinterpret_cast<u32*>(work);         // the arrays lie at the end: they stay where they are while this one grows and shrinks
+        if(!in_arrays)
+        {
+            u8* const arrays = work + L.work - 3 * one;
+            head = reinterpret_cast<u32*>(arrays); pos = reinterpret_cast<u32*>(arrays + one); pos_other = reinterpret_cast<u32*>(arrays + 2 * one);
+        }
         Isa_View iv{};
         iv.shard[0] = isa; iv.shard_size = n; iv.gpus = 1;
         // every rank that this generation reads is read before any is written
         CSA_TRY(launch_gather_ranks(ctx, front + idle, ns, isa, n, h, secs));
-        u64* const keysA = other + (n - nl);
-        u64* const keysB = front + (n - nl);
+        // behind what refine_by_ranks writes, on a 16-byte boundary where there is room: the sort and the ranking then load two keys at once
+        const u64 keys_at = (n - nl) - ((n - nl) & (n - nl > idle + ns ? 1 : 0));
+        u64* const keysA = other + keys_at;
+        u64* const keysB = front + keys_at;
         const int sec_bits = bits_for(n - 1 + h), prim_bits = std::max(1, bits_for(n - 1));
         if(nl)
         {
             if(sec_bits + prim_bits > 64) return csa_fail(ctx, CSA_E_LIMIT, "build: rank pair does not fit a 64-bit key");
-            if(all_by_sort) CSA_TRY(launch_unpack_list(ctx, front + idle, small - idle, head + large, posA + large));
-            CSA_TRY(launch_unpack_list(ctx, large_list(front), large, head, posA));
-            CSA_TRY(launch_keys_gen(ctx, head, posA, nl, n, h, sec_bits, iv, keysA));
+            if(all_by_sort) CSA_TRY(launch_unpack_list(ctx, front + idle, small - idle, head + large, pos + large));
+            if(!in_arrays) CSA_TRY(launch_unpack_list(ctx, large_list(front), large, head, pos));
+            CSA_TRY(launch_keys_gen(ctx, head, pos, nl, n, h, sec_bits, iv, keysA));
         }
         if(idle) CSA_CUDA(ctx, cudaMemcpyAsync(other, front, idle * 8, cudaMemcpyDeviceToDevice, ctx->stream));
         CSA_TRY(set_count(&Build_Counts::next_small, u32(idle)));
         CSA_TRY(set_count(&Build_Counts::large, 0));
         CSA_TRY(launch_refine_by_ranks(ctx, front + idle, ns, secs, isa, sa, other, counts));
+        Build_Counts c;
         if(nl)
         {
             int in_alt = 0;
-            CSA_TRY(csa_sort_pairs(ctx, reinterpret_cast<uint64_t*>(keysA), reinterpret_cast<uint64_t*>(keysB), posA, posB, 4, nl, 0, sec_bits + prim_bits, sort_ws, L.sort_ws, &in_alt));
+            CSA_TRY(csa_sort_pairs(ctx, reinterpret_cast<uint64_t*>(keysA), reinterpret_cast<uint64_t*>(keysB), pos, pos_other, 4, nl, 0, sec_bits + prim_bits, sort_ws, L.sort_ws, &in_alt));
             u64* const ks = in_alt ? keysB : keysA;
             u64* const upd = in_alt ? keysA : keysB;
-            u32* const pn = in_alt ? posA : posB;
+            if(in_alt) std::swap(pos, pos_other);       // pos: the sorted positions; the tied ones go to the other array
             CSA_CUDA(ctx, cudaMemsetAsync(ctx->d_scalars, 0, 8, ctx->stream));
             const Slot_Map whole{nullptr, nullptr, 0, 0};
-            CSA_TRY(launch_rank_and_compact(ctx, ks, in_alt ? posB : posA, nl, sec_bits, 0, iv, whole, sa, head, pn, ctx->d_scalars, scratch, upd, false));
+            CSA_TRY(launch_rank_and_compact(ctx, ks, pos, nl, sec_bits, 0, iv, whole, sa, head, pos_other, ctx->d_scalars, scratch, upd, false));
+            std::swap(pos, pos_other);
             CSA_TRY(apply_updates_in_address_order(ctx, isa, upd, ks, nl, bits_for(n - 1), sort_ws, L.sort_ws));
-            CSA_TRY(launch_split_by_size(ctx, head, pn, nl, ctx->d_scalars, other, n, counts, scratch));
+            CSA_TRY(launch_count_by_size(ctx, head, nl, ctx->d_scalars, counts, scratch));
         }
-        Build_Counts c;
         CSA_TRY(read_counts(c));
-        std::swap(front, other);
         small = c.next_small; large = c.large;
+        in_arrays = nl != 0 && large != 0 && 2 * h <= MAX_SMALL_H && u64(c.now_small) * 8 <= u64(c.now_small) + c.large;
+        if(in_arrays) { small -= c.now_small; large += c.now_small; }
+        else if(nl) CSA_TRY(launch_split_by_size(ctx, head, pos, nl, ctx->d_scalars, other, n, scratch));
+        std::swap(front, other);
         return CSA_OK;
     }
 };
@@ -225,7 +244,17 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
         CSA_TRY(b.more_memory());
         CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));
         u64 idle = b.large ? b.small : 0;               // in small groups already, hence ordered up to `depth`
-        u64 h = b.large ? depth0 : depth;
+        u64 h = depth;
+        if(b.large)
+        {
+            // A large group was not compared in the text: it shares the whole symbols of generation 0's key. Frequent symbols, of which large groups
+            // are made, have short code words, so that is more than what any key holds (depth0 = 1): one symbol repeated 2^24 times starts at 25
+            // and takes 22 generations instead of 26.
+            CSA_TRY(launch_large_depth(ctx, b.large_list(b.front), b.large, T, n, b.tab.code, b.ps.key_bits, b.counts));
+            CSA_TRY(b.read_counts(c));
+            if(c.large_depth < depth0 || c.large_depth > u64(b.ps.key_bits)) return csa_fail(ctx, CSA_E_DEVICE, "build: the large groups' depth is out of range");
+            h = std::min<u64>(c.large_depth, depth);
+        }
         while(b.small || b.large)
         {
             const u64 active = b.small + b.large;
@@ -299,7 +328,8 @@ int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tab
     const Slot_Map whole{nullptr, nullptr, 0, 0};
     CSA_TRY(launch_rank_and_compact(ctx, ks, in_alt ? posB : posA, M, 32, 0, none, whole, sa, head, in_alt ? posA : posB, ctx->d_scalars, b.scratch, in_alt ? keysA : keysB, true));
     CSA_TRY(set_build_count(ctx, &counts->next_small, c.small));
-    CSA_TRY(launch_split_by_size(ctx, head, in_alt ? posA : posB, M, ctx->d_scalars, front, n, counts, b.scratch));
+    CSA_TRY(launch_count_by_size(ctx, head, M, ctx->d_scalars, counts, b.scratch));
+    CSA_TRY(launch_split_by_size(ctx, head, in_alt ? posA : posB, M, ctx->d_scalars, front, n, b.scratch));
     CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
     CSA_TRY(set_build_count(ctx, &counts->next_small, 0));
     return set_build_count(ctx, &counts->oversize, 0);

@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                 __syncthreads();
                 if(tid == 0) start[m] = u16(m);
             }
-            bool by_network = __syncthreads_or(longest > LONG_BIN);
+            const bool by_network = __syncthreads_or(longest > LONG_BIN);
             #pragma unroll
             for(int i = 0; i < LOCAL_ITEMS; ++i)
             {

@@ -23,6 +23,8 @@ struct Build_Counts
     u32 partitions;     // contiguous ranges of the suffix array, at most as many as asked for, that the first split's buckets form
     u32 max_partition;  // suffixes of the largest
     u32 medium;         // children that fit the local sort's larger blocks only
+    u32 now_small;      // entries that the last count by size found in small groups
+    u32 large_depth;    // symbols that the suffixes of a large group share at least after the initial sort (launch_large_depth)
 };
 static_assert(sizeof(Build_Counts) <= (CSA_STATUS_WORD - CSA_COUNTS_WORD) * 8, "the counters lie before the status word");
 

@@ -27,10 +27,16 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 // counts->next_small entries that are there.
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts);
 
-// Splits a list (heads, positions) of groups of any size into small groups (behind the counts->next_small entries at the front
-// of next) and large ones (in front of the counts->large entries at the back of next, which holds cap entries). The list holds
-// *count_dev entries, at most `most`. scratch: 2 words per RANK_TILE entries.
-int launch_split_by_size(csa_ctx* ctx, const u32* head, const u32* pos, u64 most, const u64* count_dev, u64* next, u64 cap, Build_Counts* counts, u32* scratch);
+// A list of groups of any size (heads, positions; *count_dev entries, at most `most`), group by group: how many of its entries are in small groups
+// (counts->now_small) and where each tile's go; counts->next_small and counts->large are advanced by the two kinds. scratch: 2 words per
+// RANK_TILE entries, for the call below.
+int launch_count_by_size(csa_ctx* ctx, const u32* head, u64 most, const u64* count_dev, Build_Counts* counts, u32* scratch);
+// Writes what was counted: small groups behind the entries that were at the front of next, large ones in front of those at its back; next
+// holds cap entries.
+int launch_split_by_size(csa_ctx* ctx, const u32* head, const u32* pos, u64 most, const u64* count_dev, u64* next, u64 cap, u32* scratch);
+// counts->large_depth = how many symbols the suffixes of every group of the list share at least, as generation 0 leaves it (groups of one and the
+// same key of key_bits bits, side by side).
+int launch_large_depth(csa_ctx* ctx, const u64* list, u64 count, const u16* T, u64 n, const u32* code, int key_bits, Build_Counts* counts);
 // Heads and positions of the entries of a list.
 int launch_unpack_list(csa_ctx* ctx, const u64* list, u64 count, u32* head, u32* pos);
 

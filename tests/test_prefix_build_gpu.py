@@ -75,6 +75,33 @@ def test_texts_of_the_rarer_paths(ctx, oracle, n, kind):
     assert st.n == len(T) and 1 <= st.partitions <= 8 and 0 < st.max_partition <= len(T)
 
 
+@pytest.mark.parametrize("shared", [6, 30, 90])
+@pytest.mark.parametrize("spread", [1, 40])
+def test_groups_about_as_large_as_the_small_ones_may_be(ctx, oracle, shared, spread):
+    """Phrases that begin alike and then fall apart into groups of 1 to 2049 members, around the 256 up to which a group is small, at any place
+    of a tile of the list: most are found in one large group first, and the stretch that they share is longer or shorter than what is
+    compared in the text."""
+    rng = np.random.default_rng(shared + spread)
+    sizes = [1, 2, 31, 32, 33, 254, 255, 256, 257, 258, 511, 512, 513, 2047, 2048, 2049] + [int(x) for x in rng.integers(200, 300, spread)]
+    begin = rng.integers(1, 60000, shared)
+    pieces = []
+    for c in sizes:
+        end = rng.integers(1, 60000, 5)
+        pieces += [np.concatenate([begin, end, rng.integers(1, 60000, int(rng.integers(1, 4)))]) for _ in range(c)]
+    rng.shuffle(pieces)
+    st = _check(ctx, oracle, np.concatenate(pieces))
+    assert st.generations >= 2, "no group was ranked"
+
+
+@pytest.mark.parametrize("n", [300, 5000, 70_001])
+def test_nothing_but_zeros_and_zeros_behind_a_text(ctx, oracle, n):
+    """The padding behind a text is zeros as well: large groups whose members end inside the symbols that they share."""
+    _check(ctx, oracle, np.zeros(n))
+    T = np.random.default_rng(n).integers(0, 2, n)
+    T[n // 2:] = 0
+    _check(ctx, oracle, T)
+
+
 def _pairs_text(n, medium, oversize, seed):
     """Random symbols, and pairs of symbols that stand together many times: a child of 4097 to 8192 suffixes for each of the `medium`
     pairs, one of more than 8192 for each of the `oversize` ones, spread over the whole array."""
