@@ -100,10 +100,19 @@ struct Build
         return cv.ok ? CSA_OK : csa_fail(ctx, CSA_E_NOMEM, "build: workspace too small");
     }
 
+    // The few children of an ordinary text take buffers of their size; ranking, if it comes to that, asks for its own then.
     int sort_oversize(const Build_Counts& c)
     {
-        CSA_TRY(more_memory());
-        return sort_oversize_children(ctx, ps, tab, c, n, front, other, sa, counts, {sort_ws, L.sort_ws, scratch, work, L.work});
+        const u64 few = n / OVERSIZE_SHARE;
+        if(c.oversize_records > few)
+        {
+            CSA_TRY(more_memory());
+            return sort_oversize_children(ctx, ps, tab, c, n, front, other, sa, counts, {sort_ws, L.sort_ws, scratch, work, L.work});
+        }
+        const size_t bytes = oversize_buffers_bytes(few);
+        void* p = nullptr;
+        CSA_TRY(csa_aux(ctx, bytes, &p));
+        return sort_oversize_children(ctx, ps, tab, c, n, front, other, sa, counts, oversize_buffers(p, few));
     }
 
     // One generation of prefix doubling: the suffixes of every group ordered by the ranks of those h symbols further on. The first
@@ -305,6 +314,13 @@ int check_build_args(csa_ctx* ctx, const void* text, u64 n, u32 p, const void* o
 
 size_t oversize_scratch_bytes(u64 records) { return align256(div_up(records, RANK_TILE) * 3 * 4 + 256); }
 size_t oversize_work_bytes(u64 records) { return align256(records * 12) + 16 * 256; }
+size_t oversize_buffers_bytes(u64 records) { return align256(csa_sort_workspace_bytes(records)) + oversize_scratch_bytes(records) + oversize_work_bytes(records); }
+Oversize_Buffers oversize_buffers(void* at, u64 records)
+{
+    const size_t sort_bytes = align256(csa_sort_workspace_bytes(records)), scratch_bytes = oversize_scratch_bytes(records);
+    u8* const p = static_cast<u8*>(at);
+    return {p, sort_bytes, reinterpret_cast<u32*>(p + sort_bytes), p + sort_bytes + scratch_bytes, oversize_work_bytes(records)};
+}
 
 int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& tab, const Build_Counts& c, u64 n, u64* front, u64* other, u32* sa, Build_Counts* counts,
                            const Oversize_Buffers& b)

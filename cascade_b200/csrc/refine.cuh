@@ -54,5 +54,10 @@ struct Oversize_Buffers
 };
 size_t oversize_scratch_bytes(u64 records);
 size_t oversize_work_bytes(u64 records);
+// The same carved from one piece of oversize_buffers_bytes, for up to `records` of them.
+size_t oversize_buffers_bytes(u64 records);
+Oversize_Buffers oversize_buffers(void* at, u64 records);
+// An ordinary text has a few suffixes in a thousand in such children; a share of up to one in this many is room enough for them.
+constexpr u64 OVERSIZE_SHARE = 64;
 int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& tab, const Build_Counts& c, u64 n, u64* front, u64* other, u32* sa, Build_Counts* counts,
                            const Oversize_Buffers& b);

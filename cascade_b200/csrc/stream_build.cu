@@ -842,7 +842,6 @@ namespace
 // about 0.9 ns a suffix over PCIe: up to this many parts the direct way moves less.
 constexpr u64 DIRECT_MAX_PARTS = 64;
 constexpr u64 DIRECT_MIN = 1 << 14;
-constexpr u64 DIRECT_OVERSIZE = 64;         // up to this share of a part's suffixes may lie in children that go through the radix sort
 
 }   // namespace
 
@@ -858,7 +857,8 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     const Prefix_Sort ps = prefix_sort_part_plan(n);
     const u64 most = n < part_suffixes ? n : part_suffixes;
     const size_t rec = align_up256(most * 8), slots = align_up256(most * 4 + 64), out_bytes = align_up256(most * 5 + CSA_SA_PAD_BYTES);
-    const size_t total = align_up256(prefix_sort_table_bytes(ps)) + 2 * rec + slots + 2 * out_bytes + 4096;
+    const size_t over_bytes = align_up256(oversize_buffers_bytes(most / OVERSIZE_SHARE));          // children that go through the radix sort
+    const size_t total = align_up256(prefix_sort_table_bytes(ps)) + 2 * rec + slots + 2 * out_bytes + over_bytes + 4096;
     void* ws = nullptr;
     CSA_TRY(csa_arena(ctx, total, &ws));
     Carver cv(ws, total);
@@ -867,6 +867,7 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     u64* const recB = cv.take<u64>(rec / 8);
     u32* const sa = cv.take<u32>(slots / 4);
     u8* const out[2] = {cv.take<u8>(out_bytes), cv.take<u8>(out_bytes)};
+    u8* const over_at = cv.take<u8>(over_bytes);
     if(!cv.ok || !prefix_sort_carve(cv, ps, tab)) return csa_fail(ctx, CSA_E_NOMEM, "streamed build: workspace too small");
     CSA_TRY(csa_lanes(ctx));
     Build_Counts* const counts = reinterpret_cast<Build_Counts*>(ctx->d_scalars + CSA_COUNTS_WORD);
@@ -897,8 +898,6 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     const cudaStream_t copy_stream = ctx->lane[0];
     const cudaEvent_t packed = ctx->lane_event[0], copied[2] = {ctx->lane_event[1], ctx->lane_event[2]};
     struct Drain { cudaStream_t s; ~Drain() { cudaStreamSynchronize(s); } } drain{copy_stream};       // no copy outlives the call, nor runs under the general way
-    Dev_Buffer extra;           // for children that go through the radix sort
-    size_t extra_bytes = 0;
     u64 active = 0;
     u32 rounds = 0;
     for(u32 u = 0; u < parts; ++u)
@@ -911,18 +910,9 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
         CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
         Build_Counts c;
         CSA_TRY(read_build_counts(ctx, S, c));
-        if(c.oversize && c.oversize_records <= S / DIRECT_OVERSIZE)
+        if(c.oversize && c.oversize_records <= S / OVERSIZE_SHARE)
         {
-            const u64 M = c.oversize_records;
-            const size_t sort_bytes = align_up256(csa_sort_workspace_bytes(M)), scratch_bytes = align_up256(oversize_scratch_bytes(M)), work_bytes = oversize_work_bytes(M);
-            if(extra_bytes < sort_bytes + scratch_bytes + work_bytes)
-            {
-                if(extra.p) { CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream)); cudaFree(extra.p); extra.p = nullptr; }
-                extra_bytes = 2 * (sort_bytes + scratch_bytes + work_bytes);
-                CSA_TRY(extra.alloc(ctx, extra_bytes));
-            }
-            u8* const at = static_cast<u8*>(extra.p);
-            CSA_TRY(sort_oversize_children(ctx, ps, tab, c, S, list, next, sa, counts, {at, sort_bytes, reinterpret_cast<u32*>(at + sort_bytes), at + sort_bytes + scratch_bytes, work_bytes}));
+            CSA_TRY(sort_oversize_children(ctx, ps, tab, c, S, list, next, sa, counts, oversize_buffers(over_at, most / OVERSIZE_SHARE)));
             CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
             CSA_TRY(read_build_counts(ctx, S, c));
         }

@@ -133,3 +133,30 @@ def test_blocks_that_go_on_behind_a_child_left_to_others(ctx, oracle):
         sa, st = api.build_sa_streamed(ctx, Tp, n, 8)
         assert np.array_equal(sa[:5 * n], want)
         assert st.sort_passes > 2 and st.generations == 1, "not straight from the text, or no child went through the radix sort"
+
+
+def _held_by_a_build(T):
+    """Device memory that a new context holds after one build, and the build's statistics."""
+    from cascade_b200 import api
+    n = len(T)
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    out = torch.zeros(5 * n + api.SA_PAD_BYTES, dtype=torch.uint8, device="cuda")
+    held = 0
+    for _ in range(2):              # the first build loads the kernels' code, too
+        torch.cuda.empty_cache()
+        c = api.Context(0)
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        _, st = api.build_sa(c, Td, n, 8, out=out)
+        torch.cuda.synchronize()
+        held = free - torch.cuda.mem_get_info()[0]
+        c.close()
+    return held, st
+
+
+def test_a_few_oversize_children_take_no_ranking_memory():
+    """20 bytes a suffix and a sixteenth of head-room, tables, and buffers for one suffix in 64: not the 16 bytes a suffix that ranks need."""
+    T = _pairs_text(21_000_003, 230, 24, 5)
+    held, st = _held_by_a_build(T)
+    assert st.sort_passes > 2, "no child went through the radix sort"
+    assert held < 24 * len(T), held / len(T)
