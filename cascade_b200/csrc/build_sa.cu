@@ -355,7 +355,7 @@ extern "C" size_t csa_build_device_bytes(uint64_t n, uint32_t p)
 {
     (void)p;
     const Build_Layout L = layout_for(n);
-    return L.total + L.more;
+    return L.total + L.more + CSA_ALLOC_SLACK;
 }
 
 extern "C" int csa_build_sa(csa_ctx* ctx, const uint16_t* text, uint64_t n, uint32_t p, uint64_t seed, uint8_t* sa40, csa_build_stats* stats)
@@ -364,9 +364,10 @@ extern "C" int csa_build_sa(csa_ctx* ctx, const uint16_t* text, uint64_t n, uint
     if((reinterpret_cast<uintptr_t>(text) & 15) || (reinterpret_cast<uintptr_t>(sa40) & 15))
         return csa_fail(ctx, CSA_E_INVALID, "build: text and output must be 16-byte aligned");
     CSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    const size_t bytes = layout_for(n).total;
+    const Build_Layout L = layout_for(n);
+    const size_t bytes = L.total;
     void* ws = nullptr;
-    CSA_TRY(csa_arena(ctx, bytes, &ws));
+    CSA_TRY(csa_arena(ctx, bytes, &ws, L.more));
     return build_core(ctx, text, n, p, seed, sa40, stats, ws, bytes);
 }
 
@@ -374,7 +375,8 @@ extern "C" int csa_build_sa_host(csa_ctx* ctx, const uint16_t* text_host, uint64
 {
     CSA_TRY(check_build_args(ctx, text_host, n, p, sa40_host));
     CSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    const size_t core = layout_for(n).total;
+    const Build_Layout L = layout_for(n);
+    const size_t core = L.total;
     const size_t text_bytes = align256((n + CSA_TEXT_PAD) * 2), out_bytes = align256(5 * n + CSA_SA_PAD_BYTES);
     const u16* text_at = text_host;
     if(n >= HOST_PARTS_MIN)
@@ -405,7 +407,7 @@ extern "C" int csa_build_sa_host(csa_ctx* ctx, const uint16_t* text_host, uint64
     }
     const size_t bytes = core + text_bytes + out_bytes;
     void* ws = nullptr;
-    CSA_TRY(csa_arena(ctx, bytes, &ws));
+    CSA_TRY(csa_arena(ctx, bytes, &ws, L.more));
     u8* base = static_cast<u8*>(ws);
     u16* text_dev = reinterpret_cast<u16*>(base);
     u8* out_dev = base + text_bytes;

@@ -120,8 +120,10 @@ struct On_Stream
     On_Stream& operator=(const On_Stream&) = delete;
 };
 
-// Returns in *out a scratch pointer of at least `bytes` bytes from the context's grow-only arena.
-int csa_arena(csa_ctx* ctx, size_t bytes, void** out);
+// Returns in *out a scratch pointer of at least `bytes` bytes from the context's grow-only arena. aux_later: what the caller may yet ask of
+// the second buffer; the arena's head-room is not taken from that.
+constexpr size_t CSA_ALLOC_SLACK = size_t(2) << 21;         // two allocations, each rounded up to 2 MiB by the driver
+int csa_arena(csa_ctx* ctx, size_t bytes, void** out, size_t aux_later = 0);
 int csa_aux(csa_ctx* ctx, size_t bytes, void** out);
 int csa_host_aux(csa_ctx* ctx, size_t bytes, void** out);
 

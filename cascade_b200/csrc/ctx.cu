@@ -88,7 +88,7 @@ int csa_lanes(csa_ctx* ctx)
     return CSA_OK;
 }
 
-int csa_arena(csa_ctx* ctx, size_t bytes, void** out)
+int csa_arena(csa_ctx* ctx, size_t bytes, void** out, size_t aux_later)
 {
     if(bytes > ctx->arena_bytes)
     {
@@ -96,7 +96,9 @@ int csa_arena(csa_ctx* ctx, size_t bytes, void** out)
         if(ctx->arena) { cudaFree(ctx->arena); ctx->arena = nullptr; ctx->arena_bytes = 0; }
         // A little head-room, so that a slightly larger request later (another deal of the partitions, say) does not regrow the
         // arena: other GPUs may still hold a mapping of it, and its memory is not given back before they let go.
-        const size_t want = bytes + bytes / 16;
+        size_t want = bytes + bytes / 16;
+        size_t free_bytes = 0, total_bytes = 0;
+        if(aux_later > ctx->aux_bytes && cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess && free_bytes + ctx->aux_bytes < want + aux_later + CSA_ALLOC_SLACK) want = bytes;
         cudaError_t e = cudaMalloc(&ctx->arena, want);
         if(e == cudaSuccess) bytes = want;
         else { cudaGetLastError(); e = cudaMalloc(&ctx->arena, bytes); }

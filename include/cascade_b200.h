@@ -171,7 +171,8 @@ typedef struct csa_build_stats
     uint64_t file_bytes_written;
 } csa_build_stats;
 
-/* Device bytes that csa_build_sa allocates for a text of n symbols in p partitions (beyond text and output). */
+/* Device bytes that csa_build_sa allocates at most for a text of n symbols in p partitions (beyond text and output): 36 a symbol and
+ * tables. A text without long repeats takes 20 a symbol; with more memory free, head-room for a later build is added. */
 size_t csa_build_device_bytes(uint64_t n, uint32_t p);
 /* Builds the suffix array of text_dev[0, n) (n < 2^32 - 2^26; CSA_TEXT_PAD zero symbols must follow the text)
  * into sa40_dev as 5-byte little-endian entries in numeric symbol order with shorter suffixes first

@@ -160,3 +160,27 @@ def test_a_few_oversize_children_take_no_ranking_memory():
     held, st = _held_by_a_build(T)
     assert st.sort_passes > 2, "no child went through the radix sort"
     assert held < 24 * len(T), held / len(T)
+
+
+def test_a_build_that_ranks_fits_what_it_says_it_needs(ctx):
+    """With no more device memory free than csa_build_device_bytes, a text whose repeats need ranks is built: the first buffer's head-room is not
+    taken from what the ranks need later."""
+    from cascade_b200 import api
+    n = 120_000_007
+    piece = torch.randint(1, 60000, (1000,), dtype=torch.int32, device="cuda", generator=torch.Generator(device="cuda").manual_seed(2)).to(torch.int16)
+    Td = torch.zeros(n + api.TEXT_PAD, dtype=torch.int16, device="cuda")
+    Td[:n] = piece.repeat(n // 1000 + 1)[:n]
+    Td = Td.view(torch.uint16)
+    out = torch.zeros(5 * n + api.SA_PAD_BYTES, dtype=torch.uint8, device="cuda")
+    _held_by_a_build(np.resize(np.arange(1, 1000, dtype=np.uint16), 300_000))        # the kernels' code is on the device
+    c = api.Context(0)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    need = c.L.csa_build_device_bytes(n, 8) + (16 << 20)
+    rest = torch.empty(torch.cuda.mem_get_info()[0] - need, dtype=torch.uint8, device="cuda")
+    _, st = api.build_sa(c, Td, n, 8, out=out)
+    assert st.generations > 10, "no ranks were needed"
+    c.close()
+    del rest
+    torch.cuda.empty_cache()
+    assert api.validate_sa(ctx, Td, n, out)["ok"]
