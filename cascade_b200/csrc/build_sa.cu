@@ -397,7 +397,6 @@ extern "C" int csa_build_sa_host(csa_ctx* ctx, const uint16_t* text_host, uint64
         if(done)
         {
             st.ms_total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
-            st.host_parts = 0;          // no lists of parts are kept
             st.kernel_launches = ctx->counters[0] - launches_before;
             st.sort_passes = ctx->counters[1] - passes_before;
             st.sort_records = ctx->counters[2] - records_before;

@@ -952,8 +952,7 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     bs.generations = rounds;
     bs.ms_partition = ms_counted;
     bs.ms_gen0 = ms_since(t_start) - ms_counted;
-    bs.host_parts = parts;
-    done = true;
+    done = true;                // no lists of parts were kept: host_parts and file_parts stay 0
     return CSA_OK;
 }
 

@@ -166,7 +166,7 @@ typedef struct csa_build_stats
                                          * generation 0 (positions, keys, first ranks), [t] = doubling generation t (rank requests,
                                          * responses and updates) */
     uint32_t host_parts;        /* csa_build_sa_tiered: parts whose lists stayed in host memory */
-    uint32_t file_parts;        /*   and parts whose lists went through files */
+    uint32_t file_parts;        /*   and parts whose lists went through files; both 0 where the parts were ordered straight from the text */
     uint64_t file_bytes_read;   /*   bytes read from and written to those files */
     uint64_t file_bytes_written;
 } csa_build_stats;

@@ -320,4 +320,6 @@ def test_parts_straight_from_the_text(ctx, oracle, n, part_suffixes, tail):
         T[n // 3:n // 3 + 3000] = np.resize([65535, 65534, 65535], 3000)
     sa, st = api.build_sa_streamed(ctx, _padded(T), n, 16, part_suffixes=part_suffixes)
     assert np.array_equal(sa[:5 * n], oracle.build_sa40(T)[:5 * n])
-    assert 1 <= st.partitions <= 16 and 0 < st.max_partition <= n and st.host_parts >= 1
+    assert 1 <= st.partitions <= 16 and 0 < st.max_partition <= n
+    straight = part_suffixes != 1500 and tail != "period_in_the_last_part"      # no lists of parts are kept then
+    assert st.file_parts == 0 and (st.host_parts == 0) == straight
