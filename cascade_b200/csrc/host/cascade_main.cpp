@@ -126,10 +126,9 @@ int main(int argc, char** argv)
         csa_build_stats st{};
         const int rc = by_parts ? csa_build_sa_tiered(ctx, T, n, p, 0, SA, &tiers, &st) : csa_build_sa_host(ctx, T, n, p, 0, SA, &st);
         if(rc != CSA_OK) { std::fprintf(stderr, "error: build failed (%d): %s\n", rc, csa_last_error(ctx)); return EXIT_FAILURE; }
-        if(by_parts && st.host_parts + st.file_parts == 0)
-            std::fprintf(stderr, "Built part by part (%s): every part straight from the text.\n", forced ? "GPU_SACA_FORCE_SPILL" : "the resident build does not fit the device");
-        else if(by_parts) std::fprintf(stderr, "Built part by part (%s): the lists of %u parts in host memory, of %u parts in files (%.2f GB read, %.2f GB written).\n",
-                                  forced ? "GPU_SACA_FORCE_SPILL" : "the resident build does not fit the device", st.host_parts, st.file_parts,
+        if(by_parts) std::fprintf(stderr, "Built part by part (%s): %sthe lists of %u parts in host memory, of %u parts in files (%.2f GB read, %.2f GB written).\n",
+                                  forced ? "GPU_SACA_FORCE_SPILL" : "the resident build does not fit the device",
+                                  st.host_parts + st.file_parts == 0 ? "every part straight from the text, " : "", st.host_parts, st.file_parts,
                                   double(st.file_bytes_read) / 1e9, double(st.file_bytes_written) / 1e9);
         std::fprintf(stderr, "Built the suffix array: %u partitions (largest %llu), %u doubling generations, %llu digit passes.\n", st.partitions,
                      (unsigned long long)st.max_partition, st.generations, (unsigned long long)st.sort_passes);
