@@ -116,7 +116,7 @@ struct Build
     }
 
     // One generation of prefix doubling: the suffixes of every group ordered by the ranks of those h symbols further on. The first
-    // `idle` entries of the list share 2 h symbols already and stay as they are.
+    // `idle` entries of the list share more than h symbols already and stay as they are.
     //
     // What is left of the large groups is counted by size. Where few of them have become small (up to one in eight), they all stay in the arrays
     // that the ranking left, and the radix sort takes the small ones once more: to write the two lists and read them again costs 40 bytes a
@@ -253,7 +253,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
         CSA_TRY(b.more_memory());
         CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));
         u64 idle = b.large ? b.small : 0;               // in small groups already, hence ordered up to `depth`
-        u64 h = depth;
+        u64 shared = depth;                             // symbols that all others' groups share at least
         if(b.large)
         {
             // A large group was not compared in the text: it shares the whole symbols of generation 0's key. Frequent symbols, of which large groups
@@ -262,19 +262,22 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             CSA_TRY(launch_large_depth(ctx, b.large_list(b.front), b.large, T, n, b.tab.code, b.ps.key_bits, b.counts));
             CSA_TRY(b.read_counts(c));
             if(c.large_depth < depth0 || c.large_depth > u64(b.ps.key_bits)) return csa_fail(ctx, CSA_E_DEVICE, "build: the large groups' depth is out of range");
-            h = std::min<u64>(c.large_depth, depth);
+            shared = std::min<u64>(c.large_depth, depth);
         }
+        // Ranks tell `shared` symbols from any step of up to as many: doubling takes the longest step. Above 2^31 suffixes a step may be too long for
+        // a sort key of two ranks (n - 1 + h has to fit beside bits_for(n - 1) bits in 64); steps of the longest that fits go on from there.
+        const u64 longest_step = (u64(1) << (64 - bits_for(n - 1))) - n;
         while(b.small || b.large)
         {
             const u64 active = b.small + b.large;
-            if(h >= depth) idle = 0;
-            if(idle == b.small && !b.large) { h = depth; continue; }
+            if(idle && (shared >= depth || (idle == b.small && !b.large))) { shared = depth; idle = 0; }       // they join when the others have come as far
             if(gen < 48) st.active_per_gen[gen] = active;
             ++gen;
+            const u64 h = std::min(shared, longest_step);
             CSA_TRY(b.generation(h, idle));
             if(debug) std::fprintf(stderr, "[csa] generation %u: h=%llu active %llu -> %llu (%llu in large groups)\n", gen, h, active, b.small + b.large, b.large);
-            if(h > (u64(1) << 40)) return csa_fail(ctx, CSA_E_DEVICE, "build: doubling did not terminate");
-            h = h < depth && 2 * h > depth ? depth : 2 * h;     // the idle groups join when exactly their depth is reached
+            shared += h;
+            if(shared > 2 * n + 2 * depth) return csa_fail(ctx, CSA_E_DEVICE, "build: doubling did not terminate");
         }
     }
     st.generations = gen;

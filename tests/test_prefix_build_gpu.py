@@ -184,3 +184,29 @@ def test_a_build_that_ranks_fits_what_it_says_it_needs(ctx):
     del rest
     torch.cuda.empty_cache()
     assert api.validate_sa(ctx, Td, n, out)["ok"]
+
+
+def test_repeats_of_two_thousand_million_symbols_above_2_31_positions(ctx):
+    """A text of 2.26e9 symbols with a period of 1.5e8: its suffixes share up to 2.1e9 symbols, and a step of 61 * 2^25, the next after one that tells
+    2.05e9 of them, no longer fits a sort key of two ranks."""
+    from cascade_b200 import api
+    n, period = 2_260_000_000, 150_000_000
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 130e9:
+        pytest.skip("needs 130 GB of device memory")
+    T = torch.zeros(n + api.TEXT_PAD, dtype=torch.int16, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(3)
+    for at in range(0, period, 1 << 24):
+        k = min(1 << 24, period - at)
+        T[at:at + k] = torch.randint(-(1 << 15), 1 << 15, (k,), device="cuda", dtype=torch.int32, generator=g).to(torch.int16)
+    at = period
+    while at < n:               # of the text so far: always from a multiple of the period
+        k = min(at, n - at)
+        T[at:at + k] = T[:k]
+        at += k
+    T = T.view(torch.uint16)
+    c = api.Context(0)
+    out, st = api.build_sa(c, T, n, 8)
+    c.close()
+    assert st.generations > 20
+    assert api.validate_sa(ctx, T, n, out)["ok"]
