@@ -99,8 +99,7 @@ def test_config1_16m_tokens_single_partition(ctx, oracle):
 
 
 def test_just_above_16m_tokens_ranks_reach_the_inverse_array_through_buckets(ctx, oracle):
-    """Above 2^24 positions the rank updates are bucketed by the top 8 position bits before they are applied (generation 0 by
-    the counting-free bucket kernel, later generations by a digit pass); the last bucket is ragged here."""
+    """Above 2^24 positions: a text whose ties are all settled by its symbols, so that no inverse array is made (the text below has one)."""
     from cascade_b200 import api
     n = (1 << 24) + (1 << 20) + 13
     Td = api.gen_corpus_device(ctx, n, 7, 256)
@@ -109,6 +108,46 @@ def test_just_above_16m_tokens_ranks_reach_the_inverse_array_through_buckets(ctx
     Th = Td.cpu().view(torch.int16).numpy().view(np.uint16)
     want = oracle.build_sa40(Th[:n])
     assert np.array_equal(sa.cpu().numpy()[:5 * n], want[:5 * n])
+
+
+@pytest.mark.parametrize("n", [(1 << 24) + 1, (1 << 24) + (1 << 20) + 13, (1 << 25) + 77])
+def test_inverse_array_above_16m_tokens(ctx, n):
+    """Above 2^24 positions the inverse array is made through 256 buckets of positions (the last one ragged, or of a single one), from the
+    finished entries and from small and large groups of tied suffixes; later ranks go there by a digit pass."""
+    from cascade_b200 import api
+    rng = np.random.default_rng(n)
+    docs = rng.integers(1, 60000, (64, 1500)).astype(np.uint16)
+    T = docs[np.concatenate([rng.integers(1, 64, n // 1500 + 1 - 600), np.zeros(600, np.int64)])[rng.permutation(n // 1500 + 1)]].ravel()[:n]
+    hit = rng.random(n) < 0.0005
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    T[-(n // 50):] = rng.integers(1, 60000, n // 50)              # and entries that are finished from the start
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    sa, st = api.build_sa(ctx, Td, n, 16)
+    assert st.generations >= 8 and st.sort_passes > 20, "no large groups were ranked"
+    assert api.validate_sa(ctx, Td, n, sa)["ok"]
+
+
+@pytest.mark.parametrize("kind", ["zipf", "repeat_in_the_first_part", "repeat_in_the_last_part"])
+def test_host_build_in_parts(ctx, oracle, kind):
+    """From 2^23 symbols on a host build goes part by part, straight from the text, and a text with long repeats falls back to the whole build, after
+    a part of the array or nothing of it has been written; twice on one context, with buffers that grow in between."""
+    from cascade_b200 import api
+    own = api.Context(0)
+    for n in ((1 << 23) - 1, 1 << 23, (1 << 23) + 12345, 20_000_001):
+        T = api.gen_corpus_host(n, n, 512)
+        if kind != "zipf":
+            end = [0, 1, 0] if kind == "repeat_in_the_first_part" else [65535, 65534, 65535]
+            T[n // 3:n // 3 + 100_000] = np.resize(np.array(end, np.uint16), 100_000)
+        Td = torch.from_numpy(T.view(np.int16)).cuda().view(torch.uint16)
+        want, _ = api.build_sa(ctx, Td, n, 7)
+        assert api.validate_sa(ctx, Td, n, want)["ok"]
+        want = want[:5 * n].cpu().numpy()
+        for _ in range(2):
+            sa, st = api.build_sa_host(own, T, n, 7)
+            assert np.array_equal(sa[:5 * n], want)
+            assert st.n == n and 1 <= st.partitions <= 7 and 0 < st.max_partition <= n and st.host_parts == 0 and st.file_parts == 0
+            assert (st.ms_output == 0) == (kind == "zipf" and n >= 1 << 23), "not the way that was meant"      # a whole build has an output phase
+    own.close()
 
 
 def test_partition_count_does_not_change_the_result(ctx):
