@@ -44,7 +44,7 @@ Build_Layout layout_for(u64 n)
 }
 
 // From here on a host build is done in four parts, so that the array's copy to the host (9.1 of the 15.6 ms of 1e8 suffixes) runs under
-// the sorting: 13.7 ms (2e9: 270 ms, 263 of them copies). Below it the parts' launches cost what the overlap gives.
+// the sorting: 13.7 to 14.4 ms (2e9: 0.27 to 0.33 s by box, 0.26 of them copies). Below it the parts' launches cost what the overlap gives.
 constexpr u64 HOST_PARTS_MIN = u64(1) << 23;
 constexpr u64 SMALL_BUILD = u64(1) << 22;       // up to here the output is packed before the host knows whether ties are left
 
