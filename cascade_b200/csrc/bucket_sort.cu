@@ -1,0 +1,329 @@
+// The stable sort of csa_sort_pairs by its top bits first, for keys whose top bits are evenly spread: the records are split into buckets
+// of about a thousand by the top 8 to 15 sorted bits with one or two of radix_sort.cu's digit passes (stable, low digit first), and every
+// bucket is then finished inside one block. A record moves two or three times, where a pass per 8 bits moves it up to eight
+// times (31.25 M 64-bit keys with 4-byte values, whole calls: 2.22 ms, this way 1.14 ms; 10^6: 278 us, 149 us; 1000, in one block: 176 us, 71 us). Nothing is estimated: the buckets are counted
+// exactly before anything moves, and keys with a bucket that no block holds go through all their digit passes as before.
+// A list that fits one block at all is a single bucket and takes one launch.
+#include "common.cuh"
+#include "sort.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+namespace
+{
+
+// ---- the buckets' counts -----------------------------------------------------------------------------------------------------
+
+constexpr int COUNT_BLOCK = 1024, COUNT_UNROLL = 4;
+
+// One read of the keys; a block counts in shared memory (32 bits a counter, at most 128 KB, as many blocks as SMs). Bound by the read.
+__global__ void __launch_bounds__(COUNT_BLOCK) bucket_counts_kernel(const u64* __restrict__ keys, const u64 n, const int shift, const int bits, u32* __restrict__ counts)
+{
+    extern __shared__ u32 cnt[];
+    const u32 buckets = 1u << bits, mask = buckets - 1;
+    for(u32 i = threadIdx.x; i < buckets; i += COUNT_BLOCK) cnt[i] = 0;
+    __syncthreads();
+    const u64 lead = (reinterpret_cast<uintptr_t>(keys) & 8) ? 1 : 0;           // a list may start on an odd 8-byte boundary
+    const u64 pairs = (n - lead) >> 1;
+    const ulonglong2* const k2 = reinterpret_cast<const ulonglong2*>(keys + lead);
+    for(u64 i = u64(blockIdx.x) * (COUNT_BLOCK * COUNT_UNROLL) + threadIdx.x; i < pairs; i += u64(gridDim.x) * (COUNT_BLOCK * COUNT_UNROLL))
+    {
+        ulonglong2 k[COUNT_UNROLL];
+        #pragma unroll
+        for(int j = 0; j < COUNT_UNROLL; ++j) if(i + u64(j) * COUNT_BLOCK < pairs) k[j] = k2[i + u64(j) * COUNT_BLOCK];
+        #pragma unroll
+        for(int j = 0; j < COUNT_UNROLL; ++j)
+            if(i + u64(j) * COUNT_BLOCK < pairs)
+            {
+                atomicAdd(&cnt[u32(k[j].x >> shift) & mask], 1u);
+                atomicAdd(&cnt[u32(k[j].y >> shift) & mask], 1u);
+            }
+    }
+    if(blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        if(lead) atomicAdd(&cnt[u32(keys[0] >> shift) & mask], 1u);
+        if((n - lead) & 1) atomicAdd(&cnt[u32(keys[n - 1] >> shift) & mask], 1u);
+    }
+    __syncthreads();
+    for(u32 i = threadIdx.x; i < buckets; i += COUNT_BLOCK)
+        if(const u32 c = cnt[i]) atomicAdd(&counts[i], c);
+}
+
+__device__ __forceinline__ u32 warp_inclusive_sum(u32 v)
+{
+    #pragma unroll
+    for(int o = 1; o < 32; o <<= 1)
+    {
+        const u32 t = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if(int(lane_id()) >= o) v += t;
+    }
+    return v;
+}
+
+// Exclusive sum over a block of up to 1024 threads; warp_tot: a word per warp. Ends with a barrier.
+template <int BLOCK>
+__device__ __forceinline__ u32 block_exclusive_sum(const u32 v, u32* warp_tot)
+{
+    const u32 inc = warp_inclusive_sum(v);
+    if(lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+    __syncthreads();
+    const u32 t = lane_id() < BLOCK / 32 ? warp_tot[lane_id()] : 0;
+    const u32 pre = __shfl_sync(0xFFFFFFFFu, warp_inclusive_sum(t) - t, threadIdx.x >> 5);
+    __syncthreads();
+    return pre + inc - v;
+}
+
+// One block: the counts become the buckets' starts, in place (starts[buckets] = n); the digit offsets of the one or two passes by which
+// the records get there (low digit first: low_bits of them, which may be 0, then the top bits); and the size of the largest bucket.
+__global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ counts, const u32 n, const int bits, const int low_bits, u64* __restrict__ low_base,
+                                                          u64* __restrict__ high_base, u64* __restrict__ largest)
+{
+    __shared__ u32 warp_tot[32];
+    __shared__ u32 low[256];
+    __shared__ u32 most;
+    const u32 t = threadIdx.x, buckets = 1u << bits, per = (buckets + 1023) / 1024;
+    if(t < 256) low[t] = 0;
+    if(t == 0) most = 0;
+    __syncthreads();
+    const u32 first = t * per;
+    u32 sum = 0, big = 0;
+    for(u32 i = first; i < first + per && i < buckets; ++i) { const u32 c = counts[i]; sum += c; big = max(big, c); }
+    big = __reduce_max_sync(0xFFFFFFFFu, big);
+    if(lane_id() == 0) atomicMax(&most, big);
+    if(low_bits)        // thread (g, l): every buckets / 1024-th bucket of low digit l
+    {
+        const u32 lows = 1u << low_bits, l = t & (lows - 1);
+        u32 s = 0;
+        for(u32 i = t; i < buckets; i += 1024) s += counts[i];          // 1024 is a multiple of lows
+        atomicAdd(&low[l], s);
+    }
+    __syncthreads();
+    u32 run = block_exclusive_sum<1024>(sum, warp_tot);
+    for(u32 i = first; i < first + per && i < buckets; ++i)
+    {
+        const u32 c = counts[i];
+        counts[i] = run;
+        if((i & ((1u << low_bits) - 1)) == 0) high_base[i >> low_bits] = run;
+        run += c;
+    }
+    const u32 at = block_exclusive_sum<1024>(t < 256 ? low[t] : 0, warp_tot);
+    if(low_bits && t < (1u << low_bits)) low_base[t] = at;
+    if(t == 0) { counts[buckets] = n; *largest = most; }
+}
+
+// ---- a bucket inside one block -------------------------------------------------------------------------------------------------
+
+constexpr int BUCKET_ITEMS = 16;
+template <int BLOCK> constexpr u32 BUCKET_CAP = BLOCK * BUCKET_ITEMS;
+constexpr u32 LONG_BIN = 128;       // a bin with more records is not ordered by comparing all with all
+template <int BLOCK> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CAP<BLOCK>) * (8 + 2) + (BUCKET_CAP<BLOCK> / 2 + 4) * 4;
+
+// Sorts every bucket [starts[b], starts[b + 1]) (starts == nullptr: one bucket, [0, n)) by the bits `compared` of its keys, of which
+// the highest is bit top - 1, stably, from the `in` to the `out` arrays. There are as many bins as records (up to a factor of 2): a record's
+// bin is its next key bits, its place in the bin is what a shared-memory atomic hands out, and inside the bin it counts the keys before its own, equal ones
+// by the places they came from. So the order is the stable one whatever order the atomics took. The values stay in global memory
+// until a record's place is known: a bucket's are a few KB side by side.
+// A bin of more than LONG_BIN records sends the bucket through a sorting network instead. What bounds it is the issue of instructions and
+// barriers between dependent steps; blocks are therefore as small as the largest bucket allows.
+template <int BLOCK, typename V>
+__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in,
+                                                                         V* __restrict__ vals_out, const u32* __restrict__ starts, const u32 n, const u64 compared, const int top,
+                                                                         const int begin)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr u32 CAP = BUCKET_CAP<BLOCK>;
+    u64* const stage = reinterpret_cast<u64*>(smem_raw);            // [CAP]
+    u32* const bin = reinterpret_cast<u32*>(stage + CAP);           // [CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
+    u16* const start = reinterpret_cast<u16*>(bin);
+    u16* const from = reinterpret_cast<u16*>(bin + CAP / 2 + 4);    // [CAP]: the record's place in the bucket before
+    __shared__ u32 warp_tot[BLOCK / 32];
+    const u32 tid = threadIdx.x;
+    const u32 base = starts ? starts[blockIdx.x] : 0, m = (starts ? starts[blockIdx.x + 1] : n) - base;
+    if(m == 0 || m > CAP) return;       // the host has seen to it that all fit
+    keys_in += base; keys_out += base;
+    if(vals_in != nullptr) { vals_in += base; vals_out += base; }
+
+    const int bin_bits = min(32 - __clz(m - 1 | 1u), top - begin);   // bins: a power of two, at most CAP
+    const u32 bins = 1u << bin_bits;
+    const int bin_shift = top - bin_bits;
+    const u32 bin_mask = bins - 1;
+    for(u32 i = tid; i < (bins / 2 + 4) / 4; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+    u64 r[BUCKET_ITEMS];
+    u32 pl[BUCKET_ITEMS];               // bin << 16 | place in the bin
+    #pragma unroll
+    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    {
+        if(i * BLOCK >= m) break;
+        const u32 j = tid + i * BLOCK;
+        if(j < m) r[i] = keys_in[j];
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    {
+        if(i * BLOCK >= m) break;
+        if(tid + i * BLOCK < m)
+        {
+            const u32 b = u32(r[i] >> bin_shift) & bin_mask;
+            const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
+            pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
+        }
+    }
+    __syncthreads();
+    // exclusive sums of the bins' counts, in place
+    u32 longest = 0;
+    {
+        constexpr int WORDS = CAP / 2 / BLOCK;          // 8 words, 16 bins a thread
+        u32 c[WORDS], sum = 0;
+        const bool any = tid * WORDS * 2 < bins;        // of the words behind the bins' a few may hold anything: their sums are not used
+        if(any)
+        {
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k)
+            {
+                c[k] = tid * WORDS + k < (bins + 1) / 2 ? bin[tid * WORDS + k] : 0;
+                longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16));
+                sum += (c[k] & 0xFFFFu) + (c[k] >> 16);
+            }
+        }
+        u32 run = block_exclusive_sum<BLOCK>(sum, warp_tot);
+        if(any)
+        {
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k)
+            {
+                const u32 a = run, b = run + (c[k] & 0xFFFFu);
+                run = b + (c[k] >> 16);
+                if(tid * WORDS + k < (bins + 1) / 2) bin[tid * WORDS + k] = a | (b << 16);
+            }
+        }
+        __syncthreads();
+        if(tid == 0) start[bins] = u16(m);
+    }
+    const bool by_network = __syncthreads_or(longest > LONG_BIN);
+    if(by_network)
+    {
+        // Many records in one bin: a sorting network over (key, place before), padded with records behind all others.
+        u32 size = 1;
+        while(size < m) size <<= 1;
+        #pragma unroll
+        for(int i = 0; i < BUCKET_ITEMS; ++i)
+        {
+            const u32 j = tid + i * BLOCK;
+            if(j >= size) break;
+            stage[j] = j < m ? r[i] : ~0ull;
+            from[j] = j < m ? u16(j) : u16(0xFFFF);
+        }
+        __syncthreads();
+        for(u32 k = 2; k <= size; k <<= 1)
+            for(u32 d = k >> 1; d > 0; d >>= 1)
+            {
+                for(u32 t = tid; t < size / 2; t += BLOCK)
+                {
+                    const u32 a = 2 * t - (t & (d - 1)), b = a + d;
+                    const u64 x = stage[a], y = stage[b];
+                    const u16 fx = from[a], fy = from[b];
+                    const u64 cx = x & compared, cy = y & compared;
+                    // a padding record's key may equal a real one's: its place decides
+                    const bool greater = cx > cy || (cx == cy && fx > fy);
+                    if(greater == ((a & k) == 0)) { stage[a] = y; stage[b] = x; from[a] = fy; from[b] = fx; }
+                }
+                __syncthreads();
+            }
+        for(u32 j = tid; j < m; j += BLOCK)
+        {
+            keys_out[j] = stage[j];
+            if(vals_in != nullptr) vals_out[j] = vals_in[from[j]];
+        }
+        return;
+    }
+    #pragma unroll
+    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    {
+        if(i * BLOCK >= m) break;
+        const u32 j = tid + i * BLOCK;
+        if(j < m)
+        {
+            const u32 at = start[pl[i] >> 16] + (pl[i] & 0xFFFFu);
+            stage[at] = r[i];
+            from[at] = u16(j);
+        }
+    }
+    __syncthreads();
+    #pragma unroll 4
+    for(u32 j = tid; j < m; j += BLOCK)
+    {
+        const u64 v = stage[j], mine = v & compared;
+        const u32 f = from[j];
+        const u32 b = u32(v >> bin_shift) & bin_mask;
+        const u32 s = start[b], e = start[b + 1];
+        u32 place = s;
+        for(u32 k = s; k < e; ++k)
+        {
+            const u64 o = stage[k] & compared;
+            if(o < mine) ++place;
+            else if(o == mine) place += from[k] < f;
+        }
+        keys_out[place] = v;
+        if(vals_in != nullptr) vals_out[place] = vals_in[f];
+    }
+}
+
+template <int BLOCK, typename V>
+int launch_buckets(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 compared, int top, int begin)
+{
+    static std::atomic<bool> configured[64];
+    if(!configured[ctx->device & 63])
+    {
+        CSA_CUDA(ctx, cudaFuncSetAttribute(bucket_sort_kernel<BLOCK, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BUCKET_SMEM<BLOCK>)));
+        configured[ctx->device & 63] = true;
+    }
+    bucket_sort_kernel<BLOCK, V><<<buckets, BLOCK, BUCKET_SMEM<BLOCK>, ctx->stream>>>(kin, kout, vin, vout, starts, u32(n), compared, top, begin);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+template <typename V>
+int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 largest, int begin, int top)
+{
+    const u64 compared = (top >= 64 ? ~0ull : (1ull << top) - 1) & (~0ull << begin);
+    if(largest <= BUCKET_CAP<128>) return launch_buckets<128, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    if(largest <= BUCKET_CAP<256>) return launch_buckets<256, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    if(largest <= BUCKET_CAP<512>) return launch_buckets<512, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    return csa_fail(ctx, CSA_E_DEVICE, "bucket sort: a bucket does not fit a block");
+}
+
+static_assert(BUCKET_CAP<512> == BUCKET_MAX_RECORDS, "");
+
+}   // namespace
+
+int bucket_sort_bits(u64 n)
+{
+    int t = 0;
+    while(t < BUCKET_MAX_BITS && (n >> t) > 1024) ++t;
+    return t == 9 ? 8 : t;          // 9 bits would be a second pass
+}
+
+int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int end_bit, int bits, int low_bits, u32* starts, u64* low_base, u64* high_base, u64* largest_dev)
+{
+    static std::atomic<bool> configured[64];
+    if(!configured[ctx->device & 63])
+    {
+        CSA_CUDA(ctx, cudaFuncSetAttribute(bucket_counts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(4u << BUCKET_MAX_BITS)));
+        configured[ctx->device & 63] = true;
+    }
+    CSA_CUDA(ctx, cudaMemsetAsync(starts, 0, size_t(4) << bits, ctx->stream));
+    bucket_counts_kernel<<<unsigned(std::min<u64>(148, div_up(n, 2 * COUNT_BLOCK * COUNT_UNROLL))), COUNT_BLOCK, size_t(4) << bits, ctx->stream>>>(keys, n, end_bit - bits, bits, starts);
+    CSA_LAUNCH_CHECK(ctx);
+    bucket_plan_kernel<<<1, 1024, 0, ctx->stream>>>(starts, u32(n), bits, low_bits, low_base, high_base, largest_dev);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, int begin_bit,
+                       int top)
+{
+    if(val_bytes == 4) return launch_buckets_of<u32>(ctx, kin, kout, static_cast<const u32*>(vin), static_cast<u32*>(vout), starts, buckets, n, largest, begin_bit, top);
+    return launch_buckets_of<u64>(ctx, kin, kout, static_cast<const u64*>(vin), static_cast<u64*>(vout), starts, buckets, n, largest, begin_bit, top);
+}

@@ -772,6 +772,7 @@ size_t csa_sort_workspace_bytes(uint64_t n)
          + 256                                         // tile counter
          + size_t(8) * RADIX * 8 + 256                 // histograms
          + size_t(portions + 1) * 8 * RADIX * 8 + 256  // digit bases of every launch
+         + (n <= BUCKET_MAX_TOTAL ? align_up256(((size_t(1) << bucket_sort_bits(n)) + 1) * 4) : 0)     // starts of the buckets
          + 4096;
 }
 
@@ -818,6 +819,70 @@ void sort_reset_timing(csa_ctx* ctx)
     t.passes = t.records = t.bytes = 0;
 }
 
+namespace
+{
+
+// The sort by buckets (bucket_sort.cu), where it spares two digit passes or more and no bucket is too large for a block; else nothing has been
+// moved and done stays false. Not for sorts whose ties may come in any order: their keys are pairs of ranks, uneven in the top bits, and
+// their first pass is the cheap one.
+int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* vals_alt, u32 val_bytes, u64 n, int begin_bit, int end_bit, u32* counter, u32* status, u64* base,
+                    u32* starts, int* in_alt, bool& done)
+{
+    const int width = end_bit - begin_bit, passes = (width + RADIX_BITS - 1) / RADIX_BITS;
+    if(n <= BUCKET_MAX_RECORDS && passes >= 2)
+    {
+        CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, nullptr, 1, n, n, begin_bit, end_bit));
+        *in_alt = 1;
+        done = true;
+        return CSA_OK;
+    }
+    const int bits = bucket_sort_bits(n), splits = bits > RADIX_BITS ? 2 : 1, low_bits = bits > RADIX_BITS ? bits - RADIX_BITS : 0;
+    if(n > BUCKET_MAX_TOTAL || passes < splits + 2) return CSA_OK;
+    u64* const low_base = base;
+    u64* const high_base = base + RADIX;
+    u64* const largest_dev = ctx->d_scalars + 32;
+    CSA_TRY(launch_bucket_plan(ctx, keys, n, end_bit, bits, low_bits, starts, low_base, high_base, largest_dev));
+    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 32, largest_dev, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    const u64 largest = ctx->h_scalars[32];
+    if(largest > BUCKET_MAX_RECORDS) return CSA_OK;
+    Pass_Timer& timer = timer_of(ctx);
+    for(int s = 2 - splits; s < 2; ++s)
+    {
+        const int shift = s == 0 ? end_bit - bits : end_bit - bits + low_bits;
+        const u32 dmask = (1u << (s == 0 ? low_bits : bits - low_bits)) - 1;
+        const u64* const db = s == 0 ? low_base : high_base;
+        cudaEvent_t e0 = nullptr, e1 = nullptr;
+        if(timer.on)
+        {
+            CSA_CUDA(ctx, cudaEventCreate(&e0));
+            CSA_CUDA(ctx, cudaEventCreate(&e1));
+            CSA_CUDA(ctx, cudaEventRecord(e0, ctx->stream));
+        }
+        if(val_bytes == 4 || vals == nullptr)
+            CSA_TRY(launch_pass_variant<u32>(ctx, keys, keys_alt, static_cast<const u32*>(vals), static_cast<u32*>(vals_alt), n, shift, dmask, db, nullptr, status, counter));
+        else
+            CSA_TRY(launch_pass_variant<u64>(ctx, keys, keys_alt, static_cast<const u64*>(vals), static_cast<u64*>(vals_alt), n, shift, dmask, db, nullptr, status, counter));
+        if(timer.on)
+        {
+            CSA_CUDA(ctx, cudaEventRecord(e1, ctx->stream));
+            timer.ev.push_back(e0); timer.ev.push_back(e1);
+            timer.passes++; timer.records += n; timer.bytes += 2 * n * (8 + (vals ? val_bytes : 0));
+        }
+        ctx->counters[1]++;
+        ctx->counters[2] += n;
+        if(vals == nullptr) ctx->counters[3] += n;
+        std::swap(keys, keys_alt);
+        std::swap(vals, vals_alt);
+    }
+    CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, starts, 1u << bits, n, largest, begin_bit, end_bit - bits));
+    *in_alt = (splits + 1) & 1;
+    done = true;
+    return CSA_OK;
+}
+
+}   // namespace
+
 int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals, void* vals_alt, uint32_t val_bytes, uint64_t n,
                    int begin_bit, int end_bit, void* workspace, size_t workspace_bytes, int* in_alt)
 {
@@ -837,7 +902,15 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
     u32* status = cv.take<u32>(tiles_max * RADIX);
     u64* hist = cv.take<u64>(u64(8) * RADIX);
     u64* base = cv.take<u64>(u64(portions + 1) * 8 * RADIX);
+    u32* starts = n <= BUCKET_MAX_TOTAL ? cv.take<u32>((u64(1) << bucket_sort_bits(n)) + 1) : nullptr;
     if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "csa_sort_pairs: workspace too small");
+
+    if(!ctx->ties_in_any_order && portions == 1)
+    {
+        bool done = false;
+        CSA_TRY(sort_by_buckets(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, n, begin_bit, end_bit, counter, status, base, starts, in_alt, done));
+        if(done) return CSA_OK;
+    }
 
     {
         static std::atomic<bool> hist_configured[64];

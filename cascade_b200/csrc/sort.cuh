@@ -19,3 +19,16 @@ void stream_set_position_offset(u64 offset);
 size_t sort_segments_workspace_bytes(u64 n, u32 segs);
 int sort_segments(csa_ctx* ctx, u64* keys, u64* keys_alt, u32* vals, u32* vals_alt, const u64* seg_off_host, u32 segs, int begin_bit, int end_bit, void* workspace,
                   size_t workspace_bytes, int* in_alt);
+
+// Buckets by the top bits of evenly spread keys, each finished inside one block (bucket_sort.cu).
+constexpr int BUCKET_MAX_BITS = 15;                 // a block counts them in shared memory
+constexpr u64 BUCKET_MAX_RECORDS = 8192;            // what a block holds
+constexpr u64 BUCKET_MAX_TOTAL = u64(1) << 26;      // records of a sort by buckets: 2048 a bucket
+// Top bits by which n records are split into buckets of 512 to 2048 on average.
+int bucket_sort_bits(u64 n);
+// The buckets' starts (1 << bits of them, and the end), the digit offsets of the passes by the lower low_bits of the bucket number and
+// by the others, and the size of the largest bucket. Queued; starts: (1 << bits) + 1 words.
+int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int end_bit, int bits, int low_bits, u32* starts, u64* low_base, u64* high_base, u64* largest_dev);
+// Every bucket (starts == nullptr: all n records) sorted by the key bits [begin_bit, top), stably; largest: no bucket holds more.
+int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, int begin_bit,
+                       int top);

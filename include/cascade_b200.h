@@ -67,8 +67,9 @@ const char* csa_version(void);
 
 /* Bytes of workspace that csa_sort_pairs needs for n records. */
 size_t csa_sort_workspace_bytes(uint64_t n);
-/* Stable least-significant-digit radix sort of n (64-bit key, value) records on key bits [begin_bit, end_bit),
- * 8 bits per pass, each pass one sweep over the records. val_bytes is 4 or 8. The records ping-pong between
+/* Stable radix sort of n (64-bit key, value) records on key bits [begin_bit, end_bit), least significant digit first, 8 bits per pass,
+ * each pass one sweep over the records; up to 2^26 records whose top bits are evenly spread are split by those alone and finished in
+ * shared memory. val_bytes is 4 or 8. The records ping-pong between
  * (keys, vals) and (keys_alt, vals_alt); *in_alt is set to 1 if the sorted records end in the alt buffers, else 0.
  * Passes whose digit is the same for every key are skipped. With vals_dev and vals_alt_dev both null only keys are sorted. */
 int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys_dev, uint64_t* keys_alt_dev, void* vals_dev, void* vals_alt_dev,
