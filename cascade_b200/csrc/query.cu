@@ -7,6 +7,9 @@
 // counterpart there; it lists SA[lo + k] in rank order.
 #include "common.cuh"
 
+#include <algorithm>
+#include <atomic>
+
 namespace
 {
 
@@ -37,30 +40,99 @@ __device__ __forceinline__ int cmp_suffix_pattern(const u16* __restrict__ T, con
 // The ranks that can hold the two boundaries of a query's interval, from the sample table alone.
 struct Brackets { u64 lo_first, lo_last, hi_first, hi_last; };
 
-// The pattern's first min(m, K) symbols, packed like a table key, and the mask of those symbols.
-struct Table_Key
+// Up to eight symbols from address p on, most significant first, zeros behind `count` of them (1 to 8). Two 16-byte loads, the second only where the
+// symbols reach into it: a piece of 16 bytes that holds a wanted symbol lies in the allocation that holds the symbol. (One symbol at a time, a
+// comparison of a query's pattern with a suffix took up to sixteen loads of 32 scattered addresses each: the lines that a warp's loads touch, one a
+// cycle, were three quarters of the search's time.)
+__device__ __forceinline__ ulonglong2 load_symbols(const u16* p, const u32 count)
 {
-    u64 high = 0, low = 0, mask_high, mask_low;
-    __device__ __forceinline__ Table_Key(const u16* __restrict__ P, const u64 m)
+    const uintptr_t at = reinterpret_cast<uintptr_t>(p);
+    const uint4* const piece = reinterpret_cast<const uint4*>(at & ~uintptr_t(15));
+    const u32 skip = u32(at >> 1) & 7u;
+    const uint4 a = __ldg(piece);
+    uint4 b = make_uint4(0, 0, 0, 0);
+    if(skip + count > 8) b = __ldg(piece + 1);
+    u32 w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    #pragma unroll
+    for(int k = 0; k < 6; ++k) w[k] = (skip & 4) ? w[k + 2 < 8 ? k + 2 : 7] : w[k];
+    if(skip & 4) { w[6] = 0; w[7] = 0; }
+    #pragma unroll
+    for(int k = 0; k < 5; ++k) w[k] = (skip & 2) ? w[k + 1] : w[k];
+    u32 r[4];
+    #pragma unroll
+    for(int k = 0; k < 4; ++k)
     {
+        const u32 v = (skip & 1) ? __funnelshift_r(w[k], w[k + 1], 16) : w[k];
+        r[k] = __funnelshift_l(v, v, 16);
+    }
+    return make_ulonglong2((u64(r[0]) << 32) | r[1], (u64(r[2]) << 32) | r[3]);
+}
+
+// A pattern of m >= 1 symbols: its first min(m, K), packed like a table key, and the mask of those symbols.
+struct Pattern
+{
+    u64 high = 0, low = 0, mask_high = 0, mask_low = 0, m = 0;
+    __device__ __forceinline__ Pattern() {}
+    __device__ __forceinline__ Pattern(const u16* P, const u64 length)
+    {
+        set_length(length);
+        const ulonglong2 k = load_symbols(P, length < CSA_K ? u32(length) : u32(CSA_K));
+        high = k.x & mask_high; low = k.y & mask_low;
+    }
+    __device__ __forceinline__ void set_length(const u64 length)
+    {
+        m = length;
         const u32 mm = m < CSA_K ? u32(m) : u32(CSA_K);
-        for(u32 k = 0; k < mm; ++k)
-        {
-            if(k < 4) high |= u64(P[k]) << (48 - 16 * k);
-            else low |= u64(P[k]) << (48 - 16 * (k - 4));
-        }
         mask_high = mm >= 4 ? ~0ull : ~0ull << (64 - 16 * mm);
         mask_low = mm <= 4 ? 0ull : (mm == 8 ? ~0ull : ~0ull << (64 - 16 * (mm - 4)));
     }
+    // For patterns of at most K symbols.
+    __device__ __forceinline__ bool last_is_zero() const { return ((m <= 4 ? high >> (64 - 16 * m) : low >> (128 - 16 * m)) & 0xFFFFu) == 0; }
     // The (masked) key t is smaller than the pattern's; not greater.
     __device__ __forceinline__ bool less(const ulonglong2 t) const { const u64 h = t.x & mask_high; return h < high || (h == high && (t.y & mask_low) < low); }
     __device__ __forceinline__ bool not_greater(const ulonglong2 t) const { const u64 h = t.x & mask_high; return h < high || (h == high && (t.y & mask_low) <= low); }
+
+    // Order of the suffix at `pos`, truncated to m symbols, against the pattern, as cmp_suffix_pattern tells it. The text's zero padding may
+    // only make a short suffix look equal, never greater. P: the whole pattern, read where it has more than K symbols.
+    __device__ __forceinline__ int compare(const u16* __restrict__ T, const u64 n, const u64 pos, const u16* __restrict__ P) const
+    {
+        const ulonglong2 t = load_symbols(T + pos, m < CSA_K ? u32(m) : u32(CSA_K));
+        const u64 h = t.x & mask_high, l = t.y & mask_low;
+        if(h != high) return h < high ? -1 : 1;
+        if(l != low) return l < low ? -1 : 1;
+        for(u64 i = CSA_K; i < m; i += CSA_K)
+        {
+            if(pos + i >= n) return -1;
+            const u32 more = m - i < CSA_K ? u32(m - i) : u32(CSA_K);
+            const u64 keep_high = more >= 4 ? ~0ull : ~0ull << (64 - 16 * more), keep_low = more <= 4 ? 0ull : (more == 8 ? ~0ull : ~0ull << (64 - 16 * (more - 4)));
+            const ulonglong2 x = load_symbols(T + pos + i, more), y = load_symbols(P + i, more);
+            if(((x.x ^ y.x) & keep_high) != 0) return (x.x & keep_high) < (y.x & keep_high) ? -1 : 1;
+            if(((x.y ^ y.y) & keep_low) != 0) return (x.y & keep_low) < (y.y & keep_low) ? -1 : 1;
+        }
+        return n - pos < m ? -1 : 0;
+    }
 };
+
+// Entry r of a suffix array in device memory, by one 16-byte load as a rule and a second one for the quarter of the entries that cross a boundary.
+__device__ __forceinline__ u64 sa40_load_wide(const u8* sa, const u64 r)
+{
+    const uintptr_t at = reinterpret_cast<uintptr_t>(sa) + 5 * r;
+    const uint4* const piece = reinterpret_cast<const uint4*>(at & ~uintptr_t(15));
+    const u32 byte = u32(at) & 15u, word = byte >> 2;
+    const uint4 a = __ldg(piece);
+    u32 next = 0;
+    if(byte > 11) next = __ldg(reinterpret_cast<const u32*>(piece + 1));
+    const u32 lo = word == 0 ? a.x : word == 1 ? a.y : word == 2 ? a.z : a.w;
+    const u32 hi = word == 0 ? a.y : word == 1 ? a.z : word == 2 ? a.w : next;
+    const u64 v = (u64(hi) << 32) | lo;
+    return (v >> ((byte & 3) * 8)) & 0xFFFFFFFFFFull;
+}
 
 // The brackets from a = table keys (masked) smaller than the pattern's and b = those not greater, of J. Sampled rank j * stride carries
 // table key j. Ranks up to (a-1) stride are smaller than the pattern; ranks from b stride on are greater.
-__device__ __forceinline__ Brackets brackets_from(const u64 a, const u64 b, const u64 J, const u64 stride, const u64 ne, const u16* __restrict__ P, const u64 m)
+__device__ __forceinline__ Brackets brackets_from(const u64 a, const u64 b, const u64 J, const u64 stride, const u64 ne, const Pattern& p)
 {
+    const u64 m = p.m;
     Brackets br;
     br.lo_first = (a == 0) ? 0 : (a - 1) * stride + 1;
     br.hi_last = (b >= J) ? ne : b * stride;
@@ -70,7 +142,7 @@ __device__ __forceinline__ Brackets brackets_from(const u64 a, const u64 b, cons
     {
         // Every suffix whose masked key equals the pattern's matches it, except suffixes that end inside the pattern and
         // owe the equality to zero padding; there are fewer than m of them and they need the pattern to end in a zero.
-        const u64 e = (P[m - 1] == 0) ? m - 1 : 0;
+        const u64 e = p.last_is_zero() ? m - 1 : 0;
         const u64 cap = a * stride + e;
         if(cap < br.lo_last) br.lo_last = cap;
         if(b > 0 && (b - 1) * stride + 1 > br.hi_first) br.hi_first = (b - 1) * stride + 1;
@@ -78,39 +150,46 @@ __device__ __forceinline__ Brackets brackets_from(const u64 a, const u64 b, cons
     return br;
 }
 
-__device__ __forceinline__ Brackets table_brackets(const csa_index& idx, const u16* __restrict__ P, const u64 m)
+// a0, a1: the number of smaller keys lies between them; b0, b1: the number of keys not greater does.
+__device__ __forceinline__ Brackets table_brackets(const csa_index& idx, const Pattern& p, const u64 a0, const u64 a1, const u64 b0, const u64 b1)
 {
     const u64 stride = idx.stride;
     const u64 ne = idx.sa_entries ? idx.sa_entries : idx.n;      // entries of the suffix array (a slice of it in a sharded index)
-    const Table_Key key(P, m);
     const u64 J = (ne + stride - 1) / stride;
     const ulonglong2* const tab = reinterpret_cast<const ulonglong2*>(idx.table);
     u64 a, b;
     {
-        u64 x = 0, y = J;
+        u64 x = a0, y = a1;
         while(x < y)
         {
             const u64 mid = x + ((y - x) >> 1);
-            if(key.less(tab[mid])) x = mid + 1; else y = mid;
+            if(p.less(__ldg(tab + mid))) x = mid + 1; else y = mid;
         }
         a = x;
         // b lies at or shortly after a unless the pattern's K-gram is very frequent: gallop from a (1, 2, 4, ... keys ahead)
         // to the first key that is greater, then bisect what is left. Every probe is a dependent random read, and this
         // spares about twenty of them per query.
-        y = J;
+        if(x < b0) x = b0;
+        y = b1;
         for(u64 step = 1; x < y; step <<= 1)
         {
             const u64 mid = (x + step - 1 < y) ? x + step - 1 : y - 1;
-            if(key.not_greater(tab[mid])) x = mid + 1; else { y = mid; break; }
+            if(p.not_greater(__ldg(tab + mid))) x = mid + 1; else { y = mid; break; }
         }
         while(x < y)
         {
             const u64 mid = x + ((y - x) >> 1);
-            if(key.not_greater(tab[mid])) x = mid + 1; else y = mid;
+            if(p.not_greater(__ldg(tab + mid))) x = mid + 1; else y = mid;
         }
         b = x;
     }
-    return brackets_from(a, b, J, stride, ne, P, m);
+    return brackets_from(a, b, J, stride, ne, p);
+}
+
+__device__ __forceinline__ Brackets table_brackets(const csa_index& idx, const Pattern& p)
+{
+    const u64 ne = idx.sa_entries ? idx.sa_entries : idx.n, J = (ne + idx.stride - 1) / idx.stride;
+    return table_brackets(idx, p, 0, J, 0, J);
 }
 
 // The first index of [x, y) for which `before` does not hold (y if it holds for all), by a warp: 32 probes at a time, which cut the range
@@ -151,10 +230,11 @@ __device__ __forceinline__ u64 warp_partition_point_near(u64 x, u64 y, const F& 
     return warp_partition_point(x, y, before);
 }
 
-// Both boundaries of the interval by binary search inside the brackets. `sa_lo` / `sa_hi` are what entry r of the suffix
-// array is read from in each search: the array itself, or a gathered window shifted so that the same r addresses it.
-__device__ __forceinline__ void search_brackets(const csa_index& idx, const Brackets& br, const u16* __restrict__ P, const u64 m, const u8* sa_lo,
-                                                const u8* sa_hi, u64& lo_out, u64& hi_out)
+// Both boundaries of the interval by binary search inside the brackets. sa_lo(r), sa_hi(r): entry r of the suffix array in each search: of
+// the array itself, or of a gathered window.
+template <typename Lo, typename Hi>
+__device__ __forceinline__ void search_brackets(const csa_index& idx, const Brackets& br, const Pattern& p, const u16* __restrict__ P, const Lo& sa_lo, const Hi& sa_hi,
+                                                u64& lo_out, u64& hi_out)
 {
     const u64 n = idx.n;
     const u16* const T = idx.text;
@@ -162,7 +242,7 @@ __device__ __forceinline__ void search_brackets(const csa_index& idx, const Brac
     while(x < y)
     {
         const u64 mid = x + ((y - x) >> 1);
-        if(cmp_suffix_pattern(T, n, sa40_load(sa_lo, mid), P, m) < 0) x = mid + 1; else y = mid;
+        if(p.compare(T, n, sa_lo(mid), P) < 0) x = mid + 1; else y = mid;
     }
     lo_out = x;
     x = (br.hi_first > x) ? br.hi_first : x;
@@ -172,36 +252,188 @@ __device__ __forceinline__ void search_brackets(const csa_index& idx, const Brac
     for(u64 step = 1; x < y; step <<= 1)
     {
         const u64 mid = (x + step - 1 < y) ? x + step - 1 : y - 1;
-        if(cmp_suffix_pattern(T, n, sa40_load(sa_hi, mid), P, m) <= 0) x = mid + 1; else { y = mid; break; }
+        if(p.compare(T, n, sa_hi(mid), P) <= 0) x = mid + 1; else { y = mid; break; }
     }
     while(x < y)
     {
         const u64 mid = x + ((y - x) >> 1);
-        if(cmp_suffix_pattern(T, n, sa40_load(sa_hi, mid), P, m) <= 0) x = mid + 1; else y = mid;
+        if(p.compare(T, n, sa_hi(mid), P) <= 0) x = mid + 1; else y = mid;
     }
     hi_out = x;
 }
 
-__global__ void find_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const u64 q, u64* __restrict__ itv)
+__device__ __forceinline__ bool is_slice(const csa_index& idx) { return idx.sa_entries != 0 && idx.sa_entries < idx.n; }
+
+__global__ void __launch_bounds__(128) find_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const u64 q, u64* __restrict__ itv)
 {
     const u64 i = u64(blockIdx.x) * blockDim.x + threadIdx.x;
     if(i >= q) return;
-    const u64 m = off[i + 1] - off[i];
-    const u16* const P = sym + (off[i] - off[0]);
+    const u64 from = off[i], m = off[i + 1] - from;
+    const u16* const P = sym + (from - off[0]);
     if(m == 0) { itv[2 * i] = 0; itv[2 * i + 1] = idx.sa_entries ? idx.sa_entries : idx.n; return; }
-    if(idx.sa_entries != 0 && idx.sa_entries < idx.n)
+    const Pattern p(P, m);
+    if(is_slice(idx))
     {
         // One slice of a sharded array: most patterns lie wholly before or wholly after it, which its first and last suffix
         // tell with two comparisons; only a pattern that falls inside the slice's range is searched for.
         const u64 e = idx.sa_entries;
-        if(cmp_suffix_pattern(idx.text, idx.n, sa40_load(idx.sa40, 0), P, m) > 0) { itv[2 * i] = 0; itv[2 * i + 1] = 0; return; }
-        if(cmp_suffix_pattern(idx.text, idx.n, sa40_load(idx.sa40, e - 1), P, m) < 0) { itv[2 * i] = e; itv[2 * i + 1] = e; return; }
+        if(p.compare(idx.text, idx.n, sa40_load(idx.sa40, 0), P) > 0) { itv[2 * i] = 0; itv[2 * i + 1] = 0; return; }
+        if(p.compare(idx.text, idx.n, sa40_load(idx.sa40, e - 1), P) < 0) { itv[2 * i] = e; itv[2 * i + 1] = e; return; }
     }
-    const Brackets br = table_brackets(idx, P, m);
+    const Brackets br = table_brackets(idx, p);
     u64 lo, hi;
-    search_brackets(idx, br, P, m, idx.sa40, idx.sa40, lo, hi);
+    auto entry = [&](const u64 r) { return sa40_load_wide(idx.sa40, r); };
+    search_brackets(idx, br, p, P, entry, entry, lo, hi);
     itv[2 * i] = lo;
     itv[2 * i + 1] = hi;
+}
+
+// ---- large batches: the queries by where they lie in the table ---------------------------------------------------------------
+//
+// A query's reads are random ones, in the table, in the array and in the text, and a batch in its own order shares none of them. So the
+// queries of a large batch are first dealt into SLOTS by where they fall among as many keys of the table (a directory that a block keeps in shared
+// memory): the queries of a slot then read the same upper levels of the table's bisection, one stretch of the table and one of
+// the array. Nothing is sorted: the slots are counted, and a query takes the next place of its slot.
+constexpr u32 SLOT_BITS = 12, SLOTS = 1u << SLOT_BITS;
+constexpr int SLOT_BLOCK = 512, SLOT_ITEMS = 8, SLOT_TILE = SLOT_BLOCK * SLOT_ITEMS;
+constexpr size_t SLOT_SMEM = SLOTS * 8 + (SLOTS + 1) * 4;
+
+// What a query needs on its way, in the order of the slots.
+struct __align__(16) Slot_Query
+{
+    u64 high, low;          // Pattern
+    u32 index;              // of the query in its batch
+    u16 first, last;        // of the directory's keys those before `first` are smaller, those from `last` on greater
+    u64 at;                 // the pattern's first symbol in the batch's, and from bit 48 on its length (LONG_PATTERN: that or more)
+};
+static_assert(sizeof(Slot_Query) == 32, "one sector");
+constexpr u32 LONG_PATTERN = 0xFFFF;
+
+// Where a query falls in the directory, and which of its block's queries in that slot it is.
+struct Slot_Place { u16 first, last; u32 rank; };
+
+__device__ __forceinline__ u64 slot_entry(const u32 k, const u64 J) { return u64(k) * J >> SLOT_BITS; }       // J < 2^40
+
+__global__ void __launch_bounds__(256) directory_kernel(const u64* __restrict__ table, const u64 J, u64* __restrict__ directory, u32* __restrict__ counts)
+{
+    const u32 k = blockIdx.x * 256 + threadIdx.x;
+    if(k < SLOTS) directory[k] = table[2 * slot_entry(k, J)];       // the first four symbols
+    if(k <= SLOTS) counts[k] = 0;
+}
+
+// off: the offsets of this share of the batch, off_first: the batch's first, where sym begins.
+// counts[s]: queries of slot s (there is one more than directory keys). before[block][s]: those of the slot in blocks that came earlier.
+__global__ void __launch_bounds__(SLOT_BLOCK) count_slots_kernel(const u64* __restrict__ directory, const u64* __restrict__ off, const u64* __restrict__ off_first, const u16* __restrict__ sym, const u64 q,
+                                                                Slot_Place* __restrict__ places, u32* __restrict__ counts, u32* __restrict__ before)
+{
+    extern __shared__ __align__(16) u64 dir[];
+    u32* const cnt = reinterpret_cast<u32*>(dir + SLOTS);
+    for(u32 k = threadIdx.x; k < SLOTS; k += SLOT_BLOCK) { dir[k] = directory[k]; cnt[k] = 0; }
+    if(threadIdx.x == 0) cnt[SLOTS] = 0;
+    __syncthreads();
+    const u64 off0 = *off_first;
+    for(u64 tile = blockIdx.x; tile * SLOT_TILE < q; tile += gridDim.x)
+        for(int k = 0; k < SLOT_ITEMS; ++k)
+        {
+            const u64 i = tile * SLOT_TILE + k * SLOT_BLOCK + threadIdx.x;
+            if(i >= q) break;
+            const u64 from = off[i], m = off[i + 1] - from;
+            u32 x = 0, z = 0;
+            if(m)
+            {
+                const Pattern p(sym + (from - off0), m);
+                #pragma unroll
+                for(u32 step = SLOTS / 2; step; step >>= 1) if((dir[x + step - 1] & p.mask_high) < p.high) x += step;
+                if(x == SLOTS - 1 && (dir[x] & p.mask_high) < p.high) ++x;
+                z = x;
+                u32 y = SLOTS;
+                for(u32 step = 1; z < y; step <<= 1)
+                {
+                    const u32 mid = min(z + step - 1, y - 1);
+                    if((dir[mid] & p.mask_high) <= p.high) z = mid + 1; else { y = mid; break; }
+                }
+                while(z < y)
+                {
+                    const u32 mid = (z + y) >> 1;
+                    if((dir[mid] & p.mask_high) <= p.high) z = mid + 1; else y = mid;
+                }
+            }
+            places[i] = Slot_Place{u16(x), u16(z), atomicAdd(&cnt[x], 1u)};
+        }
+    __syncthreads();
+    for(u32 k = threadIdx.x; k <= SLOTS; k += SLOT_BLOCK)
+    {
+        const u32 c = cnt[k];
+        if(c) before[u64(blockIdx.x) * (SLOTS + 1) + k] = atomicAdd(&counts[k], c);
+    }
+}
+
+// The queries in the order of their slots; the same blocks take the same queries as in the kernel above.
+__global__ void __launch_bounds__(SLOT_BLOCK) deal_slots_kernel(const u64* __restrict__ off, const u64* __restrict__ off_first, const u16* __restrict__ sym, const u64 q, const Slot_Place* __restrict__ places,
+                                                               const u32* __restrict__ counts, const u32* __restrict__ before, Slot_Query* __restrict__ dealt)
+{
+    __shared__ u32 first_of[SLOTS + 1];         // where the block's queries of a slot start
+    __shared__ u32 warp_tot[SLOT_BLOCK / 32];
+    constexpr u32 PER = (SLOTS + SLOT_BLOCK) / SLOT_BLOCK;
+    const u32 k0 = threadIdx.x * PER;
+    u32 c[PER], sum = 0;
+    #pragma unroll
+    for(u32 k = 0; k < PER; ++k) { c[k] = k0 + k <= SLOTS ? counts[k0 + k] : 0; sum += c[k]; }
+    u32 inc = sum;
+    #pragma unroll
+    for(int o = 1; o < 32; o <<= 1) { const u32 t = __shfl_up_sync(0xFFFFFFFFu, inc, o); if(int(lane_id()) >= o) inc += t; }
+    if(lane_id() == 31) warp_tot[threadIdx.x >> 5] = inc;
+    __syncthreads();
+    u32 run = inc - sum;
+    for(u32 w = 0; w < (threadIdx.x >> 5); ++w) run += warp_tot[w];
+    #pragma unroll
+    for(u32 k = 0; k < PER; ++k)
+        if(k0 + k <= SLOTS) { first_of[k0 + k] = run + before[u64(blockIdx.x) * (SLOTS + 1) + k0 + k]; run += c[k]; }       // a slot without queries of this block: not used
+    __syncthreads();
+    const u64 off0 = *off_first;
+    for(u64 tile = blockIdx.x; tile * SLOT_TILE < q; tile += gridDim.x)
+        #pragma unroll 2
+        for(int k = 0; k < SLOT_ITEMS; ++k)
+        {
+            const u64 i = tile * SLOT_TILE + k * SLOT_BLOCK + threadIdx.x;
+            if(i >= q) break;
+            const Slot_Place pl = places[i];
+            const u64 from = off[i], m = off[i + 1] - from;
+            Pattern p;
+            if(m) p = Pattern(sym + (from - off0), m);
+            const u64 at = (from - off0) | (m < LONG_PATTERN ? m : u64(LONG_PATTERN)) << 48;
+            uint4* const out = reinterpret_cast<uint4*>(dealt + first_of[pl.first] + pl.rank);
+            out[0] = make_uint4(u32(p.high), u32(p.high >> 32), u32(p.low), u32(p.low >> 32));
+            out[1] = make_uint4(u32(i), u32(pl.first) | u32(pl.last) << 16, u32(at), u32(at >> 32));
+        }
+}
+
+__global__ void __launch_bounds__(128) find_dealt_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const Slot_Query* __restrict__ dealt, const u64 q,
+                                                        u64* __restrict__ itv)
+{
+    const u64 t = u64(blockIdx.x) * 128 + threadIdx.x;
+    if(t >= q) return;
+    const uint4 r0 = __ldcs(reinterpret_cast<const uint4*>(dealt + t)), r1 = __ldcs(reinterpret_cast<const uint4*>(dealt + t) + 1);
+    const u64 i = r1.x, at = (u64(r1.w) << 32) | r1.z;
+    u64 m = at >> 48;
+    if(m == LONG_PATTERN) m = off[i + 1] - off[i];
+    ulonglong2 answer = make_ulonglong2(0, idx.n);
+    if(m)
+    {
+        const u16* const P = sym + (at & ((u64(1) << 48) - 1));
+        Pattern p;
+        p.set_length(m);
+        p.high = (u64(r0.y) << 32) | r0.x; p.low = (u64(r0.w) << 32) | r0.z;
+        const u64 J = (idx.n + idx.stride - 1) / idx.stride;
+        const u32 first = r1.y & 0xFFFFu, last = r1.y >> 16;
+        const u64 from = first ? slot_entry(first - 1, J) + 1 : 0, to = last < SLOTS ? slot_entry(last, J) : J;
+        // the directory holds four symbols of a key: of a shorter pattern it tells all
+        const u64 a1 = p.mask_low ? to : (first < SLOTS ? slot_entry(first, J) : J), b0 = p.mask_low || last == 0 ? from : slot_entry(last - 1, J) + 1;
+        const Brackets br = table_brackets(idx, p, from, a1, b0, to);
+        auto entry = [&](const u64 r) { return sa40_load_wide(idx.sa40, r); };
+        search_brackets(idx, br, p, P, entry, entry, answer.x, answer.y);
+    }
+    reinterpret_cast<ulonglong2*>(itv)[i] = answer;
 }
 
 // A warp per query, for batches that do not fill the device with a thread per query: what bounds those is a chain of 25 to 40 dependent
@@ -215,20 +447,23 @@ __global__ void __launch_bounds__(128) find_by_warp_kernel(const csa_index idx, 
     const u64 ne = idx.sa_entries ? idx.sa_entries : idx.n, n = idx.n;
     u64 lo = 0, hi = 0;
     if(m == 0) hi = ne;
-    else if(idx.sa_entries != 0 && idx.sa_entries < n && cmp_suffix_pattern(idx.text, n, sa40_load(idx.sa40, 0), P, m) > 0) {}      // a slice behind the pattern
-    else if(idx.sa_entries != 0 && idx.sa_entries < n && cmp_suffix_pattern(idx.text, n, sa40_load(idx.sa40, ne - 1), P, m) < 0) { lo = ne; hi = ne; }
     else
     {
-        const Table_Key key(P, m);
-        const u64 J = (ne + idx.stride - 1) / idx.stride;
-        const ulonglong2* const tab = reinterpret_cast<const ulonglong2*>(idx.table);
-        const u64 a = warp_partition_point(0, J, [&](const u64 j) { return key.less(tab[j]); });
-        const u64 b = warp_partition_point_near(a, J, [&](const u64 j) { return key.not_greater(tab[j]); });
-        const Brackets br = brackets_from(a, b, J, idx.stride, ne, P, m);
-        lo = warp_partition_point(br.lo_first, br.lo_last, [&](const u64 r) { return cmp_suffix_pattern(idx.text, n, sa40_load(idx.sa40, r), P, m) < 0; });
-        u64 x = br.hi_first > lo ? br.hi_first : lo;
-        if(x > br.hi_last) x = br.hi_last;
-        hi = warp_partition_point_near(x, br.hi_last, [&](const u64 r) { return cmp_suffix_pattern(idx.text, n, sa40_load(idx.sa40, r), P, m) <= 0; });
+        const Pattern p(P, m);
+        if(is_slice(idx) && p.compare(idx.text, n, sa40_load(idx.sa40, 0), P) > 0) {}      // a slice behind the pattern
+        else if(is_slice(idx) && p.compare(idx.text, n, sa40_load(idx.sa40, ne - 1), P) < 0) { lo = ne; hi = ne; }
+        else
+        {
+            const u64 J = (ne + idx.stride - 1) / idx.stride;
+            const ulonglong2* const tab = reinterpret_cast<const ulonglong2*>(idx.table);
+            const u64 a = warp_partition_point(0, J, [&](const u64 j) { return p.less(tab[j]); });
+            const u64 b = warp_partition_point_near(a, J, [&](const u64 j) { return p.not_greater(tab[j]); });
+            const Brackets br = brackets_from(a, b, J, idx.stride, ne, p);
+            lo = warp_partition_point(br.lo_first, br.lo_last, [&](const u64 r) { return p.compare(idx.text, n, sa40_load(idx.sa40, r), P) < 0; });
+            u64 x = br.hi_first > lo ? br.hi_first : lo;
+            if(x > br.hi_last) x = br.hi_last;
+            hi = warp_partition_point_near(x, br.hi_last, [&](const u64 r) { return p.compare(idx.text, n, sa40_load(idx.sa40, r), P) <= 0; });
+        }
     }
     if(lane_id() == 0) { itv[2 * i] = lo; itv[2 * i + 1] = hi; }
 }
@@ -251,7 +486,7 @@ __global__ void brackets_kernel(const csa_index idx, const u64* __restrict__ off
     if(i >= q) return;
     const u64 m = off[i + 1] - off[i];
     Brackets br{0, 0, 0, 0};
-    if(m > 0) br = table_brackets(idx, sym + (off[i] - off[0]), m);
+    if(m > 0) br = table_brackets(idx, Pattern(sym + (off[i] - off[0]), m));
     out[i] = br;
 }
 
@@ -294,7 +529,8 @@ __global__ void search_windows_kernel(const csa_index idx, const u64* __restrict
         sa_hi = win + (2 * i + (shared ? 0 : 1)) * WINDOW_BYTES - ((5 * br.hi_first) & ~u64(15));
     }
     u64 lo, hi;
-    search_brackets(idx, br, sym + (off[i] - off[0]), m, sa_lo, sa_hi, lo, hi);
+    const u16* const P = sym + (off[i] - off[0]);
+    search_brackets(idx, br, Pattern(P, m), P, [&](const u64 r) { return sa40_load(sa_lo, r); }, [&](const u64 r) { return sa40_load(sa_hi, r); }, lo, hi);
     itv[2 * i] = lo;
     itv[2 * i + 1] = hi;
 }
@@ -531,7 +767,59 @@ extern "C" int csa_locate_window_packed(csa_ctx* ctx, const csa_index* index, co
     return CSA_OK;
 }
 
-extern "C" int csa_find(csa_ctx* ctx, const csa_index* index, const uint64_t* off, const uint16_t* sym, uint64_t q, uint64_t* itv)
+namespace
+{
+
+// A batch by slots, 2^22 queries at a time (the scratch is bounded: 180 MB). done stays false where nothing was queued: no room for the scratch, a
+// stream that is being captured (an allocation is not allowed there), a slice of an index, a table without levels to share.
+constexpr u64 DEAL_MIN_QUERIES = u64(1) << 15, DEAL_CHUNK = u64(1) << 22;
+
+int find_dealt(csa_ctx* ctx, const csa_index& index, const u64* off, const u16* sym, const u64 q, u64* itv, bool& done)
+{
+    const u64 J = div_up(index.n, index.stride);
+    if((index.sa_entries != 0 && index.sa_entries < index.n) || J < 4 * SLOTS || J >= (u64(1) << 40)) return CSA_OK;
+    if(reinterpret_cast<uintptr_t>(itv) & 15) return CSA_OK;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if(cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) { cudaGetLastError(); return CSA_OK; }
+    if(capturing != cudaStreamCaptureStatusNone) return CSA_OK;
+    const u64 per = std::min(q, DEAL_CHUNK);
+    const unsigned most_blocks = unsigned(std::min<u64>(div_up(per, SLOT_TILE), 148 * 3));
+    const size_t b_dealt = align_up256(per * sizeof(Slot_Query)), b_places = align_up256(per * sizeof(Slot_Place)), b_dir = align_up256(SLOTS * 8), b_counts = align_up256((SLOTS + 1) * 4),
+                 b_before = align_up256(size_t(most_blocks) * (SLOTS + 1) * 4);
+    void* aux = nullptr;
+    const std::string err = ctx->err;
+    if(const int rc = csa_aux(ctx, b_dealt + b_places + b_dir + b_counts + b_before, &aux)) { if(rc != CSA_E_NOMEM) return rc; ctx->err = err; return CSA_OK; }
+    u8* at = static_cast<u8*>(aux);
+    Slot_Query* const dealt = reinterpret_cast<Slot_Query*>(at); at += b_dealt;
+    Slot_Place* const places = reinterpret_cast<Slot_Place*>(at); at += b_places;
+    u64* const directory = reinterpret_cast<u64*>(at); at += b_dir;
+    u32* const counts = reinterpret_cast<u32*>(at); at += b_counts;
+    u32* const before = reinterpret_cast<u32*>(at);
+    static std::atomic<bool> configured[64];
+    if(!configured[ctx->device & 63])
+    {
+        CSA_CUDA(ctx, cudaFuncSetAttribute(count_slots_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SLOT_SMEM)));
+        configured[ctx->device & 63] = true;
+    }
+    for(u64 first = 0; first < q; first += per)
+    {
+        const u64 c = std::min(per, q - first);
+        const unsigned blocks = unsigned(std::min<u64>(div_up(c, SLOT_TILE), most_blocks));
+        directory_kernel<<<unsigned(div_up(SLOTS + 1, 256)), 256, 0, ctx->stream>>>(reinterpret_cast<const u64*>(index.table), J, directory, counts);
+        CSA_LAUNCH_CHECK(ctx);
+        count_slots_kernel<<<blocks, SLOT_BLOCK, SLOT_SMEM, ctx->stream>>>(directory, off + first, off, sym, c, places, counts, before);
+        CSA_LAUNCH_CHECK(ctx);
+        deal_slots_kernel<<<blocks, SLOT_BLOCK, 0, ctx->stream>>>(off + first, off, sym, c, places, counts, before, dealt);
+        CSA_LAUNCH_CHECK(ctx);
+        find_dealt_kernel<<<unsigned(div_up(c, 128)), 128, 0, ctx->stream>>>(index, off + first, sym, dealt, c, itv + 2 * first);
+        CSA_LAUNCH_CHECK(ctx);
+    }
+    done = true;
+    return CSA_OK;
+}
+
+// may_deal: the context's second buffer is free for the batch's scratch (the lanes of a host batch share it).
+int find_batch(csa_ctx* ctx, const csa_index* index, const uint64_t* off, const uint16_t* sym, uint64_t q, uint64_t* itv, const bool may_deal)
 {
     CSA_TRY(check_index(ctx, index));
     if(q == 0) return CSA_OK;
@@ -542,6 +830,12 @@ extern "C" int csa_find(csa_ctx* ctx, const csa_index* index, const uint64_t* of
     cudaGetLastError();
     if(!sa_on_host)
     {
+        if(q >= DEAL_MIN_QUERIES && may_deal)
+        {
+            bool done = false;
+            CSA_TRY(find_dealt(ctx, *index, reinterpret_cast<const u64*>(off), sym, q, reinterpret_cast<u64*>(itv), done));
+            if(done) return CSA_OK;
+        }
         if(q <= WARP_QUERIES) find_by_warp_kernel<<<unsigned(div_up(q, 4)), 128, 0, ctx->stream>>>(*index, reinterpret_cast<const u64*>(off), sym, q, reinterpret_cast<u64*>(itv));
         else find_kernel<<<unsigned(div_up(q, 128)), 128, 0, ctx->stream>>>(*index, reinterpret_cast<const u64*>(off), sym, q, reinterpret_cast<u64*>(itv));
         CSA_LAUNCH_CHECK(ctx);
@@ -578,6 +872,13 @@ extern "C" int csa_find(csa_ctx* ctx, const csa_index* index, const uint64_t* of
         CSA_LAUNCH_CHECK(ctx);
     }
     return CSA_OK;
+}
+
+}   // namespace
+
+extern "C" int csa_find(csa_ctx* ctx, const csa_index* index, const uint64_t* off, const uint16_t* sym, uint64_t q, uint64_t* itv)
+{
+    return find_batch(ctx, index, off, sym, q, itv, true);
 }
 
 extern "C" int csa_locate(csa_ctx* ctx, const csa_index* index, const uint64_t* itv, uint64_t q, uint32_t max_pos, uint64_t* pos, uint32_t* cnt)
@@ -686,7 +987,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
         const On_Stream on(ctx, ctx->lane[l]);
         CSA_CUDA(ctx, cudaMemcpyAsync(L[l].off, off_host + first, (cq + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
         if(sc) CSA_CUDA(ctx, cudaMemcpyAsync(L[l].sym, sym_host + (off_host[first] - off_host[0]), sc * 2, cudaMemcpyHostToDevice, ctx->stream));
-        CSA_TRY(csa_find(ctx, index, reinterpret_cast<uint64_t*>(L[l].off), L[l].sym, cq, reinterpret_cast<uint64_t*>(L[l].itv)));
+        CSA_TRY(find_batch(ctx, index, reinterpret_cast<uint64_t*>(L[l].off), L[l].sym, cq, reinterpret_cast<uint64_t*>(L[l].itv), false));
         CSA_CUDA(ctx, cudaMemcpyAsync(itv_host + 2 * first, L[l].itv, cq * 16, cudaMemcpyDeviceToHost, ctx->stream));
         if(want_pos)
         {
