@@ -12,6 +12,7 @@
 #include "prefix_sort.cuh"
 #include "refine.cuh"
 #include "sort.cuh"
+#include "tiny_build.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -179,6 +180,29 @@ struct Build
     }
 };
 
+// The whole build in one block, where the text fits one and is not repetitive (done). The counters come straight into pinned memory.
+int build_in_one_block(csa_ctx* ctx, const u16* T, const u64 n, u32 p, u8* sa40, csa_build_stats& st, bool& done)
+{
+    Tiny_Result* const result = reinterpret_cast<Tiny_Result*>(ctx->h_scalars + CSA_COUNTS_WORD);
+    cudaEvent_t* const ev = ctx->phase_event;
+    CSA_TRY(launch_tiny_build(ctx, T, n, sa40, p, prefix_sort_plan(n).b2, result));
+    CSA_CUDA(ctx, cudaEventRecord(ev[4], ctx->stream));
+    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if(result->status != 0) { u64 b = 0; return csa_sync(ctx, reinterpret_cast<uint64_t*>(&b)); }
+    done = result->done != 0;
+    if(!done) return CSA_OK;
+    st.partitions = result->partitions;
+    st.max_partition = result->max_partition;
+    st.active_after_gen0 = result->tied;
+    if(result->tied) { st.generations = 1; st.active_per_gen[0] = result->tied; }
+    ctx->counters[1] += 1;
+    ctx->counters[2] += n;
+    float ms = 0;
+    cudaEventElapsedTime(&ms, ev[0], ev[4]);
+    st.ms_gen0 = st.ms_total = ms;
+    return CSA_OK;
+}
+
 int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u8* sa40, csa_build_stats* stats, void* ws, size_t ws_bytes)
 {
     (void)seed;         // drives the sampling of splitters in the sharded and part-at-a-time builds; this build's sample is the same for all seeds
@@ -192,6 +216,19 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     for(auto& e : ctx->phase_event) if(!e) CSA_CUDA(ctx, cudaEventCreate(&e));
     cudaEvent_t* const ev = ctx->phase_event;
     CSA_CUDA(ctx, cudaEventRecord(ev[0], ctx->stream));
+
+    if(n <= TINY_BUILD_MAX)
+    {
+        bool done = false;
+        CSA_TRY(build_in_one_block(ctx, T, n, p, sa40, st, done));
+        if(done)
+        {
+            st.kernel_launches = ctx->counters[0] - launches_before;
+            st.sort_passes = ctx->counters[1] - passes_before;
+            st.sort_records = ctx->counters[2] - records_before;
+            return CSA_OK;
+        }
+    }
 
     Build b{ctx, T, n, layout_for(n), prefix_sort_plan(n)};
     Carver cv(ws, ws_bytes);
