@@ -927,6 +927,140 @@ struct Lane_Buffers
     u64* off; u16* sym; u64* itv; u32* cnt; u64* poff; u64* sums; u64* pos;
 };
 
+// ---- small host batches --------------------------------------------------------------------------------------------------------
+//
+// Of a batch that a warp per query answers, copies, launches and waits take longer than the search. Here it is two launches and one wait: the answers
+// are written straight into pinned host memory, the positions of a query behind those of the queries before it, whose counts a block adds up by
+// itself. (50 queries: 89 us a call with five copies, six launches and two waits, this way 35 us; 1000: 111 and 41 us, 8000: 120 and 62 us.)
+constexpr int ANSWER_BLOCK = 256, ANSWER_QUERIES = 32;
+
+// What an answer goes to; cnt, pos_off and pos may be null together.
+struct Answers { u64* itv; u32* cnt; u64* pos_off; u64* pos; u64 pos_capacity; u64* status; };
+
+__global__ void __launch_bounds__(ANSWER_BLOCK) answers_kernel(const u8* __restrict__ sa40, const ulonglong2* __restrict__ itv, const u32 q, const u32 max_pos, const u64* __restrict__ status,
+                                                              const Answers out)
+{
+    __shared__ u64 sums[ANSWER_BLOCK / 32];
+    __shared__ u64 at[ANSWER_QUERIES];
+    __shared__ ulonglong2 mine[ANSWER_QUERIES];
+    const u32 tid = threadIdx.x, first = blockIdx.x * ANSWER_QUERIES, warp = tid >> 5;
+    auto rows = [&](const ulonglong2 v) { const u64 d = v.y - v.x; return d < max_pos ? d : u64(max_pos); };
+    u64 before = 0;
+    if(out.pos)
+    {
+        for(u32 i = tid; i < first; i += ANSWER_BLOCK) before += rows(itv[i]);
+        #pragma unroll
+        for(int o = 16; o; o >>= 1) before += __shfl_xor_sync(0xFFFFFFFFu, before, o);
+        if(lane_id() == 0) sums[warp] = before;
+        __syncthreads();
+        before = 0;
+        #pragma unroll
+        for(int w = 0; w < ANSWER_BLOCK / 32; ++w) before += sums[w];
+    }
+    if(warp == 0)
+    {
+        const u32 i = first + tid;
+        const ulonglong2 v = i < q ? itv[i] : make_ulonglong2(0, 0);
+        const u64 c = out.pos ? rows(v) : 0;
+        u64 inc = c;
+        #pragma unroll
+        for(int o = 1; o < 32; o <<= 1) { const u64 t = __shfl_up_sync(0xFFFFFFFFu, inc, o); if(int(tid) >= o) inc += t; }
+        mine[tid] = v;
+        at[tid] = before + inc - c;
+        if(i < q)
+        {
+            out.itv[2 * i] = v.x;
+            out.itv[2 * i + 1] = v.y;
+            if(out.pos) { out.cnt[i] = u32(c); out.pos_off[i] = before + inc - c; }
+            if(i == q - 1)
+            {
+                if(out.pos) out.pos_off[q] = before + inc;
+                *out.status = *status;
+            }
+        }
+    }
+    if(!out.pos) return;
+    __syncthreads();
+    for(u32 k = warp; k < ANSWER_QUERIES; k += ANSWER_BLOCK / 32)
+    {
+        const ulonglong2 v = mine[k];
+        const u64 c = rows(v), o = at[k];
+        for(u64 r = lane_id(); r < c; r += 32) if(o + r < out.pos_capacity) out.pos[o + r] = sa40_load(sa40, v.x + r);
+    }
+}
+
+// The address by which the device reads and writes host memory, null for memory that is not pinned.
+template <typename T>
+T* pinned(T* host)
+{
+    cudaPointerAttributes attr;
+    const bool yes = host && cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return yes ? static_cast<T*>(attr.devicePointer) : nullptr;
+}
+
+constexpr u64 STAGED_MAX = u64(1) << 20;        // bytes of a batch from or to pageable memory that are copied by way of pinned scratch
+constexpr u64 READ_IN_PLACE = 256;              // queries that are read from pinned memory by the search itself: above that a copy costs less than the reads over PCIe
+
+// A host batch of up to WARP_QUERIES queries, the array in device memory (done). Not taken: pageable buffers of a batch that is too large to be staged.
+int query_host_small(csa_ctx* ctx, const csa_index* index, const u64* off_host, const u16* sym_host, const u64 q, const u32 max_pos, u64* itv_host, u32* cnt_host, u64* pos_off_host,
+                     u64* pos_host, const u64 pos_capacity, u64& total, bool& done)
+{
+    const bool want_pos = pos_host != nullptr;
+    if(off_host[q] < off_host[0]) return csa_fail(ctx, CSA_E_INVALID, "csa_query_host: offsets must not decrease");
+    const u64 symbols = off_host[q] - off_host[0];
+    const u64 most = want_pos ? std::min(pos_capacity, q * max_pos) : 0;
+    if(symbols && !sym_host) return CSA_OK;
+    const u64* off = pinned(const_cast<u64*>(off_host));
+    const u16* sym = symbols ? pinned(const_cast<u16*>(sym_host)) : nullptr;
+    Answers out{pinned(itv_host), want_pos ? pinned(cnt_host) : nullptr, want_pos ? pinned(pos_off_host) : nullptr, want_pos ? pinned(pos_host) : nullptr, pos_capacity,
+                ctx->h_scalars + CSA_STATUS_WORD};
+    // pinned scratch for what is not pinned
+    const size_t b_off = off ? 0 : align_up256((q + 1) * 8), b_sym = sym || !symbols ? 0 : align_up256(symbols * 2), b_itv = out.itv ? 0 : align_up256(q * 16),
+                 b_cnt = !want_pos || out.cnt ? 0 : align_up256(q * 4), b_poff = !want_pos || out.pos_off ? 0 : align_up256((q + 1) * 8),
+                 b_pos = !want_pos || out.pos ? 0 : align_up256(most * 8 + 8);
+    const size_t staged = b_off + b_sym + b_itv + b_cnt + b_poff + b_pos;
+    if(staged > STAGED_MAX) return CSA_OK;
+    void* host_ws = nullptr;
+    if(staged) CSA_TRY(csa_host_aux(ctx, staged, &host_ws));
+    u8* p = static_cast<u8*>(host_ws);
+    if(b_off) { std::memcpy(p, off_host, (q + 1) * 8); off = reinterpret_cast<u64*>(p); p += b_off; }
+    if(b_sym) { std::memcpy(p, sym_host, symbols * 2); sym = reinterpret_cast<u16*>(p); p += b_sym; }
+    if(b_itv) { out.itv = reinterpret_cast<u64*>(p); p += b_itv; }
+    if(b_cnt) { out.cnt = reinterpret_cast<u32*>(p); p += b_cnt; }
+    if(b_poff) { out.pos_off = reinterpret_cast<u64*>(p); p += b_poff; }
+    if(b_pos) { out.pos = reinterpret_cast<u64*>(p); out.pos_capacity = most; }
+
+    const size_t d_itv = align_up256(q * 16), d_off = align_up256((q + 1) * 8), d_sym = align_up256(symbols * 2 + 16);
+    void* ws = nullptr;
+    CSA_TRY(csa_arena(ctx, d_itv + d_off + d_sym, &ws));
+    u64* const itv = static_cast<u64*>(ws);
+    if(q > READ_IN_PLACE)
+    {
+        u64* const off_dev = reinterpret_cast<u64*>(static_cast<u8*>(ws) + d_itv);
+        u16* const sym_dev = reinterpret_cast<u16*>(static_cast<u8*>(ws) + d_itv + d_off);
+        CSA_CUDA(ctx, cudaMemcpyAsync(off_dev, off, (q + 1) * 8, cudaMemcpyDefault, ctx->stream));
+        if(symbols) CSA_CUDA(ctx, cudaMemcpyAsync(sym_dev, sym, symbols * 2, cudaMemcpyDefault, ctx->stream));
+        off = off_dev; sym = sym_dev;
+    }
+    find_by_warp_kernel<<<unsigned(div_up(q, 4)), 128, 0, ctx->stream>>>(*index, off, sym, q, itv);
+    CSA_LAUNCH_CHECK(ctx);
+    answers_kernel<<<unsigned(div_up(q, ANSWER_QUERIES)), ANSWER_BLOCK, 0, ctx->stream>>>(index->sa40, reinterpret_cast<const ulonglong2*>(itv), u32(q), max_pos, ctx->d_status, out);
+    CSA_LAUNCH_CHECK(ctx);
+    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    done = true;
+    if(b_itv) std::memcpy(itv_host, out.itv, q * 16);
+    if(want_pos)
+    {
+        total = (b_poff ? out.pos_off : pos_off_host)[q];
+        if(b_cnt) std::memcpy(cnt_host, out.cnt, q * 4);
+        if(b_poff) std::memcpy(pos_off_host, out.pos_off, (q + 1) * 8);
+        if(b_pos && total <= most) std::memcpy(pos_host, out.pos, total * 8);
+    }
+    if(ctx->h_scalars[CSA_STATUS_WORD] != 0) { u64 bits = 0; return csa_sync(ctx, reinterpret_cast<uint64_t*>(&bits)); }
+    return CSA_OK;
+}
+
 }   // namespace
 
 // The host batch runs as chunks of 2^18 queries over three streams, as Query_Engine::find does (src/Query_Engine.cu:1355-1516):
@@ -942,11 +1076,24 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
     if(!off_host || !itv_host) return csa_fail(ctx, CSA_E_INVALID, "csa_query_host: null buffer");
     const bool want_pos = max_pos > 0 && pos_host && cnt_host && pos_off_host;
     CSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    CSA_TRY(csa_lanes(ctx));
     // With the suffix array in host memory the search itself uses the context's one window buffer: one lane then.
     cudaPointerAttributes attr;
     const bool sa_on_host = cudaPointerGetAttributes(&attr, index->sa40) == cudaSuccess && attr.type == cudaMemoryTypeHost;
     cudaGetLastError();
+    if(!sa_on_host && q <= WARP_QUERIES)
+    {
+        u64 total = 0;
+        bool done = false;
+        CSA_TRY(query_host_small(ctx, index, reinterpret_cast<const u64*>(off_host), sym_host, q, max_pos, reinterpret_cast<u64*>(itv_host), want_pos ? cnt_host : nullptr,
+                                 want_pos ? reinterpret_cast<u64*>(pos_off_host) : nullptr, want_pos ? reinterpret_cast<u64*>(pos_host) : nullptr, pos_capacity, total, done));
+        if(done)
+        {
+            if(pos_total && want_pos) *pos_total = total;
+            if(want_pos && total > pos_capacity) return csa_fail(ctx, CSA_E_NOMEM, "csa_query_host: the positions buffer is too small");
+            return CSA_OK;
+        }
+    }
+    CSA_TRY(csa_lanes(ctx));
     const u64 chunks = div_up(q, HOST_CHUNK_QUERIES);
     const int lanes = sa_on_host ? 1 : int(chunks < u64(csa_ctx::LANES) ? chunks : u64(csa_ctx::LANES));
     const u64 cq_max = q < HOST_CHUNK_QUERIES ? q : HOST_CHUNK_QUERIES;
