@@ -29,8 +29,6 @@ constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of
 constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
-constexpr int LOCAL_ITEMS = 16;
-template <int BLOCK> constexpr int LOCAL_CAP = BLOCK * LOCAL_ITEMS;     // records that a block of the local sort holds
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
 constexpr u32 LOCAL_CHUNK = 2048, SHORT_CHUNK = 1024;
 
@@ -599,9 +597,12 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
 
 // ---- local sort: runs of children in shared memory --------------------------------------------------------------------------------
 
-template <int BLOCK> constexpr size_t LOCAL_SMEM = size_t(LOCAL_CAP<BLOCK>) * 8 + (LOCAL_CAP<BLOCK> / 2 + 4) * 4 + ((1 << MAX_B2) + 4) * 4;
+template <int BLOCK, int ITEMS> constexpr size_t LOCAL_SMEM = size_t(BLOCK * ITEMS) * 8 + (BLOCK * ITEMS / 2 + 8) * 4 + ((1 << MAX_B2) + 4) * 4;
+constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
+constexpr u32 CROWDED_BIN = 8;      // a batch with larger bins is looked through for bins of one key
+constexpr u32 MANY_TIED = 256;      // a batch with more tied records writes them to the list side by side
 constexpr u32 LONG_BIN = 256;       // a bin with more records is not ordered by comparing all with all
-static_assert(LOCAL_CAP<512> <= 8192, "slots of a batch take 13 bits");
+static_assert(MEDIUM_CAP <= 8192, "slots of a batch take 13 bits");
 
 // A record's place in its batch (13 bits), then the first place of its group or, where that is its own, the group's size (14 bits)
 // and FIRST; SMALL or LARGE by the group's size, neither for a record that is alone.
@@ -611,30 +612,32 @@ __device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, con
     return place | (place == head ? size << 13 | PL_FIRST : head << 13) | (size == 1 ? 0u : (size <= SMALL_GROUP ? PL_SMALL : PL_LARGE));
 }
 
-// What bounds it is latency and the issue of instructions, not memory (12 bytes a record at 0.9 TB/s): a block goes through
-// barriers between dependent steps. So a block finds its children in two dependent reads (chunk_first, child_off), tied records get
-// their list places from one counter in shared memory, and four small blocks share an SM (two of 512 threads: 27.7 ms at 2e9
-// records, four of 256: 24.5 ms, and 0.5 ms for the children that need the larger ones). A block reads its next chunk ahead (2^24 tokens: 618 -> 605 us a build).
+// What bounds it is the issue of instructions (7 a record and warp, 68 % of the cycles), then barriers between dependent steps; memory is not (12 bytes a
+// record). So a block finds its children in two dependent reads (chunk_first, child_off), records stay with their threads and only keys are staged,
+// what only tied records need is skipped by warps without any, and three blocks of 512 threads with up to 8 records each share an SM (two such blocks
+// 4.70 ms a build of 2e8 tokens, three 4.67 and with shorter sums of the bins 4.55; blocks of 256 with 16 records, four to an SM, 5.51, with 8 records 4.75; every record staged
+// whole and looked up again by its place 5.17). A block reads its next chunk ahead.
 // MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
-// there if a block of 512 threads holds them, and to the front, for the radix sort, if not.
-constexpr u32 MEDIUM_CAP = LOCAL_CAP<512>;
-template <int BLOCK, bool MEDIUM>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
+// there if a block of 16 records a thread holds them, and to the front, for the radix sort, if not.
+template <int BLOCK, int ITEMS, int BLOCKS, bool MEDIUM>
+__global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
                                                                    const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u64* __restrict__ list,
                                                                    const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap)
 {
-    constexpr int LOCAL_BLOCK = BLOCK, LOCAL_CAP = BLOCK * LOCAL_ITEMS;
+    constexpr int CAP = BLOCK * ITEMS;
+    static_assert(ITEMS % 8 == 0, "a thread sums whole 16-byte pieces of the bins' counts");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    u64* const stage = reinterpret_cast<u64*>(smem_raw);                            // [LOCAL_CAP]
-    u32* const bin = reinterpret_cast<u32*>(stage + LOCAL_CAP);                      // [LOCAL_CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
+    u32* const keys = reinterpret_cast<u32*>(smem_raw);                             // [CAP]
+    u32* const placed = keys + CAP;                                                 // [CAP] positions in their order
+    u32* const bin = placed + CAP;                                                  // [CAP / 2 + 8]: two 16-bit counters a word, then the bins' starts
     u16* const start = reinterpret_cast<u16*>(bin);
-    u32* const coff = bin + LOCAL_CAP / 2 + 4;                                       // [children of the chunk + 1] their offsets
-    __shared__ u32 warp_tot[LOCAL_BLOCK / 32];
+    u32* const coff = bin + CAP / 2 + 8;                                            // [children of the chunk + 1] their offsets
+    __shared__ u32 warp_tot[BLOCK / 32];
     __shared__ u32 s_tied[2], s_slot[2];            // records of small and of large groups in the batch, and their places in the list
+    __shared__ u32 mixed[CAP / 32], s_crowded;      // a bit per bin: it holds several keys; whether any bin holds many records
     const u32 tid = threadIdx.x;
     const u32 children = 1u << bits;
     const int rbits = 32 - bits;                    // key bits behind the child's
-    const u32 rmask = rbits == 32 ? 0xFFFFFFFFu : (1u << rbits) - 1;
 
     const u32 works = MEDIUM ? counts->medium : *chunks;
     u32 next_first = 0, next_end = 0;       // the children of the chunk after this one, read ahead
@@ -652,7 +655,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
         const bool more = work + gridDim.x < works;
         if(more) look_up(work + gridDim.x);
         const u32 first_digit = child0 & (children - 1);
-        for(u32 d = tid; d <= last; d += LOCAL_BLOCK) coff[d] = __ldg(child_off + child0 + d);
+        for(u32 d = tid; d <= last; d += BLOCK) coff[d] = __ldg(child_off + child0 + d);
         if(tid < 2) s_tied[tid] = 0;
         __syncthreads();
         u32 cur = 0;
@@ -667,13 +670,13 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
             // a batch: as many children as fit
             u32 e = last;
             const u32 base = coff[cur];
-            if(coff[e] - base > u32(LOCAL_CAP))
+            if(coff[e] - base > u32(CAP))
             {
-                u32 a = cur, b = last;                  // the last e with coff[e] - base <= LOCAL_CAP
+                u32 a = cur, b = last;                  // the last e with coff[e] - base <= CAP
                 while(b - a > 1)
                 {
                     const u32 m = (a + b) >> 1;
-                    if(coff[m] - base <= u32(LOCAL_CAP)) a = m; else b = m;
+                    if(coff[m] - base <= u32(CAP)) a = m; else b = m;
                 }
                 e = a;
                 if(e == cur)
@@ -694,46 +697,50 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                 }
             }
             const u32 m = coff[e] - base;
+            const bool single = e - cur == 1;
             cur = e;
             if(m == 0) continue;
 
             // Bins: a record's place inside its child by interpolation of its remaining key bits; there are as many bins as records.
-            for(u32 i = tid; i < ((m + 1) / 2 + 7) / 8 * 2; i += LOCAL_BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
-            u64 r[LOCAL_ITEMS];
-            u32 pl[LOCAL_ITEMS];                // bin << 16 | rank in the bin; later packed_place
+            for(u32 i = tid; i < (m / 2 + 8) / 8 * 2; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+            if(tid < CAP / 32) mixed[tid] = 0;
+            if(tid == 0) s_crowded = 0;
+            u64 r[ITEMS];
+            u32 pl[ITEMS];                      // bin << 16 | rank in the bin; of tied records later packed_place
             #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            for(int i = 0; i < ITEMS; ++i)
             {
-                if(i * LOCAL_BLOCK >= m) break;          // of all threads: half of a full batch is the rule
-                const u32 j = tid + i * LOCAL_BLOCK;
+                if(i * BLOCK >= m) break;       // of all threads: half of a full batch is the rule
+                const u32 j = tid + i * BLOCK;
                 if(j < m) r[i] = rec[base + j];
             }
             __syncthreads();
-            auto bin_of = [&](const u32 key) -> u32
-            {
-                const u32 d = (bits ? key >> rbits : 0u) - first_digit;
-                const u32 c0 = coff[d];
-                return c0 - base + u32((u64(key & rmask) * (coff[d + 1] - c0)) >> rbits);
-            };
             #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            for(int i = 0; i < ITEMS; ++i)
             {
-                if(i * LOCAL_BLOCK >= m) break;
-                if(tid + i * LOCAL_BLOCK < m)
+                if(i * BLOCK >= m) break;
+                if(tid + i * BLOCK < m)
                 {
-                    const u32 b = bin_of(u32(r[i] >> 32));
+                    const u32 k = u32(r[i] >> 32);
+                    u32 b;
+                    if(single) b = __umulhi(k << bits, m);
+                    else
+                    {
+                        const u32 d = (bits ? k >> rbits : 0u) - first_digit, c0 = coff[d];
+                        b = c0 - base + __umulhi(k << bits, coff[d + 1] - c0);
+                    }
                     const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
                     pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
                 }
             }
             __syncthreads();
             // exclusive sums of the bins' counts, in place; start[m] = m
-            u32 longest = 0;
+            u32 longest = 0;        // of the even and of the odd bins
             {
-                constexpr int WORDS = LOCAL_CAP / 2 / LOCAL_BLOCK;      // 8 words, 16 bins a thread
+                constexpr int WORDS = CAP / 2 / BLOCK;
                 u32 c[WORDS], sum = 0;
                 const u32 w0 = tid * WORDS;
-                const bool any = 2 * w0 < m;            // the words up to a multiple of WORDS were cleared
+                const bool any = 2 * w0 <= m;           // the words up to a multiple of WORDS were cleared
                 if(any)
                 {
                     #pragma unroll
@@ -744,60 +751,90 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                     }
                     u32 both = 0;           // two sums side by side: below 2^16 each
                     #pragma unroll
-                    for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16)); }
+                    for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = __vmaxu2(longest, c[k]); }
                     sum = (both & 0xFFFFu) + (both >> 16);
                 }
-                u32 total;
-                u32 run = block_exclusive<LOCAL_BLOCK>(sum, warp_tot, total);
+                const u32 inc = warp_inclusive(sum);
+                if(lane_id() == 31) warp_tot[tid >> 5] = inc;
+                __syncthreads();
+                u32 run = __reduce_add_sync(0xFFFFFFFFu, lane_id() < (tid >> 5) ? warp_tot[lane_id()] : 0u) + inc - sum;
                 if(any)
                 {
                     #pragma unroll
                     for(int k = 0; k < WORDS; ++k)
                     {
-                        const u32 a = run, b = run + (c[k] & 0xFFFFu);
-                        run = b + (c[k] >> 16);
-                        c[k] = a | (b << 16);
+                        const u32 a = run * 0x10001u + (c[k] << 16);        // below 2^16 each
+                        run += (c[k] & 0xFFFFu) + (c[k] >> 16);
+                        c[k] = a;
                     }
                     #pragma unroll
                     for(int k = 0; k < WORDS / 4; ++k)
                         reinterpret_cast<uint4*>(bin)[tid * (WORDS / 4) + k] = make_uint4(c[4 * k], c[4 * k + 1], c[4 * k + 2], c[4 * k + 3]);
                 }
-                __syncthreads();
-                if(tid == 0) start[m] = u16(m);
             }
+            if(m == u32(CAP) && tid == 0) start[CAP] = u16(CAP);       // behind the threads' words
+            longest = max(longest & 0xFFFFu, longest >> 16);
+            if(longest > CROWDED_BIN) s_crowded = 1;
             const bool by_network = __syncthreads_or(longest > LONG_BIN);
-            #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
-            {
-                if(i * LOCAL_BLOCK >= m) break;
-                if(tid + i * LOCAL_BLOCK < m) stage[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = r[i];
-            }
-            __syncthreads();
-
+            u32 tied = 0;           // a bit per record
             if(!by_network)
             {
-                // Order inside the bins: a record counts the smaller and the equal keys of its bin.
+                // Only the keys are staged, in their bins; a record stays with its thread and counts the smaller and the equal keys of its bin.
                 #pragma unroll
-                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                for(int i = 0; i < ITEMS; ++i)
                 {
-                    const u32 j = tid + i * LOCAL_BLOCK;
-                    if(j >= m) break;
-                    const u64 v = stage[j];
-                    const u32 key = u32(v >> 32);
-                    const u32 b = bin_of(key);
-                    const u32 s = start[b], t = start[b + 1];
-                    u32 less = 0, eq_before = 0, eq = 0;
-                    for(u32 k = s; k < t; ++k)
+                    if(i * BLOCK >= m) break;
+                    if(tid + i * BLOCK < m) keys[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = u32(r[i] >> 32);
+                }
+                __syncthreads();
+                // Bins of many records are as a rule copies of one key (documents that occur many times): their places are known then.
+                const bool crowded = s_crowded != 0;
+                if(crowded)
+                {
+                    #pragma unroll
+                    for(int i = 0; i < ITEMS; ++i)
                     {
-                        const u32 o = u32(stage[k] >> 32);
-                        less += o < key;
-                        const u32 same = o == key;
-                        eq += same;
-                        eq_before += same && k < j;
+                        if(i * BLOCK >= m) break;
+                        if(tid + i * BLOCK < m)
+                        {
+                            const u32 b = pl[i] >> 16;
+                            if(keys[start[b]] != u32(r[i] >> 32)) atomicOr(&mixed[b >> 5], 1u << (b & 31));
+                        }
                     }
-                    const u32 place = s + less + eq_before;
-                    pl[i] = packed_place(place, s + less, eq);
-                    sa[base + place] = eq == 1 ? u32(v) : SA_OPEN;
+                    __syncthreads();
+                }
+                #pragma unroll
+                for(int i = 0; i < ITEMS; ++i)
+                {
+                    if(i * BLOCK >= m) break;
+                    if(tid + i * BLOCK < m)
+                    {
+                        const u32 k = u32(r[i] >> 32), b = pl[i] >> 16, s = start[b], t = start[b + 1];
+                        u32 less = 0, upto = 0;
+                        if(crowded && t - s > 1 && (mixed[b >> 5] >> (b & 31) & 1u) == 0)
+                        {
+                            const u32 place = s + (pl[i] & 0xFFFFu);
+                            placed[place] = SA_OPEN;
+                            pl[i] = packed_place(place, s, t - s);
+                            tied |= 1u << i;
+                            continue;
+                        }
+                        #pragma unroll
+                        for(u32 j = 0; j < 4; ++j)      // most bins hold no more: four reads in flight
+                            if(s + j < t) { const u32 o = keys[s + j]; less += o < k; upto += o <= k; }
+                        for(u32 j = s + 4; j < t; ++j) { const u32 o = keys[j]; less += o < k; upto += o <= k; }
+                        const u32 head = s + less;
+                        if(upto - less == 1) placed[head] = u32(r[i]);
+                        else
+                        {
+                            const u32 mine = s + (pl[i] & 0xFFFFu);
+                            u32 place = head;
+                            for(u32 j = s; j < mine; ++j) place += keys[j] == k;
+                            placed[place] = SA_OPEN;
+                            pl[i] = packed_place(place, head, upto - less);
+                            tied |= 1u << i;
+                        }
+                    }
                 }
             }
             else
@@ -806,48 +843,63 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                 // group's ends by bisection.
                 u32 size = 1;
                 while(size < m) size <<= 1;
-                for(u32 j = m + tid; j < size; j += LOCAL_BLOCK) stage[j] = ~0ull;
+                #pragma unroll
+                for(int i = 0; i < ITEMS; ++i)
+                {
+                    const u32 j = tid + i * BLOCK;
+                    if(j >= size) break;
+                    keys[j] = j < m ? u32(r[i] >> 32) : 0xFFFFFFFFu;
+                    placed[j] = j < m ? u32(r[i]) : 0xFFFFFFFFu;        // no position: behind all records
+                }
                 __syncthreads();
                 for(u32 k = 2; k <= size; k <<= 1)
                     for(u32 d = k >> 1; d > 0; d >>= 1)
                     {
-                        for(u32 t = tid; t < size / 2; t += LOCAL_BLOCK)
+                        for(u32 t = tid; t < size / 2; t += BLOCK)
                         {
                             const u32 a = 2 * t - (t & (d - 1)), b = a + d;
-                            const u64 x = stage[a], y = stage[b];
-                            if((x > y) == ((a & k) == 0)) { stage[a] = y; stage[b] = x; }
+                            const u32 x = keys[a], y = keys[b], px = placed[a], py = placed[b];
+                            if((x > y || (x == y && px > py)) == ((a & k) == 0)) { keys[a] = y; keys[b] = x; placed[a] = py; placed[b] = px; }
                         }
                         __syncthreads();
                     }
                 #pragma unroll
-                for(int i = 0; i < LOCAL_ITEMS; ++i)
+                for(int i = 0; i < ITEMS; ++i)
                 {
-                    const u32 j = tid + i * LOCAL_BLOCK;
+                    const u32 j = tid + i * BLOCK;
                     if(j >= m) break;
-                    const u64 v = stage[j];
-                    const u32 key = u32(v >> 32);
+                    const u32 key = keys[j];
+                    r[i] = placed[j];
                     u32 a = 0, b = j;                   // first record with this key
-                    while(a < b) { const u32 mid = (a + b) >> 1; if(u32(stage[mid] >> 32) < key) a = mid + 1; else b = mid; }
+                    while(a < b) { const u32 mid = (a + b) >> 1; if(keys[mid] < key) a = mid + 1; else b = mid; }
                     u32 c = j + 1, f = m;               // first record behind with a greater key
-                    while(c < f) { const u32 mid = (c + f) >> 1; if(u32(stage[mid] >> 32) <= key) c = mid + 1; else f = mid; }
-                    const u32 eq = c - a;
-                    pl[i] = packed_place(j, a, eq);
-                    sa[base + j] = eq == 1 ? u32(v) : SA_OPEN;
+                    while(c < f) { const u32 mid = (c + f) >> 1; if(keys[mid] <= key) c = mid + 1; else f = mid; }
+                    if(c - a == 1) continue;
+                    placed[j] = SA_OPEN;
+                    pl[i] = packed_place(j, a, c - a);
+                    tied |= 1u << i;
                 }
             }
-            // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
-            u32 tied = 0;
+            const bool ties = __syncthreads_or(tied != 0);
             #pragma unroll
-            for(int i = 0; i < LOCAL_ITEMS; ++i)
+            for(int i = 0; i < ITEMS; ++i)
             {
-                if(i * LOCAL_BLOCK >= m) break;
-                if(tid + i * LOCAL_BLOCK < m) tied |= (pl[i] & (PL_SMALL | PL_LARGE)) ? 1u << i : 0u;
+                const u32 j = tid + i * BLOCK;
+                if(j >= m) break;
+                sa[base + j] = placed[j];
             }
-            if(__syncthreads_or(tied != 0))
+            // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
+            if(ties)
             {
-                #pragma unroll
-                for(int i = 0; i < LOCAL_ITEMS; ++i)
-                    if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
+                if(tied)            // a few threads of a block as a rule
+                {
+                    #pragma unroll
+                    for(int i = 0; i < ITEMS; ++i)
+                        if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
+                }
+                __syncthreads();
+                const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];
+                const bool many = all_ones > MANY_TIED;     // by way of shared memory (keys and placed are free now), side by side
                 __syncthreads();
                 if(tid < 2)
                 {
@@ -855,16 +907,37 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) local_sort_kernel(const u
                     s_slot[tid] = c ? atomicAdd(tid ? &counts->large : &counts->small, c) : 0;
                     s_tied[tid] = 0;
                 }
-                __syncthreads();
-                #pragma unroll
-                for(int i = 0; i < LOCAL_ITEMS; ++i)
-                    if(tied >> i & 1u)
+                if(!many) __syncthreads();
+                if(tied)
+                {
+                    #pragma unroll
+                    for(int i = 0; i < ITEMS; ++i)
+                        if(tied >> i & 1u)
+                        {
+                            const u32 place = pl[i] & 8191u, head = (pl[i] & PL_FIRST) ? place : pl[i] >> 13 & 8191u;
+                            const bool small = (pl[i] & PL_SMALL) != 0;
+                            const u32 at = start[head] + (place - head);
+                            if(many)
+                            {
+                                const u32 k = small ? at : small_ones + at;
+                                keys[k] = base + head;
+                                placed[k] = u32(r[i]);
+                                continue;
+                            }
+                            const u64 k = u64(s_slot[small ? 0 : 1]) + at;
+                            list[small ? k : list_cap - 1 - k] = (u64(base + head) << 32) | u32(r[i]);
+                        }
+                }
+                if(many)
+                {
+                    __syncthreads();
+                    for(u32 j = tid; j < all_ones; j += BLOCK)
                     {
-                        const u32 place = pl[i] & 8191u, head = (pl[i] & PL_FIRST) ? place : pl[i] >> 13 & 8191u;
-                        const bool small = (pl[i] & PL_SMALL) != 0;
-                        const u64 k = u64(s_slot[small ? 0 : 1]) + start[head] + (place - head);
-                        list[small ? k : list_cap - 1 - k] = (u64(base + head) << 32) | u32(stage[tid + i * LOCAL_BLOCK]);
+                        const u64 e = (u64(keys[j]) << 32) | placed[j];
+                        if(j < small_ones) list[u64(s_slot[0]) + j] = e;
+                        else list[list_cap - 1 - (u64(s_slot[1]) + (j - small_ones))] = e;
                     }
+                }
             }
             __syncthreads();        // the next batch reuses the shared arrays
         }
@@ -1030,17 +1103,17 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
     if(one_level)
     {
         static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, false>, LOCAL_SMEM<512>, configured));
-        local_sort_kernel<512, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false>, LOCAL_SMEM<512, 16>, configured));
+        local_sort_kernel<512, 16, 2, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
         CSA_LAUNCH_CHECK(ctx);
         return CSA_OK;
     }
     static std::atomic<bool> configured[2][64];
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<256, false>, LOCAL_SMEM<256>, configured[0]));
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, true>, LOCAL_SMEM<512>, configured[1]));
-    local_sort_kernel<256, false><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 4 * 8)), 256, LOCAL_SMEM<256>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 8, 3, false>, LOCAL_SMEM<512, 8>, configured[0]));
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, true>, LOCAL_SMEM<512, 16>, configured[1]));
+    local_sort_kernel<512, 8, 3, false><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 3 * 8)), 512, LOCAL_SMEM<512, 8>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
-    local_sort_kernel<512, true><<<148 * 2, 512, LOCAL_SMEM<512>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    local_sort_kernel<512, 16, 2, true><<<148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
