@@ -396,11 +396,12 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
     if(t == 0) { par_off[bins] = n; tile0[bins] = all_tiles; chunk0[bins] = all_chunks; }
 }
 
-template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<BLOCK>) * 8 + size_t(TILE_POSITIONS<BLOCK>) * 2;
+template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<BLOCK>) * 8;
 static_assert(SCATTER_TEXT_SMEM<512> >= sizeof(Tile_Code<512>) && SCATTER_TEXT_SMEM<128> >= sizeof(Tile_Code<128>), "the windows lie where the records are staged later");
 
 // Scatter by the top `bits` bits: the places inside a bucket come from shared-memory atomics and, for the tile's run of a bucket,
-// from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs.
+// from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs. What bounds it is shared memory
+// and L1 (78 % of their wavefronts): so a staged record carries its bin and its place in the tile in one word instead of its position and a bin beside it.
 // keep_top: the record keeps the top bits (there is no second split), else its key starts behind them. PART: only the suffixes of the
 // buckets [first_bin, first_bin + part_bins) are taken, and the cursors are theirs.
 template <int BLOCK, bool PART>
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);
-    u16* const stage_bin = reinterpret_cast<u16*>(stage + TILE_POSITIONS<BLOCK>);
+    static_assert(TILE_POSITIONS<BLOCK> <= 1 << 13 && MAX_B1 + 13 <= 32, "a staged record's lower word: its bin and its place in the tile");
     __shared__ u32 cnt[1 << MAX_B1];            // counts, then the bins' starts inside the tile
     __shared__ u32 base[1 << MAX_B1];           // where the tile's run of a bin goes, minus the run's start
     __shared__ u32 warp_tot[BLOCK / 32];
@@ -457,13 +458,17 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     for(int i = 0; i < TEXT_ITEMS; ++i)
         if(PART ? (taken >> i & 1u) != 0 : local + i < valid)
         {
-            const u32 bin = place[i] >> 16, at = cnt[bin] + (place[i] & 0xFFFFu);
-            stage[at] = (u64(key[i]) << 32) | u32(first + local + i);
-            stage_bin[at] = u16(bin);
+            const u32 bin = place[i] >> 16;
+            stage[cnt[bin] + (place[i] & 0xFFFFu)] = (u64(key[i]) << 32) | bin << 13 | (local + i);
         }
     __syncthreads();
     const u32 staged = PART ? total : valid;
-    for(u32 j = threadIdx.x; j < staged; j += BLOCK) out[base[stage_bin[j]] + j] = stage[j];
+    #pragma unroll 4
+    for(u32 j = threadIdx.x; j < staged; j += BLOCK)
+    {
+        const u64 v = stage[j];
+        out[base[u32(v) >> 13] + j] = (v & ~u64(0xFFFFFFFFu)) | u32(first + (u32(v) & 8191u));
+    }
 }
 
 // ---- second split: every parent by the next bits ----------------------------------------------------------------------------------
