@@ -1,7 +1,7 @@
 // The stable sort of csa_sort_pairs by its top bits first, for keys whose top bits are evenly spread: the records are split into buckets
 // of about a thousand by the top 8 to 15 sorted bits with one or two of radix_sort.cu's digit passes (stable, low digit first), and every
 // bucket is then finished inside one block. A record moves two or three times, where a pass per 8 bits moves it up to eight
-// times (31.25 M 64-bit keys with 4-byte values, whole calls: 2.22 ms, this way 1.14 ms; 10^6: 278 us, 149 us; 1000, in one block: 176 us, 71 us). Nothing is estimated: the buckets are counted
+// times (31.25 M 64-bit keys with 4-byte values, whole calls: 2.22 ms, this way 1.02 ms; 10^6: 253 us, 134 us; 1000, in one block: 174 us, 63 us). Nothing is estimated: the buckets are counted
 // exactly before anything moves, and keys with a bucket that no block holds go through all their digit passes as before.
 // A list that fits one block at all is a single bucket and takes one launch.
 #include "common.cuh"
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ cou
     }
     else
     {
-        // a warp sums buckets / 32 counts side by side, 128 at a time (a thread its 32 one by one: 62 us for 2^15 buckets, this way 8 us); there are
+        // a warp sums buckets / 32 counts side by side, 128 at a time (a thread its 32 one by one: 62 us for 2^15 buckets, this way 10 us); there are
         // two low bits or more, so every fourth bucket may start a high digit's run
         const u32 span = buckets / 32;
         constexpr int ROUNDS = (1 << BUCKET_MAX_BITS) / 32 / 128;
@@ -148,29 +148,33 @@ __global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ cou
 
 // ---- a bucket inside one block -------------------------------------------------------------------------------------------------
 
-constexpr int BUCKET_ITEMS = 16;
+constexpr int BUCKET_ITEMS = 8;
 template <int BLOCK> constexpr u32 BUCKET_CAP = BLOCK * BUCKET_ITEMS;
 constexpr u32 LONG_BIN = 128;       // a bin with more records is not ordered by comparing all with all
-template <int BLOCK> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CAP<BLOCK>) * (8 + 2) + (BUCKET_CAP<BLOCK> / 2 + 4) * 4;
+// the staged keys; then the bins and the places before, and where those were, the values
+template <int BLOCK, typename V> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CAP<BLOCK>) * 8 + (sizeof(V) == 8 ? size_t(BUCKET_CAP<BLOCK>) * 8 : size_t(BUCKET_CAP<BLOCK>) * 4 + 32);
 
 // Sorts every bucket [starts[b], starts[b + 1]) (starts == nullptr: one bucket, [0, n)) by the bits `compared` of its keys, of which
 // the highest is bit top - 1, stably, from the `in` to the `out` arrays. There are as many bins as records (up to a factor of 2): a record's
 // bin is its next key bits, its place in the bin is what a shared-memory atomic hands out, and inside the bin it counts the keys before its own, equal ones
-// by the places they came from. So the order is the stable one whatever order the atomics took. The values stay in global memory
-// until a record's place is known: a bucket's are a few KB side by side.
-// A bin of more than LONG_BIN records sends the bucket through a sorting network instead. What bounds it is the issue of instructions and
-// barriers between dependent steps; blocks are therefore as small as the largest bucket allows.
-template <int BLOCK, typename V>
-__global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in,
-                                                                         V* __restrict__ vals_out, const u32* __restrict__ starts, const u32 n, const u64 compared, const int top,
-                                                                         const int begin)
+// by the places they came from. So the order is the stable one whatever order the atomics took. A record stays with its thread until its place is known; keys
+// and values then go out by way of shared memory, side by side.
+// A bin of more than LONG_BIN records sends the bucket through a sorting network instead. What bounds it is the issue of instructions and barriers between
+// dependent steps: blocks are as small as the largest bucket allows, with 8 records a thread. (31.25 M records, 16 a thread and the values
+// gathered when the places were known: 454 us, this way 389 us.)
+template <int BLOCK, int BLOCKS, typename V>
+__global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in,
+                                                                   V* __restrict__ vals_out, const u32* __restrict__ starts, const u32 n, const u64 compared, const int top,
+                                                                   const int begin)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr u32 CAP = BUCKET_CAP<BLOCK>;
+    constexpr int ITEMS = BUCKET_ITEMS;
     u64* const stage = reinterpret_cast<u64*>(smem_raw);            // [CAP]
-    u32* const bin = reinterpret_cast<u32*>(stage + CAP);           // [CAP / 2 + 4]: two 16-bit counters a word, then the bins' starts
+    u32* const bin = reinterpret_cast<u32*>(stage + CAP);           // [CAP / 2 + 8]: two 16-bit counters a word, then the bins' starts
     u16* const start = reinterpret_cast<u16*>(bin);
-    u16* const from = reinterpret_cast<u16*>(bin + CAP / 2 + 4);    // [CAP]: the record's place in the bucket before
+    u16* const from = reinterpret_cast<u16*>(bin + CAP / 2 + 8);    // [CAP]: the record's place in the bucket before
+    V* const vals = reinterpret_cast<V*>(stage + CAP);              // [CAP], once the bins are no longer needed
     __shared__ u32 warp_tot[BLOCK / 32];
     const u32 tid = threadIdx.x;
     const u32 base = starts ? starts[blockIdx.x] : 0, m = (starts ? starts[blockIdx.x + 1] : n) - base;
@@ -178,71 +182,74 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(const 
     keys_in += base; keys_out += base;
     if(vals_in != nullptr) { vals_in += base; vals_out += base; }
 
-    const int bin_bits = min(32 - __clz(m - 1 | 1u), top - begin);   // bins: a power of two, at most CAP
+    const int bin_bits = min(32 - __clz(m - 1 | 1u), top - begin);  // bins: a power of two, at most CAP
     const u32 bins = 1u << bin_bits;
     const int bin_shift = top - bin_bits;
     const u32 bin_mask = bins - 1;
-    for(u32 i = tid; i < (bins / 2 + 4) / 4; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
-    u64 r[BUCKET_ITEMS];
-    u32 pl[BUCKET_ITEMS];               // bin << 16 | place in the bin
+    for(u32 i = tid; i < (bins / 2 + 8) / 4; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+    u64 r[ITEMS];
+    u32 pl[ITEMS];                      // place in the bin, later in the bucket
     #pragma unroll
-    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    for(int i = 0; i < ITEMS; ++i)
     {
         if(i * BLOCK >= m) break;
         const u32 j = tid + i * BLOCK;
         if(j < m) r[i] = keys_in[j];
     }
     __syncthreads();
+    auto bin_of = [&](const u64 key) { return u32(key >> bin_shift) & bin_mask; };
     #pragma unroll
-    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    for(int i = 0; i < ITEMS; ++i)
     {
         if(i * BLOCK >= m) break;
         if(tid + i * BLOCK < m)
         {
-            const u32 b = u32(r[i] >> bin_shift) & bin_mask;
+            const u32 b = bin_of(r[i]);
             const u32 old = atomicAdd(&bin[b >> 1], (b & 1) ? 0x10000u : 1u);
-            pl[i] = (b << 16) | ((b & 1) ? old >> 16 : old & 0xFFFFu);
+            pl[i] = (b & 1) ? old >> 16 : old & 0xFFFFu;
         }
     }
     __syncthreads();
-    // exclusive sums of the bins' counts, in place
+    // exclusive sums of the bins' counts, in place; start[bins] = m
     u32 longest = 0;
     {
-        constexpr int WORDS = CAP / 2 / BLOCK;          // 8 words, 16 bins a thread
+        constexpr int WORDS = CAP / 2 / BLOCK;          // 4 words, 8 bins a thread
         u32 c[WORDS], sum = 0;
-        const bool any = tid * WORDS * 2 < bins;        // of the words behind the bins' a few may hold anything: their sums are not used
+        const bool any = tid * WORDS * 2 <= bins;       // the words up to a multiple of WORDS were cleared
         if(any)
         {
+            const uint4 v = reinterpret_cast<const uint4*>(bin)[tid];
+            c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+            u32 both = 0;
             #pragma unroll
-            for(int k = 0; k < WORDS; ++k)
-            {
-                c[k] = tid * WORDS + k < (bins + 1) / 2 ? bin[tid * WORDS + k] : 0;
-                longest = max(longest, max(c[k] & 0xFFFFu, c[k] >> 16));
-                sum += (c[k] & 0xFFFFu) + (c[k] >> 16);
-            }
+            for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = __vmaxu2(longest, c[k]); }
+            sum = (both & 0xFFFFu) + (both >> 16);
         }
-        u32 run = block_exclusive_sum<BLOCK>(sum, warp_tot);
-        if(any)
-        {
-            #pragma unroll
-            for(int k = 0; k < WORDS; ++k)
-            {
-                const u32 a = run, b = run + (c[k] & 0xFFFFu);
-                run = b + (c[k] >> 16);
-                if(tid * WORDS + k < (bins + 1) / 2) bin[tid * WORDS + k] = a | (b << 16);
-            }
-        }
+        const u32 inc = warp_inclusive_sum(sum);
+        if(lane_id() == 31) warp_tot[tid >> 5] = inc;
         __syncthreads();
-        if(tid == 0) start[bins] = u16(m);
+        u32 run = __reduce_add_sync(0xFFFFFFFFu, lane_id() < (tid >> 5) ? warp_tot[lane_id()] : 0u) + inc - sum;
+        if(any)
+        {
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k)
+            {
+                const u32 a = run * 0x10001u + (c[k] << 16);        // below 2^16 each
+                run += (c[k] & 0xFFFFu) + (c[k] >> 16);
+                c[k] = a;
+            }
+            reinterpret_cast<uint4*>(bin)[tid] = make_uint4(c[0], c[1], c[2], c[3]);
+        }
+        if(bins == CAP && tid == 0) start[CAP] = u16(m);            // behind the threads' words
     }
-    const bool by_network = __syncthreads_or(longest > LONG_BIN);
+    const bool by_network = __syncthreads_or(max(longest & 0xFFFFu, longest >> 16) > LONG_BIN);
     if(by_network)
     {
         // Many records in one bin: a sorting network over (key, place before), padded with records behind all others.
         u32 size = 1;
         while(size < m) size <<= 1;
         #pragma unroll
-        for(int i = 0; i < BUCKET_ITEMS; ++i)
+        for(int i = 0; i < ITEMS; ++i)
         {
             const u32 j = tid + i * BLOCK;
             if(j >= size) break;
@@ -273,47 +280,71 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) bucket_sort_kernel(const 
         return;
     }
     #pragma unroll
-    for(int i = 0; i < BUCKET_ITEMS; ++i)
+    for(int i = 0; i < ITEMS; ++i)
     {
         if(i * BLOCK >= m) break;
         const u32 j = tid + i * BLOCK;
         if(j < m)
         {
-            const u32 at = start[pl[i] >> 16] + (pl[i] & 0xFFFFu);
-            stage[at] = r[i];
+            const u32 at = start[bin_of(r[i])] + pl[i];
+            stage[at] = r[i] & compared;
             from[at] = u16(j);
         }
     }
     __syncthreads();
-    #pragma unroll 4
-    for(u32 j = tid; j < m; j += BLOCK)
+    #pragma unroll
+    for(int i = 0; i < ITEMS; ++i)
     {
-        const u64 v = stage[j], mine = v & compared;
-        const u32 f = from[j];
-        const u32 b = u32(v >> bin_shift) & bin_mask;
-        const u32 s = start[b], e = start[b + 1];
-        u32 place = s;
-        for(u32 k = s; k < e; ++k)
+        if(i * BLOCK >= m) break;
+        const u32 f = tid + i * BLOCK;
+        if(f < m)
         {
-            const u64 o = stage[k] & compared;
-            if(o < mine) ++place;
-            else if(o == mine) place += from[k] < f;
+            const u64 mine = r[i] & compared;
+            const u32 b = bin_of(r[i]), s = start[b], e = start[b + 1];
+            u32 less = 0, upto = 0;
+            #pragma unroll
+            for(u32 k = 0; k < 3; ++k)          // most bins hold no more: three reads in flight
+                if(s + k < e) { const u64 o = stage[s + k]; less += o < mine; upto += o <= mine; }
+            for(u32 k = s + 3; k < e; ++k) { const u64 o = stage[k]; less += o < mine; upto += o <= mine; }
+            u32 place = s + less;
+            if(upto - less > 1)
+                for(u32 k = s; k < e; ++k) place += stage[k] == mine && from[k] < f;
+            pl[i] = place;
         }
-        keys_out[place] = v;
-        if(vals_in != nullptr) vals_out[place] = vals_in[f];
+    }
+    __syncthreads();        // the bins and the keys in them have been read
+    #pragma unroll
+    for(int i = 0; i < ITEMS; ++i)
+    {
+        if(i * BLOCK >= m) break;
+        const u32 j = tid + i * BLOCK;
+        if(j < m)
+        {
+            stage[pl[i]] = r[i];
+            if(vals_in != nullptr) vals[pl[i]] = vals_in[j];
+        }
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < ITEMS; ++i)
+    {
+        const u32 j = tid + i * BLOCK;
+        if(j >= m) break;
+        keys_out[j] = stage[j];
+        if(vals_in != nullptr) vals_out[j] = vals[j];
     }
 }
 
-template <int BLOCK, typename V>
+template <int BLOCK, int BLOCKS, typename V>
 int launch_buckets(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 compared, int top, int begin)
 {
     static std::atomic<bool> configured[64];
     if(!configured[ctx->device & 63])
     {
-        CSA_CUDA(ctx, cudaFuncSetAttribute(bucket_sort_kernel<BLOCK, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BUCKET_SMEM<BLOCK>)));
+        CSA_CUDA(ctx, cudaFuncSetAttribute(bucket_sort_kernel<BLOCK, BLOCKS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(BUCKET_SMEM<BLOCK, V>)));
         configured[ctx->device & 63] = true;
     }
-    bucket_sort_kernel<BLOCK, V><<<buckets, BLOCK, BUCKET_SMEM<BLOCK>, ctx->stream>>>(kin, kout, vin, vout, starts, u32(n), compared, top, begin);
+    bucket_sort_kernel<BLOCK, BLOCKS, V><<<buckets, BLOCK, BUCKET_SMEM<BLOCK, V>, ctx->stream>>>(kin, kout, vin, vout, starts, u32(n), compared, top, begin);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -322,13 +353,13 @@ template <typename V>
 int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 largest, int begin, int top)
 {
     const u64 compared = (top >= 64 ? ~0ull : (1ull << top) - 1) & (~0ull << begin);
-    if(largest <= BUCKET_CAP<128>) return launch_buckets<128, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
-    if(largest <= BUCKET_CAP<256>) return launch_buckets<256, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
-    if(largest <= BUCKET_CAP<512>) return launch_buckets<512, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    if(largest <= BUCKET_CAP<256>) return launch_buckets<256, 6, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    if(largest <= BUCKET_CAP<512>) return launch_buckets<512, 3, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
+    if(largest <= BUCKET_CAP<1024>) return launch_buckets<1024, 1, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
     return csa_fail(ctx, CSA_E_DEVICE, "bucket sort: a bucket does not fit a block");
 }
 
-static_assert(BUCKET_CAP<512> == BUCKET_MAX_RECORDS, "");
+static_assert(BUCKET_CAP<1024> == BUCKET_MAX_RECORDS, "");
 
 }   // namespace
 
