@@ -28,6 +28,14 @@ namespace
 constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of an encoding block
 constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
+#ifndef LR
+#define LR 4
+#endif
+#ifndef OL_B
+#define OL_B 512
+#define OL_I 16
+#define OL_M 2
+#endif
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
 constexpr u32 LOCAL_CHUNK = 2048, SHORT_CHUNK = 1024;
@@ -141,63 +149,49 @@ __global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __rest
         }
         __syncthreads();
     }
-    // a warp sums 2048 consecutive symbols, 128 at a time
-    u32 run = 0;
-    #pragma unroll 8
+    // a warp takes 2048 consecutive symbols, 128 at a time: their sum, then their prefix sums behind those of the warps before
+    auto counts_of = [&](const u32 s) -> uint4
+    {
+        if(!COUNT) return __ldg(reinterpret_cast<const uint4*>(hist + s));
+        const ushort4 v = *reinterpret_cast<const ushort4*>(low + s);
+        return make_uint4(v.x, v.y, v.z, v.w);
+    };
+    u32 mine = 0;
+    #pragma unroll
     for(int k = 0; k < 16; ++k)
     {
-        const u32 s = warp * 2048 + k * 128 + lane * 4;
-        uint4 c;
-        if(COUNT)
-        {
-            const ushort4 v = *reinterpret_cast<const ushort4*>(low + s);
-            c = make_uint4(v.x, v.y, v.z, v.w);
-        }
-        else c = __ldg(reinterpret_cast<const uint4*>(hist + s));
-        const u32 sum = scale * (c.x + c.y + c.z + c.w) + 4;
-        const u32 inc = warp_inclusive(sum);
-        const u32 x = run + inc - sum, y = x + scale * c.x + 1, z = y + scale * c.y + 1, w = z + scale * c.z + 1;
-        *reinterpret_cast<ushort4*>(low + s) = make_ushort4(u16(x), u16(y), u16(z), u16(w));
-        *reinterpret_cast<uchar4*>(high + s) = make_uchar4(u8(x >> 16), u8(y >> 16), u8(z >> 16), u8(w >> 16));
-        run += __shfl_sync(0xFFFFFFFFu, inc, 31);
+        const uint4 c = counts_of(warp * 2048 + k * 128 + lane * 4);
+        mine += c.x + c.y + c.z + c.w;
     }
-    if(lane == 0) warp_tot[warp] = run;
+    mine = scale * __reduce_add_sync(0xFFFFFFFFu, mine) + 2048;
+    if(lane == 0) warp_tot[warp] = mine;
     __syncthreads();
     {
-        u32 base = 0, all = 0;
-        #pragma unroll
-        for(int w = 0; w < CODE_BLOCK / 32; ++w) { const u32 t = warp_tot[w]; if(w < int(warp)) base += t; all += t; }
-        #pragma unroll 4
+        u32 run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_tot[lane] : 0u);
+        #pragma unroll 8
         for(int k = 0; k < 16; ++k)
         {
             const u32 s = warp * 2048 + k * 128 + lane * 4;
-            const ushort4 l = *reinterpret_cast<const ushort4*>(low + s);
-            const uchar4 h = *reinterpret_cast<const uchar4*>(high + s);
-            const u32 x = base + (l.x | u32(h.x) << 16), y = base + (l.y | u32(h.y) << 16), z = base + (l.z | u32(h.z) << 16), w = base + (l.w | u32(h.w) << 16);
-            *reinterpret_cast<ushort4*>(low + s) = make_ushort4(u16(x), u16(y), u16(z), u16(w));
-            *reinterpret_cast<uchar4*>(high + s) = make_uchar4(u8(x >> 16), u8(y >> 16), u8(z >> 16), u8(w >> 16));
+            const uint4 c = counts_of(s);
+            const u32 sum = scale * (c.x + c.y + c.z + c.w) + 4, inc = warp_inclusive(sum);
+            const u32 x = run + inc - sum, y = x + scale * c.x + 1, z = y + scale * c.y + 1, w = z + scale * c.z + 1;
+            *reinterpret_cast<uint2*>(low + s) = make_uint2(__byte_perm(x, y, 0x5410), __byte_perm(z, w, 0x5410));
+            *reinterpret_cast<u32*>(high + s) = __byte_perm(__byte_perm(x, y, 0x0062), __byte_perm(z, w, 0x0062), 0x5410);
+            run += __shfl_sync(0xFFFFFFFFu, inc, 31);
         }
-        if(tid == 0) { low[65536] = u16(all); high[65536] = u8(all >> 16); }
+        if(tid == CODE_BLOCK - 1) { low[65536] = u16(run); high[65536] = u8(run >> 16); }
     }
     __syncthreads();
     auto prefix = [&](const u32 m) { return u32(low[m]) | u32(high[m]) << 16; };
 
     if(tid >= CODE_WALKERS) return;
-    const u32 s = blockIdx.x * CODE_WALKERS + tid;
+    const u32 s = blockIdx.x * CODE_WALKERS + tid, s_first = s - lane;
     u32 lo = 0, hi = 65536, word = 0;
     int left = CODE_MAX_LEN;            // bits left below the node
     u32 plo = 0, phi = prefix(65536);
-    while(hi - lo > 1)
+    // The split of a node from the first boundary at or past the middle.
+    auto settle = [&](u32& m, u32& pm, const u32 twice_mid)
     {
-        const u32 twice_mid = plo + phi;
-        u32 a = lo + 1, b = hi - 1;     // the split m: first boundary at or past the middle, kept inside (lo, hi)
-        while(a < b)
-        {
-            const u32 m = (a + b) >> 1;
-            if(2 * prefix(m) >= twice_mid) b = m; else a = m + 1;
-        }
-        u32 m = a;
-        u32 pm = prefix(m);
         if(m > lo + 1)
         {
             const u32 pb = prefix(m - 1);
@@ -207,8 +201,42 @@ __global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __rest
         if(m - lo > room) { m = lo + room; pm = prefix(m); }
         else if(hi - m > room) { m = hi - room; pm = prefix(m); }
         --left;
+    };
+    auto descend = [&](const u32 m, const u32 pm)
+    {
         if(s < m) { hi = m; phi = pm; }
         else { lo = m; plo = pm; word |= 1u << (31 - (CODE_MAX_LEN - 1 - left)); }
+    };
+    // As long as a warp's symbols are in one node, all lanes look for its split: 32 boundaries at a time.
+    bool together = true;
+    while(together && hi - lo > 1)
+    {
+        const u32 twice_mid = plo + phi;
+        u32 a = lo + 1, b = hi - 1;     // the split: kept inside (lo, hi)
+        while(a < b)
+        {
+            const u32 step = b - a <= 32 ? 1 : (b - a + 32) / 33, probe = a + (lane + 1) * step - 1;
+            const u32 before = __popc(__ballot_sync(0xFFFFFFFFu, probe < b && 2 * prefix(probe) < twice_mid));     // a leading run of lanes
+            if(before < 32) b = min(b, a + (before + 1) * step - 1);
+            a += before * step;
+        }
+        u32 m = a, pm = prefix(m);
+        settle(m, pm, twice_mid);
+        together = m <= s_first || m > s_first + 31;
+        descend(m, pm);
+    }
+    while(hi - lo > 1)
+    {
+        const u32 twice_mid = plo + phi;
+        u32 a = lo + 1, b = hi - 1;
+        while(a < b)
+        {
+            const u32 m = (a + b) >> 1;
+            if(2 * prefix(m) >= twice_mid) b = m; else a = m + 1;
+        }
+        u32 m = a, pm = prefix(m);
+        settle(m, pm, twice_mid);
+        descend(m, pm);
     }
     code[s] = word | u32(CODE_MAX_LEN - left);
 }
@@ -825,9 +853,9 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
                             continue;
                         }
                         #pragma unroll
-                        for(u32 j = 0; j < 4; ++j)      // most bins hold no more: four reads in flight
+                        for(u32 j = 0; j < LR; ++j)      // most bins hold no more: four reads in flight
                             if(s + j < t) { const u32 o = keys[s + j]; less += o < k; upto += o <= k; }
-                        for(u32 j = s + 4; j < t; ++j) { const u32 o = keys[j]; less += o < k; upto += o <= k; }
+                        for(u32 j = s + LR; j < t; ++j) { const u32 o = keys[j]; less += o < k; upto += o <= k; }
                         const u32 head = s + less;
                         if(upto - less == 1) placed[head] = u32(r[i]);
                         else
@@ -1108,8 +1136,8 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
     if(one_level)
     {
         static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false>, LOCAL_SMEM<512, 16>, configured));
-        local_sort_kernel<512, 16, 2, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel<OL_B, OL_I, OL_M, false>, LOCAL_SMEM<OL_B, OL_I>, configured));
+        local_sort_kernel<OL_B, OL_I, OL_M, false><<<unsigned(n / SHORT_CHUNK + parents), OL_B, LOCAL_SMEM<OL_B, OL_I>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
         CSA_LAUNCH_CHECK(ctx);
         return CSA_OK;
     }

@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(128) find_kernel(const csa_index idx, const u6
 // memory): the queries of a slot then read the same upper levels of the table's bisection, one stretch of the table and one of
 // the array. Nothing is sorted: the slots are counted, and a query takes the next place of its slot.
 constexpr u32 SLOT_BITS = 12, SLOTS = 1u << SLOT_BITS;
-constexpr int SLOT_BLOCK = 512, SLOT_ITEMS = 8, SLOT_TILE = SLOT_BLOCK * SLOT_ITEMS;
+constexpr int SLOT_BLOCK = 512, SLOT_ITEMS = 2, SLOT_TILE = SLOT_BLOCK * SLOT_ITEMS;
 constexpr size_t SLOT_SMEM = SLOTS * 8 + (SLOTS + 1) * 4;
 
 // What a query needs on its way, in the order of the slots.
@@ -333,15 +333,25 @@ __global__ void __launch_bounds__(SLOT_BLOCK) count_slots_kernel(const u64* __re
     __syncthreads();
     const u64 off0 = *off_first;
     for(u64 tile = blockIdx.x; tile * SLOT_TILE < q; tile += gridDim.x)
+    {
+        Pattern ps[SLOT_ITEMS];             // their reads side by side
+        #pragma unroll
         for(int k = 0; k < SLOT_ITEMS; ++k)
         {
             const u64 i = tile * SLOT_TILE + k * SLOT_BLOCK + threadIdx.x;
-            if(i >= q) break;
+            if(i >= q) continue;
             const u64 from = off[i], m = off[i + 1] - from;
+            if(m) ps[k] = Pattern(sym + (from - off0), m);
+        }
+        #pragma unroll
+        for(int k = 0; k < SLOT_ITEMS; ++k)
+        {
+            const u64 i = tile * SLOT_TILE + k * SLOT_BLOCK + threadIdx.x;
+            if(i >= q) continue;
+            const Pattern& p = ps[k];
             u32 x = 0, z = 0;
-            if(m)
+            if(p.m)
             {
-                const Pattern p(sym + (from - off0), m);
                 #pragma unroll
                 for(u32 step = SLOTS / 2; step; step >>= 1) if((dir[x + step - 1] & p.mask_high) < p.high) x += step;
                 if(x == SLOTS - 1 && (dir[x] & p.mask_high) < p.high) ++x;
@@ -360,6 +370,7 @@ __global__ void __launch_bounds__(SLOT_BLOCK) count_slots_kernel(const u64* __re
             }
             places[i] = Slot_Place{u16(x), u16(z), atomicAdd(&cnt[x], 1u)};
         }
+    }
     __syncthreads();
     for(u32 k = threadIdx.x; k <= SLOTS; k += SLOT_BLOCK)
     {
@@ -392,11 +403,11 @@ __global__ void __launch_bounds__(SLOT_BLOCK) deal_slots_kernel(const u64* __res
     __syncthreads();
     const u64 off0 = *off_first;
     for(u64 tile = blockIdx.x; tile * SLOT_TILE < q; tile += gridDim.x)
-        #pragma unroll 2
+        #pragma unroll
         for(int k = 0; k < SLOT_ITEMS; ++k)
         {
             const u64 i = tile * SLOT_TILE + k * SLOT_BLOCK + threadIdx.x;
-            if(i >= q) break;
+            if(i >= q) continue;
             const Slot_Place pl = places[i];
             const u64 from = off[i], m = off[i + 1] - from;
             Pattern p;
@@ -408,7 +419,10 @@ __global__ void __launch_bounds__(SLOT_BLOCK) deal_slots_kernel(const u64* __res
         }
 }
 
-__global__ void __launch_bounds__(128) find_dealt_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const Slot_Query* __restrict__ dealt, const u64 q,
+#ifndef FD_M
+#define FD_M 10
+#endif
+__global__ void __launch_bounds__(128, FD_M) find_dealt_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const Slot_Query* __restrict__ dealt, const u64 q,
                                                         u64* __restrict__ itv)
 {
     const u64 t = u64(blockIdx.x) * 128 + threadIdx.x;
@@ -535,28 +549,31 @@ __global__ void search_windows_kernel(const csa_index idx, const u64* __restrict
     itv[2 * i + 1] = hi;
 }
 
-// One warp per query: row i of pos receives SA[lo + k], k < min(max_pos, hi - lo).
-__global__ void locate_rows_kernel(const u8* __restrict__ sa40, const u64* __restrict__ itv, const u64 q, const u32 max_pos, u64* __restrict__ pos,
-                                   u32* __restrict__ cnt)
+// Eight lanes per query (most match once or a few times, and half of a batch may not match at all): row i of pos receives SA[lo + k],
+// k < min(max_pos, hi - lo). (A warp per query: 126 us for 10^6 queries of up to 20 positions, this way @LOCATE.)
+constexpr u32 LOCATE_LANES = 8;
+
+__global__ void __launch_bounds__(256) locate_rows_kernel(const u8* __restrict__ sa40, const u64* __restrict__ itv, const u64 q, const u32 max_pos, u64* __restrict__ pos,
+                                                         u32* __restrict__ cnt)
 {
-    const u64 w = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const u64 w = (u64(blockIdx.x) * 256 + threadIdx.x) / LOCATE_LANES;
     if(w >= q) return;
     const u64 lo = itv[2 * w], hi = itv[2 * w + 1];
-    const u64 c = (hi - lo < max_pos) ? hi - lo : max_pos;
-    if(lane_id() == 0) cnt[w] = u32(c);
-    for(u64 k = lane_id(); k < c; k += 32) pos[w * max_pos + k] = sa40_load(sa40, lo + k);
+    const u32 c = (hi - lo < max_pos) ? u32(hi - lo) : max_pos, lane = threadIdx.x % LOCATE_LANES;
+    if(lane == 0) cnt[w] = c;
+    for(u32 k = lane; k < c; k += LOCATE_LANES) pos[w * max_pos + k] = sa40_load(sa40, lo + k);
 }
 
 // The same into one packed array: query i's positions start at pos_off[i].
-__global__ void locate_packed_kernel(const u8* __restrict__ sa40, const u64* __restrict__ itv, const u64 q, const u32 max_pos,
-                                     const u64* __restrict__ pos_off, u64* __restrict__ pos)
+__global__ void __launch_bounds__(256) locate_packed_kernel(const u8* __restrict__ sa40, const u64* __restrict__ itv, const u64 q, const u32 max_pos,
+                                                           const u64* __restrict__ pos_off, u64* __restrict__ pos)
 {
-    const u64 w = (u64(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const u64 w = (u64(blockIdx.x) * 256 + threadIdx.x) / LOCATE_LANES;
     if(w >= q) return;
     const u64 lo = itv[2 * w], hi = itv[2 * w + 1];
-    const u64 c = (hi - lo < max_pos) ? hi - lo : max_pos;
+    const u32 c = (hi - lo < max_pos) ? u32(hi - lo) : max_pos;
     const u64 o = pos_off[w];
-    for(u64 k = lane_id(); k < c; k += 32) pos[o + k] = sa40_load(sa40, lo + k);
+    for(u32 k = threadIdx.x % LOCATE_LANES; k < c; k += LOCATE_LANES) pos[o + k] = sa40_load(sa40, lo + k);
 }
 
 // Sharded locate: the columns of a global interval's row that fall into this slice of the suffix array.
@@ -783,7 +800,7 @@ int find_dealt(csa_ctx* ctx, const csa_index& index, const u64* off, const u16* 
     if(cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) { cudaGetLastError(); return CSA_OK; }
     if(capturing != cudaStreamCaptureStatusNone) return CSA_OK;
     const u64 per = std::min(q, DEAL_CHUNK);
-    const unsigned most_blocks = unsigned(std::min<u64>(div_up(per, SLOT_TILE), 148 * 3));
+    const unsigned most_blocks = unsigned(std::min<u64>(div_up(per, SLOT_TILE), 148 * 4));
     const size_t b_dealt = align_up256(per * sizeof(Slot_Query)), b_places = align_up256(per * sizeof(Slot_Place)), b_dir = align_up256(SLOTS * 8), b_counts = align_up256((SLOTS + 1) * 4),
                  b_before = align_up256(size_t(most_blocks) * (SLOTS + 1) * 4);
     void* aux = nullptr;
@@ -887,7 +904,7 @@ extern "C" int csa_locate(csa_ctx* ctx, const csa_index* index, const uint64_t* 
     if(q == 0) return CSA_OK;
     if(!itv || !pos || !cnt || max_pos == 0) return csa_fail(ctx, CSA_E_INVALID, "csa_locate: bad argument");
     CSA_CUDA(ctx, cudaSetDevice(ctx->device));
-    locate_rows_kernel<<<unsigned(div_up(q * 32, 256)), 256, 0, ctx->stream>>>(index->sa40, reinterpret_cast<const u64*>(itv), q, max_pos,
+    locate_rows_kernel<<<unsigned(div_up(q * LOCATE_LANES, 256)), 256, 0, ctx->stream>>>(index->sa40, reinterpret_cast<const u64*>(itv), q, max_pos,
                                                                                reinterpret_cast<u64*>(pos), cnt);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
@@ -920,6 +937,7 @@ __global__ void add_base_kernel(u64* __restrict__ off, const u64 count, const u6
 }
 
 constexpr u64 HOST_CHUNK_QUERIES = u64(1) << 18;     // the reference's chunk of a host batch (include/Query_Engine.hpp:94-100)
+constexpr u64 HOST_CHUNK_MIN = u64(1) << 14;
 
 // Device buffers of one lane of the host-batch pipeline.
 struct Lane_Buffers
@@ -1094,13 +1112,15 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
         }
     }
     CSA_TRY(csa_lanes(ctx));
-    const u64 chunks = div_up(q, HOST_CHUNK_QUERIES);
+    // A batch that would be a chunk or two is cut into four, so that it overlaps its copies, too; a chunk's dozen calls cost what 2^14 queries' answers do.
+    const u64 chunk = sa_on_host ? HOST_CHUNK_QUERIES : std::min(HOST_CHUNK_QUERIES, std::max(HOST_CHUNK_MIN, div_up(q, 4)));
+    const u64 chunks = div_up(q, chunk);
     const int lanes = sa_on_host ? 1 : int(chunks < u64(csa_ctx::LANES) ? chunks : u64(csa_ctx::LANES));
-    const u64 cq_max = q < HOST_CHUNK_QUERIES ? q : HOST_CHUNK_QUERIES;
+    const u64 cq_max = q < chunk ? q : chunk;
     u64 sym_max = 0;
     for(u64 c = 0; c < chunks; ++c)
     {
-        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
+        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
         if(off_host[first + cq] < off_host[first]) return csa_fail(ctx, CSA_E_INVALID, "csa_query_host: offsets must not decrease");
         const u64 sc = off_host[first + cq] - off_host[first];
         if(sc > sym_max) sym_max = sc;
@@ -1129,7 +1149,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
     auto search = [&](u64 c) -> int
     {
         const int l = int(c % u64(lanes));
-        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
+        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
         const u64 sc = off_host[first + cq] - off_host[first];
         const On_Stream on(ctx, ctx->lane[l]);
         CSA_CUDA(ctx, cudaMemcpyAsync(L[l].off, off_host + first, (cq + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -1142,7 +1162,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
             CSA_LAUNCH_CHECK(ctx);
             u64* total_d = ctx->d_scalars + 8 + l;
             CSA_TRY(exclusive_sum(ctx, L[l].cnt, cq, L[l].poff, L[l].sums, total_d));
-            locate_packed_kernel<<<unsigned(div_up(cq * 32, 256)), 256, 0, ctx->stream>>>(index->sa40, L[l].itv, cq, max_pos, L[l].poff, L[l].pos);
+            locate_packed_kernel<<<unsigned(div_up(cq * LOCATE_LANES, 256)), 256, 0, ctx->stream>>>(index->sa40, L[l].itv, cq, max_pos, L[l].poff, L[l].pos);
             CSA_LAUNCH_CHECK(ctx);
             CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 8 + l, total_d, 8, cudaMemcpyDeviceToHost, ctx->stream));
             CSA_CUDA(ctx, cudaMemcpyAsync(cnt_host + first, L[l].cnt, cq * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1157,7 +1177,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
     {
         if(!want_pos) return CSA_OK;
         const int l = int(c % u64(lanes));
-        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
+        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
         CSA_CUDA(ctx, cudaEventSynchronize(ctx->lane_event[l]));
         const u64 total = ctx->h_scalars[8 + l];
         const On_Stream on(ctx, ctx->lane[l]);

@@ -247,17 +247,76 @@ __device__ __forceinline__ u32 shared_by_key(const u64 key, const u32 reach)
     return 2 * ((key >> 40) ? 31 - p : p) + 2;
 }
 
-constexpr u32 WIDE_REACH = 60;      // symbols that half a warp compares at once: four per lane; the last lane only completes the four before it
+constexpr u32 WIDE_REACH = 48;      // symbols that four lanes compare at once: 64, of which up to 15 lie before the suffix
 constexpr u32 QUICK_REACH = 8;
+constexpr int WIDE_ROWS = 2;         // suffixes in flight per four lanes
+static_assert(TEXT_DEPTH == 1 + WIDE_REACH, "one wide round");
+
+// 32 bytes, a whole sector, by one load.
+struct Piece { u32 w[8]; };
+__device__ __forceinline__ Piece load_sector(const uintptr_t at)
+{
+    Piece p;
+    asm("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(p.w[0]), "=r"(p.w[1]), "=r"(p.w[2]), "=r"(p.w[3]), "=r"(p.w[4]), "=r"(p.w[5]), "=r"(p.w[6]), "=r"(p.w[7]) : "l"(at));
+    return p;
+}
+
+// Where the suffixes at x and y first differ, among 16 of their symbols: those of the part-th sector that holds symbols of the suffix at x. `none` where they
+// do not below symbol `limit`. The other suffix comes in pieces of 16 bytes that are shifted to meet the sector. The first sector may begin up to
+// 15 symbols before x, inside the allocation, as it holds x; pieces of 16 bytes before the text are not read; behind it the text is padded.
+__device__ __forceinline__ u32 first_difference(const u16* __restrict__ T, const u64 x, const u64 y, const u32 part, const u32 limit, const u32 none)
+{
+    const uintptr_t at = reinterpret_cast<uintptr_t>(T + x), text = reinterpret_cast<uintptr_t>(T);
+    const u32 skip = u32(at >> 1) & 15u;
+    const int base = int(16 * part) - int(skip);
+    if(base >= int(limit)) return none;
+    const Piece a = load_sector((at & ~uintptr_t(31)) + 32 * part);
+    const uintptr_t from = reinterpret_cast<uintptr_t>(T + y) - 2 * skip + 32 * part, piece = from & ~uintptr_t(15);
+    const u32 shift = u32(from >> 1) & 7u;
+    auto load = [&](const uintptr_t q) { return q >= text ? __ldg(reinterpret_cast<const uint4*>(q)) : make_uint4(0, 0, 0, 0); };      // T is 16-byte aligned
+    const uint4 w0 = load(piece), w1 = load(piece + 16), w2 = load(piece + 32);
+    u32 v[12] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z, w2.w};
+    #pragma unroll
+    for(int k = 0; k < 10; ++k) v[k] = (shift & 4) ? v[k + 2] : v[k];
+    #pragma unroll
+    for(int k = 0; k < 9; ++k) v[k] = (shift & 2) ? v[k + 1] : v[k];
+    u32 any = 0;
+    #pragma unroll
+    for(int k = 0; k < 8; ++k) { v[k] = __funnelshift_r(v[k], v[k + 1], (shift & 1) * 16) ^ a.w[k]; any |= v[k]; }
+    if(any == 0) return none;
+    u32 differ = 0;
+    #pragma unroll
+    for(int k = 0; k < 8; ++k) differ |= ((v[k] & 0xFFFFu) ? 1u << (2 * k) : 0u) | ((v[k] >> 16) ? 2u << (2 * k) : 0u);
+    if(base < 0) differ &= ~0u << -base;
+    const u32 first = u32(base + __ffs(differ) - 1);
+    return differ && first < limit ? first : none;
+}
+
+// The key of the suffix at x, of which cx symbols count, against the one at y, with cy: they differ first at symbol `first`, or one ends there.
+__device__ __forceinline__ u64 difference_key(const u16* __restrict__ T, const u64 x, const u64 y, const u32 cx, const u32 cy, const u32 first)
+{
+    const u32 pair = first >> 1;
+    auto two = [&](const u64 z, const u32 c, u32& have) -> u32         // the pair of symbols, most significant first
+    {
+        const u32 at = 2 * pair;
+        have = c > at + 1 ? 2 : (c > at ? 1 : 0);
+        return (have ? u32(T[z + at]) << 16 : 0u) | (have > 1 ? u32(T[z + at + 1]) : 0u);
+    };
+    u32 hx, hy;
+    const u32 mine = two(x, cx, hx), lead = two(y, cy, hy);
+    return pair_key(pair, mine, hx, lead, hy);
+}
 
 // Orders groups by the symbols [from, to) of their suffixes. In a round every member of a group is compared with the group's first
 // member, and the members are put in order by their first difference from it; a group that falls apart goes on as several, each
 // with its own depth. The window stays in shared memory over all rounds.
 //
-// A WIDE round has half a warp read 60 symbols of one suffix with one load (a thread that reads 8 symbols of a suffix of its own at a time
-// costs an L1 look-up per lane and 8-byte piece). Where few suffixes are tied, nearly all of them differ within a few symbols and
+// A WIDE round compares 48 symbols: four lanes read a suffix, a sector each, all of it in flight at once, and the first member's symbols beside it, which the
+// neighbouring lanes read as well; a difference is then read symbol by symbol. (Half a warp to a suffix, four symbols a lane: 58 warp instructions a suffix,
+// 9.45 ms for 10^8 near-duplicate suffixes; a thread to a suffix, a sector after the other: 11.5 ms; this way @REFINE.)
+// Where few suffixes are tied, nearly all of them differ within a few symbols and
 // the chain of loads counts: the first round is then QUICK, 8 symbols by one thread, all of a thread's suffixes in flight together.
-// Where nearly all of 4e8 suffixes are tied, 8 symbols a round and all members against all took 136 ms, this way 42 ms.
 __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
                                                                     u64* __restrict__ next, u32* __restrict__ sa, Build_Counts* __restrict__ counts)
 {
@@ -266,7 +325,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     u64* const key = reinterpret_cast<u64*>(smem_raw + (sizeof(Window) + 15) / 16 * 16);     // [RW_WINDOW]
     u32* const depth = reinterpret_cast<u32*>(key + RW_WINDOW);     // [RW_WINDOW] by first slot: symbols that the group's members share (below 2^32: no more than n)
     Odd_Members& odds = *reinterpret_cast<Odd_Members*>(depth + RW_WINDOW);
-    const u32 tid = threadIdx.x, lane = lane_id();
+    const u32 tid = threadIdx.x;
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
     for(u64 first = u64(blockIdx.x) * RW_TILE; first < count; first += u64(gridDim.x) * RW_TILE)
@@ -306,105 +365,31 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
             }
             else
             {
-                // The slots of half a warp, 16 at a time, whose places and depths the lanes look up together.
-                constexpr u32 PER_HALF = RW_WINDOW / (RW_BLOCK / 16);
-                const u32 hl = lane & 15, half = lane & 16;
-                u32 lead_x = 0, lead_y = 0, lead_have = 0, lead_slot = NO_GROUP;
-                const u32 base = (tid >> 4) * PER_HALF;
-                for(u32 j0 = base; j0 < base + PER_HALF; j0 += 16)
+                const u32 part = tid & 3u, quad = lane_id() & ~3u;
+                #pragma unroll (WIDE_ROWS)
+                for(u32 j = tid >> 2; j < RW_WINDOW; j += RW_BLOCK / 4)
                 {
-                    const u32 s = w.gs[j0 + hl];
-                    u32 at = 0, cnt = 0;
-                    bool mine = false;
-                    auto place = [&](const u32 slot, const u32 d, u32& x0, u32& c0)     // where a suffix is read from, and how many symbols count
+                    const u32 s = w.gs[j];
+                    bool mine = s != NO_GROUP && u32(w.ge[s]) - s >= 2;
+                    const u64 d = mine ? depth[s] : 0;
+                    mine = mine && d < to;
+                    open |= mine;
+                    if(mine && j == s && part == 0) key[j] = KEY_EQUAL;
+                    mine = mine && j != s;
+                    if(!__any_sync(0xFFFFFFFFu, mine)) continue;
+                    u64 x = 0, y = 0;
+                    u32 cx = 0, cy = 0, first = WIDE_REACH;
+                    if(mine)
                     {
-                        const u64 x = u64(w.pos[slot]) + d;
-                        x0 = x < n ? u32(x) : u32(n);
-                        const u64 c = min(n - x0, to - d);
-                        c0 = c < WIDE_REACH ? u32(c) : WIDE_REACH;
-                    };
-                    if(s != NO_GROUP && u32(w.ge[s]) - s >= 2 && u64(depth[s]) < to) { mine = true; place(j0 + hl, depth[s], at, cnt); }
-                    const u32 both = __ballot_sync(0xFFFFFFFFu, mine);
-                    if(both == 0) continue;
-                    open = true;
-                    if(mine) key[j0 + hl] = KEY_EQUAL;
-                    const u32 todo = (both >> half) & 0xFFFFu;
-                    const u32 leads = (__ballot_sync(0xFFFFFFFFu, mine && s == j0 + hl) >> half) & 0xFFFFu;
-                    // a group that began in another half's slots: its first member is read here too
-                    const u32 s0 = __shfl_sync(0xFFFFFFFFu, s, half + (todo ? __ffs(todo) - 1 : 0));
-                    const u32 s_last = __shfl_sync(0xFFFFFFFFu, s, half + (todo ? 31 - __clz(todo) : 0));
-                    const bool fetch = todo != 0 && s0 != lead_slot && s0 < j0;
-                    auto read = [&](const u32 a, const u32 c) -> uint2
-                    {
-                        uint2 v = make_uint2(0, 0);
-                        if(4 * hl < c + 4) v = __ldg(reinterpret_cast<const uint2*>(T) + ((a >> 2) + hl));      // T is 16-byte aligned
-                        return v;
-                    };
-                    auto settle = [&](uint2& v, const u32 a)      // four symbols from the suffix's first, most significant first
-                    {
-                        u32 nx = __shfl_down_sync(0xFFFFFFFFu, v.x, 1, 16);
-                        const u32 ny = __shfl_down_sync(0xFFFFFFFFu, v.y, 1, 16);
-                        if(a & 2) { v.x = v.y; v.y = nx; nx = ny; }
-                        const u32 pick = (a & 1) ? 0x3254 : 0x1032;
-                        v.x = __byte_perm(v.x, v.y, pick);
-                        v.y = __byte_perm(v.y, nx, pick);
-                    };
-                    auto cut = [&](uint2& v, const u32 c) -> u32      // how many of the four count
-                    {
-                        const int h = min(4, int(c) - int(4 * hl));
-                        if(h < 4)
-                        {
-                            const u64 keep = h > 0 ? ~0ull << (64 - 16 * h) : 0ull;
-                            v.x &= u32(keep >> 32); v.y &= u32(keep);
-                        }
-                        return h > 0 ? u32(h) : 0u;
-                    };
-                    if(__any_sync(0xFFFFFFFFu, fetch))
-                    {
-                        uint2 v = make_uint2(0, 0);
-                        u32 a = 0, c = 0;
-                        if(fetch) { place(s0, depth[s0], a, c); v = read(a, c); }
-                        settle(v, a);
-                        const u32 h = cut(v, c);
-                        if(fetch) { lead_x = v.x; lead_y = v.y; lead_have = h; }
+                        x = w.pos[j] + d; y = w.pos[s] + d;
+                        const u64 most = min(to - d, u64(WIDE_REACH));
+                        cx = x < n ? u32(min(n - x, most)) : 0u;
+                        cy = y < n ? u32(min(n - y, most)) : 0u;
+                        first = first_difference(T, x, y, part, min(cx, cy), WIDE_REACH);
                     }
-                    if(todo) lead_slot = s_last;
-                    const bool whole = __all_sync(0xFFFFFFFFu, !mine || cnt == WIDE_REACH);     // no suffix ends inside, `to` is not reached
-                    constexpr int BATCH = 4;
-                    #pragma unroll 1
-                    for(int q = 0; q < 16; q += BATCH)
-                    {
-                        if((both & (0xF000Fu << q)) == 0) continue;
-                        uint2 word[BATCH];
-                        u32 from_at[BATCH];
-                        #pragma unroll
-                        for(int b = 0; b < BATCH; ++b)
-                        {
-                            from_at[b] = __shfl_sync(0xFFFFFFFFu, at, q + b, 16);
-                            const u32 c = whole ? WIDE_REACH : __shfl_sync(0xFFFFFFFFu, cnt, q + b, 16);
-                            word[b] = make_uint2(0, 0);
-                            if(todo >> (q + b) & 1u) word[b] = read(from_at[b], c);
-                        }
-                        #pragma unroll
-                        for(int b = 0; b < BATCH; ++b)
-                        {
-                            settle(word[b], from_at[b]);
-                            u32 have = hl < 15 ? 4 : 0;
-                            if(!whole) have = cut(word[b], __shfl_sync(0xFFFFFFFFu, cnt, q + b, 16));
-                            else if(hl == 15) word[b] = make_uint2(0, 0);
-                            const u32 x = word[b].x, y = word[b].y;
-                            if(leads >> (q + b) & 1u) { lead_x = x; lead_y = y; lead_have = have; }
-                            const bool differs = (todo >> (q + b) & 1u) && (x != lead_x || y != lead_y || have != lead_have);
-                            const u32 all = __ballot_sync(0xFFFFFFFFu, differs);
-                            if(all == 0) continue;
-                            const u32 differ = (all >> half) & 0xFFFFu;
-                            if(differ && hl == __ffs(differ) - 1)
-                            {
-                                const u32 hx = min(have, 2u), lx = min(lead_have, 2u);
-                                key[j0 + q + b] = x != lead_x || hx != lx ? pair_key(2 * hl, x, hx, lead_x, lx) : pair_key(2 * hl + 1, y, have - hx, lead_y, lead_have - lx);
-                            }
-                        }
-                    }
+                    const u32 found = __ballot_sync(0xFFFFFFFFu, first != WIDE_REACH) >> quad & 15u;
+                    if(mine && part == (found ? u32(__ffs(found)) - 1 : 0u))
+                        key[j] = found || cx != cy ? difference_key(T, x, y, cx, cy, found ? first : min(cx, cy)) : KEY_EQUAL;
                 }
             }
             if(!__syncthreads_or(open)) break;
@@ -507,6 +492,7 @@ __global__ void __launch_bounds__(256) gather_ranks_kernel(const u64* __restrict
     }
 }
 
+template <typename K>
 struct Rank_Window
 {
     Group_Starts groups;
@@ -514,17 +500,19 @@ struct Rank_Window
     u32 pre[RW_WINDOW / 32];
     u32 warp_tot[RW_BLOCK / 32];
     u32 slot;
-    u32 sec[RW_WINDOW];
+    K sec[RW_WINDOW];
     Odd_Members odds;
 };
 
-__global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ isa,
+// RANKS: the new ranks go into isa (after the last ordering nobody reads them).
+template <typename K, bool RANKS>
+__global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64* __restrict__ list, const u64 count, const K* __restrict__ secs, u32* __restrict__ isa,
                                                                      u32* __restrict__ sa, u64* __restrict__ next, Build_Counts* __restrict__ counts)
 {
-    __shared__ Rank_Window w;
+    __shared__ Rank_Window<K> w;
     const u32 tid = threadIdx.x;
     const u64 first = u64(blockIdx.x) * RW_TILE;
-    u32 sec[RW_ITEMS];
+    K sec[RW_ITEMS];
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
@@ -543,7 +531,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64*
         u32 s, e;
         find_group(w.groups, entry[i], i, s, e);
         group[i] = s | e << 16;
-        const u32 lead = s != NO_GROUP ? w.sec[s] : sec[i];
+        const K lead = s != NO_GROUP ? w.sec[s] : sec[i];
         odd |= u32(sec[i] != lead) << i;
         smaller |= u32(sec[i] < lead) << i;
         mark_odd(w.odds, i, sec[i] != lead, sec[i] < lead);
@@ -566,7 +554,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64*
         member_place(w.odds, w.sec, j, s, group[i] >> 16, (odd >> i & 1u) != 0, (smaller >> i & 1u) != 0, sec[i], at, to_s, to_e);
         const u32 x = u32(entry[i]);
         new_head[i] = u32(entry[i] >> 32) + (to_s - s);
-        if(to_s != s) isa[x] = new_head[i];
+        if(RANKS && to_s != s) isa[x] = new_head[i];
         if(to_e - to_s == 1) sa[new_head[i]] = x;
         else { place[i] = at; atomicOr(&w.mask[at >> 5], 1u << (at & 31)); }
     }
@@ -578,6 +566,167 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64*
             const u32 q = place[i];
             next[base + w.pre[q >> 5] + __popc(w.mask[q >> 5] & ((1u << (q & 31)) - 1))] = (u64(new_head[i]) << 32) | u32(entry[i]);
         }
+}
+
+// ---- groups that follow one another -----------------------------------------------------------------------------------------------
+//
+// If the suffixes one symbol on from a group's are a whole group again, the two have the same order: the first symbols are the same. In documents that occur
+// many times nearly every group has such a follower, up to the next place where the documents differ. So only the groups without one, the ENDS, are ranked by
+// doubling, and the others take over the order of the end that their followers lead to. A bit per position says that its suffix's group has a follower; the
+// end is as many positions on as there are bits in a row. Some groups, one in 256 by their number, count as ends whatever follows them: no row gets long.
+constexpr u32 FORCED_END = 24;      // bits of a group's scrambled number that are 0 in one of 256
+
+// sa[first slot of every group] = its size (the slots are overwritten when their suffixes are known).
+__global__ void __launch_bounds__(RW_BLOCK) group_sizes_kernel(const u64* __restrict__ list, const u64 count, u32* __restrict__ sa)
+{
+    __shared__ Group_Starts groups;
+    u64 entry[RW_ITEMS];
+    load_entries(groups, list, count, u64(blockIdx.x) * RW_TILE, entry);
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        u32 s, e;
+        find_group(groups, entry[i], i, s, e);
+        if(s == threadIdx.x + i * RW_BLOCK) sa[u32(entry[i] >> 32)] = e - s;
+    }
+}
+
+struct Split_Window
+{
+    Group_Starts groups;
+    u32 sec[RW_WINDOW];
+    Odd_Members odds;
+    u32 keep[RW_WINDOW / 32], pass[RW_WINDOW / 32];             // ends, and groups with a follower: a bit per slot
+    u32 keep_before[RW_WINDOW / 32], pass_before[RW_WINDOW / 32];
+    u32 keep_slot, pass_slot;
+};
+
+// The list's groups into ends (front of next, counts->next_small) and groups with a follower (back of next, counts->large), whose positions' bits are set.
+// secs: what launch_gather_ranks gives one symbol on.
+__global__ void __launch_bounds__(RW_BLOCK, 4) split_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, const u32* __restrict__ sa, const u64 n,
+                                                                    u32* __restrict__ bits, u64* __restrict__ next, Build_Counts* __restrict__ counts)
+{
+    __shared__ Split_Window w;
+    const u32 tid = threadIdx.x;
+    const u64 first = u64(blockIdx.x) * RW_TILE;
+    u32 sec[RW_ITEMS];
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 j = tid + i * RW_BLOCK;
+        sec[i] = first + j < count ? __ldcs(secs + first + j) : 0;
+        w.sec[j] = sec[i];
+    }
+    u64 entry[RW_ITEMS];
+    load_entries(w.groups, list, count, first, entry);
+    u32 group[RW_ITEMS];        // first slot | end << 16
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        u32 s, e;
+        find_group(w.groups, entry[i], i, s, e);
+        group[i] = s | e << 16;
+        mark_odd(w.odds, i, s != NO_GROUP && sec[i] != w.sec[s], false);
+    }
+    __syncthreads();
+    sum_odd(w.odds);
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 s = group[i] & 0xFFFFu, e = group[i] >> 16;
+        bool followed = false;
+        if(s != NO_GROUP && ((odd_before(w.odds, e) ^ odd_before(w.odds, s)) & 0xFFFFu) == 0 && u32(entry[i] >> 32) * 2654435761u >> FORCED_END != 0)
+            followed = sec[i] >= MAX_SMALL_H && sa[sec[i] - u32(MAX_SMALL_H)] == e - s;         // the same rank for all of them: a group of several
+        const u32 f = __ballot_sync(0xFFFFFFFFu, followed), k = __ballot_sync(0xFFFFFFFFu, s != NO_GROUP && !followed);
+        if(lane_id() == 0) { w.pass[i * (RW_BLOCK / 32) + (tid >> 5)] = f; w.keep[i * (RW_BLOCK / 32) + (tid >> 5)] = k; }
+    }
+    __syncthreads();
+    static_assert(RW_WINDOW / 32 == 64, "two words a lane");
+    if(tid < 64)
+    {
+        const u32* const from = tid < 32 ? w.keep : w.pass;
+        u32* const to = tid < 32 ? w.keep_before : w.pass_before;
+        const u32 k = 2 * lane_id(), a = __popc(from[k]), b = __popc(from[k + 1]), inc = warp_sum(a + b);
+        to[k] = inc - a - b;
+        to[k + 1] = inc - b;
+        if(lane_id() == 31 && inc)
+        {
+            if(tid < 32) w.keep_slot = atomicAdd(&counts->next_small, inc);
+            else w.pass_slot = atomicAdd(&counts->large, inc);
+        }
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 j = tid + i * RW_BLOCK, word = j >> 5, below = (1u << (j & 31)) - 1;
+        if(w.keep[word] >> (j & 31) & 1u) next[u64(w.keep_slot) + w.keep_before[word] + __popc(w.keep[word] & below)] = entry[i];
+        else if(w.pass[word] >> (j & 31) & 1u)
+        {
+            next[n - 1 - (u64(w.pass_slot) + w.pass_before[word] + __popc(w.pass[word] & below))] = entry[i];
+            const u32 x = u32(entry[i]);
+            atomicOr(bits + (x >> 5), 1u << (x & 31));
+        }
+    }
+}
+
+// Bits in a row from position x on (x < n; the bit of the last position is never set).
+__device__ __forceinline__ u32 followers(const u64* __restrict__ bits, const u64 x)
+{
+    u64 word = x >> 6;
+    u64 clear = ~__ldg(bits + word) >> (x & 63);
+    if(clear) return u32(__ffsll(clear) - 1);
+    u32 row = 64 - u32(x & 63);
+    while((clear = ~__ldg(bits + ++word)) == 0) row += 64;
+    return row + u32(__ffsll(clear) - 1);
+}
+
+// secs[i]: what the i-th entry of the list of ends is ordered by, h symbols on: the rank there and, of a suffix whose group has a follower, the rank
+// of the end that it leads to: the first is of groups that were told apart before, the second orders inside one of them. A suffix of h symbols comes first.
+__global__ void __launch_bounds__(256) gather_pairs_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ isa, const u64 n, const u64 h,
+                                                          const u64* __restrict__ bits, u64* __restrict__ secs)
+{
+    const u64 first = u64(blockIdx.x) * (256 * GATHER_UNROLL) + threadIdx.x;
+    u64 v[GATHER_UNROLL];
+    #pragma unroll
+    for(int i = 0; i < GATHER_UNROLL; ++i)
+    {
+        const u64 k = first + u64(i) * 256;
+        if(k >= count) continue;
+        const u64 y = u64(u32(__ldcs(list + k))) + h;
+        v[i] = 0;
+        if(y >= n) continue;
+        const u32 rank = __ldg(isa + y), row = followers(bits, y);
+        v[i] = (u64(rank) << 32) | ((row ? __ldg(isa + y + row) : rank) + 1u);
+    }
+    #pragma unroll
+    for(int i = 0; i < GATHER_UNROLL; ++i)
+    {
+        const u64 k = first + u64(i) * 256;
+        if(k < count) __stcs(secs + k, v[i]);
+    }
+}
+
+// secs[i]: the rank of the end that the i-th entry's group leads to.
+__global__ void __launch_bounds__(256) gather_ends_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ isa, const u64* __restrict__ bits, u32* __restrict__ secs)
+{
+    const u64 first = u64(blockIdx.x) * (256 * GATHER_UNROLL) + threadIdx.x;
+    u32 v[GATHER_UNROLL];
+    #pragma unroll
+    for(int i = 0; i < GATHER_UNROLL; ++i)
+    {
+        const u64 k = first + u64(i) * 256;
+        if(k >= count) continue;
+        const u64 x = u32(__ldcs(list + k));
+        v[i] = __ldg(isa + x + followers(bits, x));
+    }
+    #pragma unroll
+    for(int i = 0; i < GATHER_UNROLL; ++i)
+    {
+        const u64 k = first + u64(i) * 256;
+        if(k < count) __stcs(secs + k, v[i]);
+    }
 }
 
 // ---- lists of groups of any size ----------------------------------------------------------------------------------------------
@@ -875,7 +1024,40 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts)
 {
     if(count == 0) return CSA_OK;
-    refine_by_ranks_kernel<<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    refine_by_ranks_kernel<u32, true><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u32* secs, u32* sa, u32* bits, u64* next, Build_Counts* counts)
+{
+    if(count == 0) return CSA_OK;
+    const unsigned tiles = unsigned(div_up(count, RW_TILE));
+    group_sizes_kernel<<<tiles, RW_BLOCK, 0, ctx->stream>>>(list, count, sa);
+    CSA_LAUNCH_CHECK(ctx);
+    CSA_TRY(launch_gather_ranks(ctx, list, count, isa, n, 1, secs));
+    CSA_CUDA(ctx, cudaMemsetAsync(bits, 0, follower_bits_bytes(n), ctx->stream));
+    split_followed_kernel<<<tiles, RW_BLOCK, 0, ctx->stream>>>(list, count, secs, sa, n, bits, next, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* secs, const u32* bits, u32* isa, u64 n, u32* sa, u64* next, Build_Counts* counts)
+{
+    if(count == 0) return CSA_OK;
+    gather_pairs_kernel<<<unsigned(div_up(count, 256 * GATHER_UNROLL)), 256, 0, ctx->stream>>>(list, count, isa, n, h, reinterpret_cast<const u64*>(bits), secs);
+    CSA_LAUNCH_CHECK(ctx);
+    refine_by_ranks_kernel<u64, true><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_order_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, u32* isa, u32* sa, u64* next, Build_Counts* counts)
+{
+    if(count == 0) return CSA_OK;
+    gather_ends_kernel<<<unsigned(div_up(count, 256 * GATHER_UNROLL)), 256, 0, ctx->stream>>>(list, count, isa, reinterpret_cast<const u64*>(bits), secs);
+    CSA_LAUNCH_CHECK(ctx);
+    refine_by_ranks_kernel<u32, false><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

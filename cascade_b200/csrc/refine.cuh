@@ -7,7 +7,7 @@
 
 // Text is compared up to this depth before ranks are: past it one more doubling costs a suffix less (an inverse rank, 64 bytes of
 // DRAM traffic) than its next symbols do.
-constexpr u64 TEXT_DEPTH = 61;         // what tied suffixes share at least (1) + a wide round (refine.cu)
+constexpr u64 TEXT_DEPTH = 49;         // what tied suffixes share at least (1) + a wide round (refine.cu)
 
 // The counters of the build as the stream leaves them; waits for the stream. Fails if a kernel reported an error or if the lists
 // hold more than `most` entries.
@@ -26,6 +26,16 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 // Orders the small groups of the list by secs; new ranks go into isa, single suffixes into sa, the others to `next` behind the
 // counts->next_small entries that are there.
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts);
+
+// Groups whose suffixes lead, one symbol on, to a whole group again (refine.cu). The list's groups are split into those and the ends: ends to the front of next
+// (counts->next_small), the others to its back (counts->large); both counters start from 0, next holds n entries. bits: follower_bits_bytes(n), a
+// bit per position; secs: a word per entry; the first slot of every group in sa receives its size. All groups are small and were ranked by isa.
+inline size_t follower_bits_bytes(u64 n) { return align_up256((n / 64 + 2) * 8); }
+int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u32* secs, u32* sa, u32* bits, u64* next, Build_Counts* counts);
+// One generation of the ends, h symbols on (they share as many): as launch_gather_ranks and launch_refine_by_ranks. secs: a double word per entry.
+int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* secs, const u32* bits, u32* isa, u64 n, u32* sa, u64* next, Build_Counts* counts);
+// The others, once no end is tied: every suffix goes to its slot of sa; next receives nothing.
+int launch_order_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, u32* isa, u32* sa, u64* next, Build_Counts* counts);
 
 // A list of groups of any size (heads, positions; *count_dev entries, at most `most`), group by group: how many of its entries are in small groups
 // (counts->now_small) and where each tile's go; counts->next_small and counts->large are advanced by the two kinds. scratch: 2 words per
