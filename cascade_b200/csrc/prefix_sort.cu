@@ -28,14 +28,6 @@ namespace
 constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of an encoding block
 constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
-#ifndef LR
-#define LR 4
-#endif
-#ifndef OL_B
-#define OL_B 512
-#define OL_I 16
-#define OL_M 2
-#endif
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
 constexpr u32 LOCAL_CHUNK = 2048, SHORT_CHUNK = 1024;
@@ -634,7 +626,7 @@ template <int BLOCK, int ITEMS> constexpr size_t LOCAL_SMEM = size_t(BLOCK * ITE
 constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
 constexpr u32 CROWDED_BIN = 8;      // a batch with larger bins is looked through for bins of one key
 constexpr u32 MANY_TIED = 256;      // a batch with more tied records writes them to the list side by side
-constexpr u32 LONG_BIN = 256;       // a bin with more records is not ordered by comparing all with all
+constexpr u32 LONG_BIN = 256;       // a bin of several keys with more records is not ordered by comparing all with all
 static_assert(MEDIUM_CAP <= 8192, "slots of a batch take 13 bits");
 
 // A record's place in its batch (13 bits), then the first place of its group or, where that is its own, the group's size (14 bits)
@@ -808,34 +800,37 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
             if(m == u32(CAP) && tid == 0) start[CAP] = u16(CAP);       // behind the threads' words
             longest = max(longest & 0xFFFFu, longest >> 16);
             if(longest > CROWDED_BIN) s_crowded = 1;
-            const bool by_network = __syncthreads_or(longest > LONG_BIN);
+            __syncthreads();
             u32 tied = 0;           // a bit per record
-            if(!by_network)
+            // Only the keys are staged, in their bins; a record stays with its thread and counts the smaller and the equal keys of its bin.
+            #pragma unroll
+            for(int i = 0; i < ITEMS; ++i)
             {
-                // Only the keys are staged, in their bins; a record stays with its thread and counts the smaller and the equal keys of its bin.
+                if(i * BLOCK >= m) break;
+                if(tid + i * BLOCK < m) keys[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = u32(r[i] >> 32);
+            }
+            __syncthreads();
+            // Bins of many records are as a rule copies of one key (documents that occur many times): their places are known then.
+            const bool crowded = s_crowded != 0;
+            bool by_network = false;
+            if(crowded)
+            {
                 #pragma unroll
                 for(int i = 0; i < ITEMS; ++i)
                 {
                     if(i * BLOCK >= m) break;
-                    if(tid + i * BLOCK < m) keys[start[pl[i] >> 16] + (pl[i] & 0xFFFFu)] = u32(r[i] >> 32);
-                }
-                __syncthreads();
-                // Bins of many records are as a rule copies of one key (documents that occur many times): their places are known then.
-                const bool crowded = s_crowded != 0;
-                if(crowded)
-                {
-                    #pragma unroll
-                    for(int i = 0; i < ITEMS; ++i)
+                    if(tid + i * BLOCK < m)
                     {
-                        if(i * BLOCK >= m) break;
-                        if(tid + i * BLOCK < m)
-                        {
-                            const u32 b = pl[i] >> 16;
-                            if(keys[start[b]] != u32(r[i] >> 32)) atomicOr(&mixed[b >> 5], 1u << (b & 31));
-                        }
+                        const u32 b = pl[i] >> 16, s = start[b];
+                        if(keys[s] == u32(r[i] >> 32)) continue;
+                        atomicOr(&mixed[b >> 5], 1u << (b & 31));
+                        by_network |= start[b + 1] - s > LONG_BIN;
                     }
-                    __syncthreads();
                 }
+                by_network = __syncthreads_or(by_network);
+            }
+            if(!by_network)
+            {
                 #pragma unroll
                 for(int i = 0; i < ITEMS; ++i)
                 {
@@ -853,9 +848,9 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
                             continue;
                         }
                         #pragma unroll
-                        for(u32 j = 0; j < LR; ++j)      // most bins hold no more: four reads in flight
+                        for(u32 j = 0; j < 4; ++j)      // most bins hold no more: four reads in flight
                             if(s + j < t) { const u32 o = keys[s + j]; less += o < k; upto += o <= k; }
-                        for(u32 j = s + LR; j < t; ++j) { const u32 o = keys[j]; less += o < k; upto += o <= k; }
+                        for(u32 j = s + 4; j < t; ++j) { const u32 o = keys[j]; less += o < k; upto += o <= k; }
                         const u32 head = s + less;
                         if(upto - less == 1) placed[head] = u32(r[i]);
                         else
@@ -872,7 +867,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
             }
             else
             {
-                // Many records in one bin: a sorting network over the batch (keys and positions), then every record finds its
+                // Many records of several keys in one bin: a sorting network over the batch (keys and positions), then every record finds its
                 // group's ends by bisection.
                 u32 size = 1;
                 while(size < m) size <<= 1;
@@ -1136,8 +1131,8 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
     if(one_level)
     {
         static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel<OL_B, OL_I, OL_M, false>, LOCAL_SMEM<OL_B, OL_I>, configured));
-        local_sort_kernel<OL_B, OL_I, OL_M, false><<<unsigned(n / SHORT_CHUNK + parents), OL_B, LOCAL_SMEM<OL_B, OL_I>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false>, LOCAL_SMEM<512, 16>, configured));
+        local_sort_kernel<512, 16, 2, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
         CSA_LAUNCH_CHECK(ctx);
         return CSA_OK;
     }

@@ -550,7 +550,7 @@ __global__ void search_windows_kernel(const csa_index idx, const u64* __restrict
 }
 
 // Eight lanes per query (most match once or a few times, and half of a batch may not match at all): row i of pos receives SA[lo + k],
-// k < min(max_pos, hi - lo). (A warp per query: 126 us for 10^6 queries of up to 20 positions, this way @LOCATE.)
+// k < min(max_pos, hi - lo). (A warp per query: 126 us for 10^6 queries of up to 20 positions, this way 48 us.)
 constexpr u32 LOCATE_LANES = 8;
 
 __global__ void __launch_bounds__(256) locate_rows_kernel(const u8* __restrict__ sa40, const u64* __restrict__ itv, const u64 q, const u32 max_pos, u64* __restrict__ pos,
@@ -788,13 +788,15 @@ namespace
 {
 
 // A batch by slots, 2^22 queries at a time (the scratch is bounded: 180 MB). done stays false where nothing was queued: no room for the scratch, a
-// stream that is being captured (an allocation is not allowed there), a slice of an index, a table without levels to share.
-constexpr u64 DEAL_MIN_QUERIES = u64(1) << 15, DEAL_CHUNK = u64(1) << 22;
+// stream that is being captured (an allocation is not allowed there), a slice of an index, or a batch or a table below the sizes from which on it
+// pays: dealing costs what the searches spare until batches share much of a table beyond L2. us a batch, dealt and in its own order: 5e8 tokens (stride 32)
+// 2^18 queries 169 and 157, 2^19 250 and 277, 2e6 645 and 797; 2e8 tokens 2^19 222 and 232, 2e6 568 and 661; 5e7 tokens (1.6e6 keys) 2^19 182 and 166, 2e6 456 and 462.
+constexpr u64 DEAL_MIN_QUERIES = u64(1) << 19, DEAL_MIN_KEYS = u64(1) << 22, DEAL_CHUNK = u64(1) << 22;
 
 int find_dealt(csa_ctx* ctx, const csa_index& index, const u64* off, const u16* sym, const u64 q, u64* itv, bool& done)
 {
     const u64 J = div_up(index.n, index.stride);
-    if((index.sa_entries != 0 && index.sa_entries < index.n) || J < 4 * SLOTS || J >= (u64(1) << 40)) return CSA_OK;
+    if((index.sa_entries != 0 && index.sa_entries < index.n) || J < DEAL_MIN_KEYS || J >= (u64(1) << 40)) return CSA_OK;
     if(reinterpret_cast<uintptr_t>(itv) & 15) return CSA_OK;
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if(cudaStreamIsCapturing(ctx->stream, &capturing) != cudaSuccess) { cudaGetLastError(); return CSA_OK; }
@@ -937,7 +939,6 @@ __global__ void add_base_kernel(u64* __restrict__ off, const u64 count, const u6
 }
 
 constexpr u64 HOST_CHUNK_QUERIES = u64(1) << 18;     // the reference's chunk of a host batch (include/Query_Engine.hpp:94-100)
-constexpr u64 HOST_CHUNK_MIN = u64(1) << 14;
 
 // Device buffers of one lane of the host-batch pipeline.
 struct Lane_Buffers
@@ -1112,15 +1113,13 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
         }
     }
     CSA_TRY(csa_lanes(ctx));
-    // A batch that would be a chunk or two is cut into four, so that it overlaps its copies, too; a chunk's dozen calls cost what 2^14 queries' answers do.
-    const u64 chunk = sa_on_host ? HOST_CHUNK_QUERIES : std::min(HOST_CHUNK_QUERIES, std::max(HOST_CHUNK_MIN, div_up(q, 4)));
-    const u64 chunks = div_up(q, chunk);
+    const u64 chunks = div_up(q, HOST_CHUNK_QUERIES);
     const int lanes = sa_on_host ? 1 : int(chunks < u64(csa_ctx::LANES) ? chunks : u64(csa_ctx::LANES));
-    const u64 cq_max = q < chunk ? q : chunk;
+    const u64 cq_max = q < HOST_CHUNK_QUERIES ? q : HOST_CHUNK_QUERIES;
     u64 sym_max = 0;
     for(u64 c = 0; c < chunks; ++c)
     {
-        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
+        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
         if(off_host[first + cq] < off_host[first]) return csa_fail(ctx, CSA_E_INVALID, "csa_query_host: offsets must not decrease");
         const u64 sc = off_host[first + cq] - off_host[first];
         if(sc > sym_max) sym_max = sc;
@@ -1149,7 +1148,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
     auto search = [&](u64 c) -> int
     {
         const int l = int(c % u64(lanes));
-        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
+        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
         const u64 sc = off_host[first + cq] - off_host[first];
         const On_Stream on(ctx, ctx->lane[l]);
         CSA_CUDA(ctx, cudaMemcpyAsync(L[l].off, off_host + first, (cq + 1) * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -1177,7 +1176,7 @@ extern "C" int csa_query_host(csa_ctx* ctx, const csa_index* index, const uint64
     {
         if(!want_pos) return CSA_OK;
         const int l = int(c % u64(lanes));
-        const u64 first = c * chunk, cq = (q - first < chunk ? q - first : chunk);
+        const u64 first = c * HOST_CHUNK_QUERIES, cq = (q - first < HOST_CHUNK_QUERIES ? q - first : HOST_CHUNK_QUERIES);
         CSA_CUDA(ctx, cudaEventSynchronize(ctx->lane_event[l]));
         const u64 total = ctx->h_scalars[8 + l];
         const On_Stream on(ctx, ctx->lane[l]);

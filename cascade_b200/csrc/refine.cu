@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     u64* const key = reinterpret_cast<u64*>(smem_raw + (sizeof(Window) + 15) / 16 * 16);     // [RW_WINDOW]
     u32* const depth = reinterpret_cast<u32*>(key + RW_WINDOW);     // [RW_WINDOW] by first slot: symbols that the group's members share (below 2^32: no more than n)
     Odd_Members& odds = *reinterpret_cast<Odd_Members*>(depth + RW_WINDOW);
-    const u32 tid = threadIdx.x;
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
     for(u64 first = u64(blockIdx.x) * RW_TILE; first < count; first += u64(gridDim.x) * RW_TILE)
@@ -335,19 +335,33 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
         for(int i = 0; i < RW_ITEMS; ++i) depth[tid + i * RW_BLOCK] = u32(from);
         __syncthreads();
         int quick = from < QUICK_REACH && to - from >= 2 * QUICK_REACH && count * 4 < n ? 2 : 0;       // rounds of that kind
+        bool again = false;
         while(true)
         {
             const u32 reach = quick ? QUICK_REACH : WIDE_REACH;
-            bool open = false;
+            // w.mask: the slots of groups that go on. Most groups are done with after the first round, and a warp passes over words without such a slot.
+            u32 open = 0;           // the thread's, a bit per item
+            #pragma unroll
+            for(int i = 0; i < RW_ITEMS; ++i)
+            {
+                const u32 word = i * (RW_BLOCK / 32) + warp;
+                if(again && w.mask[word] == 0) continue;
+                const u32 s = w.gs[tid + i * RW_BLOCK];
+                const bool mine = s != NO_GROUP && u32(w.ge[s]) - s >= 2 && u64(depth[s]) < to;
+                const u32 all = __ballot_sync(0xFFFFFFFFu, mine);
+                if(lane == 0) w.mask[word] = all;
+                open |= u32(mine) << i;
+            }
+            again = true;
+            if(!__syncthreads_or(open != 0)) break;
             if(quick)
             {
                 #pragma unroll 4
                 for(int i = 0; i < RW_ITEMS; ++i)
                 {
                     const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
-                    if(s == j) key[j] = KEY_EQUAL;
-                    if(s == NO_GROUP || j == s) continue;
-                    open = true;
+                    if((open >> i & 1u) == 0) continue;
+                    if(j == s) { key[j] = KEY_EQUAL; continue; }
                     const u64 x = u64(w.pos[j]) + depth[s], y = u64(w.pos[s]) + depth[s];
                     const ulonglong2 none = make_ulonglong2(0, 0);
                     const ulonglong2 a = x < n ? eight_symbols(T, x) : none, b = y < n ? eight_symbols(T, y) : none;
@@ -365,18 +379,17 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
             }
             else
             {
-                const u32 part = tid & 3u, quad = lane_id() & ~3u;
+                const u32 part = lane & 3u, quad = lane & ~3u;
                 #pragma unroll (WIDE_ROWS)
-                for(u32 j = tid >> 2; j < RW_WINDOW; j += RW_BLOCK / 4)
+                for(u32 j0 = warp * 8; j0 < RW_WINDOW; j0 += RW_BLOCK / 4)
                 {
-                    const u32 s = w.gs[j];
-                    bool mine = s != NO_GROUP && u32(w.ge[s]) - s >= 2;
-                    const u64 d = mine ? depth[s] : 0;
-                    mine = mine && d < to;
-                    open |= mine;
+                    const u32 eight = w.mask[j0 >> 5] >> (j0 & 31) & 0xFFu, j = j0 + (lane >> 2);
+                    if(eight == 0) continue;
+                    bool mine = eight >> (lane >> 2) & 1u;
+                    const u32 s = mine ? u32(w.gs[j]) : 0u;
                     if(mine && j == s && part == 0) key[j] = KEY_EQUAL;
                     mine = mine && j != s;
-                    if(!__any_sync(0xFFFFFFFFu, mine)) continue;
+                    const u64 d = depth[s];
                     u64 x = 0, y = 0;
                     u32 cx = 0, cy = 0, first = WIDE_REACH;
                     if(mine)
@@ -392,15 +405,20 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
                         key[j] = found || cx != cy ? difference_key(T, x, y, cx, cy, found ? first : min(cx, cy)) : KEY_EQUAL;
                 }
             }
-            if(!__syncthreads_or(open)) break;
+            __syncthreads();
             // the members take their new places
             u64 mine[RW_ITEMS];
             #pragma unroll
             for(int i = 0; i < RW_ITEMS; ++i)
             {
-                const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
+                const u32 word = i * (RW_BLOCK / 32) + warp;
                 mine[i] = KEY_EQUAL;
-                if(s != NO_GROUP && u32(w.ge[s]) - s >= 2 && u64(depth[s]) < to) mine[i] = key[j];
+                if(w.mask[word] == 0)
+                {
+                    if(lane == 0) { odds.odd[word] = 0; odds.less[word] = 0; }
+                    continue;
+                }
+                if(open >> i & 1u) mine[i] = key[tid + i * RW_BLOCK];
                 mark_odd(odds, i, mine[i] != KEY_EQUAL, mine[i] < KEY_EQUAL);
             }
             __syncthreads();
@@ -415,12 +433,9 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
             #pragma unroll
             for(int i = 0; i < RW_ITEMS; ++i)
             {
-                const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
                 go[i] = NO_GROUP;
-                if(s == NO_GROUP) continue;
-                const u32 e = w.ge[s];
-                const u32 d = depth[s];
-                if(e - s < 2 || d >= to) continue;
+                if((open >> i & 1u) == 0) continue;
+                const u32 j = tid + i * RW_BLOCK, s = w.gs[j], e = w.ge[s], d = depth[s];
                 p[i] = w.pos[j];
                 u32 at, to_s;
                 member_place(odds, key, j, s, e, mine[i] != KEY_EQUAL, mine[i] < KEY_EQUAL, mine[i], at, to_s, to_e[i]);

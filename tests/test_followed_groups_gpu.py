@@ -1,0 +1,51 @@
+"""Builds of texts whose tied groups lead to one another (from 2^22 tied suffixes on), each array checked exactly by csa_validate_sa."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from cascade_b200 import api
+    c = api.Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, T):
+    from cascade_b200 import api
+    T = np.ascontiguousarray(T, dtype=np.uint16)
+    n = len(T)
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    sa, st = api.build_sa(ctx, Td, n, 8)
+    v = api.validate_sa(ctx, Td, n, sa)
+    assert v["ok"], v
+    return st
+
+
+@pytest.mark.parametrize("copies,mutate,cut", [(2, 0, 0), (3, 1e-5, 1), (40, 1e-3, 17), (250, 1e-3, 0), (40, 0.05, 3)])
+def test_a_text_that_occurs_many_times(ctx, copies, mutate, cut):
+    """Groups of 2 to 250: rows of followers as long as the text, rows that end where the copies differ, at every few symbols, and at the text's end."""
+    rng = np.random.default_rng(copies)
+    base = rng.integers(1, 60000, 5_200_000 // copies).astype(np.uint16)
+    T = np.tile(base, copies)
+    hit = rng.random(len(T)) < mutate
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    st = _check(ctx, T[:len(T) - cut])
+    assert st.generations > 1
+
+
+def test_documents_in_another_order_every_time(ctx):
+    """Near-duplicate documents with separators, and some passages that stand in the text too often for a small group (then no group is looked at)."""
+    rng = np.random.default_rng(2)
+    docs = [np.concatenate([[65535], np.minimum(rng.zipf(1.2, int(rng.integers(20, 4000))), 50000)]).astype(np.uint16) for _ in range(60)]
+    T = np.concatenate([docs[int(k)] for k in rng.integers(0, 60, 3000)])[:5_500_001]
+    hit = rng.random(len(T)) < 1e-3
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    _check(ctx, T)
+    T[::20000] = 7
+    for k in range(0, len(T) - 40, 19000):
+        T[k:k + 30] = docs[0][1:31] if len(docs[0]) > 31 else 9
+    _check(ctx, T)
