@@ -47,10 +47,12 @@ Build_Layout layout_for(u64 n)
 // From here on a host build is done in four parts, so that the array's copy to the host (9.1 of the 15.6 ms of 1e8 suffixes) runs under
 // the sorting: 13.7 to 14.4 ms (2e9: 0.27 to 0.33 s by box, 0.26 of them copies). Below it the parts' launches cost what the overlap gives.
 constexpr u64 HOST_PARTS_MIN = u64(1) << 23;
-// Tied suffixes from which on groups are looked through for followers. Below, a generation costs its launches: near-duplicates of 10^6 tokens take 657 us
-// without and 740 with it, of 10^7 2461 and 2297 us.
+// Up to here the local sort and the ties by text write 5-byte entries themselves. It spares a pass and a launch but costs instructions, which bound the local
+// sort: 2^24 tokens 573 us without and 557 with it, 2e8 4.56 and 4.53 ms, 2e9 47.2 and 47.4 ms, and a text that is ranked has to be unpacked.
+constexpr u64 PACKED_MAX = u64(1) << 25;
+// Tied suffixes from which on (and a quarter of the text) groups are looked through for followers. Below, a generation costs its launches: near-duplicates of
+// 10^6 tokens took 657 us without and 740 with it.
 constexpr u64 FOLLOWED_MIN = u64(1) << 22;
-constexpr u64 SMALL_BUILD = u64(1) << 22;       // up to here the output is packed before the host knows whether ties are left
 
 int set_build_count(csa_ctx* ctx, u32* at, u32 value)
 {
@@ -84,7 +86,10 @@ struct Build
     u32* pos = nullptr;
     u32* pos_other = nullptr;
 
+    bool ranked = false;        // isa holds every suffix's rank
+
     u64* large_list(u64* buf) const { return buf + (n - large); }
+    u32* ranks() const { return ranked ? isa : nullptr; }
 
     int read_counts(Build_Counts& c) { return read_build_counts(ctx, n, c); }
 
@@ -255,21 +260,31 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     const Ties_In_Any_Order free_ties(ctx);     // ties of the radix sorts are resolved by what follows them
 
     // ---- generation 0, and the ties that it leaves by their symbols --------------------------------------------------------
-    CSA_TRY(launch_prefix_sort(ctx, b.ps, b.tab, T, recA, recB, b.sa, p, b.counts, &b.front, &b.other, ev[1]));
+    // A short build writes its output as positions are found; ranking, if it comes to that, makes 4-byte positions from it.
+    u32* words = n > PACKED_MAX ? b.sa : nullptr;       // b.sa, once the positions are there; the output else
+    CSA_TRY(launch_prefix_sort(ctx, b.ps, b.tab, T, recA, recB, words, sa40, p, b.counts, &b.front, &b.other, ev[1]));
     CSA_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
     const u64 depth0 = u64(b.ps.key_bits / CODE_MAX_LEN);       // symbols that tied suffixes share at least
     u64 depth = TEXT_DEPTH;
+    // More tied suffixes than this are first looked through for groups that follow one another: those need not be compared.
+    const u64 most_by_text = std::max(FOLLOWED_MIN, n / 4);
     Build_Counts c;
-    bool packed = n <= SMALL_BUILD;
-    CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, b.sa, b.counts, n));
-    if(packed) { CSA_CUDA(ctx, cudaEventRecord(ev[3], ctx->stream)); CSA_TRY(launch_pack_sa40(ctx, b.sa, n, sa40)); CSA_CUDA(ctx, cudaEventRecord(ev[4], ctx->stream)); }
+    CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text));
+    bool done = false;          // the output is complete, and the events have been waited for with the counters below
+    if(!words)
+    {
+        CSA_CUDA(ctx, cudaEventRecord(ev[3], ctx->stream));
+        CSA_CUDA(ctx, cudaEventRecord(ev[4], ctx->stream));
+        done = true;
+    }
     CSA_TRY(b.read_counts(c));
     if(c.oversize)
     {
-        packed = false;
+        done = false;
         if(debug) std::fprintf(stderr, "[csa] %u children (%u suffixes) do not fit a block\n", c.oversize, c.oversize_records);
         CSA_TRY(b.sort_oversize(c));
-        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, b.sa, b.counts, n));
+        if(!words) CSA_TRY(launch_pack_oversize(ctx, b.tab, c.oversize, b.sa, sa40));
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text));
         CSA_TRY(b.read_counts(c));
     }
     st.partitions = c.partitions;
@@ -278,19 +293,55 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     if(debug) std::fprintf(stderr, "[csa] n=%llu key bits %d: tied after generation 0: %u in small groups, %u in large ones\n", n, b.ps.key_bits, c.small, c.large);
     u32 gen = 0;
     if(st.active_after_gen0) st.active_per_gen[gen++] = st.active_after_gen0;
+    // Groups that lead, one symbol on, to a whole group again (refine.cu): where they hold half of the tied suffixes, the others alone go on, and they
+    // take over their order at the end (near-duplicate documents: nineteen in twenty).
+    u64 followed = 0;
+    u64* followed_list = nullptr;
+    u32* bits = nullptr;
+    if(c.small > most_by_text)
+    {
+        done = false;
+        u64 ends = c.small;
+        if(!c.large)
+        {
+            CSA_TRY(b.more_memory());
+            if(!words) CSA_TRY(launch_unpack_sa40(ctx, sa40, n, b.sa));
+            words = b.sa;
+            CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, c.small, nullptr, 0, b.isa, reinterpret_cast<u64*>(b.work)));
+            b.ranked = true;
+            bits = reinterpret_cast<u32*>(b.work + (b.L.work - follower_bits_bytes(n)) / 256 * 256);
+            CSA_TRY(launch_split_followed(ctx, b.front, c.small, b.isa, n, reinterpret_cast<u32*>(b.work), b.sa, bits, b.other, b.counts));
+            Build_Counts f;
+            CSA_TRY(b.read_counts(f));
+            if(u64(f.next_small) + f.large != c.small) return csa_fail(ctx, CSA_E_DEVICE, "build: the groups with and without a follower do not add up");
+            if(debug) std::fprintf(stderr, "[csa] %u of %u have a follower\n", f.large, c.small);
+            if(2 * u64(f.large) >= c.small)
+            {
+                followed = f.large;
+                followed_list = b.other + (n - followed);
+                std::swap(b.front, b.other);
+                ends = f.next_small;
+                CSA_TRY(b.set_count(&Build_Counts::small, f.next_small));
+            }
+            CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
+            CSA_TRY(b.set_count(&Build_Counts::large, 0));
+        }
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, b.ranks(), b.counts, ends, n));
+        CSA_TRY(b.read_counts(c));
+    }
     b.large = c.large;
     if(b.large) CSA_CUDA(ctx, cudaMemcpyAsync(b.large_list(b.other), b.large_list(b.front), b.large * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     std::swap(b.front, b.other);
     b.small = c.next_small;
     // Few suffixes left, in small groups: reading on in the text costs less than an inverse array of the whole text.
-    while(b.small && !b.large && b.small * depth <= n && depth < n)
+    while(b.small && !b.large && !followed && b.small * depth <= n && depth < n)
     {
-        packed = false;
+        done = false;
         if(gen < 48) st.active_per_gen[gen] = b.small;
         ++gen;
         CSA_CUDA(ctx, cudaMemcpyAsync(&b.counts->small, &b.counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
         CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
-        CSA_TRY(launch_refine_by_text(ctx, T, n, depth, 4 * depth, b.front, b.other, b.sa, b.counts, b.small));
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth, 4 * depth, b.front, b.other, words, sa40, b.ranks(), b.counts, b.small, n));
         CSA_TRY(b.read_counts(c));
         if(debug) std::fprintf(stderr, "[csa] text up to symbol %llu: %llu -> %u\n", 4 * depth, b.small, c.next_small);
         std::swap(b.front, b.other);
@@ -299,11 +350,13 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     }
 
     // ---- doubling generations -------------------------------------------------------------------------------
-    if(b.small || b.large)
+    if(b.small || b.large || followed)
     {
-        packed = false;
+        done = false;
         CSA_TRY(b.more_memory());
-        CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));
+        if(!words) CSA_TRY(launch_unpack_sa40(ctx, sa40, n, b.sa));
+        words = b.sa;
+        if(!b.ranked) CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));
         u64 idle = b.large ? b.small : 0;               // in small groups already, hence ordered up to `depth`
         u64 shared = depth;                             // symbols that all others' groups share at least
         if(b.large)
@@ -315,28 +368,6 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             CSA_TRY(b.read_counts(c));
             if(c.large_depth < depth0 || c.large_depth > u64(b.ps.key_bits)) return csa_fail(ctx, CSA_E_DEVICE, "build: the large groups' depth is out of range");
             shared = std::min<u64>(c.large_depth, depth);
-        }
-        // Of many small groups those without a follower are ranked alone, where that is at most half of them (near-duplicate documents: a twentieth).
-        u64 followed = 0;
-        u64* followed_list = nullptr;
-        u32* bits = nullptr;
-        if(!b.large && b.small >= FOLLOWED_MIN)
-        {
-            bits = reinterpret_cast<u32*>(b.work + (b.L.work - follower_bits_bytes(n)) / 256 * 256);
-            CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
-            CSA_TRY(b.set_count(&Build_Counts::large, 0));
-            CSA_TRY(launch_split_followed(ctx, b.front, b.small, b.isa, n, reinterpret_cast<u32*>(b.work), b.sa, bits, b.other, b.counts));
-            CSA_TRY(b.read_counts(c));
-            if(u64(c.next_small) + c.large != b.small) return csa_fail(ctx, CSA_E_DEVICE, "build: the groups with and without a follower do not add up");
-            if(debug) std::fprintf(stderr, "[csa] %u of %llu have a follower\n", c.large, b.small);
-            if(2 * u64(c.large) >= b.small)
-            {
-                followed = c.large;
-                followed_list = b.other + (n - followed);
-                std::swap(b.front, b.other);
-                b.small = c.next_small;
-            }
-            CSA_TRY(b.set_count(&Build_Counts::large, 0));
         }
         // Ranks tell `shared` symbols from any step of up to as many: doubling takes the longest step. Above 2^31 suffixes a step may be too long for
         // a sort key of two ranks (n - 1 + h has to fit beside bits_for(n - 1) bits in 64); steps of the longest that fits go on from there.
@@ -367,10 +398,10 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     st.generations = gen;
 
     // ---- output ------------------------------------------------------------------------------------------------
-    if(!packed)
+    if(!done)
     {
         CSA_CUDA(ctx, cudaEventRecord(ev[3], ctx->stream));
-        CSA_TRY(launch_pack_sa40(ctx, b.sa, n, sa40));
+        if(words) CSA_TRY(launch_pack_sa40(ctx, b.sa, n, sa40));
         CSA_CUDA(ctx, cudaEventRecord(ev[4], ctx->stream));
         u64 bits = 0;
         CSA_TRY(csa_sync(ctx, reinterpret_cast<uint64_t*>(&bits)));

@@ -320,6 +320,32 @@ __global__ void pack_sa40_kernel(const u32* __restrict__ sa, const u64 count, u8
     }
 }
 
+__global__ void __launch_bounds__(256) unpack_sa40_kernel(const u8* __restrict__ sa40, const u64 count, u32* __restrict__ sa)
+{
+    const u64 first = (u64(blockIdx.x) * 256 + threadIdx.x) * 16;
+    if(first >= count) return;
+    if(first + 16 <= count)
+    {
+        u32 w[20];
+        const uint4* const src = reinterpret_cast<const uint4*>(sa40 + first * 5);
+        #pragma unroll
+        for(int i = 0; i < 5; ++i) { const uint4 t = src[i]; w[4 * i] = t.x; w[4 * i + 1] = t.y; w[4 * i + 2] = t.z; w[4 * i + 3] = t.w; }
+        u32 v[16];
+        #pragma unroll
+        for(int e = 0; e < 16; ++e)
+        {
+            const int b = 5 * e, wi = b >> 2, sh = (b & 3) * 8;
+            v[e] = sh ? __funnelshift_r(w[wi], w[wi + 1], sh) : w[wi];
+        }
+        uint4* const dst = reinterpret_cast<uint4*>(sa + first);
+        #pragma unroll
+        for(int i = 0; i < 4; ++i) dst[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+    else
+        for(u64 r = first; r < count; ++r)
+            sa[r] = u32(sa40[5 * r]) | u32(sa40[5 * r + 1]) << 8 | u32(sa40[5 * r + 2]) << 16 | u32(sa40[5 * r + 3]) << 24;
+}
+
 }   // namespace
 
 int launch_keys_gen0(csa_ctx* ctx, const u16* T, const u32* pos, u64 count, u64* keys)
@@ -357,6 +383,14 @@ int launch_pack_sa40(csa_ctx* ctx, const u32* sa, u64 count, u8* sa40)
 {
     if(count == 0) return CSA_OK;
     pack_sa40_kernel<<<unsigned(div_up(div_up(count, 16), 256)), 256, 0, ctx->stream>>>(sa, count, sa40);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_unpack_sa40(csa_ctx* ctx, const u8* sa40, u64 count, u32* sa)
+{
+    if(count == 0) return CSA_OK;
+    unpack_sa40_kernel<<<unsigned(div_up(div_up(count, 16), 256)), 256, 0, ctx->stream>>>(sa40, count, sa);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -77,6 +77,8 @@ int launch_keys_add(csa_ctx* ctx, const u32* perm, const u32* resp, u64 count, u
 
 // sa40[5 r, 5 r + 5) = sa[r], little-endian, for r < count.
 int launch_pack_sa40(csa_ctx* ctx, const u32* sa, u64 count, u8* sa40);
+// The low 32 bits of the entries.
+int launch_unpack_sa40(csa_ctx* ctx, const u8* sa40, u64 count, u32* sa);
 
 // The suffix array of a text on the device, part by part into host memory (see stream_build.cu). Leaves `done` false, and whatever it
 // wrote, where the text alone does not order a part; the statistics are then untouched.

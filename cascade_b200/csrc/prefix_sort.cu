@@ -644,9 +644,42 @@ __device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, con
 // whole and looked up again by its place 5.17). A block reads its next chunk ahead.
 // MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
 // there if a block of 16 records a thread holds them, and to the front, for the radix sort, if not.
-template <int BLOCK, int ITEMS, int BLOCKS, bool MEDIUM>
+// The batch's entries [base, base + m) as 5-byte ones, from shared memory: four are 20 bytes, which begin on a word where the first's slot is a multiple of
+// four; the words of 128 entries go out side by side by way of the warp's part of `words`. The up to three entries before and behind go byte by byte.
+template <int BLOCK, int CAP>
+__device__ __forceinline__ void write_packed(u32* words, const u32* placed, const u32 m, const u32 base, u8* __restrict__ sa40)
+{
+    constexpr u32 WARPS = BLOCK / 32;
+    static_assert(CAP / WARPS >= 160, "a warp's words");
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const u32 head = min(m, (0u - base) & 3u), fours = (m - head) >> 2, tail = head + 4 * fours;
+    u32* const mine = words + warp * (CAP / WARPS);
+    u32* const out = reinterpret_cast<u32*>(sa40 + 5 * u64(base + head));
+    for(u32 q0 = warp * 32; q0 < fours; q0 += WARPS * 32)
+    {
+        if(q0 + lane < fours)
+        {
+            const u32* const v = placed + head + 4 * (q0 + lane);
+            const u32 a = v[0], b = v[1], c = v[2], d = v[3];
+            u32* const w = mine + 5 * lane;
+            w[0] = a; w[1] = b << 8; w[2] = b >> 24 | c << 16; w[3] = c >> 16 | d << 24; w[4] = d >> 8;
+        }
+        __syncwarp();
+        const u32 count = min(fours - q0, 32u) * 5;
+        for(u32 k = lane; k < count; k += 32) out[u64(q0) * 5 + k] = mine[k];
+        __syncwarp();
+    }
+    if(tid < (head + m - tail) * 5)
+    {
+        const u32 e = tid < head * 5 ? tid / 5 : tail + (tid - head * 5) / 5, byte = tid % 5;
+        sa40[5 * u64(base + e) + byte] = byte < 4 ? u8(placed[e] >> (8 * byte)) : u8(0);
+    }
+}
+
+// PACKED: the array is written to sa40 as 5-byte entries, else to sa.
+template <int BLOCK, int ITEMS, int BLOCKS, bool MEDIUM, bool PACKED>
 __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
-                                                                   const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u64* __restrict__ list,
+                                                                   const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u8* __restrict__ sa40, u64* __restrict__ list,
                                                                    const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap)
 {
     constexpr int CAP = BLOCK * ITEMS;
@@ -909,12 +942,16 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
                 }
             }
             const bool ties = __syncthreads_or(tied != 0);
-            #pragma unroll
-            for(int i = 0; i < ITEMS; ++i)
+            if(PACKED) write_packed<BLOCK, CAP>(keys, placed, m, base, sa40);
+            else
             {
-                const u32 j = tid + i * BLOCK;
-                if(j >= m) break;
-                sa[base + j] = placed[j];
+                #pragma unroll
+                for(int i = 0; i < ITEMS; ++i)
+                {
+                    const u32 j = tid + i * BLOCK;
+                    if(j >= m) break;
+                    sa[base + j] = placed[j];
+                }
             }
             // The tied records go to the list, a group's side by side: the first of a group takes its places (start[] is free now).
             if(ties)
@@ -993,6 +1030,21 @@ __global__ void __launch_bounds__(256) gather_oversize_kernel(const u64* __restr
                 vals[s_at + j] = u32(v);
             }
             __syncthreads();
+        }
+    }
+}
+
+// The entries of oversize children from sa to sa40.
+__global__ void __launch_bounds__(256) pack_oversize_kernel(const u32* __restrict__ sa, const u32* __restrict__ over, const u32 oversize, const u32* __restrict__ child_off,
+                                                           u8* __restrict__ sa40)
+{
+    for(u32 o = blockIdx.y; o < oversize; o += gridDim.y)
+    {
+        const u64 first = u64(child_off[over[o]]) * 5, end = u64(child_off[over[o] + 1]) * 5;
+        for(u64 b = first + u64(blockIdx.x) * 256 + threadIdx.x; b < end; b += u64(gridDim.x) * 256)
+        {
+            const u32 byte = u32(b % 5);
+            sa40[b] = byte < 4 ? u8(sa[b / 5] >> (8 * byte)) : u8(0);
         }
     }
 }
@@ -1124,31 +1176,32 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
 }
 
 // The second launch takes the children of 4097 to 8192 suffixes; a short text, where a launch counts, goes to the larger blocks at once.
-int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, bool one_level, u64 n, const u64* rec, u32* sa, u64* list, Build_Counts* counts)
+template <bool PACKED>
+int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, bool one_level, u64 n, const u64* rec, u32* sa, u8* sa40, u64* list, Build_Counts* counts)
 {
     const u32 over_cap = parents << b2;
     const u32* const chunks = t.chunk0 + parents;
-    if(one_level)
+    if(PACKED && one_level)     // texts of one split are short
     {
         static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false>, LOCAL_SMEM<512, 16>, configured));
-        local_sort_kernel<512, 16, 2, false><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false, PACKED>, LOCAL_SMEM<512, 16>, configured));
+        local_sort_kernel<512, 16, 2, false, PACKED><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
         CSA_LAUNCH_CHECK(ctx);
         return CSA_OK;
     }
     static std::atomic<bool> configured[2][64];
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 8, 3, false>, LOCAL_SMEM<512, 8>, configured[0]));
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, true>, LOCAL_SMEM<512, 16>, configured[1]));
-    local_sort_kernel<512, 8, 3, false><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 3 * 8)), 512, LOCAL_SMEM<512, 8>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 8, 3, false, PACKED>, LOCAL_SMEM<512, 8>, configured[0]));
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, true, PACKED>, LOCAL_SMEM<512, 16>, configured[1]));
+    local_sort_kernel<512, 8, 3, false, PACKED><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 3 * 8)), 512, LOCAL_SMEM<512, 8>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
-    local_sort_kernel<512, 16, 2, true><<<148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, list, n, counts, t.over, over_cap);
+    local_sort_kernel<512, 16, 2, true, PACKED><<<148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
 
 }   // namespace
 
-int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
+int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u8* sa40, u32 p, Build_Counts* counts,
                        u64** list, u64** records, cudaEvent_t after_first_split)
 {
     const u64 n = ps.n;
@@ -1170,7 +1223,8 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
         CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB));
         rec = recB; other = recA;
     }
-    CSA_TRY(launch_local_sort(ctx, t, ps.parents, ps.b2, one_level, n, rec, sa, other, counts));
+    CSA_TRY(sa ? launch_local_sort<false>(ctx, t, ps.parents, ps.b2, one_level, n, rec, sa, nullptr, other, counts)
+               : launch_local_sort<true>(ctx, t, ps.parents, ps.b2, one_level, n, rec, nullptr, sa40, other, counts));
     *list = other;
     *records = rec;
     return CSA_OK;
@@ -1203,7 +1257,7 @@ int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Ta
     CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
                              : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));
     CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB));
-    CSA_TRY(launch_local_sort(ctx, t, bins, ps.b2, false, size, recB, sa, recA, counts));
+    CSA_TRY(launch_local_sort<false>(ctx, t, bins, ps.b2, false, size, recB, sa, nullptr, recA, counts));
     ctx->counters[1] += 2;
     ctx->counters[2] += 2 * size;
     return CSA_OK;
@@ -1218,6 +1272,15 @@ int launch_gather_oversize(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tab
     // 2^24 suffixes took 1.2 ms; this way 0.06 ms.
     const unsigned rows = oversize < 1024 ? oversize : 1024;
     gather_oversize_kernel<<<dim3(std::max(32u, std::min(148u * 8, (1u << 14) / rows)), rows), 256, 0, ctx->stream>>>(records, t.over, oversize, t.child_off, keys, vals, cursor);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+int launch_pack_oversize(csa_ctx* ctx, const Prefix_Tables& t, u32 oversize, const u32* sa, u8* sa40)
+{
+    if(oversize == 0) return CSA_OK;
+    const unsigned rows = oversize < 1024 ? oversize : 1024;
+    pack_oversize_kernel<<<dim3(std::max(32u, std::min(148u * 8, (1u << 14) / rows)), rows), 256, 0, ctx->stream>>>(sa, t.over, oversize, t.child_off, sa40);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -56,14 +56,15 @@ struct Prefix_Tables
 };
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t);
 
-// Orders the suffixes of T by the first key_bits bits of their encoding. recA and recB: n records each. sa receives every
+// Orders the suffixes of T by the first key_bits bits of their encoding. recA and recB: n records each. sa or, where that is null, sa40 (5-byte entries) receives every
 // suffix that is alone with its key, at its final place, and SA_OPEN elsewhere; the tied ones go to `list` (the record buffer
 // that is returned as *list; *records is the other one), small groups from the front, large ones from the back, as
 // (first slot of the group << 32) | position, group by group. p only says how many partitions the statistics tell apart. Nothing is read back.
-int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u32 p, Build_Counts* counts,
+int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, const u16* T, u64* recA, u64* recB, u32* sa, u8* sa40, u32 p, Build_Counts* counts,
                        u64** list, u64** records, cudaEvent_t after_first_split);
 // The records of the children that did not fit a block, as sort records: keys = (first slot of the child << 32) | key,
 // vals = position.
+int launch_pack_oversize(csa_ctx* ctx, const Prefix_Tables& t, u32 oversize, const u32* sa, u8* sa40);      // their slots, once sorted and ranked, as 5-byte entries
 int launch_gather_oversize(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables& t, u32 oversize, const u64* records, u64* keys, u32* vals, u32* cursor);
 
 // The same for a text whose records do not all fit the device: one contiguous range of the suffix array at a time. The first split's

@@ -318,7 +318,8 @@ __device__ __forceinline__ u64 difference_key(const u16* __restrict__ T, const u
 // Where few suffixes are tied, nearly all of them differ within a few symbols and
 // the chain of loads counts: the first round is then QUICK, 8 symbols by one thread, all of a thread's suffixes in flight together.
 __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
-                                                                    u64* __restrict__ next, u32* __restrict__ sa, Build_Counts* __restrict__ counts)
+                                                                    u64* __restrict__ next, u32* __restrict__ sa, u8* __restrict__ sa40, u32* __restrict__ isa, Build_Counts* __restrict__ counts,
+                                                                    const u64 most)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Window& w = *reinterpret_cast<Window*>(smem_raw);
@@ -328,6 +329,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
+    if(count > most) return;
     for(u64 first = u64(blockIdx.x) * RW_TILE; first < count; first += u64(gridDim.x) * RW_TILE)
     {
         load_window(w, list, count, first);
@@ -465,7 +467,17 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
         {
             const u32 j = tid + i * RW_BLOCK, s = w.gs[j];
             if(s == NO_GROUP) continue;
-            if(u32(w.ge[s]) - s < 2) sa[w.head[j]] = w.pos[j];
+            const u32 x = w.pos[j];
+            if(isa) isa[x] = w.head[s];
+            if(u32(w.ge[s]) - s < 2)
+            {
+                if(sa) sa[w.head[j]] = x;
+                else
+                {
+                    u8* const at = sa40 + 5 * u64(w.head[j]);
+                    at[0] = u8(x); at[1] = u8(x >> 8); at[2] = u8(x >> 16); at[3] = u8(x >> 24); at[4] = 0;
+                }
+            }
             else { tied |= 1u << i; atomicOr(&w.mask[j >> 5], 1u << (j & 31)); }
         }
         if(__syncthreads_or(tied != 0))
@@ -1018,12 +1030,13 @@ int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c)
     return CSA_OK;
 }
 
-int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, Build_Counts* counts, u64 expected)
+int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, u8* sa40, u32* isa, Build_Counts* counts, u64 expected,
+                          u64 most)
 {
     to = to < n ? to : n;           // no two suffixes share as much
     CSA_CUDA(ctx, cudaFuncSetAttribute(refine_by_text_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TEXT_SMEM)));
     const u64 tiles = div_up(expected ? expected : 1, RW_TILE);
-    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, counts);
+    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, sa40, isa, counts, most);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

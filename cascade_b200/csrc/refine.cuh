@@ -15,9 +15,10 @@ int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c);
 
 // Orders the small groups of `list` by their suffixes' symbols [from, to) read straight from the text (a suffix that ends
 // inside them comes before those that go on): every group that is left shares `to` symbols. Suffixes that are alone now go to
-// their slots of sa, the others to next (front; counts->next_small entries). `expected`: about how many entries the list holds
+// their slots of sa or, where sa is null, as 5-byte entries to sa40, the others to next (front; counts->next_small entries). `expected`: about how many entries the list holds
 // (its length is counts->small).
-int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, Build_Counts* counts, u64 expected);
+// A list of more than `most` entries is left alone. isa (or null): every suffix's new rank goes there, too.
+int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, u8* sa40, u32* isa, Build_Counts* counts, u64 expected, u64 most);
 
 // secs[i] = what the i-th entry of the list is ordered by in the generation that compares h symbols further on: the rank of the
 // suffix h symbols on, or, where the text ends before, a smaller number that falls with the position.
@@ -28,7 +29,7 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts);
 
 // Groups whose suffixes lead, one symbol on, to a whole group again (refine.cu). The list's groups are split into those and the ends: ends to the front of next
-// (counts->next_small), the others to its back (counts->large); both counters start from 0, next holds n entries. bits: follower_bits_bytes(n), a
+// (counts->next_small), the others to its back (counts->large); both counters start from 0, next holds n entries. A group shares a symbol at least. bits: follower_bits_bytes(n), a
 // bit per position; secs: a word per entry; the first slot of every group in sa receives its size. All groups are small and were ranked by isa.
 inline size_t follower_bits_bytes(u64 n) { return align_up256((n / 64 + 2) * 8); }
 int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u32* secs, u32* sa, u32* bits, u64* next, Build_Counts* counts);

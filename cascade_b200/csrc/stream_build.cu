@@ -907,13 +907,13 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
         CSA_TRY(launch_prefix_sort_part(ctx, ps, tab, T, first_bin[u], first_bin[u + 1] - first_bin[u], S, recA, recB, sa, counts));
         u64* list = recA;
         u64* next = recB;
-        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, nullptr, nullptr, counts, S, S));
         Build_Counts c;
         CSA_TRY(read_build_counts(ctx, S, c));
         if(c.oversize && c.oversize_records <= S / OVERSIZE_SHARE)
         {
             CSA_TRY(sort_oversize_children(ctx, ps, tab, c, S, list, next, sa, counts, oversize_buffers(over_at, most / OVERSIZE_SHARE)));
-            CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, counts, S));
+            CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, TEXT_DEPTH, list, next, sa, nullptr, nullptr, counts, S, S));
             CSA_TRY(read_build_counts(ctx, S, c));
         }
         if(c.oversize || c.large) return CSA_OK;
@@ -926,7 +926,7 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
             std::swap(list, next);
             CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
             CSA_CUDA(ctx, cudaMemsetAsync(&counts->next_small, 0, 4, ctx->stream));
-            CSA_TRY(launch_refine_by_text(ctx, T, n, depth, 4 * depth, list, next, sa, counts, small));
+            CSA_TRY(launch_refine_by_text(ctx, T, n, depth, 4 * depth, list, next, sa, nullptr, nullptr, counts, small, small));
             CSA_TRY(read_build_counts(ctx, S, c));
             depth *= 4;
             ++r;
