@@ -385,15 +385,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             shared += h;
             if(shared > 2 * n + 2 * depth) return csa_fail(ctx, CSA_E_DEVICE, "build: doubling did not terminate");
         }
-        if(followed)
-        {
-            // the list lies in one of the two record buffers, what is written behind it (nothing) in the other
-            u64* const next = followed_list >= b.front && followed_list < b.front + n ? b.other : b.front;
-            CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
-            CSA_TRY(launch_order_followed(ctx, followed_list, followed, reinterpret_cast<u32*>(b.work), bits, b.isa, b.sa, next, b.counts));
-            CSA_TRY(b.read_counts(c));
-            if(c.next_small != 0) return csa_fail(ctx, CSA_E_DEVICE, "build: suffixes are tied although the ends that they lead to are not");
-        }
+        if(followed) CSA_TRY(launch_place_followed(ctx, followed_list, followed, reinterpret_cast<u32*>(b.work), bits, b.isa, b.sa));
     }
     st.generations = gen;
 

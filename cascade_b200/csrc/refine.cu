@@ -314,7 +314,8 @@ __device__ __forceinline__ u64 difference_key(const u16* __restrict__ T, const u
 //
 // A WIDE round compares 48 symbols: four lanes read a suffix, a sector each, all of it in flight at once, and the first member's symbols beside it, which the
 // neighbouring lanes read as well; a difference is then read symbol by symbol. (Half a warp to a suffix, four symbols a lane: 58 warp instructions a suffix,
-// 9.45 ms for 10^8 near-duplicate suffixes; a thread to a suffix, a sector after the other: 11.5 ms; this way @REFINE.)
+// 9.45 ms for 10^8 near-duplicate suffixes; a thread to a suffix, a sector after the other: 11.5 ms; this way 8.9 ms, and 7.8 ms
+// with what is done with passed over.)
 // Where few suffixes are tied, nearly all of them differ within a few symbols and
 // the chain of loads counts: the first round is then QUICK, 8 symbols by one thread, all of a thread's suffixes in flight together.
 __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
@@ -531,8 +532,7 @@ struct Rank_Window
     Odd_Members odds;
 };
 
-// RANKS: the new ranks go into isa (after the last ordering nobody reads them).
-template <typename K, bool RANKS>
+template <typename K>
 __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64* __restrict__ list, const u64 count, const K* __restrict__ secs, u32* __restrict__ isa,
                                                                      u32* __restrict__ sa, u64* __restrict__ next, Build_Counts* __restrict__ counts)
 {
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_ranks_kernel(const u64*
         member_place(w.odds, w.sec, j, s, group[i] >> 16, (odd >> i & 1u) != 0, (smaller >> i & 1u) != 0, sec[i], at, to_s, to_e);
         const u32 x = u32(entry[i]);
         new_head[i] = u32(entry[i] >> 32) + (to_s - s);
-        if(RANKS && to_s != s) isa[x] = new_head[i];
+        if(to_s != s) isa[x] = new_head[i];
         if(to_e - to_s == 1) sa[new_head[i]] = x;
         else { place[i] = at; atomicOr(&w.mask[at >> 5], 1u << (at & 31)); }
     }
@@ -732,6 +732,46 @@ __global__ void __launch_bounds__(256) gather_pairs_kernel(const u64* __restrict
     {
         const u64 k = first + u64(i) * 256;
         if(k < count) __stcs(secs + k, v[i]);
+    }
+}
+
+// The groups with a follower, once no end is tied: a group leads to the suffixes of one end group, whose ranks by now are its slots, one each. So a suffix is
+// as far behind its group's first slot as its end's rank is behind the least of them. (Ordered as in a generation, by counting the members of a group against one
+// another: 1.57 ms for 10^8 suffixes in groups of 16 and 20 ms for 4e8 in groups of 48; this way builds of them took 1.2 and 8.0 ms less.)
+__global__ void __launch_bounds__(RW_BLOCK) place_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ sa, u64* __restrict__ dev_status)
+{
+    __shared__ Group_Starts groups;
+    __shared__ u32 least[RW_WINDOW];            // by first slot
+    const u32 tid = threadIdx.x;
+    const u64 first = u64(blockIdx.x) * RW_TILE;
+    u32 sec[RW_ITEMS];
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 j = tid + i * RW_BLOCK;
+        sec[i] = first + j < count ? __ldcs(secs + first + j) : 0;
+        least[j] = 0xFFFFFFFFu;
+    }
+    u64 entry[RW_ITEMS];
+    load_entries(groups, list, count, first, entry);
+    u32 group[RW_ITEMS];        // first slot | end << 16
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        u32 s, e;
+        find_group(groups, entry[i], i, s, e);
+        group[i] = s | e << 16;
+        if(s != NO_GROUP) atomicMin(&least[s], sec[i]);
+    }
+    __syncthreads();
+    #pragma unroll
+    for(int i = 0; i < RW_ITEMS; ++i)
+    {
+        const u32 s = group[i] & 0xFFFFu, e = group[i] >> 16;
+        if(s == NO_GROUP) continue;
+        const u32 behind = sec[i] - least[s];
+        if(behind < e - s) sa[u32(entry[i] >> 32) + behind] = u32(entry[i]);
+        else atomicOr(reinterpret_cast<unsigned long long*>(dev_status), (unsigned long long)CSA_ST_UNSERVED);
     }
 }
 
@@ -1052,7 +1092,7 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts)
 {
     if(count == 0) return CSA_OK;
-    refine_by_ranks_kernel<u32, true><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    refine_by_ranks_kernel<u32><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1075,17 +1115,17 @@ int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* sec
     if(count == 0) return CSA_OK;
     gather_pairs_kernel<<<unsigned(div_up(count, 256 * GATHER_UNROLL)), 256, 0, ctx->stream>>>(list, count, isa, n, h, reinterpret_cast<const u64*>(bits), secs);
     CSA_LAUNCH_CHECK(ctx);
-    refine_by_ranks_kernel<u64, true><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    refine_by_ranks_kernel<u64><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
 
-int launch_order_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, u32* isa, u32* sa, u64* next, Build_Counts* counts)
+int launch_place_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, const u32* isa, u32* sa)
 {
     if(count == 0) return CSA_OK;
     gather_ends_kernel<<<unsigned(div_up(count, 256 * GATHER_UNROLL)), 256, 0, ctx->stream>>>(list, count, isa, reinterpret_cast<const u64*>(bits), secs);
     CSA_LAUNCH_CHECK(ctx);
-    refine_by_ranks_kernel<u32, false><<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, isa, sa, next, counts);
+    place_followed_kernel<<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, sa, ctx->d_status);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -35,8 +35,8 @@ inline size_t follower_bits_bytes(u64 n) { return align_up256((n / 64 + 2) * 8);
 int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u32* secs, u32* sa, u32* bits, u64* next, Build_Counts* counts);
 // One generation of the ends, h symbols on (they share as many): as launch_gather_ranks and launch_refine_by_ranks. secs: a double word per entry.
 int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* secs, const u32* bits, u32* isa, u64 n, u32* sa, u64* next, Build_Counts* counts);
-// The others, once no end is tied: every suffix goes to its slot of sa; next receives nothing.
-int launch_order_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, u32* isa, u32* sa, u64* next, Build_Counts* counts);
+// The others, once no end is tied: every suffix goes to its slot of sa.
+int launch_place_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, const u32* isa, u32* sa);
 
 // A list of groups of any size (heads, positions; *count_dev entries, at most `most`), group by group: how many of its entries are in small groups
 // (counts->now_small) and where each tile's go; counts->next_small and counts->large are advanced by the two kinds. scratch: 2 words per

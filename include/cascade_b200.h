@@ -427,7 +427,8 @@ int csa_table_build(csa_ctx* ctx, const uint16_t* text_dev, uint64_t n, const ui
                     uint64_t* table_dev);
 /* SA intervals of q queries: query i is sym_dev[off_dev[i] - off_dev[0], ...) of length off_dev[i+1] - off_dev[i];
  * itv_dev receives {lo, hi} pairs. Semantics of ref::find_one (include/CPU_Reference.hpp:42-73). Replaces
- * Query_Engine::find_async (src/Query_Engine.cu:1314) with its rank and search kernels (:176-279, :369-418). */
+ * Query_Engine::find_async (src/Query_Engine.cu:1314) with its rank and search kernels (:176-279, :369-418). Batches of 2^19 queries
+ * and more on a whole index of 2^22 table keys and more take up to 190 MB of scratch, which the context keeps; where it cannot be had, they do without. */
 int csa_find(csa_ctx* ctx, const csa_index* index, const uint64_t* off_dev, const uint16_t* sym_dev, uint64_t q,
              uint64_t* itv_dev);
 /* Positions of each query: SA[lo + k] for k < min(max_pos, hi - lo), in rank order, written to row i of
