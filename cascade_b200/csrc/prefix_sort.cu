@@ -42,6 +42,7 @@ constexpr size_t HIST_SMEM = 65536 * 2;
 // fewer than 65536 symbols.
 __global__ void __launch_bounds__(HIST_BLOCK) sample_symbols_kernel(const u16* __restrict__ T, const u64 n, const u64 vectors, u32* __restrict__ hist)
 {
+    let_next_in();
     extern __shared__ __align__(16) u32 h[];
     for(u32 i = threadIdx.x; i < 32768; i += HIST_BLOCK) h[i] = 0;
     __syncthreads();
@@ -120,6 +121,8 @@ template <bool COUNT>
 __global__ void __launch_bounds__(CODE_BLOCK) make_code_kernel(const u16* __restrict__ T, const u32 n, const u32* __restrict__ hist, const u32 scale, u32* __restrict__ code,
                                                               u32* __restrict__ cnt1, u32* __restrict__ counts)
 {
+    let_next_in();
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u16* const low = reinterpret_cast<u16*>(smem_raw);
     u8* const high = smem_raw + CODE_LOW_BYTES;
@@ -291,6 +294,8 @@ __device__ __forceinline__ u64 encode_tile(const u16* __restrict__ T, const u64 
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) count_text_kernel(const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const int bits, u32* __restrict__ counts)
 {
+    let_next_in();
+    wait_for_previous();
     __shared__ Tile_Code<BLOCK> tc;
     __shared__ u32 cnt[1 << MAX_B1];
     const u32 bins = 1u << bits;
@@ -387,6 +392,8 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
                                                              u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ chunk0, u32* __restrict__ child_off, u32* __restrict__ chunk_first,
                                                              const u32 p, Build_Counts* __restrict__ stats)
 {
+    let_next_in();
+    wait_for_previous();
     __shared__ u32 warp_tot[32];
     __shared__ u32 part[CSA_MAX_PARTITIONS];
     const u32 t = threadIdx.x;
@@ -429,6 +436,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
                                                                           const int keep_top, const u32 first_bin, const u32 part_bins, u32* __restrict__ cursor,
                                                                           u64* __restrict__ out)
 {
+    wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);
     static_assert(TILE_POSITIONS<BLOCK> <= 1 << 13 && MAX_B1 + 13 <= 32, "a staged record's lower word: its bin and its place in the tile");
@@ -1065,8 +1073,7 @@ int launch_scatter_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int 
 {
     static std::atomic<bool> configured[64];
     CSA_TRY(shared_bytes(ctx, scatter_text_kernel<BLOCK, PART>, SCATTER_TEXT_SMEM<BLOCK>, configured));
-    scatter_text_kernel<BLOCK, PART><<<unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, SCATTER_TEXT_SMEM<BLOCK>, ctx->stream>>>(T, n, code, bits, keep_top, first_bin, part_bins,
-                                                                                                                                cursor, out);
+    launch_early(scatter_text_kernel<BLOCK, PART>, unsigned(div_up(n, TILE_POSITIONS<BLOCK>)), BLOCK, SCATTER_TEXT_SMEM<BLOCK>, ctx->stream, T, n, code, bits, keep_top, first_bin, part_bins, cursor, out);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1138,8 +1145,8 @@ int launch_code(csa_ctx* ctx, const Prefix_Tables& t, const u16* T, const u64 n,
         CSA_CUDA(ctx, cudaMemsetAsync(t.hist, 0, 65536 * 4, ctx->stream));
         sample_symbols_kernel<<<unsigned(blocks > 148 ? 148 : blocks), HIST_BLOCK, HIST_SMEM, ctx->stream>>>(T, n, vectors, t.hist);
         CSA_LAUNCH_CHECK(ctx);
-        make_code_kernel<false><<<65536 / CODE_WALKERS, CODE_BLOCK, CODE_SMEM, ctx->stream>>>(T, u32(n), t.hist, u32((u64(1) << 22) / samples), t.code, t.cnt1,
-                                                                                          reinterpret_cast<u32*>(counts));
+        launch_early(make_code_kernel<false>, 65536 / CODE_WALKERS, CODE_BLOCK, CODE_SMEM, ctx->stream, T, u32(n), t.hist, u32((u64(1) << 22) / samples), t.code, t.cnt1,
+                     reinterpret_cast<u32*>(counts));
         CSA_LAUNCH_CHECK(ctx);
     }
     return CSA_OK;
@@ -1153,7 +1160,7 @@ int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bi
         CSA_TRY(shared_bytes(ctx, count_long_text_kernel, COUNT_SMEM, configured));
         count_long_text_kernel<<<148, COUNT_BLOCK, COUNT_SMEM, ctx->stream>>>(T, n, code, bits, counts);
     }
-    else count_text_kernel<128><<<unsigned(div_up(n, TILE_POSITIONS<128>)), 128, 0, ctx->stream>>>(T, n, code, bits, counts);
+    else launch_early(count_text_kernel<128>, unsigned(div_up(n, TILE_POSITIONS<128>)), 128, 0, ctx->stream, T, n, code, bits, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1181,13 +1188,16 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
 {
     const u32 over_cap = parents << b2;
     const u32* const chunks = t.chunk0 + parents;
-    if(PACKED && one_level)     // texts of one split are short
+    if constexpr(PACKED)        // texts of one split are short
     {
-        static std::atomic<bool> configured[64];
-        CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false, PACKED>, LOCAL_SMEM<512, 16>, configured));
-        local_sort_kernel<512, 16, 2, false, PACKED><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
-        CSA_LAUNCH_CHECK(ctx);
-        return CSA_OK;
+        if(one_level)
+        {
+            static std::atomic<bool> configured[64];
+            CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false, PACKED>, LOCAL_SMEM<512, 16>, configured));
+            local_sort_kernel<512, 16, 2, false, PACKED><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
+            CSA_LAUNCH_CHECK(ctx);
+            return CSA_OK;
+        }
     }
     static std::atomic<bool> configured[2][64];
     CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 8, 3, false, PACKED>, LOCAL_SMEM<512, 8>, configured[0]));
@@ -1209,7 +1219,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     const bool one_level = ps.b1 == 0;
     const int bits = one_level ? ps.b2 : ps.b1;
     if(bits > 0) CSA_TRY(launch_count_text(ctx, T, n, t.code, bits, t.cnt1));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, p, counts);
+    launch_early(parent_offsets_kernel, 1, 1024, 0, ctx->stream, t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, p, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(n) ? (launch_scatter_text<512, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA))
                           : (launch_scatter_text<128, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA)));
