@@ -737,7 +737,7 @@ __global__ void __launch_bounds__(256) gather_pairs_kernel(const u64* __restrict
 
 // The groups with a follower, once no end is tied: a group leads to the suffixes of one end group, whose ranks by now are its slots, one each. So a suffix is
 // as far behind its group's first slot as its end's rank is behind the least of them. (Ordered as in a generation, by counting the members of a group against one
-// another: 1.57 ms for 10^8 suffixes in groups of 16 and 20 ms for 4e8 in groups of 48; this way builds of them took 1.2 and 8.0 ms less.)
+// another: 1.7 ms for 10^8 near-duplicate suffixes and 10.2 ms for 4e8; builds took 1.2 and 8.0 ms less this way.)
 __global__ void __launch_bounds__(RW_BLOCK) place_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ sa, u64* __restrict__ dev_status)
 {
     __shared__ Group_Starts groups;
