@@ -296,7 +296,8 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     // Groups that lead, one symbol on, to a whole group again (refine.cu): where they hold half of the tied suffixes, the others alone go on, and they
     // take over their order at the end (near-duplicate documents: nineteen in twenty).
     u64 followed = 0;
-    u64* followed_list = nullptr;
+    u64* ends_list = nullptr;           // all ends, as they were found
+    u64 ends_found = 0;
     u32* bits = nullptr;
     if(c.small > most_by_text)
     {
@@ -318,9 +319,10 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             if(2 * u64(f.large) >= c.small)
             {
                 followed = f.large;
-                followed_list = b.other + (n - followed);
+                ends = ends_found = f.next_small;
+                ends_list = b.other + (n - ends);           // the lists that follow are no longer than half of the buffer
+                CSA_CUDA(ctx, cudaMemcpyAsync(ends_list, b.other, ends * 8, cudaMemcpyDeviceToDevice, ctx->stream));
                 std::swap(b.front, b.other);
-                ends = f.next_small;
                 CSA_TRY(b.set_count(&Build_Counts::small, f.next_small));
             }
             CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
@@ -385,7 +387,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             shared += h;
             if(shared > 2 * n + 2 * depth) return csa_fail(ctx, CSA_E_DEVICE, "build: doubling did not terminate");
         }
-        if(followed) CSA_TRY(launch_place_followed(ctx, followed_list, followed, reinterpret_cast<u32*>(b.work), bits, b.isa, b.sa));
+        if(followed) CSA_TRY(launch_place_followed(ctx, ends_list, ends_found, bits, b.isa, n, b.sa, reinterpret_cast<u64*>(b.work)));
     }
     st.generations = gen;
 

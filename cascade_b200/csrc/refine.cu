@@ -623,18 +623,18 @@ struct Split_Window
     Group_Starts groups;
     u32 sec[RW_WINDOW];
     Odd_Members odds;
-    u32 keep[RW_WINDOW / 32], pass[RW_WINDOW / 32];             // ends, and groups with a follower: a bit per slot
-    u32 keep_before[RW_WINDOW / 32], pass_before[RW_WINDOW / 32];
-    u32 keep_slot, pass_slot;
+    u32 keep[RW_WINDOW / 32], keep_before[RW_WINDOW / 32];      // ends: a bit per slot
+    u32 keep_slot, passed;
 };
 
-// The list's groups into ends (front of next, counts->next_small) and groups with a follower (back of next, counts->large), whose positions' bits are set.
+// The ends among the list's groups to next (counts->next_small); the bits of the positions whose groups have a follower (counts->large) are set.
 // secs: what launch_gather_ranks gives one symbol on.
-__global__ void __launch_bounds__(RW_BLOCK, 4) split_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, const u32* __restrict__ sa, const u64 n,
+__global__ void __launch_bounds__(RW_BLOCK, 4) split_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, const u32* __restrict__ sa,
                                                                     u32* __restrict__ bits, u64* __restrict__ next, Build_Counts* __restrict__ counts)
 {
     __shared__ Split_Window w;
     const u32 tid = threadIdx.x;
+    if(tid == 0) w.passed = 0;          // before load_entries' barriers
     const u64 first = u64(blockIdx.x) * RW_TILE;
     u32 sec[RW_ITEMS];
     #pragma unroll
@@ -665,36 +665,34 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) split_followed_kernel(const u64* 
         bool followed = false;
         if(s != NO_GROUP && ((odd_before(w.odds, e) ^ odd_before(w.odds, s)) & 0xFFFFu) == 0 && u32(entry[i] >> 32) * 2654435761u >> FORCED_END != 0)
             followed = sec[i] >= MAX_SMALL_H && sa[sec[i] - u32(MAX_SMALL_H)] == e - s;         // the same rank for all of them: a group of several
+        if(followed)
+        {
+            const u32 x = u32(entry[i]);
+            atomicOr(bits + (x >> 5), 1u << (x & 31));
+        }
         const u32 f = __ballot_sync(0xFFFFFFFFu, followed), k = __ballot_sync(0xFFFFFFFFu, s != NO_GROUP && !followed);
-        if(lane_id() == 0) { w.pass[i * (RW_BLOCK / 32) + (tid >> 5)] = f; w.keep[i * (RW_BLOCK / 32) + (tid >> 5)] = k; }
+        if(lane_id() == 0)
+        {
+            if(f) atomicAdd(&w.passed, u32(__popc(f)));
+            w.keep[i * (RW_BLOCK / 32) + (tid >> 5)] = k;
+        }
     }
     __syncthreads();
     static_assert(RW_WINDOW / 32 == 64, "two words a lane");
-    if(tid < 64)
+    if(tid < 32)
     {
-        const u32* const from = tid < 32 ? w.keep : w.pass;
-        u32* const to = tid < 32 ? w.keep_before : w.pass_before;
-        const u32 k = 2 * lane_id(), a = __popc(from[k]), b = __popc(from[k + 1]), inc = warp_sum(a + b);
-        to[k] = inc - a - b;
-        to[k + 1] = inc - b;
-        if(lane_id() == 31 && inc)
-        {
-            if(tid < 32) w.keep_slot = atomicAdd(&counts->next_small, inc);
-            else w.pass_slot = atomicAdd(&counts->large, inc);
-        }
+        const u32 k = 2 * lane_id(), a = __popc(w.keep[k]), b = __popc(w.keep[k + 1]), inc = warp_sum(a + b);
+        w.keep_before[k] = inc - a - b;
+        w.keep_before[k + 1] = inc - b;
+        if(lane_id() == 31 && inc) w.keep_slot = atomicAdd(&counts->next_small, inc);
     }
+    else if(tid == 32 && w.passed) atomicAdd(&counts->large, w.passed);
     __syncthreads();
     #pragma unroll
     for(int i = 0; i < RW_ITEMS; ++i)
     {
         const u32 j = tid + i * RW_BLOCK, word = j >> 5, below = (1u << (j & 31)) - 1;
         if(w.keep[word] >> (j & 31) & 1u) next[u64(w.keep_slot) + w.keep_before[word] + __popc(w.keep[word] & below)] = entry[i];
-        else if(w.pass[word] >> (j & 31) & 1u)
-        {
-            next[n - 1 - (u64(w.pass_slot) + w.pass_before[word] + __popc(w.pass[word] & below))] = entry[i];
-            const u32 x = u32(entry[i]);
-            atomicOr(bits + (x >> 5), 1u << (x & 31));
-        }
     }
 }
 
@@ -736,64 +734,18 @@ __global__ void __launch_bounds__(256) gather_pairs_kernel(const u64* __restrict
 }
 
 // The groups with a follower, once no end is tied: a group leads to the suffixes of one end group, whose ranks by now are its slots, one each. So a suffix is
-// as far behind its group's first slot as its end's rank is behind the least of them. (Ordered as in a generation, by counting the members of a group against one
-// another: 1.7 ms for 10^8 near-duplicate suffixes and 10.2 ms for 4e8; builds took 1.2 and 8.0 ms less this way.)
-__global__ void __launch_bounds__(RW_BLOCK) place_followed_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ secs, u32* __restrict__ sa, u64* __restrict__ dev_status)
+// as far behind its group's first slot as its end is behind its own. That distance takes the place of the end's rank here (ends: the list of them all as it
+// was before any was told apart); the inverse array is then gone through in the text's order, where a suffix and its end are neighbours (Source::FOLLOWED
+// below), and sorted into the slots. (With two random reads a suffix in the order of the slots, and the least rank of a group subtracted: 12.9 ms
+// for 4e8 near-duplicate suffixes, builds 66.3 ms and 60.5 this way; of 1e8 12.3 and 11.6, of 1e7 to 3e7 the same or less.)
+__global__ void __launch_bounds__(256) ends_behind_kernel(const u64* __restrict__ ends, const u64 count, u32* __restrict__ isa, u64* __restrict__ dev_status)
 {
-    __shared__ Group_Starts groups;
-    __shared__ u32 least[RW_WINDOW];            // by first slot
-    const u32 tid = threadIdx.x;
-    const u64 first = u64(blockIdx.x) * RW_TILE;
-    u32 sec[RW_ITEMS];
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        const u32 j = tid + i * RW_BLOCK;
-        sec[i] = first + j < count ? __ldcs(secs + first + j) : 0;
-        least[j] = 0xFFFFFFFFu;
-    }
-    u64 entry[RW_ITEMS];
-    load_entries(groups, list, count, first, entry);
-    u32 group[RW_ITEMS];        // first slot | end << 16
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        u32 s, e;
-        find_group(groups, entry[i], i, s, e);
-        group[i] = s | e << 16;
-        if(s != NO_GROUP) atomicMin(&least[s], sec[i]);
-    }
-    __syncthreads();
-    #pragma unroll
-    for(int i = 0; i < RW_ITEMS; ++i)
-    {
-        const u32 s = group[i] & 0xFFFFu, e = group[i] >> 16;
-        if(s == NO_GROUP) continue;
-        const u32 behind = sec[i] - least[s];
-        if(behind < e - s) sa[u32(entry[i] >> 32) + behind] = u32(entry[i]);
-        else atomicOr(reinterpret_cast<unsigned long long*>(dev_status), (unsigned long long)CSA_ST_UNSERVED);
-    }
-}
-
-// secs[i]: the rank of the end that the i-th entry's group leads to.
-__global__ void __launch_bounds__(256) gather_ends_kernel(const u64* __restrict__ list, const u64 count, const u32* __restrict__ isa, const u64* __restrict__ bits, u32* __restrict__ secs)
-{
-    const u64 first = u64(blockIdx.x) * (256 * GATHER_UNROLL) + threadIdx.x;
-    u32 v[GATHER_UNROLL];
-    #pragma unroll
-    for(int i = 0; i < GATHER_UNROLL; ++i)
-    {
-        const u64 k = first + u64(i) * 256;
-        if(k >= count) continue;
-        const u64 x = u32(__ldcs(list + k));
-        v[i] = __ldg(isa + x + followers(bits, x));
-    }
-    #pragma unroll
-    for(int i = 0; i < GATHER_UNROLL; ++i)
-    {
-        const u64 k = first + u64(i) * 256;
-        if(k < count) __stcs(secs + k, v[i]);
-    }
+    const u64 k = u64(blockIdx.x) * 256 + threadIdx.x;
+    if(k >= count) return;
+    const u64 e = __ldcs(ends + k);
+    const u32 behind = isa[u32(e)] - u32(e >> 32);
+    isa[u32(e)] = behind;
+    if(behind >= SMALL_GROUP) atomicOr(reinterpret_cast<unsigned long long*>(dev_status), (unsigned long long)CSA_ST_UNSERVED);
 }
 
 // ---- lists of groups of any size ----------------------------------------------------------------------------------------------
@@ -961,10 +913,22 @@ __global__ void __launch_bounds__(256) large_depth_kernel(const u64* __restrict_
 // together hold every position once, so bucket b starts at entry b << low_bits and nothing is counted first.
 constexpr int MI_BLOCK = 256, MI_ITEMS = 16, MI_TILE = MI_BLOCK * MI_ITEMS;
 
-template <bool FROM_SA>
-__device__ __forceinline__ bool inverse_record(const u32* __restrict__ sa, const u64* __restrict__ list, const u64 k, u64& out)
+// Where the pairs come from: the array (`words`), a list, or, the other way round, the inverse array as ends_behind_kernel left it with a bit for every
+// position whose group has a follower (`list`): slots and their positions then.
+enum class Source { ARRAY, LIST, FOLLOWED };
+
+template <Source FROM>
+__device__ __forceinline__ bool inverse_record(const u32* __restrict__ sa, const u64* __restrict__ list, const u64 k, const u64 n, u64& out)
 {
-    if(FROM_SA)
+    if(FROM == Source::FOLLOWED)
+    {
+        const u32 row = followers(list, k);
+        if(row == 0) return false;
+        const u64 slot = u64(__ldg(sa + k)) + __ldg(sa + k + row);
+        out = (slot << 32) | u32(k);
+        return slot < n;
+    }
+    if(FROM == Source::ARRAY)
     {
         const u32 x = __ldcs(sa + k);
         out = (u64(x) << 32) | u32(k);
@@ -975,7 +939,7 @@ __device__ __forceinline__ bool inverse_record(const u32* __restrict__ sa, const
     return true;
 }
 
-template <bool FROM_SA>
+template <Source FROM>
 __global__ void __launch_bounds__(MI_BLOCK) bucket_ranks_kernel(const u32* __restrict__ sa, const u64* __restrict__ list, const u64 count, const int low_bits,
                                                                u64* __restrict__ out, const u64 out_count, u64* __restrict__ cursor, u64* __restrict__ dev_status)
 {
@@ -994,7 +958,7 @@ __global__ void __launch_bounds__(MI_BLOCK) bucket_ranks_kernel(const u32* __res
     {
         const u64 j = tile_first + tid + k * MI_BLOCK;
         r[k] = 0xFFFFFFFFu;
-        if(j < count && inverse_record<FROM_SA>(sa, list, j, u[k])) r[k] = 0;
+        if(j < count && inverse_record<FROM>(sa, list, j, out_count, u[k])) r[k] = 0;
     }
     #pragma unroll
     for(int k = 0; k < MI_ITEMS; ++k)
@@ -1024,12 +988,12 @@ __global__ void __launch_bounds__(MI_BLOCK) bucket_ranks_kernel(const u32* __res
     }
 }
 
-template <bool FROM_SA>
-__global__ void __launch_bounds__(256) scatter_ranks_kernel(const u32* __restrict__ sa, const u64* __restrict__ list, const u64 count, u32* __restrict__ isa)
+template <Source FROM>
+__global__ void __launch_bounds__(256) scatter_ranks_kernel(const u32* __restrict__ sa, const u64* __restrict__ list, const u64 count, const u64 n, u32* __restrict__ to)
 {
     const u64 k = u64(blockIdx.x) * 256 + threadIdx.x;
     u64 u;
-    if(k < count && inverse_record<FROM_SA>(sa, list, k, u)) isa[u >> 32] = u32(u);
+    if(k < count && inverse_record<FROM>(sa, list, k, n, u)) to[u >> 32] = u32(u);
 }
 
 __global__ void __launch_bounds__(256) apply_ranks_kernel(const u64* __restrict__ upd, const u64 count, u32* __restrict__ isa)
@@ -1044,15 +1008,30 @@ __global__ void __launch_bounds__(256) apply_ranks_kernel(const u64* __restrict_
     else if(first < count) isa[upd[first] >> 32] = u32(upd[first]);
 }
 
-template <bool FROM_SA>
-int ranks_from(csa_ctx* ctx, const u32* sa, const u64* list, u64 count, u64 n, u32* isa, u64* updates, u64* cursor)
+// The same for buckets that are not full: cursor[b] entries in bucket b.
+__global__ void __launch_bounds__(256) apply_slots_kernel(const u64* __restrict__ upd, const u64 n, const int low_bits, const u64* __restrict__ cursor, u32* __restrict__ sa)
+{
+    const u64 first = (u64(blockIdx.x) * 256 + threadIdx.x) * 2;
+    if(first >= n) return;
+    const u64 filled = __ldg(cursor + (first >> low_bits)), at = first & ((u64(1) << low_bits) - 1);       // a pair lies in one bucket
+    if(at + 1 < filled && first + 1 < n)
+    {
+        const ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2*>(upd + first));
+        sa[v.x >> 32] = u32(v.x);
+        sa[v.y >> 32] = u32(v.y);
+    }
+    else if(at < filled) { const u64 v = upd[first]; sa[v >> 32] = u32(v); }
+}
+
+template <Source FROM>
+int ranks_from(csa_ctx* ctx, const u32* sa, const u64* list, u64 count, u64 n, u32* to, u64* updates, u64* cursor)
 {
     if(count == 0) return CSA_OK;
     const int bits = bits_for(n - 1);
     if(bits <= 24)        // the inverse array stays in L2: straight scatters
-        scatter_ranks_kernel<FROM_SA><<<unsigned(div_up(count, 256)), 256, 0, ctx->stream>>>(sa, list, count, isa);
+        scatter_ranks_kernel<FROM><<<unsigned(div_up(count, 256)), 256, 0, ctx->stream>>>(sa, list, count, n, to);
     else
-        bucket_ranks_kernel<FROM_SA><<<unsigned(div_up(count, MI_TILE)), MI_BLOCK, 0, ctx->stream>>>(sa, list, count, bits - 8, updates, n, cursor, ctx->d_status);
+        bucket_ranks_kernel<FROM><<<unsigned(div_up(count, MI_TILE)), MI_BLOCK, 0, ctx->stream>>>(sa, list, count, bits - 8, updates, n, cursor, ctx->d_status);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1105,7 +1084,7 @@ int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* i
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(launch_gather_ranks(ctx, list, count, isa, n, 1, secs));
     CSA_CUDA(ctx, cudaMemsetAsync(bits, 0, follower_bits_bytes(n), ctx->stream));
-    split_followed_kernel<<<tiles, RW_BLOCK, 0, ctx->stream>>>(list, count, secs, sa, n, bits, next, counts);
+    split_followed_kernel<<<tiles, RW_BLOCK, 0, ctx->stream>>>(list, count, secs, sa, bits, next, counts);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1120,13 +1099,21 @@ int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* sec
     return CSA_OK;
 }
 
-int launch_place_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, const u32* isa, u32* sa)
+int launch_place_followed(csa_ctx* ctx, const u64* ends, u64 count, const u32* bits, u32* isa, u64 n, u32* sa, u64* updates)
 {
-    if(count == 0) return CSA_OK;
-    gather_ends_kernel<<<unsigned(div_up(count, 256 * GATHER_UNROLL)), 256, 0, ctx->stream>>>(list, count, isa, reinterpret_cast<const u64*>(bits), secs);
-    CSA_LAUNCH_CHECK(ctx);
-    place_followed_kernel<<<unsigned(div_up(count, RW_TILE)), RW_BLOCK, 0, ctx->stream>>>(list, count, secs, sa, ctx->d_status);
-    CSA_LAUNCH_CHECK(ctx);
+    u64* const cursor = updates + n;
+    if(count)
+    {
+        ends_behind_kernel<<<unsigned(div_up(count, 256)), 256, 0, ctx->stream>>>(ends, count, isa, ctx->d_status);
+        CSA_LAUNCH_CHECK(ctx);
+    }
+    CSA_CUDA(ctx, cudaMemsetAsync(cursor, 0, 256 * 8, ctx->stream));
+    CSA_TRY(ranks_from<Source::FOLLOWED>(ctx, isa, reinterpret_cast<const u64*>(bits), n, n, sa, updates, cursor));
+    if(bits_for(n - 1) > 24)
+    {
+        apply_slots_kernel<<<unsigned(div_up(div_up(n, 2), 256)), 256, 0, ctx->stream>>>(updates, n, bits_for(n - 1) - 8, cursor, sa);
+        CSA_LAUNCH_CHECK(ctx);
+    }
     return CSA_OK;
 }
 
@@ -1171,9 +1158,9 @@ int launch_make_inverse(csa_ctx* ctx, const u32* sa, u64 n, const u64* small_lis
 {
     u64* const cursor = updates + n;
     CSA_CUDA(ctx, cudaMemsetAsync(cursor, 0, 256 * 8, ctx->stream));
-    CSA_TRY(ranks_from<true>(ctx, sa, nullptr, n, n, isa, updates, cursor));
-    CSA_TRY(ranks_from<false>(ctx, nullptr, small_list, small, n, isa, updates, cursor));
-    CSA_TRY(ranks_from<false>(ctx, nullptr, large_list, large, n, isa, updates, cursor));
+    CSA_TRY(ranks_from<Source::ARRAY>(ctx, sa, nullptr, n, n, isa, updates, cursor));
+    CSA_TRY(ranks_from<Source::LIST>(ctx, nullptr, small_list, small, n, isa, updates, cursor));
+    CSA_TRY(ranks_from<Source::LIST>(ctx, nullptr, large_list, large, n, isa, updates, cursor));
     if(bits_for(n - 1) > 24)
     {
         apply_ranks_kernel<<<unsigned(div_up(div_up(n, 2), 256)), 256, 0, ctx->stream>>>(updates, n, isa);

@@ -28,15 +28,16 @@ int launch_gather_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* isa
 // counts->next_small entries that are there.
 int launch_refine_by_ranks(csa_ctx* ctx, const u64* list, u64 count, const u32* secs, u32* isa, u32* sa, u64* next, Build_Counts* counts);
 
-// Groups whose suffixes lead, one symbol on, to a whole group again (refine.cu). The list's groups are split into those and the ends: ends to the front of next
-// (counts->next_small), the others to its back (counts->large); both counters start from 0, next holds n entries. A group shares a symbol at least. bits: follower_bits_bytes(n), a
-// bit per position; secs: a word per entry; the first slot of every group in sa receives its size. All groups are small and were ranked by isa.
+// Groups whose suffixes lead, one symbol on, to a whole group again (refine.cu). The list's other groups, the ends, go to next
+// (counts->next_small); counts->large receives the number of suffixes in groups that have a follower. Both counters start from 0. A group shares a symbol at least.
+// bits: follower_bits_bytes(n), a bit per position, set for those suffixes; secs: a word per entry; the first slot of every group in sa receives its size. All groups are small and were ranked by isa.
 inline size_t follower_bits_bytes(u64 n) { return align_up256((n / 64 + 2) * 8); }
 int launch_split_followed(csa_ctx* ctx, const u64* list, u64 count, const u32* isa, u64 n, u32* secs, u32* sa, u32* bits, u64* next, Build_Counts* counts);
 // One generation of the ends, h symbols on (they share as many): as launch_gather_ranks and launch_refine_by_ranks. secs: a double word per entry.
 int launch_refine_ends(csa_ctx* ctx, const u64* list, u64 count, u64 h, u64* secs, const u32* bits, u32* isa, u64 n, u32* sa, u64* next, Build_Counts* counts);
-// The others, once no end is tied: every suffix goes to its slot of sa.
-int launch_place_followed(csa_ctx* ctx, const u64* list, u64 count, u32* secs, const u32* bits, const u32* isa, u32* sa);
+// The others, once no end is tied: every suffix goes to its slot of sa. ends: the list of ends, `count` entries, as launch_split_followed gave it; isa is not the
+// inverse array any more afterwards. updates: as below.
+int launch_place_followed(csa_ctx* ctx, const u64* ends, u64 count, const u32* bits, u32* isa, u64 n, u32* sa, u64* updates);
 
 // A list of groups of any size (heads, positions; *count_dev entries, at most `most`), group by group: how many of its entries are in small groups
 // (counts->now_small) and where each tile's go; counts->next_small and counts->large are advanced by the two kinds. scratch: 2 words per

@@ -49,3 +49,14 @@ def test_documents_in_another_order_every_time(ctx):
     for k in range(0, len(T) - 40, 19000):
         T[k:k + 30] = docs[0][1:31] if len(docs[0]) > 31 else 9
     _check(ctx, T)
+
+
+@pytest.mark.parametrize("n", [(1 << 24) + 1, (1 << 25) + 12345])
+def test_slots_sorted_into_buckets(ctx, n):
+    """Above 2^24 suffixes the others' slots go through buckets by their top bits: a last bucket of one slot, and one that is partly there."""
+    rng = np.random.default_rng(n)
+    docs = rng.integers(1, 60000, (3000, 400)).astype(np.uint16)
+    T = docs[rng.integers(0, 3000, n // 400 + 1)].reshape(-1)[:n]
+    hit = rng.random(n) < 1e-3
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    _check(ctx, T)
