@@ -53,6 +53,11 @@ constexpr u64 PACKED_MAX = u64(1) << 25;
 // Tied suffixes from which on (and a quarter of the text) groups are looked through for followers. Below, a generation costs its launches: near-duplicates of
 // 10^6 tokens took 657 us without and 740 with it.
 constexpr u64 FOLLOWED_MIN = u64(1) << 22;
+// Large groups are ranked ahead of the small ones where they hold no more than one in LARGE_SHARE of their suffixes, as most of them share a few frequent symbols
+// only: every step tells depth0 symbols or more, and is the last if it leaves more than three quarters.
+// 1e9 near-duplicate suffixes with 1849 of them in large groups: 365 ms with the large groups left to the generations, so that nothing followed, 252 this way.
+constexpr u64 LARGE_SHARE = 8;
+constexpr u32 LARGE_STEPS = 12;
 
 int set_build_count(csa_ctx* ctx, u32* at, u32 value)
 {
@@ -122,6 +127,12 @@ struct Build
         void* p = nullptr;
         CSA_TRY(csa_aux(ctx, bytes, &p));
         return sort_oversize_children(ctx, ps, tab, c, n, front, other, sa, counts, oversize_buffers(p, few));
+    }
+
+    int check_large_depth(const Build_Counts& c, u64 depth0)
+    {
+        if(c.large_depth < depth0 || c.large_depth > u64(ps.key_bits)) return csa_fail(ctx, CSA_E_DEVICE, "build: the large groups' depth is out of range");
+        return CSA_OK;
     }
 
     // The same of ends (refine.cu).
@@ -293,46 +304,73 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     if(debug) std::fprintf(stderr, "[csa] n=%llu key bits %d: tied after generation 0: %u in small groups, %u in large ones\n", n, b.ps.key_bits, c.small, c.large);
     u32 gen = 0;
     if(st.active_after_gen0) st.active_per_gen[gen++] = st.active_after_gen0;
+    // The few large groups beside many small ones are ranked first, if some steps do it (LARGE_STEPS); a group that follows another is small.
     // Groups that lead, one symbol on, to a whole group again (refine.cu): where they hold half of the tied suffixes, the others alone go on, and they
     // take over their order at the end (near-duplicate documents: nineteen in twenty).
     u64 followed = 0;
     u64* ends_list = nullptr;           // all ends, as they were found
     u64 ends_found = 0;
     u32* bits = nullptr;
+    u64 large_shared = 0;               // symbols that the large groups' suffixes share, once that has been found out
     if(c.small > most_by_text)
     {
         done = false;
-        u64 ends = c.small;
-        if(!c.large)
+        b.small = c.small;
+        b.large = c.large;
+        if(c.large <= c.small / LARGE_SHARE)
         {
             CSA_TRY(b.more_memory());
             if(!words) CSA_TRY(launch_unpack_sa40(ctx, sa40, n, b.sa));
             words = b.sa;
-            CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, c.small, nullptr, 0, b.isa, reinterpret_cast<u64*>(b.work)));
+            CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));
             b.ranked = true;
+            if(b.large)
+            {
+                CSA_TRY(launch_large_depth(ctx, b.large_list(b.front), b.large, T, n, b.tab.code, b.ps.key_bits, b.counts));
+                CSA_TRY(b.read_counts(c));
+                CSA_TRY(b.check_large_depth(c, depth0));
+                large_shared = c.large_depth;
+            }
+            // Whatever the ranks tell apart: the small groups' suffixes share depth0 symbols at least.
+            for(u32 step = 0; step < LARGE_STEPS && b.large; ++step)
+            {
+                const u64 before = b.large;
+                if(gen < 48) st.active_per_gen[gen] = b.small + b.large;
+                ++gen;
+                CSA_TRY(b.generation(large_shared, b.small));
+                if(debug) std::fprintf(stderr, "[csa] large groups, h=%llu: %llu -> %llu\n", large_shared, before, b.large);
+                large_shared += depth0;
+                if(b.large > before - before / 4) break;
+            }
+        }
+        u64 ends = b.small;
+        if(b.ranked && !b.large)
+        {
+            CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
             bits = reinterpret_cast<u32*>(b.work + (b.L.work - follower_bits_bytes(n)) / 256 * 256);
-            CSA_TRY(launch_split_followed(ctx, b.front, c.small, b.isa, n, reinterpret_cast<u32*>(b.work), b.sa, bits, b.other, b.counts));
+            CSA_TRY(launch_split_followed(ctx, b.front, b.small, b.isa, n, reinterpret_cast<u32*>(b.work), b.sa, bits, b.other, b.counts));
             Build_Counts f;
             CSA_TRY(b.read_counts(f));
-            if(u64(f.next_small) + f.large != c.small) return csa_fail(ctx, CSA_E_DEVICE, "build: the groups with and without a follower do not add up");
-            if(debug) std::fprintf(stderr, "[csa] %u of %u have a follower\n", f.large, c.small);
-            if(2 * u64(f.large) >= c.small)
+            if(u64(f.next_small) + f.large != b.small) return csa_fail(ctx, CSA_E_DEVICE, "build: the groups with and without a follower do not add up");
+            if(debug) std::fprintf(stderr, "[csa] %u of %llu have a follower\n", f.large, b.small);
+            if(2 * u64(f.large) >= b.small)
             {
                 followed = f.large;
                 ends = ends_found = f.next_small;
                 ends_list = b.other + (n - ends);           // the lists that follow are no longer than half of the buffer
                 CSA_CUDA(ctx, cudaMemcpyAsync(ends_list, b.other, ends * 8, cudaMemcpyDeviceToDevice, ctx->stream));
                 std::swap(b.front, b.other);
-                CSA_TRY(b.set_count(&Build_Counts::small, f.next_small));
             }
-            CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
-            CSA_TRY(b.set_count(&Build_Counts::large, 0));
         }
+        CSA_TRY(b.set_count(&Build_Counts::small, u32(ends)));
+        CSA_TRY(b.set_count(&Build_Counts::next_small, 0));
+        CSA_TRY(b.set_count(&Build_Counts::large, u32(b.large)));
         CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, b.ranks(), b.counts, ends, n));
         CSA_TRY(b.read_counts(c));
+        c.large = u32(b.large);
     }
     b.large = c.large;
-    if(b.large) CSA_CUDA(ctx, cudaMemcpyAsync(b.large_list(b.other), b.large_list(b.front), b.large * 8, cudaMemcpyDeviceToDevice, ctx->stream));
+    if(b.large && !b.in_arrays) CSA_CUDA(ctx, cudaMemcpyAsync(b.large_list(b.other), b.large_list(b.front), b.large * 8, cudaMemcpyDeviceToDevice, ctx->stream));
     std::swap(b.front, b.other);
     b.small = c.next_small;
     // Few suffixes left, in small groups: reading on in the text costs less than an inverse array of the whole text.
@@ -366,10 +404,14 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
             // A large group was not compared in the text: it shares the whole symbols of generation 0's key. Frequent symbols, of which large groups
             // are made, have short code words, so that is more than what any key holds (depth0 = 1): one symbol repeated 2^24 times starts at 25
             // and takes 22 generations instead of 26.
-            CSA_TRY(launch_large_depth(ctx, b.large_list(b.front), b.large, T, n, b.tab.code, b.ps.key_bits, b.counts));
-            CSA_TRY(b.read_counts(c));
-            if(c.large_depth < depth0 || c.large_depth > u64(b.ps.key_bits)) return csa_fail(ctx, CSA_E_DEVICE, "build: the large groups' depth is out of range");
-            shared = std::min<u64>(c.large_depth, depth);
+            if(!large_shared)
+            {
+                CSA_TRY(launch_large_depth(ctx, b.large_list(b.front), b.large, T, n, b.tab.code, b.ps.key_bits, b.counts));
+                CSA_TRY(b.read_counts(c));
+                CSA_TRY(b.check_large_depth(c, depth0));
+                large_shared = c.large_depth;
+            }
+            shared = std::min(large_shared, depth);
         }
         // Ranks tell `shared` symbols from any step of up to as many: doubling takes the longest step. Above 2^31 suffixes a step may be too long for
         // a sort key of two ranks (n - 1 + h has to fit beside bits_for(n - 1) bits in 64); steps of the longest that fits go on from there.

@@ -38,7 +38,7 @@ def test_a_text_that_occurs_many_times(ctx, copies, mutate, cut):
 
 
 def test_documents_in_another_order_every_time(ctx):
-    """Near-duplicate documents with separators, and some passages that stand in the text too often for a small group (then no group is looked at)."""
+    """Near-duplicate documents with separators, and some passages that stand in the text too often for a small group."""
     rng = np.random.default_rng(2)
     docs = [np.concatenate([[65535], np.minimum(rng.zipf(1.2, int(rng.integers(20, 4000))), 50000)]).astype(np.uint16) for _ in range(60)]
     T = np.concatenate([docs[int(k)] for k in rng.integers(0, 60, 3000)])[:5_500_001]
@@ -59,4 +59,16 @@ def test_slots_sorted_into_buckets(ctx, n):
     T = docs[rng.integers(0, 3000, n // 400 + 1)].reshape(-1)[:n]
     hit = rng.random(n) < 1e-3
     T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    _check(ctx, T)
+
+
+@pytest.mark.parametrize("length", [6, 200])
+def test_a_few_large_groups_beside_many_small_ones(ctx, length):
+    """A passage that stands in the text 400 times: its groups are ranked first where that takes a few steps, else they stay large."""
+    rng = np.random.default_rng(length)
+    T = np.tile(rng.integers(1, 60000, 130_000).astype(np.uint16), 40)
+    hit = rng.random(len(T)) < 1e-3
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    for k in rng.integers(0, len(T) - length, 400):
+        T[k:k + length] = np.arange(1, length + 1)
     _check(ctx, T)
