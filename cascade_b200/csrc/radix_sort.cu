@@ -764,6 +764,10 @@ const u64* sort_workspace_histograms(void* workspace, size_t workspace_bytes, u6
     return cv.take<u64>(u64(8) * RADIX);
 }
 
+// Words of the buckets' starts. More than BUCKET_MAX_TOTAL records have none, but a workspace for them serves shorter lists, too: callers size one for the
+// longest of their lists, so the size never falls as n grows.
+static size_t bucket_starts(const u64 n) { return (size_t(1) << bucket_sort_bits(n < BUCKET_MAX_TOTAL ? n : BUCKET_MAX_TOTAL)) + 1; }
+
 size_t csa_sort_workspace_bytes(uint64_t n)
 {
     const u64 portions = n == 0 ? 1 : div_up(n, PORTION);
@@ -772,7 +776,7 @@ size_t csa_sort_workspace_bytes(uint64_t n)
          + 256                                         // tile counter
          + size_t(8) * RADIX * 8 + 256                 // histograms
          + size_t(portions + 1) * 8 * RADIX * 8 + 256  // digit bases of every launch
-         + (n <= BUCKET_MAX_TOTAL ? align_up256(((size_t(1) << bucket_sort_bits(n)) + 1) * 4) : 0)     // starts of the buckets
+         + align_up256(bucket_starts(n) * 4)           // starts of the buckets
          + 4096;
 }
 
@@ -902,7 +906,7 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
     u32* status = cv.take<u32>(tiles_max * RADIX);
     u64* hist = cv.take<u64>(u64(8) * RADIX);
     u64* base = cv.take<u64>(u64(portions + 1) * 8 * RADIX);
-    u32* starts = n <= BUCKET_MAX_TOTAL ? cv.take<u32>((u64(1) << bucket_sort_bits(n)) + 1) : nullptr;
+    u32* starts = cv.take<u32>(bucket_starts(n));
     if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "csa_sort_pairs: workspace too small");
 
     if(!ctx->ties_in_any_order && portions == 1)

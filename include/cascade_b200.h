@@ -65,7 +65,7 @@ const char* csa_version(void);
 
 /* ---- LSD radix sort (replaces the cub::DeviceRadixSort::SortPairs calls of src/GPU_SACA.cu:1175,1203,1783,1849) */
 
-/* Bytes of workspace that csa_sort_pairs needs for n records. */
+/* Bytes of workspace that csa_sort_pairs needs for n records or fewer: it never falls as n grows. */
 size_t csa_sort_workspace_bytes(uint64_t n);
 /* Stable radix sort of n (64-bit key, value) records on key bits [begin_bit, end_bit), least significant digit first, 8 bits per pass,
  * each pass one sweep over the records; up to 2^26 records whose top bits are evenly spread are split by those alone and finished in
