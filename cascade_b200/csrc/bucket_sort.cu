@@ -1,8 +1,10 @@
 // The stable sort of csa_sort_pairs by its top bits first, for keys whose top bits are evenly spread: the records are split into buckets
-// of about a thousand by the top 8 to 15 sorted bits with one or two of radix_sort.cu's digit passes (stable, low digit first), and every
+// of about a thousand by the top 3 to 15 sorted bits with one or two of radix_sort.cu's digit passes (stable, low digit first), and every
 // bucket is then finished inside one block. A record moves two or three times, where a pass per 8 bits moves it up to eight
-// times (31.25 M 64-bit keys with 4-byte values, whole calls: 2.22 ms, this way 1.02 ms; 10^6: 253 us, 134 us; 1000, in one block: 174 us, 63 us). Nothing is estimated: the buckets are counted
-// exactly before anything moves, and keys with a bucket that no block holds go through all their digit passes as before.
+// times (31.25 M 64-bit keys with 4-byte values, whole calls: 2.20 ms, this way 0.94 ms; 10^6: 217 us, 94 us; 1000, in one block: 140 us, 24 us). The buckets are counted
+// exactly before anything moves, and keys for which the digit passes are the better way go through those: where a bucket fits no block, and where so few digits differ
+// that most passes are skipped. (31.25 M records by digit passes alone and with the look at the keys before: all equal 97 and 99 us, 16 bits at the top 620 and 630, 20 at the bottom
+// 864 and 876, one key in half of the places 2067 and 2089. By buckets after all, but inside them by digits as a key stands a hundred times: 1979 and 1727.)
 // A list that fits one block at all is a single bucket and takes one launch.
 #include "common.cuh"
 #include "sort.cuh"
@@ -17,13 +19,56 @@ namespace
 
 constexpr int COUNT_BLOCK = 1024, COUNT_UNROLL = 4;
 
-// One read of the keys; a block counts in shared memory (32 bits a counter, at most 128 KB, as many blocks as SMs). Bound by the read.
-__global__ void __launch_bounds__(COUNT_BLOCK) bucket_counts_kernel(const u64* __restrict__ keys, const u64 n, const int shift, const int bits, u32* __restrict__ counts)
+// Of more records than this every block looks at the same COUNT_BLOCK of them first, spread over the list (2 us): where those say that the keys are not
+// for buckets, the rest is not counted. (31.25 M equal keys: 97 us by skipped digit passes alone, 178 with all of them counted first.)
+constexpr u64 LOOKED_AT_FIRST = u64(1) << 21;
+
+// Digits of 8 bits from begin_bit on in which keys differ: the digit passes that are not skipped. differ: bits in which any two keys do.
+__device__ __forceinline__ int digits_that_differ(const u64 differ, const int begin_bit, const int end_bit)
 {
+    int digits = 0;
+    for(int shift = begin_bit; shift < end_bit; shift += 8)
+        digits += (differ >> shift & ((1ull << min(8, end_bit - shift)) - 1)) != 0;
+    return digits;
+}
+
+// One read of the keys; a block counts in shared memory (32 bits a counter, at most 128 KB, as many blocks as SMs). Bound by the read.
+// found->differ: bits in which keys differ; found->uneven: the counts are not complete, the keys go through the digit passes.
+__global__ void __launch_bounds__(COUNT_BLOCK) bucket_counts_kernel(const u64* __restrict__ keys, const u64 n, const int begin_bit, const int end_bit, const int bits,
+                                                                   const int least_digits, u32* __restrict__ counts, Bucket_Findings* __restrict__ found)
+{
+    let_next_in();
     extern __shared__ u32 cnt[];
+    __shared__ u32 s_differ[2];
+    const int shift = end_bit - bits;
     const u32 buckets = 1u << bits, mask = buckets - 1;
     for(u32 i = threadIdx.x; i < buckets; i += COUNT_BLOCK) cnt[i] = 0;
+    if(threadIdx.x < 2) s_differ[threadIdx.x] = 0;
+    const u64 k0 = keys[0];
+    u64 differ = 0;
+    auto block_differ = [&]()
+    {
+        const u32 lo = __reduce_or_sync(0xFFFFFFFFu, u32(differ)), hi = __reduce_or_sync(0xFFFFFFFFu, u32(differ >> 32));
+        if(lane_id() == 0) { atomicOr(&s_differ[0], lo); atomicOr(&s_differ[1], hi); }
+    };
     __syncthreads();
+    if(n > LOOKED_AT_FIRST)
+    {
+        const u64 k = keys[u64(threadIdx.x) * (n / COUNT_BLOCK)];
+        const u32 b = u32(k >> shift) & mask;
+        differ = k ^ k0;
+        block_differ();
+        // several times what a bucket that fits a block may show here, so that keys whose buckets all fit are hardly ever refused
+        const u32 most = 8 + u32(4 * BUCKET_MAX_RECORDS * COUNT_BLOCK / n);
+        const bool heavy = __syncthreads_or(atomicAdd(&cnt[b], 1u) >= most);
+        if(heavy || digits_that_differ(u64(s_differ[1]) << 32 | s_differ[0], begin_bit, end_bit) < least_digits)
+        {
+            if(blockIdx.x == 0 && threadIdx.x == 0) found->uneven = 1;
+            return;
+        }
+        cnt[b] = 0;
+        __syncthreads();
+    }
     const u64 lead = (reinterpret_cast<uintptr_t>(keys) & 8) ? 1 : 0;           // a list may start on an odd 8-byte boundary
     const u64 pairs = (n - lead) >> 1;
     const ulonglong2* const k2 = reinterpret_cast<const ulonglong2*>(keys + lead);
@@ -38,16 +83,19 @@ __global__ void __launch_bounds__(COUNT_BLOCK) bucket_counts_kernel(const u64* _
             {
                 atomicAdd(&cnt[u32(k[j].x >> shift) & mask], 1u);
                 atomicAdd(&cnt[u32(k[j].y >> shift) & mask], 1u);
+                differ |= (k[j].x ^ k0) | (k[j].y ^ k0);
             }
     }
     if(blockIdx.x == 0 && threadIdx.x == 0)
     {
-        if(lead) atomicAdd(&cnt[u32(keys[0] >> shift) & mask], 1u);
-        if((n - lead) & 1) atomicAdd(&cnt[u32(keys[n - 1] >> shift) & mask], 1u);
+        if(lead) atomicAdd(&cnt[u32(k0 >> shift) & mask], 1u);
+        if((n - lead) & 1) { atomicAdd(&cnt[u32(keys[n - 1] >> shift) & mask], 1u); differ |= keys[n - 1] ^ k0; }
     }
+    block_differ();
     __syncthreads();
     for(u32 i = threadIdx.x; i < buckets; i += COUNT_BLOCK)
         if(const u32 c = cnt[i]) atomicAdd(&counts[i], c);
+    if(threadIdx.x == 0) atomicOr(&found->differ, u64(s_differ[1]) << 32 | s_differ[0]);
 }
 
 __device__ __forceinline__ u32 warp_inclusive_sum(u32 v)
@@ -75,10 +123,15 @@ __device__ __forceinline__ u32 block_exclusive_sum(const u32 v, u32* warp_tot)
 }
 
 // One block: the counts become the buckets' starts, in place (starts[buckets] = n); the digit offsets of the one or two passes by which
-// the records get there (low digit first: low_bits of them, which may be 0, then the top bits); and the size of the largest bucket.
-__global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ counts, const u32 n, const int bits, const int low_bits, u64* __restrict__ low_base,
-                                                          u64* __restrict__ high_base, u64* __restrict__ largest)
+// the records get there (low digit first: low_bits of them, which may be 0, then the top bits); and the verdict: found->uneven where a bucket does not fit a
+// block or fewer than least_digits digits differ. verdict (pinned host memory): the largest bucket, 0 for uneven keys.
+__global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ counts, const u32 n, const int begin_bit, const int end_bit, const int bits, const int low_bits,
+                                                          const int least_digits, u64* __restrict__ low_base, u64* __restrict__ high_base, Bucket_Findings* __restrict__ found,
+                                                          u64* __restrict__ verdict)
 {
+    let_next_in();
+    wait_for_previous();
+    if(found->uneven) { if(threadIdx.x == 0) *verdict = 0; return; }
     __shared__ u32 warp_tot[32];
     __shared__ u32 low[256];
     __shared__ u32 most;
@@ -143,14 +196,20 @@ __global__ void __launch_bounds__(1024) bucket_plan_kernel(u32* __restrict__ cou
     __syncthreads();
     const u32 at = block_exclusive_sum<1024>(t < 256 ? low[t] : 0, warp_tot);
     if(low_bits && t < (1u << low_bits)) low_base[t] = at;
-    if(t == 0) { counts[buckets] = n; *largest = most; }
+    if(t == 0)
+    {
+        counts[buckets] = n;
+        const bool even = most <= BUCKET_MAX_RECORDS && digits_that_differ(found->differ, begin_bit, end_bit) >= least_digits;
+        found->uneven = even ? 0 : 1;
+        *verdict = even ? most : 0;
+    }
 }
 
 // ---- a bucket inside one block -------------------------------------------------------------------------------------------------
 
 constexpr int BUCKET_ITEMS = 8;
 template <int BLOCK> constexpr u32 BUCKET_CAP = BLOCK * BUCKET_ITEMS;
-constexpr u32 LONG_BIN = 128;       // a bin with more records is not ordered by comparing all with all
+constexpr u32 LONG_BIN = 24;       // a bin with more records is not ordered by comparing all with all
 // the staged keys; then the bins and the places before, and where those were, the values
 template <int BLOCK, typename V> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CAP<BLOCK>) * 8 + (sizeof(V) == 8 ? size_t(BUCKET_CAP<BLOCK>) * 8 : size_t(BUCKET_CAP<BLOCK>) * 4 + 32);
 
@@ -159,7 +218,9 @@ template <int BLOCK, typename V> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CA
 // bin is its next key bits, its place in the bin is what a shared-memory atomic hands out, and inside the bin it counts the keys before its own, equal ones
 // by the places they came from. So the order is the stable one whatever order the atomics took. A record stays with its thread until its place is known; keys
 // and values then go out by way of shared memory, side by side.
-// A bin of more than LONG_BIN records sends the bucket through a sorting network instead. What bounds it is the issue of instructions and barriers between
+// A bin of more than LONG_BIN records sends the bucket through stable passes by digits instead, as many as its keys differ in (8192 equal keys in one block: 120 us by a sorting
+// network, 30 this way). Even keys have no such bin. Thirty records a key, 31.25 M records, in a row and far apart: with bins of up to 40 compared 1.49 and 2.20 ms, of up to 24
+// 1.71 and 1.79; by digit passes alone 2.03 and 2.12. What bounds it is the issue of instructions and barriers between
 // dependent steps: blocks are as small as the largest bucket allows, with 8 records a thread. (31.25 M records, 16 a thread and the values
 // gathered when the places were known: 454 us, this way 389 us.)
 template <int BLOCK, int BLOCKS, typename V>
@@ -175,7 +236,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* _
     u16* const start = reinterpret_cast<u16*>(bin);
     u16* const from = reinterpret_cast<u16*>(bin + CAP / 2 + 8);    // [CAP]: the record's place in the bucket before
     V* const vals = reinterpret_cast<V*>(stage + CAP);              // [CAP], once the bins are no longer needed
-    __shared__ u32 warp_tot[BLOCK / 32];
+    __shared__ u32 warp_tot[BLOCK / 32], s_differ[2];
+    static_assert(BLOCK / 32 * 256 <= CAP && BLOCK >= 256 && ITEMS * 32 == 256 && CAP <= 8192, "the warps' counts lie where the bins do; places take 13 bits");
     const u32 tid = threadIdx.x;
     const u32 base = starts ? starts[blockIdx.x] : 0, m = (starts ? starts[blockIdx.x + 1] : n) - base;
     if(m == 0 || m > CAP) return;       // the host has seen to it that all fit
@@ -242,36 +304,77 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* _
         }
         if(bins == CAP && tid == 0) start[CAP] = u16(m);            // behind the threads' words
     }
-    const bool by_network = __syncthreads_or(max(longest & 0xFFFFu, longest >> 16) > LONG_BIN);
-    if(by_network)
+    if(__syncthreads_or(max(longest & 0xFFFFu, longest >> 16) > LONG_BIN))
     {
-        // Many records in one bin: a sorting network over (key, place before), padded with records behind all others.
-        u32 size = 1;
-        while(size < m) size <<= 1;
+        // Many records in one bin: stable passes by 8 of the bits in which the bucket's keys differ, low ones first. A warp takes up to 256 records in a row and
+        // numbers those of a digit itself; the sums over the warps' counts give the places.
+        const u32 rounds = (m + BLOCK - 1) / BLOCK;         // 32 records a warp in each
+        u16 (*const count)[256] = reinterpret_cast<u16 (*)[256]>(bin);
+        const u32 warp = tid >> 5, lane = lane_id();
+        if(tid < 2) s_differ[tid] = 0;
         #pragma unroll
         for(int i = 0; i < ITEMS; ++i)
         {
             const u32 j = tid + i * BLOCK;
-            if(j >= size) break;
-            stage[j] = j < m ? r[i] : ~0ull;
-            from[j] = j < m ? u16(j) : u16(0xFFFF);
+            if(j >= m) break;
+            stage[j] = r[i];
+            from[j] = u16(j);
         }
         __syncthreads();
-        for(u32 k = 2; k <= size; k <<= 1)
-            for(u32 d = k >> 1; d > 0; d >>= 1)
+        {
+            u64 differ = 0;
+            const u64 k0 = stage[0];
+            #pragma unroll
+            for(int i = 0; i < ITEMS; ++i) if(tid + i * BLOCK < m) differ |= r[i] ^ k0;
+            differ &= compared;
+            const u32 lo = __reduce_or_sync(0xFFFFFFFFu, u32(differ)), hi = __reduce_or_sync(0xFFFFFFFFu, u32(differ >> 32));
+            if(lane == 0) { atomicOr(&s_differ[0], lo); atomicOr(&s_differ[1], hi); }
+        }
+        __syncthreads();
+        for(u64 rest = u64(s_differ[1]) << 32 | s_differ[0]; rest; )
+        {
+            const int shift = __ffsll(rest) - 1;
+            rest = shift + 8 >= 64 ? 0 : rest & (~0ull << (shift + 8));
+            reinterpret_cast<uint4*>(count[warp])[lane] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            auto digit_of = [&](const u64 key) { return u32((key & compared) >> shift) & 255u; };
+            const u32 first = warp * (32 * rounds) + lane;
+            #pragma unroll
+            for(int i = 0; i < ITEMS; ++i)
+                if(i < rounds && first + i * 32 < m) { r[i] = stage[first + i * 32]; pl[i] = from[first + i * 32]; }
+            #pragma unroll
+            for(int i = 0; i < ITEMS; ++i)
             {
-                for(u32 t = tid; t < size / 2; t += BLOCK)
+                if(i >= rounds) break;
+                const bool there = first + i * 32 < m;
+                const u32 d = there ? digit_of(r[i]) : 256u, same = __match_any_sync(0xFFFFFFFFu, d);
+                const u32 before = there ? count[warp][d] : 0u;
+                __syncwarp();
+                if(there)
                 {
-                    const u32 a = 2 * t - (t & (d - 1)), b = a + d;
-                    const u64 x = stage[a], y = stage[b];
-                    const u16 fx = from[a], fy = from[b];
-                    const u64 cx = x & compared, cy = y & compared;
-                    // a padding record's key may equal a real one's: its place decides
-                    const bool greater = cx > cy || (cx == cy && fx > fy);
-                    if(greater == ((a & k) == 0)) { stage[a] = y; stage[b] = x; from[a] = fy; from[b] = fx; }
+                    pl[i] |= (before + __popc(same & lanemask_lt())) << 16;
+                    if(lane == u32(__ffs(same)) - 1) count[warp][d] = u16(before + __popc(same));
                 }
-                __syncthreads();
+                __syncwarp();
             }
+            __syncthreads();
+            u32 sum = 0;
+            if(tid < 256)
+                for(u32 w = 0; w < BLOCK / 32; ++w) sum += count[w][tid];
+            u32 run = block_exclusive_sum<BLOCK>(sum, warp_tot);
+            if(tid < 256)
+                for(u32 w = 0; w < BLOCK / 32; ++w) { const u32 c = count[w][tid]; count[w][tid] = u16(run); run += c; }
+            __syncthreads();
+            #pragma unroll
+            for(int i = 0; i < ITEMS; ++i)
+                if(i < rounds && first + i * 32 < m)
+                {
+                    const u32 at = count[warp][digit_of(r[i])] + (pl[i] >> 16);
+                    stage[at] = r[i];
+                    from[at] = u16(pl[i]);
+                }
+            __syncthreads();
+        }
         for(u32 j = tid; j < m; j += BLOCK)
         {
             keys_out[j] = stage[j];
@@ -370,7 +473,8 @@ int bucket_sort_bits(u64 n)
     return t == 9 ? 8 : t;          // 9 bits would be a second pass
 }
 
-int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int end_bit, int bits, int low_bits, u32* starts, u64* low_base, u64* high_base, u64* largest_dev)
+int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int begin_bit, int end_bit, int bits, int low_bits, int least_digits, u32* starts, u64* low_base, u64* high_base,
+                       Bucket_Findings* found, u64* verdict)
 {
     static std::atomic<bool> configured[64];
     if(!configured[ctx->device & 63])
@@ -378,10 +482,10 @@ int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int end_bit, int bi
         CSA_CUDA(ctx, cudaFuncSetAttribute(bucket_counts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(4u << BUCKET_MAX_BITS)));
         configured[ctx->device & 63] = true;
     }
-    CSA_CUDA(ctx, cudaMemsetAsync(starts, 0, size_t(4) << bits, ctx->stream));
-    bucket_counts_kernel<<<unsigned(std::min<u64>(148, div_up(n, 2 * COUNT_BLOCK * COUNT_UNROLL))), COUNT_BLOCK, size_t(4) << bits, ctx->stream>>>(keys, n, end_bit - bits, bits, starts);
+    bucket_counts_kernel<<<unsigned(std::min<u64>(148, div_up(n, 2 * COUNT_BLOCK * COUNT_UNROLL))), COUNT_BLOCK, size_t(4) << bits, ctx->stream>>>(keys, n, begin_bit, end_bit, bits,
+                                                                                                                                             least_digits, starts, found);
     CSA_LAUNCH_CHECK(ctx);
-    bucket_plan_kernel<<<1, 1024, 0, ctx->stream>>>(starts, u32(n), bits, low_bits, low_base, high_base, largest_dev);
+    launch_early(bucket_plan_kernel, 1, 1024, 0, ctx->stream, starts, u32(n), begin_bit, end_bit, bits, low_bits, least_digits, low_base, high_base, found, verdict);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -26,6 +26,7 @@ enum : u64
 };
 
 constexpr int CSA_COUNTS_WORD = 40;         // of d_scalars: the counters of a resident build (Build_Counts)
+constexpr int CSA_VERDICT_WORD = 50;        // of h_scalars: what a sort's counts say about its buckets
 constexpr int CSA_STATUS_WORD = 63;         // of d_scalars: the status word
 
 // One per (device, host thread): a stream, the device status word, a grow-only scratch arena and pinned

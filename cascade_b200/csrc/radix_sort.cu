@@ -132,10 +132,14 @@ __device__ __forceinline__ void histogram_body(const u64* __restrict__ keys, con
     }
 }
 
+// only_if (or null): a word that has to be non-zero, else nothing is done.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) histogram_kernel(const u64* __restrict__ keys, const u64 n, const int begin_bit, const int end_bit, const int passes,
-                                                         u64* __restrict__ hist)
+                                                         u64* __restrict__ hist, const u32* __restrict__ only_if)
 {
+    let_next_in();
+    wait_for_previous();
+    if(only_if != nullptr && *only_if == 0) return;
     histogram_body<BLOCK>(keys, n, begin_bit, end_bit, passes, hist, RADIX, blockIdx.x, gridDim.x);
 }
 
@@ -155,8 +159,10 @@ __global__ void __launch_bounds__(BLOCK) seg_histogram_kernel(const u64* __restr
 // digit holds all n records (such a pass moves nothing and is skipped).
 // hist: [passes][RADIX]. base: [passes][launches + 1][RADIX], of which slot 0 is written here. skip: [passes].
 __global__ void __launch_bounds__(RADIX) digit_base_kernel(const u64* __restrict__ hist, const int launches, const u64 n,
-                                                          u64* __restrict__ base, u64* __restrict__ skip)
+                                                          u64* __restrict__ base, u64* __restrict__ skip, const u32* __restrict__ only_if)
 {
+    wait_for_previous();
+    if(only_if != nullptr && *only_if == 0) return;
     __shared__ u64 warp_tot[RADIX / 32];
     __shared__ int s_skip;
     const int p = blockIdx.x, d = threadIdx.x;
@@ -754,7 +760,7 @@ extern "C" int csa_debug_set(int key, uint64_t value)
 }
 
 // Device address of the digit histograms ([pass][RADIX] 64-bit counts) that the last csa_sort_pairs of n records left in
-// its workspace (the same carving as in csa_sort_pairs).
+// its workspace (the same carving as in csa_sort_pairs); a sort by buckets leaves none, and builds' sorts are never by buckets.
 const u64* sort_workspace_histograms(void* workspace, size_t workspace_bytes, u64 n)
 {
     Carver cv(workspace, workspace_bytes);
@@ -764,9 +770,9 @@ const u64* sort_workspace_histograms(void* workspace, size_t workspace_bytes, u6
     return cv.take<u64>(u64(8) * RADIX);
 }
 
-// Words of the buckets' starts. More than BUCKET_MAX_TOTAL records have none, but a workspace for them serves shorter lists, too: callers size one for the
+// Words of the buckets' starts and of what their counts say. More than BUCKET_MAX_TOTAL records have none, but a workspace for them serves shorter lists, too: callers size one for the
 // longest of their lists, so the size never falls as n grows.
-static size_t bucket_starts(const u64 n) { return (size_t(1) << bucket_sort_bits(n < BUCKET_MAX_TOTAL ? n : BUCKET_MAX_TOTAL)) + 1; }
+static size_t bucket_starts(const u64 n) { return (size_t(1) << bucket_sort_bits(n < BUCKET_MAX_TOTAL ? n : BUCKET_MAX_TOTAL)) + 1 + sizeof(Bucket_Findings) / 4; }
 
 size_t csa_sort_workspace_bytes(uint64_t n)
 {
@@ -826,30 +832,24 @@ void sort_reset_timing(csa_ctx* ctx)
 namespace
 {
 
-// The sort by buckets (bucket_sort.cu), where it spares two digit passes or more and no bucket is too large for a block; else nothing has been
-// moved and done stays false. Not for sorts whose ties may come in any order: their keys are pairs of ranks, uneven in the top bits, and
-// their first pass is the cheap one.
-int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* vals_alt, u32 val_bytes, u64 n, int begin_bit, int end_bit, u32* counter, u32* status, u64* base,
-                    u32* starts, int* in_alt, bool& done)
+// The sort by buckets (bucket_sort.cu): bits of the buckets' number, by how many digit passes the records get there, and the bits of the first of two. It is
+// for keys whose buckets fit a block and which differ in so many digits that the digit passes, those of equal digits skipped, take longer (us a call, by buckets and
+// by digits: two digits, 10^5 records 66 and 75; three digits, 10^6 records 96 to 104 and 106, 4 * 10^6 206 to 245 and 197, 31.25 M 1.14 to 2.8 and 0.89 ms). Not for sorts whose ties may come in any
+// order: their keys are pairs of ranks, uneven in the top bits, and their first pass is the cheap one.
+struct Bucket_Split
 {
-    const int width = end_bit - begin_bit, passes = (width + RADIX_BITS - 1) / RADIX_BITS;
-    if(n <= BUCKET_MAX_RECORDS && passes >= 2)
-    {
-        CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, nullptr, 1, n, n, begin_bit, end_bit));
-        *in_alt = 1;
-        done = true;
-        return CSA_OK;
-    }
-    const int bits = bucket_sort_bits(n), splits = bits > RADIX_BITS ? 2 : 1, low_bits = bits > RADIX_BITS ? bits - RADIX_BITS : 0;
-    if(n > BUCKET_MAX_TOTAL || passes < splits + 2) return CSA_OK;
-    u64* const low_base = base;
-    u64* const high_base = base + RADIX;
-    u64* const largest_dev = ctx->d_scalars + 32;
-    CSA_TRY(launch_bucket_plan(ctx, keys, n, end_bit, bits, low_bits, starts, low_base, high_base, largest_dev));
-    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 32, largest_dev, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    const u64 largest = ctx->h_scalars[32];
-    if(largest > BUCKET_MAX_RECORDS) return CSA_OK;
+    int bits, splits, low_bits;
+    explicit Bucket_Split(u64 n) : bits(bucket_sort_bits(n)), splits(bits > RADIX_BITS ? 2 : 1), low_bits(bits > RADIX_BITS ? bits - RADIX_BITS : 0) {}
+    int least_digits() const { return splits == 1 ? 2 : 4; }        // in which the keys differ
+    int least_passes() const { return splits + 2; }                 // of the bits that are sorted by
+};
+
+// The passes and the buckets, once the counts are there; largest: the size of the largest bucket.
+int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* vals_alt, u32 val_bytes, u64 n, int begin_bit, int end_bit, u32* counter, u32* status, const u64* low_base,
+                    const u64* high_base, const u32* starts, u64 largest, int* in_alt)
+{
+    const Bucket_Split split(n);
+    const int bits = split.bits, splits = split.splits, low_bits = split.low_bits;
     Pass_Timer& timer = timer_of(ctx);
     for(int s = 2 - splits; s < 2; ++s)
     {
@@ -881,7 +881,6 @@ int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* va
     }
     CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, starts, 1u << bits, n, largest, begin_bit, end_bit - bits));
     *in_alt = (splits + 1) & 1;
-    done = true;
     return CSA_OK;
 }
 
@@ -905,15 +904,14 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
     u32* counter = cv.take<u32>(64);                     // 256 bytes, directly before the status words
     u32* status = cv.take<u32>(tiles_max * RADIX);
     u64* hist = cv.take<u64>(u64(8) * RADIX);
+    u32* found_words = cv.take<u32>(bucket_starts(n));      // directly behind the histograms: zeroed with them
     u64* base = cv.take<u64>(u64(portions + 1) * 8 * RADIX);
-    u32* starts = cv.take<u32>(bucket_starts(n));
     if(!cv.ok) return csa_fail(ctx, CSA_E_NOMEM, "csa_sort_pairs: workspace too small");
 
-    if(!ctx->ties_in_any_order && portions == 1)
+    if(!ctx->ties_in_any_order && n <= BUCKET_MAX_RECORDS && passes >= 2 && portions == 1)
     {
-        bool done = false;
-        CSA_TRY(sort_by_buckets(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, n, begin_bit, end_bit, counter, status, base, starts, in_alt, done));
-        if(done) return CSA_OK;
+        *in_alt = 1;
+        return launch_bucket_sort(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, nullptr, 1, n, n, begin_bit, end_bit);
     }
 
     {
@@ -924,21 +922,37 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
             hist_configured[ctx->device & 63] = true;
         }
     }
-    CSA_CUDA(ctx, cudaMemsetAsync(hist, 0, u64(passes) * RADIX * sizeof(u64), ctx->stream));
+    // The buckets are counted first where the keys may be for them; the histograms are queued behind, for uneven keys only, so that one wait tells which way it goes.
+    const Bucket_Split split(n);
+    const bool buckets = !ctx->ties_in_any_order && portions == 1 && n <= BUCKET_MAX_TOTAL && passes >= split.least_passes();
+    Bucket_Findings* const found = reinterpret_cast<Bucket_Findings*>(found_words);
+    u32* const starts = found_words + sizeof(Bucket_Findings) / 4;
+    u64* const low_base = base;             // the digit passes' own offsets come to the same place, where it comes to those
+    u64* const high_base = base + RADIX;
+    u64* const skip_host = ctx->h_scalars + 32;         // pinned: written by the kernel
+    const u32* const only_if = buckets ? &found->uneven : nullptr;
+    if(buckets)
+    {
+        CSA_CUDA(ctx, cudaMemsetAsync(hist, 0, u64(8) * RADIX * sizeof(u64) + (sizeof(Bucket_Findings) + (size_t(4) << split.bits)), ctx->stream));
+        CSA_TRY(launch_bucket_plan(ctx, reinterpret_cast<const u64*>(keys), n, begin_bit, end_bit, split.bits, split.low_bits, split.least_digits(), starts, low_base, high_base, found,
+                                   ctx->h_scalars + CSA_VERDICT_WORD));
+    }
+    else CSA_CUDA(ctx, cudaMemsetAsync(hist, 0, u64(passes) * RADIX * sizeof(u64), ctx->stream));
     for(int P = 0; P < portions; ++P)
     {
         const u64 first = u64(P) * PORTION, cnt = (n - first < PORTION ? n - first : PORTION);
         const unsigned blocks = unsigned(cnt / (2 * 256 * HIST_UNROLL) < 1 ? 1 : (cnt / (2 * 256 * HIST_UNROLL) > 148 * 3 ? 148 * 3 : cnt / (2 * 256 * HIST_UNROLL)));
-        histogram_kernel<256><<<blocks, 256, size_t(8) * passes * RADIX * 4, ctx->stream>>>(reinterpret_cast<const u64*>(keys) + first, cnt, begin_bit, end_bit, passes, hist);
+        launch_early(histogram_kernel<256>, blocks, 256, size_t(8) * passes * RADIX * 4, ctx->stream, reinterpret_cast<const u64*>(keys) + first, cnt, begin_bit, end_bit, passes, hist, only_if);
         CSA_LAUNCH_CHECK(ctx);
     }
-    u64* d_skip = ctx->d_scalars + 32;
-    digit_base_kernel<<<passes, RADIX, 0, ctx->stream>>>(hist, portions, n, base, d_skip);
+    launch_early(digit_base_kernel, unsigned(passes), RADIX, 0, ctx->stream, hist, portions, n, base, skip_host, only_if);
     CSA_LAUNCH_CHECK(ctx);
-    CSA_CUDA(ctx, cudaMemcpyAsync(ctx->h_scalars + 32, d_skip, passes * sizeof(u64), cudaMemcpyDeviceToHost, ctx->stream));
     CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if(buckets && ctx->h_scalars[CSA_VERDICT_WORD] != 0)
+        return sort_by_buckets(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, n, begin_bit, end_bit, counter, status, low_base, high_base,
+                               starts, ctx->h_scalars[CSA_VERDICT_WORD], in_alt);
     u64 skip[8];
-    for(int p = 0; p < passes; ++p) skip[p] = ctx->h_scalars[32 + p];
+    for(int p = 0; p < passes; ++p) skip[p] = skip_host[p];
 
     Pass_Timer& timer = timer_of(ctx);
     u64* kin = reinterpret_cast<u64*>(keys); u64* kout = reinterpret_cast<u64*>(keys_alt);
@@ -1210,8 +1224,8 @@ extern "C" int csa_sort_pairs_static(void* stream_, uint64_t* keys, uint64_t* ke
     // The array keeps the last call's contents: everything that must start at zero is cleared here.
     if(cudaMemsetAsync(base_addr + ST_OFF_COUNTER, 0, ST_BYTES - ST_OFF_COUNTER, stream) != cudaSuccess) return CSA_E_CUDA;
     const unsigned hblocks = unsigned(n / (2 * 256 * HIST_UNROLL) < 1 ? 1 : (n / (2 * 256 * HIST_UNROLL) > 148 * 3 ? 148 * 3 : n / (2 * 256 * HIST_UNROLL)));
-    histogram_kernel<256><<<hblocks, 256, size_t(8) * passes * RADIX * 4, stream>>>(reinterpret_cast<const u64*>(keys), n, begin_bit, end_bit, passes, hist);
-    digit_base_kernel<<<passes, RADIX, 0, stream>>>(hist, 1, n, base, skip);
+    histogram_kernel<256><<<hblocks, 256, size_t(8) * passes * RADIX * 4, stream>>>(reinterpret_cast<const u64*>(keys), n, begin_bit, end_bit, passes, hist, nullptr);
+    digit_base_kernel<<<passes, RADIX, 0, stream>>>(hist, 1, n, base, skip, nullptr);
     u64* kin = reinterpret_cast<u64*>(keys); u64* kout = reinterpret_cast<u64*>(keys_alt);
     u32* vin = vals; u32* vout = vals_alt;
     for(int p = 0; p < passes; ++p)     // every pass runs (no read-back decides about skipping), so the result's place is known

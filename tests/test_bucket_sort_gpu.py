@@ -63,3 +63,45 @@ def test_uneven_keys(ctx, n, kind):
         keys = torch.where(index % 5 == 0, torch.full_like(r, -1), r)
     for bits in ((0, 64), (0, 40)):
         _check(ctx, keys.clone(), torch.arange(n, device="cuda", dtype=torch.int32), *bits)
+
+
+# one block; buckets in blocks of 2048 to 8192; above 2^21 records a sample is looked at before the keys are counted
+@pytest.mark.parametrize("n", [300, 4097, 8191, 8192, 262_144, 2_200_001])
+@pytest.mark.parametrize("kind", ["a_run_a_key", "runs_that_differ_low", "top_bits_and_three_values", "two_far_bits", "one_odd_key"])
+@pytest.mark.parametrize("value", [torch.int32, torch.int64])
+def test_many_records_of_a_few_keys(ctx, n, kind, value):
+    """Bins that hold hundreds of records: a block orders them by the digits in which its keys differ, equal keys as they came."""
+    r = _random(n, n + 1)
+    index = torch.arange(n, device="cuda")
+    if kind == "a_run_a_key":                   # 300 records of every key, the keys spread evenly
+        keys = (index // 300) * 0x1E37_79B9_7F4A_7C15
+    elif kind == "runs_that_differ_low":        # the same with 8 low bits of their own
+        keys = ((index % max(1, n // 300)) * 0x1E37_79B9_7F4A_7C15 & ~0xFF) | (r & 0xFF)
+    elif kind == "top_bits_and_three_values":
+        keys = (r & ~((1 << 49) - 1)) | ((r >> 3) & 0xFF) % 3
+    elif kind == "two_far_bits":                # the lowest and the highest bit: no digit holds both
+        keys = (r & 1) | (r & 2) << 62
+    else:
+        keys = torch.full_like(r, 0x0123_4567_89AB_CDEF)
+        keys[n // 2] += 1 << 20
+    for bits in ((0, 64), (1, 50)):
+        _check(ctx, keys.clone(), torch.arange(n, device="cuda", dtype=value), *bits)
+
+
+@pytest.mark.parametrize("n", [100_000, 3_000_001])
+def test_which_way_the_keys_go(ctx, n):
+    """By the launches: four of them look at the keys; then one or two splits and the buckets, or a pass for each digit that differs."""
+    from cascade_b200 import api
+    r, vals = _random(n, 3), torch.arange(n, device="cuda", dtype=torch.int32)
+    splits = 1 if n <= 1 << 19 else 2
+
+    def launches(keys):
+        before = ctx.launches
+        api.sort_pairs(ctx, keys, vals.clone())
+        return ctx.launches - before - 4
+
+    assert launches(r.clone()) == splits + 1
+    assert launches(torch.full_like(r, 5)) == 0
+    assert launches(r & 0xFF_FFFF) == 3
+    assert launches(r & ~((1 << 56) - 1)) == 1
+    assert launches(torch.where(vals % 2 == 0, r, torch.zeros_like(r))) == 8
