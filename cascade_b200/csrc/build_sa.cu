@@ -58,6 +58,14 @@ constexpr u64 FOLLOWED_MIN = u64(1) << 22;
 // 1e9 near-duplicate suffixes with 1849 of them in large groups: 365 ms with the large groups left to the generations, so that nothing followed, 252 this way.
 constexpr u64 LARGE_SHARE = 8;
 constexpr u32 LARGE_STEPS = 12;
+// And only where ranks pay, which a sample tells: nearly all suffixes have a follower, or most have and many share more symbols than the text is compared for, which need ranks
+// anyway. Else most ties are settled by the text alone. ms a build of 4e8 suffixes, ranked and by text, in brackets the sample's two shares: phrases that occur four times, of 4 symbols
+// (0.51, 0) 47.9 and 31.1, of 8 (0.83, 0) 42.7 and 39.7, of 12 (0.89, 0) 42.3 and 42.6, of 30 (0.96, 0) 42.1 and 46.1; near-duplicates with 1.3 % of their symbols replaced (0.76, 0.27)
+// 84.7 and 100.6, with 2 % (0.67, 0.14) 115 and 99.
+bool ranks_pay(const Build_Counts& c)
+{
+    return u64(c.lead_on) * 8 >= u64(c.looked_at) * 7 || (u64(c.lead_on) * 10 >= u64(c.looked_at) * 7 && u64(c.far_ties) * 5 >= c.looked_at);
+}
 
 int set_build_count(csa_ctx* ctx, u32* at, u32 value)
 {
@@ -135,18 +143,6 @@ struct Build
         return CSA_OK;
     }
 
-    // The same of ends (refine.cu).
-    int generation_of_ends(u64 h, const u32* bits)
-    {
-        CSA_TRY(set_count(&Build_Counts::next_small, 0));
-        CSA_TRY(launch_refine_ends(ctx, front, small, h, reinterpret_cast<u64*>(work), bits, isa, n, sa, other, counts));
-        Build_Counts c;
-        CSA_TRY(read_counts(c));
-        small = c.next_small;
-        std::swap(front, other);
-        return CSA_OK;
-    }
-
     // One generation of prefix doubling: the suffixes of every group ordered by the ranks of those h symbols further on. The first
     // `idle` entries of the list share more than h symbols already and stay as they are.
     //
@@ -206,6 +202,18 @@ struct Build
         in_arrays = nl != 0 && large != 0 && 2 * h <= MAX_SMALL_H && u64(c.now_small) * 8 <= u64(c.now_small) + c.large;
         if(in_arrays) { small -= c.now_small; large += c.now_small; }
         else if(nl) CSA_TRY(launch_split_by_size(ctx, head, pos, nl, ctx->d_scalars, other, n, scratch));
+        std::swap(front, other);
+        return CSA_OK;
+    }
+
+    // The same of the ends of rows of groups that follow one another (refine.cu).
+    int generation_of_ends(u64 h, const u32* bits)
+    {
+        CSA_TRY(set_count(&Build_Counts::next_small, 0));
+        CSA_TRY(launch_refine_ends(ctx, front, small, h, reinterpret_cast<u64*>(work), bits, isa, n, sa, other, counts));
+        Build_Counts c;
+        CSA_TRY(read_counts(c));
+        small = c.next_small;
         std::swap(front, other);
         return CSA_OK;
     }
@@ -280,7 +288,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     // More tied suffixes than this are first looked through for groups that follow one another: those need not be compared.
     const u64 most_by_text = std::max(FOLLOWED_MIN, n / 4);
     Build_Counts c;
-    CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text));
+    CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text, b.tab.code, b.ps.key_bits));
     bool done = false;          // the output is complete, and the events have been waited for with the counters below
     if(!words)
     {
@@ -295,7 +303,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
         if(debug) std::fprintf(stderr, "[csa] %u children (%u suffixes) do not fit a block\n", c.oversize, c.oversize_records);
         CSA_TRY(b.sort_oversize(c));
         if(!words) CSA_TRY(launch_pack_oversize(ctx, b.tab, c.oversize, b.sa, sa40));
-        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text));
+        CSA_TRY(launch_refine_by_text(ctx, T, n, depth0, depth, b.front, b.other, words, sa40, nullptr, b.counts, n, most_by_text, b.tab.code, b.ps.key_bits));
         CSA_TRY(b.read_counts(c));
     }
     st.partitions = c.partitions;
@@ -317,7 +325,10 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
         done = false;
         b.small = c.small;
         b.large = c.large;
-        if(c.large <= c.small / LARGE_SHARE)
+        bool rank = c.large <= c.small / LARGE_SHARE && ranks_pay(c);
+        if(debug) std::fprintf(stderr, "[csa] of %u tied suffixes looked at %u are tied one symbol on, %u share %llu symbols: %s\n", c.looked_at, c.lead_on, c.far_ties, depth,
+                               rank ? "ranked" : "compared in the text");
+        if(rank)
         {
             CSA_TRY(b.more_memory());
             if(!words) CSA_TRY(launch_unpack_sa40(ctx, sa40, n, b.sa));

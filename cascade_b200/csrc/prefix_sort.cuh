@@ -25,6 +25,7 @@ struct Build_Counts
     u32 medium;         // children that fit the local sort's larger blocks only
     u32 now_small;      // entries that the last count by size found in small groups
     u32 large_depth;    // symbols that the suffixes of a large group share at least after the initial sort (launch_large_depth)
+    u32 looked_at, lead_on, far_ties;       // what a sample of the small groups' entries says (launch_refine_by_text)
 };
 static_assert(sizeof(Build_Counts) <= (CSA_STATUS_WORD - CSA_COUNTS_WORD) * 8, "the counters lie before the status word");
 

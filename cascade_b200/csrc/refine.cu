@@ -308,6 +308,65 @@ __device__ __forceinline__ u64 difference_key(const u16* __restrict__ T, const u
     return pair_key(pair, mine, hx, lead, hy);
 }
 
+// A sample of a list of small groups, a warp to an entry: whether all suffixes of the entry's group still have one key one symbol on, by their symbols' code words (a key is
+// key_bits bits), and whether the entry beside it shares `depth` symbols with it. A function of its own: it takes no registers from the kernel that calls it.
+__device__ __noinline__ void sample_ties(const u64* __restrict__ list, const u64 count, const u16* __restrict__ T, const u64 n, const u32* __restrict__ code, const u32 key_bits, const u32 depth,
+                                         Build_Counts* __restrict__ counts)
+{
+    const u64 step = (count + TIE_SAMPLE - 1) / TIE_SAMPLE;
+    auto symbol = [&](const u64 at) { return at < n ? u32(__ldg(T + at)) : 0u; };
+    for(u64 k = (u64(blockIdx.x) * (RW_BLOCK / 32) + (threadIdx.x >> 5)) * step; k < count; k += u64(gridDim.x) * (RW_BLOCK / 32) * step)
+    {
+        const u64 e = __ldg(list + k), x = u32(e);
+        constexpr int PIECES = 2 * int(SMALL_GROUP) / 32;       // the entries before and behind: a small group reaches no further
+        u64 near[PIECES];
+        #pragma unroll
+        for(int c = 0; c < PIECES; ++c)
+        {
+            const long long at = (long long)(k) - int(SMALL_GROUP) + c * 32 + int(lane_id());
+            near[c] = at >= 0 && u64(at) < count && u64(at) != k ? __ldg(list + at) : ~e;
+        }
+        // The group's keys tell its first `whole` symbols, the keys one symbol on are at their end with symbol `end`.
+        u32 first = 0, bits = 0, whole = 0, end = 0, before = 0;        // before: bits from symbol 1 up to symbol `whole`
+        for(bool told = false; end == 0 || bits - first < key_bits; ++end)
+        {
+            const u32 len = __ldg(code + symbol(x + end)) & 31u;
+            if(end == 0) first = len;
+            bits += len;
+            if(!told && bits > key_bits) { told = true; whole = end; before = bits - len - first; }
+        }
+        if(whole == 0) { whole = 1; before = 0; }
+        bool leaves = false, any = false;
+        #pragma unroll
+        for(int c = 0; c < PIECES; ++c)
+        {
+            if(u32(near[c] >> 32) != u32(e >> 32)) continue;
+            any = true;
+            const u64 y = u32(near[c]);
+            u32 upto = before;
+            for(u32 d = whole; d < end; ++d)
+            {
+                const u32 a = __ldg(code + symbol(x + d)), b = __ldg(code + symbol(y + d));
+                if(a != b) { leaves |= upto + __clz((a ^ b) & ~31u) < key_bits; break; }
+                upto += a & 31u;
+            }
+        }
+        leaves = __any_sync(0xFFFFFFFFu, leaves);
+        any = __any_sync(0xFFFFFFFFu, any);
+        const u64 behind = __shfl_sync(0xFFFFFFFFu, near[PIECES / 2], 1), ahead = __shfl_sync(0xFFFFFFFFu, near[PIECES / 2 - 1], 31);
+        const u64 y = u32(u32(behind >> 32) == u32(e >> 32) ? behind : ahead);
+        bool differs = false;
+        for(u32 d = lane_id(); d < depth; d += 32) differs |= x + d >= n || y + d >= n || T[x + d] != T[y + d];
+        differs = __any_sync(0xFFFFFFFFu, differs);
+        if(lane_id() == 0 && any)
+        {
+            atomicAdd(&counts->looked_at, 1u);
+            if(!leaves) atomicAdd(&counts->lead_on, 1u);
+            if(!differs) atomicAdd(&counts->far_ties, 1u);
+        }
+    }
+}
+
 // Orders groups by the symbols [from, to) of their suffixes. In a round every member of a group is compared with the group's first
 // member, and the members are put in order by their first difference from it; a group that falls apart goes on as several, each
 // with its own depth. The window stays in shared memory over all rounds.
@@ -320,7 +379,7 @@ __device__ __forceinline__ u64 difference_key(const u16* __restrict__ T, const u
 // the chain of loads counts: the first round is then QUICK, 8 symbols by one thread, all of a thread's suffixes in flight together.
 __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* __restrict__ T, const u64 n, const u64 from, const u64 to, const u64* __restrict__ list,
                                                                     u64* __restrict__ next, u32* __restrict__ sa, u8* __restrict__ sa40, u32* __restrict__ isa, Build_Counts* __restrict__ counts,
-                                                                    const u64 most)
+                                                                    const u64 most, const u32* __restrict__ code, const u32 key_bits)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Window& w = *reinterpret_cast<Window*>(smem_raw);
@@ -330,7 +389,11 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
-    if(count > most) return;
+    if(count > most)
+    {
+        if(code != nullptr) sample_ties(list, count, T, n, code, key_bits, u32(to), counts);
+        return;
+    }
     for(u64 first = u64(blockIdx.x) * RW_TILE; first < count; first += u64(gridDim.x) * RW_TILE)
     {
         load_window(w, list, count, first);
@@ -1050,12 +1113,12 @@ int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c)
 }
 
 int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, u8* sa40, u32* isa, Build_Counts* counts, u64 expected,
-                          u64 most)
+                          u64 most, const u32* code, int key_bits)
 {
     to = to < n ? to : n;           // no two suffixes share as much
     CSA_CUDA(ctx, cudaFuncSetAttribute(refine_by_text_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TEXT_SMEM)));
     const u64 tiles = div_up(expected ? expected : 1, RW_TILE);
-    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, sa40, isa, counts, most);
+    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, sa40, isa, counts, most, code, u32(key_bits));
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -72,3 +72,55 @@ def test_a_few_large_groups_beside_many_small_ones(ctx, length):
     for k in rng.integers(0, len(T) - length, 400):
         T[k:k + length] = np.arange(1, length + 1)
     _check(ctx, T)
+
+
+# ---- which way a text goes, as the build's own diagnostics (CSA_DEBUG) say it ----------------------------------------------------
+
+
+def _way(ctx, T, capfd, monkeypatch):
+    monkeypatch.setenv("CSA_DEBUG", "1")
+    capfd.readouterr()
+    _check(ctx, T)
+    return capfd.readouterr().err
+
+
+def _mutated(T, share, rng):
+    T = T.copy()
+    hit = rng.random(len(T)) < share
+    T[hit] = rng.integers(1, 60000, int(hit.sum()))
+    return T
+
+
+def _phrases(n, length, times, rng):
+    vocab = rng.integers(1, 60000, (n // (length * times), length)).astype(np.uint16)
+    return vocab[rng.integers(0, len(vocab), n // length)].reshape(-1)
+
+
+def test_near_duplicates_are_followed(ctx, capfd, monkeypatch):
+    rng = np.random.default_rng(1)
+    err = _way(ctx, _mutated(np.tile(rng.integers(1, 60000, 150_000).astype(np.uint16), 40), 1e-3, rng), capfd, monkeypatch)
+    assert "are tied one symbol on" in err and "have a follower" in err and "large groups, h=" not in err and "generation" in err
+
+
+def test_large_groups_are_ranked_ahead_and_the_others_followed(ctx, capfd, monkeypatch):
+    """A passage of six symbols that stands in the text 400 times."""
+    rng = np.random.default_rng(2)
+    T = _mutated(np.tile(rng.integers(1, 60000, 150_000).astype(np.uint16), 40), 1e-3, rng)
+    for k in rng.integers(0, len(T) - 6, 400):
+        T[k:k + 6] = np.arange(1, 7)
+    err = _way(ctx, T, capfd, monkeypatch)
+    assert "large groups, h=" in err and "have a follower" in err
+
+
+@pytest.mark.parametrize("kind", ["phrases", "far_copies", "two_symbols"])
+def test_ties_that_the_text_settles_are_not_ranked(ctx, capfd, monkeypatch, kind):
+    """Many tied suffixes whose groups fall apart a symbol on: no inverse array is made to find that out."""
+    rng = np.random.default_rng(3)
+    if kind == "phrases":
+        T = _phrases(40_000_000, 4, 4, rng)
+    elif kind == "far_copies":
+        T = _mutated(np.tile(rng.integers(1, 60000, 300_000).astype(np.uint16), 20), 0.05, rng)
+    else:
+        T = rng.integers(0, 2, 40_000_000).astype(np.uint16)
+    err = _way(ctx, T, capfd, monkeypatch)
+    assert "are tied one symbol on" in err and "have a follower" not in err
