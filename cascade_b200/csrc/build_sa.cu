@@ -330,7 +330,14 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
                                rank ? "ranked" : "compared in the text");
         if(rank)
         {
-            CSA_TRY(b.more_memory());
+            // Without the buffers the ties are compared in the text first: the ranks may not be needed then.
+            const std::string err = ctx->err;
+            const int rc = b.more_memory();
+            if(rc != CSA_OK && rc != CSA_E_NOMEM) return rc;
+            if(rc != CSA_OK) { ctx->err = err; rank = false; }
+        }
+        if(rank)
+        {
             if(!words) CSA_TRY(launch_unpack_sa40(ctx, sa40, n, b.sa));
             words = b.sa;
             CSA_TRY(launch_make_inverse(ctx, b.sa, n, b.front, b.small, b.large_list(b.front), b.large, b.isa, reinterpret_cast<u64*>(b.work)));

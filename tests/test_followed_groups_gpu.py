@@ -124,3 +124,44 @@ def test_ties_that_the_text_settles_are_not_ranked(ctx, capfd, monkeypatch, kind
         T = rng.integers(0, 2, 40_000_000).astype(np.uint16)
     err = _way(ctx, T, capfd, monkeypatch)
     assert "are tied one symbol on" in err and "have a follower" not in err
+
+
+def test_ties_that_the_text_settles_need_no_memory_for_ranks(capfd, monkeypatch):
+    """Phrases of thirty symbols: nearly all groups are followed, but where the device has no room for the ranks the text alone tells the suffixes apart. A text
+    that needs them is refused, and the context goes on."""
+    from cascade_b200 import api
+    rng = np.random.default_rng(4)
+    n = 1 << 24
+    texts = [_phrases(n + 30, 30, 4, rng)[:n], np.tile(rng.integers(1, 60000, n // 8).astype(np.uint16), 8)]
+    T = [torch.from_numpy(np.concatenate([t, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16) for t in texts]
+    out = torch.zeros(5 * n + api.SA_PAD_BYTES, dtype=torch.uint8, device="cuda")
+    other = api.Context(0)                          # loads every kernel, so that a full device is not asked for that
+    for t in T:
+        api.build_sa(other, t, n, 8, out=out)
+    other.close()
+    ctx = api.Context(0)
+    filler = []
+    try:
+        ordinary = torch.randint(0, 60000, (n + api.TEXT_PAD,), device="cuda", dtype=torch.int32).to(torch.int16)
+        ordinary[n:] = 0
+        api.build_sa(ctx, ordinary.view(torch.uint16), n, 8, out=out)          # takes the buffers that every build of this length has
+        monkeypatch.setenv("CSA_DEBUG", "1")
+        torch.cuda.empty_cache()
+        free, _ = torch.cuda.mem_get_info()
+        need = 16 * n                                       # what the ranks take at least
+        if free > need // 2:
+            filler.append(torch.empty(free - need // 2, dtype=torch.uint8, device="cuda"))
+        capfd.readouterr()
+        api.build_sa(ctx, T[0], n, 8, out=out)
+        err = capfd.readouterr().err
+        with pytest.raises(api.CascadeError) as refused:
+            api.build_sa(ctx, T[1], n, 8, out=out)
+        assert refused.value.code == 3
+        api.build_sa(ctx, T[0], n, 8, out=out)
+        filler.clear()
+        torch.cuda.empty_cache()
+        v = api.validate_sa(ctx, T[0], n, out)
+        assert v["ok"], v
+        assert "are tied one symbol on" in err and "have a follower" not in err
+    finally:
+        ctx.close()
