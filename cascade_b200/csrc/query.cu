@@ -1043,14 +1043,25 @@ __global__ void __launch_bounds__(ANSWER_BLOCK) answers_kernel(const u8* __restr
     }
 }
 
-// The address by which the device reads and writes host memory, null for memory that is not pinned.
+// The address by which the device reads and writes `count` elements of host memory, null for memory that is not pinned to its end (a program may have
+// registered the pages of a part of it).
 template <typename T>
-T* pinned(T* host)
+T* pinned(T* host, const u64 count)
 {
-    cudaPointerAttributes attr;
-    const bool yes = host && cudaPointerGetAttributes(&attr, host) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-    cudaGetLastError();
-    return yes ? static_cast<T*>(attr.devicePointer) : nullptr;
+    auto device_address = [](const u8* at) -> u8*
+    {
+        cudaPointerAttributes attr;
+        const bool yes = cudaPointerGetAttributes(&attr, at) == cudaSuccess && attr.type == cudaMemoryTypeHost;
+        cudaGetLastError();
+        return yes ? static_cast<u8*>(attr.devicePointer) : nullptr;
+    };
+    if(!host || count == 0) return nullptr;
+    const u8* const at = reinterpret_cast<const u8*>(host);
+    u8* const first = device_address(at);
+    const u64 last = count * sizeof(T) - 1;
+    const bool one_page = ((reinterpret_cast<uintptr_t>(at) ^ (reinterpret_cast<uintptr_t>(at) + last)) >> 12) == 0;       // pages are pinned whole
+    if(!first || (!one_page && device_address(at + last) != first + last)) return nullptr;
+    return reinterpret_cast<T*>(first);
 }
 
 constexpr u64 STAGED_MAX = u64(1) << 20;        // bytes of a batch from or to pageable memory that are copied by way of pinned scratch
@@ -1065,10 +1076,11 @@ int query_host_small(csa_ctx* ctx, const csa_index* index, const u64* off_host, 
     const u64 symbols = off_host[q] - off_host[0];
     const u64 most = want_pos ? std::min(pos_capacity, q * max_pos) : 0;
     if(symbols && !sym_host) return CSA_OK;
-    const u64* off = pinned(const_cast<u64*>(off_host));
-    const u16* sym = symbols ? pinned(const_cast<u16*>(sym_host)) : nullptr;
-    Answers out{pinned(itv_host), want_pos ? pinned(cnt_host) : nullptr, want_pos ? pinned(pos_off_host) : nullptr, want_pos ? pinned(pos_host) : nullptr, pos_capacity,
-                ctx->h_scalars + CSA_STATUS_WORD};
+    u64* const pos = want_pos ? pinned(pos_host, most) : nullptr;
+    if(want_pos && !pos && most * 8 > STAGED_MAX) return CSA_OK;        // before the other buffers are asked for: a question takes microseconds of a pageable one
+    const u64* off = pinned(const_cast<u64*>(off_host), q + 1);
+    const u16* sym = pinned(const_cast<u16*>(sym_host), symbols);
+    Answers out{pinned(itv_host, 2 * q), want_pos ? pinned(cnt_host, q) : nullptr, want_pos ? pinned(pos_off_host, q + 1) : nullptr, pos, most, ctx->h_scalars + CSA_STATUS_WORD};
     // pinned scratch for what is not pinned
     const size_t b_off = off ? 0 : align_up256((q + 1) * 8), b_sym = sym || !symbols ? 0 : align_up256(symbols * 2), b_itv = out.itv ? 0 : align_up256(q * 16),
                  b_cnt = !want_pos || out.cnt ? 0 : align_up256(q * 4), b_poff = !want_pos || out.pos_off ? 0 : align_up256((q + 1) * 8),
@@ -1083,7 +1095,7 @@ int query_host_small(csa_ctx* ctx, const csa_index* index, const u64* off_host, 
     if(b_itv) { out.itv = reinterpret_cast<u64*>(p); p += b_itv; }
     if(b_cnt) { out.cnt = reinterpret_cast<u32*>(p); p += b_cnt; }
     if(b_poff) { out.pos_off = reinterpret_cast<u64*>(p); p += b_poff; }
-    if(b_pos) { out.pos = reinterpret_cast<u64*>(p); out.pos_capacity = most; }
+    if(b_pos) out.pos = reinterpret_cast<u64*>(p);
 
     const size_t d_itv = align_up256(q * 16), d_off = align_up256((q + 1) * 8), d_sym = align_up256(symbols * 2 + 16);
     void* ws = nullptr;

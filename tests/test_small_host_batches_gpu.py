@@ -79,3 +79,32 @@ def test_counts_alone_and_a_positions_buffer_that_is_too_small(ctx, oracle, pinn
     bad[0] = 1
     with pytest.raises(api.CascadeError):
         idx.query_host(bad, sym, 20)
+
+
+@pytest.mark.parametrize("what", ["off", "sym", "itv", "pos"])
+def test_buffers_of_which_only_the_first_page_is_pinned(ctx, oracle, what):
+    """Such a buffer is pageable memory: neither are its other pages read or written in place nor is the call refused."""
+    import mmap
+    T, sa, idx = _setup(ctx, oracle)
+    q, max_pos = 1000, 5
+    off, sym = _batch(T, q, 9)
+    sizes = {"off": (q + 1) * 8, "sym": len(sym) * 2, "itv": 2 * q * 8, "pos": q * max_pos * 8}
+    assert min(sizes.values()) > 4096
+    memory = mmap.mmap(-1, (sizes[what] + 4095) // 4096 * 4096)
+    buf = np.frombuffer(memory, dtype=np.uint16 if what == "sym" else np.uint64)[:sizes[what] // (2 if what == "sym" else 8)]
+    cudart = torch.cuda.cudart()
+    assert int(cudart.cudaHostRegister(buf.ctypes.data, 4096, 0)) == 0
+    try:
+        o, s, bufs = off, sym, {}
+        if what in ("off", "sym"):
+            buf[:] = off if what == "off" else sym
+            o, s = (buf, sym) if what == "off" else (off, buf)
+        else:
+            bufs = {what: buf}
+        itv, cnt, _, pos, total = idx.query_host(o, s, max_pos, bufs)
+        want = oracle.find_batch(T, sa, off, sym)
+        rows, counts = oracle.locate_batch(sa, want, max_pos)
+        assert np.array_equal(itv, want) and np.array_equal(cnt, counts) and total == int(counts.sum())
+        assert np.array_equal(pos[:total], np.concatenate([rows[i, :counts[i]] for i in range(q)]))
+    finally:
+        assert int(cudart.cudaHostUnregister(buf.ctypes.data)) == 0
