@@ -1,12 +1,12 @@
 // The suffix array of a text that one block holds in shared memory, in one launch. A build of a few thousand symbols by prefix_sort.cu's
-// kernels is launches and read-backs (3001 tokens: 60 us of kernels in a call of 119 us); this way a call takes 48 us, 8 of them in the kernel (10000
-// tokens: 123 and 61 us, 16384: 130 and 75 us).
+// kernels is launches and read-backs (3001 tokens: 60 us of kernels in a call of 107 us); this way a call takes 36 us, 15 of them in the kernel (8000
+// tokens: 108 and 44 us, 16000: 117 and 58 us).
 //
 // The symbols become their ranks among those that occur (a bit per symbol, and the bits before), so that nothing is as long as the alphabet. Every
 // suffix gets a number f that never falls from a suffix to a greater one and is nearly even over the text's suffixes: the arithmetic code of its first
 // symbols, from the exact counts, as far as 32 bits tell them apart. The suffixes are dealt into bins by f, a few bins for every suffix in short
 // texts and one in the longest; inside a bin they are ordered by f, and where that is the same, by the text itself. A text with many suffixes in one
-// bin, or with repeats that take long to compare, is left to the general build: nothing has been written then.
+// bin, or with repeats that would take long to compare, is left to the general build: nothing has been written then.
 #include "common.cuh"
 #include "tiny_build.cuh"
 
@@ -18,7 +18,9 @@ namespace
 constexpr int BLOCK = 1024, PER_MAX = int(TINY_BUILD_MAX / BLOCK);
 constexpr u32 CODE_SYMBOLS = 24;    // symbols that f looks at, at most
 constexpr u32 LONG_BIN = 64;        // suffixes of a bin at most
-constexpr u32 MOST_COMPARED = 512;  // symbols that a thread compares at most
+constexpr u32 MOST_PAIRS = 3u << 15;    // pairs of suffixes in one bin at most, of all bins: an even text has two a suffix. (16000 symbols of phrases that occur forty times, 33 a
+                                        // suffix: compared all the same 642 us, left to the general build 221.)
+constexpr u32 MOST_STEPS = 512, LEAST_STEPS = 32;       // of comparisons, four symbols each: what a warp may come to by what it has done, and from when on that is looked at
 constexpr int MAX_BIN_BITS = 14;
 
 constexpr u32 MAX = u32(TINY_BUILD_MAX);
@@ -52,6 +54,15 @@ __device__ __forceinline__ u32 exclusive(const u32 v, u32* warp_tot)
     return __reduce_add_sync(0xFFFFFFFFu, lane_id() < warp ? warp_tot[lane_id()] : 0u) + inc - v;
 }
 
+// A bit for each of four symbols, set where a and b differ. Behind the text there are symbols, too.
+__device__ __forceinline__ u32 differences(const u16* a, const u16* b)
+{
+    u32 differ = 0;
+    #pragma unroll
+    for(u32 j = 0; j < 4; ++j) differ |= a[j] != b[j] ? 1u << j : 0u;
+    return differ;
+}
+
 // One block; what bounds it is the chain of its steps and, near the longest text, their instructions.
 // bucket_bits: the statistics tell partitions by as many leading bits of f. result: pinned host memory.
 __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict__ text, const u32 n, u8* __restrict__ sa40, const u32 p, const int bucket_bits, const u64* __restrict__ status,
@@ -67,10 +78,11 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
     u16* const bits_before = reinterpret_cast<u16*>(bits + 2048);   // per word
     u16* const order = reinterpret_cast<u16*>(code);                // the array, once the code is no longer needed
     u32* const part = reinterpret_cast<u32*>(order + MAX);
+    u16* const further_ones = order + MAX;                          // before that: places in the bins of suffixes that are not told apart yet
     __shared__ u32 warp_tot[BLOCK / 32];
-    __shared__ u32 s_tied, s_partitions, s_most, s_symbols;
+    __shared__ u32 s_tied, s_partitions, s_most, s_symbols, s_pairs, s_further;
+    __shared__ volatile u32 s_left;
     const u32 tid = threadIdx.x, lane = lane_id();
-    const u32 per = (n + BLOCK - 1) / BLOCK;
     const int bin_bits = min(MAX_BIN_BITS, 34 - __clz(n));          // two to eight bins for every suffix, one in the longest texts
     const u32 bins = 1u << bin_bits;
 
@@ -78,13 +90,13 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
     if(tid < 512) reinterpret_cast<uint4*>(bits)[tid] = none;
     for(u32 i = tid; i < bins * 2 / 16 + 1; i += BLOCK) reinterpret_cast<uint4*>(start)[i] = none;
     for(u32 i = tid; i < (n + 3) / 4; i += BLOCK) reinterpret_cast<uint4*>(code)[i] = none;
-    if(tid == 0) { s_tied = 0; s_partitions = 0; s_most = 0; }
+    if(tid == 0) { s_tied = 0; s_partitions = 0; s_most = 0; s_pairs = 0; s_left = 0; s_further = 0; }
     for(u32 i = tid; i < (n + 7) / 8; i += BLOCK) reinterpret_cast<uint4*>(T)[i] = __ldg(reinterpret_cast<const uint4*>(text) + i);      // the text is padded
     __syncthreads();
     for(u32 i = tid; i < n; i += BLOCK)
     {
-        const u32 a = T[i];
-        atomicOr(bits + (a >> 5), 1u << (a & 31));
+        const u32 a = T[i], bit = 1u << (a & 31);
+        if((bits[a >> 5] & bit) == 0) atomicOr(bits + (a >> 5), bit);       // a frequent symbol's is there as a rule
     }
     __syncthreads();
     {
@@ -123,8 +135,8 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
     #pragma unroll
     for(int i = 0; i < PER_MAX; ++i)
     {
-        const u32 x = tid * per + i;
-        if(u32(i) >= per || x >= n) break;
+        const u32 x = tid + i * BLOCK;
+        if(x >= n) break;
         u32 low = 0, range = 0xFFFFFFFFu;
         for(u32 y = x, end = min(x + CODE_SYMBOLS, n); y < end && range >= 64; ++y)
         {
@@ -140,7 +152,7 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
     __syncthreads();
 
     // the bins' starts
-    u32 longest = 0, tied = 0;
+    u32 longest = 0, tied = 0, pairs = 0;
     {
         constexpr int WORDS = int(BINS_MAX) / 2 / BLOCK;
         const u32 each = max(1u, bins / 2 / BLOCK), first = tid * each;
@@ -153,6 +165,7 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
             const u32 a = c[k] & 0xFFFFu, b = c[k] >> 16;
             longest = __vmaxu2(longest, c[k]);
             tied += (a > 1 ? a : 0) + (b > 1 ? b : 0);
+            pairs += a * a + b * b;         // below 2^32, as all bins' suffixes together are below 2^15
             sum += a + b;
         }
         u32 run = exclusive(sum, warp_tot);
@@ -166,41 +179,86 @@ __global__ void __launch_bounds__(BLOCK) tiny_build_kernel(const u16* __restrict
         if(tid == 0) start[bins] = u16(n);
         tied = __reduce_add_sync(0xFFFFFFFFu, tied);
         if(lane == 0 && tied) atomicAdd(&s_tied, tied);
+        pairs = __reduce_add_sync(0xFFFFFFFFu, pairs);
+        if(lane == 0) atomicAdd(&s_pairs, pairs);
     }
-    bool left = __syncthreads_or(max(longest & 0xFFFFu, longest >> 16) > LONG_BIN);
+    bool left = __syncthreads_or(max(longest & 0xFFFFu, longest >> 16) > LONG_BIN) || s_pairs > MOST_PAIRS;
     if(!left)
     {
         #pragma unroll
         for(int i = 0; i < PER_MAX; ++i)
         {
-            const u32 x = tid * per + i;
-            if(u32(i) >= per || x >= n) break;
+            const u32 x = tid + i * BLOCK;
+            if(x >= n) break;
             rank[i] += start[f[i] >> (32 - bin_bits)];
             dealt[rank[i]] = u16(x);
             F[rank[i]] = f[i];
         }
         __syncthreads();
-        u32 compared = 0;
         #pragma unroll
         for(int i = 0; i < PER_MAX; ++i)
         {
-            const u32 x = tid * per + i;
-            if(u32(i) >= per || x >= n) break;
+            const u32 x = tid + i * BLOCK;
+            if(x >= n) break;
             const u32 b = f[i] >> (32 - bin_bits), s = start[b], e = start[b + 1];
             u32 place = s;
+            bool further = false;           // eight symbols do not tell
             for(u32 k = s; k < e; ++k)
             {
                 const u32 o = F[k];
                 place += o < f[i];
                 if(o != f[i] || k == rank[i]) continue;
                 const u32 y = dealt[k], room = n - max(x, y);
-                u32 l = 0;
-                while(l < room && compared < MOST_COMPARED && T[x + l] == T[y + l]) { ++l; ++compared; }
-                place += l < room ? T[y + l] < T[x + l] : y > x;            // the shorter suffix comes first
+                u32 differ = differences(T + x, T + y);
+                if(differ == 0 && room > 4) differ = differences(T + x + 4, T + y + 4) << 4;
+                const u32 l = differ ? __ffs(differ) - 1 : 8;
+                if(l >= room) place += y > x;               // the shorter suffix comes first
+                else if(differ) place += T[y + l] < T[x + l];
+                else further = true;
             }
-            order[place] = u16(x);
+            if(further) further_ones[atomicAdd(&s_further, 1u)] = u16(rank[i]);
+            else order[place] = u16(x);
         }
-        left = __syncthreads_or(compared >= MOST_COMPARED);
+        __syncthreads();
+        // The others, a thread to each wherever they stood: the lanes go through their bins and the comparisons side by side, so that they stay together.
+        u32 steps = 0, done = 0;
+        for(u32 first = tid - lane, count = s_further, rounds = (count - first + BLOCK - 1) / BLOCK; first < count; first += BLOCK, ++done)
+        {
+            const u32 q = first + lane;
+            u32 r = 0, x = 0, mine = 0, s = 0, e = 0;
+            if(q < count)
+            {
+                r = further_ones[q]; x = dealt[r]; mine = F[r];
+                const u32 b = mine >> (32 - bin_bits);
+                s = start[b]; e = start[b + 1];
+            }
+            u32 place = s;
+            for(u32 t = 0, most = __reduce_max_sync(0xFFFFFFFFu, e - s); t < most; ++t)
+            {
+                const u32 k = s + t;
+                u32 y = 0, room = 0, l = 0;
+                bool same = false;
+                if(k < e)
+                {
+                    const u32 o = F[k];
+                    place += o < mine;
+                    same = o == mine && k != r;
+                    if(same) { y = dealt[k]; room = n - max(x, y); }
+                }
+                while(__any_sync(0xFFFFFFFFu, same && s_left == 0))         // s_left: the whole block leaves it, what is written from here on is not used
+                {
+                    if(++steps >= LEAST_STEPS && steps * rounds * most > MOST_STEPS * (done * most + t + 1)) s_left = 1;
+                    if(!same) continue;
+                    const u32 differ = differences(T + x + l, T + y + l);
+                    l += differ ? __ffs(differ) - 1 : 4;
+                    same = differ == 0 && l < room;
+                    if(!same) place += l < room ? T[y + l] < T[x + l] : y > x;
+                }
+            }
+            if(q < count) order[place] = u16(x);
+        }
+        __syncthreads();
+        left = s_left != 0;
     }
     if(!left)
     {

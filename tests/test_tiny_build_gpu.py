@@ -67,3 +67,33 @@ def test_one_symbol_two_symbols_and_zeros_at_the_end(ctx, oracle, n):
     T[:] = np.arange(n) % 65536            # every symbol once, in order
     _check(ctx, oracle, T)
     _check(ctx, oracle, T[::-1])
+
+
+# which of them one launch makes; None: either way
+@pytest.mark.parametrize("n", [900, 3001, 16384])
+@pytest.mark.parametrize("kind,one", [("a passage twice", True), ("a short passage often", True), ("phrases of four symbols", None), ("phrases forty times", None), ("documents twenty times", None),
+                                      ("a period", False), ("two symbols in turn", False), ("zeros at the end of every document", False)])
+def test_repetitive_texts(ctx, oracle, n, kind, one):
+    """Pairs of suffixes in one bin and comparisons up to the limits and past them: what is given up is made by the general build, from the start."""
+    rng = np.random.default_rng(n)
+    T = rng.integers(1, 60000, n)
+    if kind == "a passage twice":
+        T[n // 2:n // 2 + 300] = T[10:310]
+    elif kind == "a short passage often":
+        for k in range(20):
+            T[k * (n // 20):k * (n // 20) + 12] = np.arange(12)
+    elif kind == "phrases of four symbols":
+        T = rng.integers(1, 60000, (n // 16, 4))[rng.integers(0, n // 16, n // 4 + 1)].reshape(-1)[:n]
+    elif kind == "phrases forty times":
+        T = rng.integers(1, 60000, (n // 200, 5))[rng.integers(0, n // 200, n // 5 + 1)].reshape(-1)[:n]
+    elif kind == "documents twenty times":
+        T = np.tile(T[:n // 20 + 1], 20)[:n]
+        T[rng.random(n) < 0.02] = 7
+    elif kind == "a period":
+        T = np.arange(n) % 9
+    elif kind == "two symbols in turn":
+        T = np.arange(n) % 2 * 65535
+    else:
+        T[np.arange(n) % 300 > 200] = 0
+    way = _check(ctx, oracle, T)
+    assert one is None or way == one
