@@ -61,10 +61,11 @@ constexpr u32 LARGE_STEPS = 12;
 // And only where ranks pay, which a sample tells: nearly all suffixes have a follower, or most have and many share more symbols than the text is compared for, which need ranks
 // anyway. Else most ties are settled by the text alone. ms a build of 4e8 suffixes, ranked and by text, in brackets the sample's two shares: phrases that occur four times, of 4 symbols
 // (0.51, 0) 47.9 and 31.1, of 8 (0.83, 0) 42.7 and 39.7, of 12 (0.89, 0) 42.3 and 42.6, of 30 (0.96, 0) 42.1 and 46.1; near-duplicates with 1.3 % of their symbols replaced (0.76, 0.27)
-// 84.7 and 100.6, with 2 % (0.67, 0.14) 115 and 99.
-bool ranks_pay(const Build_Counts& c)
+// 84.7 and 100.6, with 2 % (0.67, 0.14) 115 and 99. Up to 2^24 suffixes, whose ranks stay in L2, three quarters are enough: 1.2e7 suffixes, phrases of 4 symbols 1.44 and
+// 1.12 ms, of 7 (0.80, 0) 1.21 and 1.32.
+bool ranks_pay(const Build_Counts& c, const u64 n)
 {
-    return u64(c.lead_on) * 8 >= u64(c.looked_at) * 7 || (u64(c.lead_on) * 10 >= u64(c.looked_at) * 7 && u64(c.far_ties) * 5 >= c.looked_at);
+    return u64(c.lead_on) * 8 >= u64(c.looked_at) * (n <= (u64(1) << 24) ? 6 : 7) || (u64(c.lead_on) * 10 >= u64(c.looked_at) * 7 && u64(c.far_ties) * 5 >= c.looked_at);
 }
 
 int set_build_count(csa_ctx* ctx, u32* at, u32 value)
@@ -325,7 +326,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
         done = false;
         b.small = c.small;
         b.large = c.large;
-        bool rank = c.large <= c.small / LARGE_SHARE && ranks_pay(c);
+        bool rank = c.large <= c.small / LARGE_SHARE && ranks_pay(c, n);
         if(debug) std::fprintf(stderr, "[csa] of %u tied suffixes looked at %u are tied one symbol on, %u share %llu symbols: %s\n", c.looked_at, c.lead_on, c.far_ties, depth,
                                rank ? "ranked" : "compared in the text");
         if(rank)

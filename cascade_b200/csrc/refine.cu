@@ -326,16 +326,13 @@ __device__ __noinline__ void sample_ties(const u64* __restrict__ list, const u64
             const long long at = (long long)(k) - int(SMALL_GROUP) + c * 32 + int(lane_id());
             near[c] = at >= 0 && u64(at) < count && u64(at) != k ? __ldg(list + at) : ~e;
         }
-        // The group's keys tell its first `whole` symbols, the keys one symbol on are at their end with symbol `end`.
-        u32 first = 0, bits = 0, whole = 0, end = 0, before = 0;        // before: bits from symbol 1 up to symbol `whole`
-        for(bool told = false; end == 0 || bits - first < key_bits; ++end)
-        {
-            const u32 len = __ldg(code + symbol(x + end)) & 31u;
-            if(end == 0) first = len;
-            bits += len;
-            if(!told && bits > key_bits) { told = true; whole = end; before = bits - len - first; }
-        }
-        if(whole == 0) { whole = 1; before = 0; }
+        // The group's keys tell its first `whole` symbols, the keys one symbol on end before symbol `end`. A lane reads two code words, of a bit or more: a key has no more of them.
+        const u32 w0 = __ldg(code + symbol(x + lane_id())) & 31u, w1 = __ldg(code + symbol(x + 32 + lane_id())) & 31u;
+        const u32 to0 = warp_sum(w0), to1 = warp_sum(w1) + __shfl_sync(0xFFFFFFFFu, to0, 31), first = __shfl_sync(0xFFFFFFFFu, w0, 0);
+        auto symbols_upto = [&](const u32 bits) { return u32(__popc(__ballot_sync(0xFFFFFFFFu, to0 <= bits)) + __popc(__ballot_sync(0xFFFFFFFFu, to1 <= bits))); };
+        const u32 whole = max(1u, symbols_upto(key_bits)), end = symbols_upto(key_bits + first - 1) + 1;
+        const u32 last = whole - 1, upto0 = __shfl_sync(0xFFFFFFFFu, to0, last & 31), upto1 = __shfl_sync(0xFFFFFFFFu, to1, last & 31);
+        const u32 before = (last < 32 ? upto0 : upto1) - first;         // bits from symbol 1 up to symbol `whole`
         bool leaves = false, any = false;
         #pragma unroll
         for(int c = 0; c < PIECES; ++c)

@@ -20,7 +20,7 @@ int read_build_counts(csa_ctx* ctx, u64 most, Build_Counts& c);
 // A list of more than `most` entries is left alone; with the code given, about TIE_SAMPLE of its entries, spread over it, are looked at (counts->looked_at): those whose group
 // is still tied one symbol on (lead_on; about the share that launch_split_followed finds to have a follower), and those that another of their group ties with up to symbol
 // `to` (far_ties). isa (or null): every suffix's new rank goes there, too.
-constexpr u32 TIE_SAMPLE = 2048;
+constexpr u32 TIE_SAMPLE = 1024;
 int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, const u64* list, u64* next, u32* sa, u8* sa40, u32* isa, Build_Counts* counts, u64 expected, u64 most,
                           const u32* code = nullptr, int key_bits = 0);
 
