@@ -645,13 +645,6 @@ __device__ __forceinline__ u32 packed_place(const u32 place, const u32 head, con
     return place | (place == head ? size << 13 | PL_FIRST : head << 13) | (size == 1 ? 0u : (size <= SMALL_GROUP ? PL_SMALL : PL_LARGE));
 }
 
-// What bounds it is the issue of instructions (7 a record and warp, 68 % of the cycles), then barriers between dependent steps; memory is not (12 bytes a
-// record). So a block finds its children in two dependent reads (chunk_first, child_off), records stay with their threads and only keys are staged,
-// what only tied records need is skipped by warps without any, and three blocks of 512 threads with up to 8 records each share an SM (two such blocks
-// 4.70 ms a build of 2e8 tokens, three 4.67 and with shorter sums of the bins 4.55; blocks of 256 with 16 records, four to an SM, 5.51, with 8 records 4.75; every record staged
-// whole and looked up again by its place 5.17). A block reads its next chunk ahead.
-// MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
-// there if a block of 16 records a thread holds them, and to the front, for the radix sort, if not.
 // The batch's entries [base, base + m) as 5-byte ones, from shared memory: four are 20 bytes, which begin on a word where the first's slot is a multiple of
 // four; the words of 128 entries go out side by side by way of the warp's part of `words`. The up to three entries before and behind go byte by byte.
 template <int BLOCK, int CAP>
@@ -684,6 +677,13 @@ __device__ __forceinline__ void write_packed(u32* words, const u32* placed, cons
     }
 }
 
+// What bounds it is the issue of instructions (7 a record and warp, 68 % of the cycles), then barriers between dependent steps; memory is not (12 bytes a
+// record). So a block finds its children in two dependent reads (chunk_first, child_off), records stay with their threads and only keys are staged,
+// what only tied records need is skipped by warps without any, and three blocks of 512 threads with up to 8 records each share an SM (two such blocks
+// 4.70 ms a build of 2e8 tokens, three 4.67 and with shorter sums of the bins 4.55; blocks of 256 with 16 records, four to an SM, 5.51, with 8 records 4.75; every record staged
+// whole and looked up again by its place 5.17). A block reads its next chunk ahead.
+// MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
+// there if a block of 16 records a thread holds them, and to the front, for the radix sort, if not.
 // PACKED: the array is written to sa40 as 5-byte entries, else to sa.
 template <int BLOCK, int ITEMS, int BLOCKS, bool MEDIUM, bool PACKED>
 __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,

@@ -343,6 +343,9 @@ struct __align__(16) Slot_Query
 };
 static_assert(sizeof(Slot_Query) == 32, "one sector");
 constexpr u32 LONG_PATTERN = 0xFFFF;
+// Blocks of 128 threads an SM that the search of dealt queries leaves registers for: more reads in flight against spills (2 * 10^6 queries of 1 to 16 symbols on
+// 3 * 10^8 tokens, us a call: 8 blocks 624, 10 612, 12 626; of 2 to 4 symbols 565, 545 and 561).
+constexpr int FIND_DEALT_BLOCKS = 10;
 
 // Where a query falls in the directory, and which of its block's queries in that slot it is.
 struct Slot_Place { u16 first, last; u32 rank; };
@@ -454,11 +457,8 @@ __global__ void __launch_bounds__(SLOT_BLOCK) deal_slots_kernel(const u64* __res
         }
 }
 
-#ifndef FD_M
-#define FD_M 10
-#endif
-__global__ void __launch_bounds__(128, FD_M) find_dealt_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const Slot_Query* __restrict__ dealt, const u64 q,
-                                                        u64* __restrict__ itv)
+__global__ void __launch_bounds__(128, FIND_DEALT_BLOCKS) find_dealt_kernel(const csa_index idx, const u64* __restrict__ off, const u16* __restrict__ sym, const Slot_Query* __restrict__ dealt,
+                                                                           const u64 q, u64* __restrict__ itv)
 {
     const u64 t = u64(blockIdx.x) * 128 + threadIdx.x;
     if(t >= q) return;
@@ -985,7 +985,7 @@ struct Lane_Buffers
 //
 // Of a batch that a warp per query answers, copies, launches and waits take longer than the search. Here it is two launches and one wait: the answers
 // are written straight into pinned host memory, the positions of a query behind those of the queries before it, whose counts a block adds up by
-// itself. (50 queries: 89 us a call with five copies, six launches and two waits, this way 35 us; 1000: 111 and 41 us, 8000: 120 and 62 us.)
+// itself. (50 queries of up to 100 positions on 2^24 tokens: 88 us a call with five copies, six launches and two waits, this way 34 us; 1000: 92 and 43 us, 8000: 121 and 75 us.)
 constexpr int ANSWER_BLOCK = 256, ANSWER_QUERIES = 32;
 
 // What an answer goes to; cnt, pos_off and pos may be null together.
@@ -1051,9 +1051,8 @@ T* pinned(T* host, const u64 count)
     auto device_address = [](const u8* at) -> u8*
     {
         cudaPointerAttributes attr;
-        const bool yes = cudaPointerGetAttributes(&attr, at) == cudaSuccess && attr.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        return yes ? static_cast<u8*>(attr.devicePointer) : nullptr;
+        if(cudaPointerGetAttributes(&attr, at) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        return attr.type == cudaMemoryTypeHost ? static_cast<u8*>(attr.devicePointer) : nullptr;
     };
     if(!host || count == 0) return nullptr;
     const u8* const at = reinterpret_cast<const u8*>(host);
