@@ -7,6 +7,8 @@
 // counterpart there; it lists SA[lo + k] in rank order.
 #include "common.cuh"
 
+#include <cuda.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -1044,23 +1046,29 @@ __global__ void __launch_bounds__(ANSWER_BLOCK) answers_kernel(const u8* __restr
 }
 
 // The address by which the device reads and writes `count` elements of host memory, null for memory that is not pinned to its end (a program may have
-// registered the pages of a part of it).
+// registered the pages of a part of it). One question to the driver tells kind, address and range; the runtime's tells no range and takes as long.
 template <typename T>
 T* pinned(T* host, const u64 count)
 {
-    auto device_address = [](const u8* at) -> u8*
+    typedef CUresult (*Question)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Question ask = []() -> Question
     {
-        cudaPointerAttributes attr;
-        if(cudaPointerGetAttributes(&attr, at) != cudaSuccess) { cudaGetLastError(); return nullptr; }
-        return attr.type == cudaMemoryTypeHost ? static_cast<u8*>(attr.devicePointer) : nullptr;
-    };
-    if(!host || count == 0) return nullptr;
-    const u8* const at = reinterpret_cast<const u8*>(host);
-    u8* const first = device_address(at);
-    const u64 last = count * sizeof(T) - 1;
-    const bool one_page = ((reinterpret_cast<uintptr_t>(at) ^ (reinterpret_cast<uintptr_t>(at) + last)) >> 12) == 0;       // pages are pinned whole
-    if(!first || (!one_page && device_address(at + last) != first + last)) return nullptr;
-    return reinterpret_cast<T*>(first);
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if(cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &found) != cudaSuccess || found != cudaDriverEntryPointSuccess) { cudaGetLastError(); return nullptr; }
+        return reinterpret_cast<Question>(f);
+    }();
+    if(!host || count == 0 || !ask) return nullptr;
+    unsigned kind = 0, managed = 0;
+    CUdeviceptr address = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* answers[5] = {&kind, &managed, &address, &start, &size};
+    if(ask(5, what, answers, reinterpret_cast<CUdeviceptr>(host)) != CUDA_SUCCESS) return nullptr;
+    const u64 bytes = count * sizeof(T);
+    if(kind != CU_MEMORYTYPE_HOST || managed || address == 0 || address < start || address - start > size || size - (address - start) < bytes) return nullptr;
+    return reinterpret_cast<T*>(address);
 }
 
 constexpr u64 STAGED_MAX = u64(1) << 20;        // bytes of a batch from or to pageable memory that are copied by way of pinned scratch
