@@ -30,7 +30,12 @@ constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at m
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
 constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
-constexpr u32 LOCAL_CHUNK = 2048, SHORT_CHUNK = 1024;
+// The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
+constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
+constexpr int FREE_BITS = 4;                // of a key in a batch: its run of children has that many fewer bits than all of a parent's
+constexpr u32 SEGMENT = 64, SHORT_SEGMENT = 32;         // children whose batches one thread forms: they end with a segment
+constexpr u32 SHORT_BATCH = 1024;           // records of a batch of a text of one split, so that it has one for every SM
+constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
 
 // ---- the code ----------------------------------------------------------------------------------------------------------------
 
@@ -380,17 +385,80 @@ __global__ void __launch_bounds__(COUNT_BLOCK) count_long_text_kernel(const u16*
         if(cnt[i]) atomicAdd(&counts[i], cnt[i]);
 }
 
-// Child `next - 1` occupies the slots [r0, r1) of its parent: the chunks that begin behind its start begin with the next child.
-__device__ __forceinline__ void first_children(u32* __restrict__ chunk_first, const u32 chunks, const u32 chunk, const u32 r0, const u32 r1, const u32 next)
+// The batches of one parent, by a block of 1024 threads: off (shared memory) holds where its children start and where they end, from 0. A batch is a run of children of
+// one segment with up to `most` records, or a single one; its entry: the first slot, the records, the first child, the children. A child of more than
+// SORT_MOST goes to the other list. Whoever is called first ends its writes of off with a barrier.
+// A run of children of one parent in one word: there are up to 2^21 children, and 2^MAX_B2 of a parent.
+static_assert(MAX_B1 + 2 * MAX_B2 <= 32, "an entry is a word");
+__device__ __forceinline__ u32 children_entry(const u32 first, const u32 count) { return first << MAX_B2 | (count - 1); }
+
+struct Batch_Room { u32 used, at; u16 next[1 << MAX_B2]; u32 heads[(1 << MAX_B2) / 32]; };
+__device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, const u32 children, const u32 segment, const u32 most, const u32 first_slot, const u32 first_child,
+                                             uint4* __restrict__ batches, Build_Counts* __restrict__ counts, u32* __restrict__ over, u32* __restrict__ left)
 {
-    for(u32 k = r0 / chunk + 1; k <= r1 / chunk && k < chunks; ++k) chunk_first[k] = next;
+    const u32 tid = threadIdx.x;
+    if(tid < (1 << MAX_B2) / 32) room.heads[tid] = 0;
+    if(tid == 0) room.used = 0;
+    for(u32 i = tid; i < children; i += blockDim.x)
+    {
+        u32 a = i + 1, b = min(min(children, (i / segment + 1) * segment), i + max(1u, children >> FREE_BITS)) + 1;     // the last end with up to `most` records
+        while(b - a > 1)
+        {
+            const u32 m = (a + b) >> 1;
+            if(off[m] - off[i] <= most) a = m; else b = m;
+        }
+        room.next[i] = u16(a);
+    }
+    __syncthreads();
+    for(u32 s = tid; s * segment < children; s += blockDim.x)       // a segment's batches: whole words of bits
+    {
+        const u32 end = min(children, (s + 1) * segment);
+        for(u32 i = s * segment, w = i >> 5, bits = 0; i < end;)
+        {
+            if(i >> 5 != w) { room.heads[w] = bits; bits = 0; w = i >> 5; }
+            bits |= 1u << (i & 31u);
+            i = room.next[i];
+            if(i >= end || i >> 5 != w) room.heads[w] = bits;
+        }
+    }
+    __syncthreads();
+    u32 mine = 0;       // up to two children a thread: whether a batch begins there
+    #pragma unroll
+    for(int h = 0; h < 2; ++h)
+    {
+        const u32 i = tid + h * blockDim.x;
+        if(i >= children || !(room.heads[i >> 5] >> (i & 31u) & 1u)) continue;
+        const u32 m = off[room.next[i]] - off[i];
+        if(m > SORT_MOST || (m && children >> FREE_BITS == 0))
+        {
+            if(m <= MEDIUM_CAP) left[atomicAdd(&counts->medium, 1u)] = children_entry(first_child + i, 1);
+            else
+            {
+                over[atomicAdd(&counts->oversize, 1u)] = first_child + i;
+                atomicAdd(&counts->oversize_records, m);
+            }
+        }
+        else if(m) mine |= 1u << h;
+    }
+    u32 at = mine ? atomicAdd(&room.used, u32(__popc(mine))) : 0u;
+    __syncthreads();
+    if(tid == 0) room.at = atomicAdd(&counts->batches, room.used);
+    __syncthreads();
+    at += room.at;
+    #pragma unroll
+    for(int h = 0; h < 2; ++h)
+        if(mine >> h & 1u)
+        {
+            const u32 i = tid + h * blockDim.x, e = room.next[i];
+            batches[at++] = make_uint4(first_slot + off[i], off[e] - off[i], children_entry(first_child + i, e - i), 0);
+        }
 }
 
 // Offsets of the parents and the work lists that follow from their sizes. one_level: there is no second split, the bins are
 // the children of one parent that holds everything.
 __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restrict__ counts, const u32 bins, const u32 n, const int one_level, u32* __restrict__ cursor,
-                                                             u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ chunk0, u32* __restrict__ child_off, u32* __restrict__ chunk_first,
-                                                             const u32 p, Build_Counts* __restrict__ stats)
+                                                             u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ child_off,
+                                                             uint4* __restrict__ batches, u32* __restrict__ over, u32* __restrict__ left, const u32 p, Build_Counts* __restrict__ stats)
 {
     let_next_in();
     wait_for_previous();
@@ -410,17 +478,19 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
     if(formed) { atomicAdd(&stats->partitions, formed); atomicMax(&stats->max_partition, longest); }
     if(one_level)
     {
-        const u32 chunks = (n + SHORT_CHUNK - 1) / SHORT_CHUNK;
-        if(t < bins) { child_off[t] = off; first_children(chunk_first, chunks, SHORT_CHUNK, off, off + c, t + 1); }
-        if(t == 0) { child_off[bins] = n; chunk0[1] = chunks; chunk_first[0] = 0; chunk_first[chunks] = bins; }
+        __shared__ Batch_Room room;
+        __shared__ u32 s_off[(1 << MAX_B1) + 1];
+        if(t < bins) { child_off[t] = off; s_off[t] = off; }
+        if(t == 0) { child_off[bins] = n; s_off[bins] = n; }
+        __syncthreads();
+        form_batches(room, s_off, bins, SHORT_SEGMENT, SHORT_BATCH, 0, 0, batches, stats, over, left);
         return;
     }
-    const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE, chunks = (c + LOCAL_CHUNK - 1) / LOCAL_CHUNK;
-    u32 all_tiles, all_chunks;
+    const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE;
+    u32 all_tiles;
     const u32 t0 = block_exclusive<1024>(tiles, warp_tot, all_tiles);
-    const u32 c0 = block_exclusive<1024>(chunks, warp_tot, all_chunks);
-    if(t < bins) { par_off[t] = off; tile0[t] = t0; chunk0[t] = c0; }
-    if(t == 0) { par_off[bins] = n; tile0[bins] = all_tiles; chunk0[bins] = all_chunks; }
+    if(t < bins) { par_off[t] = off; tile0[t] = t0; }
+    if(t == 0) { par_off[bins] = n; tile0[bins] = all_tiles; }
 }
 
 template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<BLOCK>) * 8;
@@ -436,6 +506,7 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
                                                                           const int keep_top, const u32 first_bin, const u32 part_bins, u32* __restrict__ cursor,
                                                                           u64* __restrict__ out)
 {
+    let_next_in();
     wait_for_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);
@@ -540,24 +611,25 @@ __global__ void __launch_bounds__(SPLIT_BLOCK) count_children_kernel(const u64* 
         if(cnt[i]) atomicAdd(&counts[u64(p) * children + i], cnt[i]);
 }
 
-// One block per parent: the children's counts become their places (in counts, running) and their offsets (child_off).
+// One block per parent: the children's counts become their places (in counts, running) and their offsets (child_off), and batches of the local sort.
 __global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ counts, const u32* __restrict__ par_off, const u32 parents, const u32 children,
-                                                            u32* __restrict__ child_off, const u32* __restrict__ chunk0, u32* __restrict__ chunk_first)
+                                                            u32* __restrict__ child_off, uint4* __restrict__ batches, u32* __restrict__ over, u32* __restrict__ left, Build_Counts* __restrict__ stats)
 {
     __shared__ u32 warp_tot[32];
+    __shared__ u32 s_off[(1 << MAX_B2) + 1];
+    __shared__ Batch_Room room;
     const u32 p = blockIdx.x, t = threadIdx.x;
     u32* const c = counts + u64(p) * children;
     const u32 i0 = 2 * t, i1 = 2 * t + 1;          // up to 2048 children
     const u32 a = i0 < children ? c[i0] : 0, b = i1 < children ? c[i1] : 0;
     u32 total;
     const u32 rel = block_exclusive<1024>(a + b, warp_tot, total), off = par_off[p] + rel;
-    const u32 chunks = chunk0[p + 1] - chunk0[p];
-    if(i0 < children) first_children(chunk_first + chunk0[p], chunks, LOCAL_CHUNK, rel, rel + a, p * children + i0 + 1);
-    if(i1 < children) first_children(chunk_first + chunk0[p], chunks, LOCAL_CHUNK, rel + a, rel + a + b, p * children + i1 + 1);
-    if(t == 0 && chunks) chunk_first[chunk0[p]] = p * children;
-    if(i0 < children) { c[i0] = off; child_off[u64(p) * children + i0] = off; }
-    if(i1 < children) { c[i1] = off + a; child_off[u64(p) * children + i1] = off + a; }
-    if(p == parents - 1 && t == 0) { child_off[u64(parents) * children] = par_off[parents]; chunk_first[chunk0[parents]] = parents * children; }
+    if(i0 < children) { c[i0] = off; child_off[u64(p) * children + i0] = off; s_off[i0] = rel; }
+    if(i1 < children) { c[i1] = off + a; child_off[u64(p) * children + i1] = off + a; s_off[i1] = rel + a; }
+    if(t == 0) s_off[children] = total;
+    if(p == parents - 1 && t == 0) child_off[u64(parents) * children] = par_off[parents];
+    __syncthreads();
+    form_batches(room, s_off, children, SEGMENT, SORT_MOST, par_off[p], p * children, batches, stats, over, left);
 }
 
 constexpr size_t SPLIT_SMEM = size_t(SPLIT_TILE) * 8;
@@ -630,8 +702,625 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
 
 // ---- local sort: runs of children in shared memory --------------------------------------------------------------------------------
 
+constexpr u32 TIE_ROOM = 1024;              // tied records that a block keeps before it writes them to the list
+constexpr u32 MOST_CROWDED = 64;            // crowded bins of a batch
+// A word holds the counts of four bins, five bits each, and later where the word's records begin (12 bits) and, in the fields, where those of each bin do.
+constexpr u32 BIN_BITS = 5, BIN_MASK = (1u << BIN_BITS) - 1, START_BIT = 4 * BIN_BITS;
+constexpr u32 each_bin(const u32 v) { return v | v << BIN_BITS | v << 2 * BIN_BITS | v << 3 * BIN_BITS; }
+constexpr u32 SUMS = each_bin(1) << BIN_BITS;               // times a word of counts: the sums of the counts before each, and of all
+constexpr u32 SUMS_BEFORE = each_bin(BIN_MASK) & ~BIN_MASK, SUM_OF_ALL = BIN_MASK << START_BIT;
+constexpr u32 WINDOW_BIN = 4;               // records of the largest bin that a thread's window orders
+constexpr u32 TO_EIGHT = each_bin(8 - WINDOW_BIN - 1), EIGHT_UP = each_bin(24);     // a count above WINDOW_BIN, the first added, has bits of the second
+constexpr u32 FULL_BIN = each_bin(16);      // bits of a count from 16 on
+static_assert(SORT_CAP <= 1 << (32 - START_BIT), "a slot takes 12 bits");
+template <bool PACKED> constexpr size_t SORT_SMEM = (3 * SORT_CAP + 40) * 4 + TIE_ROOM * 8 + (PACKED ? SORT_BLOCK / 32 * 640 : 0);
+
+__device__ __forceinline__ void order(u32& a, u32& b) { const u32 t = min(a, b); b = max(a, b); a = t; }
+__device__ __forceinline__ void order(u32& a, u32& b, u32& c) { order(a, b); order(b, c); order(a, b); }
+
+// A batch goes through four steps with a barrier behind each:
+//   * every record is counted in a bin, its key's place in the batch's range of keys by interpolation (two bins to a record), and keeps its number in the bin;
+//   * the bins' counts become their starts;
+//   * key and position go to the record's slot in shared memory. The keys are in order now but for bins with several records, most of which hold two to four;
+//   * a thread orders the keys of four slots with those of the three slots before and behind, in registers: a bin of up to four records lies inside the window of every
+//     slot of it. A key carries its slot's last four bits in bits that it does not need, so min and max move whole records, and no two are equal. The four entries go out
+//     as one 16-byte store: the batch's slots begin with the first slot's place in its group of four.
+// The one or two larger bins of a batch, of up to 15 records, are ordered by a warp each. Batches with a bin of 16 or more (texts with long repeats), with crowded bins all over or
+// with too many tied records are left to crowded_batches_kernel where records of one key are many, to left_children_kernel else.
+// What bounds it: the issue of instructions (110 for 32 records, 59 % of the cycles) and the latency of dependent steps between barriers; so records stay in registers, no slow path is
+// unrolled, a block's next records and the batch after them are on their way early, and 256 threads with 16 records each share what a warp does per batch among more records than 512
+// with 8 do. A Zipf text of 1.25e8 symbols, the kernel alone: 0.66 ms; 512 threads with 8 records, two blocks an SM 0.78 and three (40 registers, spills) 1.0; two blocks of 256
+// 0.74; all keys of a bin compared with one another and every record placed by its rank (226 instructions) 1.14. Room for 2048 tied records instead of 1024 leaves L1 too small for
+// the registers that spill: 1 % of a build.
+// PACKED: the array is written to sa40 as 5-byte entries, else to sa.
+template <bool PACKED>
+__global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const uint4* __restrict__ batches, const int bits, u32* __restrict__ sa,
+                                                                             u8* __restrict__ sa40, u64* __restrict__ list, Build_Counts* __restrict__ counts, u32* __restrict__ over,
+                                                                             const u32 over_cap, u32* __restrict__ left)
+{
+    constexpr u32 BLOCK = SORT_BLOCK, ITEMS = SORT_ITEMS, CAP = SORT_CAP, WARPS = BLOCK / 32, WORDS = CAP / 2 / BLOCK, CROWD_WORDS = CAP / 32 + 4;
+    static_assert(WORDS % 4 == 0 && ITEMS % 8 == 0 && CROWD_WORDS <= BLOCK, "whole 16-byte pieces of bins, whole words of numbers, a word of marks a thread");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u32* const keys = reinterpret_cast<u32*>(smem_raw) + 4;     // [CAP + 16] in the order of the bins; four words before it
+    u32* const pos = keys + CAP + 20;                           // [CAP + 16] the positions beside them; four words before it
+    u32* const bins = pos + CAP + 16;                           // [2][CAP / 2]: of every other batch
+    u64* const tie = reinterpret_cast<u64*>(bins + CAP);        // [TIE_ROOM]
+    u32* const words = reinterpret_cast<u32*>(tie + TIE_ROOM) + (threadIdx.x >> 5) * 160;       // PACKED: a warp's entries
+    __shared__ u32 warp_tot[WARPS];
+    __shared__ u32 crowd[CROWD_WORDS];              // a bit per slot: it belongs to a crowded bin
+    __shared__ u32 crowded[MOST_CROWDED];           // such a bin's first slot and its size
+    __shared__ u32 s_crowded, s_fall[2], s_ties, s_slot;
+    __shared__ u32 s_copies;                        // the batch was left for its many records of each key
+    __shared__ u32 s_before;                        // the children of the batch before
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    let_next_in();
+    wait_for_previous();
+    const u32 works = counts->batches;
+    if(blockIdx.x >= works) return;
+
+    u32 k[ITEMS], p[ITEMS];
+    u32 full = 0, rest = 0;             // rows of the batch that have a record for every thread, and records behind them
+    auto for_each = [&](auto&& f)
+    {
+        #pragma unroll
+        for(u32 i = 0; i < ITEMS - 1; ++i)
+        {
+            if(i >= full) break;
+            f(i);
+        }
+        if(tid < rest) f(ITEMS - 1);
+    };
+    auto load = [&](const uint4& batch)
+    {
+        full = __shfl_sync(0xFFFFFFFFu, batch.y / BLOCK, 0);
+        rest = batch.y % BLOCK;
+        const u64* const at = rec + batch.x + tid;
+        #pragma unroll
+        for(u32 i = 0; i < ITEMS - 1; ++i)
+        {
+            if(i >= full) break;
+            const u64 v = at[i * BLOCK];
+            k[i] = u32(v >> 32); p[i] = u32(v);
+        }
+        if(tid < rest) { const u64 v = at[full * BLOCK]; k[ITEMS - 1] = u32(v >> 32); p[ITEMS - 1] = u32(v); }
+    };
+    auto leave_crowded = [&](const u32 children) { over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children; };      // by one thread
+    auto put = [&](const u32 slot, const u32 v)
+    {
+        if(!PACKED) { sa[slot] = v; return; }
+        u8* const b = sa40 + 5 * u64(slot);
+        b[0] = u8(v); b[1] = u8(v >> 8); b[2] = u8(v >> 16); b[3] = u8(v >> 24); b[4] = 0;
+    };
+
+    uint4 now = __ldg(batches + blockIdx.x), then = make_uint4(0, 0, 0, 0);
+    u32 next = blockIdx.x + gridDim.x, fell = 0;        // fell: batches in a row that were left
+    if(next < works) then = __ldg(batches + next);
+    load(now);
+    for(u32 i = tid; i < CAP / 4; i += BLOCK) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
+    if(tid < 4) keys[int(tid) - 4] = 0;
+    if(tid == 0) { s_fall[0] = 0; s_ties = 0; }
+    u32 turn = 0, kept = 0;             // kept: tied records in `tie` from before the batch
+    __syncthreads();
+    while(true)
+    {
+        const u32 base = now.x, m = now.y, shift = base & 3u, end = shift + m;      // the batch's records take the slots [shift, end)
+        const u32 whole = base - shift;
+        u32* const bin = bins + turn * (CAP / 2);
+        {
+            // keys from the start of the batch's range, which is cut to a power of two: FREE_BITS bits at the end are free
+            const u32 others = now.z & ((1u << MAX_B2) - 1), low = (now.z >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits);
+            const int up = bits - (32 - __clz(others));
+            for_each([&](const u32 i) { k[i] = (k[i] - low) << up; });
+        }
+        u32 seen = 0, number[ITEMS / 8] = {};       // the records' numbers in their bins, four bits each
+        for_each([&](const u32 i)
+        {
+            const u32 b = __umulhi(k[i], 2 * m), old = atomicAdd(bin + (b >> 2), 1u << (BIN_BITS * (b & 3u)));
+            seen |= old;
+            number[i / 8] |= (old >> (BIN_BITS * (b & 3u)) & 15u) << (4 * (i % 8));
+        });
+        if(seen & FULL_BIN) s_fall[turn] = 1;       // before a count runs into the next
+        __syncthreads();
+
+        const bool any = 2 * WORDS * tid < m;       // the thread has bins, its warp has
+        const bool busy = 64 * WORDS * warp < m;
+        u32 c[WORDS], sum = 0, inc = 0, many = 0;
+        if(busy)
+        {
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; w += 4)
+            {
+                const uint4 v = any ? *reinterpret_cast<const uint4*>(bin + WORDS * tid + w) : make_uint4(0, 0, 0, 0);
+                c[w] = v.x; c[w + 1] = v.y; c[w + 2] = v.z; c[w + 3] = v.w;
+            }
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; ++w)
+            {
+                many |= (c[w] + TO_EIGHT) & EIGHT_UP;
+                sum += c[w] * SUMS & SUM_OF_ALL;
+            }
+            inc = warp_inclusive(sum);
+        }
+        if(lane == 31) warp_tot[warp] = inc;
+        // what the batch before has left: its marks, and its ties where the next might find no room for its own
+        #pragma unroll
+        for(u32 w = 0; w < WORDS; w += 4) reinterpret_cast<uint4*>(bins + (turn ^ 1) * (CAP / 2))[tid + w / 4 * BLOCK] = make_uint4(0, 0, 0, 0);
+        if(tid < CROWD_WORDS) crowd[tid] = 0;
+        const bool crammed = s_ties > TIE_ROOM;             // left to the other kernel after all
+        const u32 ties = crammed ? kept : s_ties;
+        const bool write = ties != 0 && (crammed || ties + max(TIE_ROOM / 4, 2 * (ties - kept)) > TIE_ROOM);
+        if(tid == 0)
+        {
+            s_crowded = 0;
+            s_fall[turn ^ 1] = 0;
+            if(crammed) leave_crowded(s_before);
+            s_before = now.z;
+            if(write) s_slot = atomicAdd(&counts->small, ties);
+        }
+        __syncthreads();
+        if(16 * tid < then.y) asm volatile("prefetch.global.L2 [%0];" :: "l"(rec + then.x + 16 * tid));
+        if(busy)
+        {
+            u32 run = (shift << START_BIT) + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_tot[lane] : 0u) + inc - sum;
+            if(any)
+            {
+                #pragma unroll
+                for(u32 w = 0; w < WORDS; w += 4)
+                {
+                    uint4 v;
+                    v.x = (c[w] * SUMS & SUMS_BEFORE) | run; run += c[w] * SUMS & SUM_OF_ALL;
+                    v.y = (c[w + 1] * SUMS & SUMS_BEFORE) | run; run += c[w + 1] * SUMS & SUM_OF_ALL;
+                    v.z = (c[w + 2] * SUMS & SUMS_BEFORE) | run; run += c[w + 2] * SUMS & SUM_OF_ALL;
+                    v.w = (c[w + 3] * SUMS & SUMS_BEFORE) | run; run += c[w + 3] * SUMS & SUM_OF_ALL;
+                    *reinterpret_cast<uint4*>(bin + WORDS * tid + w) = v;
+                }
+            }
+            if(many)
+            {
+                #pragma unroll
+                for(u32 w = 0; w < WORDS; ++w)
+                    #pragma unroll 1
+                    for(u32 f = (c[w] + TO_EIGHT) & EIGHT_UP; f;)
+                    {
+                        const u32 bit = (__ffs(f) - 1) / BIN_BITS * BIN_BITS, size = c[w] >> bit & BIN_MASK, v = bin[WORDS * tid + w];
+                        const u32 at = (v >> START_BIT) + (v >> bit & BIN_MASK), o = atomicAdd(&s_crowded, 1u);
+                        f &= ~(BIN_MASK << bit);
+                        if(o < MOST_CROWDED) crowded[o] = at | size << 16;
+                        const u64 marks = u64((1u << size) - 1) << (at & 31u);
+                        atomicOr(&crowd[at >> 5], u32(marks));
+                        if(marks >> 32) atomicOr(&crowd[(at >> 5) + 1], u32(marks >> 32));
+                        u32 all = 0;
+                        for(int b = 0; b < 4; ++b) all += c[w] >> (BIN_BITS * b) & BIN_MASK;
+                        if(o >= MOST_CROWDED || (c[w] & FULL_BIN) || all > BIN_MASK) s_fall[turn] = 1;
+                    }
+            }
+        }
+        if(write)
+            #pragma unroll 1
+            for(u32 j = tid; j < ties; j += BLOCK) list[u64(s_slot) + j] = tie[j];
+        kept = write ? 0 : ties;
+        __syncthreads();
+
+        const bool fall = s_fall[turn] != 0;
+        if(tid == 0 && (write || crammed)) s_ties = kept;
+        if(!fall)
+        {
+            for_each([&](const u32 i)
+            {
+                const u32 b = __umulhi(k[i], 2 * m), v = bin[b >> 2], slot = (v >> START_BIT) + (v >> (BIN_BITS * (b & 3u)) & BIN_MASK) + (number[i / 8] >> (4 * (i % 8)) & 15u);
+                keys[slot] = k[i] | (slot & 15u);
+                pos[slot] = p[i];
+            });
+            if(tid < shift) keys[tid] = 0;                      // no key is below, or above those behind
+            if(tid < 8) keys[end + tid] = 0xFFFFFFFFu;
+        }
+        else if(warp == 0)
+        {
+            // many records of each key, or many keys close together: of 32 records of the batch, four times, do any have the same key?
+            bool twins = false;
+            #pragma unroll
+            for(u32 i = 0; i < 4; ++i)
+                if(i < full) twins |= __popc(__match_any_sync(0xFFFFFFFFu, k[i])) > 1;
+            const bool copies = __any_sync(0xFFFFFFFFu, twins);
+            if(lane == 0)
+            {
+                s_copies = copies;
+                if(copies) leave_crowded(now.z); else left[atomicAdd(&counts->medium, 1u)] = now.z;
+            }
+        }
+        __syncthreads();
+
+        if(next < works) load(then);            // on their way while the batch is ordered
+        if(!fall)
+        {
+            const u32 crowds = s_crowded;
+            #pragma unroll 1
+            for(u32 q0 = warp * 32; 4 * q0 < end; q0 += BLOCK)
+            {
+                const u32 q = q0 + lane, window = 4 * q - 3;
+                const uint4* const K = reinterpret_cast<const uint4*>(keys - 4) + q;
+                const uint4 L = K[0], O = K[1], R = K[2];
+                u32 a0 = L.y, a1 = L.z, a2 = L.w, x0 = O.x, x1 = O.y, x2 = O.z, x3 = O.w, r0 = R.x, r1 = R.y, r2 = R.z;
+                order(x0, x1); order(x2, x3); order(x0, x2); order(x1, x3); order(x1, x2);
+                order(a0, a1, a2);
+                order(r0, r1, r2);
+                const u32 before = max(max(min(a0, x2), min(a1, x1)), min(a2, x0));        // the key at the place before the four, and the one behind them
+                x2 = max(a0, x2); x1 = max(a1, x1); x0 = max(a2, x0);
+                order(x0, x1, x2);
+                const u32 behind = min(min(max(x1, r2), max(x2, r1)), max(x3, r0));
+                x1 = min(x1, r2); x2 = min(x2, r1); x3 = min(x3, r0);
+                order(x1, x2, x3);
+                const u32* const at = pos + 4 * q - 3;
+                u32 v[4] = {at[(x0 - window) & 15u], at[(x1 - window) & 15u], at[(x2 - window) & 15u], at[(x3 - window) & 15u]};
+                u32 wanted = 4 * q < end ? 15u : 0u;            // a bit per entry: it is the batch's, and of no crowded bin
+                if(4 * q < shift) wanted = 15u << shift & 15u;
+                if(4 * q + 4 > end && wanted) wanted &= 15u >> (4 * q + 4 - end);
+                if(crowds) wanted &= ~(crowd[q >> 3] >> (4 * (q & 7u)));
+                const u32 x[6] = {before, x0, x1, x2, x3, behind};
+                bool tied = min(min(min(before ^ x0, x0 ^ x1), min(x1 ^ x2, x2 ^ x3)), x3 ^ behind) < 16;
+                if(tied && wanted != 15u)       // the words around the batch are alike
+                {
+                    tied = false;
+                    #pragma unroll
+                    for(u32 i = 0; i < 4; ++i)
+                        tied |= (wanted >> i & 1u) && (((x[i] ^ x[i + 1]) < 16 && 4 * q + i > shift) || ((x[i + 1] ^ x[i + 2]) < 16 && 4 * q + i + 1 < end));
+                }
+                if(tied)
+                {
+                    #pragma unroll
+                    for(u32 i = 0; i < 4; ++i)
+                    {
+                        if(!(wanted >> i & 1u) || ((x[i] ^ x[i + 1]) >= 16 && (x[i + 1] ^ x[i + 2]) >= 16)) continue;
+                        const u32 first = max(4 * q + i, shift + 3) - 3, stop = min(4 * q + i + 4, end);
+                        u32 smaller = 0, group = 0;
+                        #pragma unroll 1
+                        for(u32 s = first; s < stop; ++s)
+                            if((keys[s] ^ x[i + 1]) < 16) { ++group; smaller += keys[s] < x[i + 1]; }
+                        if(group <= 1) continue;
+                        v[i] = SA_OPEN;
+                        if(smaller) continue;            // the first of a group writes it
+                        u32 o = atomicAdd(&s_ties, group);
+                        if(o + group > TIE_ROOM) continue;
+                        #pragma unroll 1
+                        for(u32 s = first; s < stop; ++s)
+                            if((keys[s] ^ x[i + 1]) < 16) tie[o++] = u64(whole + 4 * q + i) << 32 | pos[s];
+                    }
+                }
+                if(!PACKED)
+                {
+                    u32* const to = sa + whole + 4 * q;
+                    if(wanted == 15u) *reinterpret_cast<uint4*>(to) = make_uint4(v[0], v[1], v[2], v[3]);
+                    else
+                        #pragma unroll
+                        for(u32 i = 0; i < 4; ++i)
+                            if(wanted >> i & 1u) to[i] = v[i];
+                }
+                else
+                {
+                    // four entries are 20 bytes, and begin on a word: the words of the warp's go out side by side
+                    u32* const w = words + 5 * lane;
+                    w[0] = v[0]; w[1] = v[1] << 8; w[2] = v[1] >> 24 | v[2] << 16; w[3] = v[2] >> 16 | v[3] << 24; w[4] = v[3] >> 8;
+                    const u32 all_four = __ballot_sync(0xFFFFFFFFu, wanted == 15u);
+                    __syncwarp();
+                    u32* const to = reinterpret_cast<u32*>(sa40) + u64(whole / 4 + q0) * 5;
+                    #pragma unroll
+                    for(u32 j = lane; j < 160; j += 32)
+                        if(all_four >> (j / 5) & 1u) to[j] = words[j];
+                    if(wanted != 15u)
+                        #pragma unroll
+                        for(u32 i = 0; i < 4; ++i)
+                            if(wanted >> i & 1u) put(whole + 4 * q + i, v[i]);
+                    __syncwarp();
+                }
+            }
+            #pragma unroll 1
+            for(u32 o = WARPS - 1 - warp; o < crowds; o += WARPS)       // the last warps have the fewest windows
+            {
+                const u32 s = crowded[o] & 0xFFFFu, size = crowded[o] >> 16;
+                const bool mine = lane < size;
+                const u32 key = mine ? keys[s + lane] >> FREE_BITS : ~0u, at = mine ? pos[s + lane] : 0u;
+                u32 less = 0, equal = 0;
+                #pragma unroll 4
+                for(u32 j = 0; j < 16; ++j)
+                {
+                    const u32 other = __shfl_sync(0xFFFFFFFFu, key, j);
+                    less += other < key;
+                    equal |= u32(other == key) << j;
+                }
+                const u32 before = __popc(equal & ((1u << lane) - 1u)), group = __popc(equal);
+                u32 to = 0;
+                if(mine && group > 1 && before == 0) to = atomicAdd(&s_ties, group);
+                to = __shfl_sync(0xFFFFFFFFu, to, max(__ffs(equal), 1) - 1);
+                if(mine)
+                {
+                    const u32 head = whole + s + less;
+                    put(head + before, group > 1 ? SA_OPEN : at);
+                    if(group > 1 && to + group <= TIE_ROOM) tie[to + before] = u64(head) << 32 | at;
+                }
+            }
+        }
+        if(next >= works) break;
+        now = then;
+        // where one batch after the other is left, only one in eight is tried
+        fell = (fall && s_copies) || crammed ? fell + 1 : 0;
+        const u32 jump = fell < 2 ? 1u : 8u, passed = next + (tid + 1) * gridDim.x;
+        if(tid + 1 < jump && passed < works) leave_crowded(__ldg(&batches[passed].z));
+        next += jump * gridDim.x;
+        then.y = 0;
+        if(next < works) then = __ldg(batches + next);
+        turn ^= 1;
+    }
+    __syncthreads();
+    const bool crammed = s_ties > TIE_ROOM;
+    const u32 ties = crammed ? kept : s_ties;
+    if(tid == 0)
+    {
+        if(crammed) leave_crowded(now.z);
+        if(ties) s_slot = atomicAdd(&counts->small, ties);
+    }
+    __syncthreads();
+    #pragma unroll 1
+    for(u32 j = tid; j < ties; j += BLOCK) list[u64(s_slot) + j] = tie[j];
+}
+
+// ---- crowded batches ------------------------------------------------------------------------------------------------------------------
+
+constexpr u32 CROWD_BLOCK = 256, CROWD_ITEMS = 16, CROWD_CAP = CROWD_BLOCK * CROWD_ITEMS;
+constexpr u32 MOST_ROUNDS = 16;             // a bin with more keys: the batch goes on to the kernel behind this one
+constexpr size_t CROWD_SMEM = size_t(CROWD_CAP) * (4 + 2 * 5 + 4);
+static_assert(CROWD_CAP > SORT_MOST && CROWD_CAP <= 4096, "a record's number in its batch takes 12 bits, with two flags and one pattern to spare in 16");
+
+// Batches in which many records have the same key (near-duplicate documents: some fifty a key). A key is ordered once, however many records have it: each round, the records that have
+// no key yet write themselves into their bin of the interpolation; the one that stands there then brings its key, and those of the same key are counted for it and numbered. One round does
+// for all but a few records as a rule; those left over go on as a list. The keys of a bin, one a round, are a list too: a key's place is behind the smaller ones of its list and the bins before, and a
+// record's is its key's and its number.
+// Bound by the issue of instructions (178 for 32 records) and the latency of its steps: 0.54 ms for 6e7 near-duplicate suffixes where the kernel that compares all records of a bin takes 1.9 ms (the build of
+// 4e8 of them 60.5 -> 52.6 ms).
+template <bool PACKED>
+__global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u64* __restrict__ rec, const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u8* __restrict__ sa40,
+                                                                         u64* __restrict__ list, const u64 list_cap, Build_Counts* __restrict__ counts, const u32* __restrict__ over,
+                                                                         const u32 over_cap, u32* __restrict__ left)
+{
+    constexpr u32 BLOCK = CROWD_BLOCK, ITEMS = CROWD_ITEMS, CAP = CROWD_CAP, WORDS = CAP / 2 / BLOCK, NONE = 0xFFFFu, SETTLED = 1u << 12, WON = 1u << 13, RECORD = SETTLED - 1;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u32* const keys = reinterpret_cast<u32*>(smem_raw);                 // [CAP] of the records; then positions of tied ones
+    u32* const res = keys + CAP;                                        // [CAP] place of the key that the record brought; of a record of the list: its key's record and its number << 16, or
+                                                                        // its key's place, its number << 16 and bit 31 where it brought the key
+    u32* const bin = res + CAP;                                         // [CAP / 2] two 16-bit counts a word: records of each bin, then the bins' starts
+    u16* const start = reinterpret_cast<u16*>(bin);                     // at first who stands in the bin
+    u16* const head = start + CAP;                                      // [CAP] the last key of every bin's list, by its record
+    u32* const heads = bin;                                             // [CAP] both, when they are done with: first slots of tied records
+    u32* const cnt2 = bin + CAP;                                        // [CAP / 2] two 16-bit counts a word: records of each key
+    u16* const cnt = reinterpret_cast<u16*>(cnt2);
+    u16* const link = cnt + CAP;                                        // [CAP] the key before it in its list; then where its records go among the tied ones
+    u16* const lines = link + CAP;                                      // [CAP] records without a key after the first round, from the front; those that brought one in it, from the back
+    __shared__ u32 warp_tot[BLOCK / 32];
+    __shared__ u32 s_lines, s_tied[2], s_slot[2];
+    const u32 tid = threadIdx.x, lane = lane_id();
+    auto put = [&](const u32 slot, const u32 v)
+    {
+        if(!PACKED) { sa[slot] = v; return; }
+        u8* const b = sa40 + 5 * u64(slot);
+        b[0] = u8(v); b[1] = u8(v >> 8); b[2] = u8(v >> 16); b[3] = u8(v >> 24); b[4] = 0;
+    };
+    let_next_in();
+    wait_for_previous();
+    const u32 works = counts->crowded;
+    if(blockIdx.x >= works) return;
+    // the batch and the one after it, whose records are on their way while the one before is finished
+    u32 entry = over[over_cap - 1 - blockIdx.x], next_entry = 0, next_base = 0, next_end = 0;
+    u32 base = __ldg(child_off + (entry >> MAX_B2)), m = __ldg(child_off + (entry >> MAX_B2) + (entry & ((1u << MAX_B2) - 1)) + 1) - base;
+    u32 k[ITEMS], p[ITEMS];
+    auto load = [&]()
+    {
+        #pragma unroll
+        for(u32 i = 0; i < ITEMS; ++i)
+        {
+            if(i * BLOCK >= m) break;
+            const u32 j = tid + i * BLOCK;
+            if(j < m) { const u64 v = rec[base + j]; k[i] = u32(v >> 32); p[i] = u32(v); }
+        }
+    };
+    load();
+    for(u32 work = blockIdx.x; work < works; work += gridDim.x)
+    {
+        const u32 others = entry & ((1u << MAX_B2) - 1), low = (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits);
+        const int up = bits - (32 - __clz(others));
+        const bool more_work = work + gridDim.x < works;
+        if(more_work) next_entry = over[over_cap - 1 - work - gridDim.x];
+        auto for_each = [&](auto&& f)
+        {
+            #pragma unroll
+            for(u32 i = 0; i < ITEMS; ++i)
+            {
+                if(i * BLOCK >= m) break;
+                if(tid + i * BLOCK < m) f(i, tid + i * BLOCK);
+            }
+        };
+        for(u32 i = tid; i < (m + 7) / 8; i += BLOCK)
+        {
+            reinterpret_cast<uint4*>(head)[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            reinterpret_cast<uint4*>(cnt2)[i] = make_uint4(0, 0, 0, 0);
+        }
+        if(tid == 0) s_lines = 0;
+        if(tid < 2) s_tied[tid] = 0;
+        u32 key_of[ITEMS];      // the record that brought the key, and the number << 16
+        for_each([&](const u32 i, const u32 j)
+        {
+            k[i] = (k[i] - low) << up;
+            keys[j] = k[i];
+            start[__umulhi(k[i], m)] = u16(j);
+        });
+        __syncthreads();
+        u32 won = 0, open = 0;
+        for_each([&](const u32 i, const u32 j)
+        {
+            const u32 b = __umulhi(k[i], m), e = start[b];
+            if(keys[e] == k[i])
+            {
+                const u32 number = atomicAdd(&cnt2[e >> 1], (e & 1) ? 0x10000u : 1u);
+                key_of[i] = e | ((e & 1) ? number & 0xFFFF0000u : number << 16);
+                if(e == j) { head[b] = u16(e); link[e] = u16(NONE); won |= 1u << i; }
+            }
+            else open |= 1u << i;
+        });
+        {
+            const u32 mine = __popc(open) | __popc(won) << 16, inc = warp_inclusive(mine);
+            u32 at = 0;
+            if(lane == 31) at = atomicAdd(&s_lines, inc);
+            at = __shfl_sync(0xFFFFFFFFu, at, 31) + inc - mine;
+            u32 front = at & 0xFFFFu, back = CAP - 1 - (at >> 16);
+            if(mine) for_each([&](const u32 i, const u32 j)
+            {
+                if(open >> i & 1u) lines[front++] = u16(j);
+                else if(won >> i & 1u) lines[back--] = u16(j);
+            });
+        }
+        __syncthreads();
+        const u32 open_ones = s_lines & 0xFFFFu, winners = s_lines >> 16;
+        u32 rounds = 1;
+        for(bool more = open_ones != 0; more; ++rounds)
+        {
+            if(rounds == MOST_ROUNDS) break;
+            #pragma unroll 1
+            for(u32 t = tid; t < open_ones; t += BLOCK)
+            {
+                const u32 j = lines[t];
+                if(!(j & SETTLED)) start[__umulhi(keys[j], m)] = u16(j);
+            }
+            __syncthreads();
+            bool here = false;
+            #pragma unroll 1
+            for(u32 t = tid; t < open_ones; t += BLOCK)
+            {
+                const u32 j = lines[t];
+                if(j & SETTLED) continue;
+                const u32 key = keys[j], b = __umulhi(key, m), e = start[b];
+                if(keys[e] != key) { here = true; continue; }
+                const u32 number = atomicAdd(&cnt2[e >> 1], (e & 1) ? 0x10000u : 1u);
+                res[j] = e | ((e & 1) ? number & 0xFFFF0000u : number << 16);
+                if(e == j) { link[e] = head[b]; head[b] = u16(e); }
+                lines[t] = u16(j | SETTLED | (e == j ? WON : 0u));
+            }
+            more = __syncthreads_or(here);
+        }
+        if(more_work)
+        {
+            next_base = __ldg(child_off + (next_entry >> MAX_B2));
+            next_end = __ldg(child_off + (next_entry >> MAX_B2) + (next_entry & ((1u << MAX_B2) - 1)) + 1);
+        }
+        auto go_on = [&]() { entry = next_entry; base = next_base; m = next_end - next_base; if(more_work) load(); };
+        if(rounds == MOST_ROUNDS)
+        {
+            if(tid == 0) left[atomicAdd(&counts->medium, 1u)] = entry;
+            go_on();
+            __syncthreads();
+            continue;
+        }
+        // f(record) for every record that brought a key, by one thread
+        auto for_each_key = [&](auto&& f)
+        {
+            #pragma unroll 1
+            for(u32 t = tid; t < winners; t += BLOCK) f(u32(lines[CAP - 1 - t]));
+            #pragma unroll 1
+            for(u32 t = tid; t < open_ones; t += BLOCK) if(lines[t] & WON) f(u32(lines[t]) & RECORD);
+        };
+        for(u32 i = tid; i < (m + 7) / 8; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+        if(!PACKED)
+            #pragma unroll 1
+            for(u32 j = tid; j < m; j += BLOCK) sa[base + j] = SA_OPEN;         // suffixes that are alone go there later
+        else
+            #pragma unroll 1
+            for(u32 j = tid; j < 5 * m; j += BLOCK) sa40[5 * u64(base) + j] = j % 5 < 4 ? u8(SA_OPEN) : u8(0);
+        __syncthreads();
+        for_each_key([&](const u32 e)
+        {
+            const u32 b = __umulhi(keys[e], m);
+            atomicAdd(&bin[b >> 1], u32(cnt[e]) << (16 * (b & 1u)));
+        });
+        __syncthreads();
+        // exclusive sums of the bins' counts, in place
+        {
+            u32 c[WORDS], sum = 0;
+            const u32 w0 = tid * WORDS;
+            const bool any = 2 * w0 < m;            // the words up to a multiple of four were cleared
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; w += 4)
+            {
+                const uint4 v = any && 2 * (w0 + w) < m ? *reinterpret_cast<const uint4*>(bin + w0 + w) : make_uint4(0, 0, 0, 0);
+                c[w] = v.x; c[w + 1] = v.y; c[w + 2] = v.z; c[w + 3] = v.w;
+            }
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; ++w) sum += (c[w] & 0xFFFFu) + (c[w] >> 16);
+            const u32 inc = warp_inclusive(sum);
+            if(lane == 31) warp_tot[tid >> 5] = inc;
+            __syncthreads();
+            u32 run = __reduce_add_sync(0xFFFFFFFFu, lane < (tid >> 5) ? warp_tot[lane] : 0u) + inc - sum;
+            if(any)
+            {
+                #pragma unroll
+                for(u32 w = 0; w < WORDS; ++w)
+                {
+                    bin[w0 + w] = run * 0x10001u + (c[w] << 16);        // below 2^16 each
+                    run += (c[w] & 0xFFFFu) + (c[w] >> 16);
+                }
+            }
+        }
+        __syncthreads();
+        // a key's place: behind the smaller ones of its list
+        for_each_key([&](const u32 e)
+        {
+            const u32 key = keys[e], b = __umulhi(key, m);
+            u32 place = start[b];
+            for(u32 o = head[b]; o != NONE; o = link[o])
+                if(keys[o] < key) place += cnt[o];
+            res[e] = place | (res[e] & 0x7FFF0000u) | 1u << 31;
+        });
+        __syncthreads();
+        for_each_key([&](const u32 e)
+        {
+            const u32 size = cnt[e];
+            if(size > 1) link[e] = u16(atomicAdd(&s_tied[size <= SMALL_GROUP ? 0 : 1], size));
+        });
+        __syncthreads();
+        const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];
+        if(tid < 2)
+        {
+            const u32 c = s_tied[tid];
+            s_slot[tid] = c ? atomicAdd(tid ? &counts->large : &counts->small, c) : 0;
+        }
+        for_each([&](const u32 i, const u32 j)
+        {
+            u32 e, number;
+            if(open >> i & 1u)
+            {
+                const u32 x = res[j];
+                e = x >> 31 ? j : x & 0xFFFFu;
+                number = x >> 16 & 0x7FFFu;
+            }
+            else { e = key_of[i] & 0xFFFFu; number = key_of[i] >> 16; }
+            const u32 first = res[e] & 0xFFFFu, size = cnt[e];
+            if(size == 1) { put(base + first, p[i]); return; }
+            const u32 o = link[e] + number + (size <= SMALL_GROUP ? 0u : small_ones);
+            heads[o] = base + first;
+            keys[o] = p[i];
+        });
+        __syncthreads();
+        go_on();
+        #pragma unroll 2
+        for(u32 j = tid; j < all_ones; j += BLOCK)
+        {
+            const u64 e = u64(heads[j]) << 32 | keys[j];
+            if(j < small_ones) list[u64(s_slot[0]) + j] = e;
+            else list[list_cap - 1 - (u64(s_slot[1]) + (j - small_ones))] = e;
+        }
+        __syncthreads();        // the next batch reuses the shared arrays
+    }
+}
+
+// ---- what the kernels above leave -------------------------------------------------------------------------------------------------------
+
 template <int BLOCK, int ITEMS> constexpr size_t LOCAL_SMEM = size_t(BLOCK * ITEMS) * 8 + (BLOCK * ITEMS / 2 + 8) * 4 + ((1 << MAX_B2) + 4) * 4;
-constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
 constexpr u32 CROWDED_BIN = 8;      // a batch with larger bins is looked through for bins of one key
 constexpr u32 MANY_TIED = 256;      // a batch with more tied records writes them to the list side by side
 constexpr u32 LONG_BIN = 256;       // a bin of several keys with more records is not ordered by comparing all with all
@@ -660,8 +1349,8 @@ __device__ __forceinline__ void write_packed(u32* words, const u32* placed, cons
     {
         if(q0 + lane < fours)
         {
-            const u32* const v = placed + head + 4 * (q0 + lane);
-            const u32 a = v[0], b = v[1], c = v[2], d = v[3];
+            const u32 e = head + 4 * (q0 + lane);
+            const u32 a = placed[e], b = placed[e + 1], c = placed[e + 2], d = placed[e + 3];
             u32* const w = mine + 5 * lane;
             w[0] = a; w[1] = b << 8; w[2] = b >> 24 | c << 16; w[3] = c >> 16 | d << 24; w[4] = d >> 8;
         }
@@ -677,18 +1366,12 @@ __device__ __forceinline__ void write_packed(u32* words, const u32* placed, cons
     }
 }
 
-// What bounds it is the issue of instructions (7 a record and warp, 68 % of the cycles), then barriers between dependent steps; memory is not (12 bytes a
-// record). So a block finds its children in two dependent reads (chunk_first, child_off), records stay with their threads and only keys are staged,
-// what only tied records need is skipped by warps without any, and three blocks of 512 threads with up to 8 records each share an SM (two such blocks
-// 4.70 ms a build of 2e8 tokens, three 4.67 and with shorter sums of the bins 4.55; blocks of 256 with 16 records, four to an SM, 5.51, with 8 records 4.75; every record staged
-// whole and looked up again by its place 5.17). A block reads its next chunk ahead.
-// MEDIUM: the work list is `over` from its back, single children that were too large for the smaller block; else such children go
-// there if a block of 16 records a thread holds them, and to the front, for the radix sort, if not.
+// Single children of SORT_MOST to MEDIUM_CAP suffixes, and what the kernels above leave: one or two batches in ten thousand of a Zipf text. Every record is compared with all of its bin, of which there are as many as
+// records; a bin of one key takes no comparisons, and a bin of many records of several keys sends the batch through a sorting network. The chain of its steps takes 20 us whatever there is to do.
 // PACKED: the array is written to sa40 as 5-byte entries, else to sa.
-template <int BLOCK, int ITEMS, int BLOCKS, bool MEDIUM, bool PACKED>
-__global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const u32* __restrict__ chunk_first, const u32* __restrict__ chunks,
-                                                                   const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u8* __restrict__ sa40, u64* __restrict__ list,
-                                                                   const u64 list_cap, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap)
+template <int BLOCK, int ITEMS, int BLOCKS, bool PACKED>
+__global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64* __restrict__ rec, const int bits, const u32* __restrict__ child_off, u32* __restrict__ sa, u8* __restrict__ sa40,
+                                                                      u64* __restrict__ list, const u64 list_cap, Build_Counts* __restrict__ counts, const u32* __restrict__ left)
 {
     constexpr int CAP = BLOCK * ITEMS;
     static_assert(ITEMS % 8 == 0, "a thread sums whole 16-byte pieces of the bins' counts");
@@ -697,7 +1380,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
     u32* const placed = keys + CAP;                                                 // [CAP] positions in their order
     u32* const bin = placed + CAP;                                                  // [CAP / 2 + 8]: two 16-bit counters a word, then the bins' starts
     u16* const start = reinterpret_cast<u16*>(bin);
-    u32* const coff = bin + CAP / 2 + 8;                                            // [children of the chunk + 1] their offsets
+    u32* const coff = bin + CAP / 2 + 8;                                            // [children of the batch + 1] their offsets
     __shared__ u32 warp_tot[BLOCK / 32];
     __shared__ u32 s_tied[2], s_slot[2];            // records of small and of large groups in the batch, and their places in the list
     __shared__ u32 mixed[CAP / 32], s_crowded;      // a bit per bin: it holds several keys; whether any bin holds many records
@@ -705,32 +1388,17 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
     const u32 children = 1u << bits;
     const int rbits = 32 - bits;                    // key bits behind the child's
 
-    const u32 works = MEDIUM ? counts->medium : *chunks;
-    u32 next_first = 0, next_end = 0;       // the children of the chunk after this one, read ahead
-    auto look_up = [&](const u32 w)
-    {
-        next_first = MEDIUM ? over[over_cap - 1 - w] : __ldg(chunk_first + w);
-        next_end = MEDIUM ? next_first + 1 : __ldg(chunk_first + w + 1);
-    };
-    if(blockIdx.x < works) look_up(blockIdx.x);
+    let_next_in();
+    wait_for_previous();
+    const u32 works = counts->medium;
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
-        // the block's children: at most all of one parent
-        const u32 child0 = next_first;
-        const u32 last = min(next_end, ((child0 >> bits) + 1) << bits) - child0;        // parents without suffixes may lie between
-        const bool more = work + gridDim.x < works;
-        if(more) look_up(work + gridDim.x);
+        const u32 entry = left[work], child0 = entry >> MAX_B2, last = (entry & ((1u << MAX_B2) - 1)) + 1;
         const u32 first_digit = child0 & (children - 1);
         for(u32 d = tid; d <= last; d += BLOCK) coff[d] = __ldg(child_off + child0 + d);
         if(tid < 2) s_tied[tid] = 0;
         __syncthreads();
         u32 cur = 0;
-        if(!MEDIUM && more)         // the next chunk's records on their way to L2: 16 to a line
-        {
-            const u64 at = u64(__ldg(child_off + next_first)) + tid * 16;
-            if(at < list_cap) asm volatile("prefetch.global.L2 [%0];" :: "l"(rec + at));
-        }
-
         while(cur < last)
         {
             // a batch: as many children as fit
@@ -745,19 +1413,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) local_sort_kernel(const u64* __
                     if(coff[m] - base <= u32(CAP)) a = m; else b = m;
                 }
                 e = a;
-                if(e == cur)
+                if(e == cur)            // no such child is left here
                 {
-                    // a child that does not fit: left to the radix sort
-                    if(tid == 0)
-                    {
-                        const u32 size = coff[cur + 1] - base;
-                        if(!MEDIUM && size <= MEDIUM_CAP) over[over_cap - 1 - atomicAdd(&counts->medium, 1u)] = child0 + cur;
-                        else
-                        {
-                            over[atomicAdd(&counts->oversize, 1u)] = child0 + cur;
-                            atomicAdd(&counts->oversize_records, size);
-                        }
-                    }
                     ++cur;
                     continue;
                 }
@@ -1086,8 +1743,12 @@ Prefix_Sort prefix_sort_plan(u64 n)
 {
     Prefix_Sort ps;
     ps.n = n;
-    int t = 0;                                          // children of at most 2048 suffixes on average
-    while(t < MAX_B1 + MAX_B2 && (n >> t) > 2048) ++t;
+    // Children of at most 2048 suffixes on average. Between 2^21 and 2^26 suffixes, 1536: a child that the local sort leaves to its second kernel, one in a thousand at 2048, costs 20 us wherever
+    // that one ends (2^24 tokens 502 -> 490 us, 8e6 315 -> 299); above, runs of twice as many records in the second split are worth more (1.25e8 tokens 2.44 ms against 2.40).
+    int t = 0;
+    while(t < MAX_B1 && (n >> t) > 2048) ++t;
+    if((n >> t) > 2048)
+        while(t < MAX_B1 + MAX_B2 && (n >> t) > (n < (u64(1) << 26) ? 1536 : 2048)) ++t;
     ps.b1 = t <= MAX_B1 ? 0 : t / 2;
     ps.b2 = t - ps.b1;
     ps.key_bits = ps.b1 + 32;
@@ -1096,10 +1757,17 @@ Prefix_Sort prefix_sort_plan(u64 n)
     return ps;
 }
 
+// Entries of the list of batches: two neighbours of one segment have more than SHORT_BATCH records together (SORT_MOST where there are two splits).
+static u64 most_batches(const Prefix_Sort& ps)
+{
+    const u64 all = u64(ps.parents) * ps.children;
+    return std::min(all, ps.b1 ? 2 * ps.n / SORT_MOST + all / SEGMENT + ps.parents : 2 * ps.n / SHORT_BATCH + all / SHORT_SEGMENT + 1);
+}
+
 size_t prefix_sort_table_bytes(const Prefix_Sort& ps)
 {
     const u64 all = u64(ps.parents) * ps.children;
-    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 5 + align_up256(all * 4) * 2 + align_up256((all + 1) * 4) + align_up256((ps.n / SHORT_CHUNK + (size_t(1) << MAX_B1) + 2) * 4) + 4096;
+    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 4 + align_up256(all * 4) * 3 + align_up256((all + 1) * 4) + align_up256(most_batches(ps) * sizeof(uint4)) + 4096;
 }
 
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
@@ -1111,11 +1779,11 @@ bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
     t.cur1 = cv.take<u32>(size_t(1) << MAX_B1);
     t.par_off = cv.take<u32>((size_t(1) << MAX_B1) + 1);
     t.tile0 = cv.take<u32>((size_t(1) << MAX_B1) + 1);
-    t.chunk0 = cv.take<u32>((size_t(1) << MAX_B1) + 1);
     t.cnt2 = cv.take<u32>(all);
     t.child_off = cv.take<u32>(all + 1);
     t.over = cv.take<u32>(all);
-    t.chunk_first = cv.take<u32>(ps.n / SHORT_CHUNK + (u64(1) << MAX_B1) + 2);
+    t.left = cv.take<u32>(all);
+    t.batches = cv.take<uint4>(most_batches(ps));
     return cv.ok;
 }
 
@@ -1166,14 +1834,14 @@ int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bi
 }
 
 // The second split of `parents` buckets with n records in all (recA to recB).
-int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB)
+int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB, Build_Counts* counts)
 {
     const unsigned tiles = unsigned(n / SPLIT_TILE + parents);
     const u32 children = 1u << b2;
     CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(parents) * children * 4, ctx->stream));
     count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2);
     CSA_LAUNCH_CHECK(ctx);
-    child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off, t.chunk0, t.chunk_first);
+    child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off, t.batches, t.over, t.left, counts);
     CSA_LAUNCH_CHECK(ctx);
     static std::atomic<bool> configured[64];
     CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
@@ -1182,29 +1850,20 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
     return CSA_OK;
 }
 
-// The second launch takes the children of 4097 to 8192 suffixes; a short text, where a launch counts, goes to the larger blocks at once.
+// The second and the third launch take what the ones before leave: little or nothing as a rule, so their blocks are let in early.
 template <bool PACKED>
-int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, bool one_level, u64 n, const u64* rec, u32* sa, u8* sa40, u64* list, Build_Counts* counts)
+int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* rec, u32* sa, u8* sa40, u64* list, Build_Counts* counts)
 {
     const u32 over_cap = parents << b2;
-    const u32* const chunks = t.chunk0 + parents;
-    if constexpr(PACKED)        // texts of one split are short
-    {
-        if(one_level)
-        {
-            static std::atomic<bool> configured[64];
-            CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, false, PACKED>, LOCAL_SMEM<512, 16>, configured));
-            local_sort_kernel<512, 16, 2, false, PACKED><<<unsigned(n / SHORT_CHUNK + parents), 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
-            CSA_LAUNCH_CHECK(ctx);
-            return CSA_OK;
-        }
-    }
-    static std::atomic<bool> configured[2][64];
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 8, 3, false, PACKED>, LOCAL_SMEM<512, 8>, configured[0]));
-    CSA_TRY(shared_bytes(ctx, local_sort_kernel<512, 16, 2, true, PACKED>, LOCAL_SMEM<512, 16>, configured[1]));
-    local_sort_kernel<512, 8, 3, false, PACKED><<<unsigned(std::min<u64>(n / LOCAL_CHUNK + parents, 148 * 3 * 8)), 512, LOCAL_SMEM<512, 8>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
+    static std::atomic<bool> configured[3][64];
+    CSA_TRY(shared_bytes(ctx, local_sort_kernel<PACKED>, SORT_SMEM<PACKED>, configured[0]));
+    CSA_TRY(shared_bytes(ctx, crowded_batches_kernel<PACKED>, CROWD_SMEM, configured[1]));
+    CSA_TRY(shared_bytes(ctx, left_children_kernel<512, 16, 2, PACKED>, LOCAL_SMEM<512, 16>, configured[2]));
+    launch_early(local_sort_kernel<PACKED>, unsigned(std::min<u64>(over_cap, 148 * SORT_BLOCKS * 8)), SORT_BLOCK, SORT_SMEM<PACKED>, ctx->stream, rec, t.batches, b2, sa, sa40, list, counts, t.over, over_cap, t.left);
     CSA_LAUNCH_CHECK(ctx);
-    local_sort_kernel<512, 16, 2, true, PACKED><<<148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream>>>(rec, t.chunk_first, chunks, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap);
+    launch_early(crowded_batches_kernel<PACKED>, 148 * 3, CROWD_BLOCK, CROWD_SMEM, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap, t.left);
+    CSA_LAUNCH_CHECK(ctx);
+    launch_early(left_children_kernel<512, 16, 2, PACKED>, 148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.left);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }
@@ -1219,7 +1878,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     const bool one_level = ps.b1 == 0;
     const int bits = one_level ? ps.b2 : ps.b1;
     if(bits > 0) CSA_TRY(launch_count_text(ctx, T, n, t.code, bits, t.cnt1));
-    launch_early(parent_offsets_kernel, 1, 1024, 0, ctx->stream, t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, p, counts);
+    launch_early(parent_offsets_kernel, 1, 1024, 0, ctx->stream, t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, p, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(n) ? (launch_scatter_text<512, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA))
                           : (launch_scatter_text<128, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA)));
@@ -1230,11 +1889,11 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     u64* other = recB;
     if(!one_level)
     {
-        CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB));
+        CSA_TRY(launch_second_split(ctx, t, ps.parents, ps.b2, n, recA, recB, counts));
         rec = recB; other = recA;
     }
-    CSA_TRY(sa ? launch_local_sort<false>(ctx, t, ps.parents, ps.b2, one_level, n, rec, sa, nullptr, other, counts)
-               : launch_local_sort<true>(ctx, t, ps.parents, ps.b2, one_level, n, rec, nullptr, sa40, other, counts));
+    CSA_TRY(sa ? launch_local_sort<false>(ctx, t, ps.parents, ps.b2, n, rec, sa, nullptr, other, counts)
+               : launch_local_sort<true>(ctx, t, ps.parents, ps.b2, n, rec, nullptr, sa40, other, counts));
     *list = other;
     *records = rec;
     return CSA_OK;
@@ -1262,12 +1921,12 @@ int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Ta
                             Build_Counts* counts)
 {
     CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.chunk0, t.child_off, t.chunk_first, 1, counts);
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, 1, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
                              : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));
-    CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB));
-    CSA_TRY(launch_local_sort<false>(ctx, t, bins, ps.b2, false, size, recB, sa, nullptr, recA, counts));
+    CSA_TRY(launch_second_split(ctx, t, bins, ps.b2, size, recA, recB, counts));
+    CSA_TRY(launch_local_sort<false>(ctx, t, bins, ps.b2, size, recB, sa, nullptr, recA, counts));
     ctx->counters[1] += 2;
     ctx->counters[2] += 2 * size;
     return CSA_OK;

@@ -22,7 +22,9 @@ struct Build_Counts
     u32 next_small;     // the same of the list being made
     u32 partitions;     // contiguous ranges of the suffix array, at most as many as asked for, that the first split's buckets form
     u32 max_partition;  // suffixes of the largest
-    u32 medium;         // children that fit the local sort's larger blocks only
+    u32 batches;        // runs of children that the local sort takes
+    u32 crowded;        // and leaves to its second kernel
+    u32 medium;         // runs for its third
     u32 now_small;      // entries that the last count by size found in small groups
     u32 large_depth;    // symbols that the suffixes of a large group share at least after the initial sort (launch_large_depth)
     u32 looked_at, lead_on, far_ties;       // what a sample of the small groups' entries says (launch_refine_by_text)
@@ -49,11 +51,11 @@ struct Prefix_Tables
     u32* cur1;          // [parents] running places
     u32* par_off;       // [parents + 1] where each parent starts in the suffix array
     u32* tile0;         // [parents + 1] first tile of each parent in the second split
-    u32* chunk0;        // [parents + 1] first chunk of each parent in the local sort
     u32* cnt2;          // [parents][children] records by second digit, then running places
     u32* child_off;     // [parents * children + 1] where each child starts in the suffix array
-    u32* chunk_first;   // first child of every chunk of the local sort (parent * children + child), and the end
-    u32* over;          // children that did not fit a block: their indices
+    uint4* batches;     // the local sort's batches (counts->batches of them): first slot, records, first child (parent * children + child), children
+    u32* over;          // children that did not fit a block, by their indices, from the front; runs of children left to the local sort's second kernel from the back
+    u32* left;          // runs left to its third
 };
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t);
 

@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     u32* const depth = reinterpret_cast<u32*>(key + RW_WINDOW);     // [RW_WINDOW] by first slot: symbols that the group's members share (below 2^32: no more than n)
     Odd_Members& odds = *reinterpret_cast<Odd_Members*>(depth + RW_WINDOW);
     const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    wait_for_previous();
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
     if(count > most)
@@ -1115,7 +1116,7 @@ int launch_refine_by_text(csa_ctx* ctx, const u16* T, u64 n, u64 from, u64 to, c
     to = to < n ? to : n;           // no two suffixes share as much
     CSA_CUDA(ctx, cudaFuncSetAttribute(refine_by_text_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TEXT_SMEM)));
     const u64 tiles = div_up(expected ? expected : 1, RW_TILE);
-    refine_by_text_kernel<<<unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream>>>(T, n, from, to, list, next, sa, sa40, isa, counts, most, code, u32(key_bits));
+    launch_early(refine_by_text_kernel, unsigned(tiles < 148 * 4 ? tiles : 148 * 4), RW_BLOCK, TEXT_SMEM, ctx->stream, T, n, from, to, list, next, sa, sa40, isa, counts, most, code, u32(key_bits));
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

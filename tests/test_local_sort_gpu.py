@@ -1,0 +1,56 @@
+"""The local sort's ways through a batch of children, by how many records share a key and how evenly the keys lie: bins that a thread's window orders, crowded
+bins, batches of more tied records than a block keeps, batches of many records of each key, of many keys close together, and large groups. Each array
+byte for byte against the oracle's."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from cascade_b200 import api
+    c = api.Context(0)
+    yield c
+    c.close()
+
+
+def _check(ctx, oracle, T):
+    from cascade_b200 import api
+    T = np.ascontiguousarray(T, dtype=np.uint16)
+    n = len(T)
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    sa, st = api.build_sa(ctx, Td, n, 8)
+    assert np.array_equal(sa[:5 * n].cpu().numpy(), oracle.build_sa40(T)[:5 * n])
+    return st
+
+
+# one split, two splits; copies of every piece: 2 to 4 records of a key lie in a window, 5 to 15 make a crowded bin, 16 and more a crowded batch, 300 a large group
+@pytest.mark.parametrize("n,copies", [(n, c) for n in (40_000, 300_001) for c in (2, 3, 4, 5, 8, 15, 16, 17, 31, 33, 40, 300)] + [(2_300_003, c) for c in (3, 9, 40)])
+def test_pieces_that_stand_so_many_times(ctx, oracle, n, copies):
+    rng = np.random.default_rng(n + copies)
+    piece = 23
+    base = rng.integers(0, 50000, (n // (2 * piece * copies) + 1, piece))
+    pieces = np.repeat(base, copies, axis=0)
+    rng.shuffle(pieces)
+    T = np.concatenate([pieces.ravel()[:n // 2], rng.integers(0, 50000, n - n // 2)])     # half of the text is told apart by its first symbols
+    st = _check(ctx, oracle, T)
+    assert st.active_after_gen0 > n // 4
+
+
+@pytest.mark.parametrize("n", [300_000, 2_500_000])
+@pytest.mark.parametrize("kind", ["steep", "few_symbols", "one_in_two", "twice"])
+def test_keys_that_lie_unevenly(ctx, oracle, n, kind):
+    rng = np.random.default_rng(n)
+    if kind == "steep":                 # a hundred symbols, each half as frequent as the one before
+        T = np.minimum(rng.geometric(0.5, n), 100)
+    elif kind == "few_symbols":         # children that hold nearly everything or nothing
+        T = np.where(rng.random(n) < 0.9, 5, rng.integers(0, 4, n))
+    elif kind == "one_in_two":          # every other symbol is one of three
+        T = rng.integers(0, 60000, n)
+        T[::2] = rng.integers(0, 3, (n + 1) // 2)
+    else:                               # every piece stands twice: more ties than a block keeps
+        pieces = rng.integers(0, 60000, (n // 120, 60))
+        T = np.concatenate([pieces, rng.permutation(pieces)]).ravel()
+    _check(ctx, oracle, T)
