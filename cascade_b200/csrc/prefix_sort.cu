@@ -497,8 +497,9 @@ template <int BLOCK> constexpr size_t SCATTER_TEXT_SMEM = size_t(TILE_POSITIONS<
 static_assert(SCATTER_TEXT_SMEM<512> >= sizeof(Tile_Code<512>) && SCATTER_TEXT_SMEM<128> >= sizeof(Tile_Code<128>), "the windows lie where the records are staged later");
 
 // Scatter by the top `bits` bits: the places inside a bucket come from shared-memory atomics and, for the tile's run of a bucket,
-// from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs. What bounds it is shared memory
-// and L1 (78 % of their wavefronts): so a staged record carries its bin and its place in the tile in one word instead of its position and a bin beside it.
+// from one global atomic (the order inside a bucket is free); records are staged in bucket order and written as runs. The global atomics are on their way from the moment that the counts
+// are known, and waited for only behind the staging (with each waited for where it was made, as many after one another as a thread has buckets, 1.25e8 symbols took 0.52 ms instead of 0.51, and the split
+// of the buckets 0.54 instead of 0.45). What bounds it is shared memory and L1 (80 % of their wavefronts): so a staged record carries its bin and its place in the tile in one word instead of its position and a bin beside it.
 // keep_top: the record keeps the top bits (there is no second split), else its key starts behind them. PART: only the suffixes of the
 // buckets [first_bin, first_bin + part_bins) are taken, and the cursors are theirs.
 template <int BLOCK, bool PART>
@@ -536,20 +537,19 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
     }
     __syncthreads();
     constexpr int PER = (1 << MAX_B1) / BLOCK;      // bins per thread
-    u32 mine[PER], sum = 0;
+    u32 mine[PER], got[PER], sum = 0;
     #pragma unroll
     for(int k = 0; k < PER; ++k) { const u32 b = threadIdx.x * PER + k; mine[k] = b < bins ? cnt[b] : 0; sum += mine[k]; }
+    #pragma unroll
+    for(int k = 0; k < PER; ++k) { got[k] = 0; if(mine[k]) got[k] = atomicAdd(&cursor[threadIdx.x * PER + k], mine[k]); }     // all on their way at once, and needed last
     u32 total;
-    u32 run = block_exclusive<BLOCK>(sum, warp_tot, total);
+    const u32 before_mine = block_exclusive<BLOCK>(sum, warp_tot, total);
+    u32 run = before_mine;
     #pragma unroll
     for(int k = 0; k < PER; ++k)
     {
         const u32 b = threadIdx.x * PER + k;
-        if(b < bins)
-        {
-            cnt[b] = run;
-            if(mine[k]) base[b] = atomicAdd(&cursor[b], mine[k]) - run;
-        }
+        if(b < bins) cnt[b] = run;
         run += mine[k];
     }
     __syncthreads();
@@ -560,6 +560,14 @@ __global__ void __launch_bounds__(BLOCK, 1024 / BLOCK) scatter_text_kernel(const
             const u32 bin = place[i] >> 16;
             stage[cnt[bin] + (place[i] & 0xFFFFu)] = (u64(key[i]) << 32) | bin << 13 | (local + i);
         }
+    run = before_mine;
+    #pragma unroll
+    for(int k = 0; k < PER; ++k)
+    {
+        const u32 b = threadIdx.x * PER + k;
+        if(b < bins) base[b] = got[k] - run;
+        run += mine[k];
+    }
     __syncthreads();
     const u32 staged = PART ? total : valid;
     #pragma unroll 4
@@ -666,20 +674,19 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
     }
     __syncthreads();
     constexpr int PER = (1 << MAX_B2) / SPLIT_BLOCK;
-    u32 mine[PER], sum = 0;
+    u32 mine[PER], got[PER], sum = 0;
     #pragma unroll
     for(int k = 0; k < PER; ++k) { const u32 b = threadIdx.x * PER + k; mine[k] = b < children ? cnt[b] : 0; sum += mine[k]; }
+    #pragma unroll
+    for(int k = 0; k < PER; ++k) { got[k] = 0; if(mine[k]) got[k] = atomicAdd(&cursor[u64(p) * children + threadIdx.x * PER + k], mine[k]); }      // all on their way at once, and needed last
     u32 total;
-    u32 run = block_exclusive<SPLIT_BLOCK>(sum, warp_tot, total);
+    const u32 before_mine = block_exclusive<SPLIT_BLOCK>(sum, warp_tot, total);
+    u32 run = before_mine;
     #pragma unroll
     for(int k = 0; k < PER; ++k)
     {
         const u32 b = threadIdx.x * PER + k;
-        if(b < children)
-        {
-            cnt[b] = run;
-            if(mine[k]) base[b] = atomicAdd(&cursor[u64(p) * children + b], mine[k]) - run;
-        }
+        if(b < children) cnt[b] = run;
         run += mine[k];
     }
     __syncthreads();
@@ -687,6 +694,14 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
     for(int i = 0; i < SPLIT_ITEMS; ++i)
         if(threadIdx.x + i * SPLIT_BLOCK < valid)
             stage[cnt[u32(r[i] >> 32) >> (32 - bits)] + ((place2[i >> 1] >> ((i & 1) * 16)) & 0xFFFFu)] = r[i];
+    run = before_mine;
+    #pragma unroll
+    for(int k = 0; k < PER; ++k)
+    {
+        const u32 b = threadIdx.x * PER + k;
+        if(b < children) base[b] = got[k] - run;
+        run += mine[k];
+    }
     __syncthreads();
     #pragma unroll
     for(int i = 0; i < SPLIT_ITEMS; ++i)
