@@ -54,3 +54,9 @@ def test_keys_that_lie_unevenly(ctx, oracle, n, kind):
         pieces = rng.integers(0, 60000, (n // 120, 60))
         T = np.concatenate([pieces, rng.permutation(pieces)]).ravel()
     _check(ctx, oracle, T)
+
+
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, (1 << 19) + 1, 1_000_003])
+def test_one_split_by_small_and_by_wide_tiles(ctx, oracle, n):
+    rng = np.random.default_rng(n)
+    _check(ctx, oracle, np.minimum(rng.zipf(1.2, n), 50257))

@@ -32,7 +32,7 @@ def _zipf(n, seed, sigma=50257):
 
 
 # tile of 128 threads: 1984 positions; child: 2048 suffixes; batch of the local sort: 8192; window of a list: 1792 + 256;
-# second split above 2^21, wide tiles (8128 positions) from 2^22 on
+# second split above 2^21, wide tiles (8128 positions) from 2^19 on
 @pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 63, 64, 65, 1983, 1984, 1985, 2047, 2048, 2049, 3968, 3969, 4096, 4097, 8191, 8192, 8193, 16385, (1 << 21) - 1, 1 << 21, (1 << 21) + 1,
                                (1 << 22) - 1, (1 << 22) + 1])
 def test_sizes_at_the_edges(ctx, oracle, n):
