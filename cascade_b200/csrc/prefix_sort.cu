@@ -33,7 +33,7 @@ constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SP
 // The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
 constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
 constexpr int FREE_BITS = 4;                // of a key in a batch: its run of children has that many fewer bits than all of a parent's
-constexpr u32 SEGMENT = 64, SHORT_SEGMENT = 32;         // children whose batches one thread forms: they end with a segment
+constexpr u32 SEGMENT = 64, SHORT_SEGMENT = 8;          // children whose batches one thread forms: they end with a segment
 constexpr u32 SHORT_BATCH = 1024;           // records of a batch of a text of one split, so that it has one for every SM
 constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
 
@@ -394,7 +394,7 @@ __device__ __forceinline__ u32 children_entry(const u32 first, const u32 count) 
 
 struct Batch_Room { u32 used, at; u16 next[1 << MAX_B2]; u32 heads[(1 << MAX_B2) / 32]; };
 __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, const u32 children, const u32 segment, const u32 most, const u32 first_slot, const u32 first_child,
-                                             uint4* __restrict__ batches, Build_Counts* __restrict__ counts, u32* __restrict__ over, u32* __restrict__ left)
+                                             const bool only, uint4* __restrict__ batches, Build_Counts* __restrict__ counts, u32* __restrict__ over, u32* __restrict__ left)
 {
     const u32 tid = threadIdx.x;
     if(tid < (1 << MAX_B2) / 32) room.heads[tid] = 0;
@@ -410,17 +410,8 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
         room.next[i] = u16(a);
     }
     __syncthreads();
-    for(u32 s = tid; s * segment < children; s += blockDim.x)       // a segment's batches: whole words of bits
-    {
-        const u32 end = min(children, (s + 1) * segment);
-        for(u32 i = s * segment, w = i >> 5, bits = 0; i < end;)
-        {
-            if(i >> 5 != w) { room.heads[w] = bits; bits = 0; w = i >> 5; }
-            bits |= 1u << (i & 31u);
-            i = room.next[i];
-            if(i >= end || i >> 5 != w) room.heads[w] = bits;
-        }
-    }
+    for(u32 s = tid; s * segment < children; s += blockDim.x)
+        for(u32 i = s * segment, end = min(children, (s + 1) * segment); i < end; i = room.next[i]) atomicOr(&room.heads[i >> 5], 1u << (i & 31u));
     __syncthreads();
     u32 mine = 0;       // up to two children a thread: whether a batch begins there
     #pragma unroll
@@ -442,7 +433,10 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
     }
     u32 at = mine ? atomicAdd(&room.used, u32(__popc(mine))) : 0u;
     __syncthreads();
-    if(tid == 0) room.at = atomicAdd(&counts->batches, room.used);
+    if(tid == 0)
+    {
+        if(only) { room.at = 0; counts->batches = room.used; } else room.at = atomicAdd(&counts->batches, room.used);
+    }
     __syncthreads();
     at += room.at;
     #pragma unroll
@@ -483,7 +477,7 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
         if(t < bins) { child_off[t] = off; s_off[t] = off; }
         if(t == 0) { child_off[bins] = n; s_off[bins] = n; }
         __syncthreads();
-        form_batches(room, s_off, bins, SHORT_SEGMENT, SHORT_BATCH, 0, 0, batches, stats, over, left);
+        form_batches(room, s_off, bins, SHORT_SEGMENT, SHORT_BATCH, 0, 0, true, batches, stats, over, left);
         return;
     }
     const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE;
@@ -637,7 +631,7 @@ __global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ c
     if(t == 0) s_off[children] = total;
     if(p == parents - 1 && t == 0) child_off[u64(parents) * children] = par_off[parents];
     __syncthreads();
-    form_batches(room, s_off, children, SEGMENT, SORT_MOST, par_off[p], p * children, batches, stats, over, left);
+    form_batches(room, s_off, children, SEGMENT, SORT_MOST, par_off[p], p * children, false, batches, stats, over, left);
 }
 
 constexpr size_t SPLIT_SMEM = size_t(SPLIT_TILE) * 8;
@@ -747,7 +741,7 @@ __device__ __forceinline__ void order(u32& a, u32& b, u32& c) { order(a, b); ord
 // with 8 do. A Zipf text of 1.25e8 symbols, the kernel alone: 0.66 ms; 512 threads with 8 records, two blocks an SM 0.78 and three (40 registers, spills) 1.0; two blocks of 256
 // 0.74; all keys of a bin compared with one another and every record placed by its rank (226 instructions) 1.14. Room for 2048 tied records instead of 1024 leaves L1 too small for
 // the registers that spill: 1 % of a build.
-// PACKED: the array is written to sa40 as 5-byte entries, else to sa.
+// PACKED: the array is written to sa40 as 5-byte entries, else to sa. over_cap: 0 where crowded_batches_kernel is not launched.
 template <bool PACKED>
 __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(const u64* __restrict__ rec, const uint4* __restrict__ batches, const int bits, u32* __restrict__ sa,
                                                                              u8* __restrict__ sa40, u64* __restrict__ list, Build_Counts* __restrict__ counts, u32* __restrict__ over,
@@ -799,7 +793,11 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         }
         if(tid < rest) { const u64 v = at[full * BLOCK]; k[ITEMS - 1] = u32(v >> 32); p[ITEMS - 1] = u32(v); }
     };
-    auto leave_crowded = [&](const u32 children) { over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children; };      // by one thread
+    auto leave = [&](const u32 children, const bool copies)        // by one thread
+    {
+        if(copies && over_cap) over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children;
+        else left[atomicAdd(&counts->medium, 1u)] = children;
+    };
     auto put = [&](const u32 slot, const u32 v)
     {
         if(!PACKED) { sa[slot] = v; return; }
@@ -868,7 +866,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         {
             s_crowded = 0;
             s_fall[turn ^ 1] = 0;
-            if(crammed) leave_crowded(s_before);
+            if(crammed) leave(s_before, true);
             s_before = now.z;
             if(write) s_slot = atomicAdd(&counts->small, ties);
         }
@@ -940,7 +938,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
             if(lane == 0)
             {
                 s_copies = copies;
-                if(copies) leave_crowded(now.z); else left[atomicAdd(&counts->medium, 1u)] = now.z;
+                leave(now.z, copies);
             }
         }
         __syncthreads();
@@ -1059,7 +1057,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         // where one batch after the other is left, only one in eight is tried
         fell = (fall && s_copies) || crammed ? fell + 1 : 0;
         const u32 jump = fell < 2 ? 1u : 8u, passed = next + (tid + 1) * gridDim.x;
-        if(tid + 1 < jump && passed < works) leave_crowded(__ldg(&batches[passed].z));
+        if(tid + 1 < jump && passed < works) leave(__ldg(&batches[passed].z), true);
         next += jump * gridDim.x;
         then.y = 0;
         if(next < works) then = __ldg(batches + next);
@@ -1070,7 +1068,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
     const u32 ties = crammed ? kept : s_ties;
     if(tid == 0)
     {
-        if(crammed) leave_crowded(now.z);
+        if(crammed) leave(now.z, true);
         if(ties) s_slot = atomicAdd(&counts->small, ties);
     }
     __syncthreads();
@@ -1872,14 +1870,18 @@ template <bool PACKED>
 int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* rec, u32* sa, u8* sa40, u64* list, Build_Counts* counts)
 {
     const u32 over_cap = parents << b2;
+    const bool crowds = parents > 1;        // a text of one split goes to the third kernel with what it leaves: a launch counts there, and 1e6 near-duplicates take as long either way
     static std::atomic<bool> configured[3][64];
     CSA_TRY(shared_bytes(ctx, local_sort_kernel<PACKED>, SORT_SMEM<PACKED>, configured[0]));
     CSA_TRY(shared_bytes(ctx, crowded_batches_kernel<PACKED>, CROWD_SMEM, configured[1]));
     CSA_TRY(shared_bytes(ctx, left_children_kernel<512, 16, 2, PACKED>, LOCAL_SMEM<512, 16>, configured[2]));
-    launch_early(local_sort_kernel<PACKED>, unsigned(std::min<u64>(over_cap, 148 * SORT_BLOCKS * 8)), SORT_BLOCK, SORT_SMEM<PACKED>, ctx->stream, rec, t.batches, b2, sa, sa40, list, counts, t.over, over_cap, t.left);
+    launch_early(local_sort_kernel<PACKED>, unsigned(std::min<u64>(over_cap, 148 * SORT_BLOCKS * 8)), SORT_BLOCK, SORT_SMEM<PACKED>, ctx->stream, rec, t.batches, b2, sa, sa40, list, counts, t.over, crowds ? over_cap : 0u, t.left);
     CSA_LAUNCH_CHECK(ctx);
-    launch_early(crowded_batches_kernel<PACKED>, 148 * 3, CROWD_BLOCK, CROWD_SMEM, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap, t.left);
-    CSA_LAUNCH_CHECK(ctx);
+    if(crowds)
+    {
+        launch_early(crowded_batches_kernel<PACKED>, 148 * 3, CROWD_BLOCK, CROWD_SMEM, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap, t.left);
+        CSA_LAUNCH_CHECK(ctx);
+    }
     launch_early(left_children_kernel<512, 16, 2, PACKED>, 148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.left);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
