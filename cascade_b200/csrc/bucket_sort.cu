@@ -223,28 +223,24 @@ template <int BLOCK, typename V> constexpr size_t BUCKET_SMEM = size_t(BUCKET_CA
 // 1.71 and 1.79; by digit passes alone 2.03 and 2.12. What bounds it is the issue of instructions and barriers between
 // dependent steps: blocks are as small as the largest bucket allows, with 8 records a thread. (31.25 M records, 16 a thread and the values
 // gathered when the places were known: 454 us, this way 389 us.)
-template <int BLOCK, int BLOCKS, typename V>
-__global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in,
-                                                                   V* __restrict__ vals_out, const u32* __restrict__ starts, const u32 n, const u64 compared, const int top,
-                                                                   const int begin)
+template <int BLOCK, int ITEMS, typename V>
+__device__ __forceinline__ void sort_bucket(unsigned char* const smem_raw, const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in, V* __restrict__ vals_out,
+                                            const u32 base, const u32 m, const u64 compared, const int top, const int begin)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr u32 CAP = BUCKET_CAP<BLOCK>;
-    constexpr int ITEMS = BUCKET_ITEMS;
+    constexpr u32 CAP = BLOCK * ITEMS;
     u64* const stage = reinterpret_cast<u64*>(smem_raw);            // [CAP]
     u32* const bin = reinterpret_cast<u32*>(stage + CAP);           // [CAP / 2 + 8]: two 16-bit counters a word, then the bins' starts
     u16* const start = reinterpret_cast<u16*>(bin);
     u16* const from = reinterpret_cast<u16*>(bin + CAP / 2 + 8);    // [CAP]: the record's place in the bucket before
     V* const vals = reinterpret_cast<V*>(stage + CAP);              // [CAP], once the bins are no longer needed
     __shared__ u32 warp_tot[BLOCK / 32], s_differ[2];
-    static_assert(BLOCK / 32 * 256 <= CAP && BLOCK >= 256 && ITEMS * 32 == 256 && CAP <= 8192, "the warps' counts lie where the bins do; places take 13 bits");
+    static_assert(BLOCK / 32 * 256 <= CAP && BLOCK >= 256 && CAP <= 8192, "the warps' counts lie where the bins do; places take 13 bits");
     const u32 tid = threadIdx.x;
-    const u32 base = starts ? starts[blockIdx.x] : 0, m = (starts ? starts[blockIdx.x + 1] : n) - base;
     if(m == 0 || m > CAP) return;       // the host has seen to it that all fit
     keys_in += base; keys_out += base;
     if(vals_in != nullptr) { vals_in += base; vals_out += base; }
 
-    const int bin_bits = min(32 - __clz(m - 1 | 1u), top - begin);  // bins: a power of two, at most CAP
+    const int bin_bits = min(min(32 - __clz(m - 1 | 1u), 31 - __clz(CAP)), top - begin);     // bins: a power of two, at most CAP
     const u32 bins = 1u << bin_bits;
     const int bin_shift = top - bin_bits;
     const u32 bin_mask = bins - 1;
@@ -275,13 +271,13 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* _
     // exclusive sums of the bins' counts, in place; start[bins] = m
     u32 longest = 0;
     {
-        constexpr int WORDS = CAP / 2 / BLOCK;          // 4 words, 8 bins a thread
+        constexpr int WORDS = CAP / 2 / BLOCK;
         u32 c[WORDS], sum = 0;
         const bool any = tid * WORDS * 2 <= bins;       // the words up to a multiple of WORDS were cleared
         if(any)
         {
-            const uint4 v = reinterpret_cast<const uint4*>(bin)[tid];
-            c[0] = v.x; c[1] = v.y; c[2] = v.z; c[3] = v.w;
+            #pragma unroll
+            for(int k = 0; k < WORDS; ++k) c[k] = bin[tid * WORDS + k];
             u32 both = 0;
             #pragma unroll
             for(int k = 0; k < WORDS; ++k) { both += c[k]; longest = __vmaxu2(longest, c[k]); }
@@ -298,9 +294,8 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* _
             {
                 const u32 a = run * 0x10001u + (c[k] << 16);        // below 2^16 each
                 run += (c[k] & 0xFFFFu) + (c[k] >> 16);
-                c[k] = a;
+                bin[tid * WORDS + k] = a;
             }
-            reinterpret_cast<uint4*>(bin)[tid] = make_uint4(c[0], c[1], c[2], c[3]);
         }
         if(bins == CAP && tid == 0) start[CAP] = u16(m);            // behind the threads' words
     }
@@ -439,6 +434,270 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* _
 }
 
 template <int BLOCK, int BLOCKS, typename V>
+__global__ void __launch_bounds__(BLOCK, BLOCKS) bucket_sort_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in, V* __restrict__ vals_out,
+                                                                   const u32* __restrict__ starts, const u32 n, const u64 compared, const int top, const int begin)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const u32 base = starts ? starts[blockIdx.x] : 0, m = (starts ? starts[blockIdx.x + 1] : n) - base;
+    sort_bucket<BLOCK, BUCKET_ITEMS, V>(smem_raw, keys_in, keys_out, vals_in, vals_out, base, m, compared, top, begin);
+}
+
+// Apart, so that the kernel below keeps its registers.
+template <int BLOCK, int ITEMS, typename V>
+__device__ __noinline__ void sort_bucket_apart(unsigned char* const smem_raw, const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in, V* __restrict__ vals_out,
+                                               const u32 base, const u32 m, const u64 compared, const int top, const int begin)
+{
+    sort_bucket<BLOCK, ITEMS, V>(smem_raw, keys_in, keys_out, vals_in, vals_out, base, m, compared, top, begin);
+}
+
+// ---- a bucket inside one block, evenly spread keys -----------------------------------------------------------------------------------------
+
+constexpr int ORDER_BLOCK = 256;
+// words of the records and their bins; then their keys and values as they came
+template <int ITEMS> constexpr u32 ORDER_CAP = ORDER_BLOCK * ITEMS;
+template <int ITEMS> constexpr u32 ORDER_MOST = ORDER_CAP<ITEMS> - 4;
+template <int ITEMS, typename V> constexpr size_t ORDER_SMEM = size_t(ORDER_CAP<ITEMS>) * (4 + 2 + 8 + sizeof(V)) + 80;
+constexpr int FROM_BITS = 12, WORD_BITS = 32 - FROM_BITS;       // a word: the first bits of a key that the buckets do not tell, and the record's place in the bucket before
+constexpr u32 MOST_CROWDED = 64;
+// Four counts of five bits a word, later where the word's records begin (12 bits) and, in the fields, where those of each bin do.
+constexpr u32 each_bin(const u32 v) { return v | v << 5 | v << 10 | v << 15; }
+constexpr u32 SUMS = each_bin(1) << 5, SUMS_BEFORE = each_bin(31) & ~31u, SUM_OF_ALL = 31u << 20;
+constexpr u32 TO_EIGHT = each_bin(3), EIGHT_UP = each_bin(24), FULL_BIN = each_bin(16);
+
+__device__ __forceinline__ void order(u32& a, u32& b) { const u32 t = min(a, b); b = max(a, b); a = t; }
+__device__ __forceinline__ void order(u32& a, u32& b, u32& c) { order(a, b); order(b, c); order(a, b); }
+
+// As the resident build's local sort: records are counted in two bins each by interpolation of their words, the words go to shared memory in the order of the bins, and a thread orders
+// the words of four slots with those of the three slots before and behind by min and max: bins of up to four records lie inside the window of every slot of theirs, the few of up to 15 are
+// ordered by a warp. A word ends in the record's place in the bucket before, so equal keys stay in their order; where a word does not hold all compared bits, records of the same first bits
+// are told apart by their whole keys. Keys and values are read from shared memory by that place and go out as 16-byte stores.
+// A bucket with a bin of 16 or more is sorted as above; where one in eight is, the others are not tried in this way.
+// Bound by the issue of instructions (159 for 32 records, 48 % of the cycles) and the chain of a single bucket in a block: 31.25 M records of 64-bit keys and 4-byte values in buckets of 1907, 296 us where
+// bucket_sort_kernel takes 378; whole calls 1123 -> 1034 us, by 32 bits 972 -> 834.
+template <int ITEMS, int BLOCKS, typename V>
+__global__ void __launch_bounds__(ORDER_BLOCK, BLOCKS) order_buckets_kernel(const u64* __restrict__ keys_in, u64* __restrict__ keys_out, const V* __restrict__ vals_in, V* __restrict__ vals_out,
+                                                                            const u32* __restrict__ starts, Bucket_Findings* __restrict__ found, const u64 compared, const int top, const int begin)
+{
+    constexpr u32 BLOCK = ORDER_BLOCK, CAP = ORDER_CAP<ITEMS>, WARPS = BLOCK / 32, WORDS = CAP / 2 / BLOCK, CROWD_WORDS = CAP / 32 + 4;
+    static_assert(CAP <= 1u << FROM_BITS && CROWD_WORDS <= BLOCK && WORDS * 2 * BLOCK == CAP, "places take 12 bits");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u64* const key = reinterpret_cast<u64*>(smem_raw);                  // [CAP]
+    V* const val = reinterpret_cast<V*>(key + CAP);                     // [CAP]
+    u32* const words = reinterpret_cast<u32*>(val + CAP) + 4;           // [CAP + 16] in the order of the bins; four before it
+    u32* const bin = words + CAP + 16;                                  // [CAP / 2]
+    __shared__ u32 warp_tot[WARPS], crowd[CROWD_WORDS], crowded[MOST_CROWDED], s_crowded, s_fall;
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
+    const u32 base = starts[blockIdx.x], m = starts[blockIdx.x + 1] - base;
+    if(m == 0) return;
+    const u32 full = __shfl_sync(0xFFFFFFFFu, m / BLOCK, 0), rest = m % BLOCK, shift = base & 3u, end = shift + m, whole = base - shift;
+    auto for_each = [&](auto&& f)
+    {
+        #pragma unroll
+        for(u32 i = 0; i < ITEMS - 1; ++i)
+        {
+            if(i >= full) break;
+            f(i, tid + i * BLOCK);
+        }
+        if(tid < rest) f(ITEMS - 1, tid + full * BLOCK);
+    };
+    u64 r[ITEMS];
+    V v[ITEMS];
+    for_each([&](const u32 i, const u32 j) { r[i] = keys_in[base + j]; if(vals_in != nullptr) v[i] = vals_in[base + j]; });
+    #pragma unroll
+    for(u32 w = 0; w < WORDS; ++w) bin[tid + w * BLOCK] = 0;
+    if(tid < CROWD_WORDS) crowd[tid] = 0;
+    if(tid < 4) words[int(tid) - 4] = 0;
+    if(tid == 0) { s_crowded = 0; s_fall = found->left > blockIdx.x / 8 + 64; }
+    u32 k[ITEMS];
+    for_each([&](const u32 i, const u32 j)
+    {
+        key[j] = r[i];
+        if(vals_in != nullptr) val[j] = v[i];
+        k[i] = u32(((r[i] & compared) << (64 - top)) >> 32) & ~((1u << FROM_BITS) - 1);
+    });
+    __syncthreads();
+    if(s_fall)
+    {
+        sort_bucket_apart<ORDER_BLOCK, ITEMS, V>(smem_raw, keys_in, keys_out, vals_in, vals_out, base, m, compared, top, begin);
+        return;
+    }
+    u32 seen = 0, number[(ITEMS + 7) / 8] = {};
+    for_each([&](const u32 i, const u32)
+    {
+        const u32 b = __umulhi(k[i], 2 * m), old = atomicAdd(bin + (b >> 2), 1u << (5 * (b & 3u)));
+        seen |= old;
+        number[i / 8] |= (old >> (5 * (b & 3u)) & 15u) << (4 * (i % 8));
+    });
+    if(seen & FULL_BIN) s_fall = 1;
+    __syncthreads();
+    const bool any = 2 * WORDS * tid < m, busy = 64 * WORDS * warp < m;
+    u32 c[WORDS], sum = 0, inc = 0, many = 0;
+    if(busy)
+    {
+        #pragma unroll
+        for(u32 w = 0; w < WORDS; ++w)
+        {
+            c[w] = any ? bin[WORDS * tid + w] : 0u;
+            many |= (c[w] + TO_EIGHT) & EIGHT_UP;
+            sum += c[w] * SUMS & SUM_OF_ALL;
+        }
+        inc = warp_inclusive_sum(sum);
+    }
+    if(lane == 31) warp_tot[warp] = inc;
+    __syncthreads();
+    if(busy)
+    {
+        u32 run = (shift << 20) + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_tot[lane] : 0u) + inc - sum;
+        if(any)
+        {
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; ++w) { bin[WORDS * tid + w] = (c[w] * SUMS & SUMS_BEFORE) | run; run += c[w] * SUMS & SUM_OF_ALL; }
+        }
+        if(many)
+        {
+            #pragma unroll
+            for(u32 w = 0; w < WORDS; ++w)
+                #pragma unroll 1
+                for(u32 f = (c[w] + TO_EIGHT) & EIGHT_UP; f;)
+                {
+                    const u32 bit = (__ffs(f) - 1) / 5 * 5, size = c[w] >> bit & 31u, x = bin[WORDS * tid + w];
+                    const u32 at = (x >> 20) + (x >> bit & 31u), o = atomicAdd(&s_crowded, 1u);
+                    f &= ~(31u << bit);
+                    if(o < MOST_CROWDED) crowded[o] = at | size << 16;
+                    const u64 marks = u64((1u << size) - 1) << (at & 31u);
+                    if((at >> 5) + 1 < CROWD_WORDS)
+                    {
+                        atomicOr(&crowd[at >> 5], u32(marks));
+                        if(marks >> 32) atomicOr(&crowd[(at >> 5) + 1], u32(marks >> 32));
+                    }
+                    u32 all = 0;
+                    for(int b = 0; b < 4; ++b) all += c[w] >> (5 * b) & 31u;
+                    if(o >= MOST_CROWDED || (c[w] & FULL_BIN) || all > 31) s_fall = 1;
+                }
+        }
+    }
+    __syncthreads();
+    if(s_fall)
+    {
+        if(tid == 0) atomicAdd(&found->left, 1u);
+        sort_bucket_apart<ORDER_BLOCK, ITEMS, V>(smem_raw, keys_in, keys_out, vals_in, vals_out, base, m, compared, top, begin);
+        return;
+    }
+    for_each([&](const u32 i, const u32 j)
+    {
+        const u32 b = __umulhi(k[i], 2 * m), x = bin[b >> 2], slot = (x >> 20) + (x >> (5 * (b & 3u)) & 31u) + (number[i / 8] >> (4 * (i % 8)) & 15u);
+        words[slot] = k[i] | j;
+    });
+    if(tid < shift) words[tid] = 0;                     // no word is below, or above those behind
+    if(tid < 8) words[end + tid] = 0xFFFFFFFFu;
+    __syncthreads();
+    constexpr u32 FROM = (1u << FROM_BITS) - 1;
+    const bool told = top - begin <= WORD_BITS;         // a word holds all of a key that is compared
+    const bool aligned = ((reinterpret_cast<uintptr_t>(keys_out) | reinterpret_cast<uintptr_t>(vals_out)) & 15) == 0;
+    // The record of a group of the same first bits that comes at place `rank` of it; the group lies inside the slots [first, stop).
+    auto whole_less = [&](const u32 a, const u32 b) { const u64 x = key[a & FROM] & compared, y = key[b & FROM] & compared; return x < y || (x == y && a < b); };
+    const u32 crowds = s_crowded;
+    #pragma unroll 1
+    for(u32 q0 = warp * 32; 4 * q0 < end; q0 += BLOCK)
+    {
+        const u32 q = q0 + lane;
+        const uint4* const K = reinterpret_cast<const uint4*>(words - 4) + q;
+        const uint4 L = K[0], O = K[1], R = K[2];
+        u32 a0 = L.y, a1 = L.z, a2 = L.w, x0 = O.x, x1 = O.y, x2 = O.z, x3 = O.w, r0 = R.x, r1 = R.y, r2 = R.z;
+        order(x0, x1); order(x2, x3); order(x0, x2); order(x1, x3); order(x1, x2);
+        order(a0, a1, a2);
+        order(r0, r1, r2);
+        const u32 before = max(max(min(a0, x2), min(a1, x1)), min(a2, x0));
+        x2 = max(a0, x2); x1 = max(a1, x1); x0 = max(a2, x0);
+        order(x0, x1, x2);
+        const u32 behind = min(min(max(x1, r2), max(x2, r1)), max(x3, r0));
+        x1 = min(x1, r2); x2 = min(x2, r1); x3 = min(x3, r0);
+        order(x1, x2, x3);
+        u32 x[4] = {x0, x1, x2, x3};
+        u32 wanted = 4 * q < end ? 15u : 0u;
+        if(4 * q < shift) wanted = 15u << shift & 15u;
+        if(4 * q + 4 > end && wanted) wanted &= 15u >> (4 * q + 4 - end);
+        if(crowds) wanted &= ~(crowd[q >> 3] >> (4 * (q & 7u)));
+        if(!told && min(min(min(before ^ x0, x0 ^ x1), min(x1 ^ x2, x2 ^ x3)), x3 ^ behind) <= FROM)
+        {
+            #pragma unroll
+            for(u32 i = 0; i < 4; ++i)
+            {
+                if(!(wanted >> i & 1u)) continue;
+                const u32 mine = x[i], first = max(4 * q + i, shift + 3) - 3, stop = min(4 * q + i + 4, end);
+                u32 rank = 0, group = 0;
+                #pragma unroll 1
+                for(u32 s = first; s < stop; ++s)
+                    if((words[s] ^ mine) <= FROM) { ++group; rank += words[s] < mine; }
+                if(group <= 1) continue;
+                #pragma unroll 1
+                for(u32 s = first; s < stop; ++s)
+                {
+                    if((words[s] ^ mine) > FROM) continue;
+                    u32 less = 0;
+                    #pragma unroll 1
+                    for(u32 o = first; o < stop; ++o)
+                        if((words[o] ^ mine) <= FROM && whole_less(words[o], words[s])) ++less;
+                    if(less == rank) x[i] = words[s];
+                }
+            }
+        }
+        const u64 to = u64(whole) + 4 * q;
+        if(aligned && wanted == 15u)
+        {
+            reinterpret_cast<ulonglong2*>(keys_out + to)[0] = make_ulonglong2(key[x[0] & FROM], key[x[1] & FROM]);
+            reinterpret_cast<ulonglong2*>(keys_out + to)[1] = make_ulonglong2(key[x[2] & FROM], key[x[3] & FROM]);
+            if(vals_in != nullptr)
+            {
+                if constexpr(sizeof(V) == 4) *reinterpret_cast<uint4*>(vals_out + to) = make_uint4(val[x[0] & FROM], val[x[1] & FROM], val[x[2] & FROM], val[x[3] & FROM]);
+                else
+                {
+                    reinterpret_cast<ulonglong2*>(vals_out + to)[0] = make_ulonglong2(val[x[0] & FROM], val[x[1] & FROM]);
+                    reinterpret_cast<ulonglong2*>(vals_out + to)[1] = make_ulonglong2(val[x[2] & FROM], val[x[3] & FROM]);
+                }
+            }
+        }
+        else
+            #pragma unroll
+            for(u32 i = 0; i < 4; ++i)
+                if(wanted >> i & 1u)
+                {
+                    keys_out[to + i] = key[x[i] & FROM];
+                    if(vals_in != nullptr) vals_out[to + i] = val[x[i] & FROM];
+                }
+    }
+    #pragma unroll 1
+    for(u32 o = WARPS - 1 - warp; o < crowds; o += WARPS)
+    {
+        const u32 s = crowded[o] & 0xFFFFu, size = crowded[o] >> 16;
+        const u32 mine = words[s + min(lane, size - 1)];
+        u32 less = 0;
+        #pragma unroll 1
+        for(u32 j = 0; j < size; ++j) less += whole_less(words[s + j], mine);
+        if(lane < size)
+        {
+            keys_out[u64(whole) + s + less] = key[mine & FROM];
+            if(vals_in != nullptr) vals_out[u64(whole) + s + less] = val[mine & FROM];
+        }
+    }
+}
+
+template <int ITEMS, int BLOCKS, typename V>
+int launch_order(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, Bucket_Findings* found, u64 compared, int top, int begin)
+{
+    static std::atomic<bool> configured[64];
+    static_assert(ORDER_SMEM<ITEMS, V> >= size_t(ORDER_CAP<ITEMS>) * 8 + (sizeof(V) == 8 ? size_t(ORDER_CAP<ITEMS>) * 8 : size_t(ORDER_CAP<ITEMS>) * 4 + 32), "room for sort_bucket");
+    if(!configured[ctx->device & 63])
+    {
+        CSA_CUDA(ctx, cudaFuncSetAttribute(order_buckets_kernel<ITEMS, BLOCKS, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ORDER_SMEM<ITEMS, V>)));
+        configured[ctx->device & 63] = true;
+    }
+    order_buckets_kernel<ITEMS, BLOCKS, V><<<buckets, ORDER_BLOCK, ORDER_SMEM<ITEMS, V>, ctx->stream>>>(kin, kout, vin, vout, starts, found, compared, top, begin);
+    CSA_LAUNCH_CHECK(ctx);
+    return CSA_OK;
+}
+
+template <int BLOCK, int BLOCKS, typename V>
 int launch_buckets(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 compared, int top, int begin)
 {
     static std::atomic<bool> configured[64];
@@ -452,10 +711,19 @@ int launch_buckets(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vou
     return CSA_OK;
 }
 
+// 31.25 M records: see the kernel; 4 and 1 M the same either way; 1e5 with few bits that differ 64 us by bucket_sort_kernel, 76 by order_buckets_kernel, which leaves such buckets after a try.
+constexpr u64 ORDER_MIN = u64(1) << 22;
+
 template <typename V>
-int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 largest, int begin, int top)
+int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 largest, Bucket_Findings* found, int begin, int top)
 {
     const u64 compared = (top >= 64 ? ~0ull : (1ull << top) - 1) & (~0ull << begin);
+    if(n >= ORDER_MIN)
+    {
+        if(largest <= ORDER_MOST<8>) return launch_order<8, 5, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
+        if(largest <= ORDER_MOST<10>) return launch_order<10, 4, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
+        if(largest <= ORDER_MOST<16>) return launch_order<16, 2, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
+    }
     if(largest <= BUCKET_CAP<256>) return launch_buckets<256, 6, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
     if(largest <= BUCKET_CAP<512>) return launch_buckets<512, 3, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
     if(largest <= BUCKET_CAP<1024>) return launch_buckets<1024, 1, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
@@ -490,9 +758,9 @@ int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int begin_bit, int 
     return CSA_OK;
 }
 
-int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, int begin_bit,
-                       int top)
+int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, Bucket_Findings* found,
+                       int begin_bit, int top)
 {
-    if(val_bytes == 4) return launch_buckets_of<u32>(ctx, kin, kout, static_cast<const u32*>(vin), static_cast<u32*>(vout), starts, buckets, n, largest, begin_bit, top);
-    return launch_buckets_of<u64>(ctx, kin, kout, static_cast<const u64*>(vin), static_cast<u64*>(vout), starts, buckets, n, largest, begin_bit, top);
+    if(val_bytes == 4) return launch_buckets_of<u32>(ctx, kin, kout, static_cast<const u32*>(vin), static_cast<u32*>(vout), starts, buckets, n, largest, found, begin_bit, top);
+    return launch_buckets_of<u64>(ctx, kin, kout, static_cast<const u64*>(vin), static_cast<u64*>(vout), starts, buckets, n, largest, found, begin_bit, top);
 }

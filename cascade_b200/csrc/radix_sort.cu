@@ -846,7 +846,7 @@ struct Bucket_Split
 
 // The passes and the buckets, once the counts are there; largest: the size of the largest bucket.
 int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* vals_alt, u32 val_bytes, u64 n, int begin_bit, int end_bit, u32* counter, u32* status, const u64* low_base,
-                    const u64* high_base, const u32* starts, u64 largest, int* in_alt)
+                    const u64* high_base, const u32* starts, u64 largest, Bucket_Findings* found, int* in_alt)
 {
     const Bucket_Split split(n);
     const int bits = split.bits, splits = split.splits, low_bits = split.low_bits;
@@ -879,7 +879,7 @@ int sort_by_buckets(csa_ctx* ctx, u64* keys, u64* keys_alt, void* vals, void* va
         std::swap(keys, keys_alt);
         std::swap(vals, vals_alt);
     }
-    CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, starts, 1u << bits, n, largest, begin_bit, end_bit - bits));
+    CSA_TRY(launch_bucket_sort(ctx, keys, keys_alt, vals, vals_alt, val_bytes, starts, 1u << bits, n, largest, found, begin_bit, end_bit - bits));
     *in_alt = (splits + 1) & 1;
     return CSA_OK;
 }
@@ -911,7 +911,7 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
     if(!ctx->ties_in_any_order && n <= BUCKET_MAX_RECORDS && passes >= 2 && portions == 1)
     {
         *in_alt = 1;
-        return launch_bucket_sort(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, nullptr, 1, n, n, begin_bit, end_bit);
+        return launch_bucket_sort(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, nullptr, 1, n, n, nullptr, begin_bit, end_bit);
     }
 
     {
@@ -950,7 +950,7 @@ int csa_sort_pairs(csa_ctx* ctx, uint64_t* keys, uint64_t* keys_alt, void* vals,
     CSA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if(buckets && ctx->h_scalars[CSA_VERDICT_WORD] != 0)
         return sort_by_buckets(ctx, reinterpret_cast<u64*>(keys), reinterpret_cast<u64*>(keys_alt), vals, vals_alt, val_bytes, n, begin_bit, end_bit, counter, status, low_base, high_base,
-                               starts, ctx->h_scalars[CSA_VERDICT_WORD], in_alt);
+                               starts, ctx->h_scalars[CSA_VERDICT_WORD], found, in_alt);
     u64 skip[8];
     for(int p = 0; p < passes; ++p) skip[p] = skip_host[p];
 

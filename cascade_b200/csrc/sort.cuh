@@ -31,13 +31,13 @@ struct Bucket_Findings
 {
     u64 differ;         // bits in which keys differ
     u32 uneven;         // a bucket does not fit a block, or digit passes would skip so many digits that they are the faster way
-    u32 unused;
+    u32 left;           // buckets that turned out to be uneven inside
 };
 // The buckets' starts (1 << bits of them, and the end; zeroed before), the digit offsets of the passes by the lower low_bits of the bucket number and
 // by the others, and the verdict: `found`, and in *verdict (pinned host memory, once the stream has been waited for) the size of the largest bucket or 0
 // for uneven keys. Queued. least_digits: digits of 8 bits from begin_bit on in which the keys have to differ.
 int launch_bucket_plan(csa_ctx* ctx, const u64* keys, u64 n, int begin_bit, int end_bit, int bits, int low_bits, int least_digits, u32* starts, u64* low_base, u64* high_base,
                        Bucket_Findings* found, u64* verdict);
-// Every bucket (starts == nullptr: all n records) sorted by the key bits [begin_bit, top), stably; largest: no bucket holds more.
-int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, int begin_bit,
-                       int top);
+// Every bucket (starts == nullptr: all n records) sorted by the key bits [begin_bit, top), stably; largest: no bucket holds more. found->left is counted up.
+int launch_bucket_sort(csa_ctx* ctx, const u64* kin, u64* kout, const void* vin, void* vout, u32 val_bytes, const u32* starts, u32 buckets, u64 n, u64 largest, Bucket_Findings* found,
+                       int begin_bit, int top);
