@@ -28,7 +28,10 @@ namespace
 constexpr int TEXT_ITEMS = 16;              // consecutive symbols per thread of an encoding block
 constexpr int LOOKAHEAD = 64;               // a key of up to 64 bits needs at most 64 symbols
 constexpr int MAX_B1 = 10, MAX_B2 = 11;
-constexpr int SPLIT_BLOCK = 512, SPLIT_ITEMS = 16, SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
+constexpr int SPLIT_ITEMS = 16;             // records per thread of the second split
+// Threads of its blocks. Where a parent has 1024 children a tile of 16384 records writes runs of 16 of them and one of 8192 only 8: a build of 2e9 tokens 36.8 ms by blocks of 1024 threads, 38.0 by 512,
+// 1e9 18.3 and 18.9. With 512 children the smaller blocks, two to an SM, are 1 to 2 % faster (5e8: 8.84 and 9.00 ms).
+inline int split_block(const int b2) { return b2 >= 10 ? 1024 : 512; }
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
 // The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
 constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
@@ -452,7 +455,7 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
 // the children of one parent that holds everything.
 __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restrict__ counts, const u32 bins, const u32 n, const int one_level, u32* __restrict__ cursor,
                                                              u32* __restrict__ par_off, u32* __restrict__ tile0, u32* __restrict__ child_off,
-                                                             uint4* __restrict__ batches, u32* __restrict__ over, u32* __restrict__ left, const u32 p, Build_Counts* __restrict__ stats)
+                                                             uint4* __restrict__ batches, u32* __restrict__ over, u32* __restrict__ left, const u32 split_tile, const u32 p, Build_Counts* __restrict__ stats)
 {
     let_next_in();
     wait_for_previous();
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(1024) parent_offsets_kernel(const u32* __restr
         form_batches(room, s_off, bins, SHORT_SEGMENT, SHORT_BATCH, 0, 0, true, batches, stats, over, left);
         return;
     }
-    const u32 tiles = (c + SPLIT_TILE - 1) / SPLIT_TILE;
+    const u32 tiles = (c + split_tile - 1) / split_tile;
     u32 all_tiles;
     const u32 t0 = block_exclusive<1024>(tiles, warp_tot, all_tiles);
     if(t < bins) { par_off[t] = off; tile0[t] = t0; }
@@ -586,9 +589,11 @@ __device__ __forceinline__ u32 parent_of_block(const u32* __restrict__ first, co
     return *found;
 }
 
+template <int SPLIT_BLOCK>
 __global__ void __launch_bounds__(SPLIT_BLOCK) count_children_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ tile0,
                                                                     const u32 parents, const int bits, u32* __restrict__ counts)
 {
+    constexpr int SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
     __shared__ u32 cnt[1 << MAX_B2];
     __shared__ u32 found;
     const u32 children = 1u << bits;
@@ -634,11 +639,13 @@ __global__ void __launch_bounds__(1024) child_offsets_kernel(u32* __restrict__ c
     form_batches(room, s_off, children, SEGMENT, SORT_MOST, par_off[p], p * children, false, batches, stats, over, left);
 }
 
-constexpr size_t SPLIT_SMEM = size_t(SPLIT_TILE) * 8;
+template <int SPLIT_BLOCK> constexpr size_t SPLIT_SMEM = size_t(SPLIT_BLOCK * SPLIT_ITEMS) * 8;
 
-__global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ tile0,
+template <int SPLIT_BLOCK>
+__global__ void __launch_bounds__(SPLIT_BLOCK, 1024 / SPLIT_BLOCK) scatter_children_kernel(const u64* __restrict__ rec, const u32* __restrict__ par_off, const u32* __restrict__ tile0,
                                                                          const u32 parents, const int bits, u32* __restrict__ cursor, u64* __restrict__ out)
 {
+    constexpr int SPLIT_TILE = SPLIT_BLOCK * SPLIT_ITEMS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u64* const stage = reinterpret_cast<u64*>(smem_raw);
     __shared__ u32 cnt[1 << MAX_B2];
@@ -652,7 +659,7 @@ __global__ void __launch_bounds__(SPLIT_BLOCK, 2) scatter_children_kernel(const 
     const u32 end = par_off[p + 1], first = par_off[p] + (blockIdx.x - tile0[p]) * SPLIT_TILE;
     const u32 valid = end - first < u32(SPLIT_TILE) ? end - first : u32(SPLIT_TILE);
     u64 r[SPLIT_ITEMS];
-    u32 place2[SPLIT_ITEMS / 2];         // ranks below 8192, two a register
+    u32 place2[SPLIT_ITEMS / 2];         // ranks below 2^16, two a register
     #pragma unroll
     for(int i = 0; i < SPLIT_ITEMS; ++i)
     {
@@ -1848,21 +1855,27 @@ int launch_count_text(csa_ctx* ctx, const u16* T, u64 n, const u32* code, int bi
     return CSA_OK;
 }
 
-// The second split of `parents` buckets with n records in all (recA to recB).
-int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB, Build_Counts* counts)
+template <int BLOCK>
+int launch_split_kernels(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB, Build_Counts* counts)
 {
-    const unsigned tiles = unsigned(n / SPLIT_TILE + parents);
+    const unsigned tiles = unsigned(n / (BLOCK * SPLIT_ITEMS) + parents);
     const u32 children = 1u << b2;
-    CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, size_t(parents) * children * 4, ctx->stream));
-    count_children_kernel<<<tiles, SPLIT_BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2);
+    count_children_kernel<BLOCK><<<tiles, BLOCK, 0, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2);
     CSA_LAUNCH_CHECK(ctx);
     child_offsets_kernel<<<parents, 1024, 0, ctx->stream>>>(t.cnt2, t.par_off, parents, children, t.child_off, t.batches, t.over, t.left, counts);
     CSA_LAUNCH_CHECK(ctx);
     static std::atomic<bool> configured[64];
-    CSA_TRY(shared_bytes(ctx, scatter_children_kernel, SPLIT_SMEM, configured));
-    scatter_children_kernel<<<tiles, SPLIT_BLOCK, SPLIT_SMEM, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2, recB);
+    CSA_TRY(shared_bytes(ctx, scatter_children_kernel<BLOCK>, SPLIT_SMEM<BLOCK>, configured));
+    scatter_children_kernel<BLOCK><<<tiles, BLOCK, SPLIT_SMEM<BLOCK>, ctx->stream>>>(recA, t.par_off, t.tile0, parents, b2, t.cnt2, recB);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
+}
+
+// The second split of `parents` buckets with n records in all (recA to recB).
+int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* recA, u64* recB, Build_Counts* counts)
+{
+    CSA_CUDA(ctx, cudaMemsetAsync(t.cnt2, 0, (size_t(parents) << b2) * 4, ctx->stream));
+    return split_block(b2) == 1024 ? launch_split_kernels<1024>(ctx, t, parents, b2, n, recA, recB, counts) : launch_split_kernels<512>(ctx, t, parents, b2, n, recA, recB, counts);
 }
 
 // The second and the third launch take what the ones before leave: little or nothing as a rule, so their blocks are let in early.
@@ -1897,7 +1910,7 @@ int launch_prefix_sort(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tables&
     const bool one_level = ps.b1 == 0;
     const int bits = one_level ? ps.b2 : ps.b1;
     if(bits > 0) CSA_TRY(launch_count_text(ctx, T, n, t.code, bits, t.cnt1));
-    launch_early(parent_offsets_kernel, 1, 1024, 0, ctx->stream, t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, p, counts);
+    launch_early(parent_offsets_kernel, 1, 1024, 0, ctx->stream, t.cnt1, 1u << bits, u32(n), one_level ? 1 : 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, u32(split_block(ps.b2) * SPLIT_ITEMS), p, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(n) ? (launch_scatter_text<512, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA))
                           : (launch_scatter_text<128, false>(ctx, T, n, t.code, bits, one_level ? 1 : 0, 0, 0, t.cur1, recA)));
@@ -1940,7 +1953,7 @@ int launch_prefix_sort_part(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Ta
                             Build_Counts* counts)
 {
     CSA_CUDA(ctx, cudaMemsetAsync(counts, 0, sizeof(Build_Counts), ctx->stream));
-    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, 1, counts);
+    parent_offsets_kernel<<<1, 1024, 0, ctx->stream>>>(t.cnt1 + first_bin, bins, u32(size), 0, t.cur1, t.par_off, t.tile0, t.child_off, t.batches, t.over, t.left, u32(split_block(ps.b2) * SPLIT_ITEMS), 1, counts);
     CSA_LAUNCH_CHECK(ctx);
     CSA_TRY(wide_tiles(ps.n) ? (launch_scatter_text<512, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA))
                              : (launch_scatter_text<128, true>(ctx, T, ps.n, t.code, ps.b1, 0, first_bin, bins, t.cur1, recA)));

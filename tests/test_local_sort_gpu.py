@@ -60,3 +60,12 @@ def test_keys_that_lie_unevenly(ctx, oracle, n, kind):
 def test_one_split_by_small_and_by_wide_tiles(ctx, oracle, n):
     rng = np.random.default_rng(n)
     _check(ctx, oracle, np.minimum(rng.zipf(1.2, n), 50257))
+
+
+def test_a_split_into_a_thousand_children_of_a_parent(ctx):
+    """The larger blocks of the second split: from 2^29 suffixes on. Checked by the validator, which looks at every entry."""
+    from cascade_b200 import api
+    n = (1 << 29) + (1 << 25) + 7
+    T = api.gen_corpus_device(ctx, n, 3, 1024)
+    sa, _ = api.build_sa(ctx, T, n, 8)
+    assert api.validate_sa(ctx, T, n, sa)["ok"]
