@@ -521,6 +521,7 @@ int sort_oversize_children(csa_ctx* ctx, const Prefix_Sort& ps, const Prefix_Tab
     CSA_TRY(launch_split_by_size(ctx, head, in_alt ? posA : posB, M, ctx->d_scalars, front, n, b.scratch));
     CSA_CUDA(ctx, cudaMemcpyAsync(&counts->small, &counts->next_small, 4, cudaMemcpyDeviceToDevice, ctx->stream));
     CSA_TRY(set_build_count(ctx, &counts->next_small, 0));
+    CSA_TRY(set_build_count(ctx, &counts->wide, 1));
     return set_build_count(ctx, &counts->oversize, 0);
 }
 

@@ -1308,6 +1308,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         {
             const u32 size = cnt[e];
             if(size > 1) link[e] = u16(atomicAdd(&s_tied[size <= SMALL_GROUP ? 0 : 1], size));
+            if(size > NARROW_GROUP) counts->wide = 1;
         });
         __syncthreads();
         const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];
@@ -1652,7 +1653,12 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
                 {
                     #pragma unroll
                     for(int i = 0; i < ITEMS; ++i)
-                        if((tied >> i & 1u) && (pl[i] & PL_FIRST)) start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], pl[i] >> 13 & 16383u));
+                        if((tied >> i & 1u) && (pl[i] & PL_FIRST))
+                        {
+                            const u32 size = pl[i] >> 13 & 16383u;
+                            start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], size));
+                            if(size > NARROW_GROUP) counts->wide = 1;
+                        }
                 }
                 __syncthreads();
                 const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];

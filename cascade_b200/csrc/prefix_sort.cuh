@@ -9,6 +9,7 @@ constexpr int CODE_MAX_LEN = 22;
 
 // Groups of up to this many tied suffixes are ordered inside one block; larger ones go through the radix sort.
 constexpr u32 SMALL_GROUP = 256;
+constexpr u32 NARROW_GROUP = 15;
 // What an entry of the suffix array holds while its suffix is still tied (no position: a resident build's n is below 2^32 - 2^26).
 constexpr u32 SA_OPEN = 0xFFFFFFFFu;
 
@@ -25,6 +26,7 @@ struct Build_Counts
     u32 batches;        // runs of children that the local sort takes
     u32 crowded;        // and leaves to its second kernel
     u32 medium;         // runs for its third
+    u32 wide;           // not 0: a small group may have more than NARROW_GROUP members
     u32 now_small;      // entries that the last count by size found in small groups
     u32 large_depth;    // symbols that the suffixes of a large group share at least after the initial sort (launch_large_depth)
     u32 looked_at, lead_on, far_ties;       // what a sample of the small groups' entries says (launch_refine_by_text)

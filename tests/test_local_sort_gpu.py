@@ -56,6 +56,20 @@ def test_keys_that_lie_unevenly(ctx, oracle, n, kind):
     _check(ctx, oracle, T)
 
 
+# few tied suffixes, which a thread each compares where a group has up to 15 members: pieces shorter and longer than what is compared at once, and a copy that the text's end cuts off
+@pytest.mark.parametrize("length", [23, 49, 80, 300])
+@pytest.mark.parametrize("copies", [2, 3, 15, 16])
+@pytest.mark.parametrize("n", [17_003, 200_001])
+def test_few_ties(ctx, oracle, n, copies, length):
+    rng = np.random.default_rng(n + copies + length)
+    pieces = np.repeat(rng.integers(0, 60000, (8000 // (copies * length) + 1, length)), copies, axis=0)
+    T = rng.integers(0, 60000, n)
+    for k, at in enumerate(rng.permutation(n // (length + 1) - 1)[:len(pieces)]):
+        T[at * (length + 1):][:length] = pieces[k]
+    T[-length // 2:] = pieces[0][:length // 2 + length % 2]
+    _check(ctx, oracle, T)
+
+
 @pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, (1 << 19) + 1, 1_000_003])
 def test_one_split_by_small_and_by_wide_tiles(ctx, oracle, n):
     rng = np.random.default_rng(n)
