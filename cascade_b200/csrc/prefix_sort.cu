@@ -35,7 +35,8 @@ inline int split_block(const int b2) { return b2 >= 10 ? 1024 : 512; }
 // Children that start inside one chunk of slots belong to one block: one child as a rule.
 // The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
 constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
-constexpr int FREE_BITS = 4;                // of a key in a batch: its run of children has that many fewer bits than all of a parent's
+constexpr int FREE_BITS = 4;                // of a key in a batch take its slot's last bits. A run of children has that many fewer bits than all of a parent's, or, where a parent has few children, up to
+constexpr u32 FEW_CHILDREN = 4;             // so many, and the key's last bits are not looked at: what they told apart is left to the ties
 constexpr u32 SEGMENT = 64, SHORT_SEGMENT = 8;          // children whose batches one thread forms: they end with a segment
 constexpr u32 SHORT_BATCH = 1024;           // records of a batch of a text of one split, so that it has one for every SM
 constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
@@ -405,7 +406,7 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
     if(tid == 0) room.used = 0;
     for(u32 i = tid; i < children; i += blockDim.x)
     {
-        u32 a = i + 1, b = min(min(children, (i / segment + 1) * segment), i + max(1u, children >> FREE_BITS)) + 1;     // the last end with up to `most` records
+        u32 a = i + 1, b = min(min(children, (i / segment + 1) * segment), i + max(children >> FREE_BITS, min(children, FEW_CHILDREN))) + 1;     // the last end with up to `most` records
         while(b - a > 1)
         {
             const u32 m = (a + b) >> 1;
@@ -424,7 +425,7 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
         const u32 i = tid + h * blockDim.x;
         if(i >= children || !(room.heads[i >> 5] >> (i & 31u) & 1u)) continue;
         const u32 m = off[room.next[i]] - off[i];
-        if(m > SORT_MOST || (m && children >> FREE_BITS == 0))
+        if(m > SORT_MOST)
         {
             if(m <= MEDIUM_CAP) left[atomicAdd(&counts->medium, 1u)] = children_entry(first_child + i, 1);
             else
@@ -834,10 +835,10 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         const u32 whole = base - shift;
         u32* const bin = bins + turn * (CAP / 2);
         {
-            // keys from the start of the batch's range, which is cut to a power of two: FREE_BITS bits at the end are free
-            const u32 others = now.z & ((1u << MAX_B2) - 1), low = (now.z >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits);
+            // keys from the start of the batch's range, which is cut to a power of two
+            const u32 others = now.z & ((1u << MAX_B2) - 1), low = bits ? (now.z >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
             const int up = bits - (32 - __clz(others));
-            for_each([&](const u32 i) { k[i] = (k[i] - low) << up; });
+            for_each([&](const u32 i) { k[i] = ((k[i] - low) << up) & ~((1u << FREE_BITS) - 1); });
         }
         u32 seen = 0, number[ITEMS / 8] = {};       // the records' numbers in their bins, four bits each
         for_each([&](const u32 i)
@@ -1151,7 +1152,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
     load();
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
-        const u32 others = entry & ((1u << MAX_B2) - 1), low = (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits);
+        const u32 others = entry & ((1u << MAX_B2) - 1), low = bits ? (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
         const int up = bits - (32 - __clz(others));
         const bool more_work = work + gridDim.x < works;
         if(more_work) next_entry = over[over_cap - 1 - work - gridDim.x];

@@ -83,3 +83,14 @@ def test_a_split_into_a_thousand_children_of_a_parent(ctx):
     T = api.gen_corpus_device(ctx, n, 3, 1024)
     sa, _ = api.build_sa(ctx, T, n, 8)
     assert api.validate_sa(ctx, T, n, sa)["ok"]
+
+
+@pytest.mark.parametrize("n", [1_000_003, 4_000_001, 9_000_001, 13_000_003])
+def test_parents_of_few_children(ctx, n):
+    """Parts straight from the text, whose parents have two to sixteen children: batches of up to four of them, whose keys give up their last bits."""
+    from cascade_b200 import api
+    T = api.gen_corpus_device(ctx, n, 9, 512)
+    Th = T.cpu()
+    sa, st = api.build_sa_streamed(ctx, Th.view(torch.int16).numpy().view(np.uint16), n, 64)
+    assert st.host_parts == 0, "not straight from the text"
+    assert api.validate_sa(ctx, T, n, torch.from_numpy(sa).cuda())["ok"]
