@@ -32,7 +32,6 @@ constexpr int SPLIT_ITEMS = 16;             // records per thread of the second 
 // Threads of its blocks. Where a parent has 1024 children a tile of 16384 records writes runs of 16 of them and one of 8192 only 8: a build of 2e9 tokens 36.8 ms by blocks of 1024 threads, 38.0 by 512,
 // 1e9 18.3 and 18.9. With 512 children the smaller blocks, two to an SM, are 1 to 2 % faster (5e8: 8.84 and 9.00 ms).
 inline int split_block(const int b2) { return b2 >= 10 ? 1024 : 512; }
-// Children that start inside one chunk of slots belong to one block: one child as a rule.
 // The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
 constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
 constexpr int FREE_BITS = 4;                // of a key in a batch take its slot's last bits. A run of children has that many fewer bits than all of a parent's, or, where a parent has few children, up to
@@ -390,9 +389,9 @@ __global__ void __launch_bounds__(COUNT_BLOCK) count_long_text_kernel(const u16*
         if(cnt[i]) atomicAdd(&counts[i], cnt[i]);
 }
 
-// The batches of one parent, by a block of 1024 threads: off (shared memory) holds where its children start and where they end, from 0. A batch is a run of children of
-// one segment with up to `most` records, or a single one; its entry: the first slot, the records, the first child, the children. A child of more than
-// SORT_MOST goes to the other list. Whoever is called first ends its writes of off with a barrier.
+// The batches of one parent, by a block of 1024 threads: off (shared memory, a barrier behind its writes) holds where its children start and where they end, from 0. A batch is a run of
+// children of one segment with up to `most` records, or a single one; its entry: the first slot, the records, the children (children_entry). A child of more than SORT_MOST goes to
+// one of the other lists. only: there is no other parent. The batches of a segment follow from one another, so a thread forms them; bisecting and writing are side by side.
 // A run of children of one parent in one word: there are up to 2^21 children, and 2^MAX_B2 of a parent.
 static_assert(MAX_B1 + 2 * MAX_B2 <= 32, "an entry is a word");
 __device__ __forceinline__ u32 children_entry(const u32 first, const u32 count) { return first << MAX_B2 | (count - 1); }
@@ -1705,7 +1704,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
             }
             __syncthreads();        // the next batch reuses the shared arrays
         }
-        __syncthreads();            // a chunk may end in a child that was left or in an empty one: coff is still being read then
+        __syncthreads();            // a run may end in an empty child: coff is still being read then
     }
 }
 

@@ -55,7 +55,7 @@ struct Prefix_Tables
     u32* tile0;         // [parents + 1] first tile of each parent in the second split
     u32* cnt2;          // [parents][children] records by second digit, then running places
     u32* child_off;     // [parents * children + 1] where each child starts in the suffix array
-    uint4* batches;     // the local sort's batches (counts->batches of them): first slot, records, first child (parent * children + child), children
+    uint4* batches;     // the local sort's batches (counts->batches of them): first slot, records, the run of children
     u32* over;          // children that did not fit a block, by their indices, from the front; runs of children left to the local sort's second kernel from the back
     u32* left;          // runs left to its third
 };
