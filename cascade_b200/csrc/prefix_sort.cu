@@ -17,6 +17,7 @@
 // how many children do not fit a block and go through the radix sort instead.
 //
 // It stands for select_pivots, partition and the sort of initial_rank (src/GPU_SACA.cu:290-364, 737-826, 1111-1331).
+#include "batches.hpp"
 #include "prefix_sort.cuh"
 
 #include <algorithm>
@@ -32,12 +33,7 @@ constexpr int SPLIT_ITEMS = 16;             // records per thread of the second 
 // Threads of its blocks. Where a parent has 1024 children a tile of 16384 records writes runs of 16 of them and one of 8192 only 8: a build of 2e9 tokens 36.8 ms by blocks of 1024 threads, 38.0 by 512,
 // 1e9 18.3 and 18.9. With 512 children the smaller blocks, two to an SM, are 1 to 2 % faster (5e8: 8.84 and 9.00 ms).
 inline int split_block(const int b2) { return b2 >= 10 ? 1024 : 512; }
-// The local sort takes batches: runs of children of one parent with up to SORT_MOST records.
-constexpr u32 SORT_BLOCK = 256, SORT_ITEMS = 16, SORT_CAP = SORT_BLOCK * SORT_ITEMS, SORT_BLOCKS = 3, SORT_MOST = SORT_CAP - 4;
-constexpr int FREE_BITS = 4;                // of a key in a batch take its slot's last bits. A run of children has that many fewer bits than all of a parent's, or, where a parent has few children, up to
-constexpr u32 FEW_CHILDREN = 4;             // so many, and the key's last bits are not looked at: what they told apart is left to the ties
-constexpr u32 SEGMENT = 64, SHORT_SEGMENT = 8;          // children whose batches one thread forms: they end with a segment
-constexpr u32 SHORT_BATCH = 1024;           // records of a batch of a text of one split, so that it has one for every SM
+constexpr u32 SORT_BLOCKS = 3;               // of the local sort an SM
 constexpr u32 MEDIUM_CAP = 512 * 16;        // records of the largest child that a block holds
 
 // ---- the code ----------------------------------------------------------------------------------------------------------------
@@ -390,7 +386,7 @@ __global__ void __launch_bounds__(COUNT_BLOCK) count_long_text_kernel(const u16*
 }
 
 // The batches of one parent, by a block of 1024 threads: off (shared memory, a barrier behind its writes) holds where its children start and where they end, from 0. A batch is a run of
-// children of one segment with up to `most` records, or a single one; its entry: the first slot, the records, the children (children_entry). A child of more than SORT_MOST goes to
+// children of one segment with up to `most` records, no longer than longest_run, or a single child (batch_end); its entry: the first slot, the records, the children (children_entry). A child of more than SORT_MOST goes to
 // one of the other lists. only: there is no other parent. The batches of a segment follow from one another, so a thread forms them; bisecting and writing are side by side.
 // A run of children of one parent in one word: there are up to 2^21 children, and 2^MAX_B2 of a parent.
 static_assert(MAX_B1 + 2 * MAX_B2 <= 32, "an entry is a word");
@@ -403,16 +399,7 @@ __device__ __forceinline__ void form_batches(Batch_Room& room, const u32* off, c
     const u32 tid = threadIdx.x;
     if(tid < (1 << MAX_B2) / 32) room.heads[tid] = 0;
     if(tid == 0) room.used = 0;
-    for(u32 i = tid; i < children; i += blockDim.x)
-    {
-        u32 a = i + 1, b = min(min(children, (i / segment + 1) * segment), i + max(children >> FREE_BITS, min(children, FEW_CHILDREN))) + 1;     // the last end with up to `most` records
-        while(b - a > 1)
-        {
-            const u32 m = (a + b) >> 1;
-            if(off[m] - off[i] <= most) a = m; else b = m;
-        }
-        room.next[i] = u16(a);
-    }
+    for(u32 i = tid; i < children; i += blockDim.x) room.next[i] = u16(batch_end(off, i, children, segment, most));
     __syncthreads();
     for(u32 s = tid; s * segment < children; s += blockDim.x)
         for(u32 i = s * segment, end = min(children, (s + 1) * segment); i < end; i = room.next[i]) atomicOr(&room.heads[i >> 5], 1u << (i & 31u));
@@ -1792,17 +1779,10 @@ Prefix_Sort prefix_sort_plan(u64 n)
     return ps;
 }
 
-// Entries of the list of batches: two neighbours of one segment have more than SHORT_BATCH records together (SORT_MOST where there are two splits).
-static u64 most_batches(const Prefix_Sort& ps)
-{
-    const u64 all = u64(ps.parents) * ps.children;
-    return std::min(all, ps.b1 ? 2 * ps.n / SORT_MOST + all / SEGMENT + ps.parents : 2 * ps.n / SHORT_BATCH + all / SHORT_SEGMENT + 1);
-}
-
 size_t prefix_sort_table_bytes(const Prefix_Sort& ps)
 {
     const u64 all = u64(ps.parents) * ps.children;
-    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 4 + align_up256(all * 4) * 3 + align_up256((all + 1) * 4) + align_up256(most_batches(ps) * sizeof(uint4)) + 4096;
+    return align_up256(65536 * 4) * 2 + align_up256((size_t(1) << MAX_B1) * 4 + 4) * 4 + align_up256(all * 4) * 3 + align_up256((all + 1) * 4) + align_up256(most_batches(ps.parents, ps.children) * sizeof(uint4)) + 4096;
 }
 
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
@@ -1818,7 +1798,7 @@ bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t)
     t.child_off = cv.take<u32>(all + 1);
     t.over = cv.take<u32>(all);
     t.left = cv.take<u32>(all);
-    t.batches = cv.take<uint4>(most_batches(ps));
+    t.batches = cv.take<uint4>(most_batches(ps.parents, ps.children));
     return cv.ok;
 }
 

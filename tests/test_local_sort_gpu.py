@@ -1,6 +1,8 @@
 """The local sort's ways through a batch of children, by how many records share a key and how evenly the keys lie: bins that a thread's window orders, crowded
 bins, batches of more tied records than a block keeps, batches of many records of each key, of many keys close together, and large groups. Each array
 byte for byte against the oracle's."""
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -94,3 +96,16 @@ def test_parents_of_few_children(ctx, n):
     sa, st = api.build_sa_streamed(ctx, Th.view(torch.int16).numpy().view(np.uint16), n, 64)
     assert st.host_parts == 0, "not straight from the text"
     assert api.validate_sa(ctx, T, n, torch.from_numpy(sa).cuda())["ok"]
+
+
+@pytest.mark.parametrize("n,by_records", [(2_200_003, 2 * 2_200_003 // 4092 + 2048 // 64 + 32), (4_500_003, 2 * 4_500_003 // 4092 + 4096 // 64 + 64)])
+def test_runs_of_nearly_empty_children(ctx, oracle, monkeypatch, capfd, n, by_records):
+    """Two alphabets of 32 symbols by turns, one position in a hundred off: parents whose children hold nearly everything or nothing, and more batches than records and segments account for (4.5e6; the list
+    has an entry for every child)."""
+    rng = np.random.default_rng(n)
+    odd = (np.arange(n) & 1).astype(bool) ^ (rng.random(n) < 0.01)
+    T = np.where(odd, 65000, 0) + rng.integers(0, 32, n)
+    monkeypatch.setenv("CSA_DEBUG", "1")
+    _check(ctx, oracle, T)
+    batches = int(re.search(r"of (\d+) batches", capfd.readouterr().err).group(1))
+    assert batches > by_records or n < 4_000_000
