@@ -486,6 +486,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK, BLOCKS) order_buckets_kernel(cons
     u32* const words = reinterpret_cast<u32*>(val + CAP) + 4;           // [CAP + 16] in the order of the bins; four before it
     u32* const bin = words + CAP + 16;                                  // [CAP / 2]
     __shared__ u32 warp_tot[WARPS], crowd[CROWD_WORDS], crowded[MOST_CROWDED], s_crowded, s_fall;
+    __shared__ u32 s_untried;       // apart from s_fall, which a thread that is ahead sets while another still asks whether the bucket is tried
     const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     const u32 base = starts[blockIdx.x], m = starts[blockIdx.x + 1] - base;
     if(m == 0) return;
@@ -507,7 +508,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK, BLOCKS) order_buckets_kernel(cons
     for(u32 w = 0; w < WORDS; ++w) bin[tid + w * BLOCK] = 0;
     if(tid < CROWD_WORDS) crowd[tid] = 0;
     if(tid < 4) words[int(tid) - 4] = 0;
-    if(tid == 0) { s_crowded = 0; s_fall = found->left > blockIdx.x / 8 + 64; }
+    if(tid == 0) { s_crowded = 0; s_fall = 0; s_untried = found->left > blockIdx.x / 8 + 64; }
     u32 k[ITEMS];
     for_each([&](const u32 i, const u32 j)
     {
@@ -516,7 +517,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK, BLOCKS) order_buckets_kernel(cons
         k[i] = u32(((r[i] & compared) << (64 - top)) >> 32) & ~((1u << FROM_BITS) - 1);
     });
     __syncthreads();
-    if(s_fall)
+    if(s_untried)
     {
         sort_bucket_apart<ORDER_BLOCK, ITEMS, V>(smem_raw, keys_in, keys_out, vals_in, vals_out, base, m, compared, top, begin);
         return;

@@ -27,7 +27,7 @@ def _check(ctx, keys, vals, b0, b1):
 # buckets of 525 records on average where the keys fill their range, of more where they fill a part: up to 2044, 2556 and 4092 a block, beyond them the larger blocks
 @pytest.mark.parametrize("part", [1, 4, 6, 9])
 @pytest.mark.parametrize("bits,value", [((0, 64), torch.int32), ((0, 32), torch.int32), ((5, 45), torch.int64)])
-@pytest.mark.parametrize("kind", ["spread", "odd_place", "sorted", "pairs", "few_bits_behind", "heap_in_one"])
+@pytest.mark.parametrize("kind", ["spread", "odd_place", "sorted", "pairs", "few_bits_behind", "heap_in_one", "heaps_in_some", "heaps_in_most"])
 def test_long_lists(ctx, part, bits, value, kind):
     n, (b0, b1) = 4_300_001, bits
     g = torch.Generator(device="cuda").manual_seed(part)
@@ -44,5 +44,8 @@ def test_long_lists(ctx, part, bits, value, kind):
     elif kind == "heap_in_one":                             # one value in some hundred places, and as many keys right behind it
         keys[:900] = keys[0]
         keys[900:1500] = keys[0] + (torch.arange(600, device="cuda") << b0)
+    elif kind in ("heaps_in_some", "heaps_in_most"):        # buckets that turn out to be uneven, one in thirty and nearly all: the last are not tried once that is known
+        heaps = 280 if kind == "heaps_in_some" else 20_000
+        keys[:40 * heaps] = keys[:heaps].repeat(40)
     keys = keys[1:] if kind == "odd_place" else keys[:n].clone()          # an odd place starts on an odd 8-byte boundary
     _check(ctx, keys, torch.arange(n, device="cuda", dtype=value), b0, b1)
