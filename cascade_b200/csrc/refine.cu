@@ -364,8 +364,10 @@ __device__ __noinline__ void sample_ties(const u64* __restrict__ list, const u64
     }
 }
 
-// A list of few entries whose groups have up to NARROW_GROUP members: a thread for an entry compares its suffix with the others of its group, eight symbols at a time. What the kernel below takes
-// is mostly the fetching of its instructions and a chain of steps then: 2^18 tokens 14.7 us, this way 6.5; 2^24 24 and 8.5 (a build 459 and 441).
+// A list of few entries whose groups have up to NARROW_GROUP members, in the first round, up to symbol TEXT_DEPTH: a thread for an entry compares its suffix with the others of its group, eight symbols at a
+// time. What the kernel below takes is mostly the fetching of its instructions and a chain of steps then: 2^18 tokens 14.7 us, this way 6.5; 2^24 24 and 8.5 (a build 459 and 441). What is left to the
+// rounds behind that is alike for hundreds of symbols, and a thread would read all of them, of every other member, one after the other: 1e7 tokens with a passage of 1500 fifteen times 6.29 ms a build,
+// with one of 500 1.79; by the kernel below from the second round on 1.23 and 0.74. Two copies of 500 take 0.49 and 0.54.
 constexpr u32 NARROW_MOST = 1u << 15;
 
 // -1, 0, 1: the suffix at x comes before the one at y, shares symbols [from, to) with it, comes behind it.
@@ -448,7 +450,7 @@ __global__ void __launch_bounds__(RW_BLOCK, 4) refine_by_text_kernel(const u16* 
     wait_for_previous();
     if(counts->oversize != 0) return;           // children still wait for the radix sort: their records lie where `next` would go
     const u64 count = counts->small;
-    if(count <= NARROW_MOST && counts->wide == 0 && isa == nullptr && count <= most)
+    if(to <= TEXT_DEPTH && count <= NARROW_MOST && counts->wide == 0 && isa == nullptr && count <= most)
     {
         refine_narrow(T, n, from, to, list, u32(count), next, sa, sa40, counts);
         return;
