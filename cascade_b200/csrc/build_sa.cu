@@ -284,7 +284,7 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     u32* words = n > PACKED_MAX ? b.sa : nullptr;       // b.sa, once the positions are there; the output else
     CSA_TRY(launch_prefix_sort(ctx, b.ps, b.tab, T, recA, recB, words, sa40, p, b.counts, &b.front, &b.other, ev[1]));
     CSA_CUDA(ctx, cudaEventRecord(ev[2], ctx->stream));
-    const u64 depth0 = u64(b.ps.key_bits / CODE_MAX_LEN);       // symbols that tied suffixes share at least
+    const u64 depth0 = shared_symbols(b.ps);
     u64 depth = TEXT_DEPTH;
     // More tied suffixes than this are first looked through for groups that follow one another: those need not be compared.
     const u64 most_by_text = std::max(FOLLOWED_MIN, n / 4);

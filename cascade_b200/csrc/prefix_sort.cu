@@ -17,7 +17,6 @@
 // how many children do not fit a block and go through the radix sort instead.
 //
 // It stands for select_pivots, partition and the sort of initial_rank (src/GPU_SACA.cu:290-364, 737-826, 1111-1331).
-#include "batches.hpp"
 #include "prefix_sort.cuh"
 
 #include <algorithm>

@@ -1,5 +1,6 @@
 // Internal declarations of the resident build's generation 0: suffixes sorted by the first bits of their encoded symbols.
 #pragma once
+#include "batches.hpp"
 #include "common.cuh"
 
 // An order-preserving prefix code of the 16-bit symbols: entry s of a 65536-word table holds the symbol's code word in the top
@@ -37,11 +38,13 @@ struct Prefix_Sort
 {
     u64 n;
     int b1, b2;             // bits of the first and the second split; b1 = 0: one split (or none) of b2 bits
-    int key_bits;           // bits by which the suffixes end up sorted: b1 + 32
+    int key_bits;           // bits by which the suffixes end up sorted: b1 + 32, and up to FREE_BITS fewer where a parent has few children
     u32 parents, children;  // 1 << b1, 1 << b2
 };
 
 Prefix_Sort prefix_sort_plan(u64 n);
+// Symbols that suffixes still tied after the sort share at least.
+inline u64 shared_symbols(const Prefix_Sort& ps) { return u64((ps.key_bits - FREE_BITS) / CODE_MAX_LEN); }
 // Device bytes of the tables (code, counts, offsets) beside the two record buffers of n 8-byte records.
 size_t prefix_sort_table_bytes(const Prefix_Sort& ps);
 
@@ -61,7 +64,7 @@ struct Prefix_Tables
 };
 bool prefix_sort_carve(Carver& cv, const Prefix_Sort& ps, Prefix_Tables& t);
 
-// Orders the suffixes of T by the first key_bits bits of their encoding. recA and recB: n records each. sa or, where that is null, sa40 (5-byte entries) receives every
+// Orders the suffixes of T by the first key_bits bits of their encoding, up to FREE_BITS fewer where a parent has few children (shared_symbols). recA and recB: n records each. sa or, where that is null, sa40 (5-byte entries) receives every
 // suffix that is alone with its key, at its final place, and SA_OPEN elsewhere; the tied ones go to `list` (the record buffer
 // that is returned as *list; *records is the other one), small groups from the front, large ones from the back, as
 // (first slot of the group << 32) | position, group by group. p only says how many partitions the statistics tell apart. Nothing is read back.

@@ -894,7 +894,7 @@ int build_direct_parts(csa_ctx* ctx, const u16* T, const u64 n, const u32 p, con
     if(parts > DIRECT_MAX_PARTS) return CSA_OK;
     const double ms_counted = ms_since(t_start);
 
-    const u64 depth0 = u64(ps.key_bits / CODE_MAX_LEN);
+    const u64 depth0 = shared_symbols(ps);
     const cudaStream_t copy_stream = ctx->lane[0];
     const cudaEvent_t packed = ctx->lane_event[0], copied[2] = {ctx->lane_event[1], ctx->lane_event[2]};
     struct Drain { cudaStream_t s; ~Drain() { cudaStreamSynchronize(s); } } drain{copy_stream};       // no copy outlives the call, nor runs under the general way

@@ -98,6 +98,21 @@ def test_parents_of_few_children(ctx, n):
     assert api.validate_sa(ctx, T, n, torch.from_numpy(sa).cuda())["ok"]
 
 
+@pytest.mark.parametrize("n", [1_000_003, 4_000_001, 9_000_001])
+@pytest.mark.parametrize("copies", [2, 5, 15])
+def test_parents_of_few_children_with_ties(ctx, n, copies):
+    """The same with a tenth of the text in pieces that stand several times: what the keys' last bits told apart is told by the text."""
+    from cascade_b200 import api
+    rng = np.random.default_rng(n + copies)
+    pieces = np.repeat(rng.integers(0, 50000, (n // (10 * 23 * copies), 23)), copies, axis=0)
+    rng.shuffle(pieces)
+    T = np.concatenate([rng.integers(0, 50000, n - pieces.size), pieces.ravel()]).astype(np.uint16)
+    sa, st = api.build_sa_streamed(ctx, T, n, 64)
+    assert st.host_parts == 0 and st.active_after_gen0 > n // 20, "not straight from the text, or no ties"
+    Td = torch.from_numpy(np.concatenate([T, np.zeros(api.TEXT_PAD, np.uint16)]).view(np.int16)).cuda().view(torch.uint16)
+    assert api.validate_sa(ctx, Td, n, torch.from_numpy(sa).cuda())["ok"]
+
+
 @pytest.mark.parametrize("n,by_records", [(2_200_003, 2 * 2_200_003 // 4092 + 2048 // 64 + 32), (4_500_003, 2 * 4_500_003 // 4092 + 4096 // 64 + 64)])
 def test_runs_of_nearly_empty_children(ctx, oracle, monkeypatch, capfd, n, by_records):
     """Two alphabets of 32 symbols by turns, one position in a hundred off: parents whose children hold nearly everything or nothing, and more batches than records and segments account for (4.5e6; the list
