@@ -1135,6 +1135,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         }
     };
     load();
+    bool wide = false;          // told once a block: with a store a key to the one word, builds of near-duplicates wait for it
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
         const u32 others = entry & ((1u << MAX_B2) - 1), low = bits ? (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
@@ -1294,7 +1295,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         {
             const u32 size = cnt[e];
             if(size > 1) link[e] = u16(atomicAdd(&s_tied[size <= SMALL_GROUP ? 0 : 1], size));
-            if(size > NARROW_GROUP) counts->wide = 1;
+            wide |= size > NARROW_GROUP;
         });
         __syncthreads();
         const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];
@@ -1330,6 +1331,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         }
         __syncthreads();        // the next batch reuses the shared arrays
     }
+    if(__syncthreads_or(wide) && tid == 0) counts->wide = 1;
 }
 
 // ---- what the kernels above leave -------------------------------------------------------------------------------------------------------
@@ -1405,6 +1407,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
     let_next_in();
     wait_for_previous();
     const u32 works = counts->medium;
+    bool wide = false;
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
         const u32 entry = left[work], child0 = entry >> MAX_B2, last = (entry & ((1u << MAX_B2) - 1)) + 1;
@@ -1643,7 +1646,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
                         {
                             const u32 size = pl[i] >> 13 & 16383u;
                             start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], size));
-                            if(size > NARROW_GROUP) counts->wide = 1;
+                            wide |= size > NARROW_GROUP;
                         }
                 }
                 __syncthreads();
@@ -1692,6 +1695,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
         }
         __syncthreads();            // a run may end in an empty child: coff is still being read then
     }
+    if(__syncthreads_or(wide) && tid == 0) counts->wide = 1;
 }
 
 // Every oversize child is copied by the blocks of one grid row (blockIdx.y): keys = (first slot << 32) | key, vals = position.
