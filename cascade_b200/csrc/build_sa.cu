@@ -310,7 +310,8 @@ int build_core(csa_ctx* ctx, const u16* T, const u64 n, u32 p, const u64 seed, u
     st.partitions = c.partitions;
     st.max_partition = c.max_partition;
     st.active_after_gen0 = u64(c.small) + c.large;
-    if(debug) std::fprintf(stderr, "[csa] n=%llu key bits %d: tied after generation 0: %u in small groups, %u in large ones; %u of %u batches crowded, %u runs left\n", n, b.ps.key_bits, c.small, c.large, c.crowded, c.batches, c.medium);
+    if(debug) std::fprintf(stderr, "[csa] n=%llu key bits %d: tied after generation 0: %u in small groups, %u in large ones; %u of %u batches crowded, %u runs left, %u of %u first batches uneven\n", n, b.ps.key_bits, c.small, c.large, c.crowded, c.batches, c.medium, c.tries & 0xFFFFu,
+                           c.tries >> 16);
     u32 gen = 0;
     if(st.active_after_gen0) st.active_per_gen[gen++] = st.active_after_gen0;
     // The few large groups beside many small ones are ranked first, if some steps do it (LARGE_STEPS); a group that follows another is small.

@@ -727,6 +727,343 @@ template <bool PACKED> constexpr size_t SORT_SMEM = (3 * SORT_CAP + 40) * 4 + TI
 __device__ __forceinline__ void order(u32& a, u32& b) { const u32 t = min(a, b); b = max(a, b); a = t; }
 __device__ __forceinline__ void order(u32& a, u32& b, u32& c) { order(a, b); order(b, c); order(a, b); }
 
+// A warp's entries [4 q0, 4 q0 + 128) of a batch go out, four a lane: the wanted ones of v. whole: the slot of the array that the batch's slot 0 is. words: 160 of the warp's in shared memory.
+template <bool PACKED>
+__device__ __forceinline__ void write_four(u32* const words, const u32 whole, const u32 q0, const u32 wanted, const uint4& v, u32* __restrict__ sa, u8* __restrict__ sa40)
+{
+    const u32 lane = lane_id(), first = whole + 4 * (q0 + lane);
+    const u32 e[4] = {v.x, v.y, v.z, v.w};
+    if(!PACKED)
+    {
+        if(wanted == 15u) *reinterpret_cast<uint4*>(sa + first) = v;
+        else
+            #pragma unroll
+            for(u32 i = 0; i < 4; ++i)
+                if(wanted >> i & 1u) sa[first + i] = e[i];
+        return;
+    }
+    // four entries are 20 bytes, and begin on a word: the words of the warp's go out side by side
+    u32* const w = words + 5 * lane;
+    w[0] = v.x; w[1] = v.y << 8; w[2] = v.y >> 24 | v.z << 16; w[3] = v.z >> 16 | v.w << 24; w[4] = v.w >> 8;
+    const u32 all_four = __ballot_sync(0xFFFFFFFFu, wanted == 15u);
+    __syncwarp();
+    u32* const to = reinterpret_cast<u32*>(sa40) + u64(whole / 4 + q0) * 5;
+    #pragma unroll
+    for(u32 j = lane; j < 160; j += 32)
+        if(all_four >> (j / 5) & 1u) to[j] = words[j];
+    if(wanted != 15u)
+        #pragma unroll
+        for(u32 i = 0; i < 4; ++i)
+            if(wanted >> i & 1u)
+            {
+                u8* const b = sa40 + 5 * u64(first + i);
+                b[0] = u8(e[i]); b[1] = u8(e[i] >> 8); b[2] = u8(e[i] >> 16); b[3] = u8(e[i] >> 24); b[4] = 0;
+            }
+    __syncwarp();
+}
+
+// ---- batches that lie unevenly ----------------------------------------------------------------------------------------------------------
+
+constexpr u32 SORT_RESIDENT = 148 * SORT_BLOCKS, SORT_GRID = SORT_RESIDENT * 8;         // blocks of the local sort at a time, and at most
+constexpr u32 MOST_ROUNDS = (1u << (MAX_B1 + MAX_B2)) / SORT_GRID + 1, UNEVEN_WORDS = (MOST_ROUNDS + 8) / 32 + 2;          // batches of a block, and words of a bit for each and some behind them
+constexpr u32 SORT_POS = 4 + SORT_CAP + 20, SORT_BINS = SORT_POS + SORT_CAP + 16;       // words of shared memory before the positions, before the bins
+constexpr u32 STRETCH_BITS = 10;            // 1024 stretches: by 256, half as many crowded records again
+constexpr u32 MOST_COMPARED = 48;           // comparisons a record, on average; by 16, 8e6 tokens of which six in ten come from successors take 965 us instead of 880 (the kernel behind does the rest)
+// Of 256 records, those with the key of another beside them: from so many on the batch is left for its copies, where crowded_batches_kernel is not launched only from more on, and from fewer on if it cannot be
+// done here. Builds of near-duplicates, by 16, 24 and 40: 1.9e6 tokens (one split) 848, 846 and 832 us, 2.9e6 1027, 1045 and 1043, 5.8e6 1097, 1104 and 1117; of dependent tokens (six in ten, 8e6) 851, 814 and 808.
+constexpr u32 MANY_TWINS = 20, MANY_TWINS_SHORT = 48, SOME_TWINS = 16;
+
+// Keys of one batch from the start of the batch's range, which is cut to a power of two.
+struct Batch_Keys
+{
+    u32 low; int up;
+    __device__ __forceinline__ Batch_Keys(const u32 entry, const int bits)
+    {
+        const u32 others = entry & ((1u << MAX_B2) - 1);
+        low = bits ? (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
+        up = bits - (32 - __clz(others));
+    }
+    __device__ __forceinline__ u32 operator()(const u32 key) const { return ((key - low) << up) & ~((1u << FREE_BITS) - 1); }
+};
+
+// A batch or a child goes to one of the kernels behind the local sort, by one thread; copies: many of its records have the same key, which is the second one's work where it is launched (over_cap).
+__device__ __forceinline__ void leave_batch(const u32 children, const bool copies, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap, u32* __restrict__ left)
+{
+    if(copies && over_cap) over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children;
+    else left[atomicAdd(&counts->medium, 1u)] = children;
+}
+
+// A batch whose keys lie unevenly in its range, as those of texts do whose symbols depend on the ones before. Its records are counted in 1024 stretches of the range first, and a stretch gets two bins a
+// record. A record of a bin of up to WINDOW_BIN is compared with the others of its bin where it is; those of larger bins stand in a list, so that the threads of a warp have bins of one size as a rule.
+// The array's entries are put together in shared memory, the tied records go to the list of the build at once. false: a bin of more than SMALL_GROUP records, or too many comparisons.
+// What bounds it is the chain of ten steps between barriers, some 45,000 cycles for 2900 records where three blocks share an SM. Texts of 8e6 and 1.25e8 tokens, three in ten of which come from 32 successors of
+// the one before: 685 us and 5.3 ms a build; every record compared with all of its bin by even bins (which the kernel behind does) 800 us and 6.2 ms, by that way alone 720 us and 5.8 ms. Crowded bins
+// by a warp each, 16 steps a bin: 25,000 cycles of 75,000. Stretches with their least and largest key: a third fewer crowded records, but two more atomics for each.
+template <bool PACKED>
+__device__ __noinline__ bool spread_batch(const u64* __restrict__ rec, const u32 base, const u32 m, const u32 entry, const int bits, u32* __restrict__ sa, u8* __restrict__ sa40,
+                                          u64* __restrict__ list, Build_Counts* __restrict__ counts)
+{
+    constexpr u32 BLOCK = SORT_BLOCK, ITEMS = SORT_ITEMS, CAP = SORT_CAP, WARPS = BLOCK / 32, PER = CAP / BLOCK;
+    static_assert((1u << STRETCH_BITS) == 4 * BLOCK && 2 * CAP <= 1u << 13 && CAP <= 1u << 12 && PER % 4 == 0, "a thread sums four stretches; bins take 13 bits and slots 12");
+    static_assert(CAP / (WINDOW_BIN + 1) <= 2 * TIE_ROOM && WINDOW_BIN == 4 && SMALL_GROUP <= 256 && (1u << STRETCH_BITS) <= CAP, "the lists and tables have room; sizes have their bits");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    u32* const keys = reinterpret_cast<u32*>(smem_raw) + 4;             // [CAP] in the order of the bins; then the positions in their order
+    u32* const pos = reinterpret_cast<u32*>(smem_raw) + SORT_POS;       // [CAP] of crowded bins' records
+    u32* const bin = reinterpret_cast<u32*>(smem_raw) + SORT_BINS;      // [CAP] two 16-bit counts a word, then the bins' starts; then of every crowded record its bin, then where it goes
+    u16* const start = reinterpret_cast<u16*>(bin);
+    u32* const crowded = bin + CAP;                                     // of a crowded bin its first slot, its size - 1 << 12 and the crowded records before it << 20
+    u16* const tie = reinterpret_cast<u16*>(crowded);                   // [CAP] then, by place, of a tied record TIED and the number of its group's before it, of a group's first HEAD and where the group goes
+    u32* const words = crowded + 2 * TIE_ROOM + (threadIdx.x >> 5) * 160;       // PACKED: a warp's entries
+    u32* const stretch = pos;                                           // [1024] records, later those before << 16
+    __shared__ u32 warp_tot[WARPS], crowded_tot[WARPS];
+    __shared__ u32 s_crowds, s_crowded, s_work, s_left, s_tied, s_slot, s_wide;
+    const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, full = __shfl_sync(0xFFFFFFFFu, m / BLOCK, 0), rest = m % BLOCK, shift = base & 3u, end = shift + m, whole = base - shift;
+    const Batch_Keys batch_key(entry, bits);
+    auto for_each = [&](auto&& f)
+    {
+        #pragma unroll
+        for(u32 i = 0; i < ITEMS - 1; ++i)
+        {
+            if(i >= full) break;
+            f(i, tid + i * BLOCK);
+        }
+        if(tid < rest) f(ITEMS - 1, tid + full * BLOCK);
+    };
+    u32 k[ITEMS], p[ITEMS], at[ITEMS];          // at: the record's bin, and its number there << 13
+    for_each([&](const u32 i, const u32 j) { const u64 v = rec[base + j]; k[i] = batch_key(u32(v >> 32)); p[i] = u32(v); });
+    reinterpret_cast<uint4*>(stretch)[tid] = make_uint4(0, 0, 0, 0);
+    for(u32 i = tid; 4 * i < m; i += BLOCK) reinterpret_cast<uint4*>(bin)[i] = make_uint4(0, 0, 0, 0);
+    if(tid == 0) { s_work = 0; s_left = 0; s_tied = 0; s_wide = 0; }
+    __syncthreads();
+    for_each([&](const u32 i, const u32) { atomicAdd(stretch + (k[i] >> (32 - STRETCH_BITS)), 1u); });
+    __syncthreads();
+    {
+        const uint4 v = reinterpret_cast<const uint4*>(stretch)[tid];
+        const u32 sum = v.x + v.y + v.z + v.w, inc = warp_inclusive(sum);
+        if(lane == 31) warp_tot[warp] = inc;
+        __syncthreads();
+        const u32 x = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_tot[lane] : 0u) + inc - sum, y = x + v.x, z = y + v.y, w = z + v.z;
+        reinterpret_cast<uint4*>(stretch)[tid] = make_uint4(x << 16 | v.x, y << 16 | v.y, z << 16 | v.z, w << 16 | v.w);
+    }
+    __syncthreads();
+    for_each([&](const u32 i, const u32)
+    {
+        const u32 v = stretch[k[i] >> (32 - STRETCH_BITS)], b = 2 * (v >> 16) + __umulhi(k[i] << STRETCH_BITS, 2 * (v & 0xFFFFu));
+        const u32 old = atomicAdd(bin + (b >> 1), (b & 1) ? 0x10000u : 1u);
+        at[i] = b | ((b & 1) ? old >> 16 : old & 0xFFFFu) << 13;
+    });
+    __syncthreads();
+    {
+        u32 sum = 0, crowd = 0, work = 0, largest = 0;          // records, and crowded bins << 16; their records
+        auto see = [&](const u32 c)
+        {
+            sum += c;
+            if(c <= WINDOW_BIN) return;
+            sum += 1u << 16;
+            crowd += c;
+            work += c * c;
+            largest = max(largest, c);
+        };
+        #pragma unroll 1
+        for(u32 w = 0; w < PER && tid * PER + w < m; w += 4)
+        {
+            const uint4 v = *reinterpret_cast<const uint4*>(bin + tid * PER + w);       // no bins behind 2 m, and zeros up to a multiple of four words
+            see(v.x & 0xFFFFu); see(v.x >> 16); see(v.y & 0xFFFFu); see(v.y >> 16); see(v.z & 0xFFFFu); see(v.z >> 16); see(v.w & 0xFFFFu); see(v.w >> 16);
+        }
+        const u32 inc = warp_inclusive(sum), inc_crowd = warp_inclusive(crowd);
+        work = __reduce_add_sync(0xFFFFFFFFu, work);
+        if(lane == 31) { warp_tot[warp] = inc; crowded_tot[warp] = inc_crowd; }
+        if(lane == 0 && work) atomicAdd(&s_work, work);
+        if(largest > SMALL_GROUP) s_left = 1;
+        __syncthreads();
+        if(s_left || s_work > MOST_COMPARED * m) return false;
+        u32 run = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? warp_tot[lane] : 0u) + inc - sum;
+        u32 before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? crowded_tot[lane] : 0u) + inc_crowd - crowd, o = run >> 16;
+        run = shift + (run & 0xFFFFu);
+        auto note = [&](const u32 c)
+        {
+            if(c > WINDOW_BIN)
+            {
+                crowded[o++] = run | (c - 1) << 12 | before << 20;
+                before += c;
+            }
+            run += c;
+        };
+        auto starts = [&](const u32 c) { const u32 v = run | (run + (c & 0xFFFFu)) << 16; note(c & 0xFFFFu); note(c >> 16); return v; };
+        #pragma unroll 1
+        for(u32 w = 0; w < PER && tid * PER + w < m; w += 4)
+        {
+            uint4 v = *reinterpret_cast<const uint4*>(bin + tid * PER + w);
+            v.x = starts(v.x); v.y = starts(v.y); v.z = starts(v.z); v.w = starts(v.w);
+            *reinterpret_cast<uint4*>(bin + tid * PER + w) = v;
+        }
+        if(tid == BLOCK - 1)
+        {
+            s_crowds = o;
+            s_crowded = before;
+            if(m % 4 == 0) bin[m] = run;        // the end behind the last bin; else it is in the last words above
+        }
+    }
+    __syncthreads();
+    constexpr u32 CROWDED = 1u << 16;           // at, from here on: the record's slot, its number in the bin << 12, the bin's size - 1 << 14; or this
+    for_each([&](const u32 i, const u32)
+    {
+        const u32 b = at[i] & 0x1FFFu, number = at[i] >> 13, first = start[b], size = start[b + 1] - first, slot = first + number;
+        keys[slot] = k[i];
+        at[i] = slot | number << 12 | (size - 1) << 14;
+        if(size > WINDOW_BIN) { pos[slot] = p[i]; at[i] = CROWDED; }
+    });
+    __syncthreads();
+    #pragma unroll 1
+    for(u32 o = tid; o < s_crowds; o += BLOCK)
+    {
+        const u32 size = (crowded[o] >> 12 & 255u) + 1, before = crowded[o] >> 20;
+        #pragma unroll 4
+        for(u32 i = 0; i < size; ++i) bin[before + i] = o;
+    }
+    u32 tied = 0;               // of the groups whose first record the thread has
+    for_each([&](const u32 i, const u32)
+    {
+        const u32 slot = at[i] & 0xFFFu, number = at[i] >> 12 & 3u, last = at[i] >> 14;
+        if(last == 0 || at[i] == CROWDED) { if(last == 0) at[i] = slot; return; }
+        u32 less = 0, before = 0, group = 1;
+        #pragma unroll
+        for(u32 j = 0; j < WINDOW_BIN; ++j)
+        {
+            if(j > last) break;
+            const u32 other = keys[slot - number + j];
+            less += other < k[i];
+            if(j != number && other == k[i]) { ++group; before += j < number; }
+        }
+        at[i] = (slot - number + less + before) | before << 12 | (group - 1) << 14;        // its place, the same before it, how many others are tied with it
+        if(group > 1 && before == 0) tied += group;
+    });
+    __syncthreads();
+    const u32 count = s_crowded;
+    #pragma unroll 1
+    for(u32 t = tid; t < count; t += BLOCK)
+    {
+        const u32 e = crowded[bin[t]], first = e & 0xFFFu, stop = first + (e >> 12 & 255u) + 1, slot = first + t - (e >> 20), key = keys[slot];
+        u32 less = 0, upto = 0, before = 0;
+        #pragma unroll 4
+        for(u32 j = first; j < stop; ++j)
+        {
+            const u32 other = keys[j];
+            if(j == slot) before = upto - less;
+            less += other < key;
+            upto += other <= key;
+        }
+        const u32 group = upto - less, place = first + less + before;
+        // its place, its slot from there on << 12, and of a tied one the number of its group's before it or, of the first, behind it << 21
+        bin[t] = place | (slot + 256 - place) << 12 | (group == 1 ? 0u : before ? before << 21 | 1u << 29 : (group - 1) << 21 | 3u << 29);
+        if(group > 1 && before == 0)
+        {
+            tied += group;
+            if(group > NARROW_GROUP) s_wide = 1;
+        }
+    }
+    const u32 inc = warp_inclusive(tied);
+    u32 to = 0;
+    if(lane == 31 && inc) to = atomicAdd(&s_tied, inc);
+    to = __shfl_sync(0xFFFFFFFFu, to, 31) + inc - tied;
+    __syncthreads();
+    u32 got = 0;                // on its way while the places are written
+    if(tid == 0 && s_tied)
+    {
+        got = atomicAdd(&counts->small, s_tied);
+        if(s_wide) counts->wide = 1;
+    }
+    constexpr u32 TIED = 1u << 15, HEAD = 1u << 14;
+    for_each([&](const u32 i, const u32)
+    {
+        if(at[i] == CROWDED) return;
+        const u32 place = at[i] & 0xFFFu, before = at[i] >> 12 & 3u, others = at[i] >> 14;
+        keys[place] = p[i];
+        tie[place] = u16(others == 0 ? 0u : before ? TIED | before : TIED | HEAD | to);
+        if(others && before == 0) to += others + 1;
+    });
+    #pragma unroll 1
+    for(u32 t = tid; t < count; t += BLOCK)
+    {
+        const u32 x = bin[t], place = x & 0xFFFu, number = x >> 21 & 255u;
+        keys[place] = pos[place + (x >> 12 & 511u) - 256];
+        tie[place] = u16((x >> 29 & 1u) == 0 ? 0u : (x >> 30) == 0 ? TIED | number : TIED | HEAD | to);
+        if(x >> 30) to += number + 1;
+    }
+    if(tid == 0) s_slot = got;
+    __syncthreads();
+    u64* const ties = s_tied ? list + s_slot : nullptr;
+    #pragma unroll 1
+    for(u32 q0 = warp * 32; 4 * q0 < end; q0 += BLOCK)
+    {
+        const u32 q = q0 + lane;
+        const uint4 x = reinterpret_cast<const uint4*>(keys)[q];
+        u32 wanted = 4 * q < end ? 15u : 0u;
+        if(4 * q < shift) wanted = 15u << shift & 15u;
+        if(4 * q + 4 > end && wanted) wanted &= 15u >> (4 * q + 4 - end);
+        u32 v[4] = {x.x, x.y, x.z, x.w};
+        if(ties)
+        {
+            const uint2 w = reinterpret_cast<const uint2*>(tie)[q];
+            const u32 e[4] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16};
+            #pragma unroll
+            for(u32 i = 0; i < 4; ++i)
+                if((wanted >> i & 1u) && (e[i] & TIED))
+                {
+                    const u32 before = e[i] & HEAD ? 0u : e[i] & 255u, head = 4 * q + i - before;
+                    ties[(before ? tie[head] & (HEAD - 1) : e[i] & (HEAD - 1)) + before] = u64(whole + head) << 32 | v[i];
+                    v[i] = SA_OPEN;
+                }
+        }
+        write_four<PACKED>(words, whole, q0, wanted, make_uint4(v[0], v[1], v[2], v[3]), sa, sa40);
+    }
+    return true;
+}
+
+// The batches of a block that lie unevenly (a bit each in `uneven`). One of many batches goes to left_children_kernel, which does those of all blocks side by side: a block that has one when the others
+// have ended takes another 15 us (1.25e8 tokens 2289 us a build, this way 2270). Batches with many records of each key are another kernel's; where one after the other is, only one in eight is looked at.
+template <bool PACKED>
+__device__ __noinline__ void order_uneven(const u32* const uneven, const u64* __restrict__ rec, const uint4* __restrict__ batches, const u32 works, const int bits, u32* __restrict__ sa,
+                                          u8* __restrict__ sa40, u64* __restrict__ list, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap, u32* __restrict__ left)
+{
+    const u32 tid = threadIdx.x, rounds = (works - 1 - blockIdx.x) / gridDim.x + 1;
+    auto lies_unevenly = [&](const u32 r) { return (uneven[r / 32] >> (r % 32) & 1u) != 0; };
+    u32 all = 0;
+    for(u32 w = 0; w < (rounds + 31) / 32; ++w) all += __popc(uneven[w]);
+    if(8 * all < rounds)
+    {
+        for(u32 r = tid; r < rounds; r += SORT_BLOCK)
+            if(lies_unevenly(r)) leave_batch(__ldg(&batches[blockIdx.x + r * gridDim.x].z), false, counts, over, over_cap, left);
+        return;
+    }
+    u32 copied = 0;             // batches in a row that were left for their many records of each key
+    #pragma unroll 1
+    for(u32 r = 0; r < rounds; ++r)
+    {
+        if(!lies_unevenly(r)) continue;
+        if(copied >= 2)
+        {
+            if(tid < 7 && r + tid < rounds && lies_unevenly(r + tid)) leave_batch(__ldg(&batches[blockIdx.x + (r + tid) * gridDim.x].z), true, counts, over, over_cap, left);
+            r += 6;
+            copied = 1;
+            continue;
+        }
+        const uint4 batch = __ldg(batches + blockIdx.x + r * gridDim.x);
+        // many records of each key, or keys that lie unevenly: how many of 32 records, eight times, have the key of another?
+        if(16 * tid < batch.y) asm volatile("prefetch.global.L2 [%0];" :: "l"(rec + batch.x + 16 * tid));
+        const bool looked_at = tid < batch.y;
+        const u64 key = looked_at ? rec[batch.x + tid] >> 32 : ~u64(tid);
+        const u32 alike = __popc(__match_any_sync(0xFFFFFFFFu, key));
+        const u32 twins = __syncthreads_count(looked_at && alike > 1);
+        const bool copies = twins >= (over_cap ? MANY_TWINS : MANY_TWINS_SHORT);
+        copied = copies ? copied + 1 : 0;
+        const bool done = !copies && spread_batch<PACKED>(rec, batch.x, batch.y, batch.z, bits, sa, sa40, list, counts);
+        if(tid == 0 && !done) leave_batch(batch.z, twins >= SOME_TWINS, counts, over, over_cap, left);
+    }
+}
+
+// ---- the local sort ------------------------------------------------------------------------------------------------------------------------
+
 // A batch goes through four steps with a barrier behind each:
 //   * every record is counted in a bin, its key's place in the batch's range of keys by interpolation (two bins to a record), and keeps its number in the bin;
 //   * the bins' counts become their starts;
@@ -734,8 +1071,8 @@ __device__ __forceinline__ void order(u32& a, u32& b, u32& c) { order(a, b); ord
 //   * a thread orders the keys of four slots with those of the three slots before and behind, in registers: a bin of up to four records lies inside the window of every
 //     slot of it. A key carries its slot's last four bits in bits that it does not need, so min and max move whole records, and no two are equal. The four entries go out
 //     as one 16-byte store: the batch's slots begin with the first slot's place in its group of four.
-// The one or two larger bins of a batch, of up to 15 records, are ordered by a warp each. Batches with a bin of 16 or more (texts with long repeats), with crowded bins all over or
-// with too many tied records are left to crowded_batches_kernel where records of one key are many, to left_children_kernel else.
+// The one or two larger bins of a batch, of up to 15 records, are ordered by a warp each. Batches with a bin of 16 or more, with crowded bins all over or with too many tied records wait until the block has
+// tried its others (order_uneven): the registers of a kernel that orders them where they turn up cost even texts 4 to 5 %.
 // What bounds it: the issue of instructions (110 for 32 records, 59 % of the cycles) and the latency of dependent steps between barriers; so records stay in registers, no slow path is
 // unrolled, a block's next records and the batch after them are on their way early, and 256 threads with 16 records each share what a warp does per batch among more records than 512
 // with 8 do. A Zipf text of 1.25e8 symbols, the kernel alone: 0.66 ms; 512 threads with 8 records, two blocks an SM 0.78 and three (40 registers, spills) 1.0; two blocks of 256
@@ -751,20 +1088,22 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
     static_assert(WORDS % 4 == 0 && ITEMS % 8 == 0 && CROWD_WORDS <= BLOCK, "whole 16-byte pieces of bins, whole words of numbers, a word of marks a thread");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     u32* const keys = reinterpret_cast<u32*>(smem_raw) + 4;     // [CAP + 16] in the order of the bins; four words before it
-    u32* const pos = keys + CAP + 20;                           // [CAP + 16] the positions beside them; four words before it
-    u32* const bins = pos + CAP + 16;                           // [2][CAP / 2]: of every other batch
+    u32* const pos = reinterpret_cast<u32*>(smem_raw) + SORT_POS;       // [CAP + 16] the positions beside them; four words before it
+    u32* const bins = reinterpret_cast<u32*>(smem_raw) + SORT_BINS;     // [2][CAP / 2]: of every other batch
     u64* const tie = reinterpret_cast<u64*>(bins + CAP);        // [TIE_ROOM]
     u32* const words = reinterpret_cast<u32*>(tie + TIE_ROOM) + (threadIdx.x >> 5) * 160;       // PACKED: a warp's entries
     __shared__ u32 warp_tot[WARPS];
     __shared__ u32 crowd[CROWD_WORDS];              // a bit per slot: it belongs to a crowded bin
     __shared__ u32 crowded[MOST_CROWDED];           // such a bin's first slot and its size
     __shared__ u32 s_crowded, s_fall[2], s_ties, s_slot;
-    __shared__ u32 s_copies;                        // the batch was left for its many records of each key
-    __shared__ u32 s_before;                        // the children of the batch before
+    __shared__ u32 s_uneven[UNEVEN_WORDS];          // a bit per batch of the block: it lies unevenly (bits behind its last may stand, too)
+    __shared__ u32 s_some_uneven, s_round, s_next_round;    // which of the block's batches this one and the next are
+    __shared__ u32 s_before;                        // the round of the batch before
     const u32 tid = threadIdx.x, lane = lane_id(), warp = tid >> 5;
     let_next_in();
     wait_for_previous();
-    const u32 works = counts->batches;
+    const uint2 found = __ldcg(reinterpret_cast<const uint2*>(&counts->batches));
+    const u32 works = found.x;
     if(blockIdx.x >= works) return;
 
     u32 k[ITEMS], p[ITEMS];
@@ -793,11 +1132,6 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         }
         if(tid < rest) { const u64 v = at[full * BLOCK]; k[ITEMS - 1] = u32(v >> 32); p[ITEMS - 1] = u32(v); }
     };
-    auto leave = [&](const u32 children, const bool copies)        // by one thread
-    {
-        if(copies && over_cap) over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children;
-        else left[atomicAdd(&counts->medium, 1u)] = children;
-    };
     auto put = [&](const u32 slot, const u32 v)
     {
         if(!PACKED) { sa[slot] = v; return; }
@@ -806,24 +1140,31 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
     };
 
     uint4 now = __ldg(batches + blockIdx.x), then = make_uint4(0, 0, 0, 0);
-    u32 next = blockIdx.x + gridDim.x, fell = 0;        // fell: batches in a row that were left
-    if(next < works) then = __ldg(batches + next);
     load(now);
+    const u32 tries = tid == 0 && blockIdx.x % 8 ? found.y : 0u;
     for(u32 i = tid; i < CAP / 4; i += BLOCK) reinterpret_cast<uint4*>(bins)[i] = make_uint4(0, 0, 0, 0);
     if(tid < 4) keys[int(tid) - 4] = 0;
-    if(tid == 0) { s_fall[0] = 0; s_ties = 0; }
+    if(tid < UNEVEN_WORDS) s_uneven[tid] = 0;
+    if(tid == 0) { s_fall[0] = 0; s_ties = 0; s_round = 0; s_next_round = 1; s_some_uneven = 0; }
     u32 turn = 0, kept = 0;             // kept: tied records in `tie` from before the batch
-    __syncthreads();
-    while(true)
+    u32 next = blockIdx.x + gridDim.x, fell = 0;        // fell: batches in a row that are not done here
+    // One block in eight tries its first batch in any case. Where most of those that have come to an end did not do it, the others do not try their first seven (1e7 tokens of which most stand five times: some 40 us of 1320).
+    if(__syncthreads_or(2 * (tries & 0xFFFFu) > tries >> 16))
+    {
+        if(tid == 0) { s_uneven[0] = 127; s_some_uneven = 1; s_round = 7; s_next_round = 8; }
+        next += 7 * gridDim.x; fell = 7;
+        now.y = 0;
+        if(next - gridDim.x < works) { now = __ldg(batches + (next - gridDim.x)); load(now); }
+    }
+    if(next < works) then = __ldg(batches + next);
+    while(now.y)
     {
         const u32 base = now.x, m = now.y, shift = base & 3u, end = shift + m;      // the batch's records take the slots [shift, end)
         const u32 whole = base - shift;
         u32* const bin = bins + turn * (CAP / 2);
         {
-            // keys from the start of the batch's range, which is cut to a power of two
-            const u32 others = now.z & ((1u << MAX_B2) - 1), low = bits ? (now.z >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
-            const int up = bits - (32 - __clz(others));
-            for_each([&](const u32 i) { k[i] = ((k[i] - low) << up) & ~((1u << FREE_BITS) - 1); });
+            const Batch_Keys batch_key(now.z, bits);
+            for_each([&](const u32 i) { k[i] = batch_key(k[i]); });
         }
         u32 seen = 0, number[ITEMS / 8] = {};       // the records' numbers in their bins, four bits each
         for_each([&](const u32 i)
@@ -859,15 +1200,15 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         #pragma unroll
         for(u32 w = 0; w < WORDS; w += 4) reinterpret_cast<uint4*>(bins + (turn ^ 1) * (CAP / 2))[tid + w / 4 * BLOCK] = make_uint4(0, 0, 0, 0);
         if(tid < CROWD_WORDS) crowd[tid] = 0;
-        const bool crammed = s_ties > TIE_ROOM;             // left to the other kernel after all
+        const bool crammed = s_ties > TIE_ROOM;             // to be done again
         const u32 ties = crammed ? kept : s_ties;
         const bool write = ties != 0 && (crammed || ties + max(TIE_ROOM / 4, 2 * (ties - kept)) > TIE_ROOM);
         if(tid == 0)
         {
             s_crowded = 0;
             s_fall[turn ^ 1] = 0;
-            if(crammed) leave(s_before, true);
-            s_before = now.z;
+            if(crammed) { s_uneven[s_before >> 5] |= 1u << (s_before & 31u); s_some_uneven = 1; }
+            s_before = s_round;
             if(write) s_slot = atomicAdd(&counts->small, ties);
         }
         __syncthreads();
@@ -927,20 +1268,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
             if(tid < shift) keys[tid] = 0;                      // no key is below, or above those behind
             if(tid < 8) keys[end + tid] = 0xFFFFFFFFu;
         }
-        else if(warp == 0)
-        {
-            // many records of each key, or many keys close together: of 32 records of the batch, four times, do any have the same key?
-            bool twins = false;
-            #pragma unroll
-            for(u32 i = 0; i < 4; ++i)
-                if(i < full) twins |= __popc(__match_any_sync(0xFFFFFFFFu, k[i])) > 1;
-            const bool copies = __any_sync(0xFFFFFFFFu, twins);
-            if(lane == 0)
-            {
-                s_copies = copies;
-                leave(now.z, copies);
-            }
-        }
+        else if(tid == 0) { s_uneven[s_round >> 5] |= 1u << (s_round & 31u); s_some_uneven = 1; }
         __syncthreads();
 
         if(next < works) load(then);            // on their way while the batch is ordered
@@ -999,32 +1327,7 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
                             if((keys[s] ^ x[i + 1]) < 16) tie[o++] = u64(whole + 4 * q + i) << 32 | pos[s];
                     }
                 }
-                if(!PACKED)
-                {
-                    u32* const to = sa + whole + 4 * q;
-                    if(wanted == 15u) *reinterpret_cast<uint4*>(to) = make_uint4(v[0], v[1], v[2], v[3]);
-                    else
-                        #pragma unroll
-                        for(u32 i = 0; i < 4; ++i)
-                            if(wanted >> i & 1u) to[i] = v[i];
-                }
-                else
-                {
-                    // four entries are 20 bytes, and begin on a word: the words of the warp's go out side by side
-                    u32* const w = words + 5 * lane;
-                    w[0] = v[0]; w[1] = v[1] << 8; w[2] = v[1] >> 24 | v[2] << 16; w[3] = v[2] >> 16 | v[3] << 24; w[4] = v[3] >> 8;
-                    const u32 all_four = __ballot_sync(0xFFFFFFFFu, wanted == 15u);
-                    __syncwarp();
-                    u32* const to = reinterpret_cast<u32*>(sa40) + u64(whole / 4 + q0) * 5;
-                    #pragma unroll
-                    for(u32 j = lane; j < 160; j += 32)
-                        if(all_four >> (j / 5) & 1u) to[j] = words[j];
-                    if(wanted != 15u)
-                        #pragma unroll
-                        for(u32 i = 0; i < 4; ++i)
-                            if(wanted >> i & 1u) put(whole + 4 * q + i, v[i]);
-                    __syncwarp();
-                }
+                write_four<PACKED>(words, whole, q0, wanted, make_uint4(v[0], v[1], v[2], v[3]), sa, sa40);
             }
             #pragma unroll 1
             for(u32 o = WARPS - 1 - warp; o < crowds; o += WARPS)       // the last warps have the fewest windows
@@ -1054,10 +1357,16 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
         }
         if(next >= works) break;
         now = then;
-        // where one batch after the other is left, only one in eight is tried
-        fell = (fall && s_copies) || crammed ? fell + 1 : 0;
-        const u32 jump = fell < 2 ? 1u : 8u, passed = next + (tid + 1) * gridDim.x;
-        if(tid + 1 < jump && passed < works) leave(__ldg(&batches[passed].z), true);
+        // where one batch after the other is not done here, only one in eight is tried
+        fell = fall || crammed ? fell + 1 : 0;
+        const u32 jump = fell < 2 ? 1u : 8u;
+        if(tid == 0)
+        {
+            const u32 passed = s_next_round + 1;
+            if(jump == 8) { s_uneven[passed >> 5] |= 127u << (passed & 31u); s_uneven[(passed >> 5) + 1] |= u32(127ull << (passed & 31u) >> 32); }
+            s_round = s_next_round;
+            s_next_round += jump;
+        }
         next += jump * gridDim.x;
         then.y = 0;
         if(next < works) then = __ldg(batches + next);
@@ -1068,18 +1377,20 @@ __global__ void __launch_bounds__(SORT_BLOCK, SORT_BLOCKS) local_sort_kernel(con
     const u32 ties = crammed ? kept : s_ties;
     if(tid == 0)
     {
-        if(crammed) leave(now.z, true);
+        if(crammed) { s_uneven[s_round >> 5] |= 1u << (s_round & 31u); s_some_uneven = 1; }
+        if(blockIdx.x % 8 == 0) atomicAdd(&counts->tries, 1u << 16 | (s_uneven[0] & 1u));
         if(ties) s_slot = atomicAdd(&counts->small, ties);
     }
     __syncthreads();
     #pragma unroll 1
     for(u32 j = tid; j < ties; j += BLOCK) list[u64(s_slot) + j] = tie[j];
+    if(s_some_uneven) order_uneven<PACKED>(s_uneven, rec, batches, works, bits, sa, sa40, list, counts, over, over_cap, left);
 }
 
 // ---- crowded batches ------------------------------------------------------------------------------------------------------------------
 
 constexpr u32 CROWD_BLOCK = 256, CROWD_ITEMS = 16, CROWD_CAP = CROWD_BLOCK * CROWD_ITEMS;
-constexpr u32 MOST_ROUNDS = 16;             // a bin with more keys: the batch goes on to the kernel behind this one
+constexpr u32 MOST_KEYS = 16;               // a bin with more keys: the batch goes on to the kernel behind this one
 constexpr size_t CROWD_SMEM = size_t(CROWD_CAP) * (4 + 2 * 5 + 4);
 static_assert(CROWD_CAP > SORT_MOST && CROWD_CAP <= 4096, "a record's number in its batch takes 12 bits, with two flags and one pattern to spare in 16");
 
@@ -1195,7 +1506,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         u32 rounds = 1;
         for(bool more = open_ones != 0; more; ++rounds)
         {
-            if(rounds == MOST_ROUNDS) break;
+            if(rounds == MOST_KEYS) break;
             #pragma unroll 1
             for(u32 t = tid; t < open_ones; t += BLOCK)
             {
@@ -1224,7 +1535,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
             next_end = __ldg(child_off + (next_entry >> MAX_B2) + (next_entry & ((1u << MAX_B2) - 1)) + 1);
         }
         auto go_on = [&]() { entry = next_entry; base = next_base; m = next_end - next_base; if(more_work) load(); };
-        if(rounds == MOST_ROUNDS)
+        if(rounds == MOST_KEYS)
         {
             if(tid == 0) left[atomicAdd(&counts->medium, 1u)] = entry;
             go_on();
@@ -1382,7 +1693,8 @@ __device__ __forceinline__ void write_packed(u32* words, const u32* placed, cons
     }
 }
 
-// Single children of SORT_MOST to MEDIUM_CAP suffixes, and what the kernels above leave: one or two batches in ten thousand of a Zipf text. Every record is compared with all of its bin, of which there are as many as
+// Single children of SORT_MOST to MEDIUM_CAP suffixes, and what the kernels above leave: one or two batches in ten thousand where symbols are independent, those with bins of more than SMALL_GROUP records
+// or too many comparisons else. Every record is compared with all of its bin, of which there are as many as
 // records; a bin of one key takes no comparisons, and a bin of many records of several keys sends the batch through a sorting network. The chain of its steps takes 20 us whatever there is to do.
 // PACKED: the array is written to sa40 as 5-byte entries, else to sa.
 template <int BLOCK, int ITEMS, int BLOCKS, bool PACKED>
@@ -1874,7 +2186,7 @@ int launch_second_split(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b
     return split_block(b2) == 1024 ? launch_split_kernels<1024>(ctx, t, parents, b2, n, recA, recB, counts) : launch_split_kernels<512>(ctx, t, parents, b2, n, recA, recB, counts);
 }
 
-// The second and the third launch take what the ones before leave: little or nothing as a rule, so their blocks are let in early.
+// The second launch takes batches of many copies, the third what else the ones before leave: little or nothing as a rule, so their blocks are let in early.
 template <bool PACKED>
 int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2, u64 n, const u64* rec, u32* sa, u8* sa40, u64* list, Build_Counts* counts)
 {
@@ -1884,7 +2196,7 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
     CSA_TRY(shared_bytes(ctx, local_sort_kernel<PACKED>, SORT_SMEM<PACKED>, configured[0]));
     CSA_TRY(shared_bytes(ctx, crowded_batches_kernel<PACKED>, CROWD_SMEM, configured[1]));
     CSA_TRY(shared_bytes(ctx, left_children_kernel<512, 16, 2, PACKED>, LOCAL_SMEM<512, 16>, configured[2]));
-    launch_early(local_sort_kernel<PACKED>, unsigned(std::min<u64>(over_cap, 148 * SORT_BLOCKS * 8)), SORT_BLOCK, SORT_SMEM<PACKED>, ctx->stream, rec, t.batches, b2, sa, sa40, list, counts, t.over, crowds ? over_cap : 0u, t.left);
+    launch_early(local_sort_kernel<PACKED>, unsigned(std::min<u64>(over_cap, SORT_GRID)), SORT_BLOCK, SORT_SMEM<PACKED>, ctx->stream, rec, t.batches, b2, sa, sa40, list, counts, t.over, crowds ? over_cap : 0u, t.left);
     CSA_LAUNCH_CHECK(ctx);
     if(crowds)
     {

@@ -23,10 +23,11 @@ struct Build_Counts
     u32 oversize_records;
     u32 next_small;     // the same of the list being made
     u32 partitions;     // contiguous ranges of the suffix array, at most as many as asked for, that the first split's buckets form
-    u32 max_partition;  // suffixes of the largest
-    u32 batches;        // runs of children that the local sort takes
-    u32 crowded;        // and leaves to its second kernel
+    alignas(8) u32 batches;     // runs of children that the local sort takes
+    u32 tries;          // and, beside it, blocks that have tried their first by even bins << 16 and those of them that have it still to order
+    u32 crowded;        // and leaves to its second kernel: many of their records have the same key
     u32 medium;         // runs for its third
+    u32 max_partition;  // suffixes of the largest partition
     u32 wide;           // not 0: a small group may have more than NARROW_GROUP members
     u32 now_small;      // entries that the last count by size found in small groups
     u32 large_depth;    // symbols that the suffixes of a large group share at least after the initial sort (launch_large_depth)
