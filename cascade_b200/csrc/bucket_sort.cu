@@ -714,6 +714,8 @@ int launch_buckets(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vou
 
 // 31.25 M records: see the kernel; 4 and 1 M the same either way; 1e5 with few bits that differ 64 us by bucket_sort_kernel, 76 by order_buckets_kernel, which leaves such buckets after a try.
 constexpr u64 ORDER_MIN = u64(1) << 22;
+// The largest of its blocks only where a word holds all that is compared and the buckets are as large as those of random keys (seven standard deviations above their mean): 5.5e7 records by 32 bits 1647 and 1340 us,
+// but by 64 bits, where the registers do not do, 1584 and 1635 (two blocks an SM 1760), and of keys that stand eight or 64 times, whose buckets are left after a try, by 32 bits and with 8-byte values 2520 and 2810.
 
 template <typename V>
 int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* vout, const u32* starts, u32 buckets, u64 n, u64 largest, Bucket_Findings* found, int begin, int top)
@@ -723,7 +725,8 @@ int launch_buckets_of(csa_ctx* ctx, const u64* kin, u64* kout, const V* vin, V* 
     {
         if(largest <= ORDER_MOST<8>) return launch_order<8, 5, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
         if(largest <= ORDER_MOST<10>) return launch_order<10, 4, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
-        if(largest <= ORDER_MOST<16>) return launch_order<16, 2, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
+        const u64 mean = n / buckets, over = largest - mean;
+        if(largest <= ORDER_MOST<16> && top - begin <= WORD_BITS && over * over <= 49 * mean) return launch_order<16, sizeof(V) == 4 ? 3 : 2, V>(ctx, kin, kout, vin, vout, starts, buckets, found, compared, top, begin);
     }
     if(largest <= BUCKET_CAP<256>) return launch_buckets<256, 6, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);
     if(largest <= BUCKET_CAP<512>) return launch_buckets<512, 3, V>(ctx, kin, kout, vin, vout, starts, buckets, n, compared, top, begin);

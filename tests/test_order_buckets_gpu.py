@@ -24,7 +24,7 @@ def _check(ctx, keys, vals, b0, b1):
     assert torch.equal(v0[order], vo)
 
 
-# buckets of 525 records on average where the keys fill their range, of more where they fill a part: up to 2044, 2556 and 4092 a block, beyond them the larger blocks
+# buckets of 525 records on average where the keys fill their range, of more where they fill a part: up to 2044 and 2556 a block, beyond them the kernel of larger blocks
 @pytest.mark.parametrize("part", [1, 4, 6, 9])
 @pytest.mark.parametrize("bits,value", [((0, 64), torch.int32), ((0, 32), torch.int32), ((5, 45), torch.int64)])
 @pytest.mark.parametrize("kind", ["spread", "odd_place", "sorted", "pairs", "few_bits_behind", "heap_in_one", "heaps_in_some", "heaps_in_most"])
@@ -49,3 +49,17 @@ def test_long_lists(ctx, part, bits, value, kind):
         keys[:40 * heaps] = keys[:heaps].repeat(40)
     keys = keys[1:] if kind == "odd_place" else keys[:n].clone()          # an odd place starts on an odd 8-byte boundary
     _check(ctx, keys, torch.arange(n, device="cuda", dtype=value), b0, b1)
+
+
+# buckets of 2441 records on average: the largest of the blocks where a word holds all of a key that is compared, the kernel before it where it does not or keys stand many times; of 4091: beyond both
+@pytest.mark.parametrize("n", [40_000_003, (1 << 26) - 77])
+@pytest.mark.parametrize("bits,value", [((0, 32), torch.int32), ((9, 41), torch.int64), ((0, 64), torch.int32)])
+@pytest.mark.parametrize("kind", ["spread", "pairs", "eights"])
+def test_the_longest_lists(ctx, n, bits, value, kind):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    keys = torch.randint(-(1 << 62), 1 << 62, (n,), device="cuda", dtype=torch.int64, generator=g)
+    if kind == "pairs":                 # two of a key here and there, which stay in their order
+        keys[: n // 100] = keys[n // 2: n // 2 + n // 100]
+    elif kind == "eights":
+        keys = keys[torch.randint(0, n // 8, (n,), device="cuda", generator=g)]
+    _check(ctx, keys, torch.arange(n, device="cuda", dtype=value), *bits)
