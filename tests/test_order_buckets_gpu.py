@@ -24,10 +24,10 @@ def _check(ctx, keys, vals, b0, b1):
     assert torch.equal(v0[order], vo)
 
 
-# buckets of 525 records on average where the keys fill their range, of more where they fill a part: up to 2044 and 2556 a block, beyond them the kernel of larger blocks
+# buckets of 525 records on average where the keys fill their range, of more where they fill a part: up to 2044, 2556 and 4092 a block, beyond them the larger blocks
 @pytest.mark.parametrize("part", [1, 4, 6, 9])
 @pytest.mark.parametrize("bits,value", [((0, 64), torch.int32), ((0, 32), torch.int32), ((5, 45), torch.int64)])
-@pytest.mark.parametrize("kind", ["spread", "odd_place", "sorted", "pairs", "few_bits_behind", "heap_in_one", "heaps_in_some", "heaps_in_most"])
+@pytest.mark.parametrize("kind", ["spread", "odd_place", "sorted", "pairs", "few_bits_behind", "heap_in_one"])
 def test_long_lists(ctx, part, bits, value, kind):
     n, (b0, b1) = 4_300_001, bits
     g = torch.Generator(device="cuda").manual_seed(part)
@@ -44,10 +44,22 @@ def test_long_lists(ctx, part, bits, value, kind):
     elif kind == "heap_in_one":                             # one value in some hundred places, and as many keys right behind it
         keys[:900] = keys[0]
         keys[900:1500] = keys[0] + (torch.arange(600, device="cuda") << b0)
-    elif kind in ("heaps_in_some", "heaps_in_most"):        # buckets that turn out to be uneven, one in thirty and nearly all: the last are not tried once that is known
-        heaps = 280 if kind == "heaps_in_some" else 20_000
-        keys[:40 * heaps] = keys[:heaps].repeat(40)
     keys = keys[1:] if kind == "odd_place" else keys[:n].clone()          # an odd place starts on an odd 8-byte boundary
+    _check(ctx, keys, torch.arange(n, device="cuda", dtype=value), b0, b1)
+
+
+@pytest.mark.parametrize("part", [1, 6])
+@pytest.mark.parametrize("bits,value", [((0, 64), torch.int32), ((0, 32), torch.int32), ((5, 45), torch.int64)])
+@pytest.mark.parametrize("heaps", [280, 20_000])
+def test_heaps_of_equal_keys(ctx, part, bits, value, heaps):
+    """Buckets that turn out to be uneven, one in thirty and nearly all: the last are not tried once that is known."""
+    n, (b0, b1) = 4_300_001, bits
+    g = torch.Generator(device="cuda").manual_seed(part)
+    keys = torch.randint(0, 1 << 31, (n,), device="cuda", dtype=torch.int64, generator=g) << 32
+    keys += torch.randint(0, 1 << 32, (n,), device="cuda", dtype=torch.int64, generator=g)
+    if part > 1 and b1 < 64:
+        keys = (keys & ~((1 << b1) - 1)) | ((keys & ((1 << b1) - 1)) // 9 * part)
+    keys[:40 * heaps] = keys[:heaps].repeat(40)
     _check(ctx, keys, torch.arange(n, device="cuda", dtype=value), b0, b1)
 
 

@@ -108,3 +108,41 @@ def test_short_texts_of_few_symbols_that_depend(ctx, oracle, monkeypatch, capfd,
     T = _dependent(n, 0.7, n + symbols, 4) % symbols
     _, sa, _ = _build(ctx, T, monkeypatch, capfd)
     _check(oracle, T, sa)
+
+
+# the first and the last sizes of plans of two splits: parents and children double at 1537 suffixes a child, from 2^26 on at 2049; children are the smallest behind such a size and the largest before it
+@pytest.mark.parametrize("n", [12_591_103, 12_591_104, 25_182_208, 50_364_415, 50_364_416, (1 << 26) - 1, 1 << 26, 2049 << 15])
+def test_at_the_edges_of_the_plans(ctx, n):
+    from cascade_b200 import api
+    g = torch.Generator(device="cuda").manual_seed(n)
+    steps = 512
+    lanes = -(-n // steps)
+
+    def zipf(*shape):
+        u = torch.rand(shape, device="cuda", generator=g, dtype=torch.float64).clamp_(min=1e-12)
+        return u.pow_(-1 / 0.3).clamp_(max=50257).to(torch.int64)
+
+    table, out = zipf(50258, 32), torch.empty((steps, lanes), dtype=torch.int16, device="cuda")
+    now = zipf(lanes)
+    for s in range(steps):
+        out[s] = now.to(torch.int16)
+        followed = torch.rand(lanes, device="cuda", generator=g) < 0.5
+        now = torch.where(followed, table[now, torch.randint(0, 32, (lanes,), device="cuda", generator=g)], zipf(lanes))
+    T = torch.zeros(n + api.TEXT_PAD, dtype=torch.int16, device="cuda")
+    T[:n] = out.t().reshape(-1)[:n]
+    T = T.view(torch.uint16)
+    sa, _ = api.build_sa(ctx, T, n, 64)
+    assert api.validate_sa(ctx, T, n, sa)["ok"]
+
+
+# blocks of one batch each, the last one of a block, whose tied records are fewer or more than a block keeps (1024 of some 2900): symbols all as frequent, so that bins are small
+@pytest.mark.parametrize("share", [0.2, 0.3, 0.35, 0.4, 0.5])
+def test_ties_of_a_blocks_last_batch(ctx, monkeypatch, capfd, share):
+    from cascade_b200 import api
+    n = 6_000_011
+    rng = np.random.default_rng(int(100 * share))
+    pairs = np.repeat(rng.integers(0, 50000, (int(n * share) // 46, 23)), 2, axis=0)
+    rng.shuffle(pairs)
+    T = np.concatenate([rng.integers(0, 50000, n - pairs.size), pairs.ravel()])
+    Td, sa, at = _build(ctx, T, monkeypatch, capfd)
+    assert at["batches"] < 3552 and api.validate_sa(ctx, Td, n, sa)["ok"]
