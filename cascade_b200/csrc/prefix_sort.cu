@@ -1420,6 +1420,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
     u16* const lines = link + CAP;                                      // [CAP] records without a key after the first round, from the front; those that brought one in it, from the back
     __shared__ u32 warp_tot[BLOCK / 32];
     __shared__ u32 s_lines, s_tied[2], s_slot[2];
+    __shared__ u32 s_wide;      // told once a block: with a store a key to the one word, builds of near-duplicates wait for it
     const u32 tid = threadIdx.x, lane = lane_id();
     auto put = [&](const u32 slot, const u32 v)
     {
@@ -1446,7 +1447,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         }
     };
     load();
-    bool wide = false;          // told once a block: with a store a key to the one word, builds of near-duplicates wait for it
+    if(tid == 0) s_wide = 0;    // several barriers before it is told
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
         const u32 others = entry & ((1u << MAX_B2) - 1), low = bits ? (entry >> MAX_B2 & ((1u << bits) - 1)) << (32 - bits) : 0u;
@@ -1606,7 +1607,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         {
             const u32 size = cnt[e];
             if(size > 1) link[e] = u16(atomicAdd(&s_tied[size <= SMALL_GROUP ? 0 : 1], size));
-            wide |= size > NARROW_GROUP;
+            if(size > NARROW_GROUP) s_wide = 1;
         });
         __syncthreads();
         const u32 small_ones = s_tied[0], all_ones = small_ones + s_tied[1];
@@ -1642,7 +1643,7 @@ __global__ void __launch_bounds__(CROWD_BLOCK, 3) crowded_batches_kernel(const u
         }
         __syncthreads();        // the next batch reuses the shared arrays
     }
-    if(__syncthreads_or(wide) && tid == 0) counts->wide = 1;
+    if(tid == 0 && s_wide) counts->wide = 1;
 }
 
 // ---- what the kernels above leave -------------------------------------------------------------------------------------------------------
@@ -1710,6 +1711,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
     u16* const start = reinterpret_cast<u16*>(bin);
     u32* const coff = bin + CAP / 2 + 8;                                            // [children of the batch + 1] their offsets
     __shared__ u32 warp_tot[BLOCK / 32];
+    __shared__ u32 s_wide;
     __shared__ u32 s_tied[2], s_slot[2];            // records of small and of large groups in the batch, and their places in the list
     __shared__ u32 mixed[CAP / 32], s_crowded;      // a bit per bin: it holds several keys; whether any bin holds many records
     const u32 tid = threadIdx.x;
@@ -1719,7 +1721,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
     let_next_in();
     wait_for_previous();
     const u32 works = counts->medium;
-    bool wide = false;
+    if(tid == 0) s_wide = 0;    // a barrier of the first batch comes before it is told
     for(u32 work = blockIdx.x; work < works; work += gridDim.x)
     {
         const u32 entry = left[work], child0 = entry >> MAX_B2, last = (entry & ((1u << MAX_B2) - 1)) + 1;
@@ -1958,7 +1960,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
                         {
                             const u32 size = pl[i] >> 13 & 16383u;
                             start[pl[i] & 8191u] = u16(atomicAdd(&s_tied[(pl[i] & PL_SMALL) ? 0 : 1], size));
-                            wide |= size > NARROW_GROUP;
+                            if(size > NARROW_GROUP) s_wide = 1;
                         }
                 }
                 __syncthreads();
@@ -2007,7 +2009,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCKS) left_children_kernel(const u64*
         }
         __syncthreads();            // a run may end in an empty child: coff is still being read then
     }
-    if(__syncthreads_or(wide) && tid == 0) counts->wide = 1;
+    if(tid == 0 && s_wide) counts->wide = 1;
 }
 
 // Every oversize child is copied by the blocks of one grid row (blockIdx.y): keys = (first slot << 32) | key, vals = position.
