@@ -769,9 +769,9 @@ constexpr u32 MOST_ROUNDS = (1u << (MAX_B1 + MAX_B2)) / SORT_GRID + 1, UNEVEN_WO
 constexpr u32 SORT_POS = 4 + SORT_CAP + 20, SORT_BINS = SORT_POS + SORT_CAP + 16;       // words of shared memory before the positions, before the bins
 constexpr u32 STRETCH_BITS = 10;            // 1024 stretches: by 256, half as many crowded records again
 constexpr u32 MOST_COMPARED = 48;           // comparisons a record, on average; by 16, 8e6 tokens of which six in ten come from successors take 965 us instead of 880 (the kernel behind does the rest)
-// Of 256 records, those with the key of another beside them: from so many on the batch is left for its copies, where crowded_batches_kernel is not launched only from more on, and from fewer on if it cannot be
-// done here. Builds of near-duplicates, by 16, 24 and 40: 1.9e6 tokens (one split) 848, 846 and 832 us, 2.9e6 1027, 1045 and 1043, 5.8e6 1097, 1104 and 1117; of dependent tokens (six in ten, 8e6) 851, 814 and 808.
-constexpr u32 MANY_TWINS = 20, MANY_TWINS_SHORT = 48, SOME_TWINS = 16;
+// Of 256 records, those with the key of another beside them: from so many on the batch is left for its copies, and from fewer on if it cannot be done here. Builds of near-duplicates, by 16, 24 and 40: 2.9e6 tokens
+// 1027, 1045 and 1043 us, 5.8e6 1097, 1104 and 1117; of dependent tokens (six in ten, 8e6) 851, 814 and 808.
+constexpr u32 MANY_TWINS = 20, SOME_TWINS = 16;
 
 // Keys of one batch from the start of the batch's range, which is cut to a power of two.
 struct Batch_Keys
@@ -786,10 +786,10 @@ struct Batch_Keys
     __device__ __forceinline__ u32 operator()(const u32 key) const { return ((key - low) << up) & ~((1u << FREE_BITS) - 1); }
 };
 
-// A batch or a child goes to one of the kernels behind the local sort, by one thread; copies: many of its records have the same key, which is the second one's work where it is launched (over_cap).
+// A batch or a child goes to one of the kernels behind the local sort, by one thread; copies: many of its records have the same key, which is the second one's work.
 __device__ __forceinline__ void leave_batch(const u32 children, const bool copies, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap, u32* __restrict__ left)
 {
-    if(copies && over_cap) over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children;
+    if(copies) over[over_cap - 1 - atomicAdd(&counts->crowded, 1u)] = children;
     else left[atomicAdd(&counts->medium, 1u)] = children;
 }
 
@@ -1021,7 +1021,9 @@ __device__ __noinline__ bool spread_batch(const u64* __restrict__ rec, const u32
 }
 
 // The batches of a block that lie unevenly (a bit each in `uneven`). One of many batches goes to left_children_kernel, which does those of all blocks side by side: a block that has one when the others
-// have ended takes another 15 us (1.25e8 tokens 2289 us a build, this way 2270). Batches with many records of each key are another kernel's; where one after the other is, only one in eight is looked at.
+// have ended takes another 15 us (1.25e8 tokens 2289 us a build, this way 2270). So do those of texts of one split (over_cap 0), which are few and small: that kernel has their largest children to do in
+// any case, and does them beside those (1e5 tokens, three in ten from the successors, 158 us a build as here and 144 this way; 4e5 346 and 338, 2e6 484 and 492). Batches with many records of each key
+// are another kernel's; where one after the other is, only one in eight is looked at.
 template <bool PACKED>
 __device__ __noinline__ void order_uneven(const u32* const uneven, const u64* __restrict__ rec, const uint4* __restrict__ batches, const u32 works, const int bits, u32* __restrict__ sa,
                                           u8* __restrict__ sa40, u64* __restrict__ list, Build_Counts* __restrict__ counts, u32* __restrict__ over, const u32 over_cap, u32* __restrict__ left)
@@ -1030,7 +1032,7 @@ __device__ __noinline__ void order_uneven(const u32* const uneven, const u64* __
     auto lies_unevenly = [&](const u32 r) { return (uneven[r / 32] >> (r % 32) & 1u) != 0; };
     u32 all = 0;
     for(u32 w = 0; w < (rounds + 31) / 32; ++w) all += __popc(uneven[w]);
-    if(8 * all < rounds)
+    if(8 * all < rounds || over_cap == 0)
     {
         for(u32 r = tid; r < rounds; r += SORT_BLOCK)
             if(lies_unevenly(r)) leave_batch(__ldg(&batches[blockIdx.x + r * gridDim.x].z), false, counts, over, over_cap, left);
@@ -1055,7 +1057,7 @@ __device__ __noinline__ void order_uneven(const u32* const uneven, const u64* __
         const u64 key = looked_at ? rec[batch.x + tid] >> 32 : ~u64(tid);
         const u32 alike = __popc(__match_any_sync(0xFFFFFFFFu, key));
         const u32 twins = __syncthreads_count(looked_at && alike > 1);
-        const bool copies = twins >= (over_cap ? MANY_TWINS : MANY_TWINS_SHORT);
+        const bool copies = twins >= MANY_TWINS;
         copied = copies ? copied + 1 : 0;
         const bool done = !copies && spread_batch<PACKED>(rec, batch.x, batch.y, batch.z, bits, sa, sa40, list, counts);
         if(tid == 0 && !done) leave_batch(batch.z, twins >= SOME_TWINS, counts, over, over_cap, left);

@@ -69,7 +69,7 @@ def test_symbols_that_depend_on_the_one_before(ctx, oracle, monkeypatch, capfd, 
     _check(oracle, T, sa)
     if n >= 300_000 and share >= 0.3:           # of one block in eight
         assert at["uneven"] > 0, "even batches: nothing is shown"
-    if share < 0.9:             # children of more suffixes than a batch holds are among those left: some sixty of 2.5e6 suffixes
+    if share < 0.9 and n > 1 << 21:     # texts of one split leave them all to the last kernel; children of more suffixes than a batch holds, some sixty of 2.5e6, go to it too
         assert at["crowded"] + at["left"] < at["batches"] / 4
 
 
@@ -79,7 +79,7 @@ def test_passages_that_stand_several_times(ctx, oracle, monkeypatch, capfd, n, c
     T = _copies(n, copies, n + copies)
     _, sa, at = _build(ctx, T, monkeypatch, capfd)
     _check(oracle, T, sa)
-    if copies <= 3:
+    if copies <= 3 and n > 1 << 21:
         assert at["crowded"] + at["left"] < at["batches"] / 4
     if copies == 60 and n > 2_000_000:
         assert at["crowded"] > at["batches"] / 2, "not left for its copies"
