@@ -764,6 +764,10 @@ __device__ __forceinline__ void write_four(u32* const words, const u32 whole, co
 
 // ---- batches that lie unevenly ----------------------------------------------------------------------------------------------------------
 
+constexpr u32 LEFT_BLOCKS = 148 * 2;        // of left_children_kernel, all resident
+// Where large children are left for that kernel, batches are left beside them until it has so many. By 0, 148 and 296, a text of 4e6 tokens, uneven but independent: 508, 498 and 486 us, one in ten from the successors
+// 528, 521 and 530, three in ten 570, 563 and 576; 2.2e6 and one in ten 440, 437 and 451. Where none are left, a chain of that kernel's would be added: 4e6 Zipf tokens 206 us, with batches left 213.
+constexpr u32 LEFT_BESIDE = 148;
 constexpr u32 SORT_RESIDENT = 148 * SORT_BLOCKS, SORT_GRID = SORT_RESIDENT * 8;         // blocks of the local sort at a time, and at most
 constexpr u32 MOST_ROUNDS = (1u << (MAX_B1 + MAX_B2)) / SORT_GRID + 1, UNEVEN_WORDS = (MOST_ROUNDS + 8) / 32 + 2;          // batches of a block, and words of a bit for each and some behind them
 constexpr u32 SORT_POS = 4 + SORT_CAP + 20, SORT_BINS = SORT_POS + SORT_CAP + 16;       // words of shared memory before the positions, before the bins
@@ -1059,7 +1063,9 @@ __device__ __noinline__ void order_uneven(const u32* const uneven, const u64* __
         const u32 twins = __syncthreads_count(looked_at && alike > 1);
         const bool copies = twins >= MANY_TWINS;
         copied = copies ? copied + 1 : 0;
-        const bool done = !copies && spread_batch<PACKED>(rec, batch.x, batch.y, batch.z, bits, sa, sa40, list, counts);
+        // the first few go beside what the kernel behind has to do in any case
+        const bool room = __syncthreads_or(tid == 0 && !copies && __ldcg(&counts->medium) - 1 < LEFT_BESIDE - 1);
+        const bool done = !copies && !room && spread_batch<PACKED>(rec, batch.x, batch.y, batch.z, bits, sa, sa40, list, counts);
         if(tid == 0 && !done) leave_batch(batch.z, twins >= SOME_TWINS, counts, over, over_cap, left);
     }
 }
@@ -2207,7 +2213,7 @@ int launch_local_sort(csa_ctx* ctx, const Prefix_Tables& t, u32 parents, int b2,
         launch_early(crowded_batches_kernel<PACKED>, 148 * 3, CROWD_BLOCK, CROWD_SMEM, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.over, over_cap, t.left);
         CSA_LAUNCH_CHECK(ctx);
     }
-    launch_early(left_children_kernel<512, 16, 2, PACKED>, 148 * 2, 512, LOCAL_SMEM<512, 16>, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.left);
+    launch_early(left_children_kernel<512, 16, 2, PACKED>, LEFT_BLOCKS, 512, LOCAL_SMEM<512, 16>, ctx->stream, rec, b2, t.child_off, sa, sa40, list, n, counts, t.left);
     CSA_LAUNCH_CHECK(ctx);
     return CSA_OK;
 }

@@ -69,8 +69,8 @@ def test_symbols_that_depend_on_the_one_before(ctx, oracle, monkeypatch, capfd, 
     _check(oracle, T, sa)
     if n >= 300_000 and share >= 0.3:           # of one block in eight
         assert at["uneven"] > 0, "even batches: nothing is shown"
-    if share < 0.9 and n > 1 << 21:     # texts of one split leave them all to the last kernel; children of more suffixes than a batch holds, some sixty of 2.5e6, go to it too
-        assert at["crowded"] + at["left"] < at["batches"] / 4
+    if share < 0.9 and n > 1 << 21:     # texts of one split leave them all to the last kernel; children of more suffixes than a batch holds, some sixty of 2.5e6, go to it too, and where there are any, batches beside them until it has 148
+        assert at["crowded"] + at["left"] < at["batches"] / 4 + 148 < at["batches"]
 
 
 @pytest.mark.parametrize("copies", [2, 3, 5, 8, 15, 16, 17, 40, 60, 300])
@@ -80,7 +80,7 @@ def test_passages_that_stand_several_times(ctx, oracle, monkeypatch, capfd, n, c
     _, sa, at = _build(ctx, T, monkeypatch, capfd)
     _check(oracle, T, sa)
     if copies <= 3 and n > 1 << 21:
-        assert at["crowded"] + at["left"] < at["batches"] / 4
+        assert at["crowded"] + at["left"] < at["batches"] / 4 + 148 < at["batches"]
     if copies == 60 and n > 2_000_000:
         assert at["crowded"] > at["batches"] / 2, "not left for its copies"
 
